@@ -1,33 +1,39 @@
 // Shared device-side definitions of the BPE merge-loop engine (sm_100a).
 //
 // Data layout in HBM
-//   token stream : tiles of STBPE_TILE uint32 words; a tile keeps its live tokens compacted
-//                  at the front, its length lives in the tile record.  Bit 31 of a word
-//                  marks the first token of a row; a pair (i, i+1) is countable iff token
-//                  i+1 does not carry that bit (rows are the only pair-breaking boundary,
-//                  gpu_tokenizer/utils.py:586).
+//   token stream : tiles of STBPE_TILE tokens, 16 bits each while every id fits 15 bits and 32 bits
+//                  otherwise (stream.cuh).  The top bit of a token marks the first token of a row; a
+//                  pair (i, j) of consecutive live tokens is countable iff token j does not carry
+//                  that bit (rows are the only pair-breaking boundary, gpu_tokenizer/utils.py:586).
+//                  A merge drops a token by overwriting it with the hole value (all ones), so it
+//                  stores only the 16-byte units it changes; holes are squeezed out when a quarter
+//                  of the stream is holes (repack_copy_kernel).
 //   tile records : two versioned 32-byte records per tile {ver, len, first three live
-//                  tokens, last live token}.  During merge number m a tile is rewritten in
-//                  place by exactly one CTA, while neighbouring CTAs need its PRE-merge
-//                  head and tail.  A writer therefore fills the record with the older
+//                  tokens, last two live tokens}.  During merge number m a tile is rewritten in
+//                  place by exactly one warp, while the warps of neighbouring tiles need its
+//                  PRE-merge head and tail.  A writer therefore fills the record with the older
 //                  version and stamps it m; readers use the record with the largest
 //                  version below m, which nobody writes during merge m.
 //   pair table   : open addressing, linear probing, 16-byte slots {key = (a<<32)|b,
 //                  int64 count}.  Keys are never removed; a count may return to zero.
-//   block maxima : best (count, smallest key) of every block of 256 slots, and of every
-//                  256 blocks above that; only blocks touched by a merge are recomputed, the
-//                  arg-max reduces the few top-level maxima.
+//   candidates   : (one rank) the slots of all pairs at or above a threshold in selection order, a few
+//                  hundred of the millions.  An add that lifts a pair over the threshold appends its
+//                  slot, so the best pair is the best of the list until the list has run dry; then a
+//                  scan of the table sets a lower threshold (candidate kernels in kernels.cuh).
+//   block maxima : (several ranks) best (count, smallest key) of every block of slots.  An add that may
+//                  change the maximum of its block sets the block's bit in a bitmap, and only those
+//                  blocks are recomputed; the arg-max reduces the block maxima.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#define STBPE_TILE 1024  // tokens per tile: one consumer warp owns a whole tile
+#define STBPE_TILE 1024  // tokens per tile: one warp owns a whole tile, 32 consecutive tokens per lane
 #define STBPE_NONE 0xFFFFFFFFu
 #define STBPE_FLAG 0x80000000u
 #define STBPE_IDMASK 0x7FFFFFFFu
 #define STBPE_EMPTY 0xFFFFFFFFFFFFFFFFull
-#define STBPE_BLK 256
 #define STBPE_PROWS 16384  // rows of the pair filter: pair keys are hashed onto them (three hashes)
+#define STBPE_PPITCH (STBPE_PROWS + 32)  // words per group of 32 tiles: the rows and the wildcard word (row STBPE_PROWS)
 #define STBPE_MAX_PROBE (1u << 20)
 
 // device error bits
@@ -36,7 +42,9 @@
 #define STBPE_DERR_LTABLE_FULL 4u
 #define STBPE_DERR_KEY_MISSING 8u
 #define STBPE_DERR_BAD_ID 16u
+#define STBPE_DERR_TIMEOUT 32u
 #define STBPE_DERR_DENSE_OVERFLOW 64u
+#define STBPE_DERR_NARROW 128u  // an id does not fit the 16-bit stream: the host widens it and packs again
 
 typedef unsigned long long u64;
 typedef long long i64;
@@ -48,12 +56,13 @@ struct __align__(16) Slot {
 
 struct __align__(16) TileRec {
     int ver;  // merge number that wrote this record; 0 = written at load; <0 = never written
-    int len;
+    int len;  // live tokens when the record was written; exact below 3, otherwise only known to be >= 3
     uint32_t head[3];
     uint32_t tail;   // last live token
     uint32_t tail2;  // second to last live token (STBPE_NONE when len < 2)
     uint32_t pad;
 };
+static_assert(sizeof(TileRec) == 32, "merge_tile writes records word by word");
 
 struct DevState {
     int cur_a, cur_b, cur_new;
@@ -62,7 +71,7 @@ struct DevState {
     i64 cur_count;
     int merges_done, target, base_vocab, stopped;
     int stop_reason;
-    unsigned int n_dirty;
+    int run_exit;              // why the last loop_kernel launch returned (STBPE_EXIT_*)
     unsigned int error;
     unsigned int ticket;
     u64 n_keys;
@@ -74,16 +83,42 @@ struct DevState {
     unsigned int n_ltouched;   // entries of the rank-local delta table awaiting the drain
     unsigned int n_lkept;      // entries the last drain had to keep (outbox chunk full)
     i64 export_n;
-    unsigned int n_dirty2;     // super-blocks whose maximum must be recomputed
-    unsigned int pad1;
-    int n_work;                // tiles on this merge's worklist; < 0 = every tile
-    int pad3;
-    unsigned int n_fixups;     // partners dropped in a tile the merge did not visit (statistics)
-    int pad2;
+    int n_work;                // tiles visited by the last merge; < 0 = every tile
+    unsigned int n_fixups;     // matches whose dropped token sits in another tile than their head (statistics)
     int exchange_only;         // multi-GPU: deltas still in flight, the next round only exchanges
     int round_incomplete;      // multi-GPU: this rank saw a full chunk or kept entries this round
-    u64 tile_bytes_in;         // merge kernel: bytes its bulk copies and record look-ups brought in ...
-    u64 tile_bytes_out;        // ... and bytes it stored (rewritten tile parts and records), since the load
+    int forced_done;           // host-given merges the last loop_kernel launch applied
+    unsigned int n_cand;       // entries of the candidate list (may exceed its capacity: then it is incomplete)
+    i64 theta_count;           // the list holds every pair with a larger count, or with this count and
+    u64 theta_key;             // a key below this one
+    int cand_state;            // STBPE_CAND_*
+    int peek_valid;            // peek_key / peek_count are the best pair of the table as it stands
+    // range a too coarse threshold search has to be continued in (cand_decide_kernel)
+    i64 refine_lo, refine_hi;
+    u64 refine_klo, refine_khi;
+    i64 refine_above;          // pairs above the range
+    u64 tile_bytes_in;         // merges: bytes of tiles and records read ...
+    u64 tile_bytes_out;        // ... and bytes stored (rewritten 16-byte units and records), since the load
+};
+#define STBPE_EXIT_STOP 0      // a stop rule fired (DevState::stop_reason) or the given merges are done
+#define STBPE_EXIT_REPACK 1    // a quarter of the stream is holes
+#define STBPE_EXIT_FILTER 2    // the pair filter starts to pay: build it
+#define STBPE_EXIT_WIDEN 3     // the next id does not fit 15 bits
+#define STBPE_EXIT_REFILL 4    // the candidate list has run dry or over
+#define STBPE_CAND_NONE 0      // no candidate list (fresh count)
+#define STBPE_CAND_READY 1
+#define STBPE_CAND_REFINE 2    // the threshold search needs another pass
+#define STBPE_CAND_CAP 4096    // capacity of the candidate list
+#define STBPE_CAND_MOST 1024   // a new threshold admits at most this many pairs ...
+#define STBPE_CAND_LEAST 256   // ... and, if it can, at least this many
+#define STBPE_CAND_BUCKETS 2048
+
+// Synchronisation block of loop_kernel (loop.cuh), zeroed before every launch.
+struct __align__(128) LoopSync {
+    unsigned int arrived;                   // CTAs whose deltas are in the table, over all merges
+    unsigned int pad0[31];
+    unsigned int chosen;                    // CTAs that have read the candidates' counts, over all merges
+    unsigned int pad1[31];
 };
 
 // Peer mailboxes (multi-GPU exchange over NVLink peer memory, no library collective).  Every rank owns
@@ -102,31 +137,32 @@ static_assert(sizeof(MailHeader) <= STBPE_MAIL_HEADER_BYTES, "mailbox header doe
 
 struct EngineDev {
     unsigned char *mail[STBPE_MAX_PEERS];  // mailbox of every rank ([rank] = own), or null
-    uint32_t *tiles;
-    TileRec *recs;  // 2 per tile
+    void *tiles;            // token stream: uint16_t or uint32_t tokens (stream.cuh)
+    TileRec *recs;          // 2 per tile
+    unsigned int *tile_live;  // live tokens per tile
     int n_tiles;
     Slot *table;
     u64 mask;
     int slot_bits;  // slot index bits below the table slice of a partition (slots = slices << slot_bits)
+    unsigned int *cand;        // slots of the candidates
+    unsigned int *cand_hist;   // STBPE_CAND_BUCKETS counters of the threshold search
     Slot *blockmax;
-    unsigned int *dirty_flag;
-    unsigned int *dirty_list;
+    unsigned int *dirty_bits;  // one bit per block
     unsigned int n_blocks;
-    // presence[r][w]: bit t of word w of row r says "a pair whose key hashes to r may start in tile
-    // 32*w + t" (the tile of the pair's left token; set when such a pair comes into being, never
-    // cleared until the next re-pack).  A Bloom filter with three hashes per pair: false positives
+    int blk_shift;             // log2 of the slots per block
+    // presence[w * PPITCH + r]: bit t says "a pair whose key hashes to row r may have a token in tile
+    // 32*w + t" (set when such a pair comes into being, never cleared until the next re-pack).  The rows
+    // of 32 tiles lie together (64 KB): entering a pair stays inside one page, where a row-major layout
+    // took a TLB miss per entry, and the look-up of a merge reads three words per 32 tiles.
+    // A pair whose two tokens sit in different tiles is entered for both, so a merge finds every tile
+    // it has to change by itself.  A Bloom filter with three hashes per pair: false positives
     // cost a wasted visit, never a missed one.  Row STBPE_PROWS is a wildcard: tiles that every
     // merge visits because the pair that starts at their last token is not known exactly (their
     // last token is the result of a run of equal tokens that ran on into the next tile).
     unsigned int *presence;
-    unsigned int presence_words;  // words per row
-    unsigned int *cand_bits;      // tiles the current merge must visit
-    unsigned int *worklist;
-    Slot *supermax;             // best entry of every 256 blocks (second level of the arg-max)
-    unsigned int *dirty2_flag;
-    unsigned int *dirty2_list;
-    unsigned int n_super2;
+    unsigned int presence_groups;  // groups of 32 tiles there is room for
     DevState *st;
+    LoopSync *sync;
     int32_t *merges;
     i64 *merge_counts;
     i64 *live_before;
@@ -198,22 +234,25 @@ __device__ __forceinline__ int owner_of(u64 key, int world) {
 // residue modulo the number of ranks: their slices are numbered densely (partition / ranks), so the
 // whole table is in use whatever the number of ranks.
 __device__ __forceinline__ unsigned int slice_of(const EngineDev &e, unsigned int part) {
-    return part / (unsigned int)e.world;
+    return e.world == 1 ? part : part / (unsigned int)e.world;
 }
-// first slot probed for a key: its partition's slice in the top bits, then the top bits of the 64-bit mix
-__device__ __forceinline__ u64 slot_of(const EngineDev &e, u64 key) {
-    return ((u64)slice_of(e, part_of(key)) << e.slot_bits) | (mix64(key) >> (64 - e.slot_bits));
+__device__ __forceinline__ unsigned int hash32(u64 key) {
+    unsigned int a = (unsigned int)(key >> 32), b = (unsigned int)key;
+    unsigned int h = a * 0x9E3779B1u ^ (b * 0x85EBCA77u + 0x7F4A7C15u);
+    h ^= h >> 15;
+    h *= 0x2C1B3C6Du;
+    h ^= h >> 13;
+    return h;
 }
 
-// Programmatic dependent launch: inside the captured loop every kernel is launched with the
-// programmatic-serialisation attribute, so its CTAs may become resident while the kernel before it
-// still runs.  dep_release() lets the next kernel's CTAs be scheduled as soon as all CTAs of this
-// one have started; dep_wait() returns when the kernel before this one has completed and its writes
-// are visible.  Every thread executes dep_wait() before it touches global memory or returns (a
-// kernel that ended without waiting would complete before its predecessor).  Launched without the
-// attribute both are no-ops.
-__device__ __forceinline__ void dep_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// first slot probed for a key: its partition's slice in the top bits, then the top bits of a 32-bit hash (32-bit
+// arithmetic: the 64-bit finaliser cost a fifth of the time of a merge's table adds)
+__device__ __forceinline__ u64 slot_in_slice(const EngineDev &e, u64 top, u64 key) {
+    return top | (u64)(hash32(key) >> (32 - e.slot_bits));
+}
+__device__ __forceinline__ u64 slot_of(const EngineDev &e, u64 key) {
+    return slot_in_slice(e, (u64)slice_of(e, part_of(key)) << e.slot_bits, key);
+}
 
 __device__ __forceinline__ bool better(u64 k1, i64 c1, u64 k2, i64 c2) {
     // (k1, c1) beats (k2, c2): larger count, ties to the smaller packed key
@@ -221,49 +260,73 @@ __device__ __forceinline__ bool better(u64 k1, i64 c1, u64 k2, i64 c2) {
     return c1 > c2 || (c1 == c2 && k1 < k2);
 }
 
-__device__ __forceinline__ void mark_dirty(const EngineDev &e, u64 slot_index) {
-    unsigned int blk = (unsigned int)(slot_index / STBPE_BLK);
-    if (*(volatile unsigned int *)&e.dirty_flag[blk] == 0u) {
-        if (atomicExch(&e.dirty_flag[blk], 1u) == 0u) {
-            unsigned int i = atomicAdd(&e.st->n_dirty, 1u);
-            if (i < e.n_blocks) e.dirty_list[i] = blk;
-        }
-    }
+// The host and every kernel read mutable state through L2: loop_kernel keeps running while other
+// SMs write it, and the L1 caches are not coherent.
+__device__ __forceinline__ Slot ldcg_slot(const Slot *p) {
+    const uint4 raw = __ldcg(reinterpret_cast<const uint4 *>(p));
+    Slot s;
+    s.key = ((u64)raw.y << 32) | raw.x;
+    s.count = (i64)(((u64)raw.w << 32) | raw.z);
+    return s;
 }
 
-// add delta to key in the pair table, inserting the key when absent
-__device__ __forceinline__ void table_add(const EngineDev &e, u64 key, i64 delta) {
+__device__ __forceinline__ void mark_dirty(const EngineDev &e, u64 slot_index) {
+    const unsigned int blk = (unsigned int)(slot_index >> e.blk_shift);
+    atomicOr(&e.dirty_bits[blk >> 5], 1u << (blk & 31));  // result unused: a reduction
+}
+
+// threshold of the candidate list in selection order: a larger count, or the same count and a key below `key`
+struct Theta {
+    i64 count;
+    u64 key;
+    __device__ __forceinline__ bool admits(i64 c, u64 k) const { return c > count || (c == count && k < key); }
+};
+
+// Add delta to key in the pair table, inserting the key when absent.  `fresh` counts inserted keys
+// (the caller adds them to DevState::n_keys).  `made`: the key probably does not exist yet, so the first
+// access is the compare-and-swap that claims a slot instead of a load that would find it empty.
+// NOTE says what the arg-max has to learn of the add:
+//   NOTE_NONE   nothing (first counts: candidates / maxima are built afterwards)
+//   NOTE_CAND   the add that lifts a pair over the candidates' threshold appends its slot to the list.  Only
+//               adds look at the count they leave; a subtraction never lifts a pair.
+//   NOTE_DIRTY  the maximum of the slot's block can only change if this key is the recorded maximum or if its
+//               count now reaches it (the recorded maxima do not change while deltas are applied).  An add sees
+//               a count that is at least the key's final one when subtractions of the same key follow
+//               it, so the check after adds alone is enough.
+enum { NOTE_NONE, NOTE_CAND, NOTE_DIRTY };
+template <int NOTE>
+__device__ __forceinline__ void table_add(const EngineDev &e, u64 key, i64 delta, bool made, unsigned int &fresh,
+                                          const Theta &theta = Theta()) {
     u64 h = slot_of(e, key);
-    // the recorded maximum and the dirty flag of the block the key hashes to, fetched together with
-    // the first probe (a key that was pushed into the next block re-reads them below)
-    const u64 blk0 = h / STBPE_BLK;
-    uint4 raw = __ldcg(reinterpret_cast<const uint4 *>(e.blockmax + blk0));
-    unsigned int flagged = *(volatile unsigned int *)&e.dirty_flag[blk0];
+    const u64 blk = h >> e.blk_shift;
+    Slot mx;
+    if (NOTE == NOTE_DIRTY) mx = ldcg_slot(e.blockmax + blk);  // fetched together with the first probe
+#pragma unroll 1
     for (unsigned int probe = 0; probe < STBPE_MAX_PROBE; ++probe) {
         Slot *s = &e.table[h];
-        u64 k = *(volatile u64 *)&s->key;
+        u64 k = made ? STBPE_EMPTY : __ldcg(&s->key);
         if (k == STBPE_EMPTY) {
-            u64 old = atomicCAS(&s->key, STBPE_EMPTY, key);
-            if (old == STBPE_EMPTY) {
-                atomicAdd(&e.st->n_keys, 1ull);
+            k = atomicCAS(&s->key, STBPE_EMPTY, key);
+            if (k == STBPE_EMPTY) {
+                ++fresh;
                 k = key;
-            } else {
-                k = old;
             }
         }
         if (k == key) {
-            const i64 now = (i64)atomicAdd((u64 *)&s->count, (u64)delta) + delta;
-            // The maximum of the slot's block can only change if this key is the recorded maximum or
-            // if its count now reaches it (the add that brings a key to its final count sees that
-            // count, because the adds on one slot are serialised; the recorded maxima do not change
-            // while deltas are applied).  Only those blocks are recomputed by refresh_kernel.
-            if (h / STBPE_BLK != blk0) {
-                raw = __ldcg(reinterpret_cast<const uint4 *>(e.blockmax + (h / STBPE_BLK)));
-                flagged = 0u;
+            if (NOTE == NOTE_NONE || (NOTE == NOTE_CAND && delta < 0)) {
+                atomicAdd((u64 *)&s->count, (u64)delta);  // result unused: a reduction
+                return;
             }
-            const u64 mk = ((u64)raw.y << 32) | raw.x;
-            const i64 mc = (i64)(((u64)raw.w << 32) | raw.z);
-            if (!flagged && (key == mk || now > mc || (now == mc && key < mk))) mark_dirty(e, h);
+            const i64 was = (i64)atomicAdd((u64 *)&s->count, (u64)delta), now = was + delta;
+            if (NOTE == NOTE_CAND) {
+                if (theta.admits(now, key) && !theta.admits(was, key)) {
+                    const unsigned int i = atomicAdd(&e.st->n_cand, 1u);
+                    if (i < STBPE_CAND_CAP) e.cand[i] = (unsigned int)h;
+                }
+            } else {
+                if ((h >> e.blk_shift) != blk) mx = ldcg_slot(e.blockmax + (h >> e.blk_shift));
+                if (key == mx.key || (delta > 0 && (now > mx.count || (now == mx.count && key < mx.key)))) mark_dirty(e, h);
+            }
             return;
         }
         h = (h + 1) & e.mask;
@@ -274,6 +337,7 @@ __device__ __forceinline__ void table_add(const EngineDev &e, u64 key, i64 delta
 // rank-local delta table (multi-GPU): same probing, first touch recorded for the drain
 __device__ __forceinline__ void ltable_add(const EngineDev &e, u64 key, i64 delta) {
     u64 h = mix64(key * 0x9E3779B97F4A7C15ULL + 1) & e.lmask;
+#pragma unroll 1
     for (unsigned int probe = 0; probe <= (unsigned int)e.lmask; ++probe) {
         Slot *s = &e.ltable[h];
         u64 k = *(volatile u64 *)&s->key;
@@ -296,12 +360,16 @@ __device__ __forceinline__ void ltable_add(const EngineDev &e, u64 key, i64 delt
     atomicOr(&e.st->error, STBPE_DERR_LTABLE_FULL);
 }
 
+// first counts: into the rank-local delta table, or straight into the pair table
 template <bool MG>
 __device__ __forceinline__ void sink_add(const EngineDev &e, u64 key, i64 delta) {
-    if (MG)
+    if (MG) {
         ltable_add(e, key, delta);
-    else
-        table_add(e, key, delta);
+    } else {
+        unsigned int fresh = 0;
+        table_add<NOTE_NONE>(e, key, delta, false, fresh);
+        if (fresh) atomicAdd(&e.st->n_keys, (u64)fresh);
+    }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -341,15 +409,6 @@ __device__ __forceinline__ void smem_table_clear(const SmemTable &t) {
     }
 }
 
-__device__ __forceinline__ unsigned int hash32(u64 key) {
-    unsigned int a = (unsigned int)(key >> 32), b = (unsigned int)key;
-    unsigned int h = a * 0x9E3779B1u ^ (b * 0x85EBCA77u + 0x7F4A7C15u);
-    h ^= h >> 15;
-    h *= 0x2C1B3C6Du;
-    h ^= h >> 13;
-    return h;
-}
-
 // pair filter: the three rows of a pair key, and setting the pair's bits for a tile.  The filter is
 // kept only while it pays: a merge with more matches than tiles visits nearly every tile anyway, and
 // entering its new pairs costs more than the whole rewrite (measured: 37 of 61 ms on the first 20
@@ -369,17 +428,21 @@ __device__ __forceinline__ void filter_rows(u64 key, unsigned int &r1, unsigned 
     r2 = (h >> 14) & (STBPE_PROWS - 1);
     r3 = (g >> 9) & (STBPE_PROWS - 1);
 }
-__device__ __forceinline__ void filter_set(const EngineDev &e, int tile, u64 key) {
-    if (tile < 0) return;
+// enter a pair for the tiles of its two tokens (tile2 < 0: one tile)
+__device__ __forceinline__ void filter_set(const EngineDev &e, int tile, int tile2, u64 key) {
     unsigned int r1, r2, r3;
     filter_rows(key, r1, r2, r3);
-    const unsigned int w = (unsigned int)tile >> 5, bit = 1u << (tile & 31);
-    unsigned int *p1 = e.presence + (size_t)r1 * e.presence_words + w;
-    unsigned int *p2 = e.presence + (size_t)r2 * e.presence_words + w;
-    unsigned int *p3 = e.presence + (size_t)r3 * e.presence_words + w;
-    if (!(*(volatile unsigned int *)p1 & bit)) atomicOr(p1, bit);
-    if (!(*(volatile unsigned int *)p2 & bit)) atomicOr(p2, bit);
-    if (!(*(volatile unsigned int *)p3 & bit)) atomicOr(p3, bit);
+#pragma unroll 1
+    for (;;) {
+        unsigned int *g = e.presence + (size_t)((unsigned int)tile >> 5) * STBPE_PPITCH;
+        const unsigned int bit = 1u << (tile & 31);
+        // results unused: reductions, nothing waits for them
+        atomicOr(g + r1, bit);
+        atomicOr(g + r2, bit);
+        atomicOr(g + r3, bit);
+        if (tile2 < 0 || tile2 == tile) return;
+        tile = tile2;
+    }
 }
 
 // slow path: probe for the key, claim an empty slot, or give up after a few probes
@@ -435,7 +498,7 @@ __device__ __forceinline__ void smem_table_flush(const SmemTable &t, const Engin
 __device__ __forceinline__ TileRec load_rec(const TileRec *p) {
     TileRec r;
     const uint4 *q = reinterpret_cast<const uint4 *>(p);
-    uint4 x = q[0], y = q[1];
+    const uint4 x = __ldcg(q), y = __ldcg(q + 1);
     r.ver = (int)x.x;
     r.len = (int)x.y;
     r.head[0] = x.z;
@@ -459,46 +522,64 @@ __device__ __forceinline__ int current_rec(const EngineDev &e, int tile, int m, 
     return s;
 }
 
-// Live tokens around a tile, in stream order: the last two live tokens before it and up to
-// three live tokens after it (STBPE_NONE where the stream ends).  Walks records only.
-// `before` / `after`: the records of tiles tile - 1 and tile + 1 when the caller has loaded them
-// already (together with the tile's own, so that the three look-ups are one round trip).
-__device__ __forceinline__ void gather_halo(const EngineDev &e, int tile, int m, uint32_t &prev,
-                                            uint32_t &prev2, uint32_t nxt[3], int &next_tile, int &prev_tile,
-                                            const TileRec *before = nullptr, const TileRec *after = nullptr) {
-    next_tile = prev_tile = -1;
-    prev = prev2 = STBPE_NONE;
-    nxt[0] = nxt[1] = nxt[2] = STBPE_NONE;
+// Live tokens around a tile, in stream order: the last two live tokens before it and the next three
+// after it (STBPE_NONE where the stream ends), with the tiles that hold prev, nxt[0] and nxt[1].
+struct Halo {
+    uint32_t prev, prev2, nxt[3];
+    int prev_tile, next_tile, next2_tile;
+};
+
+// Walks records only; for tiles whose neighbours hold too few tokens to answer by themselves.
+static __device__ __noinline__ void gather_halo(const EngineDev &e, int tile, int m, Halo &h) {
+    h.prev_tile = h.next_tile = h.next2_tile = -1;
+    h.prev = h.prev2 = STBPE_NONE;
+    h.nxt[0] = h.nxt[1] = h.nxt[2] = STBPE_NONE;
     TileRec r;
     int back = 0;
     for (int t = tile - 1; t >= 0 && back < 2; --t) {
-        if (before && t == tile - 1)
-            r = *before;
-        else
-            current_rec(e, t, m, r);
+        current_rec(e, t, m, r);
         if (r.len > 0) {
             if (back == 0) {
-                prev = r.tail;
-                prev_tile = t;
+                h.prev = r.tail;
+                h.prev_tile = t;
                 back = 1;
                 if (r.len > 1) {
-                    prev2 = r.tail2;
+                    h.prev2 = r.tail2;
                     back = 2;
                 }
             } else {
-                prev2 = r.tail;
+                h.prev2 = r.tail;
                 back = 2;
             }
         }
     }
     int have = 0;
     for (int t = tile + 1; t < e.n_tiles && have < 3; ++t) {
-        if (after && t == tile + 1)
-            r = *after;
-        else
-            current_rec(e, t, m, r);
-        int take = r.len < 3 ? r.len : 3;
-        if (take > 0 && next_tile < 0) next_tile = t;
-        for (int i = 0; i < take && have < 3; ++i) nxt[have++] = r.head[i];
+        current_rec(e, t, m, r);
+        const int take = r.len < 3 ? r.len : 3;
+        for (int i = 0; i < take && have < 3; ++i) {
+            if (have == 0) h.next_tile = t;
+            if (have == 1) h.next2_tile = t;
+            h.nxt[have++] = r.head[i];
+        }
     }
+}
+
+// first live token after a tile, from the records (general count, filter build)
+__device__ __forceinline__ uint32_t first_after(const EngineDev &e, int tile, int m) {
+    for (int t = tile + 1; t < e.n_tiles; ++t) {
+        TileRec r;
+        current_rec(e, t, m, r);
+        if (r.len > 0) return r.head[0];
+    }
+    return STBPE_NONE;
+}
+// last live token before a tile
+__device__ __forceinline__ uint32_t last_before(const EngineDev &e, int tile, int m) {
+    for (int t = tile - 1; t >= 0; --t) {
+        TileRec r;
+        current_rec(e, t, m, r);
+        if (r.len > 0) return r.tail;
+    }
+    return STBPE_NONE;
 }

@@ -13,6 +13,7 @@
 
 #include "../../include/stbpe.h"
 #include "kernels.cuh"
+#include "loop.cuh"
 
 #define STBPE_VISIBLE __attribute__((visibility("default")))
 
@@ -21,14 +22,17 @@ struct stbpe_engine {
     EngineDev d;
     i64 max_tokens, n_tokens;
     int max_tiles;
+    bool wide;            // the stream holds 32-bit tokens (an id does not fit 15 bits)
+    size_t tiles_bytes, alt_bytes;  // sizes of the two stream buffers
     u64 slots;
     Slot *partial;
     i64 *cand;
     u64 lslots;
     int sm_count;
-    int merge_grid, count_grid, select_grid, refresh_grid;
-    unsigned int merge_slots, count_slots;
-    size_t merge_smem, count_smem;
+    int select_grid, refresh_grid;
+    size_t count_smem;
+    int2 *forced;         // device copy of host-given merges
+    int forced_cap;
     bool recs_stale, counted;
     bool filter_valid;    // host mirror of DevState::filter_valid
     double filter_density;  // the filter is kept while (matches of the last merge) <= filter_density x tiles
@@ -51,20 +55,18 @@ struct stbpe_engine {
     float count_ms;       // device time of the histogram kernels of the last count
     float convert_ms;     // device time of moving a dense histogram into the pair table (wide path)
     cudaEvent_t ev0, ev1;
-    uint32_t *tiles_alt;  // second stream buffer of the re-pack (at creation when memory allows)
+    void *tiles_alt;  // second stream buffer of the re-pack (at creation when memory allows)
     i64 *rp_lens, *rp_offs;  // re-pack scratch: tile lengths and their exclusive sums
     void *rp_tmp;
     size_t rp_tmp_bytes;
     int repacks;
     int repacks_since_load;
-    cudaGraphExec_t graph;
-    int graph_merges;
-    uint32_t *graph_tiles;
-    cudaStream_t graph_stream;
+    cudaGraphExec_t graph;  // a batch of peer-memory rounds (several ranks)
+    int graph_tiles_n;
+    void *graph_tiles;
+    bool graph_wide;
     bool use_graph;
     int part_group;       // partitions per launch of the second pass of the partitioned count
-    bool use_pdl;         // the captured single-GPU loop launches its kernels as programmatic dependents
-    bool pdl_now;         // set while that loop is being captured
     std::string err;
     std::vector<void *> allocs;
 };
@@ -104,6 +106,17 @@ static cudaError_t dev_alloc(stbpe_engine *e, T **p, size_t count) {
     return c;
 }
 
+static void dev_free(stbpe_engine *e, void *p) {
+    if (!p) return;
+    for (auto &q : e->allocs)
+        if (q == p) {
+            cudaFree(p);
+            q = e->allocs.back();
+            e->allocs.pop_back();
+            return;
+        }
+}
+
 static u64 next_pow2(u64 x) {
     u64 p = 1;
     while (p < x) p <<= 1;
@@ -119,27 +132,25 @@ static bool is_device_pointer(const void *p) {
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
-// Launch of a loop kernel; with `dependent` and pdl_now set (capture of the single-GPU loop) as a
-// programmatic dependent of the kernel before it in the stream: its CTAs may be scheduled once all
-// CTAs of that kernel have started, and wait in dep_wait() for it to complete.  Measured on merges
-// 8000-10000 of the 1 GiB corpus (61-63 us per merge with plain launches): the worklist and merge
-// kernels as dependents save 3.5 us per merge (the merge kernel's shared-memory set-up and CTA
-// launch run under the kernels before it); refresh and select as dependents gain nothing, and all
-// four together cost 9 us, so only those two are launched this way.
-template <typename... Params, typename... Args>
-static cudaError_t launch_loop_kernel(const stbpe_engine *e, bool dependent, void (*kernel)(Params...), unsigned int grid,
-                                      unsigned int block, size_t smem, cudaStream_t s, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = (e->pdl_now && dependent) ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+// Calls f(uint16_t{}) or f(uint32_t{}) for the engine's stream.
+template <typename F>
+static auto with_tok(const stbpe_engine *e, F &&f) {
+    return e->wide ? f(uint32_t{}) : f(uint16_t{});
+}
+// Whether a fresh stream starts with 32-bit tokens.  Several ranks run rounds without a look from the host, so
+// there the ids of all merges must fit from the start; a single rank widens its stream when it gets there.
+static bool starts_wide(const stbpe_config &c) {
+    const i64 last = (i64)c.base_vocab + (c.world_size > 1 ? c.max_merges : 0);
+    return last >= (i64)Tok<uint16_t>::IDMASK;
+}
+static size_t tok_bytes(const stbpe_engine *e) { return e->wide ? 4 : 2; }
+
+// log2 of the tiles a CTA takes together from the pair filter: words of the filter once every CTA gets two of
+// them, fewer tiles on smaller streams, so that the visited tiles spread over all CTAs
+static int unit_shift(const stbpe_engine *e, int grid) {
+    int sh = 5;
+    while (sh > 0 && (((i64)e->d.n_tiles + (1 << sh) - 1) >> sh) < 2 * (i64)grid) --sh;
+    return sh;
 }
 
 extern "C" {
@@ -195,42 +206,15 @@ STBPE_VISIBLE int stbpe_create(stbpe_engine **out, const stbpe_config *cfg) {
         return fail(nullptr, STBPE_E_BADARG, "invalid configuration");
     if ((i64)cfg->base_vocab + (i64)cfg->max_merges >= 0x7FFFFFFFll)
         return fail(nullptr, STBPE_E_ID_OVERFLOW, "Token id overflow: ids must stay below 2^31-1");
-    stbpe_engine *e = new stbpe_engine();
+    stbpe_engine *e = new stbpe_engine();  // all members zero
     e->cfg = *cfg;
-    e->graph = nullptr;
-    e->graph_merges = 0;
-    e->tiles_alt = nullptr;
-    e->rp_lens = e->rp_offs = nullptr;
-    e->rp_tmp = nullptr;
-    e->rp_tmp_bytes = 0;
-    e->repacks = 0;
-    e->repacks_since_load = 0;
-    e->count_ms = 0.f;
-    e->convert_ms = 0.f;
-    e->ev0 = e->ev1 = nullptr;
-    e->comm = nullptr;
-    e->all_cands = nullptr;
-    e->own_boxes = false;
-    memset(&e->parts, 0, sizeof(e->parts));
-    e->wide_block = nullptr;
-    e->wide_dense = nullptr;
-    memset(e->wide_mapped, 0, sizeof(e->wide_mapped));
-    memset(&e->wide_peers, 0, sizeof(e->wide_peers));
-    e->wide_open = e->wide_counted = e->full_refresh_pending = false;
     e->dense32_min = 1ll << 24;
     if (const char *v = getenv("STBPE_DENSE32_MIN_TOKENS")) e->dense32_min = atoll(v);
-    e->mail_own = nullptr;
-    memset(e->mail_mapped, 0, sizeof(e->mail_mapped));
-    e->peers_open = false;
     e->use_graph = getenv("STBPE_NO_GRAPH") == nullptr;
     e->part_group = STBPE_PARTS;
     if (const char *v = getenv("STBPE_PART_GROUP")) e->part_group = atoi(v) > 0 ? atoi(v) : STBPE_PARTS;
-    e->use_pdl = getenv("STBPE_NO_PDL") == nullptr;
-    e->pdl_now = false;
-    e->filter_valid = false;
     e->filter_density = 1.0;
     if (const char *v = getenv("STBPE_FILTER_DENSITY")) e->filter_density = atof(v);
-    memset(&e->d, 0, sizeof(e->d));
     auto bail = [&](int code) {
         g_create_err = e->err;
         stbpe_destroy(e);
@@ -262,34 +246,43 @@ STBPE_VISIBLE int stbpe_create(stbpe_engine **out, const stbpe_config *cfg) {
     u64 slices = next_pow2(((u64)STBPE_PARTS + cfg->world_size - 1) / cfg->world_size);
     e->d.slot_bits = 0;
     while ((slices << e->d.slot_bits) < slots) ++e->d.slot_bits;
-    e->d.n_blocks = (unsigned int)(slots / STBPE_BLK);
+    // blocks of the arg-max over several ranks: at most 2^19
+    e->d.blk_shift = 6;
+    while ((slots >> e->d.blk_shift) > (1u << 19)) ++e->d.blk_shift;
+    e->d.n_blocks = (unsigned int)(slots >> e->d.blk_shift);
     e->d.world = cfg->world_size;
     e->d.rank = cfg->rank;
 
 #define ALLOC(ptr, n)                                                  \
     if ((c = dev_alloc(e, &(ptr), (size_t)(n))) != cudaSuccess) return bail(cuda_fail(e, c, "cudaMalloc " #ptr))
-    ALLOC(e->d.tiles, (size_t)e->max_tiles * STBPE_TILE);
+    e->wide = starts_wide(*cfg);
+    {
+        unsigned char *t = nullptr;
+        e->tiles_bytes = (size_t)e->max_tiles * STBPE_TILE * tok_bytes(e);
+        ALLOC(t, e->tiles_bytes);
+        e->d.tiles = t;
+    }
     ALLOC(e->d.recs, (size_t)e->max_tiles * 2);
+    ALLOC(e->d.tile_live, (size_t)e->max_tiles);
     ALLOC(e->d.table, slots);
-    ALLOC(e->d.blockmax, e->d.n_blocks);
-    ALLOC(e->d.dirty_flag, e->d.n_blocks);
-    ALLOC(e->d.dirty_list, e->d.n_blocks);
-    e->d.n_super2 = (e->d.n_blocks + 255) / 256;
-    ALLOC(e->d.supermax, e->d.n_super2);
-    ALLOC(e->d.dirty2_flag, e->d.n_super2);
-    ALLOC(e->d.dirty2_list, e->d.n_super2);
+    if (cfg->world_size > 1) {
+        ALLOC(e->d.blockmax, e->d.n_blocks);
+        ALLOC(e->d.dirty_bits, (e->d.n_blocks + 31) / 32);
+        ALLOC(e->partial, 4096);
+    } else {
+        ALLOC(e->d.cand, STBPE_CAND_CAP);
+        ALLOC(e->d.cand_hist, STBPE_CAND_BUCKETS);
+    }
     ALLOC(e->d.st, 1);
+    ALLOC(e->d.sync, 1);
     ALLOC(e->d.merges, (size_t)2 * (cfg->max_merges + 1));
     ALLOC(e->d.merge_counts, (size_t)cfg->max_merges + 1);
     ALLOC(e->d.live_before, (size_t)cfg->max_merges + 1);
-    ALLOC(e->partial, 4096);
     ALLOC(e->dense, 65536);
     ALLOC(e->cand, 4);
     ALLOC(e->all_cands, (size_t)4 * cfg->world_size);
-    e->d.presence_words = (unsigned int)(((size_t)e->max_tiles + 31) / 32);
-    ALLOC(e->d.presence, (size_t)(STBPE_PROWS + 1) * e->d.presence_words);
-    ALLOC(e->d.cand_bits, e->d.presence_words + 1);
-    ALLOC(e->d.worklist, (size_t)e->max_tiles + 32);
+    e->d.presence_groups = (unsigned int)(((size_t)e->max_tiles + 31) / 32);
+    ALLOC(e->d.presence, (size_t)STBPE_PPITCH * e->d.presence_groups);
     // the re-pack allocates nothing inside the merge loop: its scratch is sized here for the largest
     // stream, and the second stream buffer too unless it would take more than half of what is free
     ALLOC(e->rp_lens, (size_t)e->max_tiles + 1);
@@ -302,9 +295,12 @@ STBPE_VISIBLE int stbpe_create(stbpe_engine **out, const stbpe_config *cfg) {
     }
     {
         size_t free_b = 0, total_b = 0;
-        const size_t want = (size_t)e->max_tiles * STBPE_TILE * sizeof(uint32_t);
-        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && want <= free_b / 2)
-            ALLOC(e->tiles_alt, (size_t)e->max_tiles * STBPE_TILE);
+        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && e->tiles_bytes <= free_b / 2) {
+            unsigned char *t = nullptr;
+            ALLOC(t, e->tiles_bytes);
+            e->tiles_alt = t;
+            e->alt_bytes = e->tiles_bytes;
+        }
     }
     if (cfg->world_size > 1) {
         e->lslots = 1ull << 22;
@@ -323,31 +319,32 @@ STBPE_VISIBLE int stbpe_create(stbpe_engine **out, const stbpe_config *cfg) {
         }
     }
 #undef ALLOC
-    c = cudaMemset(e->d.dirty_flag, 0, e->d.n_blocks * sizeof(unsigned int));
-    if (c != cudaSuccess) return bail(cuda_fail(e, c, "cudaMemset"));
-    c = cudaMemset(e->d.dirty2_flag, 0, e->d.n_super2 * sizeof(unsigned int));
+    c = e->d.dirty_bits ? cudaMemset(e->d.dirty_bits, 0, (e->d.n_blocks + 31) / 32 * sizeof(unsigned int))
+                        : cudaMemset(e->d.cand_hist, 0, STBPE_CAND_BUCKETS * sizeof(unsigned int));
     if (c != cudaSuccess) return bail(cuda_fail(e, c, "cudaMemset"));
 
-    // launch geometry: persistent CTAs, a whole number per SM
-    e->merge_slots = 1024;
-    e->count_slots = 8192;
-    e->merge_smem = TilePipe::bytes(e->merge_slots);
-    e->count_smem = TilePipe::bytes(e->count_slots);
-    int occ = 0;
-#define SETUP(kern, smem, grid)                                                                         \
-    c = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem));           \
-    if (c != cudaSuccess) return bail(cuda_fail(e, c, "cudaFuncSetAttribute"));                         \
-    c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, STBPE_CTA_THREADS, smem);                      \
-    if (c != cudaSuccess) return bail(cuda_fail(e, c, "cudaOccupancyMaxActiveBlocksPerMultiprocessor")); \
-    grid = e->sm_count * (occ > 0 ? occ : 1)
-    int g1 = 0, g2 = 0;
-    SETUP(merge_kernel<false>, e->merge_smem, e->merge_grid);
-    SETUP(merge_kernel<true>, e->merge_smem, g1);
-    SETUP(count_kernel<false>, e->count_smem, e->count_grid);
-    SETUP(count_kernel<true>, e->count_smem, g2);
-    if (g1 < e->merge_grid) e->merge_grid = g1;
-    if (g2 < e->count_grid) e->count_grid = g2;
-#undef SETUP
+    // kernels that use more shared memory than the default limit
+    e->count_smem = (size_t)STBPE_COUNT_SLOTS * 12;
+#define SMEM(kern, bytes)                                                                                      \
+    if ((c = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes))) != cudaSuccess) \
+    return bail(cuda_fail(e, c, "cudaFuncSetAttribute"))
+    SMEM((merge_kernel<uint16_t, false>), MergeGeom<uint16_t>::BYTES);
+    SMEM((merge_kernel<uint16_t, true>), MergeGeom<uint16_t>::BYTES);
+    SMEM((merge_kernel<uint32_t, false>), MergeGeom<uint32_t>::BYTES);
+    SMEM((merge_kernel<uint32_t, true>), MergeGeom<uint32_t>::BYTES);
+    SMEM(loop_kernel<uint16_t>, prop.sharedMemPerBlockOptin - 4096);
+    SMEM(loop_kernel<uint32_t>, prop.sharedMemPerBlockOptin - 4096);
+    SMEM((count_kernel<uint16_t, false>), e->count_smem);
+    SMEM((count_kernel<uint16_t, true>), e->count_smem);
+    SMEM((count_kernel<uint32_t, false>), e->count_smem);
+    SMEM((count_kernel<uint32_t, true>), e->count_smem);
+    SMEM(count_dense_kernel<uint16_t>, 32768 * 4);
+    SMEM(count_dense_kernel<uint32_t>, 32768 * 4);
+    SMEM(partition_pairs_kernel<uint16_t>, STBPE_PART_SMEM_BYTES);
+    SMEM(partition_pairs_kernel<uint32_t>, STBPE_PART_SMEM_BYTES);
+    SMEM(presence_rebuild_kernel<uint16_t>, STBPE_PROWS * sizeof(unsigned int));
+    SMEM(presence_rebuild_kernel<uint32_t>, STBPE_PROWS * sizeof(unsigned int));
+#undef SMEM
     e->select_grid = e->sm_count;
     e->refresh_grid = e->sm_count * 4;
     int rc = reset_state(e, 0);
@@ -361,6 +358,8 @@ STBPE_VISIBLE int stbpe_reset(stbpe_engine *e) {
     CK(cudaSetDevice(e->cfg.device));
     return reset_state(e, 0);
 }
+
+static int widen_stream(stbpe_engine *e, cudaStream_t s);
 
 static int append_common(stbpe_engine *e, const void *data, i64 n, size_t elem, const i64 *row_offsets,
                          i64 n_rows, cudaStream_t s) {
@@ -378,28 +377,32 @@ static int append_common(stbpe_engine *e, const void *data, i64 n, size_t elem, 
         if (h.merges_done > 0 || e->repacks_since_load > 0)
             return fail(e, STBPE_E_STATE, "rows cannot be appended after a merge has been applied; call stbpe_reset first");
     }
-    uint32_t *dst = e->d.tiles + e->n_tokens;
+    if (e->n_tokens == 0) e->wide = starts_wide(e->cfg);  // a fresh stream
+    const i64 at0 = e->n_tokens;
     unsigned int *bad = &e->d.st->error;
-    auto pack = [&](const void *src, i64 cnt, uint32_t *out) {
-        if (elem == 1) {
-            i64 blocks = (cnt / 16 + 255) / 256 + 1;
-            if (blocks > 65535 * 16) blocks = 65535 * 16;
-            pack_bytes_kernel<<<(unsigned int)blocks, 256, 0, s>>>((const uint8_t *)src, cnt, out);
-        } else {
-            i64 blocks = (cnt + 255) / 256;
-            if (blocks > 65535 * 16) blocks = 65535 * 16;
-            pack_ids_kernel<<<(unsigned int)blocks, 256, 0, s>>>((const int32_t *)src, cnt, out, bad);
-        }
+    auto pack = [&](const void *src, i64 cnt, i64 at) {
+        with_tok(e, [&](auto t) {
+            typedef decltype(t) T;
+            if (elem == 1) {
+                i64 blocks = (cnt / 32 + 2 + 255) / 256;
+                if (blocks > (i64)e->sm_count * 32) blocks = (i64)e->sm_count * 32;
+                pack_bytes_kernel<T><<<(unsigned int)blocks, 256, 0, s>>>((const uint8_t *)src, cnt, e->d.tiles, at);
+            } else {
+                i64 blocks = (cnt + 255) / 256;
+                if (blocks > (i64)e->sm_count * 32) blocks = (i64)e->sm_count * 32;
+                pack_ids_kernel<T><<<(unsigned int)blocks, 256, 0, s>>>((const int32_t *)src, cnt, e->d.tiles, at, bad);
+            }
+        });
     };
     void *staged = nullptr;
     if (is_device_pointer(data)) {
-        pack(data, n, dst);
+        pack(data, n, at0);
     } else {
         // host data is staged on the device before the pack kernel reads it: in the second stream
         // buffer when the engine has one (it is idle until the first re-pack, and an allocation of this
         // size costs as much as the copy), else in stream-ordered scratch
         char *stage = (char *)e->tiles_alt;
-        if (!stage || (size_t)n * elem > (size_t)e->max_tiles * STBPE_TILE * sizeof(uint32_t)) {
+        if (!stage || (size_t)n * elem > e->alt_bytes) {
             CK(cudaMallocAsync(&staged, (size_t)n * elem, s));
             stage = (char *)staged;
         }
@@ -408,7 +411,7 @@ static int append_common(stbpe_engine *e, const void *data, i64 n, size_t elem, 
         const i64 piece = (i64)((size_t)(64 << 20) / elem);
         if (n <= piece) {
             CK(cudaMemcpyAsync(stage, data, (size_t)n * elem, cudaMemcpyHostToDevice, s));
-            pack(stage, n, dst);
+            pack(stage, n, at0);
         } else {
             cudaStream_t cs = nullptr;
             cudaEvent_t ready = nullptr, landed = nullptr;
@@ -423,7 +426,7 @@ static int append_common(stbpe_engine *e, const void *data, i64 n, size_t elem, 
                                      (size_t)cnt * elem, cudaMemcpyHostToDevice, cs);
                 if (ce == cudaSuccess) ce = cudaEventRecord(landed, cs);
                 if (ce == cudaSuccess) ce = cudaStreamWaitEvent(s, landed, 0);  // waits for the record just made
-                if (ce == cudaSuccess) pack(stage + (size_t)at * elem, cnt, dst + at);
+                if (ce == cudaSuccess) pack(stage + (size_t)at * elem, cnt, at0 + at);
             }
             if (ce == cudaSuccess) ce = cudaStreamSynchronize(cs);
             if (ready) cudaEventDestroy(ready);
@@ -446,10 +449,33 @@ static int append_common(stbpe_engine *e, const void *data, i64 n, size_t elem, 
             return fail(e, STBPE_E_BADARG, "row_offsets must start at 0 and end at n");
         }
     }
+    if (elem == 4 && !e->wide) {
+        // an id that 15 bits cannot hold: what the stream holds so far is widened, and this piece is packed
+        // again (it is still on the device, in the caller's buffer or in the staging buffer)
+        unsigned int err = 0;
+        CK(cudaMemcpyAsync(&err, bad, sizeof(err), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        if (err & STBPE_DERR_NARROW) {
+            err &= ~STBPE_DERR_NARROW;
+            CK(cudaMemcpyAsync(bad, &err, sizeof(err), cudaMemcpyHostToDevice, s));
+            const void *src = is_device_pointer(data) ? data : staged;
+            if (!src) {  // staged in the second stream buffer, which the widening takes over
+                CK(cudaMallocAsync(&staged, (size_t)n * elem, s));
+                CK(cudaMemcpyAsync(staged, data, (size_t)n * elem, cudaMemcpyHostToDevice, s));
+                src = staged;
+            }
+            int rc = widen_stream(e, s);
+            if (rc != STBPE_OK) return rc;
+            pack(src, n, at0);
+            CK(cudaGetLastError());
+        }
+    }
     i64 *doff = nullptr;
     CK(cudaMallocAsync((void **)&doff, (size_t)(rows + 1) * sizeof(i64), s));
     CK(cudaMemcpyAsync(doff, off, (size_t)(rows + 1) * sizeof(i64), cudaMemcpyHostToDevice, s));
-    mark_row_starts_kernel<<<(unsigned int)((rows + 255) / 256), 256, 0, s>>>(doff, rows, dst);
+    with_tok(e, [&](auto t) {
+        mark_row_starts_kernel<decltype(t)><<<(unsigned int)((rows + 255) / 256), 256, 0, s>>>(doff, rows, e->d.tiles, at0);
+    });
     CK(cudaGetLastError());
     CK(cudaFreeAsync(doff, s));
     if (staged) CK(cudaFreeAsync(staged, s));
@@ -474,10 +500,7 @@ STBPE_VISIBLE int stbpe_append_ids(stbpe_engine *e, const int32_t *ids, int64_t 
     return append_common(e, ids, n, 4, (const i64 *)row_offsets, n_rows, (cudaStream_t)stream);
 }
 
-static int check_device_error(stbpe_engine *e, cudaStream_t s) {
-    unsigned int err = 0;
-    CK(cudaMemcpyAsync(&err, &e->d.st->error, sizeof(err), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+static int check_error_bits(stbpe_engine *e, unsigned int err) {
     if (err & STBPE_DERR_BAD_ID)
         return fail(e, STBPE_E_ID_OVERFLOW, "Token id overflow: ids must be in [0, 2^31-2]");
     if (err & STBPE_DERR_TABLE_FULL)
@@ -489,13 +512,22 @@ static int check_device_error(stbpe_engine *e, cudaStream_t s) {
     return STBPE_OK;
 }
 
+static int check_device_error(stbpe_engine *e, cudaStream_t s) {
+    unsigned int err = 0;
+    CK(cudaMemcpyAsync(&err, &e->d.st->error, sizeof(err), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    return check_error_bits(e, err);
+}
+
 static int prepare_stream_state(stbpe_engine *e, cudaStream_t s) {
     if (e->recs_stale) {
         int rc = check_device_error(e, s);  // id range flag from the pack kernels
         if (rc != STBPE_OK) return rc;
         e->d.n_tiles = (int)((e->n_tokens + STBPE_TILE - 1) / STBPE_TILE);
         if (e->d.n_tiles > 0) {
-            init_recs_kernel<<<(e->d.n_tiles + 255) / 256, 256, 0, s>>>(e->d, e->n_tokens);
+            with_tok(e, [&](auto t) {
+                init_recs_kernel<decltype(t)><<<(e->d.n_tiles + 255) / 256, 256, 0, s>>>(e->d, e->n_tokens);
+            });
             CK(cudaGetLastError());
         }
         DevState h;
@@ -522,9 +554,9 @@ static int rebuild_presence(stbpe_engine *e, cudaStream_t s) {
     CK(cudaGetLastError());
     e->filter_valid = true;
     if (e->d.n_tiles > 0) {
-        CK(cudaFuncSetAttribute(presence_rebuild_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                STBPE_PROWS * (int)sizeof(unsigned int)));
-        presence_rebuild_kernel<<<e->sm_count * 2, 1024, STBPE_PROWS * sizeof(unsigned int), s>>>(e->d);
+        with_tok(e, [&](auto t) {
+            presence_rebuild_kernel<decltype(t)><<<e->sm_count * 2, 1024, STBPE_PROWS * sizeof(unsigned int), s>>>(e->d);
+        });
         CK(cudaGetLastError());
     }
     return STBPE_OK;
@@ -563,12 +595,13 @@ static int count_prologue(stbpe_engine *e, cudaStream_t s) {
     if (rc != STBPE_OK) return rc;
     clear_table_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d);
     CK(cudaGetLastError());
-    CK(cudaMemsetAsync(e->d.dirty_flag, 0, e->d.n_blocks * sizeof(unsigned int), s));
-    CK(cudaMemsetAsync(e->d.dirty2_flag, 0, e->d.n_super2 * sizeof(unsigned int), s));
-    CK(cudaMemsetAsync(e->d.blockmax, 0, (size_t)e->d.n_blocks * sizeof(Slot), s));  // count 0 = no candidate
-    CK(cudaMemsetAsync(e->d.supermax, 0, (size_t)e->d.n_super2 * sizeof(Slot), s));
-    CK(cudaMemsetAsync(&e->d.st->n_dirty, 0, sizeof(unsigned int), s));
-    CK(cudaMemsetAsync(&e->d.st->n_dirty2, 0, sizeof(unsigned int), s));
+    if (e->cfg.world_size > 1) {
+        CK(cudaMemsetAsync(e->d.dirty_bits, 0, (e->d.n_blocks + 31) / 32 * sizeof(unsigned int), s));
+        CK(cudaMemsetAsync(e->d.blockmax, 0, (size_t)e->d.n_blocks * sizeof(Slot), s));  // count 0 = no candidate
+    } else {
+        cand_none_kernel<<<1, 1, 0, s>>>(e->d);
+        CK(cudaGetLastError());
+    }
     CK(cudaMemsetAsync(&e->d.st->n_keys, 0, sizeof(u64), s));
     if (!e->ev0) {
         CK(cudaEventCreate(&e->ev0));
@@ -588,8 +621,9 @@ static int wide_pass1(stbpe_engine *e, int *ok, cudaStream_t s) {
     *ok = 0;
     CK(cudaMemsetAsync(e->wide_dense, 0, 65536 * sizeof(u64), s));
     CK(cudaEventRecord(e->ev0, s));
-    CK(cudaFuncSetAttribute(partition_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STBPE_PART_SMEM_BYTES));
-    partition_pairs_kernel<<<pb.n_cta, STBPE_PART_THREADS, STBPE_PART_SMEM_BYTES, s>>>(e->d, e->n_tokens, e->wide_dense, pb);
+    with_tok(e, [&](auto t) {
+        partition_pairs_kernel<decltype(t)><<<pb.n_cta, STBPE_PART_THREADS, STBPE_PART_SMEM_BYTES, s>>>(e->d, e->wide_dense, pb);
+    });
     CK(cudaGetLastError());
     CK(cudaEventRecord(e->ev1, s));
     unsigned int derr = 0;
@@ -618,8 +652,9 @@ static int launch_count(stbpe_engine *e, bool mg, cudaStream_t s) {
         // byte-level fast path: dense stream, ids < 256
         CK(cudaMemsetAsync(e->dense, 0, 65536 * sizeof(u64), s));
         CK(cudaEventRecord(e->ev0, s));
-        CK(cudaFuncSetAttribute(count_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 32768 * 4));
-        count_dense_kernel<<<e->sm_count, STBPE_DENSE_THREADS, 32768 * 4, s>>>(e->d, e->n_tokens, e->dense);
+        with_tok(e, [&](auto t) {
+            count_dense_kernel<decltype(t)><<<e->sm_count, STBPE_DENSE_THREADS, 32768 * 4, s>>>(e->d, e->dense);
+        });
         CK(cudaGetLastError());
         unsigned int derr = 0;
         CK(cudaMemcpyAsync(&derr, &e->d.st->error, sizeof(derr), cudaMemcpyDeviceToHost, s));
@@ -672,12 +707,16 @@ static int launch_count(stbpe_engine *e, bool mg, cudaStream_t s) {
         // an id of 65 536 or more, or a region outgrew its buffer: the general kernel counts
     }
     if (e->d.n_tiles > 0) {
-        int grid = e->count_grid < e->d.n_tiles ? e->count_grid : e->d.n_tiles;
+        const int warps = STBPE_COUNT_THREADS / 32, need = (e->d.n_tiles + warps - 1) / warps;
+        const int grid = need < 2 * e->sm_count ? need : 2 * e->sm_count;
         CK(cudaEventRecord(e->ev0, s));
-        if (mg)
-            count_kernel<true><<<grid, STBPE_CTA_THREADS, e->count_smem, s>>>(e->d, e->count_slots);
-        else
-            count_kernel<false><<<grid, STBPE_CTA_THREADS, e->count_smem, s>>>(e->d, e->count_slots);
+        with_tok(e, [&](auto t) {
+            typedef decltype(t) T;
+            if (mg)
+                count_kernel<T, true><<<grid, STBPE_COUNT_THREADS, e->count_smem, s>>>(e->d);
+            else
+                count_kernel<T, false><<<grid, STBPE_COUNT_THREADS, e->count_smem, s>>>(e->d);
+        });
         CK(cudaGetLastError());
         CK(cudaEventRecord(e->ev1, s));
         CK(cudaEventSynchronize(e->ev1));
@@ -687,12 +726,8 @@ static int launch_count(stbpe_engine *e, bool mg, cudaStream_t s) {
 }
 
 static int launch_refresh(stbpe_engine *e, int all, cudaStream_t s) {
-    CK(launch_loop_kernel(e, false, refresh_kernel, e->refresh_grid, 256, 0, s, e->d, all));
-    if (all) {  // rebuild the second level as well (a peek changes nothing else)
-        CK(cudaMemsetAsync(e->d.dirty2_flag, 0, e->d.n_super2 * sizeof(unsigned int), s));
-        select_kernel<<<e->select_grid, STBPE_SELECT_THREADS, 0, s>>>(e->d, 0, 1, e->cand);
-        CK(cudaGetLastError());
-    }
+    refresh_kernel<<<e->refresh_grid, 256, 0, s>>>(e->d, all);
+    CK(cudaGetLastError());
     return STBPE_OK;
 }
 
@@ -703,10 +738,42 @@ STBPE_VISIBLE int stbpe_count_initial(stbpe_engine *e, void *stream) {
     if (e->cfg.world_size > 1) return fail(e, STBPE_E_STATE, "use stbpe_mg_count_local on a multi-rank engine");
     int rc = launch_count(e, false, s);
     if (rc != STBPE_OK) return rc;
-    rc = launch_refresh(e, 1, s);
-    if (rc != STBPE_OK) return rc;
     e->counted = true;
     return check_device_error(e, s);
+}
+
+// Candidate list of the pair table as it stands: threshold search (one pass over the table in the usual case,
+// further ones while a bucket holds too many pairs), then the list.
+static int refill_candidates(stbpe_engine *e, cudaStream_t s) {
+    const u64 key_hi = e->wide ? 0x7FFFFFFFFFFFFFFFull : ((u64)Tok<uint16_t>::IDMASK << 32) | Tok<uint16_t>::IDMASK;
+    const i64 want = ((i64)e->slots + 511) / 512;
+    const unsigned int grid = (unsigned int)(want < e->sm_count * 4 ? want : e->sm_count * 4);
+    CK(cudaMemsetAsync(&e->d.st->cand_state, 0, sizeof(int), s));
+    for (int pass = 0; pass < 16; ++pass) {
+        cand_hist_kernel<<<grid, 512, 0, s>>>(e->d);
+        cand_decide_kernel<<<1, 1024, 0, s>>>(e->d, key_hi);
+        cand_collect_kernel<<<grid, 512, 0, s>>>(e->d);
+        CK(cudaGetLastError());
+        DevState h;
+        CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        if (h.cand_state == STBPE_CAND_READY) return STBPE_OK;
+    }
+    return fail(e, STBPE_E_STATE, "no candidate threshold found");
+}
+
+// Best pair of the table into the device state, or as the loop's next step; *h = the state afterwards.
+static int choose(stbpe_engine *e, bool advance, DevState *h, cudaStream_t s) {
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        choose_kernel<<<1, 1024, 0, s>>>(e->d, advance ? 1 : 0);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(h, e->d.st, sizeof(*h), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        if (h->peek_valid || (advance && h->stopped)) return STBPE_OK;
+        int rc = refill_candidates(e, s);
+        if (rc != STBPE_OK) return rc;
+    }
+    return fail(e, STBPE_E_STATE, "no candidate found");
 }
 
 STBPE_VISIBLE int stbpe_select_best(stbpe_engine *e, uint64_t *key, int64_t *count, int64_t *n_ties,
@@ -715,14 +782,19 @@ STBPE_VISIBLE int stbpe_select_best(stbpe_engine *e, uint64_t *key, int64_t *cou
     cudaStream_t s = (cudaStream_t)stream;
     CK(cudaSetDevice(e->cfg.device));
     if (!e->counted) return fail(e, STBPE_E_STATE, "count the pairs before selecting");
-    select_kernel<<<e->select_grid, STBPE_SELECT_THREADS, 0, s>>>(e->d, 0, 0, e->cand);
-    CK(cudaGetLastError());
+    DevState h;
+    if (e->cfg.world_size > 1) {
+        select_kernel<<<e->select_grid, STBPE_SELECT_THREADS, 0, s>>>(e->d, 0, e->partial, e->cand);
+        CK(cudaGetLastError());
+    } else {
+        int rc = choose(e, false, &h, s);
+        if (rc != STBPE_OK) return rc;
+    }
     if (n_ties) {
         CK(cudaMemsetAsync(&e->d.st->peek_ties, 0, sizeof(i64), s));
         count_ties_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d);
         CK(cudaGetLastError());
     }
-    DevState h;
     CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     *key = h.peek_count > 0 ? h.peek_key : 0;
@@ -732,19 +804,18 @@ STBPE_VISIBLE int stbpe_select_best(stbpe_engine *e, uint64_t *key, int64_t *cou
 }
 
 static int filter_policy(stbpe_engine *e, const DevState &h, bool layout_changed, cudaStream_t s);
+static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t first_new, int64_t *n_matches, cudaStream_t s);
 
 static int launch_merge(stbpe_engine *e, bool mg, cudaStream_t s) {
-    if (e->d.n_tiles > 0) {
-        const int wl_words = (e->d.n_tiles + 31) / 32;
-        int wl_grid = (wl_words + 1023) / 1024;
-        if (wl_grid > 32) wl_grid = 32;
-        CK(launch_loop_kernel(e, true, worklist_kernel, wl_grid, 1024, 0, s, e->d));
-        int grid = e->merge_grid < e->d.n_tiles ? e->merge_grid : e->d.n_tiles;
+    if (e->d.n_tiles < 1) return STBPE_OK;
+    with_tok(e, [&](auto t) {
+        typedef decltype(t) T;
         if (mg)
-            CK(launch_loop_kernel(e, true, merge_kernel<true>, grid, STBPE_CTA_THREADS, e->merge_smem, s, e->d, e->merge_slots));
+            merge_kernel<T, true><<<e->sm_count, MergeGeom<T>::THREADS, MergeGeom<T>::BYTES, s>>>(e->d, unit_shift(e, e->sm_count));
         else
-            CK(launch_loop_kernel(e, true, merge_kernel<false>, grid, STBPE_CTA_THREADS, e->merge_smem, s, e->d, e->merge_slots));
-    }
+            merge_kernel<T, false><<<e->sm_count, MergeGeom<T>::THREADS, MergeGeom<T>::BYTES, s>>>(e->d, unit_shift(e, e->sm_count));
+    });
+    CK(cudaGetLastError());
     return STBPE_OK;
 }
 
@@ -757,28 +828,11 @@ STBPE_VISIBLE int stbpe_apply_merge(stbpe_engine *e, int32_t a, int32_t b, int32
     if (e->cfg.world_size > 1) return fail(e, STBPE_E_STATE, "single-rank entry point");
     if (a < 0 || b < 0 || new_id < 0 || a == 0x7FFFFFFF || b == 0x7FFFFFFF || new_id == 0x7FFFFFFF)
         return fail(e, STBPE_E_ID_OVERFLOW, "Token id overflow: ids must be in [0, 2^31-2]");
-    DevState h;
-    CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    if (h.merges_done >= e->cfg.max_merges) return fail(e, STBPE_E_CAPACITY, "merge log full");
-    force_merge_kernel<<<1, 1, 0, s>>>(e->d, a, b, new_id);
-    CK(cudaGetLastError());
-    // the count the table held for (a, b) decides whether this merge keeps the pair filter
-    CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    {
-        int rc = filter_policy(e, h, false, s);
-        if (rc != STBPE_OK) return rc;
-    }
-    int rc = launch_merge(e, false, s);
-    if (rc != STBPE_OK) return rc;
-    rc = launch_refresh(e, 0, s);
-    if (rc != STBPE_OK) return rc;
-    CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    if (n_matches) *n_matches = h.n_matches;
-    return check_device_error(e, s);
+    const int32_t pair[2] = {a, b};
+    return run_forced(e, pair, 1, new_id, n_matches, s);
 }
+
+static int maybe_repack(stbpe_engine *e, bool force, int *did, cudaStream_t s);
 
 // Keep or drop the pair filter.  A merge whose matches outnumber the tiles visits nearly every tile
 // whatever the filter says, while entering its new pairs into the filter costs more than the
@@ -790,6 +844,7 @@ static int filter_policy(stbpe_engine *e, const DevState &h, bool layout_changed
     if (e->d.n_tiles < 1) return STBPE_OK;
     i64 cnt = h.merges_done > 0 ? h.cur_count : h.peek_count;  // last selected pair, else the best pair of the count
     cnt /= e->cfg.world_size;  // the count is global, the tiles are this rank's
+    if (h.merges_done == 0 && h.peek_count == 0) return STBPE_OK;  // nothing has been selected yet
     const bool want = (double)cnt <= e->filter_density * (double)e->d.n_tiles;
     if (want && (!e->filter_valid || layout_changed)) return rebuild_presence(e, s);
     if (layout_changed) {
@@ -798,6 +853,80 @@ static int filter_policy(stbpe_engine *e, const DevState &h, bool layout_changed
         e->filter_valid = false;
     }
     return STBPE_OK;
+}
+
+// Live tokens into the other stream buffer, densely, as 16- or 32-bit tokens; fresh tile records.
+static int repack_stream(stbpe_engine *e, bool to_wide, i64 *total, cudaStream_t s) {
+    const int nt = e->d.n_tiles;
+    i64 *lens = e->rp_lens, *offs = e->rp_offs;
+    CK(cudaMemsetAsync(lens + nt, 0, sizeof(i64), s));
+    tile_lens_kernel<<<(nt + 255) / 256, 256, 0, s>>>(e->d, lens);
+    CK(cudaGetLastError());
+    size_t tmp_bytes = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, lens, offs, nt + 1, s);
+    if (tmp_bytes > e->rp_tmp_bytes) return fail(e, STBPE_E_STATE, "re-pack scratch too small");
+    tmp_bytes = e->rp_tmp_bytes;
+    cub::DeviceScan::ExclusiveSum(e->rp_tmp, tmp_bytes, lens, offs, nt + 1, s);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(total, offs + nt, sizeof(i64), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    const size_t want = (size_t)((*total + STBPE_TILE - 1) / STBPE_TILE) * STBPE_TILE * (to_wide ? 4 : 2);
+    if (want > e->alt_bytes || !e->tiles_alt) {
+        unsigned char *t = nullptr;
+        cudaError_t c = dev_alloc(e, &t, want);
+        if (c != cudaSuccess) return cuda_fail(e, c, "cudaMalloc second stream buffer");
+        e->tiles_alt = t;
+        e->alt_bytes = want;
+    }
+    const int warps = STBPE_REPACK_THREADS / 32;
+    const int need = (nt + warps - 1) / warps, grid = need < e->sm_count * 16 ? need : e->sm_count * 16;
+    if (e->wide)
+        repack_copy_kernel<uint32_t, uint32_t, false><<<grid, STBPE_REPACK_THREADS, 0, s>>>(e->d, offs, (uint32_t *)e->tiles_alt);
+    else if (to_wide)
+        repack_copy_kernel<uint16_t, uint32_t, false><<<grid, STBPE_REPACK_THREADS, 0, s>>>(e->d, offs, (uint32_t *)e->tiles_alt);
+    else
+        repack_copy_kernel<uint16_t, uint16_t, false><<<grid, STBPE_REPACK_THREADS, 0, s>>>(e->d, offs, (uint16_t *)e->tiles_alt);
+    CK(cudaGetLastError());
+    std::swap(e->d.tiles, e->tiles_alt);
+    std::swap(e->tiles_bytes, e->alt_bytes);
+    e->wide = to_wide;
+    e->d.n_tiles = (int)((*total + STBPE_TILE - 1) / STBPE_TILE);
+    e->n_tokens = *total;  // capacity in use; the merge log keeps the live counts
+    if (e->d.n_tiles > 0) {
+        with_tok(e, [&](auto t) {
+            init_recs_kernel<decltype(t)><<<(e->d.n_tiles + 255) / 256, 256, 0, s>>>(e->d, *total);
+        });
+        CK(cudaGetLastError());
+    }
+    return STBPE_OK;
+}
+
+// The 16-bit stream becomes a 32-bit one: an id of 15 bits or more has to go in (a new merge's id, or an id
+// of the caller's).  A stream that is still being loaded is converted as it stands, one that merges have
+// rewritten is re-packed on the way (its pair filter must then be rebuilt by the caller's policy).
+static int widen_stream(stbpe_engine *e, cudaStream_t s) {
+    if (e->wide) return STBPE_OK;
+    const size_t full = (size_t)e->max_tiles * STBPE_TILE * 4;
+    if (e->recs_stale) {
+        unsigned char *t = nullptr;
+        cudaError_t c = dev_alloc(e, &t, full);
+        if (c != cudaSuccess) return cuda_fail(e, c, "cudaMalloc 32-bit token stream");
+        if (e->n_tokens > 0) {
+            widen_copy_kernel<<<e->sm_count * 8, 256, 0, s>>>((const uint16_t *)e->d.tiles, (uint32_t *)t, e->n_tokens);
+            CK(cudaGetLastError());
+        }
+        CK(cudaStreamSynchronize(s));
+        dev_free(e, e->d.tiles);
+        dev_free(e, e->tiles_alt);
+        e->tiles_alt = nullptr;
+        e->alt_bytes = 0;
+        e->d.tiles = t;
+        e->tiles_bytes = full;
+        e->wide = true;
+        return STBPE_OK;
+    }
+    i64 total = 0;
+    return repack_stream(e, true, &total, s);
 }
 
 // Maintenance between batches of merges: dense re-pack of the stream when at most three quarters of
@@ -812,35 +941,11 @@ static int maybe_repack(stbpe_engine *e, bool force, int *did, cudaStream_t s) {
     CK(cudaStreamSynchronize(s));
     if (nt < 2 || (!force && (h.n_live * 4 > (i64)nt * STBPE_TILE * 3 || nt < 64)))  // re-pack at <= 75 % fill
         return filter_policy(e, h, false, s);
-    if (!e->tiles_alt) CK(dev_alloc(e, &e->tiles_alt, (size_t)e->max_tiles * STBPE_TILE));
-    i64 *lens = e->rp_lens, *offs = e->rp_offs;
-    CK(cudaMemsetAsync(lens + nt, 0, sizeof(i64), s));
-    tile_lens_kernel<<<(nt + 255) / 256, 256, 0, s>>>(e->d, lens);
-    CK(cudaGetLastError());
-    size_t tmp_bytes = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, lens, offs, nt + 1, s);
-    if (tmp_bytes > e->rp_tmp_bytes) return fail(e, STBPE_E_STATE, "re-pack scratch too small");
-    tmp_bytes = e->rp_tmp_bytes;
-    cub::DeviceScan::ExclusiveSum(e->rp_tmp, tmp_bytes, lens, offs, nt + 1, s);
-    CK(cudaGetLastError());
-    repack_copy_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d, offs, e->tiles_alt);
-    CK(cudaGetLastError());
     i64 total = 0;
-    CK(cudaMemcpyAsync(&total, offs + nt, sizeof(i64), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    uint32_t *old = e->d.tiles;
-    e->d.tiles = e->tiles_alt;
-    e->tiles_alt = old;
-    e->d.n_tiles = (int)((total + STBPE_TILE - 1) / STBPE_TILE);
-    e->n_tokens = total;  // capacity in use; the merge log keeps the live counts
-    if (e->d.n_tiles > 0) {
-        init_recs_kernel<<<(e->d.n_tiles + 255) / 256, 256, 0, s>>>(e->d, total);
-        CK(cudaGetLastError());
-    }
-    {
-        int rc = filter_policy(e, h, true, s);
-        if (rc != STBPE_OK) return rc;
-    }
+    int rc = repack_stream(e, e->wide, &total, s);
+    if (rc != STBPE_OK) return rc;
+    rc = filter_policy(e, h, true, s);
+    if (rc != STBPE_OK) return rc;
     CK(cudaStreamSynchronize(s));
     e->repacks++;
     e->repacks_since_load++;
@@ -861,15 +966,74 @@ __global__ void set_target_kernel(EngineDev e, int target) {
     e.st->n_matches = 0;
 }
 
-// One iteration of the single-GPU loop: select, worklist, merge, refresh.  (Folding refresh, select
-// and the worklist into one launch was tried: the CTA that finishes last then recomputes the dirty
-// super-block maxima and walks the filter rows alone, and since early in a run nearly every
-// super-block is dirty that took 85-400 us per merge instead of the 30 us of the three launches.)
-static int enqueue_iteration(stbpe_engine *e, cudaStream_t s) {
-    CK(launch_loop_kernel(e, false, select_kernel, e->select_grid, STBPE_SELECT_THREADS, 0, s, e->d, 1, 0, e->cand, 0));
-    int rc = launch_merge(e, false, s);
-    if (rc != STBPE_OK) return rc;
-    return launch_refresh(e, 0, s);
+// CTAs of a loop launch: one per SM, fewer on a stream of few tiles (every CTA is a participant of two
+// grid-wide exchanges per merge); enough of them that the block maxima fit their shared memory
+static int loop_grid(const stbpe_engine *e) {
+    return e->sm_count;
+}
+
+// Runs loop_kernel until a stop rule fires, doing the maintenance it asks for between launches.  `forced`
+// (device, n_forced pairs): these merges instead of the best pairs.  *out = the device state at the end.
+static int run_loop(stbpe_engine *e, int target, const int2 *forced, int n_forced, int forced_new, DevState *out,
+                    cudaStream_t s) {
+    LoopArgs la;
+    int at = 0;
+    for (;;) {
+        const int grid = loop_grid(e);
+        la.target = target;
+        la.forced = forced ? forced + at : nullptr;
+        la.n_forced = n_forced - at;
+        la.forced_new = forced_new + at;
+        const double fc = e->filter_density * (double)e->d.n_tiles;
+        la.filter_count = fc >= 9e18 ? (i64)9000000000000000000ll : (i64)fc;
+        la.repack_tiles = 64;
+        la.unit_shift = unit_shift(e, grid);
+        EngineDev d = e->d;
+        void *args[2] = {&d, &la};
+        CK(cudaMemsetAsync(e->d.sync, 0, sizeof(LoopSync), s));
+        const cudaError_t c = with_tok(e, [&](auto t) {
+            typedef decltype(t) T;
+            return cudaLaunchCooperativeKernel((const void *)loop_kernel<T>, dim3(grid), dim3(MergeGeom<T>::THREADS), args,
+                                               MergeGeom<T>::BYTES + STBPE_CAND_CAP * sizeof(unsigned int), s);
+        });
+        if (c != cudaSuccess) return cuda_fail(e, c, "cudaLaunchCooperativeKernel");
+        CK(cudaMemcpyAsync(out, e->d.st, sizeof(*out), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        at += forced ? out->forced_done : 0;
+        int rc = check_error_bits(e, out->error);
+        if (rc != STBPE_OK) return rc;
+        if (out->run_exit == STBPE_EXIT_STOP) return STBPE_OK;
+        if (out->run_exit == STBPE_EXIT_REFILL) {
+            rc = refill_candidates(e, s);
+        } else if (out->run_exit == STBPE_EXIT_REPACK) {
+            rc = maybe_repack(e, false, nullptr, s);
+        } else if (out->run_exit == STBPE_EXIT_FILTER) {
+            rc = rebuild_presence(e, s);
+        } else {
+            rc = widen_stream(e, s);
+            if (rc == STBPE_OK) rc = filter_policy(e, *out, true, s);
+        }
+        if (rc != STBPE_OK) return rc;
+    }
+}
+
+// host-given merges, applied in order as merges of the log
+static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t first_new, int64_t *n_matches, cudaStream_t s) {
+    DevState h;
+    CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    if ((i64)h.merges_done + n > e->cfg.max_merges) return fail(e, STBPE_E_CAPACITY, "merge log full");
+    if (n > e->forced_cap) {
+        dev_free(e, e->forced);
+        e->forced = nullptr;
+        cudaError_t c = dev_alloc(e, &e->forced, (size_t)n);
+        if (c != cudaSuccess) return cuda_fail(e, c, "cudaMalloc merges");
+        e->forced_cap = n;
+    }
+    CK(cudaMemcpyAsync(e->forced, pairs, (size_t)n * sizeof(int2), cudaMemcpyHostToDevice, s));
+    int rc = run_loop(e, e->cfg.max_merges, e->forced, n, first_new, &h, s);
+    if (rc == STBPE_OK && n_matches) *n_matches = h.n_matches;
+    return rc;
 }
 
 STBPE_VISIBLE int stbpe_train(stbpe_engine *e, int32_t n_merges, void *stream) {
@@ -883,71 +1047,7 @@ STBPE_VISIBLE int stbpe_train(stbpe_engine *e, int32_t n_merges, void *stream) {
     CK(cudaStreamSynchronize(s));
     i64 target = (i64)h.merges_done + n_merges;
     if (target > e->cfg.max_merges) target = e->cfg.max_merges;
-    set_target_kernel<<<1, 1, 0, s>>>(e->d, (int)target);
-    CK(cudaGetLastError());
-    int todo = (int)(target - h.merges_done);
-    const int G = 32, CHECK = 256;  // merges per graph replay / per look at the device state
-    while (todo > 0) {
-        int rc = maybe_repack(e, false, nullptr, s);
-        if (rc != STBPE_OK) return rc;
-        // while the pair filter is stale the counts are looked at after every graph replay, so that
-        // tile skipping starts soon after it begins to pay
-        const int chk = (e->filter_valid || e->d.n_tiles < 64) ? CHECK : G;
-        int batch = todo < chk ? todo : chk;
-        todo -= batch;
-        if (e->use_graph && batch >= G) {
-            // the kernels take all their work from device state, so one captured batch of G
-            // iterations is replayed; iterations past a stop rule return immediately
-            if (e->graph && (e->graph_merges != e->d.n_tiles || e->graph_tiles != e->d.tiles)) {
-                cudaGraphExecDestroy(e->graph);
-                e->graph = nullptr;
-            }
-            if (!e->graph) {
-                cudaStream_t cs;
-                CK(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-                cudaGraph_t g;
-                CK(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-                int rc2 = STBPE_OK;
-                e->pdl_now = e->use_pdl;
-                for (int i = 0; i < G && rc2 == STBPE_OK; ++i) rc2 = enqueue_iteration(e, cs);
-                e->pdl_now = false;
-                cudaError_t ce = cudaStreamEndCapture(cs, &g);
-                if (rc2 != STBPE_OK) {
-                    cudaStreamDestroy(cs);
-                    return rc2;
-                }
-                if (ce != cudaSuccess) {
-                    cudaStreamDestroy(cs);
-                    return cuda_fail(e, ce, "cudaStreamEndCapture");
-                }
-                ce = cudaGraphInstantiate(&e->graph, g, 0);
-                cudaGraphDestroy(g);
-                cudaStreamDestroy(cs);
-                if (ce != cudaSuccess) return cuda_fail(e, ce, "cudaGraphInstantiate");
-                e->graph_merges = e->d.n_tiles;  // the capture froze the stream pointer, n_tiles and the grids
-                e->graph_tiles = e->d.tiles;
-            }
-            while (batch > 0) {
-                CK(cudaGraphLaunch(e->graph, s));
-                batch -= G;
-            }
-        } else {
-            for (int i = 0; i < batch; ++i) {
-                rc = enqueue_iteration(e, s);
-                if (rc != STBPE_OK) return rc;
-            }
-        }
-        if (todo > 0) {  // stop early when a stop rule fired
-            CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
-            CK(cudaStreamSynchronize(s));
-            if (h.stopped) break;
-        }
-    }
-    // one more selection decides the stop reason without applying anything when the target is reached
-    select_kernel<<<e->select_grid, STBPE_SELECT_THREADS, 0, s>>>(e->d, 1, 0, e->cand);
-    CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(s));
-    return check_device_error(e, s);
+    return run_loop(e, (int)target, nullptr, 0, 0, &h, s);
 }
 
 // Same loop as stbpe_train, launched kernel by kernel with CUDA events around every launch so
@@ -967,6 +1067,7 @@ STBPE_VISIBLE int stbpe_train_timed(stbpe_engine *e, int32_t n_merges, float *ke
     CK(cudaGetLastError());
     const int todo = (int)(target - h.merges_done);
     const int P = 128;
+    DevState h2;
     std::vector<cudaEvent_t> ev(4 * P);
     for (auto &x : ev) CK(cudaEventCreate(&x));
     kernel_ms[0] = kernel_ms[1] = kernel_ms[2] = kernel_ms[3] = 0.f;
@@ -991,13 +1092,23 @@ STBPE_VISIBLE int stbpe_train_timed(stbpe_engine *e, int32_t n_merges, float *ke
         }
         const int step = (e->filter_valid || e->d.n_tiles < 64) ? P : 32;
         n = todo - base < step ? todo - base : step;
+        if (!e->wide && (i64)e->cfg.base_vocab + h.merges_done + base + n >= (i64)Tok<uint16_t>::IDMASK) {
+            rc = widen_stream(e, s);
+            if (rc == STBPE_OK) {
+                CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
+                CK(cudaStreamSynchronize(s));
+                h.merges_done -= base;
+                rc = filter_policy(e, h, true, s);
+            }
+            if (rc != STBPE_OK) break;
+        }
         for (int i = 0; i < n && rc == STBPE_OK; ++i) {
             cudaEventRecord(ev[4 * i], s);
-            select_kernel<<<e->select_grid, STBPE_SELECT_THREADS, 0, s>>>(e->d, 1, 0, e->cand);
+            rc = choose(e, true, &h2, s);
             cudaEventRecord(ev[4 * i + 1], s);
+            if (rc != STBPE_OK) break;
             rc = launch_merge(e, false, s);
             cudaEventRecord(ev[4 * i + 2], s);
-            if (rc == STBPE_OK) rc = launch_refresh(e, 0, s);
             cudaEventRecord(ev[4 * i + 3], s);
         }
         cudaStreamSynchronize(s);
@@ -1012,10 +1123,8 @@ STBPE_VISIBLE int stbpe_train_timed(stbpe_engine *e, int32_t n_merges, float *ke
     cudaEventDestroy(r0);
     cudaEventDestroy(r1);
     if (rc != STBPE_OK) return rc;
-    select_kernel<<<e->select_grid, STBPE_SELECT_THREADS, 0, s>>>(e->d, 1, 0, e->cand);
-    CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(s));
-    return check_device_error(e, s);
+    rc = choose(e, true, &h2, s);
+    return rc != STBPE_OK ? rc : check_device_error(e, s);
 }
 
 STBPE_VISIBLE int stbpe_get_state(stbpe_engine *e, stbpe_state *out, void *stream) {
@@ -1113,24 +1222,23 @@ STBPE_VISIBLE int stbpe_export_stream(stbpe_engine *e, int32_t *ids, int64_t cap
     const int nt = e->d.n_tiles;
     *n_out = 0;
     if (nt == 0) return STBPE_OK;
-    i64 *dl = nullptr;
-    CK(cudaMallocAsync((void **)&dl, (size_t)(nt + 1) * sizeof(i64), s));
-    tile_lens_kernel<<<(nt + 255) / 256, 256, 0, s>>>(e->d, dl);
+    i64 *lens = e->rp_lens, *offs = e->rp_offs, total = 0;
+    CK(cudaMemsetAsync(lens + nt, 0, sizeof(i64), s));
+    tile_lens_kernel<<<(nt + 255) / 256, 256, 0, s>>>(e->d, lens);
     CK(cudaGetLastError());
-    std::vector<i64> lens(nt + 1), off(nt + 1);
-    CK(cudaMemcpyAsync(lens.data(), dl, (size_t)nt * sizeof(i64), cudaMemcpyDeviceToHost, s));
+    size_t tmp_bytes = e->rp_tmp_bytes;
+    cub::DeviceScan::ExclusiveSum(e->rp_tmp, tmp_bytes, lens, offs, nt + 1, s);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(&total, offs + nt, sizeof(i64), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    off[0] = 0;
-    for (int t = 0; t < nt; ++t) off[t + 1] = off[t] + lens[t];
-    *n_out = off[nt];
-    if (off[nt] > cap) {
-        cudaFreeAsync(dl, s);
-        return fail(e, STBPE_E_CAPACITY, "export buffer too small");
-    }
-    CK(cudaMemcpyAsync(dl, off.data(), (size_t)(nt + 1) * sizeof(i64), cudaMemcpyHostToDevice, s));
-    export_stream_kernel<<<e->sm_count * 4, 256, 0, s>>>(e->d, dl, ids);
+    *n_out = total;
+    if (total > cap) return fail(e, STBPE_E_CAPACITY, "export buffer too small");
+    const int warps = STBPE_REPACK_THREADS / 32;
+    const int need = (nt + warps - 1) / warps, grid = need < e->sm_count * 16 ? need : e->sm_count * 16;
+    with_tok(e, [&](auto t) {
+        repack_copy_kernel<decltype(t), uint32_t, true><<<grid, STBPE_REPACK_THREADS, 0, s>>>(e->d, offs, (uint32_t *)ids);
+    });
     CK(cudaGetLastError());
-    CK(cudaFreeAsync(dl, s));
     CK(cudaStreamSynchronize(s));
     return STBPE_OK;
 }
@@ -1204,7 +1312,7 @@ STBPE_VISIBLE int stbpe_mg_candidate(stbpe_engine *e, void *cand_dev, void *stre
     if (!e || !cand_dev) return STBPE_E_BADARG;
     cudaStream_t s = (cudaStream_t)stream;
     CK(cudaSetDevice(e->cfg.device));
-    select_kernel<<<e->select_grid, STBPE_SELECT_THREADS, 0, s>>>(e->d, 2, 0, (i64 *)cand_dev);
+    select_kernel<<<e->select_grid, STBPE_SELECT_THREADS, 0, s>>>(e->d, 2, e->partial, (i64 *)cand_dev);
     CK(cudaGetLastError());
     return STBPE_OK;
 }
@@ -1451,7 +1559,7 @@ static int enqueue_peer_round(stbpe_engine *e, bool count_round, cudaStream_t s)
     e->full_refresh_pending = false;
     rc = launch_refresh(e, all, s);
     if (rc != STBPE_OK) return rc;
-    select_kernel<<<e->select_grid, STBPE_SELECT_THREADS, 0, s>>>(e->d, 3, 0, e->cand, e->cfg.max_merges);
+    select_kernel<<<e->select_grid, STBPE_SELECT_THREADS, 0, s>>>(e->d, 3, e->partial, e->cand, e->cfg.max_merges);
     CK(cudaGetLastError());
     return STBPE_OK;
 }
@@ -1473,7 +1581,7 @@ STBPE_VISIBLE int stbpe_mg_peer_run(stbpe_engine *e, int first, int n_rounds, vo
     const int G = 16;  // rounds per graph replay
     while (r < n_rounds) {
         if (e->use_graph && n_rounds - r >= G) {
-            if (e->graph && (e->graph_merges != e->d.n_tiles || e->graph_tiles != e->d.tiles)) {
+            if (e->graph && (e->graph_tiles_n != e->d.n_tiles || e->graph_tiles != e->d.tiles || e->graph_wide != e->wide)) {
                 cudaGraphExecDestroy(e->graph);
                 e->graph = nullptr;
             }
@@ -1483,9 +1591,7 @@ STBPE_VISIBLE int stbpe_mg_peer_run(stbpe_engine *e, int first, int n_rounds, vo
                 cudaGraph_t g;
                 CK(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
                 int rc2 = STBPE_OK;
-                e->pdl_now = e->use_pdl;
                 for (int i = 0; i < G && rc2 == STBPE_OK; ++i) rc2 = enqueue_peer_round(e, false, cs);
-                e->pdl_now = false;
                 cudaError_t ce = cudaStreamEndCapture(cs, &g);
                 if (rc2 != STBPE_OK) {
                     cudaStreamDestroy(cs);
@@ -1499,8 +1605,9 @@ STBPE_VISIBLE int stbpe_mg_peer_run(stbpe_engine *e, int first, int n_rounds, vo
                 cudaGraphDestroy(g);
                 cudaStreamDestroy(cs);
                 if (ce != cudaSuccess) return cuda_fail(e, ce, "cudaGraphInstantiate");
-                e->graph_merges = e->d.n_tiles;
+                e->graph_tiles_n = e->d.n_tiles;  // the capture froze the stream pointer, n_tiles and the grids
                 e->graph_tiles = e->d.tiles;
+                e->graph_wide = e->wide;
             }
             CK(cudaGraphLaunch(e->graph, s));
             r += G;

@@ -1,67 +1,97 @@
 // Kernels of the BPE merge-loop engine (sm_100a).  See common.cuh for the data layout.
 #pragma once
-#include "common.cuh"
+#include "merge.cuh"
 
 // ---------------------------------------------------------------------------------------
-// K1  pack: bytes / ids -> uint32 stream words, row-start flags, tile records
+// K1  pack: bytes / ids -> stream tokens, row-start flags, tile records
 // ---------------------------------------------------------------------------------------
-// identity byte -> id map of the reference's packer (gpu_tokenizer/cpu_packer.py:17-26)
-__global__ void pack_bytes_kernel(const uint8_t *__restrict__ src, i64 n, uint32_t *__restrict__ dst) {
-    i64 i = ((i64)blockIdx.x * blockDim.x + threadIdx.x) * 16;
-    i64 stride = (i64)gridDim.x * blockDim.x * 16;
-    bool aligned = ((((uintptr_t)src) | ((uintptr_t)dst)) & 15) == 0;
-    for (; i < n; i += stride) {
-        if (aligned && i + 16 <= n) {
-            uint4 v = *reinterpret_cast<const uint4 *>(src + i);
-            uint32_t w[4] = {v.x, v.y, v.z, v.w};
+// identity byte -> id map of the reference's packer (gpu_tokenizer/cpu_packer.py:17-26).
+// Streaming copy, one group of 32 tokens per thread: 32 source bytes become the group's 16 words (a byte
+// permutation per word).  `at` = stream position of src[0]; groups that the append covers only in part, and
+// sources that are not 16-byte aligned relative to the groups, are written token by token.
+template <typename T>
+__device__ __forceinline__ void put_token(void *tiles, i64 pos, uint32_t v) {
+    reinterpret_cast<T *>(tiles)[Tok<T>::index(pos)] = (T)v;
+}
+
+template <typename T>
+__global__ void pack_bytes_kernel(const uint8_t *__restrict__ src, i64 n, void *tiles, i64 at) {
+    const i64 g0 = at >> 5, g1 = (at + n + 31) >> 5;
+    for (i64 g = g0 + (i64)blockIdx.x * blockDim.x + threadIdx.x; g < g1; g += (i64)gridDim.x * blockDim.x) {
+        const i64 p = g * 32;
+        const uint8_t *q = src + (p - at);
+        if (p >= at && p + 32 <= at + n && ((uintptr_t)q & 15) == 0) {
+            const uint4 x = __ldcs(reinterpret_cast<const uint4 *>(q)), y = __ldcs(reinterpret_cast<const uint4 *>(q) + 1);
+            const uint32_t lo[4] = {x.x, x.y, x.z, x.w}, hi[4] = {y.x, y.y, y.z, y.w};
+            uint4 *d = reinterpret_cast<uint4 *>(reinterpret_cast<T *>(tiles) + p);
+            if (sizeof(T) == 2) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                uint4 o;
-                o.x = w[q] & 0xFF;
-                o.y = (w[q] >> 8) & 0xFF;
-                o.z = (w[q] >> 16) & 0xFF;
-                o.w = w[q] >> 24;
-                *reinterpret_cast<uint4 *>(dst + i + 4 * q) = o;
+                for (int j = 0; j < 4; ++j) {  // word 4j + i = byte i of lo[j] | byte i of hi[j] << 16
+                    const uint32_t a = __byte_perm(lo[j], 0, 0x4140), b = __byte_perm(lo[j], 0, 0x4342);
+                    const uint32_t c = __byte_perm(hi[j], 0, 0x4140), e = __byte_perm(hi[j], 0, 0x4342);
+                    d[j] = make_uint4(__byte_perm(a, c, 0x5410), __byte_perm(a, c, 0x7632), __byte_perm(b, e, 0x5410),
+                                      __byte_perm(b, e, 0x7632));
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const uint32_t w = j < 4 ? lo[j & 3] : hi[j & 3];
+                    d[j] = make_uint4(w & 0xFFu, (w >> 8) & 0xFFu, (w >> 16) & 0xFFu, w >> 24);
+                }
             }
         } else {
-            for (i64 k = i; k < n && k < i + 16; ++k) dst[k] = src[k];
+            for (int i = 0; i < 32; ++i)
+                if (p + i >= at && p + i < at + n) put_token<T>(tiles, p + i, q[i]);
         }
     }
 }
 
-__global__ void pack_ids_kernel(const int32_t *__restrict__ src, i64 n, uint32_t *__restrict__ dst,
-                                unsigned int *bad) {
-    i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    i64 stride = (i64)gridDim.x * blockDim.x;
-    for (; i < n; i += stride) {
-        int32_t v = src[i];
-        if (v < 0 || v == 0x7FFFFFFF) atomicOr(bad, STBPE_DERR_BAD_ID);  // ids must leave bit 31 and NONE free
-        dst[i] = (uint32_t)v & STBPE_IDMASK;
+// ids must leave the top bit and the hole value free: out-of-range ids raise BAD_ID, ids that only a wider
+// stream can hold NARROW (the host then widens the stream and packs again)
+template <typename T>
+__global__ void pack_ids_kernel(const int32_t *__restrict__ src, i64 n, void *tiles, i64 at, unsigned int *bad) {
+    unsigned int err = 0;
+    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
+        const int32_t v = __ldcs(src + i);
+        if (v < 0 || v == 0x7FFFFFFF)
+            err |= STBPE_DERR_BAD_ID;
+        else if ((uint32_t)v >= Tok<T>::IDMASK)
+            err |= STBPE_DERR_NARROW;
+        put_token<T>(tiles, at + i, (uint32_t)v & Tok<T>::IDMASK);
+    }
+    if (err) atomicOr(bad, err);
+}
+
+template <typename T>
+__global__ void mark_row_starts_kernel(const i64 *__restrict__ off, i64 n_rows, void *tiles, i64 at) {
+    const i64 r = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r < n_rows && off[r] < off[r + 1]) {
+        T *t = reinterpret_cast<T *>(tiles) + Tok<T>::index(at + off[r]);
+        *t = (T)(*t | Tok<T>::FLAG);
     }
 }
 
-__global__ void mark_row_starts_kernel(const i64 *__restrict__ off, i64 n_rows, uint32_t *stream) {
-    i64 r = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < n_rows && off[r] < off[r + 1]) stream[off[r]] |= STBPE_FLAG;
-}
-
+// records of a dense stream; the positions of the last tile past its end become holes
+template <typename T>
 __global__ void init_recs_kernel(EngineDev e, i64 n_tokens) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= e.n_tiles) return;
-    i64 base = (i64)t * STBPE_TILE;
-    i64 rem = n_tokens - base;
-    int len = rem >= STBPE_TILE ? STBPE_TILE : (int)rem;
+    T *tok = tile_ptr<T>(e, t);
+    const i64 rem = n_tokens - (i64)t * STBPE_TILE;
+    const int len = rem >= STBPE_TILE ? STBPE_TILE : (int)rem;
+    for (int i = len; i < STBPE_TILE; ++i) tok[Tok<T>::index(i)] = (T)Tok<T>::HOLE;
     TileRec r;
     r.ver = 0;
     r.len = len;
-    for (int i = 0; i < 3; ++i) r.head[i] = i < len ? e.tiles[base + i] : STBPE_NONE;
-    r.tail = len > 0 ? e.tiles[base + len - 1] : STBPE_NONE;
-    r.tail2 = len > 1 ? e.tiles[base + len - 2] : STBPE_NONE;
+    for (int i = 0; i < 3; ++i) r.head[i] = i < len ? Tok<T>::widen(tok[Tok<T>::index(i)]) : STBPE_NONE;
+    r.tail = len > 0 ? Tok<T>::widen(tok[Tok<T>::index(len - 1)]) : STBPE_NONE;
+    r.tail2 = len > 1 ? Tok<T>::widen(tok[Tok<T>::index(len - 2)]) : STBPE_NONE;
     r.pad = 0;
     e.recs[2 * t] = r;
     r.ver = -1;
     r.len = 0;
     e.recs[2 * t + 1] = r;
+    e.tile_live[t] = (unsigned int)len;
 }
 
 __global__ void clear_table_kernel(EngineDev e) {
@@ -75,7 +105,34 @@ __global__ void clear_table_kernel(EngineDev e) {
     }
 }
 
-#include "tile_kernels.cuh"
+// ---------------------------------------------------------------------------------------
+// K2  full adjacent-pair histogram of any stream (gpu_tokenizer/utils.py:558-635 without the sort): one warp
+// per tile, one group of tokens per lane; every countable pair adds +1 into the CTA's shared-memory
+// table, flushed at the end into the pair table (or, multi-GPU, into the rank-local delta table).
+// ---------------------------------------------------------------------------------------
+#define STBPE_COUNT_THREADS 512
+#define STBPE_COUNT_SLOTS 8192
+template <typename T, bool MG>
+__global__ void __launch_bounds__(STBPE_COUNT_THREADS, 2) count_kernel(const __grid_constant__ EngineDev e) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    SmemTable tab;
+    tab.keys = reinterpret_cast<u64 *>(smem_raw);
+    tab.vals = reinterpret_cast<int *>(smem_raw + STBPE_COUNT_SLOTS * sizeof(u64));
+    tab.mask = STBPE_COUNT_SLOTS - 1;
+    smem_table_clear(tab);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    for (i64 t = (i64)blockIdx.x * warps + (threadIdx.x >> 5); t < e.n_tiles; t += (i64)gridDim.x * warps) {
+        uint32_t w[Tok<T>::VEC * 4];
+        load_group<T>(e, (int)t, lane, w);
+        const uint32_t nxt = first_after(e, (int)t, 0x7FFFFFFF);
+        for_each_pair<T>(w, live_mask<T>(w), lane, nxt, [&](uint32_t t0, uint32_t t1) {
+            if (!(t1 & STBPE_FLAG)) smem_table_add<MG>(tab, e, ((u64)(t0 & STBPE_IDMASK) << 32) | (u64)t1, 1);
+        });
+    }
+    __syncthreads();
+    smem_table_flush<MG>(tab, e);
+}
 
 // ---------------------------------------------------------------------------------------
 // K2, byte-level fast path.  Right after a load of bytes the stream is dense (every tile full)
@@ -108,10 +165,10 @@ __device__ __noinline__ void dense_hand_over(unsigned int *s_tab, u64 *g_dense, 
     // 0x8000 < h <= 0xC000: another thread is handing this counter over; h < 0x8000: it was the other half
 }
 
+// t1 is below 256: a right-hand token that starts no row
 __device__ __forceinline__ void dense_add(unsigned int *s_tab, u64 *g_dense, unsigned int *derr, uint32_t t0,
                                           uint32_t t1) {
-    if ((int)t1 < 0) return;  // the right token starts a row (or lies past the end): bit 31 set
-    // key = (low byte of t0) << 8 | t1; bytes 1 and 2 of t1 are zero for ids below 256
+    // key = (low byte of t0) << 8 | t1; bytes 1 and 2 of t1 are zero
     const unsigned int key = __byte_perm(t1, t0, 0x2140);
     const unsigned int inc = (key & 1u) ? 0x10000u : 1u;
     const unsigned int now = atomicAdd(&s_tab[dense_word(key)], inc) + inc;
@@ -120,43 +177,25 @@ __device__ __forceinline__ void dense_add(unsigned int *s_tab, u64 *g_dense, uns
 
 #define STBPE_DENSE_THREADS 1024
 #define STBPE_DENSE_UNROLL 4
+template <typename T>
 __global__ void __launch_bounds__(STBPE_DENSE_THREADS, 1)
-    count_dense_kernel(EngineDev e, i64 n_tokens, u64 *g_dense) {
+    count_dense_kernel(EngineDev e, u64 *g_dense) {
     extern __shared__ __align__(16) unsigned int s_tab[];  // 32 768 words
     for (int i = threadIdx.x; i < 32768; i += STBPE_DENSE_THREADS) s_tab[i] = 0u;
     __syncthreads();
-    const uint32_t *tok = e.tiles;
     unsigned int *derr = &e.st->error;
-    const int lane = threadIdx.x & 31;
-    const i64 span = (i64)STBPE_DENSE_THREADS * 4;  // tokens per CTA step
-    for (i64 base = (i64)blockIdx.x * span * STBPE_DENSE_UNROLL; base < n_tokens;
-         base += (i64)gridDim.x * span * STBPE_DENSE_UNROLL) {
+    const uint4 *units = reinterpret_cast<const uint4 *>(e.tiles);
+    const i64 n_units = (i64)e.n_tiles * (STBPE_TILE * sizeof(T) / 16);
+    const i64 step = (i64)gridDim.x * STBPE_DENSE_THREADS * STBPE_DENSE_UNROLL;
+    for (i64 base = (i64)blockIdx.x * STBPE_DENSE_THREADS * STBPE_DENSE_UNROLL; base < n_units; base += step) {
         uint4 v[STBPE_DENSE_UNROLL];
         uint32_t nx[STBPE_DENSE_UNROLL];
+        load_unit_batch<T, STBPE_DENSE_UNROLL, STBPE_DENSE_THREADS>(units, base, n_units, v, nx);
 #pragma unroll
-        for (int u = 0; u < STBPE_DENSE_UNROLL; ++u) {  // all loads first: several in flight per thread
-            const i64 i = base + u * span + (i64)threadIdx.x * 4;
-            if (i + 4 <= n_tokens) {
-                v[u] = *reinterpret_cast<const uint4 *>(tok + i);
-            } else {
-                v[u].x = i < n_tokens ? tok[i] : STBPE_NONE;
-                v[u].y = i + 1 < n_tokens ? tok[i + 1] : STBPE_NONE;
-                v[u].z = i + 2 < n_tokens ? tok[i + 2] : STBPE_NONE;
-                v[u].w = i + 3 < n_tokens ? tok[i + 3] : STBPE_NONE;
-            }
-            nx[u] = (lane == 31) ? (i + 4 < n_tokens ? tok[i + 4] : STBPE_NONE) : 0u;
-        }
-        // tokens past the end were loaded as STBPE_NONE: as a right-hand token NONE carries the
-        // row-start flag (no pair), and a left-hand NONE is always followed by another NONE
-#pragma unroll
-        for (int u = 0; u < STBPE_DENSE_UNROLL; ++u) {
-            uint32_t n0 = __shfl_down_sync(0xFFFFFFFFu, v[u].x, 1);
-            if (lane == 31) n0 = nx[u];
-            dense_add(s_tab, g_dense, derr, v[u].x, v[u].y);
-            dense_add(s_tab, g_dense, derr, v[u].y, v[u].z);
-            dense_add(s_tab, g_dense, derr, v[u].z, v[u].w);
-            dense_add(s_tab, g_dense, derr, v[u].w, n0);
-        }
+        for (int u = 0; u < STBPE_DENSE_UNROLL; ++u)
+            unit_pairs<T>(v[u], nx[u], [&](uint32_t t0, uint32_t t1) {
+                if (!(t1 & Tok<T>::FLAG)) dense_add(s_tab, g_dense, derr, t0, t1);
+            });
     }
     __syncthreads();
     for (int p = threadIdx.x; p < 32768; p += STBPE_DENSE_THREADS) {
@@ -198,57 +237,54 @@ __global__ void dense_to_table_kernel(EngineDev e, const u64 *g_dense) {
 // ---------------------------------------------------------------------------------------
 // K4  arg-max: block maxima refresh + reduction with the reference's tie-break
 // ---------------------------------------------------------------------------------------
-// recompute the maximum of blocks [w0, n) of the dirty list (or of all blocks), one warp per block
-__device__ __forceinline__ void refresh_blocks(const EngineDev &e, int all, unsigned int n, unsigned int w,
-                                               unsigned int nwarps) {
+// maximum of one block, by one warp: its entry with the largest count, ties to the smaller key
+__device__ __forceinline__ Slot block_max(const EngineDev &e, unsigned int blk, int lane) {
+    const Slot *base = e.table + ((u64)blk << e.blk_shift);
+    Slot best;
+    best.key = STBPE_EMPTY;
+    best.count = 0;
+#pragma unroll 8
+    for (int q = lane; q < (1 << e.blk_shift); q += 32) {
+        const Slot x = ldcg_slot(base + q);
+        if (x.key != STBPE_EMPTY && x.count > 0 && better(x.key, x.count, best.key, best.count)) best = x;
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        Slot o;
+        o.key = __shfl_down_sync(0xFFFFFFFFu, best.key, d);
+        o.count = __shfl_down_sync(0xFFFFFFFFu, best.count, d);
+        if (better(o.key, o.count, best.key, best.count)) best = o;
+    }
+    return best;
+}
+
+// recompute the maxima of the dirty blocks (or of all blocks), one warp per word of the bitmap / per block
+__global__ void refresh_kernel(EngineDev e, int all) {
     const unsigned int lane = threadIdx.x & 31;
-    for (; w < n; w += nwarps) {
-        const unsigned int blk = all ? w : e.dirty_list[w];
-        const Slot *base = e.table + (u64)blk * STBPE_BLK;
-        u64 bk = STBPE_EMPTY;
-        i64 bc = 0;
-#pragma unroll
-        for (int j = 0; j < STBPE_BLK / 32; ++j) {
-            const uint4 raw = *reinterpret_cast<const uint4 *>(base + j * 32 + lane);
-            const u64 k = ((u64)raw.y << 32) | raw.x;
-            const i64 c = (i64)(((u64)raw.w << 32) | raw.z);
-            if (k != STBPE_EMPTY && c > 0 && better(k, c, bk, bc)) {
-                bk = k;
-                bc = c;
-            }
+    const unsigned int w0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    if (all) {
+        for (unsigned int blk = w0; blk < e.n_blocks; blk += nw) {
+            const Slot s = block_max(e, blk, lane);
+            if (lane == 0) e.blockmax[blk] = s;
         }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            const u64 ok = __shfl_down_sync(0xFFFFFFFFu, bk, d);
-            const i64 oc = __shfl_down_sync(0xFFFFFFFFu, bc, d);
-            if (better(ok, oc, bk, bc)) {
-                bk = ok;
-                bc = oc;
-            }
-        }
-        if (lane == 0) {
-            Slot s;
-            s.key = bk;
-            s.count = bc;
-            const Slot was = e.blockmax[blk];
-            e.blockmax[blk] = s;
-            e.dirty_flag[blk] = 0u;
-            const unsigned int sb = blk >> 8;
-            // the super-block is recomputed only if this block's maximum really changed
-            if (!all && (was.key != s.key || was.count != s.count) && atomicExch(&e.dirty2_flag[sb], 1u) == 0u)
-                e.dirty2_list[atomicAdd(&e.st->n_dirty2, 1u)] = sb;
+        for (unsigned int w = blockIdx.x * blockDim.x + threadIdx.x; w < (e.n_blocks + 31) / 32; w += gridDim.x * blockDim.x)
+            e.dirty_bits[w] = 0u;
+        return;
+    }
+    for (unsigned int w = w0; w < (e.n_blocks + 31) / 32; w += nw) {
+        unsigned int bits = __ldcg(&e.dirty_bits[w]);
+        if (!bits) continue;
+        __syncwarp();
+        if (lane == 0) e.dirty_bits[w] = 0u;
+        for (; bits; bits &= bits - 1u) {
+            const unsigned int blk = w * 32 + __ffs(bits) - 1;
+            const Slot s = block_max(e, blk, lane);
+            if (lane == 0) e.blockmax[blk] = s;
         }
     }
 }
 
-__global__ void refresh_kernel(EngineDev e, int all) {
-    dep_release();
-    dep_wait();
-    const unsigned int n = all ? e.n_blocks : min(e.st->n_dirty, e.n_blocks);
-    refresh_blocks(e, all, n, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5);
-}
-
-__device__ __forceinline__ i64 find_slot(const EngineDev &e, u64 key) {
+static __device__ __noinline__ i64 find_slot(const EngineDev &e, u64 key) {
     u64 h = slot_of(e, key);
     for (unsigned int probe = 0; probe < STBPE_MAX_PROBE; ++probe) {
         const u64 k = *(volatile u64 *)&e.table[h].key;
@@ -274,20 +310,151 @@ __device__ __forceinline__ void begin_merge(const EngineDev &e, u64 key, i64 cou
     st->cur_new = new_id;
     st->cur_count = count;
     st->merges_done = mnum + 1;
-    st->n_work = 0;  // the worklist of this merge starts empty (worklist_kernel appends)
+    st->n_work = 0;
     const i64 h = find_slot(e, key);
     if (h >= 0) {
         e.table[h].count = 0;
-        mark_dirty(e, (u64)h);
+        if (e.world > 1) mark_dirty(e, (u64)h);
     } else if (!may_be_absent) {
         atomicOr(&st->error, STBPE_DERR_KEY_MISSING);
+    }
+}
+
+// ---------------------------------------------------------------------------------------
+// Candidate list (one rank).  A new threshold is found by a histogram of the table over 2048 buckets in
+// selection order: first logarithmic in the count (5 bits below the leading one), then, should one bucket
+// hold too many pairs (ties late in a run, very flat histograms), linear inside that bucket, first over its
+// counts and, when a single count is left, over the keys.
+// ---------------------------------------------------------------------------------------
+__device__ __forceinline__ int log_bucket(i64 c) {  // monotone in c >= 1
+    if (c < 64) return (int)c;
+    const int lg = 63 - __clzll(c);
+    return 64 + (lg - 6) * 32 + (int)((c >> (lg - 5)) & 31);
+}
+__device__ __forceinline__ i64 log_bucket_low(int b) {
+    if (b < 64) return b;
+    const int lg = (b - 64) / 32 + 6;
+    return ((i64)(32 + ((b - 64) & 31))) << (lg - 5);
+}
+// width of a linear bucket over [lo, hi]: a power of two that needs at most STBPE_CAND_BUCKETS of them
+__device__ __forceinline__ int linear_shift(u64 lo, u64 hi) {
+    int sh = 0;
+    while (((hi - lo) >> sh) >= STBPE_CAND_BUCKETS) ++sh;
+    return sh;
+}
+
+// a fresh count: no list, and no add is admitted to one
+__global__ void cand_none_kernel(EngineDev e) {
+    e.st->cand_state = STBPE_CAND_NONE;
+    e.st->n_cand = 0;
+    e.st->theta_count = 0x7FFFFFFFFFFFFFFFll;
+    e.st->theta_key = 0;
+    e.st->peek_valid = 0;
+}
+
+// pass over the table; larger bucket = earlier in selection order
+__global__ void __launch_bounds__(512) cand_hist_kernel(EngineDev e) {
+    __shared__ unsigned int s_h[STBPE_CAND_BUCKETS];
+    const DevState *st = e.st;
+    const bool refine = st->cand_state == STBPE_CAND_REFINE;
+    const i64 lo = st->refine_lo, hi = st->refine_hi;
+    const u64 klo = st->refine_klo, khi = st->refine_khi;
+    const bool by_key = refine && lo == hi;
+    const int sh = !refine ? 0 : (by_key ? linear_shift(klo, khi) : linear_shift((u64)lo, (u64)hi));
+    for (int i = threadIdx.x; i < STBPE_CAND_BUCKETS; i += blockDim.x) s_h[i] = 0u;
+    __syncthreads();
+#pragma unroll 4
+    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i <= e.mask; i += (u64)gridDim.x * blockDim.x) {
+        const Slot s = ldcg_slot(e.table + i);
+        if (s.key == STBPE_EMPTY || s.count <= 0) continue;
+        int b;
+        if (!refine) {
+            b = log_bucket(s.count);
+        } else if (by_key) {
+            if (s.count != lo || s.key < klo || s.key > khi) continue;
+            b = (int)((khi - s.key) >> sh);
+        } else {
+            if (s.count < lo || s.count > hi) continue;
+            b = (int)((u64)(s.count - lo) >> sh);
+        }
+        atomicAdd(&s_h[b], 1u);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < STBPE_CAND_BUCKETS; i += blockDim.x)
+        if (s_h[i]) atomicAdd(&e.cand_hist[i], s_h[i]);
+}
+
+// The threshold out of the histogram (which is left zeroed for the next search): buckets are taken from the top
+// while the list stays within STBPE_CAND_MOST; with too few taken and the next one too large, that bucket
+// is searched again (STBPE_CAND_REFINE).
+__global__ void __launch_bounds__(1024) cand_decide_kernel(EngineDev e, u64 key_hi) {
+    __shared__ unsigned int s_h[STBPE_CAND_BUCKETS];
+    DevState *st = e.st;
+    for (int i = threadIdx.x; i < STBPE_CAND_BUCKETS; i += blockDim.x) {
+        s_h[i] = e.cand_hist[i];
+        e.cand_hist[i] = 0u;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    st->n_cand = 0;
+    const bool refine = st->cand_state == STBPE_CAND_REFINE;
+    const i64 lo = st->refine_lo, hi = st->refine_hi;
+    const u64 klo = st->refine_klo, khi = st->refine_khi;
+    const bool by_key = refine && lo == hi;
+    const int sh = !refine ? 0 : (by_key ? linear_shift(klo, khi) : linear_shift((u64)lo, (u64)hi));
+    i64 taken = refine ? st->refine_above : 0;
+    int b = STBPE_CAND_BUCKETS - 1;
+    for (; b >= 0 && taken + (i64)s_h[b] <= STBPE_CAND_MOST; --b) taken += s_h[b];
+    // bucket b does not fit (or b < 0: everything does); the list takes the buckets above it
+    if (b >= 0 && taken < STBPE_CAND_LEAST) {
+        st->cand_state = STBPE_CAND_REFINE;
+        st->refine_above = taken;
+        if (by_key) {
+            st->refine_khi = khi - ((u64)b << sh);
+            const u64 w = (1ull << sh) - 1;
+            st->refine_klo = st->refine_khi - klo < w ? klo : st->refine_khi - w;
+        } else if (refine) {
+            st->refine_lo = lo + (i64)((u64)b << sh);
+            const i64 top = st->refine_lo + (i64)(1ull << sh) - 1;
+            st->refine_hi = top < hi ? top : hi;
+            st->refine_klo = 0;
+            st->refine_khi = key_hi;
+        } else {
+            st->refine_lo = log_bucket_low(b);
+            st->refine_hi = log_bucket_low(b + 1) - 1;
+            st->refine_klo = 0;
+            st->refine_khi = key_hi;
+        }
+        return;
+    }
+    if (by_key) {  // the taken buckets hold the keys up to khi - ((b + 1) << sh)
+        st->theta_count = lo;
+        st->theta_key = khi - ((u64)(b + 1) << sh) + 1;
+    } else {
+        const i64 from = b < 0 && !refine ? 1 : (refine ? lo + (i64)((u64)(b + 1) << sh) : log_bucket_low(b + 1));
+        st->theta_count = from - 1;  // the smallest count taken is `from`
+        st->theta_key = 0;
+    }
+    st->cand_state = STBPE_CAND_READY;
+}
+
+__global__ void __launch_bounds__(512) cand_collect_kernel(EngineDev e) {
+    if (e.st->cand_state != STBPE_CAND_READY) return;
+    Theta t;
+    t.count = e.st->theta_count, t.key = e.st->theta_key;
+#pragma unroll 4
+    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i <= e.mask; i += (u64)gridDim.x * blockDim.x) {
+        const Slot s = ldcg_slot(e.table + i);
+        if (s.key != STBPE_EMPTY && s.count > 0 && t.admits(s.count, s.key)) {
+            const unsigned int j = atomicAdd(&e.st->n_cand, 1u);
+            if (j < STBPE_CAND_CAP) e.cand[j] = (unsigned int)i;
+        }
     }
 }
 
 // stop rules of the loop: bpe_trainer.py:4304-4308 (no pairs), :2491-2494 / :4361-4364 (count < 2)
 __device__ __forceinline__ void advance_or_stop(const EngineDev &e, u64 key, i64 count) {
     DevState *st = e.st;
-    st->n_dirty = 0;
     if (st->error) {
         st->stopped = 1;
         st->stop_reason = 4;
@@ -305,10 +472,41 @@ __device__ __forceinline__ void advance_or_stop(const EngineDev &e, u64 key, i64
     }
 }
 
-// mode 0: peek (result into st->peek_*), 1: advance the loop, 2: write candidate to cand[0..3].
-// all2 != 0: recompute every super-block maximum (after a full rebuild of the block maxima),
-// otherwise only the super-blocks the last refresh marked.  The last CTA to finish reduces the
-// super-block maxima and finalises.
+// Best pair of the candidate list by one CTA: as a peek into the state, or as the loop's next step.
+// peek_valid = 0 when the list has run dry or over: the host then searches a new threshold and asks again.
+__global__ void __launch_bounds__(1024) choose_kernel(EngineDev e, int advance) {
+    __shared__ u64 s_k[32];
+    __shared__ i64 s_c[32];
+    DevState *st = e.st;
+    if (advance && st->stopped) return;
+    const unsigned int n = st->n_cand;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    u64 bk = STBPE_EMPTY;
+    i64 bc = 0;
+    for (unsigned int i = threadIdx.x; i < min(n, STBPE_CAND_CAP); i += blockDim.x) {
+        const Slot x = ldcg_slot(e.table + e.cand[i]);
+        if (x.count > 0 && better(x.key, x.count, bk, bc)) bk = x.key, bc = x.count;
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        const u64 ok = __shfl_down_sync(0xFFFFFFFFu, bk, d);
+        const i64 oc = __shfl_down_sync(0xFFFFFFFFu, bc, d);
+        if (better(ok, oc, bk, bc)) bk = ok, bc = oc;
+    }
+    if (lane == 0) s_k[warp] = bk, s_c[warp] = bc;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < (int)blockDim.x / 32; ++w)
+        if (better(s_k[w], s_c[w], bk, bc)) bk = s_k[w], bc = s_c[w];
+    Theta t;
+    t.count = st->theta_count, t.key = st->theta_key;
+    const bool valid = st->cand_state == STBPE_CAND_READY && n <= STBPE_CAND_CAP && (t.admits(bc, bk) || (bc <= 0 && t.count == 0));
+    st->peek_valid = valid;
+    st->peek_key = bk;
+    st->peek_count = bc;
+    if (advance && valid) advance_or_stop(e, bk, bc);
+}
+
 #define STBPE_SELECT_THREADS 256
 __device__ __forceinline__ void block_best(u64 &bk, i64 &bc, u64 *s_k, i64 *s_c) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -337,87 +535,45 @@ __device__ __forceinline__ void block_best(u64 &bk, i64 &bc, u64 *s_k, i64 *s_c)
 
 #include "peer_kernels.cuh"
 
-// recompute the maximum of super-blocks [w, n) of the second dirty list (or of all): one warp per
-// super-block, 256 block maxima, 8 per lane
-__device__ __forceinline__ void refresh_super_blocks(const EngineDev &e, int all2, unsigned int n2, unsigned int w,
-                                                     unsigned int nwarps) {
-    const unsigned int lane = threadIdx.x & 31;
-    for (unsigned int i = w; i < n2; i += nwarps) {
-        const unsigned int sb = all2 ? i : e.dirty2_list[i];
-        u64 bk = STBPE_EMPTY;
-        i64 bc = 0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const unsigned int blk = sb * 256u + j * 32u + lane;
-            if (blk < e.n_blocks) {
-                const uint4 raw = __ldcg(reinterpret_cast<const uint4 *>(e.blockmax + blk));
-                const u64 k = ((u64)raw.y << 32) | raw.x;
-                const i64 c = (i64)(((u64)raw.w << 32) | raw.z);
-                if (c > 0 && better(k, c, bk, bc)) {
-                    bk = k;
-                    bc = c;
-                }
-            }
-        }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            const u64 ok = __shfl_down_sync(0xFFFFFFFFu, bk, d);
-            const i64 oc = __shfl_down_sync(0xFFFFFFFFu, bc, d);
-            if (better(ok, oc, bk, bc)) {
-                bk = ok;
-                bc = oc;
-            }
-        }
-        if (lane == 0) {
-            Slot s;
-            s.key = bk;
-            s.count = bc;
-            e.supermax[sb] = s;
-            e.dirty2_flag[sb] = 0u;
-        }
-    }
-}
-
+// Best pair over all block maxima: every CTA reduces its share, the last one to finish reduces theirs.
 // mode 0: peek (result into the state); 1: single rank, advance or stop; 2: candidate of this rank
 // into cand; 3: candidate of this rank into every peer mailbox, then wait for the peers' candidates
 // and commit (target = the merge target of the engine)
 __global__ void __launch_bounds__(STBPE_SELECT_THREADS)
-    select_kernel(EngineDev e, int mode, int all2, i64 *cand, int target = 0) {
-    dep_release();
-    dep_wait();
+    select_kernel(EngineDev e, int mode, Slot *partial, i64 *cand, int target = 0) {
     DevState *st = e.st;
-    const int stopped = st->stopped;            // both in one round trip
-    const unsigned int n_dirty2 = st->n_dirty2;
-    if (mode == 1 && stopped) return;
+    if (mode == 1 && st->stopped) return;
     __shared__ u64 s_k[STBPE_SELECT_THREADS / 32];
     __shared__ i64 s_c[STBPE_SELECT_THREADS / 32];
     __shared__ int s_last;
-    const unsigned int n2 = all2 ? e.n_super2 : min(n_dirty2, e.n_super2);
-    refresh_super_blocks(e, all2, n2, blockIdx.x * (STBPE_SELECT_THREADS / 32) + (threadIdx.x >> 5),
-                         gridDim.x * (STBPE_SELECT_THREADS / 32));
-    __syncthreads();
+    u64 bk = STBPE_EMPTY;
+    i64 bc = 0;
+#pragma unroll 4
+    for (unsigned int i = blockIdx.x * STBPE_SELECT_THREADS + threadIdx.x; i < e.n_blocks; i += gridDim.x * STBPE_SELECT_THREADS) {
+        const Slot x = ldcg_slot(e.blockmax + i);
+        if (x.count > 0 && better(x.key, x.count, bk, bc)) bk = x.key, bc = x.count;
+    }
+    block_best(bk, bc, s_k, s_c);
     if (threadIdx.x == 0) {
+        Slot x;
+        x.key = bk;
+        x.count = bc;
+        partial[blockIdx.x] = x;
         __threadfence();
         s_last = (atomicAdd(&st->ticket, 1u) == gridDim.x - 1);
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    u64 bk = STBPE_EMPTY;
-    i64 bc = 0;
-    for (unsigned int i = threadIdx.x; i < e.n_super2; i += STBPE_SELECT_THREADS) {
-        const volatile Slot *p = e.supermax + i;
-        const u64 k = p->key;
-        const i64 c = p->count;
-        if (c > 0 && better(k, c, bk, bc)) {
-            bk = k;
-            bc = c;
-        }
+    bk = STBPE_EMPTY;
+    bc = 0;
+    for (unsigned int i = threadIdx.x; i < gridDim.x; i += STBPE_SELECT_THREADS) {
+        const Slot x = ldcg_slot(partial + i);
+        if (x.count > 0 && better(x.key, x.count, bk, bc)) bk = x.key, bc = x.count;
     }
     block_best(bk, bc, s_k, s_c);
     if (threadIdx.x != 0) return;
     st->ticket = 0;
-    st->n_dirty2 = 0;
     if (mode == 0) {
         st->peek_key = bk;
         st->peek_count = bc;
@@ -435,72 +591,14 @@ __global__ void __launch_bounds__(STBPE_SELECT_THREADS)
 }
 
 // ---------------------------------------------------------------------------------------
-// Tile skipping.  A merge (a,b) changes a tile only if a match head sits in it (the pair (a,b)
-// starts there) or if its first token is the partner of a head that ends the tile before it.  The
-// pair filter records, per tile, which pairs start in it (including the pair formed by its last
-// token and the first token of the next non-empty tile), so
-//     visit tile t  iff  all three filter rows of (a,b) have bit t set.
-// A partner in a tile that is not visited is dropped by the warp that owns the head (fix-up in the
-// merge kernel).  This kernel builds the bitmap of visited tiles and the compact worklist.
+// Tile skipping.  A merge (a,b) changes a tile only if one of its tokens is half of a pair (a,b).  The pair
+// filter records, per tile, the pairs that have a token in it (the pair across a seam is entered for
+// both tiles), so
+//     visit tile t  iff  all three filter rows of (a,b) have bit t set, or t is a wildcard tile.
+// (Re)build from the stream: one CTA handles 32 consecutive tiles, i.e. one word of every row: it
+// collects the bits in shared memory and then writes the group's words with plain stores.
 // ---------------------------------------------------------------------------------------
-// the tiles merge (cur_a, cur_b) must visit: bitmap and compact list; `block` of `n_blocks` thread
-// blocks of blockDim.x threads share the words of the bitmap
-__device__ __forceinline__ void build_worklist(const EngineDev &e, int block, int n_blocks, int cur_a, int cur_b) {
-    DevState *st = e.st;
-    unsigned int r1, r2, r3;
-    filter_rows(((u64)(uint32_t)cur_a << 32) | (u64)(uint32_t)cur_b, r1, r2, r3);
-    const unsigned int *row1 = e.presence + (size_t)r1 * e.presence_words;
-    const unsigned int *row2 = e.presence + (size_t)r2 * e.presence_words;
-    const unsigned int *row3 = e.presence + (size_t)r3 * e.presence_words;
-    const unsigned int *wild = e.presence + (size_t)STBPE_PROWS * e.presence_words;
-    const int n_words = (e.n_tiles + 31) / 32;
-    const int lane = threadIdx.x & 31;
-    for (int w0 = block * blockDim.x; w0 < n_words; w0 += n_blocks * blockDim.x) {
-        const int w = w0 + threadIdx.x;
-        unsigned int c = 0;
-        if (w < n_words) {
-            c = (__ldcg(row1 + w) & __ldcg(row2 + w) & __ldcg(row3 + w)) | __ldcg(wild + w);
-            const int rem = e.n_tiles - w * 32;
-            if (rem < 32) c &= (1u << rem) - 1u;
-            e.cand_bits[w] = c;
-        }
-        // warp-aggregated append of the set bits
-        const int cnt = __popc(c);
-        int incl = cnt;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int n = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-            if (lane >= d) incl += n;
-        }
-        const int total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-        int base = 0;
-        if (lane == 31 && total) base = atomicAdd(&st->n_work, total);
-        base = __shfl_sync(0xFFFFFFFFu, base, 31) + incl - cnt;
-        while (c) {
-            const int bit = __ffs(c) - 1;
-            c &= c - 1;
-            e.worklist[base++] = (unsigned int)(w * 32 + bit);
-        }
-    }
-}
-
-__global__ void __launch_bounds__(1024) worklist_kernel(EngineDev e) {
-    dep_release();
-    dep_wait();
-    DevState *st = e.st;
-    const int stopped = st->stopped, exchange_only = st->exchange_only, filter_valid = st->filter_valid;
-    const int cur_a = st->cur_a, cur_b = st->cur_b;  // all in one round trip
-    if (stopped || exchange_only) return;
-    if (!filter_valid) {  // stale filter: the merge visits every tile
-        if (blockIdx.x == 0 && threadIdx.x == 0) st->n_work = -1;
-        return;
-    }
-    build_worklist(e, blockIdx.x, gridDim.x, cur_a, cur_b);
-}
-
-// (Re)build the pair filter from the stream: after a load and after every re-pack.  One CTA handles
-// 32 consecutive tiles, i.e. one word of every row: it collects the bits in shared memory and then
-// writes the STBPE_PROWS words with plain stores.
+template <typename T>
 __global__ void __launch_bounds__(1024) presence_rebuild_kernel(EngineDev e) {
     extern __shared__ unsigned int s_rows[];  // STBPE_PROWS words
     const int n_groups = (e.n_tiles + 31) / 32;
@@ -510,34 +608,34 @@ __global__ void __launch_bounds__(1024) presence_rebuild_kernel(EngineDev e) {
         __syncthreads();
         const int tile = grp * 32 + warp;  // blockDim.x == 1024: one warp per tile of the group
         if (tile < e.n_tiles) {
-            TileRec r;
-            current_rec(e, tile, 0x7FFFFFFF, r);
-            if (r.len > 0) {
-                const uint32_t *g = e.tiles + (i64)tile * STBPE_TILE;
-                uint32_t nxt0 = STBPE_NONE;  // first live token after the tile
-                for (int t = tile + 1; t < e.n_tiles; ++t) {
-                    TileRec rn;
-                    current_rec(e, t, 0x7FFFFFFF, rn);
-                    if (rn.len > 0) {
-                        nxt0 = rn.head[0];
-                        break;
-                    }
-                }
-                for (int i = lane; i < r.len; i += 32) {
-                    const uint32_t t1 = (i + 1 < r.len) ? g[i + 1] : nxt0;
-                    if (t1 & STBPE_FLAG) continue;  // not a countable pair
-                    unsigned int r1, r2, r3;
-                    filter_rows(((u64)(g[i] & STBPE_IDMASK) << 32) | (u64)t1, r1, r2, r3);
-                    atomicOr(&s_rows[r1], 1u << warp);
-                    atomicOr(&s_rows[r2], 1u << warp);
-                    atomicOr(&s_rows[r3], 1u << warp);
+            auto enter = [&](uint32_t t0, uint32_t t1) {
+                if (t1 & STBPE_FLAG) return;  // not a countable pair
+                unsigned int r1, r2, r3;
+                filter_rows(((u64)(t0 & STBPE_IDMASK) << 32) | (u64)t1, r1, r2, r3);
+                atomicOr(&s_rows[r1], 1u << warp);
+                atomicOr(&s_rows[r2], 1u << warp);
+                atomicOr(&s_rows[r3], 1u << warp);
+            };
+            uint32_t w[Tok<T>::VEC * 4];
+            load_group<T>(e, tile, lane, w);
+            const uint32_t L = live_mask<T>(w);
+            const uint32_t ne = __ballot_sync(0xFFFFFFFFu, L != 0u);
+            if (ne) {
+                for_each_pair<T>(w, L, lane, first_after(e, tile, 0x7FFFFFFF), enter);
+                if (lane == __ffs(ne) - 1) {  // the pair that ends at this tile's first token
+                    uint32_t first = STBPE_NONE;
+#pragma unroll
+                    for (int i = 31; i >= 0; --i)
+                        if ((L >> i) & 1u) first = Tok<T>::get(w, i);
+                    const uint32_t prev = last_before(e, tile, 0x7FFFFFFF);
+                    if (prev != STBPE_NONE) enter(prev, first);
                 }
             }
         }
         __syncthreads();
         for (int i = threadIdx.x; i < STBPE_PROWS; i += blockDim.x)
-            e.presence[(size_t)i * e.presence_words + grp] = s_rows[i];
-        if (threadIdx.x == 0) e.presence[(size_t)STBPE_PROWS * e.presence_words + grp] = 0u;  // no wildcards
+            e.presence[(size_t)grp * STBPE_PPITCH + i] = s_rows[i];
+        if (threadIdx.x == 0) e.presence[(size_t)grp * STBPE_PPITCH + STBPE_PROWS] = 0u;  // no wildcards
         __syncthreads();
     }
 }
@@ -553,19 +651,6 @@ __global__ void count_ties_kernel(EngineDev e) {
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) n += __shfl_down_sync(0xFFFFFFFFu, n, d);
     if ((threadIdx.x & 31) == 0 && n) atomicAdd((u64 *)&e.st->peek_ties, (u64)n);
-}
-
-// host-requested merge (stbpe_apply_merge): same bookkeeping as a selected one
-__global__ void force_merge_kernel(EngineDev e, int a, int b, int new_id) {
-    DevState *st = e.st;
-    st->n_dirty = 0;
-    st->stopped = 0;
-    st->stop_reason = 0;
-    st->n_matches = 0;
-    const u64 key = ((u64)(uint32_t)a << 32) | (u64)(uint32_t)b;
-    const i64 h = find_slot(e, key);
-    const i64 count = h >= 0 ? e.table[h].count : 0;
-    begin_merge(e, key, count, new_id, true);  // merging a pair that never occurs is legal
 }
 
 // ---------------------------------------------------------------------------------------
@@ -595,35 +680,55 @@ __global__ void export_ties_kernel(EngineDev e, i64 count, u64 *keys, i64 cap) {
     }
 }
 
-// tile_off[t] = exclusive prefix of the current tile lengths (computed by the host)
-__global__ void export_stream_kernel(EngineDev e, const i64 *__restrict__ tile_off, int32_t *out) {
-    for (int tile = blockIdx.x; tile < e.n_tiles; tile += gridDim.x) {
-        const int len = (int)(tile_off[tile + 1] - tile_off[tile]);
-        const uint32_t *g = e.tiles + (i64)tile * STBPE_TILE;
-        for (int i = threadIdx.x; i < len; i += blockDim.x) out[tile_off[tile] + i] = (int32_t)g[i];
+// Live tokens of all tiles, in order, into a dense stream (tile_off = exclusive prefix of the live counts):
+//   re-pack : after many merges a stream is full of holes, and every pass over it pays for them; also the step
+//             from a 16-bit to a 32-bit stream (TD wider than TS)
+//   export  : as int32 ids with bit 31 = row start, in stream order
+// One warp per tile: the tile's live tokens are squeezed together in shared memory (rank = live tokens before
+// it, from the lanes' masks), then stored 32 consecutive positions at a time.
+#define STBPE_REPACK_THREADS 256
+template <typename TS, typename TD, bool EXPORT>
+__global__ void __launch_bounds__(STBPE_REPACK_THREADS) repack_copy_kernel(EngineDev e, const i64 *__restrict__ tile_off, TD *__restrict__ dst) {
+    __shared__ TS s_tok[STBPE_REPACK_THREADS / 32][STBPE_TILE];
+    const int warps = blockDim.x >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (i64 tile = (i64)blockIdx.x * warps + warp; tile < e.n_tiles; tile += (i64)gridDim.x * warps) {
+        uint32_t w[Tok<TS>::VEC * 4];
+        load_group<TS>(e, (int)tile, lane, w);
+        const uint32_t L = live_mask<TS>(w);
+        int incl = __popc(L);
+        const int mine = incl;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int n = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+            if (lane >= d) incl += n;
+        }
+        const int len = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        int r = incl - mine;
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+            if ((L >> i) & 1u) s_tok[warp][r++] = (TS)(sizeof(TS) == 2 ? (i < 16 ? w[i] & 0xFFFFu : w[i & 15] >> 16) : w[i % (Tok<TS>::VEC * 4)]);
+        __syncwarp();
+        const i64 o = tile_off[tile];
+        for (int i = lane; i < len; i += 32) {
+            const uint32_t c = Tok<TS>::widen(s_tok[warp][i]);
+            if (EXPORT)
+                dst[o + i] = (TD)c;
+            else
+                dst[Tok<TD>::index(o + i)] = (TD)Tok<TD>::narrow(c);
+        }
     }
 }
 
-// Re-pack: tiles only ever shrink, so after many merges they are sparsely filled and the per-tile
-// cost of the pipeline is spread over few tokens.  The live tokens of all tiles are copied, in
-// order, into a dense stream (tile_off = exclusive prefix of the tile lengths).
-__global__ void repack_copy_kernel(EngineDev e, const i64 *__restrict__ tile_off, uint32_t *__restrict__ dst) {
-    const int warps_per_block = blockDim.x >> 5, lane = threadIdx.x & 31;
-    for (long long tile = (long long)blockIdx.x * warps_per_block + (threadIdx.x >> 5); tile < e.n_tiles;
-         tile += (long long)gridDim.x * warps_per_block) {
-        const i64 o = tile_off[tile];
-        const int len = (int)(tile_off[tile + 1] - o);
-        const uint32_t *g = e.tiles + (i64)tile * STBPE_TILE;
-        for (int i = lane; i < len; i += 32) dst[o + i] = g[i];
-    }
+// a stream that is still being loaded, token by token into the wider format
+__global__ void widen_copy_kernel(const uint16_t *__restrict__ src, uint32_t *__restrict__ dst, i64 n) {
+    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x)
+        dst[i] = Tok<uint16_t>::widen(src[Tok<uint16_t>::index(i)]);
 }
 
 __global__ void tile_lens_kernel(EngineDev e, i64 *lens) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= e.n_tiles) return;
-    TileRec r;
-    current_rec(e, t, 0x7FFFFFFF, r);
-    lens[t] = r.len;
+    if (t < e.n_tiles) lens[t] = (i64)e.tile_live[t];
 }
 
 // ---------------------------------------------------------------------------------------
@@ -697,6 +802,7 @@ __global__ void apply_inbox_kernel(EngineDev e) {
         h.count = 0;
         e.outbox[(i64)threadIdx.x * (e.cap_per_peer + 1)] = h;
     }
+    unsigned int fresh = 0;
     for (int p = 0; p < e.world; ++p) {
         const Slot *chunk = e.inbox + (i64)p * (e.cap_per_peer + 1);
         i64 n = (i64)chunk[0].key;
@@ -706,9 +812,10 @@ __global__ void apply_inbox_kernel(EngineDev e) {
         }
         for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
             const Slot v = chunk[1 + i];
-            table_add(e, v.key, v.count);
+            table_add<NOTE_DIRTY>(e, v.key, v.count, false, fresh);
         }
     }
+    if (fresh) atomicAdd(&e.st->n_keys, (u64)fresh);
 }
 
 // Every rank evaluates the same gathered candidates {key, count, incomplete, -} and reaches the
@@ -732,7 +839,6 @@ __global__ void commit_kernel(EngineDev e, const i64 *all_cands, int target) {
         }
     }
     if (incomplete) {
-        st->n_dirty = 0;
         st->exchange_only = 1;
         return;
     }

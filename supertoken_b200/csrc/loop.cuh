@@ -1,0 +1,261 @@
+// The merge loop of one GPU as one persistent cooperative kernel: one CTA per SM takes every step
+//     choose the best pair -> apply the merge, deltas into the pair table -> refresh the maxima the deltas changed
+// without returning to the host; the launch ends when a stop rule fires or the host has maintenance to do.
+//
+// A late merge changes a few thousand places of a stream of any size, so its cost is the latency of the steps,
+// not bandwidth: as four launches per merge (select, worklist, merge, refresh) inside a replayed graph a step
+// took 31 us on a 1 MiB corpus and 42-58 us late in a 256 MiB one.  Here the CTAs meet once per merge, at a grid
+// barrier when all deltas are in the table: a counter in L2 that every CTA increments (release) and polls
+// (acquire), 1.3 us with nothing outstanding.  (Measured on the same 148 CTAs: one CTA collecting flags and
+// answering 2.0-2.2 us, all CTAs polling all flags 2.9 us; fewer CTAs are no faster.)  Then every CTA
+// re-reads the counts of all candidates, a few hundred slots that are in L2, and takes the same decision from
+// the same values.  (With block maxima in shared memory, refreshed through a bitmap of dirty blocks, and a
+// vote of the CTAs on the best of them, the same step took 4.3 us instead of 1.5.)
+// A second counter keeps the CTAs apart the other way round: a CTA adds its deltas of merge m only when all have
+// read the counts that chose merge m; that wait runs under the rewriting of the tiles.
+// Nothing else is exchanged: the tiles a merge must visit come out of the pair filter inside each CTA.
+//
+// All waits are bounded (STBPE_LOOP_WAIT_NS): a CTA that gives up sets STBPE_DERR_TIMEOUT and leaves, and so do
+// the others, each at its own limit at the latest.  The cooperative launch guarantees that all CTAs are resident.
+#pragma once
+#include "kernels.cuh"
+
+#define STBPE_LOOP_WAIT_NS 4000000000ull
+
+struct LoopArgs {
+    int target;             // merge count to stop at
+    const int2 *forced;     // host-given merges (a, b) applied in order instead of the best pair, or null
+    int n_forced, forced_new;  // forced merge i gets id forced_new + i
+    i64 filter_count;       // leave to build the pair filter when the merge's count has fallen to this
+    int repack_tiles;       // leave for a re-pack at three quarters live from this many tiles on
+    int unit_shift;         // tiles per filter unit, log2 (cta_merge)
+};
+
+__device__ __forceinline__ u64 loop_timer_ns() {
+    u64 t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ void red_release_u32(unsigned int *p, unsigned int v) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int *p) {
+    unsigned int v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+// retries of a bounded wait; false when the time is up or another wait has given up
+struct BoundedWait {
+    u64 t0;
+    unsigned int n;
+    __device__ __forceinline__ BoundedWait() : t0(0), n(0) {}
+    __device__ __forceinline__ bool again(DevState *st) {
+        if ((++n & 1023u) != 0u) return true;
+        const u64 t = loop_timer_ns();
+        if (t0 == 0) t0 = t;
+        if (t - t0 > STBPE_LOOP_WAIT_NS) atomicOr(&st->error, STBPE_DERR_TIMEOUT);
+        return (*(volatile unsigned int *)&st->error & STBPE_DERR_TIMEOUT) == 0u;
+    }
+};
+
+// The arg-max in registers.  With 15-bit ids a pair and its count fit 64 bits whose order is the
+// order of the selection (larger count, then smaller key), and a warp's maximum is two redux steps.
+template <typename T>
+struct Best;
+template <>
+struct Best<uint16_t> {
+    typedef u64 type;
+    static __device__ __forceinline__ u64 none() { return 0ull; }
+    static __device__ __forceinline__ u64 make(u64 key, i64 count) {
+        const u64 k30 = ((key >> 32) << 15) | (key & 0x7FFFull);
+        return count > 0 ? ((u64)count << 30) | (0x3FFFFFFFull - k30) : 0ull;
+    }
+    static __device__ __forceinline__ u64 max2(u64 x, u64 y) { return x > y ? x : y; }
+    static __device__ __forceinline__ u64 warp_max(u64 v) {
+        const uint32_t hi = __reduce_max_sync(0xFFFFFFFFu, (uint32_t)(v >> 32));
+        const uint32_t lo = __reduce_max_sync(0xFFFFFFFFu, (uint32_t)(v >> 32) == hi ? (uint32_t)v : 0u);
+        return ((u64)hi << 32) | lo;
+    }
+    static __device__ __forceinline__ Slot slot(u64 v) {
+        Slot s;
+        s.count = (i64)(v >> 30);
+        const u64 k30 = 0x3FFFFFFFull - (v & 0x3FFFFFFFull);
+        s.key = v ? ((k30 >> 15) << 32) | (k30 & 0x7FFFull) : STBPE_EMPTY;
+        return s;
+    }
+};
+template <>
+struct Best<uint32_t> {
+    typedef Slot type;
+    static __device__ __forceinline__ Slot make(u64 key, i64 count) {
+        Slot s;
+        s.key = count > 0 ? key : STBPE_EMPTY;
+        s.count = count > 0 ? count : 0;
+        return s;
+    }
+    static __device__ __forceinline__ Slot none() { return make(STBPE_EMPTY, 0); }
+    static __device__ __forceinline__ Slot max2(const Slot &x, const Slot &y) { return better(y.key, y.count, x.key, x.count) ? y : x; }
+    static __device__ __forceinline__ Slot warp_max(Slot v) {
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            Slot o;
+            o.key = __shfl_xor_sync(0xFFFFFFFFu, v.key, d);
+            o.count = __shfl_xor_sync(0xFFFFFFFFu, v.count, d);
+            v = max2(v, o);
+        }
+        return v;
+    }
+    static __device__ __forceinline__ Slot slot(const Slot &v) { return v; }
+};
+
+
+template <typename T>
+__global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __grid_constant__ EngineDev e, const __grid_constant__ LoopArgs la) {
+    typedef Best<T> Bs;
+    typedef typename Bs::type Bt;
+    constexpr int THREADS = MergeGeom<T>::THREADS, WARPS = THREADS / 32;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ int s_ctr[CTR_N];
+    __shared__ Bt s_best[2][32];          // the warps' best candidates, alternating between steps
+    __shared__ i64 s_live, s_forced;      // live tokens, count of the next host-given pair
+    __shared__ unsigned int s_err;        // device error bits
+    __shared__ int s_ok;                  // every wait so far succeeded
+    __shared__ int s_work;                // CTA 0: tiles the last merge visited
+    CtaMerge s;
+    unsigned int *s_cand = reinterpret_cast<unsigned int *>(s.carve<T>(smem_raw, s_ctr));  // slots of the candidates
+    s.clear();
+    DevState *st = e.st;
+    LoopSync *sync = e.sync;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned int G = gridDim.x, cta = blockIdx.x;
+    int merges_done = st->merges_done, forced_i = 0;
+    const int base_vocab = st->base_vocab;
+    const bool fv = st->filter_valid != 0;
+    MergeCtx mc;
+    mc.fv = fv;
+    mc.theta.count = st->theta_count, mc.theta.key = st->theta_key;
+    unsigned int n_cand = 0;  // candidates this CTA knows
+    if (tid == 0) s_ok = 1;
+    if (cta == 0 && tid == 32) {
+        s_work = st->n_work;
+        st->n_work = 0;
+        if (la.forced) st->n_matches = 0;
+    }
+
+#pragma unroll 1
+    for (unsigned int step = 0;; ++step) {
+        // ---- choose: the counts of all candidates as the last merge left them
+        {
+            const unsigned int n = __ldcg(&st->n_cand), n_have = min(n, STBPE_CAND_CAP);
+            Bt x = Bs::none();
+#pragma unroll 2
+            for (unsigned int i = tid; i < n_cand; i += THREADS) {
+                const Slot y = ldcg_slot(e.table + s_cand[i]);
+                x = Bs::max2(x, Bs::make(y.key, y.count));
+            }
+#pragma unroll 1
+            for (unsigned int i = n_cand + tid; i < n_have; i += THREADS) {  // appended by the last merge
+                const unsigned int at = __ldcg(e.cand + i);
+                s_cand[i] = at;
+                const Slot y = ldcg_slot(e.table + at);
+                x = Bs::max2(x, Bs::make(y.key, y.count));
+            }
+            n_cand = n_have;
+            x = Bs::warp_max(x);
+            if (lane == 0) s_best[step & 1][warp] = x;
+            if (tid == THREADS - 1) {
+                s_live = (i64)__ldcg((const u64 *)&st->n_live);
+                s_err = __ldcg(&st->error) | (n > STBPE_CAND_CAP ? 0x80000000u : 0u);
+                if (la.forced && forced_i < la.n_forced) {
+                    const i64 at = find_slot(e, ((u64)(uint32_t)la.forced[forced_i].x << 32) | (uint32_t)la.forced[forced_i].y);
+                    s_forced = at >= 0 ? (i64)__ldcg((const u64 *)&e.table[at].count) : 0;
+                }
+                if (cta == 0 && step > 0) {
+                    s_work = fv ? __ldcg(&st->n_work) : -1;
+                    st->n_work = 0;
+                }
+            }
+        }
+        __syncthreads();
+        if (tid == THREADS - 1) red_release_u32(&sync->chosen, 1u);  // the CTA has read everything it decides by
+        // every warp decides by itself
+        bool forced = false;
+        i64 count;
+        {
+            const Slot best = Bs::slot(Bs::warp_max(lane < WARPS ? s_best[step & 1][lane] : Bs::none()));
+            const unsigned int err = s_err;
+            const bool over = (err >> 31) != 0u;
+            const bool dry = over || !(mc.theta.admits(best.count, best.key) || (best.count <= 0 && mc.theta.count == 0));
+            int stop = 0, why = STBPE_EXIT_STOP, go = 0;
+            u64 key = best.key;
+            count = best.count;
+            const bool host = la.forced != nullptr;
+            forced = host && forced_i < la.n_forced;
+            if (forced) {
+                key = ((u64)(uint32_t)la.forced[forced_i].x << 32) | (uint32_t)la.forced[forced_i].y;
+                count = s_forced;
+            }
+            mc.a = (uint32_t)(key >> 32), mc.b = (uint32_t)key;
+            mc.nw = (uint32_t)(host ? la.forced_new + forced_i : base_vocab + merges_done);
+            // stop rules of the loop: bpe_trainer.py:4304-4308 (no pairs), :2491-2494 / :4361-4364 (count < 2)
+            if (err & 0x7FFFFFFFu) stop = 4;
+            else if (host && !forced) stop = 0;
+            else if (!host && merges_done >= la.target) stop = 1;
+            // maintenance the host does between launches
+            else if (!host && dry) why = STBPE_EXIT_REFILL;
+            else if (!host && count <= 0) stop = 2;
+            else if (!host && count < 2) stop = 3;
+            else if (e.n_tiles >= la.repack_tiles && s_live * 4 <= (i64)e.n_tiles * STBPE_TILE * 3) why = STBPE_EXIT_REPACK;
+            else if (!fv && e.n_tiles > 0 && count <= la.filter_count) why = STBPE_EXIT_FILTER;
+            else if (sizeof(T) == 2 && max(mc.nw, max(mc.a, mc.b)) >= Tok<uint16_t>::IDMASK) why = STBPE_EXIT_WIDEN;
+            else go = 1;
+            if (cta == 0 && tid == 0) {
+                if (go) {
+                    e.merges[2 * merges_done] = (int32_t)mc.a;
+                    e.merges[2 * merges_done + 1] = (int32_t)mc.b;
+                    e.merge_counts[merges_done] = count;
+                    e.live_before[merges_done] = s_live;
+                    st->cur_a = (int)mc.a, st->cur_b = (int)mc.b, st->cur_new = (int)mc.nw;
+                    st->cur_count = count;
+                } else {
+                    st->merges_done = merges_done;
+                    st->run_exit = why;
+                    st->stopped = stop > 0;
+                    st->stop_reason = stop;
+                    st->peek_key = best.key;
+                    st->peek_count = best.count;
+                    st->peek_valid = !dry;
+                    st->forced_done = forced_i;
+                    st->n_work = s_work;
+                }
+            }
+            if (!go || !s_ok) return;
+        }
+        // ---- the merge
+        mc.m = ++merges_done;
+        mc.zero = cta == G - 1 ? count : 0;
+        ++forced_i;
+        cta_merge<T, false>(e, s, mc, la.unit_shift, [&] {
+            if (tid == THREADS - 1) {
+                BoundedWait wait;
+                while (ld_acquire_u32(&sync->chosen) < G * (step + 1))
+                    if (!wait.again(st)) {
+                        s_ok = 0;
+                        break;
+                    }
+            }
+        });
+        // ---- grid barrier: every delta is in the table
+        __syncthreads();
+        if (tid == 0) {
+            red_release_u32(&sync->arrived, 1u);
+            BoundedWait wait;
+            while (ld_acquire_u32(&sync->arrived) < G * (step + 1))
+                if (!wait.again(st)) {
+                    s_ok = 0;
+                    break;
+                }
+        }
+        __syncthreads();
+    }
+}

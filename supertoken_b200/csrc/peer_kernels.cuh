@@ -15,7 +15,6 @@
 // guaranteed to make progress as separate launches on one device.
 #pragma once
 #include "common.cuh"
-#include "tile_kernels.cuh"
 
 #define STBPE_PEER_WAIT_NS 2000000000ull  // a peer wait gives up after two seconds
 
@@ -125,6 +124,7 @@ __global__ void apply_peer_kernel(EngineDev e) {
     if ((int)threadIdx.x < e.world && s_ok) s_n[threadIdx.x] = (i64)__ldcg(&mail_chunk(e, e.rank, threadIdx.x)[0].key);
     __syncthreads();
     if (!s_ok) return;
+    unsigned int fresh = 0;
     for (int p = 0; p < e.world; ++p) {
         const Slot *chunk = mail_chunk(e, e.rank, p);
         i64 n = s_n[p];
@@ -134,9 +134,10 @@ __global__ void apply_peer_kernel(EngineDev e) {
         }
         for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
             const ulonglong2 raw = __ldcg(reinterpret_cast<const ulonglong2 *>(chunk + 1 + i));
-            table_add(e, raw.x, (i64)raw.y);
+            table_add<NOTE_DIRTY>(e, raw.x, (i64)raw.y, false, fresh);
         }
     }
+    if (fresh) atomicAdd(&st->n_keys, (u64)fresh);
 }
 
 // This rank's candidate {key, count, incomplete, 0} into every mailbox (called by the one thread
@@ -192,7 +193,6 @@ __device__ __forceinline__ void commit_from_mailbox(const EngineDev &e, int targ
         }
     }
     if (incomplete) {
-        st->n_dirty = 0;
         st->exchange_only = 1;
         return;
     }

@@ -28,7 +28,7 @@
 // An id of 65 536 or more, or a partition region that outgrows its buffer, raises
 // STBPE_DERR_DENSE_OVERFLOW and the host recounts with the general kernel.
 #pragma once
-#include "common.cuh"
+#include "stream.cuh"
 
 #define STBPE_PART_RING 64          // words per partition and CTA between two flushes
 #define STBPE_PART_THREADS 1024
@@ -96,7 +96,6 @@ __device__ __forceinline__ void part_pair(const PartBuffers &pb, unsigned int *s
                                           unsigned int *derr, uint32_t t0, uint32_t t1) {
     // the classes are worked out first and the two kinds of add follow one another, so that the lanes
     // of a warp, whose pairs fall into different classes, share the instructions of each kind
-    t0 &= ~STBPE_FLAG;
     const uint32_t both = t0 | t1;             // bit 31 set: the right token starts a row or lies past the end
     const bool hot = both < 256u;
     const bool wide = !hot && both < 65536u;
@@ -105,8 +104,10 @@ __device__ __forceinline__ void part_pair(const PartBuffers &pb, unsigned int *s
     if (!hot && !wide && !(t1 & STBPE_FLAG)) atomicOr(derr, STBPE_DERR_DENSE_OVERFLOW);
 }
 
+template <typename T>
 __global__ void __launch_bounds__(STBPE_PART_THREADS, 1)
-    partition_pairs_kernel(EngineDev e, i64 n_tokens, u64 *g_dense, PartBuffers pb) {
+    partition_pairs_kernel(EngineDev e, u64 *g_dense, PartBuffers pb) {
+    constexpr int UNROLL = sizeof(T) == 2 ? 2 : STBPE_PART_UNROLL;  // a unit is eight or four tokens
     extern __shared__ __align__(16) unsigned int s_all[];
     unsigned int *s_tab = s_all;                                  // 32 768 words of 16-bit counters
     unsigned int *s_ring = s_all + 32768;                         // STBPE_PARTS rings
@@ -115,43 +116,25 @@ __global__ void __launch_bounds__(STBPE_PART_THREADS, 1)
     for (int i = threadIdx.x; i < 32768; i += STBPE_PART_THREADS) s_tab[i] = 0u;
     for (int i = threadIdx.x; i < STBPE_PARTS; i += STBPE_PART_THREADS) s_cur[i] = s_fill[i] = 0u;
     __syncthreads();
-    const uint32_t *tok = e.tiles;
+    const uint4 *units = reinterpret_cast<const uint4 *>(e.tiles);
+    const i64 n_units = (i64)e.n_tiles * (STBPE_TILE * sizeof(T) / 16);
     unsigned int *derr = &e.st->error;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const i64 span = (i64)STBPE_PART_THREADS * 4;
-    uint4 v[STBPE_PART_UNROLL];
-    uint32_t nx[STBPE_PART_UNROLL];
+    uint4 v[UNROLL];
+    uint32_t nx[UNROLL];
     // the loads of a batch are issued before the flush of the batch before it, so that their trip to
     // memory runs under the flush and its two CTA barriers
-    auto load_batch = [&](i64 base) {
+    const i64 step = (i64)gridDim.x * STBPE_PART_THREADS * UNROLL;
+    i64 base = (i64)blockIdx.x * STBPE_PART_THREADS * UNROLL;
+    if (base < n_units) load_unit_batch<T, UNROLL, STBPE_PART_THREADS>(units, base, n_units, v, nx);
+    for (; base < n_units; base += step) {
 #pragma unroll
-        for (int u = 0; u < STBPE_PART_UNROLL; ++u) {
-            const i64 i = base + u * span + (i64)threadIdx.x * 4;
-            if (i + 4 <= n_tokens) {
-                v[u] = __ldcs(reinterpret_cast<const uint4 *>(tok + i));
-            } else {
-                v[u].x = i < n_tokens ? tok[i] : STBPE_NONE;
-                v[u].y = i + 1 < n_tokens ? tok[i + 1] : STBPE_NONE;
-                v[u].z = i + 2 < n_tokens ? tok[i + 2] : STBPE_NONE;
-                v[u].w = i + 3 < n_tokens ? tok[i + 3] : STBPE_NONE;
-            }
-            nx[u] = (lane == 31) ? (i + 4 < n_tokens ? tok[i + 4] : STBPE_NONE) : 0u;
-        }
-    };
-    const i64 step = (i64)gridDim.x * span * STBPE_PART_UNROLL;
-    i64 base = (i64)blockIdx.x * span * STBPE_PART_UNROLL;
-    if (base < n_tokens) load_batch(base);
-    for (; base < n_tokens; base += step) {
-#pragma unroll
-        for (int u = 0; u < STBPE_PART_UNROLL; ++u) {
-            uint32_t n0 = __shfl_down_sync(0xFFFFFFFFu, v[u].x, 1);
-            if (lane == 31) n0 = nx[u];
-            part_pair(pb, s_tab, s_ring, s_cur, s_fill, g_dense, derr, v[u].x, v[u].y);
-            part_pair(pb, s_tab, s_ring, s_cur, s_fill, g_dense, derr, v[u].y, v[u].z);
-            part_pair(pb, s_tab, s_ring, s_cur, s_fill, g_dense, derr, v[u].z, v[u].w);
-            part_pair(pb, s_tab, s_ring, s_cur, s_fill, g_dense, derr, v[u].w, n0);
-        }
-        if (base + step < n_tokens) load_batch(base + step);
+        for (int u = 0; u < UNROLL; ++u)
+            unit_pairs<T>(v[u], nx[u], [&](uint32_t t0, uint32_t t1) {
+                if (sizeof(T) == 2) t1 = (t1 & 0x7FFFu) | ((t1 & 0x8000u) << 16);
+                part_pair(pb, s_tab, s_ring, s_cur, s_fill, g_dense, derr, t0 & Tok<T>::IDMASK, t1);
+            });
+        if (base + step < n_units) load_unit_batch<T, UNROLL, STBPE_PART_THREADS>(units, base + step, n_units, v, nx);
         __syncthreads();
         // flush into this CTA's regions: a warp serves its eight rings at once, four lanes per ring
         // (one ring at a time cost eight times the bookkeeping: the pass was bound by instruction
@@ -216,7 +199,7 @@ __device__ __forceinline__ bool table_count_n(const EngineDev &e, u64 key, u64 h
 __device__ __forceinline__ void part_word_to_table(const EngineDev &e, uint32_t x, u64 n, unsigned int &fresh, u64 top) {
     const uint32_t ab = unmix32(x);
     const u64 key = ((u64)(ab >> 16) << 32) | (u64)(ab & 0xFFFFu);
-    const u64 h = top | (mix64(key) >> (64 - e.slot_bits));
+    const u64 h = slot_in_slice(e, top, key);
     table_count_n(e, key, h, n, fresh);
 }
 
@@ -344,5 +327,5 @@ __global__ void dense_peers_to_table_kernel(EngineDev e, WidePeers wp, int n_cta
     if (owner_of(key, wp.world) != wp.rank) return;
     u64 c = 0;
     for (int r = 0; r < wp.world; ++r) c += __ldcg(wide_dense(wp.block[r], n_cta) + k);
-    if (c) table_add(e, key, (i64)c);
+    if (c) sink_add<false>(e, key, (i64)c);
 }
