@@ -378,7 +378,7 @@ class GPUBPETrainer(BaseTrainer):
                         self._readbacks.append({"merge": len(self.merges) + len(got) - 1, "merges": len(got),
                                                 "bytes_d2h": len(got) * 24})
                     self.merges.extend(got)
-                    self.merge_counts.extend(int(c) for c in counts)
+                    self.merge_counts.extend(counts.tolist())
                     self.vocab_size = self.base_vocab + len(self.merges)
                     remaining = self.target_merges - len(self.merges)
                     reason = st.stop_reason
@@ -521,7 +521,7 @@ class GPUBPETrainer(BaseTrainer):
             loop_s = time.perf_counter() - t
             got, counts, _ = engines[0].merges(0, done)
             self.merges = list(got)
-            self.merge_counts = [int(c) for c in counts]
+            self.merge_counts = counts.tolist()
             self.vocab_size = self.base_vocab + len(self.merges)
             st = engines[0].state()
             if mode == "ranks":

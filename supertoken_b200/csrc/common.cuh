@@ -73,7 +73,9 @@ struct DevState {
     int stop_reason;
     int run_exit;              // why the last loop_kernel launch returned (STBPE_EXIT_*)
     unsigned int error;
+    unsigned int max_id;       // largest id packed
     unsigned int ticket;
+    int pad0;
     u64 n_keys;
     i64 n_live;
     i64 n_matches;
@@ -105,6 +107,7 @@ struct DevState {
 #define STBPE_EXIT_FILTER 2    // the pair filter starts to pay: build it
 #define STBPE_EXIT_WIDEN 3     // the next id does not fit 15 bits
 #define STBPE_EXIT_REFILL 4    // the candidate list has run dry or over
+#define STBPE_EXIT_GROW 5      // the pair table fills up
 #define STBPE_CAND_NONE 0      // no candidate list (fresh count)
 #define STBPE_CAND_READY 1
 #define STBPE_CAND_REFINE 2    // the threshold search needs another pass
@@ -160,7 +163,6 @@ struct EngineDev {
     // merge visits because the pair that starts at their last token is not known exactly (their
     // last token is the result of a run of equal tokens that ran on into the next tile).
     unsigned int *presence;
-    unsigned int presence_groups;  // groups of 32 tiles there is room for
     DevState *st;
     LoopSync *sync;
     int32_t *merges;

@@ -12,8 +12,16 @@
 #include <vector>
 
 #include "../../include/stbpe.h"
+#include "host_copy.h"
 #include "kernels.cuh"
 #include "loop.cuh"
+
+#include <mutex>
+#include <utility>
+
+#define STBPE_PINNED_BYTES ((size_t)4 << 20)
+#define STBPE_PINNED_STATE 4096  // bytes in front that the device state travels through
+#define STBPE_COUNT_SMEM (STBPE_COUNT_SLOTS * 12)
 
 #define STBPE_VISIBLE __attribute__((visibility("default")))
 
@@ -52,6 +60,7 @@ struct stbpe_engine {
     unsigned char *mail_own;               // this rank's mailbox (peer-memory rounds)
     void *mail_mapped[STBPE_MAX_PEERS];    // peers' mailboxes as mapped into this process
     bool peers_open;
+    bool count_timed;     // ev0 / ev1 span the histogram kernels of the last count; not yet read into count_ms
     float count_ms;       // device time of the histogram kernels of the last count
     float convert_ms;     // device time of moving a dense histogram into the pair table (wide path)
     cudaEvent_t ev0, ev1;
@@ -63,16 +72,36 @@ struct stbpe_engine {
     int repacks_since_load;
     cudaGraphExec_t graph;  // a batch of peer-memory rounds (several ranks)
     int graph_tiles_n;
-    void *graph_tiles;
+    void *graph_tiles, *graph_filter;
     bool graph_wide;
     bool use_graph;
     int part_group;       // partitions per launch of the second pass of the partitioned count
     std::string err;
-    std::vector<void *> allocs;
+    std::vector<stbpe::Block> allocs;
+    bool broken;          // a CUDA call failed: work of this engine may still be pending
+    stbpe::Block pinned;  // host side of small transfers: the device state, then small inputs
+    unsigned int max_id;  // largest id appended through stbpe_append_ids
+    unsigned int load_err;  // error bits of the rows appended so far
+    bool state_stale;     // the device state is that of a stream that has been dropped
+    bool table_auto;      // the table is sized by the stream and grows with the keys
+    u64 table_cap;        // slots the allocated table has room for
+    size_t presence_cap;  // groups of 32 tiles the pair filter has room for
+    void *off_dev;        // row offsets of an append
+    size_t off_cap;
 };
 
+// what differs between GPUs, asked once per device
+struct DeviceInfo {
+    int sm_count = 0;
+    cudaError_t err = cudaSuccess;
+    const char *what = "";
+};
+extern "C" {
+static const DeviceInfo &device_info(int dev);
+}
+
 static thread_local std::string g_create_err;
-namespace { struct NcclApi; NcclApi &nccl_api(); void nccl_comm_destroy(void *comm); }
+namespace { struct NcclApi; NcclApi &nccl_api(); }
 
 static int fail(stbpe_engine *e, int code, const std::string &msg) {
     if (e)
@@ -86,6 +115,7 @@ static int cuda_fail(stbpe_engine *e, cudaError_t c, const char *what) {
     std::string m = std::string(what) + ": " + cudaGetErrorString(c);
     if (c == cudaErrorMemoryAllocation) m = "CUDA out of memory (" + m + ")";
     cudaGetLastError();
+    if (e) e->broken = true;
     return fail(e, STBPE_E_CUDA, m);
 }
 
@@ -95,41 +125,67 @@ static int cuda_fail(stbpe_engine *e, cudaError_t c, const char *what) {
         if (c_ != cudaSuccess) return cuda_fail(e, c_, #call);    \
     } while (0)
 
+// Memory of an engine.  One-rank engines share the block cache; the buffers of several ranks are mapped by other
+// processes (CUDA IPC) and stay plain allocations.
 template <typename T>
 static cudaError_t dev_alloc(stbpe_engine *e, T **p, size_t count) {
-    void *q = nullptr;
-    cudaError_t c = cudaMalloc(&q, count * sizeof(T) > 0 ? count * sizeof(T) : 16);
+    stbpe::Block b;
+    const size_t bytes = count * sizeof(T) > 0 ? count * sizeof(T) : 16;
+    cudaError_t c = cudaSuccess;
+    if (e->cfg.world_size > 1) {
+        c = cudaMalloc(&b.p, bytes);
+        b.size = bytes;
+    } else {
+        c = stbpe::device_blocks().get(e->cfg.device, bytes, &b);
+    }
     if (c == cudaSuccess) {
-        e->allocs.push_back(q);
-        *p = reinterpret_cast<T *>(q);
+        e->allocs.push_back(b);
+        *p = reinterpret_cast<T *>(b.p);
     }
     return c;
 }
 
+static void give_back(stbpe_engine *e, const stbpe::Block &b) {
+    if (e->cfg.world_size > 1 || e->broken)
+        cudaFree(b.p);
+    else
+        stbpe::device_blocks().put(e->cfg.device, b);
+}
+
+// no work that uses the memory may be pending
 static void dev_free(stbpe_engine *e, void *p) {
     if (!p) return;
     for (auto &q : e->allocs)
-        if (q == p) {
-            cudaFree(p);
+        if (q.p == p) {
+            give_back(e, q);
             q = e->allocs.back();
             e->allocs.pop_back();
             return;
         }
 }
 
+// pieces of one allocation
+struct Arena {
+    std::vector<std::pair<void **, size_t>> parts;
+    size_t total = 0;
+    template <typename T>
+    void add(T **p, size_t count) {
+        parts.push_back({reinterpret_cast<void **>(p), total});
+        total += (count * sizeof(T) + 255) & ~(size_t)255;
+    }
+    cudaError_t alloc(stbpe_engine *e) {
+        unsigned char *base = nullptr;
+        const cudaError_t c = dev_alloc(e, &base, total);
+        if (c == cudaSuccess)
+            for (auto &q : parts) *q.first = base + q.second;
+        return c;
+    }
+};
+
 static u64 next_pow2(u64 x) {
     u64 p = 1;
     while (p < x) p <<= 1;
     return p;
-}
-
-static bool is_device_pointer(const void *p) {
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
 // Calls f(uint16_t{}) or f(uint32_t{}) for the engine's stream.
@@ -178,17 +234,86 @@ STBPE_VISIBLE int stbpe_destroy(stbpe_engine *e) {
     // the NCCL communicator is shared by the engines of this process and lives until exit
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->ev1) cudaEventDestroy(e->ev1);
-    for (void *p : e->allocs) cudaFree(p);
+    // every entry point of a one-rank engine ends synchronised, so nothing is pending unless a call failed
+    if (e->broken) cudaDeviceSynchronize();
+    for (const stbpe::Block &b : e->allocs) give_back(e, b);
+    stbpe::pinned_blocks().put(0, e->pinned);
     delete e;
     return STBPE_OK;
 }
 
-static int reset_state(stbpe_engine *e, cudaStream_t s) {
-    DevState h;
-    memset(&h, 0, sizeof(h));
-    h.base_vocab = e->cfg.base_vocab;
-    CK(cudaMemcpyAsync(e->d.st, &h, sizeof(h), cudaMemcpyHostToDevice, s));
+static const DeviceInfo &device_info(int dev) {
+    static std::mutex mu;
+    static DeviceInfo infos[64];
+    static bool known[64] = {};
+    const int k = dev >= 0 && dev < 64 ? dev : 0;
+    std::lock_guard<std::mutex> lock(mu);
+    DeviceInfo &i = infos[k];
+    if (known[k] && i.err == cudaSuccess) return i;
+    known[k] = true;
+    int optin = 0;
+    i.what = "cudaDeviceGetAttribute";
+    i.err = cudaDeviceGetAttribute(&i.sm_count, cudaDevAttrMultiProcessorCount, dev);
+    if (i.err == cudaSuccess) i.err = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (i.err != cudaSuccess) return i;
+    // kernels that use more shared memory than the default limit
+    i.what = "cudaFuncSetAttribute";
+#define SMEM(kern, bytes) \
+    if (i.err == cudaSuccess) i.err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes))
+    SMEM((merge_kernel<uint16_t, false>), MergeGeom<uint16_t>::BYTES);
+    SMEM((merge_kernel<uint16_t, true>), MergeGeom<uint16_t>::BYTES);
+    SMEM((merge_kernel<uint32_t, false>), MergeGeom<uint32_t>::BYTES);
+    SMEM((merge_kernel<uint32_t, true>), MergeGeom<uint32_t>::BYTES);
+    SMEM(loop_kernel<uint16_t>, optin - 4096);
+    SMEM(loop_kernel<uint32_t>, optin - 4096);
+    SMEM((count_kernel<uint16_t, false>), STBPE_COUNT_SMEM);
+    SMEM((count_kernel<uint16_t, true>), STBPE_COUNT_SMEM);
+    SMEM((count_kernel<uint32_t, false>), STBPE_COUNT_SMEM);
+    SMEM((count_kernel<uint32_t, true>), STBPE_COUNT_SMEM);
+    SMEM(count_dense_kernel<uint16_t>, 32768 * 4);
+    SMEM(count_dense_kernel<uint32_t>, 32768 * 4);
+    SMEM(partition_pairs_kernel<uint16_t>, STBPE_PART_SMEM_BYTES);
+    SMEM(partition_pairs_kernel<uint32_t>, STBPE_PART_SMEM_BYTES);
+    SMEM(presence_rebuild_kernel<uint16_t>, STBPE_PROWS * sizeof(unsigned int));
+    SMEM(presence_rebuild_kernel<uint32_t>, STBPE_PROWS * sizeof(unsigned int));
+#undef SMEM
+    return i;
+}
+
+// Slots of a table that is sized by the caller's stream of ids: keys are never removed, so it must hold every
+// pair a run ever creates; 2^27 slots carried 32 000 merges on 2^30 tokens, streams of 2^32 tokens and more get
+// 2^29 (8 GiB).
+static u64 auto_slots(i64 max_tokens) {
+    const u64 cap = max_tokens >= (1ll << 32) ? (1ull << 29) : (1ull << 27);
+    u64 slots = (u64)max_tokens / 4;
+    if (slots < (1ull << 20)) slots = 1ull << 20;
+    return slots < cap ? slots : cap;
+}
+
+static void set_slots(stbpe_engine *e, u64 want) {
+    const u64 slots = next_pow2(want < (u64)2 * STBPE_PARTS ? (u64)2 * STBPE_PARTS : want);
+    e->slots = slots;
+    e->d.mask = slots - 1;
+    // table slices: one per partition this rank can own (partitions with its residue modulo the
+    // number of ranks), rounded up to a power of two
+    const u64 slices = next_pow2(((u64)STBPE_PARTS + e->cfg.world_size - 1) / e->cfg.world_size);
+    e->d.slot_bits = 0;
+    while ((slices << e->d.slot_bits) < slots) ++e->d.slot_bits;
+    // blocks of the arg-max over several ranks: at most 2^19
+    e->d.blk_shift = 6;
+    while ((slots >> e->d.blk_shift) > (1u << 19)) ++e->d.blk_shift;
+    e->d.n_blocks = (unsigned int)(slots >> e->d.blk_shift);
+}
+
+// The device state by way of pinned memory.  Synchronises the stream.
+static int read_state(stbpe_engine *e, DevState *h, cudaStream_t s) {
+    CK(cudaMemcpyAsync(e->pinned.p, e->d.st, sizeof(DevState), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    memcpy(h, e->pinned.p, sizeof(DevState));
+    return STBPE_OK;
+}
+
+static void drop_stream(stbpe_engine *e) {
     e->n_tokens = 0;
     e->d.n_tiles = 0;
     e->recs_stale = true;
@@ -196,6 +321,16 @@ static int reset_state(stbpe_engine *e, cudaStream_t s) {
     e->only_bytes = true;
     e->filter_valid = false;
     e->wide_counted = e->full_refresh_pending = false;
+    e->load_err = e->max_id = 0;
+    e->state_stale = true;
+}
+
+// the device state of an empty stream, before the first work on it
+static int fresh_state(stbpe_engine *e, cudaStream_t s) {
+    if (!e->state_stale) return STBPE_OK;
+    init_state_kernel<<<1, 1, 0, s>>>(e->d, e->cfg.base_vocab, 0);
+    CK(cudaGetLastError());
+    e->state_stale = false;
     return STBPE_OK;
 }
 
@@ -222,86 +357,61 @@ STBPE_VISIBLE int stbpe_create(stbpe_engine **out, const stbpe_config *cfg) {
     };
     cudaError_t c = cudaSetDevice(cfg->device);
     if (c != cudaSuccess) return bail(cuda_fail(e, c, "cudaSetDevice"));
-    cudaDeviceProp prop;
-    c = cudaGetDeviceProperties(&prop, cfg->device);
-    if (c != cudaSuccess) return bail(cuda_fail(e, c, "cudaGetDeviceProperties"));
-    e->sm_count = prop.multiProcessorCount;
+    const DeviceInfo &info = device_info(cfg->device);
+    if (info.err != cudaSuccess) return bail(cuda_fail(e, info.err, info.what));
+    e->sm_count = info.sm_count;
 
     e->max_tokens = cfg->max_tokens;
     e->max_tiles = (int)((cfg->max_tokens + STBPE_TILE - 1) / STBPE_TILE);
     if (e->max_tiles < 1) e->max_tiles = 1;
-    u64 slots = cfg->table_slots > 0 ? (u64)cfg->table_slots : (u64)cfg->max_tokens / 4;
-    if (cfg->table_slots <= 0) {
-        // keys are never removed, so the table must hold every pair a run ever creates: 2^27 slots
-        // carried 32 000 merges on 2^30 tokens; streams of 2^32 tokens and more get 2^29 (8 GiB)
-        const u64 cap = cfg->max_tokens >= (1ll << 32) ? (1ull << 29) : (1ull << 27);
-        if (slots < (1ull << 20)) slots = 1ull << 20;
-        if (slots > cap) slots = cap;
-    }
-    slots = next_pow2(slots < (u64)2 * STBPE_PARTS ? (u64)2 * STBPE_PARTS : slots);
-    e->slots = slots;
-    e->d.mask = slots - 1;
-    // table slices: one per partition this rank can own (partitions with its residue modulo the
-    // number of ranks), rounded up to a power of two
-    u64 slices = next_pow2(((u64)STBPE_PARTS + cfg->world_size - 1) / cfg->world_size);
-    e->d.slot_bits = 0;
-    while ((slices << e->d.slot_bits) < slots) ++e->d.slot_bits;
-    // blocks of the arg-max over several ranks: at most 2^19
-    e->d.blk_shift = 6;
-    while ((slots >> e->d.blk_shift) > (1u << 19)) ++e->d.blk_shift;
-    e->d.n_blocks = (unsigned int)(slots >> e->d.blk_shift);
     e->d.world = cfg->world_size;
     e->d.rank = cfg->rank;
+    e->wide = starts_wide(*cfg);
+    e->table_auto = cfg->table_slots <= 0 && cfg->world_size == 1;
+    set_slots(e, cfg->table_slots > 0 ? (u64)cfg->table_slots : auto_slots(cfg->max_tokens));
 
 #define ALLOC(ptr, n)                                                  \
     if ((c = dev_alloc(e, &(ptr), (size_t)(n))) != cudaSuccess) return bail(cuda_fail(e, c, "cudaMalloc " #ptr))
-    e->wide = starts_wide(*cfg);
     {
         unsigned char *t = nullptr;
         e->tiles_bytes = (size_t)e->max_tiles * STBPE_TILE * tok_bytes(e);
         ALLOC(t, e->tiles_bytes);
         e->d.tiles = t;
     }
-    ALLOC(e->d.recs, (size_t)e->max_tiles * 2);
-    ALLOC(e->d.tile_live, (size_t)e->max_tiles);
-    ALLOC(e->d.table, slots);
-    if (cfg->world_size > 1) {
-        ALLOC(e->d.blockmax, e->d.n_blocks);
-        ALLOC(e->d.dirty_bits, (e->d.n_blocks + 31) / 32);
-        ALLOC(e->partial, 4096);
-    } else {
-        ALLOC(e->d.cand, STBPE_CAND_CAP);
-        ALLOC(e->d.cand_hist, STBPE_CAND_BUCKETS);
-    }
-    ALLOC(e->d.st, 1);
-    ALLOC(e->d.sync, 1);
-    ALLOC(e->d.merges, (size_t)2 * (cfg->max_merges + 1));
-    ALLOC(e->d.merge_counts, (size_t)cfg->max_merges + 1);
-    ALLOC(e->d.live_before, (size_t)cfg->max_merges + 1);
-    ALLOC(e->dense, 65536);
-    ALLOC(e->cand, 4);
-    ALLOC(e->all_cands, (size_t)4 * cfg->world_size);
-    e->d.presence_groups = (unsigned int)(((size_t)e->max_tiles + 31) / 32);
-    ALLOC(e->d.presence, (size_t)STBPE_PPITCH * e->d.presence_groups);
-    // the re-pack allocates nothing inside the merge loop: its scratch is sized here for the largest
-    // stream, and the second stream buffer too unless it would take more than half of what is free
-    ALLOC(e->rp_lens, (size_t)e->max_tiles + 1);
-    ALLOC(e->rp_offs, (size_t)e->max_tiles + 1);
-    cub::DeviceScan::ExclusiveSum(nullptr, e->rp_tmp_bytes, e->rp_lens, e->rp_offs, e->max_tiles + 1, 0);
     {
-        unsigned char *t = nullptr;
-        ALLOC(t, e->rp_tmp_bytes ? e->rp_tmp_bytes : 16);
-        e->rp_tmp = t;
-    }
-    {
-        size_t free_b = 0, total_b = 0;
-        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && e->tiles_bytes <= free_b / 2) {
-            unsigned char *t = nullptr;
-            ALLOC(t, e->tiles_bytes);
-            e->tiles_alt = t;
-            e->alt_bytes = e->tiles_bytes;
+        // everything small in one allocation; the pair table, the second stream buffer and the pair filter follow
+        // when they are needed, in the size that is needed then
+        Arena a;
+        a.add(&e->d.recs, (size_t)e->max_tiles * 2);
+        a.add(&e->d.tile_live, (size_t)e->max_tiles);
+        a.add(&e->rp_lens, (size_t)e->max_tiles + 1);
+        a.add(&e->rp_offs, (size_t)e->max_tiles + 1);
+        cub::DeviceScan::ExclusiveSum(nullptr, e->rp_tmp_bytes, e->rp_lens, e->rp_offs, e->max_tiles + 1, 0);
+        a.add((unsigned char **)&e->rp_tmp, e->rp_tmp_bytes ? e->rp_tmp_bytes : 16);
+        a.add(&e->d.st, 1);
+        a.add(&e->d.sync, 1);
+        a.add(&e->d.merges, (size_t)2 * (cfg->max_merges + 1));
+        a.add(&e->d.merge_counts, (size_t)cfg->max_merges + 1);
+        a.add(&e->d.live_before, (size_t)cfg->max_merges + 1);
+        a.add(&e->dense, 65536);
+        a.add(&e->cand, 4);
+        a.add(&e->all_cands, (size_t)4 * cfg->world_size);
+        if (cfg->world_size > 1) {
+            a.add(&e->d.blockmax, e->d.n_blocks);
+            a.add(&e->d.dirty_bits, (e->d.n_blocks + 31) / 32);
+            a.add(&e->partial, 4096);
+        } else {
+            a.add(&e->d.cand, STBPE_CAND_CAP);
+            a.add(&e->d.cand_hist, STBPE_CAND_BUCKETS);
         }
+        if ((c = a.alloc(e)) != cudaSuccess) return bail(cuda_fail(e, c, "cudaMalloc engine state"));
     }
+    if (!e->table_auto) {
+        ALLOC(e->d.table, e->slots);
+        e->table_cap = e->slots;
+    }
+    c = stbpe::pinned_blocks().get(0, STBPE_PINNED_BYTES, &e->pinned);
+    if (c != cudaSuccess) return bail(cuda_fail(e, c, "cudaMallocHost"));
     if (cfg->world_size > 1) {
         e->lslots = 1ull << 22;
         e->d.lmask = e->lslots - 1;
@@ -323,40 +433,18 @@ STBPE_VISIBLE int stbpe_create(stbpe_engine **out, const stbpe_config *cfg) {
                         : cudaMemset(e->d.cand_hist, 0, STBPE_CAND_BUCKETS * sizeof(unsigned int));
     if (c != cudaSuccess) return bail(cuda_fail(e, c, "cudaMemset"));
 
-    // kernels that use more shared memory than the default limit
-    e->count_smem = (size_t)STBPE_COUNT_SLOTS * 12;
-#define SMEM(kern, bytes)                                                                                      \
-    if ((c = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes))) != cudaSuccess) \
-    return bail(cuda_fail(e, c, "cudaFuncSetAttribute"))
-    SMEM((merge_kernel<uint16_t, false>), MergeGeom<uint16_t>::BYTES);
-    SMEM((merge_kernel<uint16_t, true>), MergeGeom<uint16_t>::BYTES);
-    SMEM((merge_kernel<uint32_t, false>), MergeGeom<uint32_t>::BYTES);
-    SMEM((merge_kernel<uint32_t, true>), MergeGeom<uint32_t>::BYTES);
-    SMEM(loop_kernel<uint16_t>, prop.sharedMemPerBlockOptin - 4096);
-    SMEM(loop_kernel<uint32_t>, prop.sharedMemPerBlockOptin - 4096);
-    SMEM((count_kernel<uint16_t, false>), e->count_smem);
-    SMEM((count_kernel<uint16_t, true>), e->count_smem);
-    SMEM((count_kernel<uint32_t, false>), e->count_smem);
-    SMEM((count_kernel<uint32_t, true>), e->count_smem);
-    SMEM(count_dense_kernel<uint16_t>, 32768 * 4);
-    SMEM(count_dense_kernel<uint32_t>, 32768 * 4);
-    SMEM(partition_pairs_kernel<uint16_t>, STBPE_PART_SMEM_BYTES);
-    SMEM(partition_pairs_kernel<uint32_t>, STBPE_PART_SMEM_BYTES);
-    SMEM(presence_rebuild_kernel<uint16_t>, STBPE_PROWS * sizeof(unsigned int));
-    SMEM(presence_rebuild_kernel<uint32_t>, STBPE_PROWS * sizeof(unsigned int));
-#undef SMEM
+    e->count_smem = STBPE_COUNT_SMEM;
     e->select_grid = e->sm_count;
     e->refresh_grid = e->sm_count * 4;
-    int rc = reset_state(e, 0);
-    if (rc != STBPE_OK) return bail(rc);
+    drop_stream(e);
     *out = e;
     return STBPE_OK;
 }
 
 STBPE_VISIBLE int stbpe_reset(stbpe_engine *e) {
     if (!e) return STBPE_E_BADARG;
-    CK(cudaSetDevice(e->cfg.device));
-    return reset_state(e, 0);
+    drop_stream(e);
+    return STBPE_OK;
 }
 
 static int widen_stream(stbpe_engine *e, cudaStream_t s);
@@ -372,12 +460,32 @@ static int append_common(stbpe_engine *e, const void *data, i64 n, size_t elem, 
         // the stream has been counted: appending is still fine while no merge has rewritten a tile
         // (the tiles are dense and n_tokens is their true length), not afterwards
         DevState h;
-        CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
+        if (int rc_ = read_state(e, &h, s)) return rc_;
         if (h.merges_done > 0 || e->repacks_since_load > 0)
             return fail(e, STBPE_E_STATE, "rows cannot be appended after a merge has been applied; call stbpe_reset first");
     }
-    if (e->n_tokens == 0) e->wide = starts_wide(e->cfg);  // a fresh stream
+    const i64 single[2] = {0, n};
+    const i64 *off = row_offsets ? row_offsets : single;
+    const i64 rows = row_offsets ? n_rows : 1;
+    if (off[0] != 0 || off[rows] != n) return fail(e, STBPE_E_BADARG, "row_offsets must start at 0 and end at n");
+    if (int rc = fresh_state(e, s)) return rc;
+    if (e->n_tokens == 0) {  // a fresh stream, into a buffer that takes all it may become (a re-pack may have left a smaller one)
+        e->wide = starts_wide(e->cfg);
+        const size_t full = (size_t)e->max_tiles * STBPE_TILE * tok_bytes(e);
+        if (e->tiles_bytes < full && e->alt_bytes >= full) {
+            std::swap(e->d.tiles, e->tiles_alt);
+            std::swap(e->tiles_bytes, e->alt_bytes);
+        }
+        if (e->tiles_bytes < full) {
+            dev_free(e, e->d.tiles);
+            e->d.tiles = nullptr;
+            e->tiles_bytes = 0;
+            unsigned char *t = nullptr;
+            CK(dev_alloc(e, &t, full));
+            e->d.tiles = t;
+            e->tiles_bytes = full;
+        }
+    }
     const i64 at0 = e->n_tokens;
     unsigned int *bad = &e->d.st->error;
     auto pack = [&](const void *src, i64 cnt, i64 at) {
@@ -393,94 +501,74 @@ static int append_common(stbpe_engine *e, const void *data, i64 n, size_t elem, 
                 pack_ids_kernel<T><<<(unsigned int)blocks, 256, 0, s>>>((const int32_t *)src, cnt, e->d.tiles, at, bad);
             }
         });
+        return cudaGetLastError();
     };
-    void *staged = nullptr;
-    if (is_device_pointer(data)) {
-        pack(data, n, at0);
-    } else {
-        // host data is staged on the device before the pack kernel reads it: in the second stream
-        // buffer when the engine has one (it is idle until the first re-pack, and an allocation of this
-        // size costs as much as the copy), else in stream-ordered scratch
-        char *stage = (char *)e->tiles_alt;
-        if (!stage || (size_t)n * elem > e->alt_bytes) {
-            CK(cudaMallocAsync(&staged, (size_t)n * elem, s));
-            stage = (char *)staged;
-        }
-        // the copy goes in pieces on a stream of its own, and every piece is packed on the caller's
-        // stream as soon as it has landed, so the pack kernel runs under the following copies
-        const i64 piece = (i64)((size_t)(64 << 20) / elem);
-        if (n <= piece) {
-            CK(cudaMemcpyAsync(stage, data, (size_t)n * elem, cudaMemcpyHostToDevice, s));
-            pack(stage, n, at0);
+    cudaPointerAttributes attr;
+    if (cudaPointerGetAttributes(&attr, data) != cudaSuccess) {
+        cudaGetLastError();
+        attr.type = cudaMemoryTypeUnregistered;
+    }
+    const bool on_device = attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
+    // The row offsets, and host data while they fit beside them, travel in one copy out of the engine's pinned
+    // block; larger host data goes through a staging buffer in pieces, each packed as soon as it has landed.
+    const size_t off_bytes = ((size_t)(rows + 1) * sizeof(i64) + 255) & ~(size_t)255, n_bytes = (size_t)n * elem;
+    const size_t room = STBPE_PINNED_BYTES - STBPE_PINNED_STATE;
+    const bool small = !on_device && off_bytes + n_bytes <= room;
+    const size_t dev_bytes = off_bytes + (small ? n_bytes : 0);
+    if (dev_bytes > e->off_cap) {
+        dev_free(e, e->off_dev);
+        e->off_dev = nullptr;
+        e->off_cap = 0;
+        unsigned char *t = nullptr;
+        CK(dev_alloc(e, &t, dev_bytes));
+        e->off_dev = t;
+        e->off_cap = dev_bytes;
+    }
+    for (;;) {
+        if (off_bytes <= room) {
+            char *pin = (char *)e->pinned.p + STBPE_PINNED_STATE;
+            memcpy(pin, off, (size_t)(rows + 1) * sizeof(i64));
+            if (small) memcpy(pin + off_bytes, data, n_bytes);
+            CK(cudaMemcpyAsync(e->off_dev, pin, dev_bytes, cudaMemcpyHostToDevice, s));
         } else {
-            cudaStream_t cs = nullptr;
-            cudaEvent_t ready = nullptr, landed = nullptr;
-            CK(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-            cudaError_t ce = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
-            if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&landed, cudaEventDisableTiming);
-            if (ce == cudaSuccess) ce = cudaEventRecord(ready, s);  // the staging buffer is free once s got here
-            if (ce == cudaSuccess) ce = cudaStreamWaitEvent(cs, ready, 0);
-            for (i64 at = 0; at < n && ce == cudaSuccess; at += piece) {
-                const i64 cnt = n - at < piece ? n - at : piece;
-                ce = cudaMemcpyAsync(stage + (size_t)at * elem, (const char *)data + (size_t)at * elem,
-                                     (size_t)cnt * elem, cudaMemcpyHostToDevice, cs);
-                if (ce == cudaSuccess) ce = cudaEventRecord(landed, cs);
-                if (ce == cudaSuccess) ce = cudaStreamWaitEvent(s, landed, 0);  // waits for the record just made
-                if (ce == cudaSuccess) pack(stage + (size_t)at * elem, cnt, at0 + at);
-            }
-            if (ce == cudaSuccess) ce = cudaStreamSynchronize(cs);
-            if (ready) cudaEventDestroy(ready);
-            if (landed) cudaEventDestroy(landed);
-            cudaStreamDestroy(cs);
-            CK(ce);
+            CK(cudaMemcpyAsync(e->off_dev, off, (size_t)(rows + 1) * sizeof(i64), cudaMemcpyHostToDevice, s));
         }
-    }
-    CK(cudaGetLastError());
-    // row starts
-    std::vector<i64> single = {0, n};
-    const i64 *off = row_offsets;
-    i64 rows = n_rows;
-    if (!off) {
-        off = single.data();
-        rows = 1;
-    } else {
-        if (off[0] != 0 || off[rows] != n) {
-            if (staged) cudaFreeAsync(staged, s);
-            return fail(e, STBPE_E_BADARG, "row_offsets must start at 0 and end at n");
+        if (on_device) {
+            CK(pack(data, n, at0));
+        } else if (small) {
+            CK(pack((char *)e->off_dev + off_bytes, n, at0));
+        } else {
+            const size_t half = n_bytes < ((size_t)32 << 20) ? ((n_bytes + 255) & ~(size_t)255) : (size_t)32 << 20;
+            unsigned char *stage = nullptr;
+            CK(dev_alloc(e, &stage, 2 * half));
+            const cudaError_t c = stbpe::staged_copy(data, (size_t)n, elem, attr.type == cudaMemoryTypeUnregistered, stage, half, s,
+                                                     [&](void *src, size_t at, size_t cnt) { return pack(src, (i64)cnt, at0 + (i64)at); });
+            const cudaError_t c2 = cudaStreamSynchronize(s);
+            dev_free(e, stage);
+            CK(c);
+            CK(c2);
         }
-    }
-    if (elem == 4 && !e->wide) {
-        // an id that 15 bits cannot hold: what the stream holds so far is widened, and this piece is packed
-        // again (it is still on the device, in the caller's buffer or in the staging buffer)
-        unsigned int err = 0;
-        CK(cudaMemcpyAsync(&err, bad, sizeof(err), cudaMemcpyDeviceToHost, s));
+        with_tok(e, [&](auto t) {
+            mark_row_starts_kernel<decltype(t)><<<(unsigned int)((rows + 255) / 256), 256, 0, s>>>((const i64 *)e->off_dev, rows, e->d.tiles, at0);
+        });
+        CK(cudaGetLastError());
+        // the host offsets (and a host source) must stay valid until the copies ran
+        if (elem == 1) {
+            CK(cudaStreamSynchronize(s));
+            break;
+        }
+        unsigned int *err = (unsigned int *)e->pinned.p;  // error bits and the largest id behind them
+        CK(cudaMemcpyAsync(err, bad, 2 * sizeof(*err), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        if (err & STBPE_DERR_NARROW) {
-            err &= ~STBPE_DERR_NARROW;
-            CK(cudaMemcpyAsync(bad, &err, sizeof(err), cudaMemcpyHostToDevice, s));
-            const void *src = is_device_pointer(data) ? data : staged;
-            if (!src) {  // staged in the second stream buffer, which the widening takes over
-                CK(cudaMallocAsync(&staged, (size_t)n * elem, s));
-                CK(cudaMemcpyAsync(staged, data, (size_t)n * elem, cudaMemcpyHostToDevice, s));
-                src = staged;
-            }
-            int rc = widen_stream(e, s);
-            if (rc != STBPE_OK) return rc;
-            pack(src, n, at0);
-            CK(cudaGetLastError());
-        }
+        if (err[1] > e->max_id) e->max_id = err[1];
+        e->load_err |= *err & ~STBPE_DERR_NARROW;
+        if (!(*err & STBPE_DERR_NARROW)) break;
+        // an id that 15 bits cannot hold: what the stream holds so far is widened, and this piece is packed again
+        *err &= ~STBPE_DERR_NARROW;
+        CK(cudaMemcpyAsync(bad, err, sizeof(*err), cudaMemcpyHostToDevice, s));
+        int rc = widen_stream(e, s);
+        if (rc != STBPE_OK) return rc;
     }
-    i64 *doff = nullptr;
-    CK(cudaMallocAsync((void **)&doff, (size_t)(rows + 1) * sizeof(i64), s));
-    CK(cudaMemcpyAsync(doff, off, (size_t)(rows + 1) * sizeof(i64), cudaMemcpyHostToDevice, s));
-    with_tok(e, [&](auto t) {
-        mark_row_starts_kernel<decltype(t)><<<(unsigned int)((rows + 255) / 256), 256, 0, s>>>(doff, rows, e->d.tiles, at0);
-    });
-    CK(cudaGetLastError());
-    CK(cudaFreeAsync(doff, s));
-    if (staged) CK(cudaFreeAsync(staged, s));
-    // the host offsets (and a host source) must stay valid until the copies ran
-    CK(cudaStreamSynchronize(s));
     e->n_tokens += n;
     e->recs_stale = true;
     e->counted = false;
@@ -521,7 +609,7 @@ static int check_device_error(stbpe_engine *e, cudaStream_t s) {
 
 static int prepare_stream_state(stbpe_engine *e, cudaStream_t s) {
     if (e->recs_stale) {
-        int rc = check_device_error(e, s);  // id range flag from the pack kernels
+        int rc = check_error_bits(e, e->load_err);  // id range flag from the pack kernels
         if (rc != STBPE_OK) return rc;
         e->d.n_tiles = (int)((e->n_tokens + STBPE_TILE - 1) / STBPE_TILE);
         if (e->d.n_tiles > 0) {
@@ -530,12 +618,9 @@ static int prepare_stream_state(stbpe_engine *e, cudaStream_t s) {
             });
             CK(cudaGetLastError());
         }
-        DevState h;
-        memset(&h, 0, sizeof(h));
-        h.base_vocab = e->cfg.base_vocab;
-        h.n_live = e->n_tokens;
-        CK(cudaMemcpyAsync(e->d.st, &h, sizeof(h), cudaMemcpyHostToDevice, s));
-        CK(cudaStreamSynchronize(s));
+        init_state_kernel<<<1, 1, 0, s>>>(e->d, e->cfg.base_vocab, e->n_tokens);
+        CK(cudaGetLastError());
+        e->state_stale = false;
         e->recs_stale = false;
         e->repacks_since_load = 0;
         e->filter_valid = false;  // a fresh stream starts without a pair filter (see filter_policy)
@@ -550,6 +635,15 @@ __global__ void clear_skip_state_kernel(EngineDev e, int valid) {
 
 // The pair filter follows the tile layout: it is rebuilt from the stream, or declared stale.
 static int rebuild_presence(stbpe_engine *e, cudaStream_t s) {
+    const size_t groups = ((size_t)e->d.n_tiles + 31) / 32;
+    if (groups > e->presence_cap) {
+        CK(cudaStreamSynchronize(s));
+        dev_free(e, e->d.presence);
+        e->d.presence = nullptr;
+        e->presence_cap = 0;
+        CK(dev_alloc(e, &e->d.presence, (size_t)STBPE_PPITCH * groups));
+        e->presence_cap = groups;
+    }
     clear_skip_state_kernel<<<1, 1, 0, s>>>(e->d, 1);
     CK(cudaGetLastError());
     e->filter_valid = true;
@@ -588,11 +682,59 @@ static int wide_alloc(stbpe_engine *e) {
     return STBPE_OK;
 }
 
+// the pair table has `want` slots; its memory is kept while it is large enough
+static int set_table(stbpe_engine *e, u64 want) {
+    set_slots(e, want);
+    if (e->d.table && e->table_cap >= e->slots) return STBPE_OK;
+    dev_free(e, e->d.table);
+    e->d.table = nullptr;
+    e->table_cap = 0;
+    cudaError_t c = dev_alloc(e, &e->d.table, e->slots);
+    if (c != cudaSuccess) return cuda_fail(e, c, "cudaMalloc pair table");
+    e->table_cap = e->slots;
+    return STBPE_OK;
+}
+
+// Four times the slots: the keys that still have a count move over.  Slots change, so the candidate list ends.
+static int grow_table(stbpe_engine *e, cudaStream_t s) {
+    Slot *old = e->d.table;
+    const u64 old_slots = e->slots;
+    Slot *fresh = nullptr;
+    cudaError_t c = dev_alloc(e, &fresh, old_slots * 4);
+    if (c != cudaSuccess) {
+        cudaGetLastError();
+        e->table_auto = false;  // no room: go on in the table there is, a full one is an error status
+        return STBPE_OK;
+    }
+    set_slots(e, old_slots * 4);
+    e->d.table = fresh;
+    e->table_cap = e->slots;
+    clear_table_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d);
+    cand_none_kernel<<<1, 1, 0, s>>>(e->d);
+    CK(cudaMemsetAsync(&e->d.st->n_keys, 0, sizeof(u64), s));
+    rehash_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d, old, old_slots);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(s));
+    dev_free(e, old);
+    return STBPE_OK;
+}
+
 // what every count starts with: tile records of a fresh stream, an empty table, no maxima
 static int count_prologue(stbpe_engine *e, cudaStream_t s) {
-    e->convert_ms = 0.f;
+    const bool fresh = e->recs_stale;
+    e->convert_ms = e->count_ms = 0.f;
+    e->count_timed = false;
     int rc = prepare_stream_state(e, s);
     if (rc != STBPE_OK) return rc;
+    if (e->table_auto) {
+        // A stream of bytes starts with at most 65 536 pairs and its table grows with the keys (grow_table): a table
+        // of 16 MB stays in L2 and costs nothing to clear or scan, one for every pair a run might create is
+        // half a gigabyte on 128 MB of text.  Other streams may hold any number of pairs from the start.
+        u64 want = e->only_bytes ? (u64)1 << 20 : auto_slots(e->max_tokens);
+        if (!fresh && e->slots > want) want = e->slots;  // a recount of the rewritten stream
+        rc = set_table(e, want);
+        if (rc != STBPE_OK) return rc;
+    }
     clear_table_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d);
     CK(cudaGetLastError());
     if (e->cfg.world_size > 1) {
@@ -656,24 +798,26 @@ static int launch_count(stbpe_engine *e, bool mg, cudaStream_t s) {
             count_dense_kernel<decltype(t)><<<e->sm_count, STBPE_DENSE_THREADS, 32768 * 4, s>>>(e->d, e->dense);
         });
         CK(cudaGetLastError());
-        unsigned int derr = 0;
-        CK(cudaMemcpyAsync(&derr, &e->d.st->error, sizeof(derr), cudaMemcpyDeviceToHost, s));
+        // one rank: into the table at once, an overflow is looked at with the final error check and counts again;
+        // several ranks: the deltas of a failed count must not reach the rank-local table
+        if (!mg) dense_to_table_kernel<false><<<256, 256, 0, s>>>(e->d, e->dense);
+        CK(cudaGetLastError());
+        CK(cudaEventRecord(e->ev1, s));
+        e->count_timed = true;
+        unsigned int *derr = (unsigned int *)e->pinned.p;
+        CK(cudaMemcpyAsync(derr, &e->d.st->error, sizeof(*derr), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        if (!(derr & STBPE_DERR_DENSE_OVERFLOW)) {
-            if (mg)
-                dense_to_table_kernel<true><<<256, 256, 0, s>>>(e->d, e->dense);
-            else
-                dense_to_table_kernel<false><<<256, 256, 0, s>>>(e->d, e->dense);
+        if (!(*derr & STBPE_DERR_DENSE_OVERFLOW)) {
+            if (mg) dense_to_table_kernel<true><<<256, 256, 0, s>>>(e->d, e->dense);
             CK(cudaGetLastError());
-            CK(cudaEventRecord(e->ev1, s));
-            CK(cudaEventSynchronize(e->ev1));
-            CK(cudaEventElapsedTime(&e->count_ms, e->ev0, e->ev1));
             return STBPE_OK;
         }
         // a 16-bit counter came too close to its limit: discard and count with the general kernel
-        derr &= ~STBPE_DERR_DENSE_OVERFLOW;
-        CK(cudaMemcpyAsync(&e->d.st->error, &derr, sizeof(derr), cudaMemcpyHostToDevice, s));
+        *derr &= ~STBPE_DERR_DENSE_OVERFLOW;
+        CK(cudaMemcpyAsync(&e->d.st->error, derr, sizeof(*derr), cudaMemcpyHostToDevice, s));
         CK(cudaStreamSynchronize(s));
+        rc = count_prologue(e, s);
+        if (rc != STBPE_OK) return rc;
     }
     if (!mg && wide_eligible(e, fresh)) {
         // 16-bit vocabulary: partition the pairs, then count partition by partition inside L2
@@ -719,8 +863,7 @@ static int launch_count(stbpe_engine *e, bool mg, cudaStream_t s) {
         });
         CK(cudaGetLastError());
         CK(cudaEventRecord(e->ev1, s));
-        CK(cudaEventSynchronize(e->ev1));
-        CK(cudaEventElapsedTime(&e->count_ms, e->ev0, e->ev1));
+        e->count_timed = true;
     }
     return STBPE_OK;
 }
@@ -755,8 +898,7 @@ static int refill_candidates(stbpe_engine *e, cudaStream_t s) {
         cand_collect_kernel<<<grid, 512, 0, s>>>(e->d);
         CK(cudaGetLastError());
         DevState h;
-        CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
+        if (int rc_ = read_state(e, &h, s)) return rc_;
         if (h.cand_state == STBPE_CAND_READY) return STBPE_OK;
     }
     return fail(e, STBPE_E_STATE, "no candidate threshold found");
@@ -767,8 +909,7 @@ static int choose(stbpe_engine *e, bool advance, DevState *h, cudaStream_t s) {
     for (int attempt = 0; attempt < 2; ++attempt) {
         choose_kernel<<<1, 1024, 0, s>>>(e->d, advance ? 1 : 0);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(h, e->d.st, sizeof(*h), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
+        if (int rc_ = read_state(e, h, s)) return rc_;
         if (h->peek_valid || (advance && h->stopped)) return STBPE_OK;
         int rc = refill_candidates(e, s);
         if (rc != STBPE_OK) return rc;
@@ -795,8 +936,7 @@ STBPE_VISIBLE int stbpe_select_best(stbpe_engine *e, uint64_t *key, int64_t *cou
         count_ties_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d);
         CK(cudaGetLastError());
     }
-    CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    if (int rc_ = read_state(e, &h, s)) return rc_;
     *key = h.peek_count > 0 ? h.peek_key : 0;
     *count = h.peek_count;
     if (n_ties) *n_ties = h.peek_count > 0 ? h.peek_ties : 0;
@@ -937,8 +1077,7 @@ static int maybe_repack(stbpe_engine *e, bool force, int *did, cudaStream_t s) {
     const int nt = e->d.n_tiles;
     if (nt < 1 || e->recs_stale) return STBPE_OK;
     DevState h;
-    CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    if (int rc_ = read_state(e, &h, s)) return rc_;
     if (nt < 2 || (!force && (h.n_live * 4 > (i64)nt * STBPE_TILE * 3 || nt < 64)))  // re-pack at <= 75 % fill
         return filter_policy(e, h, false, s);
     i64 total = 0;
@@ -987,6 +1126,8 @@ static int run_loop(stbpe_engine *e, int target, const int2 *forced, int n_force
         const double fc = e->filter_density * (double)e->d.n_tiles;
         la.filter_count = fc >= 9e18 ? (i64)9000000000000000000ll : (i64)fc;
         la.repack_tiles = 64;
+        la.grow_keys = e->table_auto ? (i64)(e->slots / 4) : (i64)0x7FFFFFFFFFFFFFFFll;
+        la.ids_below = e->only_bytes ? 0 : (int)e->max_id + 1;
         la.unit_shift = unit_shift(e, grid);
         EngineDev d = e->d;
         void *args[2] = {&d, &la};
@@ -997,13 +1138,15 @@ static int run_loop(stbpe_engine *e, int target, const int2 *forced, int n_force
                                                MergeGeom<T>::BYTES + STBPE_CAND_CAP * sizeof(unsigned int), s);
         });
         if (c != cudaSuccess) return cuda_fail(e, c, "cudaLaunchCooperativeKernel");
-        CK(cudaMemcpyAsync(out, e->d.st, sizeof(*out), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
+        if (int rc_ = read_state(e, out, s)) return rc_;
         at += forced ? out->forced_done : 0;
         int rc = check_error_bits(e, out->error);
         if (rc != STBPE_OK) return rc;
         if (out->run_exit == STBPE_EXIT_STOP) return STBPE_OK;
-        if (out->run_exit == STBPE_EXIT_REFILL) {
+        if (out->run_exit == STBPE_EXIT_GROW) {
+            rc = grow_table(e, s);
+            if (rc == STBPE_OK) rc = refill_candidates(e, s);
+        } else if (out->run_exit == STBPE_EXIT_REFILL) {
             rc = refill_candidates(e, s);
         } else if (out->run_exit == STBPE_EXIT_REPACK) {
             rc = maybe_repack(e, false, nullptr, s);
@@ -1020,8 +1163,7 @@ static int run_loop(stbpe_engine *e, int target, const int2 *forced, int n_force
 // host-given merges, applied in order as merges of the log
 static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t first_new, int64_t *n_matches, cudaStream_t s) {
     DevState h;
-    CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    if (int rc_ = read_state(e, &h, s)) return rc_;
     if ((i64)h.merges_done + n > e->cfg.max_merges) return fail(e, STBPE_E_CAPACITY, "merge log full");
     if (n > e->forced_cap) {
         dev_free(e, e->forced);
@@ -1043,8 +1185,7 @@ STBPE_VISIBLE int stbpe_train(stbpe_engine *e, int32_t n_merges, void *stream) {
     if (!e->counted) return fail(e, STBPE_E_STATE, "count the pairs before training");
     if (e->cfg.world_size > 1) return fail(e, STBPE_E_STATE, "single-rank entry point");
     DevState h;
-    CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    if (int rc_ = read_state(e, &h, s)) return rc_;
     i64 target = (i64)h.merges_done + n_merges;
     if (target > e->cfg.max_merges) target = e->cfg.max_merges;
     return run_loop(e, (int)target, nullptr, 0, 0, &h, s);
@@ -1059,8 +1200,7 @@ STBPE_VISIBLE int stbpe_train_timed(stbpe_engine *e, int32_t n_merges, float *ke
     if (!e->counted) return fail(e, STBPE_E_STATE, "count the pairs before training");
     if (e->cfg.world_size > 1) return fail(e, STBPE_E_STATE, "single-rank entry point");
     DevState h;
-    CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    if (int rc_ = read_state(e, &h, s)) return rc_;
     i64 target = (i64)h.merges_done + n_merges;
     if (target > e->cfg.max_merges) target = e->cfg.max_merges;
     set_target_kernel<<<1, 1, 0, s>>>(e->d, (int)target);
@@ -1106,6 +1246,10 @@ STBPE_VISIBLE int stbpe_train_timed(stbpe_engine *e, int32_t n_merges, float *ke
             cudaEventRecord(ev[4 * i], s);
             rc = choose(e, true, &h2, s);
             cudaEventRecord(ev[4 * i + 1], s);
+            if (rc == STBPE_OK && e->table_auto && (i64)h2.n_keys + 131072 > (i64)(e->slots / 4)) {
+                rc = grow_table(e, s);  // every merge adds at most two pairs per id of the vocabulary
+                if (rc == STBPE_OK) rc = refill_candidates(e, s);
+            }
             if (rc != STBPE_OK) break;
             rc = launch_merge(e, false, s);
             cudaEventRecord(ev[4 * i + 2], s);
@@ -1132,8 +1276,9 @@ STBPE_VISIBLE int stbpe_get_state(stbpe_engine *e, stbpe_state *out, void *strea
     cudaStream_t s = (cudaStream_t)stream;
     CK(cudaSetDevice(e->cfg.device));
     DevState h;
-    CK(cudaMemcpyAsync(&h, e->d.st, sizeof(h), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    if (int rc_ = fresh_state(e, s)) return rc_;
+    if (int rc_ = read_state(e, &h, s)) return rc_;
+    if (e->count_timed && cudaEventElapsedTime(&e->count_ms, e->ev0, e->ev1) == cudaSuccess) e->count_timed = false;
     out->merges_done = h.merges_done;
     out->stop_reason = h.stopped ? h.stop_reason : STBPE_RUNNING;
     out->live_tokens = e->recs_stale ? e->n_tokens : h.n_live;
@@ -1168,6 +1313,8 @@ STBPE_VISIBLE int stbpe_export_histogram(stbpe_engine *e, uint64_t *keys, int64_
     if (!e || !n_out || cap < 0) return STBPE_E_BADARG;
     cudaStream_t s = (cudaStream_t)stream;
     CK(cudaSetDevice(e->cfg.device));
+    *n_out = 0;
+    if (!e->d.table) return STBPE_OK;  // nothing has been counted
     u64 *tk = nullptr;
     i64 *tc = nullptr;
     CK(cudaMallocAsync((void **)&tk, (size_t)(cap > 0 ? cap : 1) * sizeof(u64), s));
@@ -1202,6 +1349,8 @@ STBPE_VISIBLE int stbpe_export_ties(stbpe_engine *e, int64_t count, uint64_t *ke
     if (!e || !n_out || cap < 0 || (cap > 0 && !keys)) return STBPE_E_BADARG;
     cudaStream_t s = (cudaStream_t)stream;
     CK(cudaSetDevice(e->cfg.device));
+    *n_out = 0;
+    if (!e->d.table) return STBPE_OK;  // nothing has been counted
     CK(cudaMemsetAsync(&e->d.st->export_n, 0, sizeof(i64), s));
     export_ties_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d, count, (u64 *)keys, cap);
     CK(cudaGetLastError());
@@ -1581,7 +1730,7 @@ STBPE_VISIBLE int stbpe_mg_peer_run(stbpe_engine *e, int first, int n_rounds, vo
     const int G = 16;  // rounds per graph replay
     while (r < n_rounds) {
         if (e->use_graph && n_rounds - r >= G) {
-            if (e->graph && (e->graph_tiles_n != e->d.n_tiles || e->graph_tiles != e->d.tiles || e->graph_wide != e->wide)) {
+            if (e->graph && (e->graph_tiles_n != e->d.n_tiles || e->graph_tiles != e->d.tiles || e->graph_wide != e->wide || e->graph_filter != e->d.presence)) {
                 cudaGraphExecDestroy(e->graph);
                 e->graph = nullptr;
             }
@@ -1608,6 +1757,7 @@ STBPE_VISIBLE int stbpe_mg_peer_run(stbpe_engine *e, int first, int n_rounds, vo
                 e->graph_tiles_n = e->d.n_tiles;  // the capture froze the stream pointer, n_tiles and the grids
                 e->graph_tiles = e->d.tiles;
                 e->graph_wide = e->wide;
+                e->graph_filter = e->d.presence;
             }
             CK(cudaGraphLaunch(e->graph, s));
             r += G;
@@ -1664,9 +1814,6 @@ NcclApi &nccl_api() {
         }
     }
     return api;
-}
-void nccl_comm_destroy(void *comm) {
-    if (comm && nccl_api().ok) nccl_api().CommDestroy((ncclComm_t)comm);
 }
 }  // namespace
 

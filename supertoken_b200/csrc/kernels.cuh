@@ -50,9 +50,10 @@ __global__ void pack_bytes_kernel(const uint8_t *__restrict__ src, i64 n, void *
 // stream can hold NARROW (the host then widens the stream and packs again)
 template <typename T>
 __global__ void pack_ids_kernel(const int32_t *__restrict__ src, i64 n, void *tiles, i64 at, unsigned int *bad) {
-    unsigned int err = 0;
+    unsigned int err = 0, largest = 0;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
         const int32_t v = __ldcs(src + i);
+        largest = max(largest, (unsigned int)v & STBPE_IDMASK);
         if (v < 0 || v == 0x7FFFFFFF)
             err |= STBPE_DERR_BAD_ID;
         else if ((uint32_t)v >= Tok<T>::IDMASK)
@@ -60,6 +61,8 @@ __global__ void pack_ids_kernel(const int32_t *__restrict__ src, i64 n, void *ti
         put_token<T>(tiles, at + i, (uint32_t)v & Tok<T>::IDMASK);
     }
     if (err) atomicOr(bad, err);
+    largest = __reduce_max_sync(0xFFFFFFFFu, largest);
+    if ((threadIdx.x & 31) == 0) atomicMax(bad + 1, largest);  // DevState::max_id
 }
 
 template <typename T>
@@ -92,6 +95,13 @@ __global__ void init_recs_kernel(EngineDev e, i64 n_tokens) {
     r.len = 0;
     e.recs[2 * t + 1] = r;
     e.tile_live[t] = (unsigned int)len;
+}
+
+__global__ void init_state_kernel(EngineDev e, int base_vocab, i64 n_tokens) {
+    DevState h = {};
+    h.base_vocab = base_vocab;
+    h.n_live = n_tokens;
+    *e.st = h;
 }
 
 __global__ void clear_table_kernel(EngineDev e) {
@@ -221,6 +231,17 @@ __device__ __forceinline__ bool table_insert_unique(const EngineDev &e, u64 key,
     }
     atomicOr(&e.st->error, STBPE_DERR_TABLE_FULL);
     return false;
+}
+
+// keys with a count from a smaller table into this one (grow_table)
+__global__ void rehash_kernel(EngineDev e, const Slot *__restrict__ old, u64 n) {
+    unsigned int moved = 0;
+    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
+        const Slot s = old[i];
+        if (s.key != STBPE_EMPTY && s.count != 0 && table_insert_unique(e, s.key, s.count)) ++moved;
+    }
+    moved = __reduce_add_sync(0xFFFFFFFFu, moved);
+    if ((threadIdx.x & 31) == 0 && moved) atomicAdd(&e.st->n_keys, (u64)moved);
 }
 
 #include "wide_count.cuh"

@@ -29,6 +29,8 @@ struct LoopArgs {
     i64 filter_count;       // leave to build the pair filter when the merge's count has fallen to this
     int repack_tiles;       // leave for a re-pack at three quarters live from this many tiles on
     int unit_shift;         // tiles per filter unit, log2 (cta_merge)
+    i64 grow_keys;          // leave for a larger pair table when a merge could take the number of keys beyond this ...
+    int ids_below;          // ... given that the stream's own ids lie below this (0: below the merges' ids)
 };
 
 __device__ __forceinline__ u64 loop_timer_ns() {
@@ -117,7 +119,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ int s_ctr[CTR_N];
     __shared__ Bt s_best[2][32];          // the warps' best candidates, alternating between steps
-    __shared__ i64 s_live, s_forced;      // live tokens, count of the next host-given pair
+    __shared__ i64 s_live, s_keys, s_forced;  // live tokens, keys in the table, count of the next host-given pair
     __shared__ unsigned int s_err;        // device error bits
     __shared__ int s_ok;                  // every wait so far succeeded
     __shared__ int s_work;                // CTA 0: tiles the last merge visited
@@ -165,6 +167,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             if (lane == 0) s_best[step & 1][warp] = x;
             if (tid == THREADS - 1) {
                 s_live = (i64)__ldcg((const u64 *)&st->n_live);
+                s_keys = (i64)__ldcg(&st->n_keys);
                 s_err = __ldcg(&st->error) | (n > STBPE_CAND_CAP ? 0x80000000u : 0u);
                 if (la.forced && forced_i < la.n_forced) {
                     const i64 at = find_slot(e, ((u64)(uint32_t)la.forced[forced_i].x << 32) | (uint32_t)la.forced[forced_i].y);
@@ -207,6 +210,8 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             else if (!host && count < 2) stop = 3;
             else if (e.n_tiles >= la.repack_tiles && s_live * 4 <= (i64)e.n_tiles * STBPE_TILE * 3) why = STBPE_EXIT_REPACK;
             else if (!fv && e.n_tiles > 0 && count <= la.filter_count) why = STBPE_EXIT_FILTER;
+            // every merge makes at most two pairs per match and two per id
+            else if (s_keys + 2 * min(count, (i64)max((int)mc.nw, la.ids_below)) + 2 > la.grow_keys) why = STBPE_EXIT_GROW;
             else if (sizeof(T) == 2 && max(mc.nw, max(mc.a, mc.b)) >= Tok<uint16_t>::IDMASK) why = STBPE_EXIT_WIDEN;
             else go = 1;
             if (cta == 0 && tid == 0) {

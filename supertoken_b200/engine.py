@@ -164,7 +164,7 @@ class Engine:
         if n > 0:
             self._check(self._lib.stbpe_get_merges(self._h, first, n, m.ctypes.data, c.ctypes.data,
                                                    lb.ctypes.data))
-        return [(int(x), int(y)) for x, y in m], c, lb
+        return list(zip(m[:, 0].tolist(), m[:, 1].tolist())), c, lb
 
     def export_histogram(self, cap: Optional[int] = None):
         """(keys int64 ascending, counts int64) on the device, zero counts dropped."""
