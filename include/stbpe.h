@@ -108,6 +108,16 @@ int stbpe_select_best(stbpe_engine *e, uint64_t *key, int64_t *count, int64_t *n
 int stbpe_apply_merge(stbpe_engine *e, int32_t a, int32_t b, int32_t new_id, int64_t *n_matches,
                       void *stream);
 
+/* n merges in order, pairs = n x (a, b) in host memory, merge i gets id first_new_id + i: stbpe_apply_merge n
+ * times in one launch (warm start, gpu_tokenizer/bpe_trainer.py:4058-4182). */
+int stbpe_apply_merges(stbpe_engine *e, const int32_t *pairs, int32_t n, int32_t first_new_id, void *stream);
+
+/* One step of a loop that breaks ties on the host (gpu_tokenizer/bpe_trainer.py:915-923): applies (a, b) ->
+ * new_id (nothing when new_id < 0), then returns the best count and the keys that hold it, ascending, into
+ * keys (host, cap entries; not written when *n_ties exceeds cap).  count 0 = empty histogram. */
+int stbpe_next_tied(stbpe_engine *e, int32_t a, int32_t b, int32_t new_id, int64_t *count, uint64_t *keys,
+                    int64_t cap, int64_t *n_ties, void *stream);
+
 /* The merge loop (gpu_tokenizer/bpe_trainer.py:4193-4517) run on the device without
  * a host round trip per merge: select -> stop rules -> apply, n_merges times or until a
  * stop rule fires.  Synchronises the stream before returning. */
@@ -255,6 +265,12 @@ int stbpe_rows_count_pairs(const int32_t *tokens, const uint8_t *valid, int64_t 
                            int64_t *length_dev, void *stream);
 int stbpe_rows_apply_merge(int32_t *tokens, uint8_t *valid, int32_t *lengths, int64_t B, int64_t L,
                            int32_t a, int32_t b, int32_t new_id, uint8_t *spans, void *stream);
+
+/* stbpe_select_pair <- select_best_pair without a tie breaker (gpu_tokenizer/trainers/bpe_gpu.py:96-130) on an
+ * exported histogram (device arrays of n entries): maximum count, ties to the smallest key; index = its place,
+ * -1 when no count is positive.  Synchronises the stream. */
+int stbpe_select_pair(const int64_t *keys, const int64_t *counts, int64_t n, int64_t *key, int64_t *count,
+                      int64_t *index, void *stream);
 
 /* stbpe_rows_count_pairs for callers that must not allocate device memory.  It has no
  * counterpart in the reference.  Same inputs, outputs and result as stbpe_rows_count_pairs, but

@@ -45,6 +45,8 @@ SIGNATURES = {
     "stbpe_count_initial": (_int, [_vp, _vp]),
     "stbpe_select_best": (_int, [_vp, _P(ctypes.c_uint64), _P(_i64), _P(_i64), _vp]),
     "stbpe_apply_merge": (_int, [_vp, _i32, _i32, _i32, _P(_i64), _vp]),
+    "stbpe_apply_merges": (_int, [_vp, _vp, _i32, _i32, _vp]),
+    "stbpe_next_tied": (_int, [_vp, _i32, _i32, _i32, _P(_i64), _vp, _i64, _P(_i64), _vp]),
     "stbpe_train": (_int, [_vp, _i32, _vp]),
     "stbpe_train_timed": (_int, [_vp, _i32, _P(ctypes.c_float), _vp]),
     "stbpe_repack": (_int, [_vp, _int, _P(_int), _vp]),
@@ -76,6 +78,7 @@ SIGNATURES = {
     "stbpe_mg_wide_pass1": (_int, [_vp, _P(_i32), _vp]),
     "stbpe_mg_wide_pass2": (_int, [_vp, _vp]),
     "stbpe_mg_wide_close": (_int, [_vp]),
+    "stbpe_select_pair": (_int, [_vp, _vp, _i64, _P(_i64), _P(_i64), _P(_i64), _vp]),
     "stbpe_rows_count_pairs": (_int, [_vp, _vp, _i64, _i64, _vp, _vp, _i64, _vp, _vp]),
     "stbpe_rows_count_pairs_noalloc": (_int, [_vp, _vp, _i64, _i64, _vp, _vp, _i64, _vp, _vp,
                                               ctypes.c_char_p, ctypes.c_size_t]),

@@ -344,13 +344,14 @@ class GPUBPETrainer(BaseTrainer):
 
         # warm start: seeded merges are applied without selection (bpe_trainer.py:4058-4182)
         warm_applied = 0
-        for a, b in warm[: self.target_merges]:
-            if max(a, b, self.vocab_size) > UINT32_MAX:
-                raise OverflowError(f"Token id overflow: encountered id above UINT32_MAX (limit {UINT32_MAX}).")
-            eng.apply_merge(int(a), int(b), self.vocab_size)
-            self.merges.append((int(a), int(b)))
-            self.vocab_size += 1
-            warm_applied += 1
+        seed = [(int(a), int(b)) for a, b in warm[: self.target_merges]]
+        bad = next((i for i, (a, b) in enumerate(seed) if max(a, b, self.vocab_size + i) > UINT32_MAX), len(seed))
+        eng.apply_merges(seed[:bad], self.vocab_size)
+        self.merges.extend(seed[:bad])
+        self.vocab_size += bad
+        warm_applied += bad
+        if bad < len(seed):
+            raise OverflowError(f"Token id overflow: encountered id above UINT32_MAX (limit {UINT32_MAX}).")
 
         def checkpoint():
             self.save_checkpoint(checkpoint_dir, dataset_state=dataset_state)
@@ -540,21 +541,24 @@ class GPUBPETrainer(BaseTrainer):
         ``trainers/bpe_gpu.py:112-123``).  ``checkpoint`` is called every ``checkpoint_interval``
         merges (the checkpoint carries the generator's state, so a resumed run draws on)."""
         since = 0
+        count, cands = eng.next_tied() if remaining > 0 else (0, [])
         while remaining > 0:
-            key, count, ties = eng.select_best(with_ties=True)
-            if key is None:
+            if not cands:
                 return L.STOP_NO_PAIRS
             if count < 2:
                 return L.STOP_LOW_COUNT
-            if ties > 1 and self._tie_rng is not None:
-                cands = eng.tied_keys(count, ties)
+            key = cands[0]
+            if len(cands) > 1 and self._tie_rng is not None:
                 key = cands[self._tie_rng.randrange(len(cands))]
             a, b = key >> 32, key & 0xFFFFFFFF
-            eng.apply_merge(a, b, self.vocab_size)
             self.merges.append((a, b))
             self.merge_counts.append(count)
-            self.vocab_size += 1
             remaining -= 1
+            if remaining > 0:
+                count, cands = eng.next_tied((a, b, self.vocab_size))
+            else:
+                eng.apply_merge(a, b, self.vocab_size)
+            self.vocab_size += 1
             since += 1
             if checkpoint is not None and checkpoint_interval and since >= checkpoint_interval and remaining > 0:
                 checkpoint()

@@ -102,6 +102,9 @@ struct DevState {
     u64 tile_bytes_in;         // merges: bytes of tiles and records read ...
     u64 tile_bytes_out;        // ... and bytes stored (rewritten 16-byte units and records), since the load
 };
+#define STBPE_TIES_OFFSET 512   // tied keys of ties_kernel lie this far behind the state
+#define STBPE_TIES_CAP 1024
+static_assert(sizeof(DevState) <= STBPE_TIES_OFFSET, "the tied keys follow the state");
 #define STBPE_EXIT_STOP 0      // a stop rule fired (DevState::stop_reason) or the given merges are done
 #define STBPE_EXIT_REPACK 1    // a quarter of the stream is holes
 #define STBPE_EXIT_FILTER 2    // the pair filter starts to pay: build it

@@ -16,11 +16,12 @@
 #include "kernels.cuh"
 #include "loop.cuh"
 
+#include <algorithm>
 #include <mutex>
 #include <utility>
 
 #define STBPE_PINNED_BYTES ((size_t)4 << 20)
-#define STBPE_PINNED_STATE 4096  // bytes in front that the device state travels through
+#define STBPE_PINNED_STATE 16384  // bytes in front that the device state travels through
 #define STBPE_COUNT_SMEM (STBPE_COUNT_SLOTS * 12)
 
 #define STBPE_VISIBLE __attribute__((visibility("default")))
@@ -82,6 +83,8 @@ struct stbpe_engine {
     stbpe::Block pinned;  // host side of small transfers: the device state, then small inputs
     unsigned int max_id;  // largest id appended through stbpe_append_ids
     unsigned int load_err;  // error bits of the rows appended so far
+    bool merges_known;    // merges_done mirrors the device (several host-driven merges in a row)
+    int merges_done;
     bool state_stale;     // the device state is that of a stream that has been dropped
     bool table_auto;      // the table is sized by the stream and grows with the keys
     u64 table_cap;        // slots the allocated table has room for
@@ -305,9 +308,9 @@ static void set_slots(stbpe_engine *e, u64 want) {
     e->d.n_blocks = (unsigned int)(slots >> e->d.blk_shift);
 }
 
-// The device state by way of pinned memory.  Synchronises the stream.
+// The device state, and the tied keys behind it, by way of pinned memory.  Synchronises the stream.
 static int read_state(stbpe_engine *e, DevState *h, cudaStream_t s) {
-    CK(cudaMemcpyAsync(e->pinned.p, e->d.st, sizeof(DevState), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(e->pinned.p, e->d.st, STBPE_TIES_OFFSET + STBPE_TIES_CAP * sizeof(u64), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     memcpy(h, e->pinned.p, sizeof(DevState));
     return STBPE_OK;
@@ -322,6 +325,7 @@ static void drop_stream(stbpe_engine *e) {
     e->filter_valid = false;
     e->wide_counted = e->full_refresh_pending = false;
     e->load_err = e->max_id = 0;
+    e->merges_known = false;
     e->state_stale = true;
 }
 
@@ -388,7 +392,7 @@ STBPE_VISIBLE int stbpe_create(stbpe_engine **out, const stbpe_config *cfg) {
         a.add(&e->rp_offs, (size_t)e->max_tiles + 1);
         cub::DeviceScan::ExclusiveSum(nullptr, e->rp_tmp_bytes, e->rp_lens, e->rp_offs, e->max_tiles + 1, 0);
         a.add((unsigned char **)&e->rp_tmp, e->rp_tmp_bytes ? e->rp_tmp_bytes : 16);
-        a.add(&e->d.st, 1);
+        a.add((unsigned char **)&e->d.st, STBPE_TIES_OFFSET + STBPE_TIES_CAP * sizeof(u64));  // state and tied keys: one copy
         a.add(&e->d.sync, 1);
         a.add(&e->d.merges, (size_t)2 * (cfg->max_merges + 1));
         a.add(&e->d.merge_counts, (size_t)cfg->max_merges + 1);
@@ -621,6 +625,7 @@ static int prepare_stream_state(stbpe_engine *e, cudaStream_t s) {
         init_state_kernel<<<1, 1, 0, s>>>(e->d, e->cfg.base_vocab, e->n_tokens);
         CK(cudaGetLastError());
         e->state_stale = false;
+        e->merges_known = false;
         e->recs_stale = false;
         e->repacks_since_load = 0;
         e->filter_valid = false;  // a fresh stream starts without a pair filter (see filter_policy)
@@ -904,6 +909,53 @@ static int refill_candidates(stbpe_engine *e, cudaStream_t s) {
     return fail(e, STBPE_E_STATE, "no candidate threshold found");
 }
 
+// The best count and the keys that hold it, ascending, out of the candidate list (or out of a scan of the table
+// when the list does not hold all of them).  `queued`: the kernel has run behind a merge and was read with it.
+static int tied_candidates(stbpe_engine *e, bool queued, std::vector<u64> *keys, i64 *count, cudaStream_t s) {
+    keys->clear();
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        DevState h;
+        if (queued) {
+            memcpy(&h, e->pinned.p, sizeof(h));
+        } else {
+            ties_kernel<<<1, 1024, 0, s>>>(e->d);
+            CK(cudaGetLastError());
+            if (int rc = read_state(e, &h, s)) return rc;
+        }
+        queued = false;
+        if (!h.peek_valid) {
+            int rc = refill_candidates(e, s);
+            if (rc != STBPE_OK) return rc;
+            continue;
+        }
+        *count = h.peek_count;
+        if (h.peek_count <= 0) return STBPE_OK;
+        if (h.peek_ties > 0 && h.peek_ties <= STBPE_TIES_CAP) {
+            const u64 *k = (const u64 *)((const char *)e->pinned.p + STBPE_TIES_OFFSET);
+            keys->assign(k, k + h.peek_ties);
+        } else {
+            CK(cudaMemsetAsync(&e->d.st->peek_ties, 0, sizeof(i64), s));
+            count_ties_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d);
+            CK(cudaGetLastError());
+            DevState h2;
+            if (int rc = read_state(e, &h2, s)) return rc;
+            stbpe::Block b;
+            CK(stbpe::device_blocks().get(e->cfg.device, (size_t)h2.peek_ties * sizeof(u64), &b));
+            CK(cudaMemsetAsync(&e->d.st->export_n, 0, sizeof(i64), s));
+            export_ties_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d, h.peek_count, (u64 *)b.p, h2.peek_ties);
+            CK(cudaGetLastError());
+            keys->resize((size_t)h2.peek_ties);
+            CK(cudaMemcpyAsync(keys->data(), b.p, keys->size() * sizeof(u64), cudaMemcpyDeviceToHost, s));
+            CK(cudaStreamSynchronize(s));
+            stbpe::device_blocks().put(e->cfg.device, b);
+        }
+        std::sort(keys->begin(), keys->end());
+        keys->erase(std::unique(keys->begin(), keys->end()), keys->end());  // a candidate may be listed twice
+        return STBPE_OK;
+    }
+    return fail(e, STBPE_E_STATE, "no candidate found");
+}
+
 // Best pair of the table into the device state, or as the loop's next step; *h = the state afterwards.
 static int choose(stbpe_engine *e, bool advance, DevState *h, cudaStream_t s) {
     for (int attempt = 0; attempt < 2; ++attempt) {
@@ -944,7 +996,7 @@ STBPE_VISIBLE int stbpe_select_best(stbpe_engine *e, uint64_t *key, int64_t *cou
 }
 
 static int filter_policy(stbpe_engine *e, const DevState &h, bool layout_changed, cudaStream_t s);
-static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t first_new, int64_t *n_matches, cudaStream_t s);
+static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t first_new, int64_t *n_matches, cudaStream_t s, bool then_ties = false);
 
 static int launch_merge(stbpe_engine *e, bool mg, cudaStream_t s) {
     if (e->d.n_tiles < 1) return STBPE_OK;
@@ -970,6 +1022,44 @@ STBPE_VISIBLE int stbpe_apply_merge(stbpe_engine *e, int32_t a, int32_t b, int32
         return fail(e, STBPE_E_ID_OVERFLOW, "Token id overflow: ids must be in [0, 2^31-2]");
     const int32_t pair[2] = {a, b};
     return run_forced(e, pair, 1, new_id, n_matches, s);
+}
+
+STBPE_VISIBLE int stbpe_apply_merges(stbpe_engine *e, const int32_t *pairs, int32_t n, int32_t first_new_id, void *stream) {
+    if (!e || n < 0 || (n > 0 && !pairs)) return STBPE_E_BADARG;
+    CK(cudaSetDevice(e->cfg.device));
+    if (!e->counted) return fail(e, STBPE_E_STATE, "count the pairs before merging");
+    if (e->cfg.world_size > 1) return fail(e, STBPE_E_STATE, "single-rank entry point");
+    if (n == 0) return STBPE_OK;
+    for (int i = 0; i < 2 * n; ++i)
+        if (pairs[i] < 0 || pairs[i] == 0x7FFFFFFF) return fail(e, STBPE_E_ID_OVERFLOW, "Token id overflow: ids must be in [0, 2^31-2]");
+    if (first_new_id < 0 || (i64)first_new_id + n - 1 >= 0x7FFFFFFFll)
+        return fail(e, STBPE_E_ID_OVERFLOW, "Token id overflow: ids must be in [0, 2^31-2]");
+    return run_forced(e, pairs, n, first_new_id, nullptr, (cudaStream_t)stream);
+}
+
+STBPE_VISIBLE int stbpe_next_tied(stbpe_engine *e, int32_t a, int32_t b, int32_t new_id, int64_t *count, uint64_t *keys, int64_t cap,
+                                  int64_t *n_ties, void *stream) {
+    if (!e || !count || !n_ties || cap < 0 || (cap > 0 && !keys)) return STBPE_E_BADARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    CK(cudaSetDevice(e->cfg.device));
+    if (!e->counted) return fail(e, STBPE_E_STATE, "count the pairs before selecting");
+    if (e->cfg.world_size > 1) return fail(e, STBPE_E_STATE, "single-rank entry point");
+    if (new_id >= 0) {
+        if (a < 0 || b < 0 || a == 0x7FFFFFFF || b == 0x7FFFFFFF || new_id == 0x7FFFFFFF)
+            return fail(e, STBPE_E_ID_OVERFLOW, "Token id overflow: ids must be in [0, 2^31-2]");
+        const int32_t pair[2] = {a, b};
+        int rc = run_forced(e, pair, 1, new_id, nullptr, s, true);
+        if (rc != STBPE_OK) return rc;
+    }
+    std::vector<u64> tied;
+    i64 c = 0;
+    int rc = tied_candidates(e, new_id >= 0, &tied, &c, s);
+    if (rc != STBPE_OK) return rc;
+    *count = c;
+    *n_ties = (i64)tied.size();
+    if ((i64)tied.size() <= cap)
+        for (size_t i = 0; i < tied.size(); ++i) keys[i] = tied[i];
+    return STBPE_OK;
 }
 
 static int maybe_repack(stbpe_engine *e, bool force, int *did, cudaStream_t s);
@@ -1114,7 +1204,7 @@ static int loop_grid(const stbpe_engine *e) {
 // Runs loop_kernel until a stop rule fires, doing the maintenance it asks for between launches.  `forced`
 // (device, n_forced pairs): these merges instead of the best pairs.  *out = the device state at the end.
 static int run_loop(stbpe_engine *e, int target, const int2 *forced, int n_forced, int forced_new, DevState *out,
-                    cudaStream_t s) {
+                    cudaStream_t s, bool then_ties = false) {
     LoopArgs la;
     int at = 0;
     for (;;) {
@@ -1138,6 +1228,10 @@ static int run_loop(stbpe_engine *e, int target, const int2 *forced, int n_force
                                                MergeGeom<T>::BYTES + STBPE_CAND_CAP * sizeof(unsigned int), s);
         });
         if (c != cudaSuccess) return cuda_fail(e, c, "cudaLaunchCooperativeKernel");
+        if (then_ties) {  // enqueued behind the merge: one round trip for both
+            ties_kernel<<<1, 1024, 0, s>>>(e->d);
+            CK(cudaGetLastError());
+        }
         if (int rc_ = read_state(e, out, s)) return rc_;
         at += forced ? out->forced_done : 0;
         int rc = check_error_bits(e, out->error);
@@ -1161,10 +1255,14 @@ static int run_loop(stbpe_engine *e, int target, const int2 *forced, int n_force
 }
 
 // host-given merges, applied in order as merges of the log
-static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t first_new, int64_t *n_matches, cudaStream_t s) {
+static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t first_new, int64_t *n_matches, cudaStream_t s,
+                      bool then_ties) {
     DevState h;
-    if (int rc_ = read_state(e, &h, s)) return rc_;
-    if ((i64)h.merges_done + n > e->cfg.max_merges) return fail(e, STBPE_E_CAPACITY, "merge log full");
+    if (!then_ties || !e->merges_known) {
+        if (int rc_ = read_state(e, &h, s)) return rc_;
+        e->merges_done = h.merges_done;
+    }
+    if ((i64)e->merges_done + n > e->cfg.max_merges) return fail(e, STBPE_E_CAPACITY, "merge log full");
     if (n > e->forced_cap) {
         dev_free(e, e->forced);
         e->forced = nullptr;
@@ -1172,8 +1270,13 @@ static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t firs
         if (c != cudaSuccess) return cuda_fail(e, c, "cudaMalloc merges");
         e->forced_cap = n;
     }
-    CK(cudaMemcpyAsync(e->forced, pairs, (size_t)n * sizeof(int2), cudaMemcpyHostToDevice, s));
-    int rc = run_loop(e, e->cfg.max_merges, e->forced, n, first_new, &h, s);
+    const void *src = pairs;
+    if ((size_t)n * sizeof(int2) <= STBPE_PINNED_BYTES - STBPE_PINNED_STATE)
+        src = memcpy((char *)e->pinned.p + STBPE_PINNED_STATE, pairs, (size_t)n * sizeof(int2));
+    CK(cudaMemcpyAsync(e->forced, src, (size_t)n * sizeof(int2), cudaMemcpyHostToDevice, s));
+    int rc = run_loop(e, e->cfg.max_merges, e->forced, n, first_new, &h, s, then_ties);
+    e->merges_known = rc == STBPE_OK;
+    e->merges_done = h.merges_done;
     if (rc == STBPE_OK && n_matches) *n_matches = h.n_matches;
     return rc;
 }
@@ -1186,6 +1289,7 @@ STBPE_VISIBLE int stbpe_train(stbpe_engine *e, int32_t n_merges, void *stream) {
     if (e->cfg.world_size > 1) return fail(e, STBPE_E_STATE, "single-rank entry point");
     DevState h;
     if (int rc_ = read_state(e, &h, s)) return rc_;
+    e->merges_known = false;
     i64 target = (i64)h.merges_done + n_merges;
     if (target > e->cfg.max_merges) target = e->cfg.max_merges;
     return run_loop(e, (int)target, nullptr, 0, 0, &h, s);
@@ -1206,6 +1310,7 @@ STBPE_VISIBLE int stbpe_train_timed(stbpe_engine *e, int32_t n_merges, float *ke
     set_target_kernel<<<1, 1, 0, s>>>(e->d, (int)target);
     CK(cudaGetLastError());
     const int todo = (int)(target - h.merges_done);
+    e->merges_known = false;
     const int P = 128;
     DevState h2;
     std::vector<cudaEvent_t> ev(4 * P);

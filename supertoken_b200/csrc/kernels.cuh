@@ -493,14 +493,11 @@ __device__ __forceinline__ void advance_or_stop(const EngineDev &e, u64 key, i64
     }
 }
 
-// Best pair of the candidate list by one CTA: as a peek into the state, or as the loop's next step.
-// peek_valid = 0 when the list has run dry or over: the host then searches a new threshold and asks again.
-__global__ void __launch_bounds__(1024) choose_kernel(EngineDev e, int advance) {
+// best pair of the candidate list, by one CTA of 1024 threads (all threads get it); false when the list has run
+// dry or over: the host then searches a new threshold and asks again
+__device__ __forceinline__ bool best_candidate(const EngineDev &e, unsigned int n, Slot &best) {
     __shared__ u64 s_k[32];
     __shared__ i64 s_c[32];
-    DevState *st = e.st;
-    if (advance && st->stopped) return;
-    const unsigned int n = st->n_cand;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     u64 bk = STBPE_EMPTY;
     i64 bc = 0;
@@ -508,24 +505,65 @@ __global__ void __launch_bounds__(1024) choose_kernel(EngineDev e, int advance) 
         const Slot x = ldcg_slot(e.table + e.cand[i]);
         if (x.count > 0 && better(x.key, x.count, bk, bc)) bk = x.key, bc = x.count;
     }
+#pragma unroll 1
+    for (int level = 0; level < 2; ++level) {
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        const u64 ok = __shfl_down_sync(0xFFFFFFFFu, bk, d);
-        const i64 oc = __shfl_down_sync(0xFFFFFFFFu, bc, d);
-        if (better(ok, oc, bk, bc)) bk = ok, bc = oc;
+        for (int d = 16; d > 0; d >>= 1) {
+            const u64 ok = __shfl_xor_sync(0xFFFFFFFFu, bk, d);
+            const i64 oc = __shfl_xor_sync(0xFFFFFFFFu, bc, d);
+            if (better(ok, oc, bk, bc)) bk = ok, bc = oc;
+        }
+        if (level == 0) {
+            if (lane == 0) s_k[warp] = bk, s_c[warp] = bc;
+            __syncthreads();
+            bk = s_k[lane], bc = s_c[lane];
+        }
     }
-    if (lane == 0) s_k[warp] = bk, s_c[warp] = bc;
+    best.key = bk;
+    best.count = bc;
+    Theta t;
+    t.count = e.st->theta_count, t.key = e.st->theta_key;
+    return e.st->cand_state == STBPE_CAND_READY && n <= STBPE_CAND_CAP && (t.admits(bc, bk) || (bc <= 0 && t.count == 0));
+}
+
+// best pair as a peek into the state, or as the loop's next step
+__global__ void __launch_bounds__(1024) choose_kernel(EngineDev e, int advance) {
+    DevState *st = e.st;
+    if (advance && st->stopped) return;
+    Slot best;
+    const bool valid = best_candidate(e, st->n_cand, best);
+    if (threadIdx.x != 0) return;
+    st->peek_valid = valid;
+    st->peek_key = best.key;
+    st->peek_count = best.count;
+    if (advance && valid) advance_or_stop(e, best.key, best.count);
+}
+
+// Best count and the keys that hold it, behind the state (a key may appear twice: the list may name it twice).
+// peek_ties = 0 when the list need not hold all of them (the threshold lies inside that count).
+__global__ void __launch_bounds__(1024) ties_kernel(EngineDev e) {
+    __shared__ int s_n;
+    DevState *st = e.st;
+    u64 *out = reinterpret_cast<u64 *>(reinterpret_cast<unsigned char *>(st) + STBPE_TIES_OFFSET);
+    const unsigned int n = st->n_cand;
+    if (threadIdx.x == 0) s_n = 0;
+    Slot best;
+    const bool valid = best_candidate(e, n, best);
+    if (valid && best.count > st->theta_count) {
+        for (unsigned int i = threadIdx.x; i < n; i += blockDim.x) {
+            const Slot x = ldcg_slot(e.table + e.cand[i]);
+            if (x.count == best.count && x.count > 0) {
+                const int j = atomicAdd(&s_n, 1);
+                if (j < STBPE_TIES_CAP) out[j] = x.key;
+            }
+        }
+    }
     __syncthreads();
     if (threadIdx.x != 0) return;
-    for (int w = 1; w < (int)blockDim.x / 32; ++w)
-        if (better(s_k[w], s_c[w], bk, bc)) bk = s_k[w], bc = s_c[w];
-    Theta t;
-    t.count = st->theta_count, t.key = st->theta_key;
-    const bool valid = st->cand_state == STBPE_CAND_READY && n <= STBPE_CAND_CAP && (t.admits(bc, bk) || (bc <= 0 && t.count == 0));
     st->peek_valid = valid;
-    st->peek_key = bk;
-    st->peek_count = bc;
-    if (advance && valid) advance_or_stop(e, bk, bc);
+    st->peek_key = best.key;
+    st->peek_count = best.count;
+    st->peek_ties = s_n;
 }
 
 #define STBPE_SELECT_THREADS 256

@@ -8,6 +8,7 @@
 #include <string>
 
 #include "../../include/stbpe.h"
+#include "block_cache.h"
 #include "common.cuh"
 
 #define STBPE_VISIBLE __attribute__((visibility("default")))
@@ -96,6 +97,167 @@ __global__ void rows_write_kernel(const u64 *__restrict__ keys, const i64 *__res
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0 && length) *length = n;
+}
+
+// ---- stbpe_rows_count_pairs
+#define ROWS_COUNT_NT 256
+#define ROWS_SMEM_SLOTS 2048
+#define ROWS_RANK_MAX 16384   // up to this many pairs are sorted by counting smaller keys, two launches instead of a radix sort's nine
+#define ROWS_RANK_TILE 2048
+
+__global__ void rows_init_kernel(RowsTable t, unsigned int *rank, unsigned int n_rank) {
+    const u64 first = (u64)blockIdx.x * blockDim.x + threadIdx.x, step = (u64)gridDim.x * blockDim.x;
+    Slot s;
+    s.key = STBPE_EMPTY;
+    s.count = 0;
+    for (u64 i = first; i <= t.mask; i += step) t.table[i] = s;
+    for (u64 i = first; i < n_rank; i += step) rank[i] = 0u;
+    if (first < 3) t.n_keys[first] = 0;  // number of keys, error, export cursor
+}
+
+// key + n into the table; a table that fills up ends the count (the host repeats it with a larger one)
+__device__ __forceinline__ void rows_add(const RowsTable &t, u64 key, u64 n) {
+    u64 h = mix64(key) & t.mask;
+#pragma unroll 1
+    for (int probe = 0; probe < 64; ++probe) {
+        Slot *s = &t.table[h];
+        u64 k = __ldcg(&s->key);
+        if (k == STBPE_EMPTY) {
+            k = atomicCAS(&s->key, STBPE_EMPTY, key);
+            if (k == STBPE_EMPTY) {
+                if (atomicAdd(t.n_keys, 1ull) >= (t.mask + 1) / 4 * 3) atomicOr(t.error, 1u);
+                k = key;
+            }
+        }
+        if (k == key) {
+            atomicAdd((u64 *)&s->count, n);
+            return;
+        }
+        h = (h + 1) & t.mask;
+    }
+    atomicOr(t.error, 1u);
+}
+
+// A pair (i, i+1) of a row counts when both positions are valid (gpu_tokenizer/utils.py:586).  Four cells per thread
+// and step as one 16-byte and one 4-byte load over the flat batch; a CTA collects its pairs in shared memory
+// and adds each distinct one once.
+__global__ void __launch_bounds__(ROWS_COUNT_NT) rows_pairs_kernel(const int32_t *__restrict__ tokens, const uint8_t *__restrict__ valid,
+                                                                   i64 B, i64 L, RowsTable t) {
+    __shared__ u64 s_key[ROWS_SMEM_SLOTS];
+    __shared__ int s_val[ROWS_SMEM_SLOTS];
+    for (int i = threadIdx.x; i < ROWS_SMEM_SLOTS; i += ROWS_COUNT_NT) s_key[i] = STBPE_EMPTY, s_val[i] = 0;
+    __syncthreads();
+    const i64 cells = B * L;
+    const int lane = threadIdx.x & 31;
+    const bool aligned = (((uintptr_t)tokens & 15) | ((uintptr_t)valid & 3)) == 0;
+    const i64 step = (i64)gridDim.x * ROWS_COUNT_NT * 4;
+    i64 q = ((i64)blockIdx.x * ROWS_COUNT_NT + threadIdx.x) * 4;
+    for (i64 q0 = (i64)blockIdx.x * ROWS_COUNT_NT * 4; q0 < cells; q0 += step, q += step) {  // uniform per CTA
+        int32_t w[5] = {0, 0, 0, 0, 0};
+        unsigned int v[5] = {0, 0, 0, 0, 0};
+        if (aligned && q + 4 <= cells) {
+            const int4 x = __ldg(reinterpret_cast<const int4 *>(tokens + q));
+            const uchar4 y = __ldg(reinterpret_cast<const uchar4 *>(valid + q));
+            w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w;
+            v[0] = y.x, v[1] = y.y, v[2] = y.z, v[3] = y.w;
+        } else {
+            for (int k = 0; k < 4; ++k)
+                if (q + k < cells) w[k] = tokens[q + k], v[k] = valid[q + k];
+        }
+        w[4] = __shfl_down_sync(0xFFFFFFFFu, w[0], 1);
+        v[4] = __shfl_down_sync(0xFFFFFFFFu, v[0], 1);
+        if (lane == 31 && q + 4 < cells) w[4] = tokens[q + 4], v[4] = valid[q + 4];
+        i64 col = q < cells ? q - q / L * L : 0;  // column of the first cell
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const bool last = ++col == L;  // the row ends here
+            if (last) col = 0;
+            if (last || !v[k] || !v[k + 1]) continue;
+            const u64 key = ((u64)(uint32_t)w[k] << 32) | (u64)(uint32_t)w[k + 1];
+            unsigned int h = hash32(key) & (ROWS_SMEM_SLOTS - 1);
+            bool done = false;
+#pragma unroll 1
+            for (int probe = 0; probe < 4 && !done; ++probe) {
+                u64 x = lds_u64_volatile(&s_key[h]);
+                if (x == STBPE_EMPTY) {
+                    x = atoms_cas_u64(&s_key[h], STBPE_EMPTY, key);
+                    if (x == STBPE_EMPTY) x = key;
+                }
+                if (x == key) {
+                    reds_add_s32(&s_val[h], 1);
+                    done = true;
+                }
+                h = (h + 1) & (ROWS_SMEM_SLOTS - 1);
+            }
+            if (!done && !(*(volatile unsigned int *)t.error)) rows_add(t, key, 1ull);
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < ROWS_SMEM_SLOTS; i += ROWS_COUNT_NT)
+        if (s_val[i] && !(*(volatile unsigned int *)t.error)) rows_add(t, s_key[i], (u64)s_val[i]);
+}
+
+// rank[i] += keys of the tile blockIdx.y that are smaller than key i
+__global__ void __launch_bounds__(256) rows_rank_kernel(const u64 *__restrict__ keys, const u64 *n_keys, const unsigned int *error, unsigned int *rank) {
+    __shared__ u64 s_k[ROWS_RANK_TILE];
+    const i64 n = (i64)*n_keys;
+    const i64 i = (i64)blockIdx.x * 256 + threadIdx.x, j0 = (i64)blockIdx.y * ROWS_RANK_TILE;
+    if (*error || n > ROWS_RANK_MAX || (i64)blockIdx.x * 256 >= n || j0 >= n) return;
+    const int m = (int)(n - j0 < ROWS_RANK_TILE ? n - j0 : ROWS_RANK_TILE);
+    for (int k = threadIdx.x; k < ROWS_RANK_TILE; k += 256) s_k[k] = k < m ? keys[j0 + k] : STBPE_EMPTY;
+    __syncthreads();
+    if (i >= n) return;
+    const u64 mine = keys[i];
+    unsigned int r = 0;
+#pragma unroll 8
+    for (int k = 0; k < ((m + 7) & ~7); ++k) r += s_k[k] < mine ? 1u : 0u;
+    if (r) atomicAdd(&rank[i], r);
+}
+
+// the histogram in ascending key order, unused rows -1 / 0, length (gpu_tokenizer/utils.py:622-635)
+__global__ void rows_place_kernel(const u64 *__restrict__ keys, const i64 *__restrict__ counts, const unsigned int *__restrict__ rank, RowsTable t,
+                                  int32_t *pair_keys, i64 *pair_counts, i64 cap, i64 *length) {
+    const i64 n = (i64)*t.n_keys;
+    if (*t.error || n > cap || n > ROWS_RANK_MAX) return;
+    const i64 first = (i64)blockIdx.x * blockDim.x + threadIdx.x, step = (i64)gridDim.x * blockDim.x;
+    for (i64 i = first; i < n; i += step) {
+        const i64 at = rank[i];
+        pair_keys[2 * at] = (int32_t)(keys[i] >> 32);
+        pair_keys[2 * at + 1] = (int32_t)(keys[i] & 0xFFFFFFFFull);
+        pair_counts[at] = counts[i];
+    }
+    for (i64 i = n + first; i < cap; i += step) {
+        if (((uintptr_t)pair_keys & 7) == 0) {
+            *reinterpret_cast<int2 *>(pair_keys + 2 * i) = make_int2(-1, -1);
+        } else {
+            pair_keys[2 * i] = -1;
+            pair_keys[2 * i + 1] = -1;
+        }
+        pair_counts[i] = 0;
+    }
+    if (first == 0 && length) *length = n;
+}
+
+// best of n entries (per CTA): key, count, index into out[blockIdx.x], out[256 + ...], out[512 + ...]
+__global__ void __launch_bounds__(256) rows_best_kernel(const i64 *keys, const i64 *counts, const i64 *index, i64 n, i64 *out) {
+    __shared__ i64 s_k[8], s_c[8], s_i[8];
+    i64 bk = 0x7FFFFFFFFFFFFFFFll, bc = 0, bi = 0x7FFFFFFFFFFFFFFFll;
+    auto take = [&](i64 k, i64 c, i64 i) {
+        if (c > bc || (c == bc && (k < bk || (k == bk && i < bi)))) bk = k, bc = c, bi = i;
+    };
+    for (i64 i = (i64)blockIdx.x * 256 + threadIdx.x; i < n; i += (i64)gridDim.x * 256) take(keys[i], counts[i], index ? index[i] : i);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        const i64 k = __shfl_down_sync(0xFFFFFFFFu, bk, d), c = __shfl_down_sync(0xFFFFFFFFu, bc, d), i = __shfl_down_sync(0xFFFFFFFFu, bi, d);
+        take(k, c, i);
+    }
+    if ((threadIdx.x & 31) == 0) s_k[threadIdx.x >> 5] = bk, s_c[threadIdx.x >> 5] = bc, s_i[threadIdx.x >> 5] = bi;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < 8; ++w) take(s_k[w], s_c[w], s_i[w]);
+    out[blockIdx.x] = bk;
+    out[256 + blockIdx.x] = bc;
+    out[512 + blockIdx.x] = bi;
 }
 
 // One CTA per row, walking the row in chunks with a running output offset.  Writes never
@@ -218,66 +380,112 @@ STBPE_VISIBLE int stbpe_rows_count_pairs(const int32_t *tokens, const uint8_t *v
     cudaStream_t s = (cudaStream_t)stream;
     if (B < 0 || L < 0 || cap < 0) return STBPE_E_BADARG;
     const i64 total = (B > 0 && L > 1) ? B * (L - 1) : 0;
-    u64 *keys = nullptr, *skeys = nullptr, *meta = nullptr;
-    i64 *counts = nullptr, *scounts = nullptr;
-    Slot *table = nullptr;
-    i64 n = 0;
+    int dev = 0;
+    RCK(cudaGetDevice(&dev));
+    // A batch of text holds a few thousand distinct pairs among millions of positions, so the table starts at 2^16
+    // slots (1 MB, cleared and scanned in microseconds; for twice the positions it was 512 MB on a batch of
+    // 2048 x 4096) and the count is repeated with sixteen times the slots when the pairs do not fit.
+    u64 largest = 1024;
+    while (largest < (u64)total * 2 && largest < (1ull << 28)) largest <<= 1;
+    u64 slots = largest < (1u << 16) ? largest : (1u << 16);
+    stbpe::Block pin;
+    RCK(stbpe::pinned_blocks().get(0, 4096, &pin));
+    volatile u64 *got = (volatile u64 *)pin.p;
     int rc = STBPE_OK;
-    if (total > 0) {
-        u64 slots = 1024;
-        while (slots < (u64)total * 2 && slots < (1ull << 28)) slots <<= 1;
-        RCK(cudaMallocAsync((void **)&table, slots * sizeof(Slot), s));
-        RCK(cudaMallocAsync((void **)&meta, 2 * sizeof(u64), s));
-        RCK(cudaMemsetAsync(meta, 0, 2 * sizeof(u64), s));
-        RowsTable t;
-        t.table = table;
-        t.mask = slots - 1;
-        t.n_keys = meta;
-        t.error = reinterpret_cast<unsigned int *>(meta + 1);
-        rows_clear_kernel<<<592, 256, 0, s>>>(t);
-        i64 blocks = (total + 255) / 256;
-        if (blocks > 148 * 32) blocks = 148 * 32;
-        rows_count_kernel<<<(unsigned int)blocks, 256, 0, s>>>(tokens, valid, B, L, t);
-        RCK(cudaGetLastError());
-        u64 hmeta[2];
-        RCK(cudaMemcpyAsync(hmeta, meta, sizeof(hmeta), cudaMemcpyDeviceToHost, s));
-        RCK(cudaStreamSynchronize(s));
-        n = (i64)hmeta[0];
-        if ((hmeta[1] & 0xFFFFFFFFull) != 0 || n > cap) {
-            rc = STBPE_E_CAPACITY;  // "pair workspace capacity exceeded" (utils.py:619-620)
-            n = 0;
-        } else if (n > 0) {
-            RCK(cudaMallocAsync((void **)&keys, n * sizeof(u64), s));
-            RCK(cudaMallocAsync((void **)&counts, n * sizeof(i64), s));
-            RCK(cudaMallocAsync((void **)&skeys, n * sizeof(u64), s));
-            RCK(cudaMallocAsync((void **)&scounts, n * sizeof(i64), s));
-            RCK(cudaMemsetAsync(meta, 0, sizeof(u64), s));
-            rows_export_kernel<<<592, 256, 0, s>>>(t, keys, counts, meta, n);
-            size_t tmp_bytes = 0;
-            cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, skeys, counts, scounts, (int)n, 0, 64, s);
-            void *tmp = nullptr;
-            RCK(cudaMallocAsync(&tmp, tmp_bytes ? tmp_bytes : 16, s));
-            cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, skeys, counts, scounts, (int)n, 0, 64, s);
-            RCK(cudaGetLastError());
-            RCK(cudaFreeAsync(tmp, s));
+    for (;;) {
+        const u64 most = slots < (u64)(total > 0 ? total : 1) ? slots : (u64)(total > 0 ? total : 1);
+        const size_t keys_at = slots * sizeof(Slot), counts_at = keys_at + most * 8, rank_at = counts_at + most * 8,
+                     meta_at = (rank_at + most * 4 + 255) & ~(size_t)255;
+        stbpe::Block b;
+        cudaError_t c = stbpe::device_blocks().get(dev, meta_at + 256, &b);
+        if (c == cudaSuccess) {
+            unsigned char *base = (unsigned char *)b.p;
+            RowsTable t;
+            t.table = (Slot *)base;
+            t.mask = slots - 1;
+            t.n_keys = (u64 *)(base + meta_at);
+            t.error = (unsigned int *)(t.n_keys + 1);
+            u64 *n_out = t.n_keys + 2;
+            u64 *keys = (u64 *)(base + keys_at);
+            i64 *counts = (i64 *)(base + counts_at);
+            unsigned int *rank = (unsigned int *)(base + rank_at);
+            const i64 quads = (B * L + 3) / 4;
+            const i64 want = (quads + ROWS_COUNT_NT - 1) / ROWS_COUNT_NT, most_ctas = 148 * 4;
+            rows_init_kernel<<<slots < (1u << 18) ? 64 : 592, 256, 0, s>>>(t, rank, (unsigned int)(most < ROWS_RANK_MAX ? most : ROWS_RANK_MAX));
+            if (total > 0) rows_pairs_kernel<<<(unsigned int)(want < most_ctas ? want : most_ctas), ROWS_COUNT_NT, 0, s>>>(tokens, valid, B, L, t);
+            if (total > 0) rows_export_kernel<<<slots < (1u << 18) ? 64 : 592, 256, 0, s>>>(t, keys, counts, n_out, (i64)most);
+            if (total > 0) rows_rank_kernel<<<dim3(ROWS_RANK_MAX / 256, ROWS_RANK_MAX / ROWS_RANK_TILE), 256, 0, s>>>(keys, t.n_keys, t.error, rank);
+            i64 wb = (cap + 255) / 256;
+            if (wb > 148 * 16) wb = 148 * 16;
+            rows_place_kernel<<<(unsigned int)(wb > 0 ? wb : 1), 256, 0, s>>>(keys, counts, rank, t, pair_keys, (i64 *)pair_counts, cap, (i64 *)length_dev);
+            c = cudaGetLastError();
+            if (c == cudaSuccess) c = cudaMemcpyAsync(pin.p, t.n_keys, 2 * sizeof(u64), cudaMemcpyDeviceToHost, s);
+            if (c == cudaSuccess) c = cudaStreamSynchronize(s);
+            if (c == cudaSuccess) {
+                const i64 n = (i64)got[0];
+                const bool full = (got[1] & 0xFFFFFFFFull) != 0;
+                if (full && slots < largest) {
+                    stbpe::device_blocks().put(dev, b);
+                    slots = slots * 16 < largest ? slots * 16 : largest;
+                    continue;
+                }
+                if (full || n > cap) {
+                    rc = STBPE_E_CAPACITY;  // "pair workspace capacity exceeded" (utils.py:619-620)
+                } else if (n > ROWS_RANK_MAX) {
+                    // many pairs: radix sort
+                    size_t tmp = 0;
+                    cub::DeviceRadixSort::SortPairs(nullptr, tmp, keys, keys, counts, counts, (int)n, 0, 64, s);
+                    stbpe::Block w;
+                    const size_t side = ((size_t)n * 8 + 255) & ~(size_t)255;
+                    c = stbpe::device_blocks().get(dev, 2 * side + tmp + 256, &w);
+                    if (c == cudaSuccess) {
+                        u64 *sk = (u64 *)w.p;
+                        i64 *sc = (i64 *)((unsigned char *)w.p + side);
+                        cub::DeviceRadixSort::SortPairs((unsigned char *)w.p + 2 * side, tmp, keys, sk, counts, sc, (int)n, 0, 64, s);
+                        rows_write_kernel<<<(unsigned int)(wb > 0 ? wb : 1), 256, 0, s>>>(sk, sc, n, pair_keys, (i64 *)pair_counts, cap, (i64 *)length_dev);
+                        c = cudaGetLastError();
+                        if (c == cudaSuccess) c = cudaStreamSynchronize(s);
+                        if (c == cudaSuccess) stbpe::device_blocks().put(dev, w);
+                    }
+                }
+            }
         }
-        RCK(cudaFreeAsync(table, s));
-        RCK(cudaFreeAsync(meta, s));
+        if (c != cudaSuccess) {  // the blocks may still be in use: they are not handed on
+            g_rows_err = cudaGetErrorString(c);
+            cudaGetLastError();
+            return STBPE_E_CUDA;
+        }
+        stbpe::device_blocks().put(dev, b);
+        break;
     }
-    if (rc == STBPE_OK && cap > 0) {
-        i64 blocks = (cap + 255) / 256;
-        if (blocks > 148 * 32) blocks = 148 * 32;
-        rows_write_kernel<<<(unsigned int)blocks, 256, 0, s>>>(skeys, scounts, n, pair_keys, (i64 *)pair_counts, cap, (i64 *)length_dev);
-        RCK(cudaGetLastError());
-    } else if (rc == STBPE_OK && length_dev) {
-        RCK(cudaMemsetAsync(length_dev, 0, sizeof(i64), s));
-    }
-    if (keys) RCK(cudaFreeAsync(keys, s));
-    if (counts) RCK(cudaFreeAsync(counts, s));
-    if (skeys) RCK(cudaFreeAsync(skeys, s));
-    if (scounts) RCK(cudaFreeAsync(scounts, s));
-    RCK(cudaStreamSynchronize(s));
+    stbpe::pinned_blocks().put(0, pin);
     return rc;
+}
+
+// Best entry of a histogram: maximum count, ties to the smallest key (gpu_tokenizer/trainers/bpe_gpu.py:106-127).
+STBPE_VISIBLE int stbpe_select_pair(const int64_t *keys, const int64_t *counts, int64_t n, int64_t *key, int64_t *count, int64_t *index,
+                                    void *stream) {
+    cudaStream_t s = (cudaStream_t)stream;
+    if (n < 0 || !key || !count || !index || (n > 0 && (!keys || !counts))) return STBPE_E_BADARG;
+    *key = 0, *count = 0, *index = -1;
+    if (n == 0) return STBPE_OK;
+    int dev = 0;
+    RCK(cudaGetDevice(&dev));
+    stbpe::Block b, pin;
+    RCK(stbpe::device_blocks().get(dev, 65536, &b));
+    RCK(stbpe::pinned_blocks().get(0, 4096, &pin));
+    const i64 want = (n + 1023) / 1024;
+    const int grid = (int)(want < 148 ? want : 148);
+    rows_best_kernel<<<grid, 256, 0, s>>>((const i64 *)keys, (const i64 *)counts, nullptr, n, (i64 *)b.p);
+    if (grid > 1) rows_best_kernel<<<1, 256, 0, s>>>((const i64 *)b.p, (const i64 *)b.p + 256, (const i64 *)b.p + 512, grid, (i64 *)b.p);
+    RCK(cudaGetLastError());
+    i64 *h = (i64 *)pin.p;
+    for (int k = 0; k < 3; ++k) RCK(cudaMemcpyAsync(h + k, (i64 *)b.p + 256 * k, sizeof(i64), cudaMemcpyDeviceToHost, s));
+    RCK(cudaStreamSynchronize(s));
+    if (h[1] > 0) *key = h[0], *count = h[1], *index = h[2];
+    stbpe::device_blocks().put(dev, b);
+    stbpe::pinned_blocks().put(0, pin);
+    return STBPE_OK;
 }
 
 STBPE_VISIBLE int stbpe_rows_apply_merge(int32_t *tokens, uint8_t *valid, int32_t *lengths, int64_t B,

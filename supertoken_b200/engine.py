@@ -121,6 +121,33 @@ class Engine:
         self._check(self._lib.stbpe_apply_merge(self._h, a, b, new_id, ctypes.byref(n), self._s))
         return int(n.value)
 
+    def apply_merges(self, pairs: Sequence[Tuple[int, int]], first_new_id: int):
+        """``apply_merge`` for every pair in order (new ids count up from ``first_new_id``), in one call."""
+        if not pairs:
+            return
+        if max(max(a, b) for a, b in pairs) > 0x7FFFFFFE or min(min(a, b) for a, b in pairs) < 0 or \
+                not 0 <= first_new_id <= 0x7FFFFFFE - (len(pairs) - 1):
+            raise OverflowError("Token id overflow: ids must be in [0, 2^31-2]")
+        p = np.asarray(pairs, dtype=np.int32)
+        self._check(self._lib.stbpe_apply_merges(self._h, p.ctypes.data, len(p), int(first_new_id), self._s))
+
+    def next_tied(self, merge: Optional[Tuple[int, int, int]] = None) -> Tuple[int, List[int]]:
+        """Apply ``merge`` = (a, b, new_id), if given, then return the best count and the keys that hold it,
+        ascending: one step of a loop that breaks ties on the host."""
+        a, b, new_id = merge if merge is not None else (0, 0, -1)
+        if max(a, b, new_id) > 0x7FFFFFFE or min(a, b) < 0:
+            raise OverflowError("Token id overflow: ids must be in [0, 2^31-2]")
+        if getattr(self, "_tied", None) is None:
+            self._tied = np.empty(1024, dtype=np.uint64)
+        count, n = ctypes.c_int64(0), ctypes.c_int64(0)
+        self._check(self._lib.stbpe_next_tied(self._h, a, b, new_id, ctypes.byref(count), self._tied.ctypes.data,
+                                              len(self._tied), ctypes.byref(n), self._s))
+        if count.value <= 0:
+            return 0, []
+        if n.value > len(self._tied):
+            return int(count.value), self.tied_keys(int(count.value), int(n.value))
+        return int(count.value), self._tied[:n.value].tolist()
+
     def train(self, n_merges: int):
         self._check(self._lib.stbpe_train(self._h, int(n_merges), self._s))
 

@@ -81,7 +81,10 @@ def apply_merge_once(seqs: torch.Tensor, valid: torch.Tensor, lengths: torch.Ten
     if B == 0:
         lengths.zero_()
         return seqs, valid, lengths, spans
-    out_len = torch.zeros(B, dtype=torch.int32, device=seqs.device)
+    direct = lengths.dtype == torch.int32 and lengths.is_contiguous() and lengths.numel() == B
+    out_len = lengths if direct else torch.empty(B, dtype=torch.int32, device=seqs.device)
+    if Lw == 0:
+        out_len.zero_()
     with torch.cuda.device(seqs.device):
         st = L.load().stbpe_rows_apply_merge(seqs.data_ptr(), valid.data_ptr(), out_len.data_ptr(), B, Lw,
                                             int(a_id), int(b_id), int(new_id),
@@ -94,7 +97,8 @@ def apply_merge_once(seqs: torch.Tensor, valid: torch.Tensor, lengths: torch.Ten
         if overflow_workspace is not None:
             overflow_workspace.copy_(out_len > 65535)
     else:
-        lengths.copy_(out_len.to(lengths.dtype))
+        if not direct:
+            lengths.copy_(out_len.to(lengths.dtype))
         if overflow_workspace is not None:
             overflow_workspace.zero_()
     if span_workspace is not None and span_workspace.shape == spans.shape:
@@ -127,6 +131,15 @@ def select_best_pair(histogram: PairHistogramResult, *,
     if histogram.is_empty():
         return None, 0, None
     counts, keys = histogram.counts, histogram.keys
+    if tie_breaker is None and counts.is_cuda and keys.is_cuda and counts.dtype == keys.dtype == torch.int64 and \
+            counts.is_contiguous() and keys.is_contiguous() and counts.numel() == keys.numel():
+        key, count, index = ctypes.c_int64(0), ctypes.c_int64(0), ctypes.c_int64(0)
+        with torch.cuda.device(counts.device):
+            st = L.load().stbpe_select_pair(keys.data_ptr(), counts.data_ptr(), counts.numel(), ctypes.byref(key),
+                                            ctypes.byref(count), ctypes.byref(index), _stream(counts))
+        if st != L.OK:
+            raise RuntimeError(f"stbpe_select_pair failed with status {st}")
+        return (None, 0, None) if index.value < 0 else (key.value, count.value, index.value)
     best = int(counts.max().item())
     if best <= 0:
         return None, 0, None
