@@ -250,14 +250,14 @@ __device__ __forceinline__ unsigned int hash32(u64 key) {
     return h;
 }
 
-// first slot probed for a key: its partition's slice in the top bits, then the top bits of a 32-bit hash (32-bit
-// arithmetic: the 64-bit finaliser cost a fifth of the time of a merge's table adds)
-__device__ __forceinline__ u64 slot_in_slice(const EngineDev &e, u64 top, u64 key) {
-    return top | (u64)(hash32(key) >> (32 - e.slot_bits));
+// First slot probed for a key: its partition's slice, then the bits of the mix below the partition's.  With one
+// rank that is the mixed word shifted right, so the slots of a range of words are contiguous (wide_count.cuh
+// builds the table range by range).
+__device__ __forceinline__ u64 slot_of_word(const EngineDev &e, uint32_t word) {
+    const u64 top = (u64)slice_of(e, word >> (32 - STBPE_PART_BITS)) << e.slot_bits;
+    return top | (u64)((word << STBPE_PART_BITS) >> (32 - e.slot_bits));
 }
-__device__ __forceinline__ u64 slot_of(const EngineDev &e, u64 key) {
-    return slot_in_slice(e, (u64)slice_of(e, part_of(key)) << e.slot_bits, key);
-}
+__device__ __forceinline__ u64 slot_of(const EngineDev &e, u64 key) { return slot_of_word(e, mix32(fold_key(key))); }
 
 __device__ __forceinline__ bool better(u64 k1, i64 c1, u64 k2, i64 c2) {
     // (k1, c1) beats (k2, c2): larger count, ties to the smaller packed key

@@ -81,6 +81,7 @@ struct stbpe_engine {
     std::vector<stbpe::Block> allocs;
     bool broken;          // a CUDA call failed: work of this engine may still be pending
     stbpe::Block pinned;  // host side of small transfers: the device state, then small inputs
+    bool foreign_ids;     // a merge of the caller's may have brought an id of 65 536 or more
     unsigned int max_id;  // largest id appended through stbpe_append_ids
     unsigned int load_err;  // error bits of the rows appended so far
     bool merges_known;    // merges_done mirrors the device (several host-driven merges in a row)
@@ -277,6 +278,8 @@ static const DeviceInfo &device_info(int dev) {
     SMEM(count_dense_kernel<uint32_t>, 32768 * 4);
     SMEM(partition_pairs_kernel<uint16_t>, STBPE_PART_SMEM_BYTES);
     SMEM(partition_pairs_kernel<uint32_t>, STBPE_PART_SMEM_BYTES);
+    SMEM(sub_partition_kernel, STBPE_SUB_CHUNK * sizeof(uint32_t));
+    SMEM(build_table_kernel, 8 << 14);
     SMEM(presence_rebuild_kernel<uint16_t>, STBPE_PROWS * sizeof(unsigned int));
     SMEM(presence_rebuild_kernel<uint32_t>, STBPE_PROWS * sizeof(unsigned int));
 #undef SMEM
@@ -325,7 +328,7 @@ static void drop_stream(stbpe_engine *e) {
     e->filter_valid = false;
     e->wide_counted = e->full_refresh_pending = false;
     e->load_err = e->max_id = 0;
-    e->merges_known = false;
+    e->merges_known = e->foreign_ids = false;
     e->state_stale = true;
 }
 
@@ -725,7 +728,7 @@ static int grow_table(stbpe_engine *e, cudaStream_t s) {
 }
 
 // what every count starts with: tile records of a fresh stream, an empty table, no maxima
-static int count_prologue(stbpe_engine *e, cudaStream_t s) {
+static int count_prologue(stbpe_engine *e, bool clear, cudaStream_t s) {
     const bool fresh = e->recs_stale;
     e->convert_ms = e->count_ms = 0.f;
     e->count_timed = false;
@@ -740,7 +743,7 @@ static int count_prologue(stbpe_engine *e, cudaStream_t s) {
         rc = set_table(e, want);
         if (rc != STBPE_OK) return rc;
     }
-    clear_table_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d);
+    if (clear) clear_table_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d);
     CK(cudaGetLastError());
     if (e->cfg.world_size > 1) {
         CK(cudaMemsetAsync(e->d.dirty_bits, 0, (e->d.n_blocks + 31) / 32 * sizeof(unsigned int), s));
@@ -758,7 +761,7 @@ static int count_prologue(stbpe_engine *e, cudaStream_t s) {
 }
 
 static bool wide_eligible(const stbpe_engine *e, bool fresh) {
-    return e->d.n_tiles > 0 && fresh && !e->only_bytes && e->cfg.base_vocab <= 65536 &&
+    return e->n_tokens > 0 && e->n_tokens < (1ll << 32) && e->slots <= (1ull << 30) && fresh && !e->only_bytes && e->cfg.base_vocab <= 65536 &&
            e->n_tokens >= e->dense32_min && !getenv("STBPE_NO_DENSE_COUNT");
 }
 
@@ -787,13 +790,57 @@ static int wide_pass1(stbpe_engine *e, int *ok, cudaStream_t s) {
     return STBPE_OK;
 }
 
+// second and third pass of the partitioned count; *ok = 0 when the spill list ran over
+static int wide_build(stbpe_engine *e, int *ok, cudaStream_t s) {
+    const PartBuffers &pb = e->parts;
+    int lg = 0;
+    while ((1ull << lg) < e->slots) ++lg;
+    // ranges of 2^13 slots: 64 KB of shared memory, three CTAs per SM; at least one bit and at most eight bits of
+    // ordering, so small tables get smaller ranges and the largest (2^30 slots) larger ones
+    int task_bits = lg - STBPE_PART_BITS - 1 < 13 ? lg - STBPE_PART_BITS - 1 : 13;
+    if (lg - STBPE_PART_BITS - task_bits > STBPE_SUB_MAX_BITS) task_bits = lg - STBPE_PART_BITS - STBPE_SUB_MAX_BITS;
+    const int sub_bits = lg - STBPE_PART_BITS - task_bits;
+    const int cpr = (int)((pb.cap + STBPE_SUB_CHUNK - 1) / STBPE_SUB_CHUNK);
+    const i64 n_chunks = (i64)STBPE_PARTS * pb.n_cta * cpr;
+    const unsigned int spill_cap = 1u << 20;
+    const size_t offs_bytes = ((size_t)n_chunks * ((1 << sub_bits) + 1) * sizeof(uint16_t) + 255) & ~(size_t)255;
+    unsigned char *scratch = nullptr;
+    CK(dev_alloc(e, &scratch, offs_bytes + (size_t)spill_cap * sizeof(uint32_t) + 256));
+    uint16_t *offs = (uint16_t *)scratch;
+    unsigned int *n_spill = (unsigned int *)(scratch + offs_bytes);
+    uint32_t *spill = (uint32_t *)(scratch + offs_bytes + 256);
+    const size_t build_smem = (size_t)8 << task_bits;
+    CK(cudaEventRecord(e->ev0, s));
+    CK(cudaMemsetAsync(n_spill, 0, sizeof(*n_spill), s));
+    sub_partition_kernel<<<e->sm_count * 3, STBPE_SUB_THREADS, STBPE_SUB_CHUNK * sizeof(uint32_t), s>>>(pb, cpr, sub_bits, offs);
+    build_table_kernel<<<e->sm_count * (build_smem > 65536 ? 1 : 3), STBPE_BUILD_THREADS, build_smem, s>>>(e->d, pb, cpr, sub_bits, task_bits, offs, spill,
+                                                                                                   n_spill, spill_cap);
+    spill_to_table_kernel<<<e->sm_count, 256, 0, s>>>(e->d, spill, n_spill, spill_cap);
+    dense_to_table_kernel<false><<<256, 256, 0, s>>>(e->d, e->wide_dense);
+    CK(cudaGetLastError());
+    CK(cudaEventRecord(e->ev1, s));
+    unsigned int *derr = (unsigned int *)e->pinned.p;
+    CK(cudaMemcpyAsync(derr, &e->d.st->error, sizeof(*derr), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    dev_free(e, scratch);
+    CK(cudaEventElapsedTime(&e->convert_ms, e->ev0, e->ev1));
+    e->count_ms += e->convert_ms;  // the pair table is complete only after all passes
+    *ok = (*derr & STBPE_DERR_DENSE_OVERFLOW) == 0;
+    if (!*ok) {
+        *derr &= ~STBPE_DERR_DENSE_OVERFLOW;
+        CK(cudaMemcpyAsync(&e->d.st->error, derr, sizeof(*derr), cudaMemcpyHostToDevice, s));
+        CK(cudaStreamSynchronize(s));
+    }
+    return STBPE_OK;
+}
+
 static int launch_count(stbpe_engine *e, bool mg, cudaStream_t s) {
     if (mg && e->wide_counted) {  // stbpe_mg_wide_pass2 has filled the table already
         e->wide_counted = false;
         return STBPE_OK;
     }
-    const bool fresh = e->recs_stale;
-    int rc = count_prologue(e, s);
+    const bool fresh = e->recs_stale, wide = !mg && wide_eligible(e, fresh);
+    int rc = count_prologue(e, !wide, s);  // the partitioned count writes every slot of the table itself
     if (rc != STBPE_OK) return rc;
     if (e->d.n_tiles > 0 && fresh && e->only_bytes && !getenv("STBPE_NO_DENSE_COUNT")) {
         // byte-level fast path: dense stream, ids < 256
@@ -821,38 +868,25 @@ static int launch_count(stbpe_engine *e, bool mg, cudaStream_t s) {
         *derr &= ~STBPE_DERR_DENSE_OVERFLOW;
         CK(cudaMemcpyAsync(&e->d.st->error, derr, sizeof(*derr), cudaMemcpyHostToDevice, s));
         CK(cudaStreamSynchronize(s));
-        rc = count_prologue(e, s);
+        rc = count_prologue(e, true, s);
         if (rc != STBPE_OK) return rc;
     }
-    if (!mg && wide_eligible(e, fresh)) {
-        // 16-bit vocabulary: partition the pairs, then count partition by partition inside L2
-        // (wide_count.cuh).  Buffers are allocated at first use and kept for later counts; without
-        // room for them the general kernel counts.
+    if (wide) {
+        // 16-bit vocabulary: partition the pairs, order them inside their partitions and build the table range
+        // by range (wide_count.cuh).  The partition buffers are allocated at first use and kept for later counts;
+        // without room for them the general kernel counts.
         int ok = 0;
         if (wide_alloc(e) == STBPE_OK) {
             rc = wide_pass1(e, &ok, s);
             if (rc != STBPE_OK) return rc;
         }
         if (ok) {
-            PartBuffers &pb = e->parts;
-            CK(cudaEventRecord(e->ev0, s));
-            dense_to_table_kernel<false><<<256, 256, 0, s>>>(e->d, e->wide_dense);
-            CK(cudaGetLastError());
-            const int per_region = 2;  // blocks per pass-1 region: a region holds some 10^4 words
-            // all partitions in a few launches: the blocks of a launch are scheduled in partition
-            // order, so two or three table slices are being filled at any time and stay in L2, and
-            // the tail of a partition runs under the start of the next
-            for (int p = 0; p < STBPE_PARTS; p += e->part_group) {
-                const int n = STBPE_PARTS - p < e->part_group ? STBPE_PARTS - p : e->part_group;
-                partition_table_kernel<<<pb.n_cta * per_region * n, 1024, 0, s>>>(e->d, pb, p, per_region);
-            }
-            CK(cudaGetLastError());
-            CK(cudaEventRecord(e->ev1, s));
-            CK(cudaEventSynchronize(e->ev1));
-            CK(cudaEventElapsedTime(&e->convert_ms, e->ev0, e->ev1));
-            e->count_ms += e->convert_ms;  // the pair table is complete only after both passes
-            return STBPE_OK;
+            rc = wide_build(e, &ok, s);
+            if (rc != STBPE_OK) return rc;
+            if (ok) return STBPE_OK;
         }
+        clear_table_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d);
+        CK(cudaMemsetAsync(&e->d.st->n_keys, 0, sizeof(u64), s));
         // an id of 65 536 or more, or a region outgrew its buffer: the general kernel counts
     }
     if (e->d.n_tiles > 0) {
@@ -1274,6 +1308,7 @@ static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t firs
     if ((size_t)n * sizeof(int2) <= STBPE_PINNED_BYTES - STBPE_PINNED_STATE)
         src = memcpy((char *)e->pinned.p + STBPE_PINNED_STATE, pairs, (size_t)n * sizeof(int2));
     CK(cudaMemcpyAsync(e->forced, src, (size_t)n * sizeof(int2), cudaMemcpyHostToDevice, s));
+    if ((i64)first_new + n > 65536) e->foreign_ids = true;
     int rc = run_loop(e, e->cfg.max_merges, e->forced, n, first_new, &h, s, then_ties);
     e->merges_known = rc == STBPE_OK;
     e->merges_done = h.merges_done;
@@ -1420,32 +1455,45 @@ STBPE_VISIBLE int stbpe_export_histogram(stbpe_engine *e, uint64_t *keys, int64_
     CK(cudaSetDevice(e->cfg.device));
     *n_out = 0;
     if (!e->d.table) return STBPE_OK;  // nothing has been counted
-    u64 *tk = nullptr;
-    i64 *tc = nullptr;
-    CK(cudaMallocAsync((void **)&tk, (size_t)(cap > 0 ? cap : 1) * sizeof(u64), s));
-    CK(cudaMallocAsync((void **)&tc, (size_t)(cap > 0 ? cap : 1) * sizeof(i64), s));
+    // While every id fits 16 bits and every count 32, the entries are sorted as 32-bit keys with 32-bit counts (half
+    // the passes over half the bytes) and widened afterwards.
+    if (int rc = fresh_state(e, s)) return rc;
+    DevState h;
+    if (int rc = read_state(e, &h, s)) return rc;
+    const i64 ids = (i64)e->cfg.base_vocab + h.merges_done;
+    const bool narrow = e->cfg.world_size == 1 && !e->foreign_ids && e->max_id < 65536 && ids <= 65536 && e->max_tokens < (1ll << 32);
+    const size_t elem = narrow ? 4 : 8, side = ((size_t)(cap > 0 ? cap : 1) * elem + 255) & ~(size_t)255;
+    size_t tmp_bytes = 0;
+    if (narrow)
+        cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (uint32_t *)nullptr, (uint32_t *)nullptr, (uint32_t *)nullptr, (uint32_t *)nullptr, (i64)cap, 0, 32, s);
+    else
+        cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (u64 *)nullptr, (u64 *)nullptr, (i64 *)nullptr, (i64 *)nullptr, (i64)cap, 0, 64, s);
+    unsigned char *scratch = nullptr;
+    CK(dev_alloc(e, &scratch, side * (narrow ? 4 : 2) + tmp_bytes + 256));
+    unsigned char *tk = scratch, *tc = scratch + side, *sk = scratch + 2 * side, *sc = scratch + 3 * side, *tmp = scratch + side * (narrow ? 4 : 2);
     CK(cudaMemsetAsync(&e->d.st->export_n, 0, sizeof(i64), s));
-    export_table_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d, tk, tc, cap);
+    if (narrow)
+        export_table_kernel<uint32_t><<<e->sm_count * 4, 512, 0, s>>>(e->d, (uint32_t *)tk, (uint32_t *)tc, cap);
+    else
+        export_table_kernel<u64><<<e->sm_count * 4, 512, 0, s>>>(e->d, (u64 *)tk, (u64 *)tc, cap);
     CK(cudaGetLastError());
-    i64 n = 0;
-    CK(cudaMemcpyAsync(&n, &e->d.st->export_n, sizeof(i64), cudaMemcpyDeviceToHost, s));
+    i64 *n_host = (i64 *)e->pinned.p;
+    CK(cudaMemcpyAsync(n_host, &e->d.st->export_n, sizeof(i64), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    const i64 n = *n_host;
     *n_out = n;
     int rc = STBPE_OK;
     if (n > cap) {
         rc = fail(e, STBPE_E_CAPACITY, "pair workspace capacity exceeded");
+    } else if (n > 0 && narrow) {
+        CK(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, (uint32_t *)tk, (uint32_t *)sk, (uint32_t *)tc, (uint32_t *)sc, n, 0, 32, s));
+        widen_entries_kernel<<<e->sm_count * 8, 256, 0, s>>>((const uint32_t *)sk, (const uint32_t *)sc, n, (u64 *)keys, (i64 *)counts);
     } else if (n > 0) {
-        size_t tmp_bytes = 0;
-        cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, tk, (u64 *)keys, tc, (i64 *)counts, (int)n, 0, 64, s);
-        void *tmp = nullptr;
-        CK(cudaMallocAsync(&tmp, tmp_bytes ? tmp_bytes : 16, s));
-        cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, tk, (u64 *)keys, tc, (i64 *)counts, (int)n, 0, 64, s);
-        CK(cudaGetLastError());
-        CK(cudaFreeAsync(tmp, s));
+        CK(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, (u64 *)tk, (u64 *)keys, (i64 *)tc, (i64 *)counts, n, 0, 64, s));
     }
-    CK(cudaFreeAsync(tk, s));
-    CK(cudaFreeAsync(tc, s));
+    CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s));
+    dev_free(e, scratch);
     return rc;
 }
 
@@ -1653,7 +1701,7 @@ STBPE_VISIBLE int stbpe_mg_wide_pass1(stbpe_engine *e, int32_t *ok, void *stream
     CK(cudaSetDevice(e->cfg.device));
     if (!e->wide_open) return fail(e, STBPE_E_STATE, "call stbpe_mg_wide_open first");
     const bool fresh = e->recs_stale;
-    int rc = count_prologue(e, s);
+    int rc = count_prologue(e, true, s);
     if (rc != STBPE_OK) return rc;
     if (e->only_bytes || e->d.n_tiles < 1 || !fresh) {
         // nothing to partition here (no rows on this rank, or bytes): an empty first pass, the peers still read it

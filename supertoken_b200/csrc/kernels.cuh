@@ -715,16 +715,62 @@ __global__ void count_ties_kernel(EngineDev e) {
 // ---------------------------------------------------------------------------------------
 // exports
 // ---------------------------------------------------------------------------------------
-__global__ void export_table_kernel(EngineDev e, u64 *keys, i64 *counts, i64 cap) {
-    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i <= e.mask; i += (u64)gridDim.x * blockDim.x) {
-        const Slot s = e.table[i];
-        if (s.key != STBPE_EMPTY && s.count != 0) {
-            const i64 j = (i64)atomicAdd((u64 *)&e.st->export_n, 1ull);
-            if (j < cap) {
-                keys[j] = s.key;
-                counts[j] = s.count;
-            }
+// Entries with a count, unordered.  K = uint32_t: (a << 16) | b and a 32-bit count (ids and counts that fit).  A
+// CTA reserves the places of its entries of a step at once.
+template <typename K>
+__global__ void __launch_bounds__(512) export_table_kernel(EngineDev e, K *keys, K *counts, i64 cap) {
+    __shared__ int s_sum[16];
+    __shared__ i64 s_base;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int PER = 8;
+    for (u64 i0 = (u64)blockIdx.x * 512 * PER; i0 <= e.mask; i0 += (u64)gridDim.x * 512 * PER) {
+        Slot s[PER];
+        int own = 0;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const u64 i = i0 + (u64)k * 512 + threadIdx.x;
+            s[k].key = STBPE_EMPTY, s[k].count = 0;
+            if (i <= e.mask) s[k] = ldcg_slot(e.table + i);
+            if (s[k].key == STBPE_EMPTY) s[k].count = 0;
+            own += s[k].count != 0;
         }
+        int incl = own;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int o = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+            if (lane >= d) incl += o;
+        }
+        if (lane == 31) s_sum[warp] = incl;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int total = 0;
+            for (int w = 0; w < 16; ++w) {
+                const int x = s_sum[w];
+                s_sum[w] = total;
+                total += x;
+            }
+            s_base = total ? (i64)atomicAdd((u64 *)&e.st->export_n, (u64)total) : 0;
+        }
+        __syncthreads();
+        i64 at = s_base + s_sum[warp] + incl - own;
+#pragma unroll
+        for (int k = 0; k < PER; ++k)
+            if (s[k].count != 0) {
+                if (at < cap) {
+                    keys[at] = sizeof(K) == 4 ? (K)(((s[k].key >> 32) << 16) | (s[k].key & 0xFFFFull)) : (K)s[k].key;
+                    counts[at] = (K)s[k].count;
+                }
+                ++at;
+            }
+        __syncthreads();
+    }
+}
+
+__global__ void widen_entries_kernel(const uint32_t *__restrict__ k, const uint32_t *__restrict__ c, i64 n, u64 *__restrict__ keys, i64 *__restrict__ counts) {
+    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
+        const uint32_t x = k[i];
+        keys[i] = ((u64)(x >> 16) << 32) | (u64)(x & 0xFFFFu);
+        counts[i] = (i64)c[i];
     }
 }
 

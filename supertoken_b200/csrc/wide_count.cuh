@@ -195,61 +195,148 @@ __device__ __forceinline__ bool table_count_n(const EngineDev &e, u64 key, u64 h
     return false;
 }
 
-// `top`: the word's table slice shifted into place (every word of a pass-2 launch is of one partition)
-__device__ __forceinline__ void part_word_to_table(const EngineDev &e, uint32_t x, u64 n, unsigned int &fresh, u64 top) {
+__device__ __forceinline__ void part_word_to_table(const EngineDev &e, uint32_t x, u64 n, unsigned int &fresh) {
     const uint32_t ab = unmix32(x);
     const u64 key = ((u64)(ab >> 16) << 32) | (u64)(ab & 0xFFFFu);
-    const u64 h = slot_in_slice(e, top, key);
-    table_count_n(e, key, h, n, fresh);
+    table_count_n(e, key, slot_of_word(e, x), n, fresh);
 }
 
-// pass 2: the words of partition p (the regions of all pass-1 CTAs) into the table slice of p.
-// Block b serves region b / per_region.  A frequent pair would otherwise be tens of thousands of
-// reductions on one address, which L2 executes one after the other (the hottest pair of a partition
-// alone took longer than everything else of its launch), so every block first collects its words in
-// a direct-mapped cache in shared memory (word -> count; a word whose entry is taken by another
-// goes straight to the table) and then adds each cached word once.
-// One launch serves several partitions: consecutive groups of n_cta * per_region blocks take
-// consecutive partitions, so the blocks resident at any time work on two or three slices.
-__global__ void __launch_bounds__(1024) partition_table_kernel(EngineDev e, PartBuffers pb, int p_first, int per_region) {
-    const int blocks_per_part = pb.n_cta * per_region;
-    const int p = p_first + (int)(blockIdx.x / blocks_per_part);
-    const int block = (int)(blockIdx.x % blocks_per_part);
-    __shared__ uint32_t s_word[STBPE_PART_CACHE];
-    __shared__ unsigned int s_cnt[STBPE_PART_CACHE];
-    for (int i = threadIdx.x; i < STBPE_PART_CACHE; i += blockDim.x) {
-        s_word[i] = 0xFFFFFFFFu;
-        s_cnt[i] = 0u;
-    }
-    __syncthreads();
-    const int region = block / per_region, part = block % per_region;
-    const u64 top = (u64)slice_of(e, (unsigned int)p) << e.slot_bits;
-    const i64 n = pb.fill[(i64)p * pb.n_cta + region];
-    const uint32_t *w = pb.words + ((i64)p * pb.n_cta + region) * pb.cap;
-    unsigned int fresh = 0;
-    // (four words per thread and step, with their four table slots loaded before any is looked at,
-    // was slower: 30 ms instead of 21 ms for the 256 launches on 2^31 ids)
-    for (i64 i = (i64)part * blockDim.x + threadIdx.x; i < n; i += (i64)per_region * blockDim.x) {
-        const uint32_t x = __ldcs(w + i);  // streamed once: keep it from displacing the table slice
-        const unsigned int c = (x * 0x9E3779B1u) >> (32 - STBPE_PART_CACHE_BITS);
-        uint32_t k = s_word[c];
-        if (k == 0xFFFFFFFFu && x != 0xFFFFFFFFu) {
-            const uint32_t old = atomicCAS(&s_word[c], 0xFFFFFFFFu, x);
-            k = old == 0xFFFFFFFFu ? x : old;
-        }
-        if (k == x && x != 0xFFFFFFFFu)
-            atomicAdd(&s_cnt[c], 1u);
-        else
-            part_word_to_table(e, x, 1ull, fresh, top);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < STBPE_PART_CACHE; i += blockDim.x) {
-        const unsigned int c = s_cnt[i];
-        if (c) part_word_to_table(e, s_word[i], (u64)c, fresh, top);
-    }
+// pass 2, one rank: the words of every chunk (a piece of a pass-1 region of at most STBPE_SUB_CHUNK words) in
+// order of their next `sub_bits` bits, in place; offs[chunk][d] = where the words of digit d start.
+// One returning shared-memory atomic per word gives its rank inside its digit, the words wait in registers
+// meanwhile and go back through shared memory in order.
+#define STBPE_SUB_THREADS 512
+#define STBPE_SUB_CHUNK 8192
+#define STBPE_SUB_MAX_BITS 8
+__global__ void __launch_bounds__(STBPE_SUB_THREADS, 3) sub_partition_kernel(PartBuffers pb, int chunks_per_region, int sub_bits, uint16_t *__restrict__ offs) {
+    extern __shared__ __align__(16) uint32_t s_out[];  // STBPE_SUB_CHUNK words
+    __shared__ unsigned int s_cnt[1 << STBPE_SUB_MAX_BITS], s_base[(1 << STBPE_SUB_MAX_BITS) + 1];
+    constexpr int PER = STBPE_SUB_CHUNK / STBPE_SUB_THREADS;
+    const int D = 1 << sub_bits, lane = threadIdx.x & 31;
+    const i64 n_chunks = (i64)STBPE_PARTS * pb.n_cta * chunks_per_region;
+    for (i64 chunk = blockIdx.x; chunk < n_chunks; chunk += gridDim.x) {
+        const i64 region = chunk / chunks_per_region, first = (chunk - region * chunks_per_region) * STBPE_SUB_CHUNK;
+        const i64 left = (i64)pb.fill[region] - first;
+        const int n = left <= 0 ? 0 : (left < STBPE_SUB_CHUNK ? (int)left : STBPE_SUB_CHUNK);
+        uint32_t *w = pb.words + region * pb.cap + first;
+        for (int i = threadIdx.x; i < D; i += STBPE_SUB_THREADS) s_cnt[i] = 0u;
+        __syncthreads();
+        uint32_t x[PER];
+        uint16_t r[PER];
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) fresh += __shfl_down_sync(0xFFFFFFFFu, fresh, d);
-    if ((threadIdx.x & 31) == 0 && fresh) atomicAdd(&e.st->n_keys, (u64)fresh);
+        for (int k = 0; k < PER; ++k) {
+            const int i = k * STBPE_SUB_THREADS + threadIdx.x;
+            x[k] = i < n ? __ldcs(w + i) : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < PER; ++k)
+            if (k * STBPE_SUB_THREADS + (int)threadIdx.x < n)
+                r[k] = (uint16_t)atomicAdd(&s_cnt[(x[k] << STBPE_PART_BITS) >> (32 - sub_bits)], 1u);
+        __syncthreads();
+        if (threadIdx.x < 32) {  // exclusive sums of the digits, D / 32 per lane (D >= 2)
+            const int per = (D + 31) / 32;
+            unsigned int own = 0;
+            for (int k = 0; k < per; ++k) own += lane * per + k < D ? s_cnt[lane * per + k] : 0u;
+            unsigned int incl = own;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const unsigned int o = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+                if (lane >= d) incl += o;
+            }
+            unsigned int at = incl - own;
+            for (int k = 0; k < per; ++k)
+                if (lane * per + k < D) {
+                    s_base[lane * per + k] = at;
+                    at += s_cnt[lane * per + k];
+                }
+            if (lane == 31) s_base[D] = incl;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < PER; ++k)
+            if (k * STBPE_SUB_THREADS + (int)threadIdx.x < n) s_out[s_base[(x[k] << STBPE_PART_BITS) >> (32 - sub_bits)] + r[k]] = x[k];
+        for (int i = threadIdx.x; i <= D; i += STBPE_SUB_THREADS) offs[chunk * (D + 1) + i] = (uint16_t)s_base[i];
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += STBPE_SUB_THREADS) w[i] = s_out[i];
+        __syncthreads();
+    }
+}
+
+// pass 3, one rank: the pair table, range by range.  A task is the range of words with one value of the first
+// 8 + sub_bits bits; it owns `1 << task_bits` consecutive slots, which it fills in shared memory (word and
+// 32-bit count) and writes out as they are, occupied or not: every slot of the table is written once with full
+// lines, nothing is cleared before and no atomic reaches L2.  A word whose probe runs over the end of the range
+// goes to the spill list, which is added to the finished table.
+#define STBPE_BUILD_THREADS 512
+__global__ void __launch_bounds__(STBPE_BUILD_THREADS, 3) build_table_kernel(EngineDev e, PartBuffers pb, int chunks_per_region, int sub_bits, int task_bits,
+                                                                          const uint16_t *__restrict__ offs, uint32_t *spill, unsigned int *n_spill,
+                                                                          unsigned int spill_cap) {
+    extern __shared__ __align__(16) uint32_t s_word[];
+    const unsigned int TS = 1u << task_bits;
+    unsigned int *s_num = s_word + TS;
+    const int D = 1 << sub_bits, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n_tasks = STBPE_PARTS << sub_bits;
+    const int shift = 32 - STBPE_PART_BITS - sub_bits - task_bits;
+    for (int task = blockIdx.x; task < n_tasks; task += gridDim.x) {
+        const uint32_t none = (uint32_t)(task ^ 1) << (32 - STBPE_PART_BITS - sub_bits);  // a word of another task
+        for (unsigned int i = threadIdx.x; i < TS; i += STBPE_BUILD_THREADS) s_word[i] = none, s_num[i] = 0u;
+        __syncthreads();
+        const int p = task >> sub_bits, d = task & (D - 1);
+        const int chunks = pb.n_cta * chunks_per_region;
+        for (int c = warp; c < chunks; c += STBPE_BUILD_THREADS / 32) {
+            const i64 chunk = (i64)p * chunks + c;
+            const unsigned int lo = offs[chunk * (D + 1) + d], hi = offs[chunk * (D + 1) + d + 1];
+            const i64 region = (i64)p * pb.n_cta + c / chunks_per_region;
+            const uint32_t *w = pb.words + region * pb.cap + (i64)(c % chunks_per_region) * STBPE_SUB_CHUNK;
+            for (unsigned int i = lo + lane; i < hi; i += 32) {
+                const uint32_t x = __ldcs(w + i);
+                unsigned int h = (x >> shift) & (TS - 1);
+                for (;;) {
+                    uint32_t k = ((volatile uint32_t *)s_word)[h];
+                    if (k == none) {
+                        k = atomicCAS(&s_word[h], none, x);
+                        if (k == none) k = x;
+                    }
+                    if (k == x) {
+                        atomicAdd(&s_num[h], 1u);
+                        break;
+                    }
+                    if (++h == TS) {
+                        const unsigned int j = atomicAdd(n_spill, 1u);
+                        if (j < spill_cap)
+                            spill[j] = x;
+                        else
+                            atomicOr(&e.st->error, STBPE_DERR_DENSE_OVERFLOW);
+                        break;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        Slot *out = e.table + ((u64)task << task_bits);
+        unsigned int keys = 0;
+        for (unsigned int i = threadIdx.x; i < TS; i += STBPE_BUILD_THREADS) {
+            Slot s;
+            s.key = STBPE_EMPTY;
+            s.count = (i64)s_num[i];
+            if (s.count) {
+                const uint32_t ab = unmix32(s_word[i]);
+                s.key = ((u64)(ab >> 16) << 32) | (u64)(ab & 0xFFFFu);
+                ++keys;
+            }
+            out[i] = s;
+        }
+        keys = __reduce_add_sync(0xFFFFFFFFu, keys);
+        if (lane == 0 && keys) atomicAdd(&e.st->n_keys, (u64)keys);
+        __syncthreads();
+    }
+}
+
+__global__ void spill_to_table_kernel(EngineDev e, const uint32_t *__restrict__ spill, const unsigned int *n_spill, unsigned int spill_cap) {
+    const unsigned int n = min(*n_spill, spill_cap);
+    unsigned int fresh = 0;
+    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) part_word_to_table(e, spill[i], 1ull, fresh);
+    if (fresh) atomicAdd(&e.st->n_keys, (u64)fresh);
 }
 
 // pass 2, several ranks: partition p, owned by this rank, out of the regions of every rank.  The grid
@@ -269,7 +356,6 @@ __global__ void __launch_bounds__(1024)
     }
     __syncthreads();
     unsigned int fresh = 0;
-    const u64 top = (u64)slice_of(e, (unsigned int)p) << e.slot_bits;
     const int n_units = wp.world * n_cta * 2;
     for (int unit = block; unit < n_units; unit += blocks_per_part) {
         const int half = unit & 1, region = (unit >> 1) % n_cta, src = (unit >> 1) / n_cta;
@@ -305,14 +391,14 @@ __global__ void __launch_bounds__(1024)
                 if (kk == x[k] && x[k] != 0xFFFFFFFFu)
                     atomicAdd(&s_cnt[c], 1u);
                 else
-                    part_word_to_table(e, x[k], 1ull, fresh, top);
+                    part_word_to_table(e, x[k], 1ull, fresh);
             }
         }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < STBPE_PART_CACHE; i += blockDim.x) {
         const unsigned int c = s_cnt[i];
-        if (c) part_word_to_table(e, s_word[i], (u64)c, fresh, top);
+        if (c) part_word_to_table(e, s_word[i], (u64)c, fresh);
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) fresh += __shfl_down_sync(0xFFFFFFFFu, fresh, d);
