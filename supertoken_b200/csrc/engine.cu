@@ -81,6 +81,7 @@ struct stbpe_engine {
     std::vector<stbpe::Block> allocs;
     bool broken;          // a CUDA call failed: work of this engine may still be pending
     stbpe::Block pinned;  // host side of small transfers: the device state, then small inputs
+    int dense_batch;
     bool foreign_ids;     // a merge of the caller's may have brought an id of 65 536 or more
     unsigned int max_id;  // largest id appended through stbpe_append_ids
     unsigned int load_err;  // error bits of the rows appended so far
@@ -353,6 +354,8 @@ STBPE_VISIBLE int stbpe_create(stbpe_engine **out, const stbpe_config *cfg) {
     e->dense32_min = 1ll << 24;
     if (const char *v = getenv("STBPE_DENSE32_MIN_TOKENS")) e->dense32_min = atoll(v);
     e->use_graph = getenv("STBPE_NO_GRAPH") == nullptr;
+    e->dense_batch = 4;
+    if (const char *v = getenv("DEV_DENSE")) e->dense_batch = atoi(v);
     e->part_group = STBPE_PARTS;
     if (const char *v = getenv("STBPE_PART_GROUP")) e->part_group = atoi(v) > 0 ? atoi(v) : STBPE_PARTS;
     e->filter_density = 1.0;
@@ -1249,6 +1252,7 @@ static int run_loop(stbpe_engine *e, int target, const int2 *forced, int n_force
         la.forced_new = forced_new + at;
         const double fc = e->filter_density * (double)e->d.n_tiles;
         la.filter_count = fc >= 9e18 ? (i64)9000000000000000000ll : (i64)fc;
+        la.dense_batch = e->dense_batch;
         la.repack_tiles = 64;
         la.grow_keys = e->table_auto ? (i64)(e->slots / 4) : (i64)0x7FFFFFFFFFFFFFFFll;
         la.ids_below = e->only_bytes ? 0 : (int)e->max_id + 1;

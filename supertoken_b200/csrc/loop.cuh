@@ -1,5 +1,5 @@
 // The merge loop of one GPU as one persistent cooperative kernel: one CTA per SM takes every step
-//     choose the best pair -> apply the merge, deltas into the pair table -> refresh the maxima the deltas changed
+//     choose the next best pairs -> apply the merges, deltas into the pair table
 // without returning to the host; the launch ends when a stop rule fires or the host has maintenance to do.
 //
 // A late merge changes a few thousand places of a stream of any size, so its cost is the latency of the steps,
@@ -13,6 +13,16 @@
 // vote of the CTAs on the best of them, the same step took 4.3 us instead of 1.5.)
 // A second counter keeps the CTAs apart the other way round: a CTA adds its deltas of merge m only when all have
 // read the counts that chose merge m; that wait runs under the rewriting of the tiles.
+//
+// A step takes several merges.  Let p1, p2, ... be the pairs in selection order (larger count, then smaller key).
+// While no two of p1 .. pj share a token, merging p1 .. pj-1 leaves the count of pj as it is, and makes or
+// raises only pairs with one of their new tokens.  Such a pair (x, new) occurs at most as often as (x, a) did, and
+// (x, a) came after pj; where the counts are equal the larger key, new > every token of pj, loses.  So pj is
+// then the best pair, exactly as if the counts had been taken after each merge, and p1 .. pj are applied at once.
+// The batch ends at the first pair that shares a token, at Batch<T>::MAX, and wherever a stop rule or
+// maintenance has to be decided first.  On text a batch is four merges on average late in a run: the grid barrier,
+// the choice and the flush of the deltas, some 9 of the 12 us of a sparse merge, are paid once for the four.
+//
 // Nothing else is exchanged: the tiles a merge must visit come out of the pair filter inside each CTA.
 //
 // All waits are bounded (STBPE_LOOP_WAIT_NS): a CTA that gives up sets STBPE_DERR_TIMEOUT and leaves, and so do
@@ -27,6 +37,7 @@ struct LoopArgs {
     const int2 *forced;     // host-given merges (a, b) applied in order instead of the best pair, or null
     int n_forced, forced_new;  // forced merge i gets id forced_new + i
     i64 filter_count;       // leave to build the pair filter when the merge's count has fallen to this
+    int dense_batch;        // merges per step while every tile is visited (no filter)
     int repack_tiles;       // leave for a re-pack at three quarters live from this many tiles on
     int unit_shift;         // tiles per filter unit, log2 (cta_merge)
     i64 grow_keys;          // leave for a larger pair table when a merge could take the number of keys beyond this ...
@@ -118,8 +129,11 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
     constexpr int THREADS = MergeGeom<T>::THREADS, WARPS = THREADS / 32;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ int s_ctr[CTR_N];
-    __shared__ Bt s_best[2][32];          // the warps' best candidates, alternating between steps
-    __shared__ i64 s_live, s_keys, s_forced;  // live tokens, keys in the table, count of the next host-given pair
+    constexpr int KB = Batch<T>::MAX, TOP = KB > 1 ? 4 : 1;  // best candidates that each warp hands over
+    __shared__ Bt s_top[32 * TOP], s_rest[32];  // the warps' best candidates in order; the best of what is left
+    __shared__ i64 s_live, s_keys;        // live tokens, keys in the table
+    __shared__ i64 s_forced[KB];          // counts of the next host-given pairs
+    __shared__ int s_go;                  // merges in this step's batch
     __shared__ unsigned int s_err;        // device error bits
     __shared__ int s_ok;                  // every wait so far succeeded
     __shared__ int s_work;                // CTA 0: tiles the last merge visited
@@ -149,30 +163,48 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
         // ---- choose: the counts of all candidates as the last merge left them
         {
             const unsigned int n = __ldcg(&st->n_cand), n_have = min(n, STBPE_CAND_CAP);
-            Bt x = Bs::none();
+            Bt x = Bs::none(), x2 = Bs::none(), rest = Bs::none();  // this thread's best two, and a bound on its others
+            auto take = [&](unsigned int at) {
+                const Slot y = ldcg_slot(e.table + at);
+                const Bt v = Bs::make(y.key, y.count);
+                if constexpr (KB > 1) {
+                    rest = max(rest, min(v, x2));
+                    x2 = max(x2, min(x, v));
+                    x = max(x, v);
+                } else {
+                    x = Bs::max2(x, v);
+                }
+            };
 #pragma unroll 2
-            for (unsigned int i = tid; i < n_cand; i += THREADS) {
-                const Slot y = ldcg_slot(e.table + s_cand[i]);
-                x = Bs::max2(x, Bs::make(y.key, y.count));
-            }
+            for (unsigned int i = tid; i < n_cand; i += THREADS) take(s_cand[i]);
 #pragma unroll 1
-            for (unsigned int i = n_cand + tid; i < n_have; i += THREADS) {  // appended by the last merge
+            for (unsigned int i = n_cand + tid; i < n_have; i += THREADS) {  // appended by the last merges
                 const unsigned int at = __ldcg(e.cand + i);
                 s_cand[i] = at;
-                const Slot y = ldcg_slot(e.table + at);
-                x = Bs::max2(x, Bs::make(y.key, y.count));
+                take(at);
             }
             n_cand = n_have;
-            x = Bs::warp_max(x);
-            if (lane == 0) s_best[step & 1][warp] = x;
+#pragma unroll
+            for (int r = 0; r < TOP; ++r) {
+                const Bt v = Bs::warp_max(x);
+                if (lane == 0) s_top[warp * TOP + r] = v;
+                if constexpr (KB > 1) {
+                    if (x == v) x = x2, x2 = Bs::none();  // (a pair sits in one slot, so one lane holds it)
+                }
+            }
+            if constexpr (KB > 1) {
+                const Bt v = Bs::warp_max(max(x, rest));
+                if (lane == 0) s_rest[warp] = v;
+            }
+            if (la.forced && warp == 0 && lane < KB && forced_i + lane < la.n_forced) {
+                const int2 f = la.forced[forced_i + lane];
+                const i64 at = find_slot(e, ((u64)(uint32_t)f.x << 32) | (uint32_t)f.y);
+                s_forced[lane] = at >= 0 ? (i64)__ldcg((const u64 *)&e.table[at].count) : 0;
+            }
             if (tid == THREADS - 1) {
                 s_live = (i64)__ldcg((const u64 *)&st->n_live);
                 s_keys = (i64)__ldcg(&st->n_keys);
                 s_err = __ldcg(&st->error) | (n > STBPE_CAND_CAP ? 0x80000000u : 0u);
-                if (la.forced && forced_i < la.n_forced) {
-                    const i64 at = find_slot(e, ((u64)(uint32_t)la.forced[forced_i].x << 32) | (uint32_t)la.forced[forced_i].y);
-                    s_forced = at >= 0 ? (i64)__ldcg((const u64 *)&e.table[at].count) : 0;
-                }
                 if (cta == 0 && step > 0) {
                     s_work = fv ? __ldcg(&st->n_work) : -1;
                     st->n_work = 0;
@@ -181,65 +213,109 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
         }
         __syncthreads();
         if (tid == THREADS - 1) red_release_u32(&sync->chosen, 1u);  // the CTA has read everything it decides by
-        // every warp decides by itself
-        bool forced = false;
-        i64 count;
-        {
-            const Slot best = Bs::slot(Bs::warp_max(lane < WARPS ? s_best[step & 1][lane] : Bs::none()));
+        // warp 0 decides; lane j holds what belongs to merge j of the batch
+        if (warp == 0) {
+            const Bt bound = KB > 1 ? Bs::warp_max(lane < WARPS ? s_rest[lane] : Bs::none()) : Bs::none();
+            Bt cur = lane < WARPS ? s_top[lane * TOP] : Bs::none();
+            int at = 0;
             const unsigned int err = s_err;
-            const bool over = (err >> 31) != 0u;
-            const bool dry = over || !(mc.theta.admits(best.count, best.key) || (best.count <= 0 && mc.theta.count == 0));
-            int stop = 0, why = STBPE_EXIT_STOP, go = 0;
-            u64 key = best.key;
-            count = best.count;
-            const bool host = la.forced != nullptr;
-            forced = host && forced_i < la.n_forced;
-            if (forced) {
-                key = ((u64)(uint32_t)la.forced[forced_i].x << 32) | (uint32_t)la.forced[forced_i].y;
-                count = s_forced;
+            const bool over = (err >> 31) != 0u, host = la.forced != nullptr;
+            const i64 live0 = s_live;
+            i64 live = live0, keys = s_keys, best_count = 0, own_count = 0, own_live = 0;
+            u64 best_key = STBPE_EMPTY;
+            bool best_dry = true;
+            uint32_t own_a = 0, own_b = 0;
+            int stop = 0, why = STBPE_EXIT_STOP, nb = 0;
+            const uint32_t nw0 = (uint32_t)(host ? la.forced_new + forced_i : base_vocab + merges_done);
+            const int most = fv ? KB : la.dense_batch < KB ? la.dense_batch : KB;
+#pragma unroll 1
+            for (;; ++nb) {
+                const Bt v = Bs::warp_max(cur);
+                const Slot best = Bs::slot(v);
+                const bool dry = over || !(mc.theta.admits(best.count, best.key) || (best.count <= 0 && mc.theta.count == 0));
+                if (nb == 0) best_key = best.key, best_count = best.count, best_dry = dry;
+                const bool forced = host && forced_i + nb < la.n_forced;
+                u64 key = best.key;
+                i64 count = best.count;
+                if (forced) {
+                    const int2 f = la.forced[forced_i + nb];
+                    key = ((u64)(uint32_t)f.x << 32) | (uint32_t)f.y;
+                    count = nb < KB ? s_forced[nb] : 0;
+                }
+                const uint32_t a = (uint32_t)(key >> 32), b = (uint32_t)key, nw = nw0 + nb;
+                // a later member of the batch: exact order so far, no token shared with the members before, none of
+                // their new tokens (a pair given by the host may name one)
+                if (nb > 0) {
+                    if (nb >= most) break;
+                    if constexpr (KB > 1) {
+                        if (!host && !(v > bound)) break;
+                    }
+                    if (max(a, b) >= nw0) break;
+                    if (__any_sync(0xFFFFFFFFu, lane < nb && (own_a == a || own_a == b || own_b == a || own_b == b))) break;
+                }
+                // stop rules of the loop: bpe_trainer.py:4304-4308 (no pairs), :2491-2494 / :4361-4364 (count < 2)
+                if (err & 0x7FFFFFFFu) stop = 4;
+                else if (host && !forced) stop = 0;
+                else if (!host && merges_done + nb >= la.target) stop = 1;
+                // maintenance the host does between launches
+                else if (!host && dry) why = STBPE_EXIT_REFILL;
+                else if (!host && count <= 0) stop = 2;
+                else if (!host && count < 2) stop = 3;
+                else if (e.n_tiles >= la.repack_tiles && live * 4 <= (i64)e.n_tiles * STBPE_TILE * 3) why = STBPE_EXIT_REPACK;
+                else if (!fv && e.n_tiles > 0 && count <= la.filter_count) why = STBPE_EXIT_FILTER;
+                // every merge makes at most two pairs per match and two per id
+                else if (keys + 2 * min(count, (i64)max((int)nw, la.ids_below)) + 2 > la.grow_keys) why = STBPE_EXIT_GROW;
+                else if (sizeof(T) == 2 && max(nw, max(a, b)) >= Tok<uint16_t>::IDMASK) why = STBPE_EXIT_WIDEN;
+                else {
+                    if (lane == nb) own_a = a, own_b = b, own_count = count, own_live = live;
+                    keys += 2 * min(count, (i64)max((int)nw, la.ids_below)) + 2;
+                    live -= count;  // a merge drops one token per occurrence of its pair (of a run, all but one)
+                    if constexpr (KB > 1) {
+                        if (cur == v) cur = ++at < TOP ? s_top[lane * TOP + at] : Bs::none();
+                    }
+                    continue;
+                }
+                break;
             }
-            mc.a = (uint32_t)(key >> 32), mc.b = (uint32_t)key;
-            mc.nw = (uint32_t)(host ? la.forced_new + forced_i : base_vocab + merges_done);
-            // stop rules of the loop: bpe_trainer.py:4304-4308 (no pairs), :2491-2494 / :4361-4364 (count < 2)
-            if (err & 0x7FFFFFFFu) stop = 4;
-            else if (host && !forced) stop = 0;
-            else if (!host && merges_done >= la.target) stop = 1;
-            // maintenance the host does between launches
-            else if (!host && dry) why = STBPE_EXIT_REFILL;
-            else if (!host && count <= 0) stop = 2;
-            else if (!host && count < 2) stop = 3;
-            else if (e.n_tiles >= la.repack_tiles && s_live * 4 <= (i64)e.n_tiles * STBPE_TILE * 3) why = STBPE_EXIT_REPACK;
-            else if (!fv && e.n_tiles > 0 && count <= la.filter_count) why = STBPE_EXIT_FILTER;
-            // every merge makes at most two pairs per match and two per id
-            else if (s_keys + 2 * min(count, (i64)max((int)mc.nw, la.ids_below)) + 2 > la.grow_keys) why = STBPE_EXIT_GROW;
-            else if (sizeof(T) == 2 && max(mc.nw, max(mc.a, mc.b)) >= Tok<uint16_t>::IDMASK) why = STBPE_EXIT_WIDEN;
-            else go = 1;
-            if (cta == 0 && tid == 0) {
-                if (go) {
-                    e.merges[2 * merges_done] = (int32_t)mc.a;
-                    e.merges[2 * merges_done + 1] = (int32_t)mc.b;
-                    e.merge_counts[merges_done] = count;
-                    e.live_before[merges_done] = s_live;
-                    st->cur_a = (int)mc.a, st->cur_b = (int)mc.b, st->cur_new = (int)mc.nw;
-                    st->cur_count = count;
-                } else {
+            if (lane < nb) {
+                s.p->a[lane] = own_a, s.p->b[lane] = own_b, s.p->nw[lane] = nw0 + lane;
+                s.p->count[lane] = own_count;
+                if (cta == 0) {
+                    const int m = merges_done + lane;
+                    e.merges[2 * m] = (int32_t)own_a;
+                    e.merges[2 * m + 1] = (int32_t)own_b;
+                    e.merge_counts[m] = own_count;
+                    e.live_before[m] = own_live;
+                    if (lane == nb - 1) {
+                        st->cur_a = (int)own_a, st->cur_b = (int)own_b, st->cur_new = (int)(nw0 + lane);
+                        st->cur_count = own_count;
+                    }
+                }
+            }
+            if (lane == 0) {
+                s.p->n = nb;
+                s_go = nb;
+                if (cta == 0 && nb == 0) {
                     st->merges_done = merges_done;
                     st->run_exit = why;
                     st->stopped = stop > 0;
                     st->stop_reason = stop;
-                    st->peek_key = best.key;
-                    st->peek_count = best.count;
-                    st->peek_valid = !dry;
+                    st->peek_key = best_key;
+                    st->peek_count = best_count;
+                    st->peek_valid = !best_dry;
                     st->forced_done = forced_i;
                     st->n_work = s_work;
                 }
             }
-            if (!go || !s_ok) return;
         }
-        // ---- the merge
-        mc.m = ++merges_done;
-        mc.zero = cta == G - 1 ? count : 0;
-        ++forced_i;
+        __syncthreads();
+        const int nb = s_go;
+        if (nb == 0 || !s_ok) return;
+        // ---- the merges
+        merges_done += nb;
+        forced_i += nb;
+        mc.m = merges_done;
+        mc.zero = cta == G - 1;
         cta_merge<T, false>(e, s, mc, la.unit_shift, [&] {
             if (tid == THREADS - 1) {
                 BoundedWait wait;

@@ -1,28 +1,27 @@
-// K3  one merge: find + rewrite + delta counts, by one CTA over its share of the tiles (cta_merge); the
-// stand-alone merge_kernel and the persistent loop_kernel both run it.
+// K3  a batch of merges: find + rewrite + delta counts, by one CTA over its share of the tiles (cta_merge); the
+// stand-alone merge_kernel (always one merge) and the persistent loop_kernel both run it.
 //
 // With M[i] = (id[i]==a && id[j]==b && token j does not start a row), j = the live token behind i,
 // evaluated on the pre-merge stream (gpu_tokenizer/utils.py:520-527), token j is dropped when M[i]
-// and token i becomes `new` (utils.py:529-531).  The histogram of the result equals a full recount of
-// the rewritten rows when these terms are added (the entry of (a,b) itself is zeroed when the merge is
-// selected):
-//   a != b, per match head (x = the token before it, y = the token behind its partner, both only if in
-//   the same row):
-//       x exists : if x is the dropped b of a preceding match  +1 (new,new)
-//                  else                                         -1 (x,a)  +1 (x,new)
-//       y exists : -1 (b,y);  +1 (new,y) unless y heads the next match (whose head then adds
-//                  the (new,new) term)
-//   a == b, per run of k >= 2 equal tokens (it collapses into ONE new token):
-//       head (first token), x exists : -1 (x,a)  +1 (x,new)
-//       tail (last token),  y exists : -1 (a,y)  +1 (new,y)
-// So the terms of a merge are a histogram of left neighbours x and one of right neighbours y, which the CTA
-// collects in shared memory by neighbour id (one 32-bit key per neighbour and side) and turns into
-// pair-table adds once per distinct neighbour.
+// and token i becomes `new` (utils.py:529-531).  A run of k >= 2 equal tokens (a == b) collapses into ONE new
+// token.  The merges of a batch share no token, so no position belongs to two of them and applying them
+// together leaves the stream that applying them one after the other leaves (loop.cuh says when the next
+// best pairs may form a batch).
+//
+// The histogram of the result equals a full recount of the rewritten rows when these terms are added (the entries
+// of the merged pairs themselves are zeroed when the merges are selected).  For every match (run) of pair k,
+// x = the token before its head and y = the token behind its last token, both only if in the same row:
+//       x exists : if x is the dropped token of a match of pair i   -1 (b_i,a_k)  +1 (new_i,new_k)
+//                  else                                              -1 (x,a_k)    +1 (x,new_k)
+//       y exists : if y heads a match: nothing, that match has x    else  -1 (b_k,y)  +1 (new_k,y)
+// So the terms are a histogram of left neighbours x and one of right neighbours y per pair, which the CTA
+// collects in shared memory by neighbour id (one 32-bit key per neighbour, pair and side) and turns into
+// pair-table adds once per distinct neighbour, and a small matrix of matches that touch.
 //
 // A warp takes a tile through registers into its shared-memory slot (the next tile's loads are in flight
-// meanwhile) and works on 32-bit masks, one group of 32 consecutive tokens per lane: live, id a, id b, row
-// start.  Match heads, dropped positions and the neighbours' positions all follow from carry arithmetic on
-// the masks (next_live_bits) and a few ballots; only neighbours and changed tokens are touched one by one.
+// meanwhile) and works on 32-bit masks, one group of 32 consecutive tokens per lane: live, row start and, per
+// pair, id a and id b.  Match heads and dropped positions follow from carry arithmetic on the masks
+// (next_live_bits) and a few ballots; only neighbours and changed tokens are touched one by one.
 // Nothing is compacted: a dropped token becomes a hole and only the 16-byte units that changed are stored.
 #pragma once
 #include "stream.cuh"
@@ -32,29 +31,67 @@
 #define STBPE_LIST 2048                   // tiles a CTA collects from the pair filter at a time
 #define STBPE_LIST_UNITS 64               // filter units (of at most 32 tiles) per batch
 
+// Pairs of a batch.  Late in a run on text four of the next best pairs on average share no token (8 in a batch;
+// 16 would give 5 % more, 4 would give 3.3), and what a late merge costs is latency.  The wide stream, whose ids leave
+// the neighbour histogram's keys no room for a pair number, takes one at a time.
+template <typename T>
+struct Batch;
+template <>
+struct Batch<uint16_t> {
+    static constexpr int MAX = 8;
+    // neighbour key: 15-bit id, side, pair
+    static __device__ __forceinline__ uint32_t key(uint32_t id, uint32_t side, uint32_t k) { return id | (side << 15) | (k << 16); }
+    static __device__ __forceinline__ uint32_t id(uint32_t key) { return key & 0x7FFFu; }
+    static __device__ __forceinline__ uint32_t side(uint32_t key) { return (key >> 15) & 1u; }
+    static __device__ __forceinline__ uint32_t pair(uint32_t key) { return key >> 16; }
+    // entry the probe starts at: while the vocabulary is small (which is when merges have many matches) the neighbours
+    // of one pair fall on distinct entries, and the pairs of a batch start far apart
+    static __device__ __forceinline__ uint32_t home(uint32_t key) { return key * 2u + side(key) + pair(key) * 1171u; }
+};
+template <>
+struct Batch<uint32_t> {
+    static constexpr int MAX = 1;
+    static __device__ __forceinline__ uint32_t key(uint32_t id, uint32_t side, uint32_t) { return id * 2u + side; }
+    static __device__ __forceinline__ uint32_t id(uint32_t key) { return key >> 1; }
+    static __device__ __forceinline__ uint32_t side(uint32_t key) { return key & 1u; }
+    static __device__ __forceinline__ uint32_t pair(uint32_t) { return 0u; }
+    static __device__ __forceinline__ uint32_t home(uint32_t key) { return key; }
+};
+struct BatchPairs {  // in shared memory
+    uint32_t a[8], b[8], nw[8];
+    i64 count[8];
+    int touch[64];  // matches of pair i (row) followed at once by one of pair k (column)
+    int n;
+};
+
 template <typename T>
 struct MergeGeom {
     static constexpr int WARPS = sizeof(T) == 2 ? 20 : 16;  // one CTA per SM; the wide stream needs twice the shared memory per warp
     static constexpr int THREADS = WARPS * 32;
     static constexpr int RAW_WORDS = 32 * Tok<T>::PITCH;
     static constexpr int WARP_WORDS = RAW_WORDS + 32;  // tile, live masks of the rewritten tile
-    static constexpr size_t BYTES = (size_t)WARPS * WARP_WORDS * 4 + (size_t)STBPE_AGG * 10 + STBPE_LIST * 4;
+    static constexpr size_t BYTES = (size_t)WARPS * WARP_WORDS * 4 + (size_t)STBPE_AGG * 10 + STBPE_LIST * 5 + STBPE_LIST_UNITS * Batch<T>::MAX * 4 + sizeof(BatchPairs);
 };
 
-enum { CTR_LIST, CTR_AGG, CTR_NN, CTR_BA, CTR_REMOVED, CTR_MATCHES, CTR_SEAM, CTR_FRESH, CTR_TILES, CTR_UNITS, CTR_RECS, CTR_N };
+enum { CTR_LIST, CTR_AGG, CTR_REMOVED, CTR_MATCHES, CTR_SEAM, CTR_FRESH, CTR_TILES, CTR_UNITS, CTR_RECS, CTR_N };
 
 struct CtaMerge {
     uint32_t *warp_mem;    // WARPS x WARP_WORDS
-    uint32_t *agg_key;     // neighbour id * 2 + side, or STBPE_NONE
+    BatchPairs *p;
+    uint32_t *agg_key;     // Batch<T>::key, or STBPE_NONE
     int *agg_val;
     uint16_t *agg_list;    // taken entries in order of arrival
-    uint32_t *list;        // tiles to visit
+    uint32_t *list;        // tiles to visit ...
+    unsigned char *list_pairs;  // ... and the pairs that may occur there
+    uint32_t *unit_bits;   // [pair][unit] tiles of the filter units at hand
     int *ctr;              // CTR_N counters
 
     template <typename T>
     __device__ __forceinline__ unsigned char *carve(unsigned char *base, int *counters) {
         warp_mem = reinterpret_cast<uint32_t *>(base);
         base += (size_t)MergeGeom<T>::WARPS * MergeGeom<T>::WARP_WORDS * 4;
+        p = reinterpret_cast<BatchPairs *>(base);
+        base += sizeof(BatchPairs);
         agg_key = reinterpret_cast<uint32_t *>(base);
         base += STBPE_AGG * 4;
         agg_val = reinterpret_cast<int *>(base);
@@ -63,6 +100,10 @@ struct CtaMerge {
         base += STBPE_AGG * 2;
         list = reinterpret_cast<uint32_t *>(base);
         base += STBPE_LIST * 4;
+        list_pairs = base;
+        base += STBPE_LIST;
+        unit_bits = reinterpret_cast<uint32_t *>(base);
+        base += STBPE_LIST_UNITS * Batch<T>::MAX * 4;
         ctr = counters;
         return base;
     }
@@ -72,14 +113,14 @@ struct CtaMerge {
             agg_val[i] = 0;
         }
         if (threadIdx.x < CTR_N) ctr[threadIdx.x] = 0;
+        if (threadIdx.x < 64) p->touch[threadIdx.x] = 0;
     }
 };
 
 struct MergeCtx {
-    uint32_t a, b, nw;
-    int m;         // number of this merge (>= 1)
+    int m;         // number of the batch's last merge (>= 1)
     bool fv;       // the pair filter is being maintained
-    i64 zero;      // this CTA takes this count off the pair (a, b) itself: none survives its own merge.  (Subtracted,
+    bool zero;     // this CTA takes the counts off the pairs (a, b) themselves: none survives its own merge.  (Subtracted,
                    // not overwritten: an id the host gives may already occur, and its pairs are being added to.)
     Theta theta;   // threshold of the candidate list (one rank)
 };
@@ -111,23 +152,23 @@ __device__ __forceinline__ uint32_t lds_u32_volatile(const uint32_t *p) {
     return v;
 }
 
-// the two pair-table terms of one neighbour: c matches had token `id` on their left (side 0) or right (side 1)
-__device__ __forceinline__ u64 gone_key(const MergeCtx &c, uint32_t id, uint32_t side) {
-    return side ? (((u64)c.b << 32) | id) : (((u64)id << 32) | c.a);
+// the two pair-table terms of one neighbour: matches of pair k had token `id` on their left (side 0) or right (side 1)
+__device__ __forceinline__ u64 gone_key(const BatchPairs *p, uint32_t k, uint32_t id, uint32_t side) {
+    return side ? (((u64)p->b[k] << 32) | id) : (((u64)id << 32) | p->a[k]);
 }
-__device__ __forceinline__ u64 made_key(const MergeCtx &c, uint32_t id, uint32_t side) {
-    return side ? (((u64)c.nw << 32) | id) : (((u64)id << 32) | c.nw);
+__device__ __forceinline__ u64 made_key(const BatchPairs *p, uint32_t k, uint32_t id, uint32_t side) {
+    return side ? (((u64)p->nw[k] << 32) | id) : (((u64)id << 32) | p->nw[k]);
 }
 
-// Slow path: probe for the entry, claim a free one, or give up.  The entry a key starts at is its low bits:
-// while the vocabulary is small (which is when merges have many matches) no two keys share one.
-template <bool MG>
-static __device__ __noinline__ void agg_probe(uint32_t *agg_key, int *ctr, const EngineDev &e, uint32_t a, uint32_t b, uint32_t nw,
-                                              i64 theta_count, u64 theta_key, uint32_t key) {
+// Slow path: probe for the entry, claim a free one, or give up.
+template <typename T, bool MG>
+static __device__ __noinline__ void agg_probe(uint32_t *agg_key, int *ctr, const EngineDev &e, const BatchPairs *p, i64 theta_count, u64 theta_key,
+                                              uint32_t key) {
     // arguments by value: a structure whose address escapes would be re-read from memory after every asm statement
+    typedef Batch<T> B;
     int *agg_val = reinterpret_cast<int *>(agg_key + STBPE_AGG);
     uint16_t *agg_list = reinterpret_cast<uint16_t *>(agg_val + STBPE_AGG);
-    uint32_t h = key & (STBPE_AGG - 1);
+    uint32_t h = B::home(key) & (STBPE_AGG - 1);
 #pragma unroll 1
     for (int probe = 0; probe < 16; ++probe) {
         uint32_t k = lds_u32_volatile(&agg_key[h]);
@@ -144,30 +185,44 @@ static __device__ __noinline__ void agg_probe(uint32_t *agg_key, int *ctr, const
         }
         h = (h + 1) & (STBPE_AGG - 1);
     }
-    MergeCtx c;
-    c.a = a, c.b = b, c.nw = nw;
-    c.theta.count = theta_count, c.theta.key = theta_key;
+    Theta theta;
+    theta.count = theta_count, theta.key = theta_key;
     unsigned int fresh = 0;
 #pragma unroll 1
     for (int made = 0; made < 2; ++made)
-        merge_sink<MG>(e, made ? made_key(c, key >> 1, key & 1u) : gone_key(c, key >> 1, key & 1u), made ? 1 : -1, made != 0, fresh, c.theta);
+        merge_sink<MG>(e, made ? made_key(p, B::pair(key), B::id(key), B::side(key)) : gone_key(p, B::pair(key), B::id(key), B::side(key)), made ? 1 : -1,
+                       made != 0, fresh, theta);
     if (fresh) atomicAdd(&e.st->n_keys, (u64)fresh);
 }
 
 // An entry keeps its key until the histogram is flushed, so a plain load that sees the key is final.
-template <bool MG>
-__device__ __forceinline__ void agg_add(const CtaMerge &s, const EngineDev &e, const MergeCtx &c, uint32_t id, uint32_t side) {
-    const uint32_t key = id * 2u + side, h = key & (STBPE_AGG - 1);
+template <typename T, bool MG>
+__device__ __forceinline__ void agg_add(const CtaMerge &s, const EngineDev &e, const MergeCtx &c, uint32_t id, uint32_t side, uint32_t pair) {
+    const uint32_t key = Batch<T>::key(id, side, pair), h = Batch<T>::home(key) & (STBPE_AGG - 1);
     uint32_t k;
     asm("ld.shared.u32 %0, [%1];" : "=r"(k) : "r"(smem_addr(&s.agg_key[h])));
     if (k == key)
         reds_add_s32(&s.agg_val[h], 1);
     else
-        agg_probe<MG>(s.agg_key, s.ctr, e, c.a, c.b, c.nw, c.theta.count, c.theta.key, key);
+        agg_probe<T, MG>(s.agg_key, s.ctr, e, s.p, c.theta.count, c.theta.key, key);
+}
+
+// the pair whose second (first) token this is; the caller knows that there is one, or n for none
+__device__ __forceinline__ int pair_ending(const BatchPairs *p, uint32_t id) {
+    int k = 0;
+#pragma unroll 1
+    while (k < p->n && p->b[k] != id) ++k;
+    return k;
+}
+__device__ __forceinline__ int pair_starting(const BatchPairs *p, uint32_t id) {
+    int k = 0;
+#pragma unroll 1
+    while (k < p->n && p->a[k] != id) ++k;
+    return k;
 }
 
 struct WarpStats {  // per lane
-    int removed, matches, nn, ba, seam, units, recs;
+    int removed, matches, seam, units, recs;
     int tiles;  // per warp
 };
 
@@ -186,17 +241,18 @@ __device__ __forceinline__ int pick_rec(const uint4 &rv, int k, int m) {
 }
 
 // One warp, one tile (already in the warp's shared-memory slot; every lane reads and writes its own group of
-// 32 tokens only).  `rv`: load_recs3 of the tile.
+// 32 tokens only).  `rv`: load_recs3 of the tile; `pm`: the pairs that may occur in it (bit k = pair k).
 template <typename T, bool MG>
 __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s, const MergeCtx &c, uint32_t *wm, int lane,
-                                           int tile, const uint4 &rv, WarpStats &ws) {
+                                           int tile, uint32_t pm, const uint4 &rv, WarpStats &ws) {
     typedef Tok<T> K;
+    constexpr bool MANY = Batch<T>::MAX > 1;
     T *tok = reinterpret_cast<T *>(wm + lane * K::PITCH);
-    const bool same = c.a == c.b;
+    const BatchPairs *const P = s.p;
 
-    uint32_t A, B, L, F;
-    group_masks((const T *)nullptr, wm + lane * K::PITCH, c.a, c.b, A, B, L, F);
-    B &= ~F;  // a partner does not start a row
+    uint32_t L, F;
+    Group<T> grp;
+    grp.load(wm + lane * K::PITCH, L, F);
     const uint32_t ne = __ballot_sync(0xFFFFFFFFu, L != 0u);
     if (ne == 0u) return;  // every token of the tile is gone
     // the live tokens right before and right behind the tile: from the neighbours' records, or by walking
@@ -219,93 +275,150 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
     const uint32_t top = L ? 0x80000000u >> __clz(L) : 0u;   // ... and its last
     const uint32_t above = ne & ~((2u << lane) - 1u), below = ne & ((1u << lane) - 1u);
     const int up = __ffs(above) - 1, down = 31 - __clz(below);  // the next lanes that hold live tokens, if any
-    // match heads: positions of A whose next live position is in B
-    const uint32_t fb = __ballot_sync(0xFFFFFFFFu, (B & low) != 0u);
-    uint32_t M = A & prev_live_bits(B, H);
-    if ((A & top) && (above ? ((fb >> up) & 1u) != 0u : h.nxt[0] == c.b)) M |= top;
+    // match heads: positions of some a_k whose next live position holds b_k.  k0, k1, k2: bits of k at the heads.
+    uint32_t M = 0, k0 = 0, k1 = 0, k2 = 0;
+    int kt = -1, kl = -1;  // the pair whose a is this lane's last token, the pair whose b is its first
+#pragma unroll 1
+    for (uint32_t left = pm; left; left &= left - 1u) {
+        const int k = MANY ? __ffs(left) - 1 : 0;
+        const uint32_t a = P->a[k], b = P->b[k];
+        const uint32_t A = grp.eq(a), B = grp.eq(b) & ~F;  // a partner does not start a row
+        const uint32_t hd = A & prev_live_bits(B, H);
+        M |= hd;
+        if (A & top) kt = k;
+        if (B & low) kl = k;
+        if (MANY) {
+            if (k & 1) k0 |= hd;
+            if (k & 2) k1 |= hd;
+            if (k & 4) k2 |= hd;
+        }
+    }
+    {
+        const int kn = __shfl_sync(0xFFFFFFFFu, kl, above ? up : lane);
+        if (kt >= 0 && (above ? kn == kt : h.nxt[0] == P->b[kt])) {
+            M |= top;
+            if (MANY) {
+                if (kt & 1) k0 |= top;
+                if (kt & 2) k1 |= top;
+                if (kt & 4) k2 |= top;
+            }
+        }
+    }
     // dropped positions: the next live position of every head
     const uint32_t hb = __ballot_sync(0xFFFFFFFFu, (M & top) != 0u);
-    const bool carry_in = below == 0u && (B & low) != 0u && (h.prev & STBPE_IDMASK) == c.a;
-    uint32_t D = next_live_bits(M, H);
-    if (below ? ((hb >> down) & 1u) != 0u : carry_in) D |= low;
+    const bool carry_in = below == 0u && kl >= 0 && (h.prev & STBPE_IDMASK) == P->a[kl];
+    const uint32_t D_in = next_live_bits(M, H);
+    const bool low_gone = below ? ((hb >> down) & 1u) != 0u : carry_in;  // this lane's first token is dropped (L != 0 implied)
+    const uint32_t D = D_in | (low_gone ? low : 0u);
     const uint32_t touched = M | D;
     if (__ballot_sync(0xFFFFFFFFu, touched != 0u) == 0u) return;  // nothing to merge here
     ws.matches += __popc(M);
     ws.removed += __popc(D);
     const int first_lane = __ffs(ne) - 1, last_lane = 31 - __clz(ne);
     const bool last_head = ((hb >> last_lane) & 1u) != 0u;  // its partner sits in another tile
-    if (!near) {
-    } else if (last_head || __any_sync(0xFFFFFFFFu, lane == last_lane && (D & top) && h.nxt[0] == c.a)) {
+    if (near) {
+        h.prev2 = __shfl_sync(0xFFFFFFFFu, rv.z, lp + 1);
         h.nxt[1] = __shfl_sync(0xFFFFFFFFu, rv.w, ln);
         h.nxt[2] = __shfl_sync(0xFFFFFFFFu, rv.x, ln + 1);
     }
-    if (near && h.prev == c.b) h.prev2 = __shfl_sync(0xFFFFFFFFu, rv.z, lp + 1);
-
-    // ---- the neighbours whose pairs change.  Every left neighbour belongs to one match (a != b) or run (a == b),
-    // and so does every right one, so their positions are all that is needed.
-    const uint32_t lefts = (same ? M & ~D : M) & ~F;  // heads that have a left neighbour
-    const uint32_t ends = same ? D & ~M : D & ~(carry_in ? low : 0u);  // what has its right neighbour accounted for here
-    uint32_t X = prev_live_bits(lefts, H), Y = next_live_bits(ends, H);
-    const uint32_t xb = __ballot_sync(0xFFFFFFFFu, (lefts & low) != 0u), yb = __ballot_sync(0xFFFFFFFFu, (ends & top) != 0u);
-    if (above && ((xb >> up) & 1u)) X |= top;
-    if (below && ((yb >> down) & 1u)) Y |= low;
-    Y &= ~F;
-    int nn = __popc(X & D), ba = __popc(Y & M);  // neighbours that belong to another match: (new, new)
-    X &= ~D;
-    Y &= ~M;
-    uint32_t x_out = STBPE_NONE, y_out = STBPE_NONE;  // neighbours in other tiles
-    int y_tile = h.next_tile;
-    if (lane == first_lane && (lefts & low)) {
-        if (!same && h.prev == c.b && (h.prev2 & STBPE_IDMASK) == c.a)
-            nn += 1;
-        else
-            x_out = h.prev & STBPE_IDMASK;
+    const uint32_t heads = M & ~D;  // (a position in both is inside a run of equal tokens)
+    // ---- the neighbours whose pairs change.  What lies beyond this lane's group, to the left (id, is it dropped) ...
+    uint32_t xid, yid;
+    bool xdrop, yskip;
+    {
+        const uint32_t tid = L ? (uint32_t)tok[K::sindex(31 - __clz(L))] & K::IDMASK : 0u;
+        const uint32_t tgone = __ballot_sync(0xFFFFFFFFu, (D & top) != 0u);
+        xid = __shfl_sync(0xFFFFFFFFu, tid, below ? down : lane);
+        xdrop = below && ((tgone >> down) & 1u);
+        // ... and to the right (id, does it start a row or head a match)
+        const uint32_t fid = L ? (uint32_t)tok[K::sindex(__ffs(L) - 1)] & K::IDMASK : 0u;
+        const uint32_t fskip = __ballot_sync(0xFFFFFFFFu, ((F | heads) & low) != 0u);
+        yid = __shfl_sync(0xFFFFFFFFu, fid, above ? up : lane);
+        yskip = above && ((fskip >> up) & 1u);
     }
-    if (lane == last_lane) {
-        uint32_t y = STBPE_NONE, y2 = STBPE_NONE;
-        if (ends & top) {
-            y = h.nxt[0], y2 = h.nxt[1];
-        } else if (!same && last_head) {
-            y = h.nxt[1], y2 = h.nxt[2];
-            y_tile = h.next2_tile;
+    if (!below) {
+        xid = h.prev & STBPE_IDMASK;
+        const int i = pair_ending(P, h.prev);
+        xdrop = i < P->n && (h.prev2 & STBPE_IDMASK) == P->a[i];
+    }
+    if (!above) {
+        yid = h.nxt[0];
+        const int i = pair_starting(P, h.nxt[0]);
+        yskip = (yid & STBPE_FLAG) || (i < P->n && h.nxt[1] == P->b[i]);
+    }
+#pragma unroll 1
+    for (uint32_t o = heads & ~F; o; o &= o - 1u) {
+        const int q = __ffs(o) - 1;
+        const uint32_t k = MANY ? ((k0 >> q) & 1u) | (((k1 >> q) & 1u) << 1) | (((k2 >> q) & 1u) << 2) : 0u;
+        const uint32_t l = L & ((1u << q) - 1u);
+        uint32_t id = xid;
+        bool drop = xdrop;
+        if (l) {
+            const int p = 31 - __clz(l);
+            id = (uint32_t)tok[K::sindex(p)] & K::IDMASK;
+            drop = (D >> p) & 1u;
         }
-        if (!(y & STBPE_FLAG)) {
-            if (!same && y == c.a && y2 == c.b)
-                ba += 1;
-            else
-                y_out = y;
+        u64 made;
+        if (drop) {
+            const int i = pair_ending(P, id);
+            reds_add_s32(&s.p->touch[i * 8 + k], 1);
+            made = ((u64)P->nw[i] << 32) | P->nw[k];
+        } else {
+            agg_add<T, MG>(s, e, c, id, 0u, k);
+            made = made_key(P, k, id, 0u);
+        }
+        if (c.fv) filter_set(e, tile, l || below ? -1 : h.prev_tile, made);
+    }
+    // of a match whose head sits in the tile before, the head's tile takes care (of a run, the last token's tile)
+    const bool foreign = carry_in && P->a[kl] != P->b[kl];
+    uint32_t d0 = 0, d1 = 0, d2 = 0;
+    if (MANY) {
+        d0 = next_live_bits(k0, H), d1 = next_live_bits(k1, H), d2 = next_live_bits(k2, H);
+        if (low_gone) {  // then kl is its pair
+            if (kl & 1) d0 |= low;
+            if (kl & 2) d1 |= low;
+            if (kl & 4) d2 |= low;
         }
     }
-    ws.nn += nn;
-    ws.ba += ba;
-    if (c.fv && __any_sync(0xFFFFFFFFu, nn + ba != 0) && lane == 0)  // either match of such a pair enters it for its own tile
-        filter_set(e, tile, -1, ((u64)c.nw << 32) | c.nw);
 #pragma unroll 1
-    for (; X; X &= X - 1u) {
-        const uint32_t id = tok[K::sindex(__ffs(X) - 1)] & K::IDMASK;
-        agg_add<MG>(s, e, c, id, 0u);
-        if (c.fv) filter_set(e, tile, -1, made_key(c, id, 0u));
+    for (uint32_t o = D & ~M & ~(foreign ? low : 0u); o; o &= o - 1u) {
+        const int r = __ffs(o) - 1;
+        const uint32_t k = MANY ? ((d0 >> r) & 1u) | (((d1 >> r) & 1u) << 1) | (((d2 >> r) & 1u) << 2) : 0u;
+        const uint32_t u = L & ~((2u << r) - 1u);
+        uint32_t id = yid;
+        bool skip = yskip;
+        if (u) {
+            const int p = __ffs(u) - 1;
+            id = (uint32_t)tok[K::sindex(p)] & K::IDMASK;
+            skip = ((F | heads) >> p) & 1u;
+        }
+        if (skip) continue;
+        agg_add<T, MG>(s, e, c, id, 1u, k);
+        if (c.fv) filter_set(e, tile, u || above ? -1 : h.next_tile, made_key(P, k, id, 1u));
     }
-#pragma unroll 1
-    for (; Y; Y &= Y - 1u) {
-        const uint32_t id = tok[K::sindex(__ffs(Y) - 1)] & K::IDMASK;
-        agg_add<MG>(s, e, c, id, 1u);
-        if (c.fv) filter_set(e, tile, -1, made_key(c, id, 1u));
-    }
-    if (x_out != STBPE_NONE || y_out != STBPE_NONE) {
-#pragma unroll 1
-        for (uint32_t side = 0; side < 2; ++side) {
-            const uint32_t id = side ? y_out : x_out;
-            if (id == STBPE_NONE) continue;
-            agg_add<MG>(s, e, c, id, side);
-            if (c.fv) filter_set(e, tile, side ? y_tile : h.prev_tile, made_key(c, id, side));
+    if (last_head && lane == last_lane) {
+        if (P->a[kt] != P->b[kt]) {
+            const uint32_t y = h.nxt[1];
+            const int i = pair_starting(P, y);
+            if (i < P->n && h.nxt[2] == P->b[i]) {
+                // y's tile counts the two touching matches, but sees the dropped token only, not the new one here
+                if (c.fv) filter_set(e, tile, -1, ((u64)P->nw[kt] << 32) | P->nw[i]);
+            } else if (!(y & STBPE_FLAG)) {
+                agg_add<T, MG>(s, e, c, y, 1u, (uint32_t)kt);
+                if (c.fv) filter_set(e, tile, h.next2_tile, made_key(P, kt, y, 1u));
+            }
+        } else if (c.fv) {
+            // a run of a's that goes on in the next tile: the pair that will start at the collapsed token is
+            // decided by whoever finds the run's tail, so visit this tile from now on
+            atomicOr(e.presence + (size_t)((unsigned int)tile >> 5) * STBPE_PPITCH + STBPE_PROWS, 1u << (tile & 31));
         }
     }
     // ---- rewrite (no neighbour counted above is a position that changes)
 #pragma unroll 1
-    for (uint32_t o = M & ~D; o; o &= o - 1u) {
+    for (uint32_t o = heads; o; o &= o - 1u) {
         const int p = __ffs(o) - 1;
-        tok[K::sindex(p)] = (T)(c.nw | ((F >> p) & 1u ? K::FLAG : 0u));
+        const uint32_t k = MANY ? ((k0 >> p) & 1u) | (((k1 >> p) & 1u) << 1) | (((k2 >> p) & 1u) << 2) : 0u;
+        tok[K::sindex(p)] = (T)(P->nw[k] | ((F >> p) & 1u ? K::FLAG : 0u));
     }
 #pragma unroll 1
     for (uint32_t o = D; o; o &= o - 1u) tok[K::sindex(__ffs(o) - 1)] = (T)K::HOLE;
@@ -322,13 +435,7 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
     const int newlen = __reduce_add_sync(0xFFFFFFFFu, __popc(NL));
     if (lane == 0) {
         e.tile_live[tile] = (unsigned int)newlen;
-        if (last_head) {
-            ws.seam += 1;
-            // a run of a's that goes on in the next tile: the pair that will start at the collapsed token is
-            // decided by whoever finds the run's tail, so visit this tile from now on
-            if (c.fv && same)
-                atomicOr(e.presence + (size_t)((unsigned int)tile >> 5) * STBPE_PPITCH + STBPE_PROWS, 1u << (tile & 31));
-        }
+        if (last_head) ws.seam += 1;
     }
     // ---- the record, unless the tile's first three and last two live tokens are as they were
     const uint32_t l2 = L & ~low, l3 = l2 & (l2 - 1u), low3 = L & ~(l3 & (l3 - 1u));
@@ -362,7 +469,7 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
     }
 }
 
-// Applies the merge to this CTA's tiles and adds its delta terms to the pair table (or, several ranks, to
+// Applies the batch of merges to this CTA's tiles and adds its delta terms to the pair table (or, several ranks, to
 // the rank-local delta table).  `unit_shift`: log2 of the tiles per filter unit; CTA c takes the units c,
 // c + gridDim.x, ... (words of the filter when there are enough of them, single tiles on a small stream).
 // Ends with all of the CTA's adds issued; the caller synchronises.
@@ -372,28 +479,49 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
     constexpr int WARPS = MergeGeom<T>::WARPS;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t *wm = s.warp_mem + (size_t)warp * MergeGeom<T>::WARP_WORDS;
-    WarpStats ws = {0, 0, 0, 0, 0, 0, 0, 0};
+    WarpStats ws = {0, 0, 0, 0, 0, 0};
+    const int nb = Batch<T>::MAX > 1 ? s.p->n : 1;
     // Without the filter: every tile, consecutive tiles on different CTAs so that a small stream uses all of
     // them.  With it: batches of filter units, each turned into a list of tiles that the warps share.
-    unsigned int r1, r2, r3;
-    filter_rows(((u64)c.a << 32) | (u64)c.b, r1, r2, r3);
     const i64 n_units = c.fv ? ((i64)e.n_tiles + (1 << unit_shift) - 1) >> unit_shift : blockIdx.x + 1;
     const uint32_t unit_bits = unit_shift == 5 ? 0xFFFFFFFFu : (1u << (1 << unit_shift)) - 1u;
 #pragma unroll 1
     for (i64 u0 = blockIdx.x; u0 < n_units; u0 += (i64)STBPE_LIST_UNITS * gridDim.x) {
         int n = (e.n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;  // tiles blockIdx.x, + gridDim.x, ...
         if (c.fv) {
-            const i64 u = u0 + (i64)threadIdx.x * gridDim.x;
-            if (threadIdx.x < STBPE_LIST_UNITS && u < n_units) {
-                const i64 t0 = u << unit_shift, w = t0 >> 5;
-                const unsigned int *g = e.presence + (size_t)w * STBPE_PPITCH;
-                uint32_t bits = (__ldcg(g + r1) & __ldcg(g + r2) & __ldcg(g + r3)) | __ldcg(g + STBPE_PROWS);
-                bits &= unit_bits << (t0 & 31);
-                if (e.n_tiles - w * 32 < 32) bits &= (1u << (e.n_tiles - w * 32)) - 1u;
-                if (bits) {
-                    int at = atoms_add_s32(&s.ctr[CTR_LIST], __popc(bits));
+            // one thread per pair and unit asks the filter ...
+            const int k = threadIdx.x / STBPE_LIST_UNITS, at = threadIdx.x % STBPE_LIST_UNITS;
+            if (k < nb) {
+                const i64 u = u0 + (i64)at * gridDim.x;
+                uint32_t bits = 0;
+                if (u < n_units) {
+                    const i64 t0 = u << unit_shift, w = t0 >> 5;
+                    const unsigned int *g = e.presence + (size_t)w * STBPE_PPITCH;
+                    unsigned int r1, r2, r3;
+                    filter_rows(((u64)s.p->a[k] << 32) | (u64)s.p->b[k], r1, r2, r3);
+                    bits = (__ldcg(g + r1) & __ldcg(g + r2) & __ldcg(g + r3)) | __ldcg(g + STBPE_PROWS);
+                    bits &= unit_bits << (t0 & 31);
+                    if (e.n_tiles - w * 32 < 32) bits &= (1u << (e.n_tiles - w * 32)) - 1u;
+                }
+                s.unit_bits[threadIdx.x] = bits;
+            }
+            __syncthreads();
+            // ... and a warp per unit lists the tiles that any pair needs, lane = tile of the filter word
 #pragma unroll 1
-                    for (; bits; bits &= bits - 1u) s.list[at++] = (uint32_t)(w * 32 + __ffs(bits) - 1);
+            for (int i = warp; i < STBPE_LIST_UNITS; i += WARPS) {
+                const uint32_t own = lane < nb ? s.unit_bits[lane * STBPE_LIST_UNITS + i] : 0u;
+                const uint32_t any = __reduce_or_sync(0xFFFFFFFFu, own);
+                if (any == 0u) continue;
+                uint32_t pairs = 0;
+#pragma unroll 1
+                for (int q = 0; q < nb; ++q) pairs |= ((__shfl_sync(0xFFFFFFFFu, own, q) >> lane) & 1u) << q;
+                int at0 = 0;
+                if (lane == 0) at0 = atoms_add_s32(&s.ctr[CTR_LIST], __popc(any));
+                at0 = __shfl_sync(0xFFFFFFFFu, at0, 0) + __popc(any & ((1u << lane) - 1u));
+                if (pairs) {
+                    const i64 w = ((u0 + (i64)i * gridDim.x) << unit_shift) >> 5;
+                    s.list[at0] = (uint32_t)(w * 32 + lane);
+                    s.list_pairs[at0] = (unsigned char)pairs;
                 }
             }
             __syncthreads();
@@ -402,22 +530,25 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
         // the loads of a tile are issued before the one before it is worked on
         uint4 v[Tok<T>::VEC], rv;
         int cur = -1;
+        uint32_t pairs = (1u << nb) - 1u, next_pairs = pairs;
 #pragma unroll 1
         for (int j = warp;; j += WARPS) {
             if (cur >= 0) store_units<T>(wm, lane, v);
             const uint4 rc = rv;
             const int next = j < n ? (c.fv ? (int)s.list[j] : (int)blockIdx.x + j * (int)gridDim.x) : -1;
             if (next >= 0) {
+                if (c.fv) next_pairs = s.list_pairs[j];
                 load_units<T>(e, next, lane, v);
                 rv = load_recs3(e, next, lane);
             }
             __syncwarp();
             if (cur >= 0) {
-                merge_tile<T, MG>(e, s, c, wm, lane, cur, rc, ws);
+                merge_tile<T, MG>(e, s, c, wm, lane, cur, pairs, rc, ws);
                 ws.tiles += 1;
                 __syncwarp();
             }
             cur = next;
+            pairs = next_pairs;
             if (cur < 0) break;
         }
         if (c.fv) {
@@ -427,10 +558,10 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
         }
     }
     {
-        const int part[8] = {ws.nn, ws.ba, ws.removed, ws.matches, ws.seam, lane == 0 ? ws.tiles : 0, ws.units, ws.recs};
-        constexpr int slot[8] = {CTR_NN, CTR_BA, CTR_REMOVED, CTR_MATCHES, CTR_SEAM, CTR_TILES, CTR_UNITS, CTR_RECS};
+        const int part[6] = {ws.removed, ws.matches, ws.seam, lane == 0 ? ws.tiles : 0, ws.units, ws.recs};
+        constexpr int slot[6] = {CTR_REMOVED, CTR_MATCHES, CTR_SEAM, CTR_TILES, CTR_UNITS, CTR_RECS};
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < 6; ++k) {
             const int x = __reduce_add_sync(0xFFFFFFFFu, part[k]);
             if (lane == 0 && x) reds_add_s32(&s.ctr[slot[k]], x);
         }
@@ -438,35 +569,39 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
     before_adds();
     __syncthreads();
     // ---- neighbour histogram -> pair table: two lanes per neighbour, one for the pair that is gone and one for
-    // the pair that came into being; behind them (new, new), (b, a) and (a, b) itself
+    // the pair that came into being; behind them, likewise, the matches that touch, and the merged pairs themselves
+    constexpr int KB = Batch<T>::MAX, TOUCH = 2 * KB * 8;
     unsigned int fresh = 0;
-    const int n = s.ctr[CTR_AGG], total = 2 * n + 3;
+    const int n = s.ctr[CTR_AGG], total = 2 * n + TOUCH + KB;
 #pragma unroll 1
     for (int base = warp * 32; base < total; base += WARPS * 32) {
-        const int i = base + lane;
-        const bool made = i < 2 * n ? (i & 1) != 0 : i == 2 * n;
+        const int i = base + lane, t = i - 2 * n;
+        bool made = (i & 1) != 0;
         u64 key = 0;
         i64 delta = 0;
-        int h = -1;
-        if (i < 2 * n) {
-            h = s.agg_list[i >> 1];
-            const uint32_t k = s.agg_key[h];
-            delta = s.agg_val[h];
-            key = made ? made_key(c, k >> 1, k & 1u) : gone_key(c, k >> 1, k & 1u);
-        } else if (i == 2 * n) {
-            key = ((u64)c.nw << 32) | c.nw;
-            delta = s.ctr[CTR_NN];
-        } else if (i == 2 * n + 1) {
-            key = ((u64)c.b << 32) | c.a;
-            delta = s.ctr[CTR_BA];
-        } else if (i == 2 * n + 2) {
-            key = ((u64)c.a << 32) | c.b;
-            delta = c.zero;
+        int *used = nullptr;
+        if (t < 0) {
+            const int h = s.agg_list[i >> 1];
+            const uint32_t x = s.agg_key[h], k = Batch<T>::pair(x), id = Batch<T>::id(x), side = Batch<T>::side(x);
+            used = &s.agg_val[h];
+            delta = *used;
+            key = made ? made_key(s.p, k, id, side) : gone_key(s.p, k, id, side);
+        } else if (t < TOUCH) {
+            used = &s.p->touch[t >> 1];
+            delta = *used;
+            const int l = t >> 4, r = (t >> 1) & 7;
+            if (delta) key = made ? ((u64)s.p->nw[l] << 32) | s.p->nw[r] : ((u64)s.p->b[l] << 32) | s.p->a[r];
+        } else {
+            made = false;
+            if (c.zero && t - TOUCH < nb) {
+                key = ((u64)s.p->a[t - TOUCH] << 32) | s.p->b[t - TOUCH];
+                delta = s.p->count[t - TOUCH];
+            }
         }
         __syncwarp();  // both lanes of the entry have read it
-        if (h >= 0 && !made) {
-            s.agg_key[h] = STBPE_NONE;
-            s.agg_val[h] = 0;
+        if (used && !made) {
+            if (t < 0) s.agg_key[used - s.agg_val] = STBPE_NONE;
+            *used = 0;
         }
         if (delta) merge_sink<MG>(e, key, made ? delta : -delta, made, fresh, c.theta);
     }
@@ -503,10 +638,10 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) merge_kernel(const _
     s.carve<T>(smem_raw, s_ctr);
     s.clear();
     MergeCtx c;
-    c.a = (uint32_t)st->cur_a, c.b = (uint32_t)st->cur_b, c.nw = (uint32_t)st->cur_new;
+    if (threadIdx.x == 0) s.p->n = 1, s.p->a[0] = (uint32_t)st->cur_a, s.p->b[0] = (uint32_t)st->cur_b, s.p->nw[0] = (uint32_t)st->cur_new;
     c.m = st->merges_done;
     c.fv = st->filter_valid != 0;
-    c.zero = 0;  // done when the merge was selected
+    c.zero = false;  // done when the merge was selected
     c.theta.count = st->theta_count, c.theta.key = st->theta_key;
     if (!c.fv && blockIdx.x == 0 && threadIdx.x == 0) st->n_work = -1;
     __syncthreads();

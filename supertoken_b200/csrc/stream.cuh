@@ -83,47 +83,61 @@ __device__ __forceinline__ void load_group(const EngineDev &e, int tile, int lan
     }
 }
 
-// Masks of one group (bit i = token i): A = token with id a, B = token with id b, L = live, F = starts a row (or a
-// hole, which no id compares equal to).
-__device__ __forceinline__ void group_masks(const uint16_t *, const uint32_t *group, uint32_t a, uint32_t b, uint32_t &A,
-                                            uint32_t &B, uint32_t &L, uint32_t &F) {
-    const uint32_t aa = a | (a << 16), bb = b | (b << 16);
-    uint32_t na = 0, nb = 0, nl = 0, f = 0;  // collected as "differs" / "is a hole"
+// One group in registers: L = live tokens, F = tokens that start a row (or holes), eq(id) = tokens with that id.
+template <typename T>
+struct Group;
+template <>
+struct Group<uint16_t> {
+    uint32_t w[16];
+    __device__ __forceinline__ void load(const uint32_t *group, uint32_t &L, uint32_t &F) {
+        uint32_t nl = 0, f = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const uint4 q = *reinterpret_cast<const uint4 *>(group + 4 * j);
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+        for (int j = 0; j < 4; ++j) {
+            const uint4 q = *reinterpret_cast<const uint4 *>(group + 4 * j);
+            w[4 * j] = q.x, w[4 * j + 1] = q.y, w[4 * j + 2] = q.z, w[4 * j + 3] = q.w;
+        }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            // per half: x + 0x7FFF carries into the top bit iff x (15 bits) is not zero
-            const uint32_t za = ((w[i] & 0x7FFF7FFFu) ^ aa) + 0x7FFF7FFFu;
-            const uint32_t zb = ((w[i] & 0x7FFF7FFFu) ^ bb) + 0x7FFF7FFFu;
-            const uint32_t zl = (w[i] & 0x7FFF7FFFu) + 0x00010001u;  // only a hole has 0x7FFF in its low bits
-            na = (na >> 1) | (za & 0x80008000u);
-            nb = (nb >> 1) | (zb & 0x80008000u);
-            nl = (nl >> 1) | (zl & 0x80008000u);
+        for (int i = 0; i < 16; ++i) {
             f = (f >> 1) | (w[i] & 0x80008000u);
+            w[i] &= 0x7FFF7FFFu;
+            nl = (nl >> 1) | ((w[i] + 0x00010001u) & 0x80008000u);  // only a hole has 0x7FFF in its low bits
+        }
+        L = ~nl, F = f;
+    }
+    __device__ __forceinline__ uint32_t eq(uint32_t id) const {
+        const uint32_t two = id | (id << 16);
+        uint32_t n = 0;
+        // per half: x + 0x7FFF carries into the top bit iff x (15 bits) is not zero
+#pragma unroll
+        for (int i = 0; i < 16; ++i) n = (n >> 1) | (((w[i] ^ two) + 0x7FFF7FFFu) & 0x80008000u);
+        return ~n;
+    }
+};
+template <>
+struct Group<uint32_t> {
+    uint32_t w[32];
+    __device__ __forceinline__ void load(const uint32_t *group, uint32_t &L, uint32_t &F) {
+        L = F = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint4 q = *reinterpret_cast<const uint4 *>(group + 4 * j);
+            w[4 * j] = q.x, w[4 * j + 1] = q.y, w[4 * j + 2] = q.z, w[4 * j + 3] = q.w;
+        }
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            if (w[i] != STBPE_NONE) L |= 1u << i;
+            if (w[i] & STBPE_FLAG) F |= 1u << i;
+            w[i] &= STBPE_IDMASK;
         }
     }
-    A = ~na, B = ~nb, L = ~nl, F = f;
-}
-__device__ __forceinline__ void group_masks(const uint32_t *, const uint32_t *group, uint32_t a, uint32_t b, uint32_t &A,
-                                            uint32_t &B, uint32_t &L, uint32_t &F) {
-    A = B = L = F = 0;
+    __device__ __forceinline__ uint32_t eq(uint32_t id) const {
+        uint32_t m = 0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const uint4 q = *reinterpret_cast<const uint4 *>(group + 4 * j);
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t bit = 1u << (4 * j + i);
-            if ((w[i] & STBPE_IDMASK) == a) A |= bit;
-            if ((w[i] & STBPE_IDMASK) == b) B |= bit;
-            if (w[i] != STBPE_NONE) L |= bit;
-            if (w[i] & STBPE_FLAG) F |= bit;
-        }
+        for (int i = 0; i < 32; ++i)
+            if (w[i] == id) m |= 1u << i;
+        return m;
     }
-}
+};
 
 // live mask of a group held in registers
 template <typename T>
