@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
                     x = Bs::max2(x, v);
                 }
             };
-#pragma unroll 2
+#pragma unroll 4
             for (unsigned int i = tid; i < n_cand; i += THREADS) take(s_cand[i]);
 #pragma unroll 1
             for (unsigned int i = n_cand + tid; i < n_have; i += THREADS) {  // appended by the last merges
@@ -213,82 +213,85 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
         }
         __syncthreads();
         if (tid == THREADS - 1) red_release_u32(&sync->chosen, 1u);  // the CTA has read everything it decides by
-        // warp 0 decides; lane j holds what belongs to merge j of the batch
+        // warp 0 decides; lane j takes the j-th best pair (or the j-th one the host gives) and tests whether it can be
+        // merge j of the batch, given that all before it are
         if (warp == 0) {
             const Bt bound = KB > 1 ? Bs::warp_max(lane < WARPS ? s_rest[lane] : Bs::none()) : Bs::none();
-            Bt cur = lane < WARPS ? s_top[lane * TOP] : Bs::none();
-            int at = 0;
-            const unsigned int err = s_err;
-            const bool over = (err >> 31) != 0u, host = la.forced != nullptr;
-            const i64 live0 = s_live;
-            i64 live = live0, keys = s_keys, best_count = 0, own_count = 0, own_live = 0;
-            u64 best_key = STBPE_EMPTY;
-            bool best_dry = true;
-            uint32_t own_a = 0, own_b = 0;
-            int stop = 0, why = STBPE_EXIT_STOP, nb = 0;
-            const uint32_t nw0 = (uint32_t)(host ? la.forced_new + forced_i : base_vocab + merges_done);
-            const int most = fv ? KB : la.dense_batch < KB ? la.dense_batch : KB;
+            Bt c[TOP], mine = Bs::none();
+#pragma unroll
+            for (int r = 0; r < TOP; ++r) c[r] = lane < WARPS ? s_top[lane * TOP + r] : Bs::none();
+            const bool host = la.forced != nullptr;
 #pragma unroll 1
-            for (;; ++nb) {
-                const Bt v = Bs::warp_max(cur);
-                const Slot best = Bs::slot(v);
-                const bool dry = over || !(mc.theta.admits(best.count, best.key) || (best.count <= 0 && mc.theta.count == 0));
-                if (nb == 0) best_key = best.key, best_count = best.count, best_dry = dry;
-                const bool forced = host && forced_i + nb < la.n_forced;
-                u64 key = best.key;
-                i64 count = best.count;
-                if (forced) {
-                    const int2 f = la.forced[forced_i + nb];
-                    key = ((u64)(uint32_t)f.x << 32) | (uint32_t)f.y;
-                    count = nb < KB ? s_forced[nb] : 0;
-                }
-                const uint32_t a = (uint32_t)(key >> 32), b = (uint32_t)key, nw = nw0 + nb;
-                // a later member of the batch: exact order so far, no token shared with the members before, none of
-                // their new tokens (a pair given by the host may name one)
-                if (nb > 0) {
-                    if (nb >= most) break;
-                    if constexpr (KB > 1) {
-                        if (!host && !(v > bound)) break;
+            for (int j = 0; j < KB; ++j) {
+                const Bt v = Bs::warp_max(c[0]);
+                if (lane == j) mine = v;
+                if constexpr (KB > 1) {
+                    if (c[0] == v) {
+#pragma unroll
+                        for (int r = 0; r + 1 < TOP; ++r) c[r] = c[r + 1];
+                        c[TOP - 1] = Bs::none();
                     }
-                    if (max(a, b) >= nw0) break;
-                    if (__any_sync(0xFFFFFFFFu, lane < nb && (own_a == a || own_a == b || own_b == a || own_b == b))) break;
                 }
-                // stop rules of the loop: bpe_trainer.py:4304-4308 (no pairs), :2491-2494 / :4361-4364 (count < 2)
-                if (err & 0x7FFFFFFFu) stop = 4;
-                else if (host && !forced) stop = 0;
-                else if (!host && merges_done + nb >= la.target) stop = 1;
-                // maintenance the host does between launches
-                else if (!host && dry) why = STBPE_EXIT_REFILL;
-                else if (!host && count <= 0) stop = 2;
-                else if (!host && count < 2) stop = 3;
-                else if (e.n_tiles >= la.repack_tiles && live * 4 <= (i64)e.n_tiles * STBPE_TILE * 3) why = STBPE_EXIT_REPACK;
-                else if (!fv && e.n_tiles > 0 && count <= la.filter_count) why = STBPE_EXIT_FILTER;
-                // every merge makes at most two pairs per match and two per id
-                else if (keys + 2 * min(count, (i64)max((int)nw, la.ids_below)) + 2 > la.grow_keys) why = STBPE_EXIT_GROW;
-                else if (sizeof(T) == 2 && max(nw, max(a, b)) >= Tok<uint16_t>::IDMASK) why = STBPE_EXIT_WIDEN;
-                else {
-                    if (lane == nb) own_a = a, own_b = b, own_count = count, own_live = live;
-                    keys += 2 * min(count, (i64)max((int)nw, la.ids_below)) + 2;
-                    live -= count;  // a merge drops one token per occurrence of its pair (of a run, all but one)
-                    if constexpr (KB > 1) {
-                        if (cur == v) cur = ++at < TOP ? s_top[lane * TOP + at] : Bs::none();
-                    }
-                    continue;
-                }
-                break;
             }
+            const unsigned int err = s_err;
+            const Slot best = Bs::slot(mine);
+            const bool dry = (err >> 31) != 0u || !(mc.theta.admits(best.count, best.key) || (best.count <= 0 && mc.theta.count == 0));
+            const bool forced = host && lane < KB && forced_i + lane < la.n_forced;
+            u64 key = best.key;
+            i64 count = best.count;
+            if (forced) {
+                const int2 f = la.forced[forced_i + lane];
+                key = ((u64)(uint32_t)f.x << 32) | (uint32_t)f.y;
+                count = s_forced[lane];
+            }
+            const uint32_t a = (uint32_t)(key >> 32), b = (uint32_t)key;
+            const uint32_t nw0 = (uint32_t)(host ? la.forced_new + forced_i : base_vocab + merges_done), nw = nw0 + lane;
+            // every merge makes at most two pairs per match and two per id, and drops one token per occurrence of its pair (of
+            // a run, all but one)
+            const i64 grow = 2 * min(count, (i64)max((int)nw, la.ids_below)) + 2;
+            i64 live = s_live, keys = s_keys + grow;
+            // a later member: the order is exact so far, it shares no token with the members before and names none of their
+            // new ones (a pair that the host gives may)
+            bool out = lane >= (fv ? KB : min(la.dense_batch, KB));
+            if constexpr (KB > 1) out = out || (!host && !(mine > bound));
+            out = out || max(a, b) >= nw0;
+#pragma unroll
+            for (int j = 0; j + 1 < KB; ++j) {
+                const uint32_t ja = __shfl_sync(0xFFFFFFFFu, a, j), jb = __shfl_sync(0xFFFFFFFFu, b, j);
+                const i64 jc = __shfl_sync(0xFFFFFFFFu, count, j), jg = __shfl_sync(0xFFFFFFFFu, grow, j);
+                if (lane > j) {
+                    out = out || ja == a || ja == b || jb == a || jb == b;
+                    live -= jc, keys += jg;
+                }
+            }
+            // stop rules of the loop: bpe_trainer.py:4304-4308 (no pairs), :2491-2494 / :4361-4364 (count < 2)
+            int stop = 0, why = STBPE_EXIT_STOP;
+            bool go = false;
+            if (err & 0x7FFFFFFFu) stop = 4;
+            else if (host && !forced) stop = 0;
+            else if (!host && merges_done + lane >= la.target) stop = 1;
+            // maintenance the host does between launches
+            else if (!host && dry) why = STBPE_EXIT_REFILL;
+            else if (!host && count <= 0) stop = 2;
+            else if (!host && count < 2) stop = 3;
+            else if (e.n_tiles >= la.repack_tiles && live * 4 <= (i64)e.n_tiles * STBPE_TILE * 3) why = STBPE_EXIT_REPACK;
+            else if (!fv && e.n_tiles > 0 && count <= la.filter_count) why = STBPE_EXIT_FILTER;
+            else if (keys > la.grow_keys) why = STBPE_EXIT_GROW;
+            else if (sizeof(T) == 2 && max(nw, max(a, b)) >= Tok<uint16_t>::IDMASK) why = STBPE_EXIT_WIDEN;
+            else go = true;
+            const uint32_t bad = __ballot_sync(0xFFFFFFFFu, lane >= KB || !go || (lane > 0 && out));
+            const int nb = __ffs(bad) - 1;
             if (lane < nb) {
-                s.p->a[lane] = own_a, s.p->b[lane] = own_b, s.p->nw[lane] = nw0 + lane;
-                s.p->count[lane] = own_count;
+                s.p->template set<T>(lane, a, b, nw);
+                s.p->count[lane] = count;
                 if (cta == 0) {
                     const int m = merges_done + lane;
-                    e.merges[2 * m] = (int32_t)own_a;
-                    e.merges[2 * m + 1] = (int32_t)own_b;
-                    e.merge_counts[m] = own_count;
-                    e.live_before[m] = own_live;
+                    *reinterpret_cast<int2 *>(e.merges + 2 * m) = make_int2((int)a, (int)b);
+                    e.merge_counts[m] = count;
+                    e.live_before[m] = live;
                     if (lane == nb - 1) {
-                        st->cur_a = (int)own_a, st->cur_b = (int)own_b, st->cur_new = (int)(nw0 + lane);
-                        st->cur_count = own_count;
+                        st->cur_a = (int)a, st->cur_b = (int)b, st->cur_new = (int)nw;
+                        st->cur_count = count;
                     }
                 }
             }
@@ -300,9 +303,9 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
                     st->run_exit = why;
                     st->stopped = stop > 0;
                     st->stop_reason = stop;
-                    st->peek_key = best_key;
-                    st->peek_count = best_count;
-                    st->peek_valid = !best_dry;
+                    st->peek_key = best.key;
+                    st->peek_count = best.count;
+                    st->peek_valid = !dry;
                     st->forced_done = forced_i;
                     st->n_work = s_work;
                 }

@@ -58,10 +58,21 @@ struct Batch<uint32_t> {
     static __device__ __forceinline__ uint32_t home(uint32_t key) { return key; }
 };
 struct BatchPairs {  // in shared memory
+    PlaneId pa[8], pb[8];  // a and b once more, as Group::eq takes them
     uint32_t a[8], b[8], nw[8];
     i64 count[8];
     int touch[64];  // matches of pair i (row) followed at once by one of pair k (column)
     int n;
+    template <typename T>
+    __device__ __forceinline__ void set(int k, uint32_t x, uint32_t y, uint32_t new_id) {
+        a[k] = x, b[k] = y, nw[k] = new_id;
+        if (sizeof(T) == 2) {
+            pa[k].set(x);
+            pb[k].set(y);
+        } else {
+            pa[k].m[0].x = x, pb[k].m[0].x = y;
+        }
+    }
 };
 
 template <typename T>
@@ -281,8 +292,7 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
 #pragma unroll 1
     for (uint32_t left = pm; left; left &= left - 1u) {
         const int k = MANY ? __ffs(left) - 1 : 0;
-        const uint32_t a = P->a[k], b = P->b[k];
-        const uint32_t A = grp.eq(a), B = grp.eq(b) & ~F;  // a partner does not start a row
+        const uint32_t A = grp.eq(P->pa[k]), B = grp.eq(P->pb[k]) & ~F;  // a partner does not start a row
         const uint32_t hd = A & prev_live_bits(B, H);
         M |= hd;
         if (A & top) kt = k;
@@ -336,21 +346,25 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
         yid = __shfl_sync(0xFFFFFFFFu, fid, above ? up : lane);
         yskip = above && ((fskip >> up) & 1u);
     }
-    if (!below) {
+    const uint32_t ends = D & ~M;  // last tokens of matches and runs
+    if (!below && (heads & ~F & low)) {
         xid = h.prev & STBPE_IDMASK;
         const int i = pair_ending(P, h.prev);
         xdrop = i < P->n && (h.prev2 & STBPE_IDMASK) == P->a[i];
     }
-    if (!above) {
+    if (!above && (ends & top)) {
         yid = h.nxt[0];
         const int i = pair_starting(P, h.nxt[0]);
         yskip = (yid & STBPE_FLAG) || (i < P->n && h.nxt[1] == P->b[i]);
     }
 #pragma unroll 1
-    for (uint32_t o = heads & ~F; o; o &= o - 1u) {
+    for (uint32_t o = heads; o; o &= o - 1u) {
         const int q = __ffs(o) - 1;
         const uint32_t k = MANY ? ((k0 >> q) & 1u) | (((k1 >> q) & 1u) << 1) | (((k2 >> q) & 1u) << 2) : 0u;
-        const uint32_t l = L & ((1u << q) - 1u);
+        const uint32_t nw = P->nw[k], l = L & ((1u << q) - 1u);
+        const bool starts = (F >> q) & 1u;
+        tok[K::sindex(q)] = (T)(nw | (starts ? K::FLAG : 0u));
+        if (starts) continue;
         uint32_t id = xid;
         bool drop = xdrop;
         if (l) {
@@ -362,15 +376,15 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
         if (drop) {
             const int i = pair_ending(P, id);
             reds_add_s32(&s.p->touch[i * 8 + k], 1);
-            made = ((u64)P->nw[i] << 32) | P->nw[k];
+            made = ((u64)P->nw[i] << 32) | nw;
         } else {
             agg_add<T, MG>(s, e, c, id, 0u, k);
-            made = made_key(P, k, id, 0u);
+            made = ((u64)id << 32) | nw;
         }
         if (c.fv) filter_set(e, tile, l || below ? -1 : h.prev_tile, made);
     }
     // of a match whose head sits in the tile before, the head's tile takes care (of a run, the last token's tile)
-    const bool foreign = carry_in && P->a[kl] != P->b[kl];
+    const uint32_t own = ends & ~(carry_in && P->a[kl] != P->b[kl] ? low : 0u);
     uint32_t d0 = 0, d1 = 0, d2 = 0;
     if (MANY) {
         d0 = next_live_bits(k0, H), d1 = next_live_bits(k1, H), d2 = next_live_bits(k2, H);
@@ -381,9 +395,9 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
         }
     }
 #pragma unroll 1
-    for (uint32_t o = D & ~M & ~(foreign ? low : 0u); o; o &= o - 1u) {
+    for (uint32_t o = D; o; o &= o - 1u) {
         const int r = __ffs(o) - 1;
-        const uint32_t k = MANY ? ((d0 >> r) & 1u) | (((d1 >> r) & 1u) << 1) | (((d2 >> r) & 1u) << 2) : 0u;
+        tok[K::sindex(r)] = (T)K::HOLE;
         const uint32_t u = L & ~((2u << r) - 1u);
         uint32_t id = yid;
         bool skip = yskip;
@@ -392,7 +406,8 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
             id = (uint32_t)tok[K::sindex(p)] & K::IDMASK;
             skip = ((F | heads) >> p) & 1u;
         }
-        if (skip) continue;
+        if (skip || !((own >> r) & 1u)) continue;
+        const uint32_t k = MANY ? ((d0 >> r) & 1u) | (((d1 >> r) & 1u) << 1) | (((d2 >> r) & 1u) << 2) : 0u;
         agg_add<T, MG>(s, e, c, id, 1u, k);
         if (c.fv) filter_set(e, tile, u || above ? -1 : h.next_tile, made_key(P, k, id, 1u));
     }
@@ -413,15 +428,7 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
             atomicOr(e.presence + (size_t)((unsigned int)tile >> 5) * STBPE_PPITCH + STBPE_PROWS, 1u << (tile & 31));
         }
     }
-    // ---- rewrite (no neighbour counted above is a position that changes)
-#pragma unroll 1
-    for (uint32_t o = heads; o; o &= o - 1u) {
-        const int p = __ffs(o) - 1;
-        const uint32_t k = MANY ? ((k0 >> p) & 1u) | (((k1 >> p) & 1u) << 1) | (((k2 >> p) & 1u) << 2) : 0u;
-        tok[K::sindex(p)] = (T)(P->nw[k] | ((F >> p) & 1u ? K::FLAG : 0u));
-    }
-#pragma unroll 1
-    for (uint32_t o = D; o; o &= o - 1u) tok[K::sindex(__ffs(o) - 1)] = (T)K::HOLE;
+    // ---- what changed goes back
     {
         uint4 *g = reinterpret_cast<uint4 *>(tile_ptr<T>(e, tile)) + lane * K::VEC;
 #pragma unroll
@@ -638,7 +645,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) merge_kernel(const _
     s.carve<T>(smem_raw, s_ctr);
     s.clear();
     MergeCtx c;
-    if (threadIdx.x == 0) s.p->n = 1, s.p->a[0] = (uint32_t)st->cur_a, s.p->b[0] = (uint32_t)st->cur_b, s.p->nw[0] = (uint32_t)st->cur_new;
+    if (threadIdx.x == 0) s.p->n = 1, s.p->set<T>(0, (uint32_t)st->cur_a, (uint32_t)st->cur_b, (uint32_t)st->cur_new);
     c.m = st->merges_done;
     c.fv = st->filter_valid != 0;
     c.zero = false;  // done when the merge was selected

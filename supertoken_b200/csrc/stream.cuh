@@ -86,31 +86,59 @@ __device__ __forceinline__ void load_group(const EngineDev &e, int tile, int lan
 // One group in registers: L = live tokens, F = tokens that start a row (or holes), eq(id) = tokens with that id.
 template <typename T>
 struct Group;
+// 16-bit stream: the group as 16 bit planes (bit p of plane i = bit i of token p).  The 16 words are two 16 x 16 bit
+// matrices side by side; four butterfly steps transpose both at once in 112 instructions, after which the live mask is
+// an AND of planes, the row starts are a plane and eq() is one logic operation per plane (15 instead of the 64
+// instructions of a compare and a shift per word; a batch of four pairs takes eight of them per group).
+struct PlaneId {  // an id as masks: word i = all ones where bit i of the id is set
+    uint4 m[4];
+    __device__ __forceinline__ void set(uint32_t id) {
+        uint32_t v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = (id >> i) & 1u ? 0xFFFFFFFFu : 0u;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) m[j] = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    }
+};
 template <>
 struct Group<uint16_t> {
     uint32_t w[16];
+    template <int S>
+    __device__ __forceinline__ void exchange(uint32_t mask) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            if (i & S) continue;
+            const uint32_t x = w[i], y = w[i + S];
+            if (S == 8) {
+                w[i] = __byte_perm(x, y, 0x6240), w[i + S] = __byte_perm(x, y, 0x7351);
+            } else {
+                w[i] = (x & mask) | ((y << S) & ~mask);
+                w[i + S] = ((x >> S) & mask) | (y & ~mask);
+            }
+        }
+    }
     __device__ __forceinline__ void load(const uint32_t *group, uint32_t &L, uint32_t &F) {
-        uint32_t nl = 0, f = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const uint4 q = *reinterpret_cast<const uint4 *>(group + 4 * j);
             w[4 * j] = q.x, w[4 * j + 1] = q.y, w[4 * j + 2] = q.z, w[4 * j + 3] = q.w;
         }
+        exchange<8>(0u);
+        exchange<4>(0x0F0F0F0Fu);
+        exchange<2>(0x33333333u);
+        exchange<1>(0x55555555u);
+        uint32_t hole = w[0] & w[1] & w[2];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            f = (f >> 1) | (w[i] & 0x80008000u);
-            w[i] &= 0x7FFF7FFFu;
-            nl = (nl >> 1) | ((w[i] + 0x00010001u) & 0x80008000u);  // only a hole has 0x7FFF in its low bits
-        }
-        L = ~nl, F = f;
+        for (int i = 3; i < 15; i += 2) hole &= w[i] & w[i + 1];  // only a hole has all 15 low bits set
+        L = ~hole, F = w[15];
     }
-    __device__ __forceinline__ uint32_t eq(uint32_t id) const {
-        const uint32_t two = id | (id << 16);
-        uint32_t n = 0;
-        // per half: x + 0x7FFF carries into the top bit iff x (15 bits) is not zero
+    __device__ __forceinline__ uint32_t eq(const PlaneId &id) const {
+        const uint4 m0 = id.m[0], m1 = id.m[1], m2 = id.m[2], m3 = id.m[3];
+        const uint32_t m[15] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w, m2.x, m2.y, m2.z, m2.w, m3.x, m3.y, m3.z};
+        uint32_t r = ~(w[0] ^ m[0]);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) n = (n >> 1) | (((w[i] ^ two) + 0x7FFF7FFFu) & 0x80008000u);
-        return ~n;
+        for (int i = 1; i < 15; ++i) r &= ~(w[i] ^ m[i]);
+        return r;
     }
 };
 template <>
@@ -130,7 +158,8 @@ struct Group<uint32_t> {
             w[i] &= STBPE_IDMASK;
         }
     }
-    __device__ __forceinline__ uint32_t eq(uint32_t id) const {
+    __device__ __forceinline__ uint32_t eq(const PlaneId &p) const {
+        const uint32_t id = p.m[0].x;
         uint32_t m = 0;
 #pragma unroll
         for (int i = 0; i < 32; ++i)
