@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ int s_ctr[CTR_N];
     constexpr int KB = Batch<T>::MAX, TOP = KB > 1 ? 4 : 1;  // best candidates that each warp hands over
+    __shared__ Bt s_sorted[32];           // all warps' best, the first KB in order
     __shared__ Bt s_top[32 * TOP], s_rest[32];  // the warps' best candidates in order; the best of what is left
     __shared__ i64 s_live, s_keys;        // live tokens, keys in the table
     __shared__ i64 s_forced[KB];          // counts of the next host-given pairs
@@ -175,13 +176,16 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
                     x = Bs::max2(x, v);
                 }
             };
+            // (the place of this thread's first appended candidate is read together with their number)
+            unsigned int i_new = n_cand + tid, new_at = i_new < STBPE_CAND_CAP ? __ldcg(e.cand + i_new) : 0u;
 #pragma unroll 4
             for (unsigned int i = tid; i < n_cand; i += THREADS) take(s_cand[i]);
 #pragma unroll 1
-            for (unsigned int i = n_cand + tid; i < n_have; i += THREADS) {  // appended by the last merges
-                const unsigned int at = __ldcg(e.cand + i);
-                s_cand[i] = at;
-                take(at);
+            while (i_new < n_have) {  // appended by the last merges
+                s_cand[i_new] = new_at;
+                take(new_at);
+                i_new += THREADS;
+                if (i_new < n_have) new_at = __ldcg(e.cand + i_new);
             }
             n_cand = n_have;
 #pragma unroll
@@ -195,6 +199,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             if constexpr (KB > 1) {
                 const Bt v = Bs::warp_max(max(x, rest));
                 if (lane == 0) s_rest[warp] = v;
+                if (tid < 32) s_sorted[tid] = Bs::none();
             }
             if (la.forced && warp == 0 && lane < KB && forced_i + lane < la.n_forced) {
                 const int2 f = la.forced[forced_i + lane];
@@ -213,87 +218,98 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
         }
         __syncthreads();
         if (tid == THREADS - 1) red_release_u32(&sync->chosen, 1u);  // the CTA has read everything it decides by
-        // warp 0 decides; lane j takes the j-th best pair (or the j-th one the host gives) and tests whether it can be
-        // merge j of the batch, given that all before it are
+        if constexpr (KB > 1) {
+            // place of this warp's candidates among those of all warps
+            constexpr int PER = (WARPS * TOP + 31) / 32;
+            Bt v[PER];
+#pragma unroll
+            for (int r = 0; r < PER; ++r) v[r] = lane + 32 * r < WARPS * TOP ? s_top[lane + 32 * r] : Bs::none();
+#pragma unroll 1
+            for (int r = 0; r < TOP; ++r) {
+                const Bt x = s_top[warp * TOP + r];
+                int place = 0;
+#pragma unroll
+                for (int q = 0; q < PER; ++q) place += __popc(__ballot_sync(0xFFFFFFFFu, v[q] > x));
+                if (place >= KB) break;
+                if (lane == 0 && x) s_sorted[place] = x;
+            }
+            __syncthreads();
+        }
+        // warp 0 decides; the lanes of pair j take the j-th best pair (or the j-th one the host gives) and test whether it
+        // can be merge j of the batch, given that all before it are
         if (warp == 0) {
             const Bt bound = KB > 1 ? Bs::warp_max(lane < WARPS ? s_rest[lane] : Bs::none()) : Bs::none();
-            Bt c[TOP], mine = Bs::none();
-#pragma unroll
-            for (int r = 0; r < TOP; ++r) c[r] = lane < WARPS ? s_top[lane * TOP + r] : Bs::none();
+            const Bt mine = KB > 1 ? s_sorted[lane >> 1] : Bs::warp_max(lane < WARPS ? s_top[lane] : Bs::none());
             const bool host = la.forced != nullptr;
-#pragma unroll 1
-            for (int j = 0; j < KB; ++j) {
-                const Bt v = Bs::warp_max(c[0]);
-                if (lane == j) mine = v;
-                if constexpr (KB > 1) {
-                    if (c[0] == v) {
-#pragma unroll
-                        for (int r = 0; r + 1 < TOP; ++r) c[r] = c[r + 1];
-                        c[TOP - 1] = Bs::none();
-                    }
-                }
-            }
+            const int j = KB > 1 ? lane >> 1 : 0;  // two lanes per pair: one for each of its tokens
             const unsigned int err = s_err;
             const Slot best = Bs::slot(mine);
             const bool dry = (err >> 31) != 0u || !(mc.theta.admits(best.count, best.key) || (best.count <= 0 && mc.theta.count == 0));
-            const bool forced = host && lane < KB && forced_i + lane < la.n_forced;
+            const bool forced = host && j < KB && forced_i + j < la.n_forced;
             u64 key = best.key;
             i64 count = best.count;
             if (forced) {
-                const int2 f = la.forced[forced_i + lane];
+                const int2 f = la.forced[forced_i + j];
                 key = ((u64)(uint32_t)f.x << 32) | (uint32_t)f.y;
-                count = s_forced[lane];
+                count = s_forced[j];
             }
             const uint32_t a = (uint32_t)(key >> 32), b = (uint32_t)key;
-            const uint32_t nw0 = (uint32_t)(host ? la.forced_new + forced_i : base_vocab + merges_done), nw = nw0 + lane;
-            // every merge makes at most two pairs per match and two per id, and drops one token per occurrence of its pair (of
-            // a run, all but one)
-            const i64 grow = 2 * min(count, (i64)max((int)nw, la.ids_below)) + 2;
-            i64 live = s_live, keys = s_keys + grow;
+            const uint32_t nw0 = (uint32_t)(host ? la.forced_new + forced_i : base_vocab + merges_done), nw = nw0 + j;
+            // a merge drops one token per occurrence of its pair (of a run, all but one), so this many are gone before it
+            i64 before = 0;
+            if constexpr (KB > 1) {
+#pragma unroll
+                for (int d = 2; d < 2 * KB; d <<= 1) {
+                    const i64 o = __shfl_up_sync(0xFFFFFFFFu, before + count, d);
+                    if (lane >= d) before += o;
+                }
+            }
+            const i64 live = s_live - before;
+            // every merge makes at most two pairs per match and two per id
+            const i64 ids = max((int)nw, la.ids_below), made = min(before + count, ids * (j + 1));
             // a later member: the order is exact so far, it shares no token with the members before and names none of their
             // new ones (a pair that the host gives may)
-            bool out = lane >= (fv ? KB : min(la.dense_batch, KB));
-            if constexpr (KB > 1) out = out || (!host && !(mine > bound));
-            out = out || max(a, b) >= nw0;
-#pragma unroll
-            for (int j = 0; j + 1 < KB; ++j) {
-                const uint32_t ja = __shfl_sync(0xFFFFFFFFu, a, j), jb = __shfl_sync(0xFFFFFFFFu, b, j);
-                const i64 jc = __shfl_sync(0xFFFFFFFFu, count, j), jg = __shfl_sync(0xFFFFFFFFu, grow, j);
-                if (lane > j) {
-                    out = out || ja == a || ja == b || jb == a || jb == b;
-                    live -= jc, keys += jg;
-                }
+            bool out = j >= (fv ? KB : min(la.dense_batch, KB));
+            if constexpr (KB > 1) {
+                const uint32_t same = __match_any_sync(0xFFFFFFFFu, lane >= 2 * KB ? 0x80000000u | lane : lane & 1 ? b : a);
+                out = out || (!host && !(mine > bound)) || max(a, b) >= nw0 || (same & ((1u << (lane & ~1)) - 1u));
             }
             // stop rules of the loop: bpe_trainer.py:4304-4308 (no pairs), :2491-2494 / :4361-4364 (count < 2)
             int stop = 0, why = STBPE_EXIT_STOP;
             bool go = false;
             if (err & 0x7FFFFFFFu) stop = 4;
             else if (host && !forced) stop = 0;
-            else if (!host && merges_done + lane >= la.target) stop = 1;
+            else if (!host && merges_done + j >= la.target) stop = 1;
             // maintenance the host does between launches
             else if (!host && dry) why = STBPE_EXIT_REFILL;
             else if (!host && count <= 0) stop = 2;
             else if (!host && count < 2) stop = 3;
-            else if (e.n_tiles >= la.repack_tiles && live * 4 <= (i64)e.n_tiles * STBPE_TILE * 3) why = STBPE_EXIT_REPACK;
+            else if (e.n_tiles >= la.repack_tiles && s_live * 4 <= (i64)e.n_tiles * STBPE_TILE * 3) why = STBPE_EXIT_REPACK;
             else if (!fv && e.n_tiles > 0 && count <= la.filter_count) why = STBPE_EXIT_FILTER;
-            else if (keys > la.grow_keys) why = STBPE_EXIT_GROW;
+            else if (s_keys + 2 * made + 2 * (j + 1) > la.grow_keys) why = STBPE_EXIT_GROW;
             else if (sizeof(T) == 2 && max(nw, max(a, b)) >= Tok<uint16_t>::IDMASK) why = STBPE_EXIT_WIDEN;
             else go = true;
-            const uint32_t bad = __ballot_sync(0xFFFFFFFFu, lane >= KB || !go || (lane > 0 && out));
-            const int nb = __ffs(bad) - 1;
-            if (lane < nb) {
-                s.p->template set<T>(lane, a, b, nw);
-                s.p->count[lane] = count;
+            const uint32_t bad = __ballot_sync(0xFFFFFFFFu, j >= KB || !go || (j > 0 && out)) | (KB > 1 ? 1u << (2 * KB) : 2u);
+            const int nb = lsb(bad) >> (KB > 1 ? 1 : 0);
+            if (KB > 1 ? j < nb && !(lane & 1) : lane < nb) {
+                s.p->a[j] = a, s.p->b[j] = b, s.p->nw[j] = nw;
+                s.p->count[j] = count;
                 if (cta == 0) {
-                    const int m = merges_done + lane;
+                    const int m = merges_done + j;
                     *reinterpret_cast<int2 *>(e.merges + 2 * m) = make_int2((int)a, (int)b);
                     e.merge_counts[m] = count;
                     e.live_before[m] = live;
-                    if (lane == nb - 1) {
+                    if (j == nb - 1) {
                         st->cur_a = (int)a, st->cur_b = (int)b, st->cur_new = (int)nw;
                         st->cur_count = count;
                     }
                 }
+            }
+            // the pairs' ids as masks, a word per lane
+#pragma unroll 1
+            for (int k = 0; k < nb; ++k) {
+                const uint32_t ka = __shfl_sync(0xFFFFFFFFu, a, KB > 1 ? 2 * k : 0), kb = __shfl_sync(0xFFFFFFFFu, b, KB > 1 ? 2 * k : 0);
+                s.p->set_planes<T>(k, ka, kb, lane);
             }
             if (lane == 0) {
                 s.p->n = nb;

@@ -63,15 +63,12 @@ struct BatchPairs {  // in shared memory
     i64 count[8];
     int touch[64];  // matches of pair i (row) followed at once by one of pair k (column)
     int n;
+    // called by the 32 lanes of a warp: word i of the masks is all ones where bit i of the id is set
     template <typename T>
-    __device__ __forceinline__ void set(int k, uint32_t x, uint32_t y, uint32_t new_id) {
-        a[k] = x, b[k] = y, nw[k] = new_id;
-        if (sizeof(T) == 2) {
-            pa[k].set(x);
-            pb[k].set(y);
-        } else {
-            pa[k].m[0].x = x, pb[k].m[0].x = y;
-        }
+    __device__ __forceinline__ void set_planes(int k, uint32_t x, uint32_t y, int lane) {
+        const uint32_t id = lane < 16 ? x : y;
+        uint32_t *w = reinterpret_cast<uint32_t *>(lane < 16 ? pa[k].m : pb[k].m) + (lane & 15);
+        *w = sizeof(T) == 4 ? id : 0u - ((id >> (lane & 15)) & 1u);
     }
 };
 
@@ -84,7 +81,7 @@ struct MergeGeom {
     static constexpr size_t BYTES = (size_t)WARPS * WARP_WORDS * 4 + (size_t)STBPE_AGG * 10 + STBPE_LIST * 5 + STBPE_LIST_UNITS * Batch<T>::MAX * 4 + sizeof(BatchPairs);
 };
 
-enum { CTR_LIST, CTR_AGG, CTR_REMOVED, CTR_MATCHES, CTR_SEAM, CTR_FRESH, CTR_TILES, CTR_UNITS, CTR_RECS, CTR_N };
+enum { CTR_LIST, CTR_AGG, CTR_REMOVED, CTR_SEAM, CTR_FRESH, CTR_TILES, CTR_UNITS, CTR_RECS, CTR_N };
 
 struct CtaMerge {
     uint32_t *warp_mem;    // WARPS x WARP_WORDS
@@ -233,7 +230,7 @@ __device__ __forceinline__ int pair_starting(const BatchPairs *p, uint32_t id) {
 }
 
 struct WarpStats {  // per lane
-    int removed, matches, seam, units, recs;
+    int removed, seam, units, recs;
     int tiles;  // per warp
 };
 
@@ -244,12 +241,16 @@ __device__ __forceinline__ uint4 load_recs3(const EngineDev &e, int tile, int la
     if (lane < 12 && t >= 0 && t < e.n_tiles) r = __ldcg(reinterpret_cast<const uint4 *>(e.recs + 2 * (i64)t) + (lane & 3));
     return r;
 }
-// lane that holds the first half of the record of tile - 1 + k that is current before merge m
-__device__ __forceinline__ int pick_rec(const uint4 &rv, int k, int m) {
-    const int v0 = (int)__shfl_sync(0xFFFFFFFFu, rv.x, 4 * k), v1 = (int)__shfl_sync(0xFFFFFFFFu, rv.x, 4 * k + 2);
-    const bool ok0 = v0 >= 0 && v0 < m, ok1 = v1 >= 0 && v1 < m;
-    return 4 * k + ((ok1 && (!ok0 || v1 > v0)) ? 2 : 0);
+// Which version of each record is current before merge m: bit 4k + 2 of the result is set when it is the second one of
+// tile - 1 + k (its first half sits in lane 4k + 2, else in lane 4k).
+__device__ __forceinline__ uint32_t pick_recs(const uint4 &rv, int m) {
+    const int own = (int)rv.x, other = (int)__shfl_xor_sync(0xFFFFFFFFu, rv.x, 2);
+    const bool ok = own >= 0 && own < m, ok_other = other >= 0 && other < m;
+    return __ballot_sync(0xFFFFFFFFu, ok && (!ok_other || own > other));
 }
+// index of the lowest set bit.  (One find-leading-one; __ffs is a bit reversal on top of it, and both run at an eighth of
+// the rate of ordinary instructions.)
+__device__ __forceinline__ int lsb(uint32_t x) { return 31 - __clz(x & (0u - x)); }
 
 // One warp, one tile (already in the warp's shared-memory slot; every lane reads and writes its own group of
 // 32 tokens only).  `rv`: load_recs3 of the tile; `pm`: the pairs that may occur in it (bit k = pair k).
@@ -269,8 +270,10 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
     // the live tokens right before and right behind the tile: from the neighbours' records, or by walking
     // when they hold too few tokens
     Halo h;
-    const int lp = pick_rec(rv, 0, c.m), ln = pick_rec(rv, 2, c.m);
-    const bool near = (int)__shfl_sync(0xFFFFFFFFu, rv.y, lp) >= 2 && (int)__shfl_sync(0xFFFFFFFFu, rv.y, ln) >= 3;
+    const uint32_t second = pick_recs(rv, c.m);
+    const int lp = second & 4u ? 2 : 0, ln = second & 0x400u ? 10 : 8;
+    const uint32_t enough = __ballot_sync(0xFFFFFFFFu, (int)rv.y >= (lane < 4 ? 2 : 3));
+    const bool near = (enough >> lp) & (enough >> ln) & 1u;
     if (near) {
         h.prev = __shfl_sync(0xFFFFFFFFu, rv.y, lp + 1);
         h.nxt[0] = __shfl_sync(0xFFFFFFFFu, rv.z, ln);
@@ -285,46 +288,38 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
     const uint32_t low = L & (0u - L);                       // this lane's first live token ...
     const uint32_t top = L ? 0x80000000u >> __clz(L) : 0u;   // ... and its last
     const uint32_t above = ne & ~((2u << lane) - 1u), below = ne & ((1u << lane) - 1u);
-    const int up = __ffs(above) - 1, down = 31 - __clz(below);  // the next lanes that hold live tokens, if any
-    // match heads: positions of some a_k whose next live position holds b_k.  k0, k1, k2: bits of k at the heads.
-    uint32_t M = 0, k0 = 0, k1 = 0, k2 = 0;
+    const int up = lsb(above), down = 31 - __clz(below);  // the next lanes that hold live tokens, if any
+    // Dropped tokens: positions of some b_k whose previous live position holds a_k.  k0, k1, k2: bits of k wherever the
+    // token is one of pair k (no token is in two pairs).
+    uint32_t D = 0, k0 = 0, k1 = 0, k2 = 0;
     int kt = -1, kl = -1;  // the pair whose a is this lane's last token, the pair whose b is its first
 #pragma unroll 1
     for (uint32_t left = pm; left; left &= left - 1u) {
-        const int k = MANY ? __ffs(left) - 1 : 0;
-        const uint32_t A = grp.eq(P->pa[k]), B = grp.eq(P->pb[k]) & ~F;  // a partner does not start a row
-        const uint32_t hd = A & prev_live_bits(B, H);
-        M |= hd;
+        const int k = MANY ? lsb(left) : 0;
+        const uint32_t A = grp.eq(P->pa[k]), B = grp.eq(P->pb[k]);
+        const uint32_t Bc = B & ~F;  // a partner does not start a row
+        D |= next_live_bits(A, H) & Bc;
         if (A & top) kt = k;
-        if (B & low) kl = k;
+        if (Bc & low) kl = k;
         if (MANY) {
-            if (k & 1) k0 |= hd;
-            if (k & 2) k1 |= hd;
-            if (k & 4) k2 |= hd;
+            if (k & 1) k0 |= A | B;
+            if (k & 2) k1 |= A | B;
+            if (k & 4) k2 |= A | B;
         }
     }
+    // heads: the previous live position of every dropped one
+    uint32_t M = prev_live_bits(D, H);
     {
         const int kn = __shfl_sync(0xFFFFFFFFu, kl, above ? up : lane);
-        if (kt >= 0 && (above ? kn == kt : h.nxt[0] == P->b[kt])) {
-            M |= top;
-            if (MANY) {
-                if (kt & 1) k0 |= top;
-                if (kt & 2) k1 |= top;
-                if (kt & 4) k2 |= top;
-            }
-        }
+        if (kt >= 0 && (above ? kn == kt : h.nxt[0] == P->b[kt])) M |= top;
     }
-    // dropped positions: the next live position of every head
     const uint32_t hb = __ballot_sync(0xFFFFFFFFu, (M & top) != 0u);
     const bool carry_in = below == 0u && kl >= 0 && (h.prev & STBPE_IDMASK) == P->a[kl];
-    const uint32_t D_in = next_live_bits(M, H);
-    const bool low_gone = below ? ((hb >> down) & 1u) != 0u : carry_in;  // this lane's first token is dropped (L != 0 implied)
-    const uint32_t D = D_in | (low_gone ? low : 0u);
+    if (below ? ((hb >> down) & 1u) != 0u : carry_in) D |= low;
     const uint32_t touched = M | D;
     if (__ballot_sync(0xFFFFFFFFu, touched != 0u) == 0u) return;  // nothing to merge here
-    ws.matches += __popc(M);
     ws.removed += __popc(D);
-    const int first_lane = __ffs(ne) - 1, last_lane = 31 - __clz(ne);
+    const int first_lane = lsb(ne), last_lane = 31 - __clz(ne);
     const bool last_head = ((hb >> last_lane) & 1u) != 0u;  // its partner sits in another tile
     if (near) {
         h.prev2 = __shfl_sync(0xFFFFFFFFu, rv.z, lp + 1);
@@ -341,7 +336,7 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
         xid = __shfl_sync(0xFFFFFFFFu, tid, below ? down : lane);
         xdrop = below && ((tgone >> down) & 1u);
         // ... and to the right (id, does it start a row or head a match)
-        const uint32_t fid = L ? (uint32_t)tok[K::sindex(__ffs(L) - 1)] & K::IDMASK : 0u;
+        const uint32_t fid = L ? (uint32_t)tok[K::sindex(lsb(L))] & K::IDMASK : 0u;
         const uint32_t fskip = __ballot_sync(0xFFFFFFFFu, ((F | heads) & low) != 0u);
         yid = __shfl_sync(0xFFFFFFFFu, fid, above ? up : lane);
         yskip = above && ((fskip >> up) & 1u);
@@ -358,8 +353,9 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
         yskip = (yid & STBPE_FLAG) || (i < P->n && h.nxt[1] == P->b[i]);
     }
 #pragma unroll 1
-    for (uint32_t o = heads; o; o &= o - 1u) {
-        const int q = __ffs(o) - 1;
+    for (uint32_t o = heads; o;) {
+        const int q = 31 - __clz(o);
+        o ^= 1u << q;
         const uint32_t k = MANY ? ((k0 >> q) & 1u) | (((k1 >> q) & 1u) << 1) | (((k2 >> q) & 1u) << 2) : 0u;
         const uint32_t nw = P->nw[k], l = L & ((1u << q) - 1u);
         const bool starts = (F >> q) & 1u;
@@ -385,29 +381,21 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
     }
     // of a match whose head sits in the tile before, the head's tile takes care (of a run, the last token's tile)
     const uint32_t own = ends & ~(carry_in && P->a[kl] != P->b[kl] ? low : 0u);
-    uint32_t d0 = 0, d1 = 0, d2 = 0;
-    if (MANY) {
-        d0 = next_live_bits(k0, H), d1 = next_live_bits(k1, H), d2 = next_live_bits(k2, H);
-        if (low_gone) {  // then kl is its pair
-            if (kl & 1) d0 |= low;
-            if (kl & 2) d1 |= low;
-            if (kl & 4) d2 |= low;
-        }
-    }
 #pragma unroll 1
-    for (uint32_t o = D; o; o &= o - 1u) {
-        const int r = __ffs(o) - 1;
+    for (uint32_t o = D; o;) {
+        const int r = 31 - __clz(o);
+        o ^= 1u << r;
         tok[K::sindex(r)] = (T)K::HOLE;
         const uint32_t u = L & ~((2u << r) - 1u);
         uint32_t id = yid;
         bool skip = yskip;
         if (u) {
-            const int p = __ffs(u) - 1;
+            const int p = lsb(u);
             id = (uint32_t)tok[K::sindex(p)] & K::IDMASK;
             skip = ((F | heads) >> p) & 1u;
         }
         if (skip || !((own >> r) & 1u)) continue;
-        const uint32_t k = MANY ? ((d0 >> r) & 1u) | (((d1 >> r) & 1u) << 1) | (((d2 >> r) & 1u) << 2) : 0u;
+        const uint32_t k = MANY ? ((k0 >> r) & 1u) | (((k1 >> r) & 1u) << 1) | (((k2 >> r) & 1u) << 2) : 0u;
         agg_add<T, MG>(s, e, c, id, 1u, k);
         if (c.fv) filter_set(e, tile, u || above ? -1 : h.next_tile, made_key(P, k, id, 1u));
     }
@@ -449,9 +437,8 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
     const uint32_t t2 = L & ~top, top2 = top | (t2 ? 0x80000000u >> __clz(t2) : 0u);
     const bool edge_ok = (lane != first_lane || (l3 && !(touched & low3))) && (lane != last_lane || (t2 && !(touched & top2)));
     if (!__all_sync(0xFFFFFFFFu, edge_ok)) {
-        const int lo = pick_rec(rv, 1, c.m);
         // readers of this merge never pick a record stamped m, so payload and stamp need no ordering
-        uint32_t *r = reinterpret_cast<uint32_t *>(e.recs + 2 * (i64)tile + ((lo & 2) ? 0 : 1));
+        uint32_t *r = reinterpret_cast<uint32_t *>(e.recs + 2 * (i64)tile + ((second & 0x40u) ? 0 : 1));
         uint32_t *mL = wm + MergeGeom<T>::RAW_WORDS;
         mL[lane] = NL;
         const uint32_t ne2 = __ballot_sync(0xFFFFFFFFu, NL != 0u);
@@ -486,7 +473,7 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
     constexpr int WARPS = MergeGeom<T>::WARPS;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t *wm = s.warp_mem + (size_t)warp * MergeGeom<T>::WARP_WORDS;
-    WarpStats ws = {0, 0, 0, 0, 0, 0};
+    WarpStats ws = {0, 0, 0, 0, 0};
     const int nb = Batch<T>::MAX > 1 ? s.p->n : 1;
     // Without the filter: every tile, consecutive tiles on different CTAs so that a small stream uses all of
     // them.  With it: batches of filter units, each turned into a list of tiles that the warps share.
@@ -565,10 +552,10 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
         }
     }
     {
-        const int part[6] = {ws.removed, ws.matches, ws.seam, lane == 0 ? ws.tiles : 0, ws.units, ws.recs};
-        constexpr int slot[6] = {CTR_REMOVED, CTR_MATCHES, CTR_SEAM, CTR_TILES, CTR_UNITS, CTR_RECS};
+        const int part[5] = {ws.removed, ws.seam, lane == 0 ? ws.tiles : 0, ws.units, ws.recs};
+        constexpr int slot[5] = {CTR_REMOVED, CTR_SEAM, CTR_TILES, CTR_UNITS, CTR_RECS};
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
+        for (int k = 0; k < 5; ++k) {
             const int x = __reduce_add_sync(0xFFFFFFFFu, part[k]);
             if (lane == 0 && x) reds_add_s32(&s.ctr[slot[k]], x);
         }
@@ -620,8 +607,10 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
         const int k = threadIdx.x, x = s.ctr[k];
         s.ctr[k] = 0;
         if (x) {  // results unused: reductions
-            if (k == CTR_REMOVED) atomicAdd((u64 *)&st->n_live, (u64)(-(i64)x));
-            if (k == CTR_MATCHES) atomicAdd((u64 *)&st->n_matches, (u64)x);
+            if (k == CTR_REMOVED) {  // one dropped token per match
+                atomicAdd((u64 *)&st->n_live, (u64)(-(i64)x));
+                atomicAdd((u64 *)&st->n_matches, (u64)x);
+            }
             if (k == CTR_SEAM) atomicAdd(&st->n_fixups, (unsigned int)x);
             if (k == CTR_FRESH && !MG) atomicAdd(&st->n_keys, (u64)x);
             if (k == CTR_TILES) {
@@ -645,7 +634,8 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) merge_kernel(const _
     s.carve<T>(smem_raw, s_ctr);
     s.clear();
     MergeCtx c;
-    if (threadIdx.x == 0) s.p->n = 1, s.p->set<T>(0, (uint32_t)st->cur_a, (uint32_t)st->cur_b, (uint32_t)st->cur_new);
+    if (threadIdx.x == 0) s.p->n = 1, s.p->a[0] = (uint32_t)st->cur_a, s.p->b[0] = (uint32_t)st->cur_b, s.p->nw[0] = (uint32_t)st->cur_new;
+    if (threadIdx.x < 32) s.p->set_planes<T>(0, (uint32_t)st->cur_a, (uint32_t)st->cur_b, (int)threadIdx.x);
     c.m = st->merges_done;
     c.fv = st->filter_valid != 0;
     c.zero = false;  // done when the merge was selected

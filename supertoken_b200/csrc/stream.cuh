@@ -90,15 +90,8 @@ struct Group;
 // matrices side by side; four butterfly steps transpose both at once in 112 instructions, after which the live mask is
 // an AND of planes, the row starts are a plane and eq() is one logic operation per plane (15 instead of the 64
 // instructions of a compare and a shift per word; a batch of four pairs takes eight of them per group).
-struct PlaneId {  // an id as masks: word i = all ones where bit i of the id is set
+struct PlaneId {  // an id as masks: word i = all ones where bit i of the id is set (32-bit stream: word 0 = the id)
     uint4 m[4];
-    __device__ __forceinline__ void set(uint32_t id) {
-        uint32_t v[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = (id >> i) & 1u ? 0xFFFFFFFFu : 0u;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) m[j] = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-    }
 };
 template <>
 struct Group<uint16_t> {
