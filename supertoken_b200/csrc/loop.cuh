@@ -57,6 +57,17 @@ __device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int *p) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+// Without ordering: for `chosen`, which says that loads have returned, not that stores are visible.  (A release here is a
+// memory barrier that held up the shuffles and shared-memory accesses of the whole SM for 2-3 us, just while
+// the batch is being decided.)
+__device__ __forceinline__ void red_relaxed_u32(unsigned int *p, unsigned int v) {
+    asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ unsigned int ld_relaxed_u32(const unsigned int *p) {
+    unsigned int v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 // retries of a bounded wait; false when the time is up or another wait has given up
 struct BoundedWait {
     u64 t0;
@@ -217,7 +228,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             }
         }
         __syncthreads();
-        if (tid == THREADS - 1) red_release_u32(&sync->chosen, 1u);  // the CTA has read everything it decides by
+        if (tid == THREADS - 1) red_relaxed_u32(&sync->chosen, 1u);  // the values of everything this CTA decides by have arrived
         if constexpr (KB > 1) {
             // place of this warp's candidates among those of all warps
             constexpr int PER = (WARPS * TOP + 31) / 32;
@@ -338,7 +349,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
         cta_merge<T, false>(e, s, mc, la.unit_shift, [&] {
             if (tid == THREADS - 1) {
                 BoundedWait wait;
-                while (ld_acquire_u32(&sync->chosen) < G * (step + 1))
+                while (ld_relaxed_u32(&sync->chosen) < G * (step + 1))
                     if (!wait.again(st)) {
                         s_ok = 0;
                         break;
