@@ -316,12 +316,6 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
                     }
                 }
             }
-            // the pairs' ids as masks, a word per lane
-#pragma unroll 1
-            for (int k = 0; k < nb; ++k) {
-                const uint32_t ka = __shfl_sync(0xFFFFFFFFu, a, KB > 1 ? 2 * k : 0), kb = __shfl_sync(0xFFFFFFFFu, b, KB > 1 ? 2 * k : 0);
-                s.p->set_planes<T>(k, ka, kb, lane);
-            }
             if (lane == 0) {
                 s.p->n = nb;
                 s_go = nb;
@@ -340,6 +334,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
         }
         __syncthreads();
         const int nb = s_go;
+        if (tid < 32 * nb) s.p->set_plane<T>(tid >> 5, lane);  // (barriers of cta_merge come before they are read)
         if (nb == 0 || !s_ok) return;
         // ---- the merges
         merges_done += nb;

@@ -65,10 +65,10 @@ struct BatchPairs {  // in shared memory
     int n;
     // called by the 32 lanes of a warp: word i of the masks is all ones where bit i of the id is set
     template <typename T>
-    __device__ __forceinline__ void set_planes(int k, uint32_t x, uint32_t y, int lane) {
-        const uint32_t id = lane < 16 ? x : y;
-        uint32_t *w = reinterpret_cast<uint32_t *>(lane < 16 ? pa[k].m : pb[k].m) + (lane & 15);
-        *w = sizeof(T) == 4 ? id : 0u - ((id >> (lane & 15)) & 1u);
+    __device__ __forceinline__ void set_plane(int k, int lane) {
+        const uint32_t id = lane < 16 ? a[k] : b[k];
+        reinterpret_cast<uint32_t *>(pa)[(lane & 16 ? (int)sizeof(pa) / 4 : 0) + k * 16 + (lane & 15)] =
+            sizeof(T) == 4 ? id : 0u - ((id >> (lane & 15)) & 1u);
     }
 };
 
@@ -475,6 +475,7 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
     uint32_t *wm = s.warp_mem + (size_t)warp * MergeGeom<T>::WARP_WORDS;
     WarpStats ws = {0, 0, 0, 0, 0};
     const int nb = Batch<T>::MAX > 1 ? s.p->n : 1;
+    if (!c.fv) __syncthreads();  // the pairs are in place (with the filter, the barriers of the list come first)
     // Without the filter: every tile, consecutive tiles on different CTAs so that a small stream uses all of
     // them.  With it: batches of filter units, each turned into a list of tiles that the warps share.
     const i64 n_units = c.fv ? ((i64)e.n_tiles + (1 << unit_shift) - 1) >> unit_shift : blockIdx.x + 1;
@@ -635,12 +636,12 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) merge_kernel(const _
     s.clear();
     MergeCtx c;
     if (threadIdx.x == 0) s.p->n = 1, s.p->a[0] = (uint32_t)st->cur_a, s.p->b[0] = (uint32_t)st->cur_b, s.p->nw[0] = (uint32_t)st->cur_new;
-    if (threadIdx.x < 32) s.p->set_planes<T>(0, (uint32_t)st->cur_a, (uint32_t)st->cur_b, (int)threadIdx.x);
     c.m = st->merges_done;
     c.fv = st->filter_valid != 0;
     c.zero = false;  // done when the merge was selected
     c.theta.count = st->theta_count, c.theta.key = st->theta_key;
     if (!c.fv && blockIdx.x == 0 && threadIdx.x == 0) st->n_work = -1;
     __syncthreads();
+    if (threadIdx.x < 32) s.p->set_plane<T>(0, (int)threadIdx.x);
     cta_merge<T, MG>(e, s, c, unit_shift, [] {});
 }
