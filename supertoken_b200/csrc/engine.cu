@@ -206,10 +206,12 @@ static bool starts_wide(const stbpe_config &c) {
 }
 static size_t tok_bytes(const stbpe_engine *e) { return e->wide ? 4 : 2; }
 
-// log2 of the tiles a CTA takes together from the pair filter: words of the filter once every CTA gets two of
-// them, fewer tiles on smaller streams, so that the visited tiles spread over all CTAs
+// log2 of the tiles a CTA takes together from the pair filter: eight once every CTA gets several units, fewer on
+// smaller streams, so that the visited tiles spread over all CTAs.  (Whole words of the filter, 32 tiles, are fewer
+// loads, but where the tiles that hold a pair lie together one CTA gets many of them: on the adversarial corpus the
+// others waited 20-30 us of a step of 80.)
 static int unit_shift(const stbpe_engine *e, int grid) {
-    int sh = 5;
+    int sh = 3;
     while (sh > 0 && (((i64)e->d.n_tiles + (1 << sh) - 1) >> sh) < 2 * (i64)grid) --sh;
     return sh;
 }

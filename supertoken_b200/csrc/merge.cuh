@@ -29,7 +29,8 @@
 #define STBPE_AGG_BITS 12
 #define STBPE_AGG (1 << STBPE_AGG_BITS)   // entries of a CTA's neighbour histogram
 #define STBPE_LIST 2048                   // tiles a CTA collects from the pair filter at a time
-#define STBPE_LIST_UNITS 64               // filter units (of at most 32 tiles) per batch
+#define STBPE_LIST_UNITS 256              // filter units (of at most 8 tiles) per batch
+static_assert(STBPE_LIST_UNITS * 8 <= STBPE_LIST, "a batch of units fits the list");
 
 // Pairs of a batch.  Late in a run on text four of the next best pairs on average share no token (8 in a batch;
 // 16 would give 5 % more, 4 would give 3.3), and what a late merge costs is latency.  The wide stream, whose ids leave
@@ -78,10 +79,10 @@ struct MergeGeom {
     static constexpr int THREADS = WARPS * 32;
     static constexpr int RAW_WORDS = 32 * Tok<T>::PITCH;
     static constexpr int WARP_WORDS = RAW_WORDS + 32;  // tile, live masks of the rewritten tile
-    static constexpr size_t BYTES = (size_t)WARPS * WARP_WORDS * 4 + (size_t)STBPE_AGG * 10 + STBPE_LIST * 5 + STBPE_LIST_UNITS * Batch<T>::MAX * 4 + sizeof(BatchPairs);
+    static constexpr size_t BYTES = (size_t)WARPS * WARP_WORDS * 4 + (size_t)STBPE_AGG * 10 + STBPE_LIST * 5 + STBPE_LIST_UNITS * Batch<T>::MAX + sizeof(BatchPairs);
 };
 
-enum { CTR_LIST, CTR_AGG, CTR_REMOVED, CTR_SEAM, CTR_FRESH, CTR_TILES, CTR_UNITS, CTR_RECS, CTR_N };
+enum { CTR_LIST, CTR_NEXT, CTR_AGG, CTR_REMOVED, CTR_SEAM, CTR_FRESH, CTR_TILES, CTR_UNITS, CTR_RECS, CTR_N };
 
 struct CtaMerge {
     uint32_t *warp_mem;    // WARPS x WARP_WORDS
@@ -91,7 +92,7 @@ struct CtaMerge {
     uint16_t *agg_list;    // taken entries in order of arrival
     uint32_t *list;        // tiles to visit ...
     unsigned char *list_pairs;  // ... and the pairs that may occur there
-    uint32_t *unit_bits;   // [pair][unit] tiles of the filter units at hand
+    unsigned char *unit_bits;  // [pair][unit] tiles of the filter units at hand
     int *ctr;              // CTR_N counters
 
     template <typename T>
@@ -110,8 +111,8 @@ struct CtaMerge {
         base += STBPE_LIST * 4;
         list_pairs = base;
         base += STBPE_LIST;
-        unit_bits = reinterpret_cast<uint32_t *>(base);
-        base += STBPE_LIST_UNITS * Batch<T>::MAX * 4;
+        unit_bits = base;
+        base += STBPE_LIST_UNITS * Batch<T>::MAX;
         ctr = counters;
         return base;
     }
@@ -479,32 +480,34 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
     // Without the filter: every tile, consecutive tiles on different CTAs so that a small stream uses all of
     // them.  With it: batches of filter units, each turned into a list of tiles that the warps share.
     const i64 n_units = c.fv ? ((i64)e.n_tiles + (1 << unit_shift) - 1) >> unit_shift : blockIdx.x + 1;
-    const uint32_t unit_bits = unit_shift == 5 ? 0xFFFFFFFFu : (1u << (1 << unit_shift)) - 1u;
+    const uint32_t unit_bits = (1u << (1 << unit_shift)) - 1u;
 #pragma unroll 1
     for (i64 u0 = blockIdx.x; u0 < n_units; u0 += (i64)STBPE_LIST_UNITS * gridDim.x) {
         int n = (e.n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;  // tiles blockIdx.x, + gridDim.x, ...
         if (c.fv) {
             // one thread per pair and unit asks the filter ...
-            const int k = threadIdx.x / STBPE_LIST_UNITS, at = threadIdx.x % STBPE_LIST_UNITS;
-            if (k < nb) {
-                const i64 u = u0 + (i64)at * gridDim.x;
+            int lg = 2;
+            while (lg < 8 && u0 + ((i64)gridDim.x << lg) < n_units) ++lg;
+#pragma unroll 2
+            for (int it = threadIdx.x; it < nb << lg; it += WARPS * 32) {
+                const int k = it >> lg;
+                const i64 u = u0 + (i64)(it & ((1 << lg) - 1)) * gridDim.x, t0 = u << unit_shift;
                 uint32_t bits = 0;
                 if (u < n_units) {
-                    const i64 t0 = u << unit_shift, w = t0 >> 5;
-                    const unsigned int *g = e.presence + (size_t)w * STBPE_PPITCH;
+                    const unsigned int *g = e.presence + (size_t)(t0 >> 5) * STBPE_PPITCH;
                     unsigned int r1, r2, r3;
                     filter_rows(((u64)s.p->a[k] << 32) | (u64)s.p->b[k], r1, r2, r3);
                     bits = (__ldcg(g + r1) & __ldcg(g + r2) & __ldcg(g + r3)) | __ldcg(g + STBPE_PROWS);
-                    bits &= unit_bits << (t0 & 31);
-                    if (e.n_tiles - w * 32 < 32) bits &= (1u << (e.n_tiles - w * 32)) - 1u;
+                    bits = (bits >> (t0 & 31)) & unit_bits;
+                    if (e.n_tiles - t0 < 8) bits &= (1u << (e.n_tiles - t0)) - 1u;
                 }
-                s.unit_bits[threadIdx.x] = bits;
+                s.unit_bits[it] = (unsigned char)bits;
             }
             __syncthreads();
-            // ... and a warp per unit lists the tiles that any pair needs, lane = tile of the filter word
+            // ... and a warp per four units lists the tiles that any pair needs: lane = tile lane % 8 of unit lane / 8
 #pragma unroll 1
-            for (int i = warp; i < STBPE_LIST_UNITS; i += WARPS) {
-                const uint32_t own = lane < nb ? s.unit_bits[lane * STBPE_LIST_UNITS + i] : 0u;
+            for (int i = warp; i < 1 << (lg - 2); i += WARPS) {
+                const uint32_t own = lane < nb ? reinterpret_cast<const uint32_t *>(s.unit_bits)[(lane << (lg - 2)) + i] : 0u;
                 const uint32_t any = __reduce_or_sync(0xFFFFFFFFu, own);
                 if (any == 0u) continue;
                 uint32_t pairs = 0;
@@ -514,20 +517,20 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
                 if (lane == 0) at0 = atoms_add_s32(&s.ctr[CTR_LIST], __popc(any));
                 at0 = __shfl_sync(0xFFFFFFFFu, at0, 0) + __popc(any & ((1u << lane) - 1u));
                 if (pairs) {
-                    const i64 w = ((u0 + (i64)i * gridDim.x) << unit_shift) >> 5;
-                    s.list[at0] = (uint32_t)(w * 32 + lane);
+                    s.list[at0] = (uint32_t)((u0 + (i64)(4 * i + (lane >> 3)) * gridDim.x) << unit_shift) + (lane & 7);
                     s.list_pairs[at0] = (unsigned char)pairs;
                 }
             }
             __syncthreads();
             n = s.ctr[CTR_LIST];
         }
-        // the loads of a tile are issued before the one before it is worked on
+        // the loads of a tile are issued before the one before it is worked on; of a list, a warp takes the
+        // next tile that is left (visiting every tile, the warps stay together: fixed shares save an atomic per tile)
         uint4 v[Tok<T>::VEC], rv;
         int cur = -1;
         uint32_t pairs = (1u << nb) - 1u, next_pairs = pairs;
 #pragma unroll 1
-        for (int j = warp;; j += WARPS) {
+        for (int j = warp, taken = 0;; j = c.fv ? __shfl_sync(0xFFFFFFFFu, taken, 0) + WARPS : j + WARPS) {
             if (cur >= 0) store_units<T>(wm, lane, v);
             const uint4 rc = rv;
             const int next = j < n ? (c.fv ? (int)s.list[j] : (int)blockIdx.x + j * (int)gridDim.x) : -1;
@@ -535,6 +538,7 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
                 if (c.fv) next_pairs = s.list_pairs[j];
                 load_units<T>(e, next, lane, v);
                 rv = load_recs3(e, next, lane);
+                if (c.fv && lane == 0) taken = atoms_add_s32(&s.ctr[CTR_NEXT], 1);
             }
             __syncwarp();
             if (cur >= 0) {
@@ -548,7 +552,7 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
         }
         if (c.fv) {
             __syncthreads();
-            if (threadIdx.x == 0) s.ctr[CTR_LIST] = 0;
+            if (threadIdx.x == 0) s.ctr[CTR_LIST] = s.ctr[CTR_NEXT] = 0;
             if (u0 + (i64)STBPE_LIST_UNITS * gridDim.x < n_units) __syncthreads();
         }
     }
