@@ -14,14 +14,17 @@
 // A second counter keeps the CTAs apart the other way round: a CTA adds its deltas of merge m only when all have
 // read the counts that chose merge m; that wait runs under the rewriting of the tiles.
 //
-// A step takes several merges.  Let p1, p2, ... be the pairs in selection order (larger count, then smaller key).
-// While no two of p1 .. pj share a token, merging p1 .. pj-1 leaves the count of pj as it is, and makes or
-// raises only pairs with one of their new tokens.  Such a pair (x, new) occurs at most as often as (x, a) did, and
-// (x, a) came after pj; where the counts are equal the larger key, new > every token of pj, loses.  So pj is
-// then the best pair, exactly as if the counts had been taken after each merge, and p1 .. pj are applied at once.
-// The batch ends at the first pair that shares a token, at Batch<T>::MAX, and wherever a stop rule or
-// maintenance has to be decided first.  On text a batch is four merges on average late in a run: the grid barrier,
-// the choice and the flush of the deltas, some 9 of the 12 us of a sparse merge, are paid once for the four.
+// A step takes several merges.  Let p1, p2, ... = (a1, b1), (a2, b2), ... be the pairs in selection order (larger count,
+// then smaller key), and let no ai be a bj with i != j (of a pair of equal tokens no token may occur elsewhere).  Then
+// an occurrence of pj overlaps no match of the others, so merging them leaves its count as it is.  They make or raise
+// only pairs with one of their new tokens; such a pair (x, new i) occurs at most as often as (x, ai) did, and (x, ai),
+// which is none of p1 .. pj, came after pj; where the counts are equal the larger key, new > every token of pj,
+// loses (and the same for (new i, y) and (bi, y)).  So pj is the best pair after p1 .. pj-1, exactly as if the
+// counts had been taken after each merge, and p1 .. pj are applied at once.
+// The batch ends at the first pair that breaks the rule, at Batch<T>::MAX, and wherever a stop rule or
+// maintenance has to be decided first.  On text a batch is 4.7 merges on average (3.9 while no token was to be
+// shared at all): the grid barrier, the choice and the flush of the deltas, some 9 of the 12 us of a sparse merge,
+// are paid once for all of them.
 //
 // Nothing else is exchanged: the tiles a merge must visit come out of the pair filter inside each CTA.
 //
@@ -278,12 +281,16 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             const i64 live = s_live - before;
             // every merge makes at most two pairs per match and two per id
             const i64 ids = max((int)nw, la.ids_below), made = min(before + count, ids * (j + 1));
-            // a later member: the order is exact so far, it shares no token with the members before and names none of their
-            // new ones (a pair that the host gives may)
+            // a later member: the order is exact so far, no token is second in one pair and first in another, none is one of
+            // the members' new ones (a pair that the host gives may name one, or be given twice)
             bool out = j >= (fv ? KB : min(la.dense_batch, KB));
             if constexpr (KB > 1) {
                 const uint32_t same = __match_any_sync(0xFFFFFFFFu, lane >= 2 * KB ? 0x80000000u | lane : lane & 1 ? b : a);
-                out = out || (!host && !(mine > bound)) || max(a, b) >= nw0 || (same & ((1u << (lane & ~1)) - 1u));
+                out = out || (!host && !(mine > bound)) || max(a, b) >= nw0 || (same & ((1u << (lane & ~1)) - 1u) & (lane & 1 ? 0x5555u : 0xAAAAu));
+                if (host) {
+                    const uint32_t twice = __match_any_sync(0xFFFFFFFFu, lane >= 2 * KB ? 0x80000000u | lane : (a << 15) | b);
+                    out = out || (twice & ((1u << (lane & ~1)) - 1u));
+                }
             }
             // stop rules of the loop: bpe_trainer.py:4304-4308 (no pairs), :2491-2494 / :4361-4364 (count < 2)
             int stop = 0, why = STBPE_EXIT_STOP;

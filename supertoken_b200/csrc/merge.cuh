@@ -4,9 +4,9 @@
 // With M[i] = (id[i]==a && id[j]==b && token j does not start a row), j = the live token behind i,
 // evaluated on the pre-merge stream (gpu_tokenizer/utils.py:520-527), token j is dropped when M[i]
 // and token i becomes `new` (utils.py:529-531).  A run of k >= 2 equal tokens (a == b) collapses into ONE new
-// token.  The merges of a batch share no token, so no position belongs to two of them and applying them
-// together leaves the stream that applying them one after the other leaves (loop.cuh says when the next
-// best pairs may form a batch).
+// token.  In a batch no pair's second token is another's first, so no position belongs to two matches and
+// applying the merges together leaves the stream that applying them one after the other leaves (loop.cuh
+// says when the next best pairs may form a batch).
 //
 // The histogram of the result equals a full recount of the rewritten rows when these terms are added (the entries
 // of the merged pairs themselves are zeroed when the merges are selected).  For every match (run) of pair k,
@@ -216,17 +216,11 @@ __device__ __forceinline__ void agg_add(const CtaMerge &s, const EngineDev &e, c
         agg_probe<T, MG>(s.agg_key, s.ctr, e, s.p, c.theta.count, c.theta.key, key);
 }
 
-// the pair whose second (first) token this is; the caller knows that there is one, or n for none
-__device__ __forceinline__ int pair_ending(const BatchPairs *p, uint32_t id) {
+// the pair (x, y) of the batch, or n when there is none (a token that starts a row, or nothing, has more bits than an id)
+__device__ __forceinline__ int find_pair(const BatchPairs *p, uint32_t x, uint32_t y) {
     int k = 0;
 #pragma unroll 1
-    while (k < p->n && p->b[k] != id) ++k;
-    return k;
-}
-__device__ __forceinline__ int pair_starting(const BatchPairs *p, uint32_t id) {
-    int k = 0;
-#pragma unroll 1
-    while (k < p->n && p->a[k] != id) ++k;
+    while (k < p->n && (p->a[k] != x || p->b[k] != y)) ++k;
     return k;
 }
 
@@ -290,33 +284,53 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
     const uint32_t top = L ? 0x80000000u >> __clz(L) : 0u;   // ... and its last
     const uint32_t above = ne & ~((2u << lane) - 1u), below = ne & ((1u << lane) - 1u);
     const int up = lsb(above), down = 31 - __clz(below);  // the next lanes that hold live tokens, if any
-    // Dropped tokens: positions of some b_k whose previous live position holds a_k.  k0, k1, k2: bits of k wherever the
-    // token is one of pair k (no token is in two pairs).
+    // Dropped tokens: positions of some b_k whose previous live position holds a_k.  k0, k1, k2: bits of k there.
     uint32_t D = 0, k0 = 0, k1 = 0, k2 = 0;
-    int kt = -1, kl = -1;  // the pair whose a is this lane's last token, the pair whose b is its first
+    uint32_t firsts = 0, seconds = 0;  // pairs whose a is this lane's last token, whose b is its first
 #pragma unroll 1
     for (uint32_t left = pm; left; left &= left - 1u) {
         const int k = MANY ? lsb(left) : 0;
-        const uint32_t A = grp.eq(P->pa[k]), B = grp.eq(P->pb[k]);
-        const uint32_t Bc = B & ~F;  // a partner does not start a row
-        D |= next_live_bits(A, H) & Bc;
-        if (A & top) kt = k;
-        if (Bc & low) kl = k;
+        const uint32_t A = grp.eq(P->pa[k]), B = grp.eq(P->pb[k]) & ~F;  // a partner does not start a row
+        const uint32_t d = next_live_bits(A, H) & B;
+        D |= d;
+        if (A & top) firsts |= 1u << k;
+        if (B & low) seconds |= 1u << k;
         if (MANY) {
-            if (k & 1) k0 |= A | B;
-            if (k & 2) k1 |= A | B;
-            if (k & 4) k2 |= A | B;
+            if (k & 1) k0 |= d;
+            if (k & 2) k1 |= d;
+            if (k & 4) k2 |= d;
         }
     }
     // heads: the previous live position of every dropped one
     uint32_t M = prev_live_bits(D, H);
+    // matches across lanes and tiles: kt = pair of the one that this lane's last token heads, kl = of the one whose
+    // partner is its first, -1 for none
+    int kt = -1, kl = -1;
     {
-        const int kn = __shfl_sync(0xFFFFFFFFu, kl, above ? up : lane);
-        if (kt >= 0 && (above ? kn == kt : h.nxt[0] == P->b[kt])) M |= top;
+        uint32_t both = firsts & __shfl_sync(0xFFFFFFFFu, seconds, above ? up : lane);
+        if (!above) {
+            both = 0;
+            for (uint32_t o = firsts; o; o &= o - 1u)
+                if (h.nxt[0] == P->b[lsb(o)]) both = o & (0u - o);
+        }
+        if (both) kt = lsb(both), M |= top;
+        kl = __shfl_sync(0xFFFFFFFFu, kt, below ? down : lane);
+        if (!below) {
+            kl = -1;
+            for (uint32_t o = seconds; o; o &= o - 1u)
+                if ((h.prev & STBPE_IDMASK) == P->a[lsb(o)]) kl = lsb(o);
+        }
+        if (L != 0u && kl >= 0) {
+            D |= low;
+            if (MANY) {
+                if (kl & 1) k0 |= low;
+                if (kl & 2) k1 |= low;
+                if (kl & 4) k2 |= low;
+            }
+        }
     }
-    const uint32_t hb = __ballot_sync(0xFFFFFFFFu, (M & top) != 0u);
-    const bool carry_in = below == 0u && kl >= 0 && (h.prev & STBPE_IDMASK) == P->a[kl];
-    if (below ? ((hb >> down) & 1u) != 0u : carry_in) D |= low;
+    const bool carry_in = below == 0u && kl >= 0;
+    const uint32_t hb = __ballot_sync(0xFFFFFFFFu, kt >= 0);
     const uint32_t touched = M | D;
     if (__ballot_sync(0xFFFFFFFFu, touched != 0u) == 0u) return;  // nothing to merge here
     ws.removed += __popc(D);
@@ -328,14 +342,18 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
         h.nxt[2] = __shfl_sync(0xFFFFFFFFu, rv.x, ln + 1);
     }
     const uint32_t heads = M & ~D;  // (a position in both is inside a run of equal tokens)
-    // ---- the neighbours whose pairs change.  What lies beyond this lane's group, to the left (id, is it dropped) ...
+    // ---- the neighbours whose pairs change.  What lies beyond this lane's group, to the left (id, the pair
+    // it is dropped for or -1) ...
     uint32_t xid, yid;
-    bool xdrop, yskip;
+    int xk;
+    bool yskip;
+    auto pair_at = [&](int r) { return MANY ? (int)(((k0 >> r) & 1u) | (((k1 >> r) & 1u) << 1) | (((k2 >> r) & 1u) << 2)) : 0; };
     {
-        const uint32_t tid = L ? (uint32_t)tok[K::sindex(31 - __clz(L))] & K::IDMASK : 0u;
-        const uint32_t tgone = __ballot_sync(0xFFFFFFFFu, (D & top) != 0u);
+        const int tp = 31 - __clz(L);
+        const uint32_t tid = L ? (uint32_t)tok[K::sindex(tp)] & K::IDMASK : 0u;
+        const int tk = D & top ? pair_at(tp) : -1;
         xid = __shfl_sync(0xFFFFFFFFu, tid, below ? down : lane);
-        xdrop = below && ((tgone >> down) & 1u);
+        xk = __shfl_sync(0xFFFFFFFFu, tk, below ? down : lane);
         // ... and to the right (id, does it start a row or head a match)
         const uint32_t fid = L ? (uint32_t)tok[K::sindex(lsb(L))] & K::IDMASK : 0u;
         const uint32_t fskip = __ballot_sync(0xFFFFFFFFu, ((F | heads) & low) != 0u);
@@ -345,37 +363,36 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
     const uint32_t ends = D & ~M;  // last tokens of matches and runs
     if (!below && (heads & ~F & low)) {
         xid = h.prev & STBPE_IDMASK;
-        const int i = pair_ending(P, h.prev);
-        xdrop = i < P->n && (h.prev2 & STBPE_IDMASK) == P->a[i];
+        const int i = find_pair(P, h.prev2 & STBPE_IDMASK, h.prev);
+        xk = i < P->n ? i : -1;
     }
     if (!above && (ends & top)) {
         yid = h.nxt[0];
-        const int i = pair_starting(P, h.nxt[0]);
-        yskip = (yid & STBPE_FLAG) || (i < P->n && h.nxt[1] == P->b[i]);
+        yskip = (yid & STBPE_FLAG) || find_pair(P, yid, h.nxt[1]) < P->n;
     }
 #pragma unroll 1
     for (uint32_t o = heads; o;) {
         const int q = 31 - __clz(o);
         o ^= 1u << q;
-        const uint32_t k = MANY ? ((k0 >> q) & 1u) | (((k1 >> q) & 1u) << 1) | (((k2 >> q) & 1u) << 2) : 0u;
-        const uint32_t nw = P->nw[k], l = L & ((1u << q) - 1u);
+        const uint32_t next = L & ~((2u << q) - 1u), l = L & ((1u << q) - 1u);
+        const int k = !MANY ? 0 : next ? pair_at(lsb(next)) : kt;
+        const uint32_t nw = P->nw[k];
         const bool starts = (F >> q) & 1u;
         tok[K::sindex(q)] = (T)(nw | (starts ? K::FLAG : 0u));
         if (starts) continue;
         uint32_t id = xid;
-        bool drop = xdrop;
+        int i = xk;
         if (l) {
             const int p = 31 - __clz(l);
             id = (uint32_t)tok[K::sindex(p)] & K::IDMASK;
-            drop = (D >> p) & 1u;
+            i = (D >> p) & 1u ? pair_at(p) : -1;
         }
         u64 made;
-        if (drop) {
-            const int i = pair_ending(P, id);
+        if (i >= 0) {
             reds_add_s32(&s.p->touch[i * 8 + k], 1);
             made = ((u64)P->nw[i] << 32) | nw;
         } else {
-            agg_add<T, MG>(s, e, c, id, 0u, k);
+            agg_add<T, MG>(s, e, c, id, 0u, (uint32_t)k);
             made = ((u64)id << 32) | nw;
         }
         if (c.fv) filter_set(e, tile, l || below ? -1 : h.prev_tile, made);
@@ -396,15 +413,15 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
             skip = ((F | heads) >> p) & 1u;
         }
         if (skip || !((own >> r) & 1u)) continue;
-        const uint32_t k = MANY ? ((k0 >> r) & 1u) | (((k1 >> r) & 1u) << 1) | (((k2 >> r) & 1u) << 2) : 0u;
-        agg_add<T, MG>(s, e, c, id, 1u, k);
+        const int k = pair_at(r);
+        agg_add<T, MG>(s, e, c, id, 1u, (uint32_t)k);
         if (c.fv) filter_set(e, tile, u || above ? -1 : h.next_tile, made_key(P, k, id, 1u));
     }
     if (last_head && lane == last_lane) {
         if (P->a[kt] != P->b[kt]) {
             const uint32_t y = h.nxt[1];
-            const int i = pair_starting(P, y);
-            if (i < P->n && h.nxt[2] == P->b[i]) {
+            const int i = find_pair(P, y, h.nxt[2]);
+            if (i < P->n) {
                 // y's tile counts the two touching matches, but sees the dropped token only, not the new one here
                 if (c.fv) filter_set(e, tile, -1, ((u64)P->nw[kt] << 32) | P->nw[i]);
             } else if (!(y & STBPE_FLAG)) {
