@@ -113,10 +113,12 @@ int stbpe_apply_merge(stbpe_engine *e, int32_t a, int32_t b, int32_t new_id, int
 int stbpe_apply_merges(stbpe_engine *e, const int32_t *pairs, int32_t n, int32_t first_new_id, void *stream);
 
 /* One step of a loop that breaks ties on the host (gpu_tokenizer/bpe_trainer.py:915-923): applies (a, b) ->
- * new_id (nothing when new_id < 0), then returns the best count and the keys that hold it, ascending, into
- * keys (host, cap entries; not written when *n_ties exceeds cap).  count 0 = empty histogram. */
-int stbpe_next_tied(stbpe_engine *e, int32_t a, int32_t b, int32_t new_id, int64_t *count, uint64_t *keys,
-                    int64_t cap, int64_t *n_ties, void *stream);
+ * new_id (nothing when a < 0), goes on with at most `most` best pairs while each is alone with its count and that
+ * is at least 2 (ids new_id + 1, ..., or new_id, ... when nothing was given), then returns the number of merges
+ * applied, the best count and the keys that hold it, ascending, into keys (host, cap entries; not written when
+ * *n_ties exceeds cap).  It may return before `most` without a tie; count 0 = empty histogram. */
+int stbpe_next_tied(stbpe_engine *e, int32_t a, int32_t b, int32_t new_id, int32_t most, int32_t *n_done,
+                    int64_t *count, uint64_t *keys, int64_t cap, int64_t *n_ties, void *stream);
 
 /* The merge loop (gpu_tokenizer/bpe_trainer.py:4193-4517) run on the device without
  * a host round trip per merge: select -> stop rules -> apply, n_merges times or until a

@@ -540,30 +540,45 @@ class GPUBPETrainer(BaseTrainer):
         into the tied candidates in ascending key order (``bpe_trainer.py:915-923``,
         ``trainers/bpe_gpu.py:112-123``).  ``checkpoint`` is called every ``checkpoint_interval``
         merges (the checkpoint carries the generator's state, so a resumed run draws on)."""
-        since = 0
-        count, cands = eng.next_tied() if remaining > 0 else (0, [])
+        # Merges without a tie need no draw, so the engine runs through them; the log brings them back.
+        first, base = eng.state().merges_done, len(self.merges)
+
+        def collect():
+            got, counts, _ = eng.merges(first + len(self.merges) - base)
+            self.merges.extend(got)
+            self.merge_counts.extend(counts.tolist())
+
+        def room():  # merges until the end or the next checkpoint
+            return min(remaining, checkpoint_interval - since) if checkpoint is not None and checkpoint_interval else remaining
+
+        since, merge, reason = 0, None, L.STOP_TARGET
         while remaining > 0:
-            if not cands:
-                return L.STOP_NO_PAIRS
-            if count < 2:
-                return L.STOP_LOW_COUNT
-            key = cands[0]
-            if len(cands) > 1 and self._tie_rng is not None:
-                key = cands[self._tie_rng.randrange(len(cands))]
-            a, b = key >> 32, key & 0xFFFFFFFF
-            self.merges.append((a, b))
-            self.merge_counts.append(count)
-            remaining -= 1
-            if remaining > 0:
-                count, cands = eng.next_tied((a, b, self.vocab_size))
+            most = room() - (merge is not None)
+            if merge is not None and remaining == 1:
+                eng.apply_merge(*merge, self.vocab_size)
+                done, count, cands = 1, 0, []
             else:
-                eng.apply_merge(a, b, self.vocab_size)
-            self.vocab_size += 1
-            since += 1
+                done, count, cands = eng.next_tied(merge, self.vocab_size, most)
+            remaining -= done
+            since += done
+            self.vocab_size += done
             if checkpoint is not None and checkpoint_interval and since >= checkpoint_interval and remaining > 0:
+                collect()
                 checkpoint()
                 since = 0
-        return L.STOP_TARGET
+            if remaining > 0:
+                if not cands:
+                    reason = L.STOP_NO_PAIRS
+                    break
+                if count < 2:
+                    reason = L.STOP_LOW_COUNT
+                    break
+                key = cands[0]
+                if len(cands) > 1 and self._tie_rng is not None:
+                    key = cands[self._tie_rng.randrange(len(cands))]
+                merge = (key >> 32, key & 0xFFFFFFFF)
+        collect()
+        return reason
 
     # ------------------------------------------------------------------ state / artifacts
     def _merges_for_metadata(self) -> list:

@@ -82,6 +82,8 @@ struct stbpe_engine {
     bool broken;          // a CUDA call failed: work of this engine may still be pending
     stbpe::Block pinned;  // host side of small transfers: the device state, then small inputs
     int dense_batch;
+    bool sync_zeroed;     // the barrier counters of the next loop launch are zero: each launch clears the other pair
+    int sync_turn;
     bool foreign_ids;     // a merge of the caller's may have brought an id of 65 536 or more
     unsigned int max_id;  // largest id appended through stbpe_append_ids
     unsigned int load_err;  // error bits of the rows appended so far
@@ -401,7 +403,7 @@ STBPE_VISIBLE int stbpe_create(stbpe_engine **out, const stbpe_config *cfg) {
         cub::DeviceScan::ExclusiveSum(nullptr, e->rp_tmp_bytes, e->rp_lens, e->rp_offs, e->max_tiles + 1, 0);
         a.add((unsigned char **)&e->rp_tmp, e->rp_tmp_bytes ? e->rp_tmp_bytes : 16);
         a.add((unsigned char **)&e->d.st, STBPE_TIES_OFFSET + STBPE_TIES_CAP * sizeof(u64));  // state and tied keys: one copy
-        a.add(&e->d.sync, 1);
+        a.add(&e->d.sync, 2);
         a.add(&e->d.merges, (size_t)2 * (cfg->max_merges + 1));
         a.add(&e->d.merge_counts, (size_t)cfg->max_merges + 1);
         a.add(&e->d.live_before, (size_t)cfg->max_merges + 1);
@@ -1035,7 +1037,8 @@ STBPE_VISIBLE int stbpe_select_best(stbpe_engine *e, uint64_t *key, int64_t *cou
 }
 
 static int filter_policy(stbpe_engine *e, const DevState &h, bool layout_changed, cudaStream_t s);
-static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t first_new, int64_t *n_matches, cudaStream_t s, bool then_ties = false);
+static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t first_new, int64_t *n_matches, cudaStream_t s, bool then_ties = false,
+                      int most = 0, int *n_done = nullptr);
 
 static int launch_merge(stbpe_engine *e, bool mg, cudaStream_t s) {
     if (e->d.n_tiles < 1) return STBPE_OK;
@@ -1076,23 +1079,26 @@ STBPE_VISIBLE int stbpe_apply_merges(stbpe_engine *e, const int32_t *pairs, int3
     return run_forced(e, pairs, n, first_new_id, nullptr, (cudaStream_t)stream);
 }
 
-STBPE_VISIBLE int stbpe_next_tied(stbpe_engine *e, int32_t a, int32_t b, int32_t new_id, int64_t *count, uint64_t *keys, int64_t cap,
-                                  int64_t *n_ties, void *stream) {
-    if (!e || !count || !n_ties || cap < 0 || (cap > 0 && !keys)) return STBPE_E_BADARG;
+STBPE_VISIBLE int stbpe_next_tied(stbpe_engine *e, int32_t a, int32_t b, int32_t new_id, int32_t most, int32_t *n_done, int64_t *count,
+                                  uint64_t *keys, int64_t cap, int64_t *n_ties, void *stream) {
+    if (!e || !count || !n_ties || !n_done || most < 0 || cap < 0 || (cap > 0 && !keys)) return STBPE_E_BADARG;
     cudaStream_t s = (cudaStream_t)stream;
     CK(cudaSetDevice(e->cfg.device));
     if (!e->counted) return fail(e, STBPE_E_STATE, "count the pairs before selecting");
     if (e->cfg.world_size > 1) return fail(e, STBPE_E_STATE, "single-rank entry point");
-    if (new_id >= 0) {
-        if (a < 0 || b < 0 || a == 0x7FFFFFFF || b == 0x7FFFFFFF || new_id == 0x7FFFFFFF)
+    const int given = a >= 0 ? 1 : 0;
+    const bool run = given || most > 0;
+    *n_done = 0;
+    if (run) {
+        if (new_id < 0 || (i64)new_id + most >= 0x7FFFFFFFll || (given && (b < 0 || a == 0x7FFFFFFF || b == 0x7FFFFFFF)))
             return fail(e, STBPE_E_ID_OVERFLOW, "Token id overflow: ids must be in [0, 2^31-2]");
         const int32_t pair[2] = {a, b};
-        int rc = run_forced(e, pair, 1, new_id, nullptr, s, true);
+        int rc = run_forced(e, pair, given, new_id, nullptr, s, true, most, n_done);
         if (rc != STBPE_OK) return rc;
     }
     std::vector<u64> tied;
     i64 c = 0;
-    int rc = tied_candidates(e, new_id >= 0, &tied, &c, s);
+    int rc = tied_candidates(e, run, &tied, &c, s);
     if (rc != STBPE_OK) return rc;
     *count = c;
     *n_ties = (i64)tied.size();
@@ -1242,15 +1248,22 @@ static int loop_grid(const stbpe_engine *e) {
 
 // Runs loop_kernel until a stop rule fires, doing the maintenance it asks for between launches.  `forced`
 // (device, n_forced pairs): these merges instead of the best pairs.  *out = the device state at the end.
-static int run_loop(stbpe_engine *e, int target, const int2 *forced, int n_forced, int forced_new, DevState *out,
-                    cudaStream_t s, bool then_ties = false) {
+static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, int2 one, int n_forced, int forced_new, DevState *out,
+                    cudaStream_t s, bool then_ties = false, int *n_done = nullptr) {
     LoopArgs la;
     int at = 0;
+    la.mode = mode;
+    la.one = one;
+    if (!e->sync_zeroed) {
+        CK(cudaMemsetAsync(e->d.sync, 0, 2 * sizeof(LoopSync), s));
+        e->sync_zeroed = true;
+    }
     for (;;) {
         const int grid = loop_grid(e);
         la.target = target;
-        la.forced = forced ? forced + at : nullptr;
-        la.n_forced = n_forced - at;
+        const int given = at < n_forced ? at : n_forced;
+        la.forced = forced ? forced + given : nullptr;
+        la.n_forced = n_forced - given;
         la.forced_new = forced_new + at;
         const double fc = e->filter_density * (double)e->d.n_tiles;
         la.filter_count = fc >= 9e18 ? (i64)9000000000000000000ll : (i64)fc;
@@ -1260,8 +1273,9 @@ static int run_loop(stbpe_engine *e, int target, const int2 *forced, int n_force
         la.ids_below = e->only_bytes ? 0 : (int)e->max_id + 1;
         la.unit_shift = unit_shift(e, grid);
         EngineDev d = e->d;
+        d.sync = e->d.sync + e->sync_turn;
+        la.other_sync = e->d.sync + (e->sync_turn ^= 1);
         void *args[2] = {&d, &la};
-        CK(cudaMemsetAsync(e->d.sync, 0, sizeof(LoopSync), s));
         const cudaError_t c = with_tok(e, [&](auto t) {
             typedef decltype(t) T;
             return cudaLaunchCooperativeKernel((const void *)loop_kernel<T>, dim3(grid), dim3(MergeGeom<T>::THREADS), args,
@@ -1273,9 +1287,13 @@ static int run_loop(stbpe_engine *e, int target, const int2 *forced, int n_force
             CK(cudaGetLastError());
         }
         if (int rc_ = read_state(e, out, s)) return rc_;
-        at += forced ? out->forced_done : 0;
+        at += out->forced_done;
+        if (n_done) *n_done = at;
         int rc = check_error_bits(e, out->error);
-        if (rc != STBPE_OK) return rc;
+        if (rc != STBPE_OK) {
+            e->sync_zeroed = false;
+            return rc;
+        }
         if (out->run_exit == STBPE_EXIT_STOP) return STBPE_OK;
         if (out->run_exit == STBPE_EXIT_GROW) {
             rc = grow_table(e, s);
@@ -1296,14 +1314,15 @@ static int run_loop(stbpe_engine *e, int target, const int2 *forced, int n_force
 
 // host-given merges, applied in order as merges of the log
 static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t first_new, int64_t *n_matches, cudaStream_t s,
-                      bool then_ties) {
+                      bool then_ties, int most, int *n_done) {
     DevState h;
     if (!then_ties || !e->merges_known) {
         if (int rc_ = read_state(e, &h, s)) return rc_;
         e->merges_done = h.merges_done;
     }
     if ((i64)e->merges_done + n > e->cfg.max_merges) return fail(e, STBPE_E_CAPACITY, "merge log full");
-    if (n > e->forced_cap) {
+    if (most > e->cfg.max_merges - e->merges_done - n) most = e->cfg.max_merges - e->merges_done - n;
+    if (n > 1 && n > e->forced_cap) {
         dev_free(e, e->forced);
         e->forced = nullptr;
         cudaError_t c = dev_alloc(e, &e->forced, (size_t)n);
@@ -1311,11 +1330,13 @@ static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t firs
         e->forced_cap = n;
     }
     const void *src = pairs;
-    if ((size_t)n * sizeof(int2) <= STBPE_PINNED_BYTES - STBPE_PINNED_STATE)
+    if (n <= 1) {
+    } else if ((size_t)n * sizeof(int2) <= STBPE_PINNED_BYTES - STBPE_PINNED_STATE)
         src = memcpy((char *)e->pinned.p + STBPE_PINNED_STATE, pairs, (size_t)n * sizeof(int2));
-    CK(cudaMemcpyAsync(e->forced, src, (size_t)n * sizeof(int2), cudaMemcpyHostToDevice, s));
-    if ((i64)first_new + n > 65536) e->foreign_ids = true;
-    int rc = run_loop(e, e->cfg.max_merges, e->forced, n, first_new, &h, s, then_ties);
+    if (n > 1) CK(cudaMemcpyAsync(e->forced, src, (size_t)n * sizeof(int2), cudaMemcpyHostToDevice, s));
+    if ((i64)first_new + n + most > 65536) e->foreign_ids = true;
+    int rc = run_loop(e, e->merges_done + n + most, most > 0 ? LOOP_UNTIED : LOOP_NONE, n > 1 ? e->forced : nullptr,
+                      n == 1 ? make_int2(pairs[0], pairs[1]) : make_int2(0, 0), n, first_new, &h, s, then_ties, n_done);
     e->merges_known = rc == STBPE_OK;
     e->merges_done = h.merges_done;
     if (rc == STBPE_OK && n_matches) *n_matches = h.n_matches;
@@ -1333,7 +1354,7 @@ STBPE_VISIBLE int stbpe_train(stbpe_engine *e, int32_t n_merges, void *stream) {
     e->merges_known = false;
     i64 target = (i64)h.merges_done + n_merges;
     if (target > e->cfg.max_merges) target = e->cfg.max_merges;
-    return run_loop(e, (int)target, nullptr, 0, 0, &h, s);
+    return run_loop(e, (int)target, LOOP_BEST, nullptr, make_int2(0, 0), 0, 0, &h, s);
 }
 
 // Same loop as stbpe_train, launched kernel by kernel with CUDA events around every launch so

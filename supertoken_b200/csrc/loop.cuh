@@ -37,8 +37,12 @@
 
 struct LoopArgs {
     int target;             // merge count to stop at
-    const int2 *forced;     // host-given merges (a, b) applied in order instead of the best pair, or null
-    int n_forced, forced_new;  // forced merge i gets id forced_new + i
+    const int2 *forced;     // host-given merges (a, b), applied in order before any choice ...
+    int2 one;               // ... or the single one, when forced is null
+    int n_forced, forced_new;  // merge i of the launch gets id forced_new + i
+    int mode;               // what follows them: LOOP_BEST the best pairs, LOOP_NONE nothing, LOOP_UNTIED the best pairs
+                            // while no other pair has the same count
+    LoopSync *other_sync;   // counters of the next launch, which this one sets to zero
     i64 filter_count;       // leave to build the pair filter when the merge's count has fallen to this
     int dense_batch;        // merges per step while every tile is visited (no filter)
     int repack_tiles;       // leave for a re-pack at three quarters live from this many tiles on
@@ -46,6 +50,8 @@ struct LoopArgs {
     i64 grow_keys;          // leave for a larger pair table when a merge could take the number of keys beyond this ...
     int ids_below;          // ... given that the stream's own ids lie below this (0: below the merges' ids)
 };
+
+enum { LOOP_BEST, LOOP_NONE, LOOP_UNTIED };
 
 __device__ __forceinline__ u64 loop_timer_ns() {
     u64 t;
@@ -170,7 +176,8 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
     if (cta == 0 && tid == 32) {
         s_work = st->n_work;
         st->n_work = 0;
-        if (la.forced) st->n_matches = 0;
+        if (la.mode != LOOP_BEST) st->n_matches = 0;
+        la.other_sync->arrived = la.other_sync->chosen = 0;
     }
 
 #pragma unroll 1
@@ -215,8 +222,8 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
                 if (lane == 0) s_rest[warp] = v;
                 if (tid < 32) s_sorted[tid] = Bs::none();
             }
-            if (la.forced && warp == 0 && lane < KB && forced_i + lane < la.n_forced) {
-                const int2 f = la.forced[forced_i + lane];
+            if (warp == 0 && lane < KB && forced_i + lane < la.n_forced) {
+                const int2 f = la.forced ? la.forced[forced_i + lane] : la.one;
                 const i64 at = find_slot(e, ((u64)(uint32_t)f.x << 32) | (uint32_t)f.y);
                 s_forced[lane] = at >= 0 ? (i64)__ldcg((const u64 *)&e.table[at].count) : 0;
             }
@@ -244,7 +251,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
                 int place = 0;
 #pragma unroll
                 for (int q = 0; q < PER; ++q) place += __popc(__ballot_sync(0xFFFFFFFFu, v[q] > x));
-                if (place >= KB) break;
+                if (place > KB) break;  // (one more than a batch holds: the count behind its last member)
                 if (lane == 0 && x) s_sorted[place] = x;
             }
             __syncthreads();
@@ -254,21 +261,21 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
         if (warp == 0) {
             const Bt bound = KB > 1 ? Bs::warp_max(lane < WARPS ? s_rest[lane] : Bs::none()) : Bs::none();
             const Bt mine = KB > 1 ? s_sorted[lane >> 1] : Bs::warp_max(lane < WARPS ? s_top[lane] : Bs::none());
-            const bool host = la.forced != nullptr;
+            const bool host = forced_i < la.n_forced;
             const int j = KB > 1 ? lane >> 1 : 0;  // two lanes per pair: one for each of its tokens
             const unsigned int err = s_err;
             const Slot best = Bs::slot(mine);
             const bool dry = (err >> 31) != 0u || !(mc.theta.admits(best.count, best.key) || (best.count <= 0 && mc.theta.count == 0));
-            const bool forced = host && j < KB && forced_i + j < la.n_forced;
+            const bool forced = j < KB && forced_i + j < la.n_forced;
             u64 key = best.key;
             i64 count = best.count;
             if (forced) {
-                const int2 f = la.forced[forced_i + j];
+                const int2 f = la.forced ? la.forced[forced_i + j] : la.one;
                 key = ((u64)(uint32_t)f.x << 32) | (uint32_t)f.y;
                 count = s_forced[j];
             }
             const uint32_t a = (uint32_t)(key >> 32), b = (uint32_t)key;
-            const uint32_t nw0 = (uint32_t)(host ? la.forced_new + forced_i : base_vocab + merges_done), nw = nw0 + j;
+            const uint32_t nw0 = (uint32_t)(la.mode != LOOP_BEST ? la.forced_new + forced_i : base_vocab + merges_done), nw = nw0 + j;
             // a merge drops one token per occurrence of its pair (of a run, all but one), so this many are gone before it
             i64 before = 0;
             if constexpr (KB > 1) {
@@ -295,9 +302,20 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             // stop rules of the loop: bpe_trainer.py:4304-4308 (no pairs), :2491-2494 / :4361-4364 (count < 2)
             int stop = 0, why = STBPE_EXIT_STOP;
             bool go = false;
+            // LOOP_UNTIED: alone with its count, among the candidates and among the pairs that are not listed.  (The pairs
+            // that the merges before it make are rarer than some pair after it, hence rarer than it.)
+            bool tied = true;
+            if constexpr (KB > 1) {
+                if (la.mode == LOOP_UNTIED) {
+                    const Slot after = Bs::slot(max(s_sorted[j + 1], bound));
+                    tied = count <= after.count || count <= mc.theta.count || count < 2 || merges_done + j >= la.target;
+                }
+            }
             if (err & 0x7FFFFFFFu) stop = 4;
-            else if (host && !forced) stop = 0;
-            else if (!host && merges_done + j >= la.target) stop = 1;
+            else if (la.mode != LOOP_BEST && host && !forced) stop = 0;
+            else if (la.mode == LOOP_NONE && !host) stop = 0;
+            else if (la.mode == LOOP_UNTIED && !host && !dry && tied) stop = 0;  // the host looks at what there is
+            else if (!host && merges_done + j >= la.target) stop = la.mode == LOOP_BEST ? 1 : 0;
             // maintenance the host does between launches
             else if (!host && dry) why = STBPE_EXIT_REFILL;
             else if (!host && count <= 0) stop = 2;

@@ -131,22 +131,23 @@ class Engine:
         p = np.asarray(pairs, dtype=np.int32)
         self._check(self._lib.stbpe_apply_merges(self._h, p.ctypes.data, len(p), int(first_new_id), self._s))
 
-    def next_tied(self, merge: Optional[Tuple[int, int, int]] = None) -> Tuple[int, List[int]]:
-        """Apply ``merge`` = (a, b, new_id), if given, then return the best count and the keys that hold it,
-        ascending: one step of a loop that breaks ties on the host."""
-        a, b, new_id = merge if merge is not None else (0, 0, -1)
-        if max(a, b, new_id) > 0x7FFFFFFE or min(a, b) < 0:
+    def next_tied(self, merge: Optional[Tuple[int, int]] = None, new_id: int = 0, most: int = 0) -> Tuple[int, int, List[int]]:
+        """One step of a loop that breaks ties on the host: apply ``merge`` = (a, b) as ``new_id``, if given, go on
+        with up to ``most`` best pairs while each is the only one with its count, and return the number of merges
+        applied, the best count and the keys that hold it, ascending."""
+        a, b = merge if merge is not None else (-1, -1)
+        if max(a, b) > 0x7FFFFFFE or new_id + most > 0x7FFFFFFE or (merge is not None and min(a, b) < 0):
             raise OverflowError("Token id overflow: ids must be in [0, 2^31-2]")
         if getattr(self, "_tied", None) is None:
             self._tied = np.empty(1024, dtype=np.uint64)
-        count, n = ctypes.c_int64(0), ctypes.c_int64(0)
-        self._check(self._lib.stbpe_next_tied(self._h, a, b, new_id, ctypes.byref(count), self._tied.ctypes.data,
-                                              len(self._tied), ctypes.byref(n), self._s))
+        done, count, n = ctypes.c_int32(0), ctypes.c_int64(0), ctypes.c_int64(0)
+        self._check(self._lib.stbpe_next_tied(self._h, a, b, new_id, most, ctypes.byref(done), ctypes.byref(count),
+                                              self._tied.ctypes.data, len(self._tied), ctypes.byref(n), self._s))
         if count.value <= 0:
-            return 0, []
+            return done.value, 0, []
         if n.value > len(self._tied):
-            return int(count.value), self.tied_keys(int(count.value), int(n.value))
-        return int(count.value), self._tied[:n.value].tolist()
+            return done.value, int(count.value), self.tied_keys(int(count.value), int(n.value))
+        return done.value, int(count.value), self._tied[:n.value].tolist()
 
     def train(self, n_merges: int):
         self._check(self._lib.stbpe_train(self._h, int(n_merges), self._s))
