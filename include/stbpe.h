@@ -75,6 +75,12 @@ int stbpe_destroy(stbpe_engine *e);
 const char *stbpe_last_error(const stbpe_engine *e);
 const char *stbpe_version(void);
 
+/* Host only: the valid prefixes of a padded batch (tokens and valid: rows x width, valid != 0 marks a token) one behind
+ * the other into out, as bytes (elem 1) or int32 ids (elem 4), and their lengths.  STBPE_E_STATE: a row's valid
+ * marks are no prefix; STBPE_E_ID_OVERFLOW: elem 1 and an id outside 0 .. 255. */
+int stbpe_flatten_rows(const int32_t *tokens, const uint8_t *valid, int64_t rows, int64_t width, int32_t elem,
+                       void *out, int64_t *lengths);
+
 /* Ingest: pack rows into the flat int32 token stream (bit 31 = first token of a row).
  * Replaces BytePacker.encode_view + the batcher fill + GPUBatchRecord.from_cpu
  * (gpu_tokenizer/cpu_packer.py:17-61, datasets.py:75-84, bpe_trainer.py:137-222).

@@ -41,6 +41,7 @@ SIGNATURES = {
     "stbpe_version": (ctypes.c_char_p, []),
     "stbpe_reset": (_int, [_vp]),
     "stbpe_append_bytes": (_int, [_vp, _vp, _i64, _vp, _i64, _vp]),
+    "stbpe_flatten_rows": (_int, [_vp, _vp, _i64, _i64, _i32, _vp, _vp]),
     "stbpe_append_ids": (_int, [_vp, _vp, _i64, _vp, _i64, _vp]),
     "stbpe_count_initial": (_int, [_vp, _vp]),
     "stbpe_select_best": (_int, [_vp, _P(ctypes.c_uint64), _P(_i64), _P(_i64), _vp]),

@@ -90,6 +90,47 @@ def _flatten_batch(batch) -> Tuple[torch.Tensor, np.ndarray]:
     return ids, off
 
 
+def _flatten_batches(batches) -> List[Tuple[torch.Tensor, np.ndarray]]:
+    """Flat ids (uint8 while every id is below 256, else int32) and row offsets: host batches of the usual types
+    through the native pass into one piece, any other batch by ``_flatten_batch`` into a piece of its own."""
+    out: List[Tuple[torch.Tensor, np.ndarray]] = []
+    host: list = []
+
+    def flush():
+        if not host:
+            return
+        room = sum(t.numel() for t, _ in host)
+        lens = np.empty(sum(t.shape[0] for t, _ in host) + 1, dtype=np.int64)
+        lens[0] = 0
+        for dtype in (torch.uint8, torch.int32):
+            ids = torch.empty(room, dtype=dtype)
+            rows = n = 0
+            for t, v in host:
+                part = lens[1 + rows:1 + rows + t.shape[0]]
+                rc = L.load().stbpe_flatten_rows(t.data_ptr(), v.data_ptr(), t.shape[0], t.shape[1], ids.element_size(),
+                                                 ids.data_ptr() + n * ids.element_size(), part.ctypes.data)
+                if rc != 0:
+                    break
+                rows, n = rows + t.shape[0], n + int(part.sum())
+            if rc == 0:
+                break
+            if rc == L.E_STATE:
+                raise ValueError("valid must mark a prefix of every row")
+        host.clear()
+        out.append((ids[:n], np.cumsum(lens)))
+
+    for b in batches:
+        t, v = b[0], b[1]
+        if t.dim() == 2 and v.shape == t.shape and not t.is_cuda and not v.is_cuda and t.dtype == torch.int32 and \
+                v.dtype in (torch.uint8, torch.bool):
+            host.append((t.contiguous(), v.contiguous()))
+        else:
+            flush()
+            out.append(_flatten_batch(b))
+    flush()
+    return out
+
+
 class GPUBPETrainer(BaseTrainer):
     """B200 implementation of the reference's ``GPUBPETrainer`` merge loop."""
 
@@ -270,18 +311,22 @@ class GPUBPETrainer(BaseTrainer):
                 self.h2d_events += 1
             return self._run_loop(eng, log_every, t0, None, checkpoint_interval, checkpoint_dir,
                                   already=list(self.merges), dataset_state=dataset_state)
-        flat: List[Tuple[torch.Tensor, np.ndarray]] = [_flatten_batch(b) for b in batches]
-        total = sum(int(ids.numel()) for ids, _ in flat)
         mode = self._sharded_mode()
         if mode is not None:
+            flat = [_flatten_batch(b) for b in batches]
             self._reject_in_sharded_mode(warm_start_merges, checkpoint_interval)
             return self._fit_sharded(mode, flat, False, log_every, t0)
+        flat = _flatten_batches(batches)
+        total = sum(int(ids.numel()) for ids, _ in flat)
         eng = self._make_engine(total)
         for ids, off in flat:
             if ids.numel():
-                eng.append_ids(ids, off)
+                if ids.dtype == torch.uint8:
+                    eng.append_bytes(ids, off)
+                else:
+                    eng.append_ids(ids, off)
                 if not ids.is_cuda:
-                    self.bytes_h2d += ids.numel() * 4
+                    self.bytes_h2d += ids.numel() * ids.element_size()
                     self.h2d_events += 1
         return self._run_loop(eng, log_every, t0, warm_start_merges, checkpoint_interval, checkpoint_dir,
                               dataset_state=dataset_state)

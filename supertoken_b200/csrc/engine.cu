@@ -590,6 +590,34 @@ static int append_common(stbpe_engine *e, const void *data, i64 n, size_t elem, 
     return STBPE_OK;
 }
 
+// Rows of a padded host batch one behind the other, as bytes (elem 1) or ids (elem 4).  One pass over the batch; the
+// same in tensor operations (sum, comparison with a prefix, boolean gather, cast) took five.
+STBPE_VISIBLE int stbpe_flatten_rows(const int32_t *tokens, const uint8_t *valid, int64_t rows, int64_t width, int32_t elem, void *out,
+                                     int64_t *lengths) {
+    if (rows < 0 || width < 0 || (elem != 1 && elem != 4) || (rows > 0 && (!lengths || (width > 0 && (!tokens || !valid || !out))))) return STBPE_E_BADARG;
+    unsigned char *to = (unsigned char *)out;
+    for (i64 r = 0; r < rows; ++r, tokens += width, valid += width) {
+        const void *end = width > 0 ? memchr(valid, 0, (size_t)width) : nullptr;
+        const i64 n = end ? (const uint8_t *)end - valid : width;
+        uint8_t later = 0;
+        for (i64 i = n; i < width; ++i) later |= valid[i];
+        if (later) return STBPE_E_STATE;
+        lengths[r] = n;
+        if (elem == 4) {
+            if (n) memcpy(to, tokens, (size_t)n * 4);
+        } else {
+            uint32_t seen = 0;
+            for (i64 i = 0; i < n; ++i) {
+                seen |= (uint32_t)tokens[i];
+                to[i] = (unsigned char)tokens[i];
+            }
+            if (seen > 255u) return STBPE_E_ID_OVERFLOW;
+        }
+        to += n * elem;
+    }
+    return STBPE_OK;
+}
+
 STBPE_VISIBLE int stbpe_append_bytes(stbpe_engine *e, const uint8_t *data, int64_t n,
                                      const int64_t *row_offsets, int64_t n_rows, void *stream) {
     if (!e) return STBPE_E_BADARG;
@@ -1270,7 +1298,7 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
         la.dense_batch = e->dense_batch;
         la.repack_tiles = 64;
         la.grow_keys = e->table_auto ? (i64)(e->slots / 4) : (i64)0x7FFFFFFFFFFFFFFFll;
-        la.ids_below = e->only_bytes ? 0 : (int)e->max_id + 1;
+        la.ids_below = e->only_bytes ? 256 : (int)e->max_id + 1;
         la.unit_shift = unit_shift(e, grid);
         EngineDev d = e->d;
         d.sync = e->d.sync + e->sync_turn;

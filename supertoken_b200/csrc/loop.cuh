@@ -48,7 +48,7 @@ struct LoopArgs {
     int repack_tiles;       // leave for a re-pack at three quarters live from this many tiles on
     int unit_shift;         // tiles per filter unit, log2 (cta_merge)
     i64 grow_keys;          // leave for a larger pair table when a merge could take the number of keys beyond this ...
-    int ids_below;          // ... given that the stream's own ids lie below this (0: below the merges' ids)
+    int ids_below;          // ... given that the stream's own ids lie below this
 };
 
 enum { LOOP_BEST, LOOP_NONE, LOOP_UNTIED };
