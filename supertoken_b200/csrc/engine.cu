@@ -84,6 +84,7 @@ struct stbpe_engine {
     int dense_batch;
     bool sync_zeroed;     // the barrier counters of the next loop launch are zero: each launch clears the other pair
     int sync_turn;
+    bool cand_stale;      // the candidate list is used up: collect one before the next choice
     bool foreign_ids;     // a merge of the caller's may have brought an id of 65 536 or more
     unsigned int max_id;  // largest id appended through stbpe_append_ids
     unsigned int load_err;  // error bits of the rows appended so far
@@ -754,6 +755,7 @@ static int grow_table(stbpe_engine *e, cudaStream_t s) {
     e->table_cap = e->slots;
     clear_table_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d);
     cand_none_kernel<<<1, 1, 0, s>>>(e->d);
+    e->cand_stale = true;
     CK(cudaMemsetAsync(&e->d.st->n_keys, 0, sizeof(u64), s));
     rehash_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d, old, old_slots);
     CK(cudaGetLastError());
@@ -785,6 +787,7 @@ static int count_prologue(stbpe_engine *e, bool clear, cudaStream_t s) {
         CK(cudaMemsetAsync(e->d.blockmax, 0, (size_t)e->d.n_blocks * sizeof(Slot), s));  // count 0 = no candidate
     } else {
         cand_none_kernel<<<1, 1, 0, s>>>(e->d);
+    e->cand_stale = true;
         CK(cudaGetLastError());
     }
     CK(cudaMemsetAsync(&e->d.st->n_keys, 0, sizeof(u64), s));
@@ -961,19 +964,26 @@ STBPE_VISIBLE int stbpe_count_initial(stbpe_engine *e, void *stream) {
 
 // Candidate list of the pair table as it stands: threshold search (one pass over the table in the usual case,
 // further ones while a bucket holds too many pairs), then the list.
-static int refill_candidates(stbpe_engine *e, cudaStream_t s) {
+static int queue_refill(stbpe_engine *e, cudaStream_t s) {
     const u64 key_hi = e->wide ? 0x7FFFFFFFFFFFFFFFull : ((u64)Tok<uint16_t>::IDMASK << 32) | Tok<uint16_t>::IDMASK;
     const i64 want = ((i64)e->slots + 511) / 512;
     const unsigned int grid = (unsigned int)(want < e->sm_count * 4 ? want : e->sm_count * 4);
+    cand_hist_kernel<<<grid, 512, 0, s>>>(e->d);
+    cand_decide_kernel<<<1, 1024, 0, s>>>(e->d, key_hi);
+    cand_collect_kernel<<<grid, 512, 0, s>>>(e->d);
+    CK(cudaGetLastError());
+    return STBPE_OK;
+}
+static int refill_candidates(stbpe_engine *e, cudaStream_t s) {
     CK(cudaMemsetAsync(&e->d.st->cand_state, 0, sizeof(int), s));
     for (int pass = 0; pass < 16; ++pass) {
-        cand_hist_kernel<<<grid, 512, 0, s>>>(e->d);
-        cand_decide_kernel<<<1, 1024, 0, s>>>(e->d, key_hi);
-        cand_collect_kernel<<<grid, 512, 0, s>>>(e->d);
-        CK(cudaGetLastError());
+        if (int rc_ = queue_refill(e, s)) return rc_;
         DevState h;
         if (int rc_ = read_state(e, &h, s)) return rc_;
-        if (h.cand_state == STBPE_CAND_READY) return STBPE_OK;
+        if (h.cand_state == STBPE_CAND_READY) {
+            e->cand_stale = false;
+            return STBPE_OK;
+        }
     }
     return fail(e, STBPE_E_STATE, "no candidate threshold found");
 }
@@ -1301,6 +1311,14 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
         la.ids_below = e->only_bytes ? 256 : (int)e->max_id + 1;
         la.unit_shift = unit_shift(e, grid);
         EngineDev d = e->d;
+        // Candidates that have run out are collected in front of the launch without waiting for the result: one pass
+        // settles the threshold but for tables with very many equal counts, and then the launch comes back at once.
+        const bool queued = e->cand_stale;
+        if (queued) {
+            CK(cudaMemsetAsync(&e->d.st->cand_state, 0, sizeof(int), s));
+            if (int rc_ = queue_refill(e, s)) return rc_;
+            e->cand_stale = false;
+        }
         d.sync = e->d.sync + e->sync_turn;
         la.other_sync = e->d.sync + (e->sync_turn ^= 1);
         void *args[2] = {&d, &la};
@@ -1325,9 +1343,11 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
         if (out->run_exit == STBPE_EXIT_STOP) return STBPE_OK;
         if (out->run_exit == STBPE_EXIT_GROW) {
             rc = grow_table(e, s);
-            if (rc == STBPE_OK) rc = refill_candidates(e, s);
         } else if (out->run_exit == STBPE_EXIT_REFILL) {
-            rc = refill_candidates(e, s);
+            if (queued && out->forced_done == 0)
+                rc = refill_candidates(e, s);
+            else
+                e->cand_stale = true;
         } else if (out->run_exit == STBPE_EXIT_REPACK) {
             rc = maybe_repack(e, false, nullptr, s);
         } else if (out->run_exit == STBPE_EXIT_FILTER) {

@@ -408,13 +408,33 @@ __global__ void __launch_bounds__(512) cand_hist_kernel(EngineDev e) {
 // The threshold out of the histogram (which is left zeroed for the next search): buckets are taken from the top
 // while the list stays within STBPE_CAND_MOST; with too few taken and the next one too large, that bucket
 // is searched again (STBPE_CAND_REFINE).
+// (One thread walking down the 2048 buckets took up to 30 us; the running sums of a block scan take 2.)
 __global__ void __launch_bounds__(1024) cand_decide_kernel(EngineDev e, u64 key_hi) {
-    __shared__ unsigned int s_h[STBPE_CAND_BUCKETS];
+    static_assert(STBPE_CAND_BUCKETS == 2 * 1024, "two buckets per thread");
+    __shared__ i64 s_sum[32];
+    __shared__ int s_first;   // place from the top of the first bucket that does not fit
+    __shared__ i64 s_taken;   // pairs in the buckets above it
     DevState *st = e.st;
-    for (int i = threadIdx.x; i < STBPE_CAND_BUCKETS; i += blockDim.x) {
-        s_h[i] = e.cand_hist[i];
-        e.cand_hist[i] = 0u;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, hi_b = STBPE_CAND_BUCKETS - 1 - 2 * (int)threadIdx.x;
+    const i64 n0 = e.cand_hist[hi_b], n1 = e.cand_hist[hi_b - 1], base = st->cand_state == STBPE_CAND_REFINE ? st->refine_above : 0;
+    e.cand_hist[hi_b] = e.cand_hist[hi_b - 1] = 0u;
+    if (threadIdx.x == 0) s_first = STBPE_CAND_BUCKETS;
+    i64 incl = n0 + n1;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const i64 o = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+        if (lane >= d) incl += o;
     }
+    if (lane == 31) s_sum[warp] = incl;
+    __syncthreads();
+    i64 before = base + incl - n0 - n1;
+    for (int w = 0; w < warp; ++w) before += s_sum[w];
+    const bool out0 = before + n0 > STBPE_CAND_MOST, out1 = before + n0 + n1 > STBPE_CAND_MOST;
+    if (out0 || out1) atomicMin(&s_first, 2 * (int)threadIdx.x + (out0 ? 0 : 1));
+    __syncthreads();
+    if (s_first == 2 * (int)threadIdx.x) s_taken = before;
+    if (s_first == 2 * (int)threadIdx.x + 1) s_taken = before + n0;
+    if (s_first == STBPE_CAND_BUCKETS && threadIdx.x == 1023) s_taken = before + n0 + n1;
     __syncthreads();
     if (threadIdx.x != 0) return;
     st->n_cand = 0;
@@ -423,9 +443,8 @@ __global__ void __launch_bounds__(1024) cand_decide_kernel(EngineDev e, u64 key_
     const u64 klo = st->refine_klo, khi = st->refine_khi;
     const bool by_key = refine && lo == hi;
     const int sh = !refine ? 0 : (by_key ? linear_shift(klo, khi) : linear_shift((u64)lo, (u64)hi));
-    i64 taken = refine ? st->refine_above : 0;
-    int b = STBPE_CAND_BUCKETS - 1;
-    for (; b >= 0 && taken + (i64)s_h[b] <= STBPE_CAND_MOST; --b) taken += s_h[b];
+    const i64 taken = s_taken;
+    const int b = STBPE_CAND_BUCKETS - 1 - s_first;
     // bucket b does not fit (or b < 0: everything does); the list takes the buckets above it
     if (b >= 0 && taken < STBPE_CAND_LEAST) {
         st->cand_state = STBPE_CAND_REFINE;

@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             if (tid == THREADS - 1) {
                 s_live = (i64)__ldcg((const u64 *)&st->n_live);
                 s_keys = (i64)__ldcg(&st->n_keys);
-                s_err = __ldcg(&st->error) | (n > STBPE_CAND_CAP ? 0x80000000u : 0u);
+                s_err = __ldcg(&st->error) | (n > STBPE_CAND_CAP || __ldcg(&st->cand_state) != STBPE_CAND_READY ? 0x80000000u : 0u);
                 if (cta == 0 && step > 0) {
                     s_work = fv ? __ldcg(&st->n_work) : -1;
                     st->n_work = 0;
