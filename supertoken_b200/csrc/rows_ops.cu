@@ -100,10 +100,16 @@ __global__ void rows_write_kernel(const u64 *__restrict__ keys, const i64 *__res
 }
 
 // ---- stbpe_rows_count_pairs
-#define ROWS_COUNT_NT 256
-#define ROWS_SMEM_SLOTS 2048
+// Threads and shared-memory slots of a counting CTA.  Small batches: short to clear, and several CTAs per SM.  From 2^18
+// cells on: a table for the some 10^4 pairs that byte-level text holds (a pair that finds no slot is added in L2 by
+// itself: with 2048 slots 2048 x 4096 cells of mixed text, 6 900 pairs, took 181 us).
+#define ROWS_SMALL_NT 256
+#define ROWS_SMALL_SLOTS 2048
+#define ROWS_LARGE_NT 1024
+#define ROWS_LARGE_SLOTS 16384
+#define ROWS_LARGE_CELLS (1 << 18)
 #define ROWS_RANK_MAX 16384   // up to this many pairs are sorted by counting smaller keys, two launches instead of a radix sort's nine
-#define ROWS_RANK_TILE 2048
+#define ROWS_RANK_TILE 512
 
 __global__ void rows_init_kernel(RowsTable t, unsigned int *rank, unsigned int n_rank) {
     const u64 first = (u64)blockIdx.x * blockDim.x + threadIdx.x, step = (u64)gridDim.x * blockDim.x;
@@ -141,10 +147,12 @@ __device__ __forceinline__ void rows_add(const RowsTable &t, u64 key, u64 n) {
 // A pair (i, i+1) of a row counts when both positions are valid (gpu_tokenizer/utils.py:586).  Four cells per thread
 // and step as one 16-byte and one 4-byte load over the flat batch; a CTA collects its pairs in shared memory
 // and adds each distinct one once.
+template <int ROWS_COUNT_NT, int ROWS_SMEM_SLOTS>
 __global__ void __launch_bounds__(ROWS_COUNT_NT) rows_pairs_kernel(const int32_t *__restrict__ tokens, const uint8_t *__restrict__ valid,
                                                                    i64 B, i64 L, RowsTable t) {
-    __shared__ u64 s_key[ROWS_SMEM_SLOTS];
-    __shared__ int s_val[ROWS_SMEM_SLOTS];
+    extern __shared__ __align__(16) unsigned char s_rows[];
+    u64 *s_key = reinterpret_cast<u64 *>(s_rows);
+    int *s_val = reinterpret_cast<int *>(s_key + ROWS_SMEM_SLOTS);
     for (int i = threadIdx.x; i < ROWS_SMEM_SLOTS; i += ROWS_COUNT_NT) s_key[i] = STBPE_EMPTY, s_val[i] = 0;
     __syncthreads();
     const i64 cells = B * L;
@@ -193,8 +201,10 @@ __global__ void __launch_bounds__(ROWS_COUNT_NT) rows_pairs_kernel(const int32_t
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < ROWS_SMEM_SLOTS; i += ROWS_COUNT_NT)
+    for (int k = threadIdx.x; k < ROWS_SMEM_SLOTS; k += ROWS_COUNT_NT) {  // each CTA from another place on
+        const int i = (k + (int)blockIdx.x * (ROWS_SMEM_SLOTS / 128)) & (ROWS_SMEM_SLOTS - 1);
         if (s_val[i] && !(*(volatile unsigned int *)t.error)) rows_add(t, s_key[i], (u64)s_val[i]);
+    }
 }
 
 // rank[i] += keys of the tile blockIdx.y that are smaller than key i
@@ -410,11 +420,20 @@ STBPE_VISIBLE int stbpe_rows_count_pairs(const int32_t *tokens, const uint8_t *v
             i64 *counts = (i64 *)(base + counts_at);
             unsigned int *rank = (unsigned int *)(base + rank_at);
             const i64 quads = (B * L + 3) / 4;
-            const i64 want = (quads + ROWS_COUNT_NT - 1) / ROWS_COUNT_NT, most_ctas = 148 * 4;
+            const i64 ranked = (i64)most < ROWS_RANK_MAX ? (i64)most : ROWS_RANK_MAX;  // more pairs than these take the radix sort
+            const bool large = B * L >= ROWS_LARGE_CELLS;
+            const int nt = large ? ROWS_LARGE_NT : ROWS_SMALL_NT;
+            const i64 want = (quads + nt - 1) / nt, most_ctas = large ? 148 : 148 * 4;
+            const unsigned int grid = (unsigned int)(want < most_ctas ? want : most_ctas);
             rows_init_kernel<<<slots < (1u << 18) ? 64 : 592, 256, 0, s>>>(t, rank, (unsigned int)(most < ROWS_RANK_MAX ? most : ROWS_RANK_MAX));
-            if (total > 0) rows_pairs_kernel<<<(unsigned int)(want < most_ctas ? want : most_ctas), ROWS_COUNT_NT, 0, s>>>(tokens, valid, B, L, t);
+            if (total > 0 && large) {
+                cudaFuncSetAttribute(rows_pairs_kernel<ROWS_LARGE_NT, ROWS_LARGE_SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_LARGE_SLOTS * 12);
+                rows_pairs_kernel<ROWS_LARGE_NT, ROWS_LARGE_SLOTS><<<grid, ROWS_LARGE_NT, ROWS_LARGE_SLOTS * 12, s>>>(tokens, valid, B, L, t);
+            } else if (total > 0) {
+                rows_pairs_kernel<ROWS_SMALL_NT, ROWS_SMALL_SLOTS><<<grid, ROWS_SMALL_NT, ROWS_SMALL_SLOTS * 12, s>>>(tokens, valid, B, L, t);
+            }
             if (total > 0) rows_export_kernel<<<slots < (1u << 18) ? 64 : 592, 256, 0, s>>>(t, keys, counts, n_out, (i64)most);
-            if (total > 0) rows_rank_kernel<<<dim3(ROWS_RANK_MAX / 256, ROWS_RANK_MAX / ROWS_RANK_TILE), 256, 0, s>>>(keys, t.n_keys, t.error, rank);
+            if (total > 0) rows_rank_kernel<<<dim3((unsigned int)((ranked + 255) / 256), (unsigned int)((ranked + ROWS_RANK_TILE - 1) / ROWS_RANK_TILE)), 256, 0, s>>>(keys, t.n_keys, t.error, rank);
             i64 wb = (cap + 255) / 256;
             if (wb > 148 * 16) wb = 148 * 16;
             rows_place_kernel<<<(unsigned int)(wb > 0 ? wb : 1), 256, 0, s>>>(keys, counts, rank, t, pair_keys, (i64 *)pair_counts, cap, (i64 *)length_dev);
