@@ -457,9 +457,27 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
     if (!__all_sync(0xFFFFFFFFu, edge_ok)) {
         // readers of this merge never pick a record stamped m, so payload and stamp need no ordering
         uint32_t *r = reinterpret_cast<uint32_t *>(e.recs + 2 * (i64)tile + ((second & 0x40u) ? 0 : 1));
+        const uint32_t ne2 = __ballot_sync(0xFFFFFFFFu, NL != 0u), n2 = NL & (NL - 1u), n3 = n2 & (n2 - 1u);
+        const uint32_t two = __ballot_sync(0xFFFFFFFFu, n2 != 0u), three = __ballot_sync(0xFFFFFFFFu, n3 != 0u);
+        const int fl = lsb(ne2), ll = 31 - __clz(ne2);
+        if (ne2 && ((three >> fl) & (two >> ll) & 1u)) {  // the usual case: one lane holds the first three, one the last two
+            if (lane == fl) {
+                ws.recs += 1;
+                r[0] = (uint32_t)c.m;
+                r[1] = (uint32_t)newlen;
+                r[2] = K::widen(tok[K::sindex(lsb(NL))]);
+                r[3] = K::widen(tok[K::sindex(lsb(n2))]);
+                r[4] = K::widen(tok[K::sindex(lsb(n3))]);
+            }
+            if (lane == ll) {
+                const int p = 31 - __clz(NL);
+                r[5] = K::widen(tok[K::sindex(p)]);
+                r[6] = K::widen(tok[K::sindex(31 - __clz(NL ^ (1u << p)))]);
+            }
+            return;
+        }
         uint32_t *mL = wm + MergeGeom<T>::RAW_WORDS;
         mL[lane] = NL;
-        const uint32_t ne2 = __ballot_sync(0xFFFFFFFFu, NL != 0u);
         __syncwarp();
         if (lane == 0) {
             ws.recs += 1;
