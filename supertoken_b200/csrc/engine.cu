@@ -81,7 +81,6 @@ struct stbpe_engine {
     std::vector<stbpe::Block> allocs;
     bool broken;          // a CUDA call failed: work of this engine may still be pending
     stbpe::Block pinned;  // host side of small transfers: the device state, then small inputs
-    int dense_batch;
     bool sync_zeroed;     // the barrier counters of the next loop launch are zero: each launch clears the other pair
     int sync_turn;
     bool cand_stale;      // the candidate list is used up: collect one before the next choice
@@ -359,8 +358,6 @@ STBPE_VISIBLE int stbpe_create(stbpe_engine **out, const stbpe_config *cfg) {
     e->dense32_min = 1ll << 24;
     if (const char *v = getenv("STBPE_DENSE32_MIN_TOKENS")) e->dense32_min = atoll(v);
     e->use_graph = getenv("STBPE_NO_GRAPH") == nullptr;
-    e->dense_batch = 4;
-    if (const char *v = getenv("DEV_DENSE")) e->dense_batch = atoi(v);
     e->part_group = STBPE_PARTS;
     if (const char *v = getenv("STBPE_PART_GROUP")) e->part_group = atoi(v) > 0 ? atoi(v) : STBPE_PARTS;
     e->filter_density = 1.0;
@@ -1305,7 +1302,6 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
         la.forced_new = forced_new + at;
         const double fc = e->filter_density * (double)e->d.n_tiles;
         la.filter_count = fc >= 9e18 ? (i64)9000000000000000000ll : (i64)fc;
-        la.dense_batch = e->dense_batch;
         la.repack_tiles = 64;
         la.grow_keys = e->table_auto ? (i64)(e->slots / 4) : (i64)0x7FFFFFFFFFFFFFFFll;
         la.ids_below = e->only_bytes ? 256 : (int)e->max_id + 1;

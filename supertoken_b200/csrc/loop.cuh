@@ -44,7 +44,6 @@ struct LoopArgs {
                             // while no other pair has the same count
     LoopSync *other_sync;   // counters of the next launch, which this one sets to zero
     i64 filter_count;       // leave to build the pair filter when the merge's count has fallen to this
-    int dense_batch;        // merges per step while every tile is visited (no filter)
     int repack_tiles;       // leave for a re-pack at three quarters live from this many tiles on
     int unit_shift;         // tiles per filter unit, log2 (cta_merge)
     i64 grow_keys;          // leave for a larger pair table when a merge could take the number of keys beyond this ...
@@ -290,7 +289,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             const i64 ids = max((int)nw, la.ids_below), made = min(before + count, ids * (j + 1));
             // a later member: the order is exact so far, no token is second in one pair and first in another, none is one of
             // the members' new ones (a pair that the host gives may name one, or be given twice)
-            bool out = j >= (fv ? KB : min(la.dense_batch, KB));
+            bool out = false;
             if constexpr (KB > 1) {
                 const uint32_t same = __match_any_sync(0xFFFFFFFFu, lane >= 2 * KB ? 0x80000000u | lane : lane & 1 ? b : a);
                 out = out || (!host && !(mine > bound)) || max(a, b) >= nw0 || (same & ((1u << (lane & ~1)) - 1u) & (lane & 1 ? 0x5555u : 0xAAAAu));

@@ -32,8 +32,9 @@
 #define STBPE_LIST_UNITS 256              // filter units (of at most 8 tiles) per batch
 static_assert(STBPE_LIST_UNITS * 8 <= STBPE_LIST, "a batch of units fits the list");
 
-// Pairs of a batch.  Late in a run on text four of the next best pairs on average share no token (8 in a batch;
-// 16 would give 5 % more, 4 would give 3.3), and what a late merge costs is latency.  The wide stream, whose ids leave
+// Pairs of a batch.  Late in a run on text 5.6 of the next best pairs on average can go together when eight may (3.6 of
+// four, 6.7 of twelve), and what a late merge costs is latency.  (Twelve: 6 % less per late merge of 256 MiB, 3 % more
+// per early one of 1 GiB, where the fourth bit of the pair number costs registers in every tile.)  The wide stream, whose ids leave
 // the neighbour histogram's keys no room for a pair number, takes one at a time.
 template <typename T>
 struct Batch;
