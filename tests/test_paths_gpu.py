@@ -1,0 +1,187 @@
+"""Dispatch edges of the CUDA engine against the CPU oracle: merges taken together, streams that widen, merges the
+host gives, many equal counts, tables that are rebuilt, the row seam's table sizes.  Every comparison is exact."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+from supertoken_b200 import ops, synth
+from supertoken_b200.engine import Engine
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True, params=["policy", "filter_always"])
+def filter_mode(request, monkeypatch):
+    if request.param == "filter_always":
+        monkeypatch.setenv("STBPE_FILTER_DENSITY", "1e30")
+    return request.param
+
+
+def _engine(ids, off, base_vocab, target, slots=1 << 18):
+    e = Engine(max(len(ids), 1), base_vocab=base_vocab, max_merges=max(target, 1), table_slots=slots)
+    e.append_ids(ids, off)
+    e.count_initial()
+    return e
+
+
+def _check(e, ids, off, base_vocab, target):
+    """A finished run: merges, counts, stream and histogram as the oracle's."""
+    m, cnt, _ = e.merges()
+    om, oc, _ = O.train_flat(ids, off, base_vocab, target, 1)
+    assert m == om and cnt.tolist() == oc
+    ids2, off2 = ids.copy(), off.copy()
+    for i, (a, b) in enumerate(om):
+        O.apply_merge_flat(ids2, off2, a, b, base_vocab + i)
+    gi, _ = e.export_stream()
+    assert np.array_equal(gi, ids2[:off2[-1]])
+    _check_histogram(e, ids2[:off2[-1]].copy(), off2)
+
+
+def _check_histogram(e, ids, off):
+    k, c = e.export_histogram()
+    ok, oc = O.count_pairs_flat(ids, off, 1)
+    assert np.array_equal(k.cpu().numpy().astype(np.uint64), ok) and np.array_equal(c.cpu().numpy(), oc)
+
+
+def _rows(ids, rng, mean):
+    cuts = np.unique(rng.randint(1, len(ids), max(len(ids) // mean, 1)))
+    return np.concatenate([[0], cuts, [len(ids)]]).astype(np.int64)
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_merges_that_share_a_token_or_touch(seed):
+    # words over few tokens: pairs with a common first or second token, chains, runs, matches side by side on tile seams
+    rng = np.random.RandomState(seed)
+    words = [[1, 2], [1, 3], [4, 2], [5, 6], [6, 7], [8, 8, 8], [2, 1], [9]]
+    ids = np.array([t for w in rng.choice(len(words), 9000, p=rng.dirichlet(np.ones(len(words)))) for t in words[w]], dtype=np.int32)
+    off = _rows(ids, rng, 700 if seed % 2 else 40)
+    e = _engine(ids, off, 16, 60)
+    e.train(60)
+    _check(e, ids, off, 16, 60)
+    e.close()
+
+
+@pytest.mark.parametrize("top", [32764, 65534])
+def test_stream_widens_while_training_and_while_appending(top):
+    # new ids pass the largest of a 16-bit stream in mid-run; ids of a later piece do so at once; exports beyond 65 535
+    rng = np.random.RandomState(top)
+    ids = rng.choice([1, 2, 3, 4], 6000).astype(np.int32)
+    off = _rows(ids, rng, 300)
+    e = _engine(ids, off, top, 12)
+    e.train(12)
+    _check(e, ids, off, top, 12)
+    e.close()
+    more = np.concatenate([ids, rng.choice([5, top, top + 1], 3000).astype(np.int32)])
+    off2 = np.concatenate([off, [len(more)]]).astype(np.int64)
+    e = Engine(len(more), base_vocab=top + 2, max_merges=12, table_slots=1 << 18)
+    e.append_ids(ids, off)
+    e.append_ids(more[len(ids):].copy())
+    e.count_initial()
+    e.train(12)
+    _check(e, more, off2, top + 2, 12)
+    e.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 9, 40])
+def test_merges_given_by_the_host(n):
+    # absent pairs, a pair twice in a row, pairs of the new ids, pairs that share tokens
+    rng = np.random.RandomState(n)
+    ids = rng.randint(0, 12, 20000).astype(np.int32)
+    off = _rows(ids, rng, 500)
+    pairs = [(1, 2), (1, 3), (1, 2), (16, 4), (5, 5), (5, 6), (900, 901), (17, 18)]
+    pairs = (pairs + [(int(a), int(b)) for a, b in rng.randint(0, 30, (40, 2))])[:n]
+    e = _engine(ids, off, 16, n)
+    e.apply_merges(pairs, 16)
+    ids2, off2 = ids.copy(), off.copy()
+    for i, (a, b) in enumerate(pairs):
+        O.apply_merge_flat(ids2, off2, a, b, 16 + i)
+    gi, _ = e.export_stream()
+    assert np.array_equal(gi, ids2[:off2[-1]]) and e.merges()[0] == pairs
+    _check_histogram(e, ids2[:off2[-1]].copy(), off2)
+    e.close()
+
+
+@pytest.mark.parametrize("most", [0, 3, 50])
+def test_ties_are_left_to_the_host(most):
+    rng = np.random.RandomState(5)
+    ids = rng.randint(0, 40, 4000).astype(np.int32)
+    off = _rows(ids, rng, 200)
+    e = _engine(ids, off, 64, 60)
+    ids2, off2 = ids.copy(), off.copy()
+    made, drawn, draws = [], None, 0
+    while len(made) < 50:
+        room = min(most, 50 - len(made) - (drawn is not None))
+        done, count, tied = e.next_tied(drawn, 64 + len(made), room)
+        assert done <= (drawn is not None) + room
+        for j in range(done):
+            k, c = O.count_pairs_flat(ids2[:off2[-1]].copy(), off2, 1)
+            best = np.sort(k[c == c.max()])
+            pair = drawn if drawn is not None and j == 0 else (int(best[0]) >> 32, int(best[0]) & 0xFFFFFFFF)
+            assert (drawn is not None and j == 0) or len(best) == 1
+            O.apply_merge_flat(ids2, off2, *pair, 64 + len(made))
+            made.append(pair)
+        k, c = O.count_pairs_flat(ids2[:off2[-1]].copy(), off2, 1)
+        assert count == c.max() and tied == np.sort(k[c == c.max()]).tolist()
+        drawn = (tied[-1] >> 32, tied[-1] & 0xFFFFFFFF)
+        draws += 1
+    assert e.merges()[0] == made and (most == 0 or draws < 50)
+    e.close()
+
+
+@pytest.mark.parametrize("n", [300, 1025, 5000, 20000])
+def test_more_equal_counts_than_candidates(n):
+    # n pairs of count 2: the threshold has to be found among the keys
+    ids = np.tile(np.random.RandomState(n).permutation(n).astype(np.int32), 2)
+    off = np.array([0, n, 2 * n], dtype=np.int64)
+    e = _engine(ids, off, n, 20, 1 << 17)
+    e.train(20)
+    _check(e, ids, off, n, 20)
+    e.close()
+
+
+@pytest.mark.parametrize("slots,n", [(1 << 10, 3), (1 << 13, 1025), (1 << 18, 8193), (1 << 21, 400001)])
+def test_partitioned_count_builds_tables_of_any_size(slots, n, monkeypatch):
+    monkeypatch.setenv("STBPE_DENSE32_MIN_TOKENS", "1")
+    rng = np.random.RandomState(n)
+    ids = (rng.zipf(1.3, n) % 65536).astype(np.int32)
+    off = _rows(ids, rng, 97)
+    e = _engine(ids, off, 65536, 4, slots)
+    _check_histogram(e, ids, off)
+    e.close()
+
+
+def test_pair_table_grows_in_mid_run():
+    c = synth.config5_adversarial(24 << 20, seed=3, device="cuda")
+    off = c.row_offsets.cpu().numpy().astype(np.int64)
+    e = Engine(24 << 20, max_merges=700)
+    e.append_bytes(c.data, off)
+    e.count_initial()
+    slots = e.state().table_slots
+    e.train(700)
+    assert e.state().table_slots > slots
+    k, n = e.export_histogram()
+    e.count_initial()  # recount of the rewritten stream
+    k2, n2 = e.export_histogram()
+    assert torch.equal(k, k2) and torch.equal(n, n2)
+    e.close()
+
+
+@pytest.mark.parametrize("rows,width,alphabet", [(1, 2, 4), (64, 4095, 128), (64, 4096, 128), (64, 4096, 129), (16, 16385, 70000),
+                                                 (40, 4000, 70000)])
+def test_seam_count_at_its_table_and_rank_limits(rows, width, alphabet):
+    # both shared-memory tables (from 2^18 cells on the large one), up to and beyond 16 384 pairs, and a repeated count
+    g = np.random.RandomState(rows * width)
+    t = g.randint(0, alphabet, (rows, width)).astype(np.int32)
+    v = (np.arange(width)[None, :] < g.randint(width // 2, width + 1, (rows, 1))).astype(np.uint8)
+    cap = rows * width
+    keys = torch.empty((cap, 2), dtype=torch.int32, device="cuda")
+    counts = torch.empty(cap, dtype=torch.int64, device="cuda")
+    length = torch.empty(1, dtype=torch.int64, device="cuda")
+    ops.count_pairs(torch.from_numpy(t).cuda(), torch.from_numpy(v).cuda(), keys, counts, length)
+    ok, oc = O.count_pairs_rows(t, v)
+    n = int(length.item())
+    got = (keys[:n, 0].to(torch.int64) << 32) | keys[:n, 1].to(torch.int64)
+    assert np.array_equal(got.cpu().numpy().astype(np.uint64), ok) and np.array_equal(counts[:n].cpu().numpy(), oc)
+    best = ops.select_best_pair(ops.PairHistogramResult(got.contiguous(), counts[:n]))
+    assert tuple(best[:2]) == O.select_best(ok, oc)
