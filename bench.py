@@ -327,8 +327,8 @@ def count_bench(wl, dev, K, W, with_e2e=True):
                    "sum_of_counts_equals_pair_positions": sum_ok,
                    "l2": "inputs larger than L2", "bytes_per_token": 4},
         "roofline": {"bound": "hbm",
-                     "kernel": ("partition_pairs_kernel + partition_table_kernel (all 256 partitions in one launch): both passes, until the "
-                                "pair table is complete") if conv and conv[0] > 0 else "count_kernel",
+                     "kernel": ("partition_pairs_kernel, sub_partition_kernel, build_table_kernel: all passes, until the pair table is "
+                                "complete") if conv and conv[0] > 0 else "count_kernel",
                      "achieved": gbs, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": gbs / peak,
                      "frac_of_8tbs": gbs / 8000.0, "kernel_ms": med, "second_pass_ms": float(np.median(conv)),
                      "call_ms": float(np.median(call)), "traffic": None},
@@ -446,7 +446,7 @@ def main():
     sel_ms, mrg_ms, ref_ms, repack_ms = eng.train_timed(K)
     torch.cuda.synchronize()
     st_t = eng.state()
-    # what the merge kernel's bulk copies moved during the timed merges
+    # what the merge kernel loaded and stored during the timed merges
     tile_bytes = float(st_t.tile_bytes_in + st_t.tile_bytes_out) - float(st_b.tile_bytes_in + st_b.tile_bytes_out)
     merges_again, _, _ = eng.merges(M, eng.state().merges_done - M)
     assert merges_again == merges_gpu, "merge list changed between two runs on the same input"
@@ -531,13 +531,13 @@ def main():
                      "algorithmic_bytes": algo_bytes, "kernel_ms": mrg_ms, "launches": done,
                      "other_kernels_ms": {"select_kernel": sel_ms, "refresh_kernel": ref_ms, "repack": repack_ms},
                      "traffic": tile_bytes / done,
-                     "traffic_note": "bytes per launch that the kernel's own bulk copies moved in this run (tiles and tile "
-                                     "records read + rewritten tile parts and records stored, counted by the kernel); "
+                     "traffic_note": "bytes per launch that the kernel loaded and stored in this run (tiles of 16-bit tokens and tile "
+                                     "records read + rewritten units and records stored, counted by the kernel); "
                                      "the ncu summaries under profiles/ give dram__bytes for the same kernel"},
         "e2e": {"value": e2e, "unit": "merges/s", "seconds": e2e_s,
                 "h2d_bytes_per_step": (n_tokens + off_np.nbytes) / max(len(learned), 1),
                 "d2h_bytes_per_step": 24.0},
-        "gpu_launches": 4 * done + 2,   # select, worklist, merge, refresh per merge; the count and the final selection
+        "gpu_launches": 7,   # at least: table clear, count, its transfer to the table, three for the candidates, the loop
         "clocks": clocks,
         "cpu_baseline": cpu,
     }

@@ -42,7 +42,7 @@ typedef struct stbpe_config {
     int32_t device;          /* CUDA device ordinal */
     int32_t base_vocab;      /* first merge gets id base_vocab (bpe_trainer.py:4365) */
     int64_t max_tokens;      /* capacity of the token stream on this engine */
-    int64_t table_slots;     /* pair table capacity, rounded up to a power of two; 0 = auto */
+    int64_t table_slots;     /* pair table capacity, rounded up to a power of two; 0 = by the stream, growing with the keys */
     int32_t max_merges;      /* capacity of the merge log */
     int32_t world_size;      /* >1: pair keys are owned by hash(key) % world_size */
     int32_t rank;
@@ -57,7 +57,7 @@ typedef struct stbpe_state {
     int64_t table_slots;
     uint32_t device_error;    /* raw device error bits (0 = none) */
     int32_t n_tiles;
-    int64_t fixups;           /* dropped partners handled outside the visited tiles (statistics) */
+    int64_t fixups;           /* matches whose dropped token sits in another tile than their head (statistics) */
     int64_t repacks;          /* dense re-packs of the stream so far */
     int64_t work_tiles;       /* tiles visited by the last merge (after the pair filter) */
     double count_kernel_ms;   /* device time of the histogram kernel(s) of the last count; on the
@@ -131,7 +131,7 @@ int stbpe_next_tied(stbpe_engine *e, int32_t a, int32_t b, int32_t new_id, int32
  * stop rule fires.  Synchronises the stream before returning. */
 int stbpe_train(stbpe_engine *e, int32_t n_merges, void *stream);
 
-/* stbpe_train with CUDA events around every kernel launch (no graph replay): kernel_ms[0..3]
+/* stbpe_train with one launch per choice and merge and CUDA events around each: kernel_ms[0..3]
  * receive the summed device time of the select, merge and refresh kernels and of the re-packs.  Measurement aid
  * for the per-stage timings the reference records (gpu_tokenizer/bpe_trainer.py:4249-4260,
  * :4385-4396). */

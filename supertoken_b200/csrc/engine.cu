@@ -1,4 +1,4 @@
-// Host side of the C ABI declared in include/stbpe.h: memory, launches, CUDA graphs.
+// Host side of the C ABI declared in include/stbpe.h: memory, launches, maintenance between them.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <cuda_runtime.h>
@@ -1275,12 +1275,6 @@ __global__ void set_target_kernel(EngineDev e, int target) {
     e.st->n_matches = 0;
 }
 
-// CTAs of a loop launch: one per SM, fewer on a stream of few tiles (every CTA is a participant of two
-// grid-wide exchanges per merge); enough of them that the block maxima fit their shared memory
-static int loop_grid(const stbpe_engine *e) {
-    return e->sm_count;
-}
-
 // Runs loop_kernel until a stop rule fires, doing the maintenance it asks for between launches.  `forced`
 // (device, n_forced pairs): these merges instead of the best pairs.  *out = the device state at the end.
 static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, int2 one, int n_forced, int forced_new, DevState *out,
@@ -1294,7 +1288,7 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
         e->sync_zeroed = true;
     }
     for (;;) {
-        const int grid = loop_grid(e);
+        const int grid = e->sm_count;  // one CTA per SM; the barrier is no faster with fewer
         la.target = target;
         const int given = at < n_forced ? at : n_forced;
         la.forced = forced ? forced + given : nullptr;
