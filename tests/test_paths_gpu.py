@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from oracle import oracle as O
-from supertoken_b200 import ops, synth
+from supertoken_b200 import ops
 from supertoken_b200.engine import Engine
 
 pytestmark = pytest.mark.gpu
@@ -152,13 +152,14 @@ def test_partitioned_count_builds_tables_of_any_size(slots, n, monkeypatch):
 
 
 def test_pair_table_grows_in_mid_run():
-    c = synth.config5_adversarial(24 << 20, seed=3, device="cuda")
-    off = c.row_offsets.cpu().numpy().astype(np.int64)
-    e = Engine(24 << 20, max_merges=700)
-    e.append_bytes(c.data, off)
+    # random bytes: every merge makes some hundred pairs that were not there before
+    n = 16 << 20
+    data = torch.randint(0, 256, (n,), dtype=torch.uint8, device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    e = Engine(n, max_merges=1000)
+    e.append_bytes(data, np.arange(0, n + 1, n // 64))
     e.count_initial()
     slots = e.state().table_slots
-    e.train(700)
+    e.train(1000)
     assert e.state().table_slots > slots
     k, n = e.export_histogram()
     e.count_initial()  # recount of the rewritten stream
