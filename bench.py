@@ -76,10 +76,17 @@ class ClockSampler:
         try:
             fd, self.path = tempfile.mkstemp(suffix=".csv")
             self.proc = subprocess.Popen(["nvidia-smi", f"--query-gpu={self.Q}", "--format=csv,noheader,nounits",
-                                          "-i", str(self.index), "-lms", "200"], stdout=fd, stderr=subprocess.DEVNULL)
+                                          "-i", str(self.index), "-lms", "20"], stdout=fd, stderr=subprocess.DEVNULL)
             os.close(fd)
         except Exception:
             self.proc = None
+
+    def wait_under_load(self, work, seconds: float = 3.0):
+        """Repeat untimed work until the first sample is there: nvidia-smi takes longer to start than the timed
+        region may last."""
+        end = time.perf_counter() + seconds
+        while self.proc is not None and time.perf_counter() < end and os.path.getsize(self.path) == 0:
+            work()
 
     def stop(self) -> dict:
         out = {"sm_mhz": None, "sm_max_mhz": None, "reasons": [], "samples": 0}
@@ -413,9 +420,17 @@ def main():
     torch.cuda.synchronize()
 
     # timed: initial histogram (reported on its own) and K merges
-    load()
     sampler = ClockSampler(local_rank)
     sampler.start()
+
+    def warm():
+        load()
+        eng.count_initial()
+        eng.train(W)
+        torch.cuda.synchronize()
+
+    sampler.wait_under_load(warm)
+    load()
     t0 = ev()
     eng.count_initial()
     tc = ev()

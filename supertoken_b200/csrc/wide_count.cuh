@@ -284,31 +284,51 @@ __global__ void __launch_bounds__(STBPE_BUILD_THREADS, 3) build_table_kernel(Eng
         __syncthreads();
         const int p = task >> sub_bits, d = task & (D - 1);
         const int chunks = pb.n_cta * chunks_per_region;
-        for (int c = warp; c < chunks; c += STBPE_BUILD_THREADS / 32) {
-            const i64 chunk = (i64)p * chunks + c;
-            const unsigned int lo = offs[chunk * (D + 1) + d], hi = offs[chunk * (D + 1) + d + 1];
-            const i64 region = (i64)p * pb.n_cta + c / chunks_per_region;
-            const uint32_t *w = pb.words + region * pb.cap + (i64)(c % chunks_per_region) * STBPE_SUB_CHUNK;
-            for (unsigned int i = lo + lane; i < hi; i += 32) {
-                const uint32_t x = __ldcs(w + i);
-                unsigned int h = (x >> shift) & (TS - 1);
-                for (;;) {
-                    uint32_t k = ((volatile uint32_t *)s_word)[h];
-                    if (k == none) {
-                        k = atomicCAS(&s_word[h], none, x);
-                        if (k == none) k = x;
-                    }
-                    if (k == x) {
-                        atomicAdd(&s_num[h], 1u);
-                        break;
-                    }
-                    if (++h == TS) {
-                        const unsigned int j = atomicAdd(n_spill, 1u);
-                        if (j < spill_cap)
-                            spill[j] = x;
-                        else
-                            atomicOr(&e.st->error, STBPE_DERR_DENSE_OVERFLOW);
-                        break;
+        // A warp takes every sixteenth chunk.  Where a chunk's words are, each lane reads for another chunk, and the
+        // next chunk's first words are on their way while one is counted: on 2^31 ids a chunk holds 32 words of
+        // a range, and one dependent load after the other took 30 ms.
+        constexpr int WARPS = STBPE_BUILD_THREADS / 32;
+        for (int c0 = warp; c0 < chunks; c0 += 32 * WARPS) {
+            const int c_own = c0 + lane * WARPS, n = min((chunks - c0 + WARPS - 1) / WARPS, 32);
+            unsigned int own_lo = 0, own_hi = 0;
+            i64 own_at = 0;
+            if (c_own < chunks) {
+                const i64 chunk = (i64)p * chunks + c_own;
+                own_lo = offs[chunk * (D + 1) + d], own_hi = offs[chunk * (D + 1) + d + 1];
+                own_at = ((i64)p * pb.n_cta + c_own / chunks_per_region) * pb.cap + (i64)(c_own % chunks_per_region) * STBPE_SUB_CHUNK;
+            }
+            unsigned int next_lo = __shfl_sync(0xFFFFFFFFu, own_lo, 0), next_hi = __shfl_sync(0xFFFFFFFFu, own_hi, 0);
+            const uint32_t *next_w = pb.words + __shfl_sync(0xFFFFFFFFu, own_at, 0);
+            uint32_t first = next_lo + lane < next_hi ? __ldcs(next_w + next_lo + lane) : 0u;
+            for (int j = 0; j < n; ++j) {
+                const unsigned int lo = next_lo, hi = next_hi;
+                const uint32_t *w = next_w;
+                uint32_t x = first;
+                const int nj = j + 1 < n ? j + 1 : j;
+                next_lo = __shfl_sync(0xFFFFFFFFu, own_lo, nj), next_hi = __shfl_sync(0xFFFFFFFFu, own_hi, nj);
+                next_w = pb.words + __shfl_sync(0xFFFFFFFFu, own_at, nj);
+                first = j + 1 < n && next_lo + lane < next_hi ? __ldcs(next_w + next_lo + lane) : 0u;
+                for (unsigned int i = lo + lane; i < hi; i += 32) {
+                    if (i != lo + lane) x = __ldcs(w + i);
+                    unsigned int h = (x >> shift) & (TS - 1);
+                    for (;;) {
+                        uint32_t k = ((volatile uint32_t *)s_word)[h];
+                        if (k == none) {
+                            k = atomicCAS(&s_word[h], none, x);
+                            if (k == none) k = x;
+                        }
+                        if (k == x) {
+                            atomicAdd(&s_num[h], 1u);
+                            break;
+                        }
+                        if (++h == TS) {
+                            const unsigned int j = atomicAdd(n_spill, 1u);
+                            if (j < spill_cap)
+                                spill[j] = x;
+                            else
+                                atomicOr(&e.st->error, STBPE_DERR_DENSE_OVERFLOW);
+                            break;
+                        }
                     }
                 }
             }
