@@ -283,7 +283,7 @@ static const DeviceInfo &device_info(int dev) {
     SMEM(count_dense_kernel<uint32_t>, 32768 * 4);
     SMEM(partition_pairs_kernel<uint16_t>, STBPE_PART_SMEM_BYTES);
     SMEM(partition_pairs_kernel<uint32_t>, STBPE_PART_SMEM_BYTES);
-    SMEM(sub_partition_kernel, STBPE_SUB_CHUNK * sizeof(uint32_t));
+    SMEM(sub_partition_kernel<16384>, 16384 * sizeof(uint32_t));
     SMEM(build_table_kernel, 8 << 14);
     SMEM(presence_rebuild_kernel<uint16_t>, STBPE_PROWS * sizeof(unsigned int));
     SMEM(presence_rebuild_kernel<uint32_t>, STBPE_PROWS * sizeof(unsigned int));
@@ -835,7 +835,8 @@ static int wide_build(stbpe_engine *e, int *ok, cudaStream_t s) {
     int task_bits = lg - STBPE_PART_BITS - 1 < 13 ? lg - STBPE_PART_BITS - 1 : 13;
     if (lg - STBPE_PART_BITS - task_bits > STBPE_SUB_MAX_BITS) task_bits = lg - STBPE_PART_BITS - STBPE_SUB_MAX_BITS;
     const int sub_bits = lg - STBPE_PART_BITS - task_bits;
-    const int cpr = (int)((pb.cap + STBPE_SUB_CHUNK - 1) / STBPE_SUB_CHUNK);
+    const int chunk = sub_bits > 6 ? 16384 : 8192;
+    const int cpr = (int)((pb.cap + chunk - 1) / chunk);
     const i64 n_chunks = (i64)STBPE_PARTS * pb.n_cta * cpr;
     const unsigned int spill_cap = 1u << 20;
     const size_t offs_bytes = ((size_t)n_chunks * ((1 << sub_bits) + 1) * sizeof(uint16_t) + 255) & ~(size_t)255;
@@ -847,8 +848,11 @@ static int wide_build(stbpe_engine *e, int *ok, cudaStream_t s) {
     const size_t build_smem = (size_t)8 << task_bits;
     CK(cudaEventRecord(e->ev0, s));
     CK(cudaMemsetAsync(n_spill, 0, sizeof(*n_spill), s));
-    sub_partition_kernel<<<e->sm_count * 3, STBPE_SUB_THREADS, STBPE_SUB_CHUNK * sizeof(uint32_t), s>>>(pb, cpr, sub_bits, offs);
-    build_table_kernel<<<e->sm_count * (build_smem > 65536 ? 1 : 3), STBPE_BUILD_THREADS, build_smem, s>>>(e->d, pb, cpr, sub_bits, task_bits, offs, spill,
+    if (chunk == 8192)
+        sub_partition_kernel<8192><<<e->sm_count * 3, STBPE_SUB_THREADS, 8192 * sizeof(uint32_t), s>>>(pb, cpr, sub_bits, offs);
+    else
+        sub_partition_kernel<16384><<<e->sm_count * 2, STBPE_SUB_THREADS, 16384 * sizeof(uint32_t), s>>>(pb, cpr, sub_bits, offs);
+    build_table_kernel<<<e->sm_count * (build_smem > 65536 ? 1 : 3), STBPE_BUILD_THREADS, build_smem, s>>>(e->d, pb, chunk, cpr, sub_bits, task_bits, offs, spill,
                                                                                                    n_spill, spill_cap);
     spill_to_table_kernel<<<e->sm_count, 256, 0, s>>>(e->d, spill, n_spill, spill_cap);
     dense_to_table_kernel<false><<<256, 256, 0, s>>>(e->d, e->wide_dense);

@@ -202,23 +202,26 @@ __device__ __forceinline__ void part_word_to_table(const EngineDev &e, uint32_t 
     table_count_n(e, key, slot_of_word(e, x), n, fresh);
 }
 
-// pass 2, one rank: the words of every chunk (a piece of a pass-1 region of at most STBPE_SUB_CHUNK words) in
+// pass 2, one rank: the words of every chunk (a piece of a pass-1 region of at most CHUNK words) in
 // order of their next `sub_bits` bits, in place; offs[chunk][d] = where the words of digit d start.
 // One returning shared-memory atomic per word gives its rank inside its digit, the words wait in registers
 // meanwhile and go back through shared memory in order.
 #define STBPE_SUB_THREADS 512
-#define STBPE_SUB_CHUNK 8192
 #define STBPE_SUB_MAX_BITS 8
-__global__ void __launch_bounds__(STBPE_SUB_THREADS, 3) sub_partition_kernel(PartBuffers pb, int chunks_per_region, int sub_bits, uint16_t *__restrict__ offs) {
-    extern __shared__ __align__(16) uint32_t s_out[];  // STBPE_SUB_CHUNK words
+// CHUNK: 8192 words, 16 registers of them per thread and three CTAs per SM; 16 384 where the table has so many ranges
+// that a piece of 8192 words would leave less than one full load per range (more than six bits; 2^31 ids: 17.7 instead of
+// 20.4 ms for this and the next pass, but 1.86 instead of 1.56 ms on 200 M ids).
+template <int CHUNK>
+__global__ void __launch_bounds__(STBPE_SUB_THREADS, CHUNK > 8192 ? 2 : 3) sub_partition_kernel(PartBuffers pb, int chunks_per_region, int sub_bits, uint16_t *__restrict__ offs) {
+    extern __shared__ __align__(16) uint32_t s_out[];  // CHUNK words
     __shared__ unsigned int s_cnt[1 << STBPE_SUB_MAX_BITS], s_base[(1 << STBPE_SUB_MAX_BITS) + 1];
-    constexpr int PER = STBPE_SUB_CHUNK / STBPE_SUB_THREADS;
+    constexpr int PER = CHUNK / STBPE_SUB_THREADS;
     const int D = 1 << sub_bits, lane = threadIdx.x & 31;
     const i64 n_chunks = (i64)STBPE_PARTS * pb.n_cta * chunks_per_region;
     for (i64 chunk = blockIdx.x; chunk < n_chunks; chunk += gridDim.x) {
-        const i64 region = chunk / chunks_per_region, first = (chunk - region * chunks_per_region) * STBPE_SUB_CHUNK;
+        const i64 region = chunk / chunks_per_region, first = (chunk - region * chunks_per_region) * CHUNK;
         const i64 left = (i64)pb.fill[region] - first;
-        const int n = left <= 0 ? 0 : (left < STBPE_SUB_CHUNK ? (int)left : STBPE_SUB_CHUNK);
+        const int n = left <= 0 ? 0 : (left < CHUNK ? (int)left : CHUNK);
         uint32_t *w = pb.words + region * pb.cap + first;
         for (int i = threadIdx.x; i < D; i += STBPE_SUB_THREADS) s_cnt[i] = 0u;
         __syncthreads();
@@ -269,7 +272,7 @@ __global__ void __launch_bounds__(STBPE_SUB_THREADS, 3) sub_partition_kernel(Par
 // lines, nothing is cleared before and no atomic reaches L2.  A word whose probe runs over the end of the range
 // goes to the spill list, which is added to the finished table.
 #define STBPE_BUILD_THREADS 512
-__global__ void __launch_bounds__(STBPE_BUILD_THREADS, 3) build_table_kernel(EngineDev e, PartBuffers pb, int chunks_per_region, int sub_bits, int task_bits,
+__global__ void __launch_bounds__(STBPE_BUILD_THREADS, 3) build_table_kernel(EngineDev e, PartBuffers pb, int chunk_words, int chunks_per_region, int sub_bits, int task_bits,
                                                                           const uint16_t *__restrict__ offs, uint32_t *spill, unsigned int *n_spill,
                                                                           unsigned int spill_cap) {
     extern __shared__ __align__(16) uint32_t s_word[];
@@ -295,7 +298,7 @@ __global__ void __launch_bounds__(STBPE_BUILD_THREADS, 3) build_table_kernel(Eng
             if (c_own < chunks) {
                 const i64 chunk = (i64)p * chunks + c_own;
                 own_lo = offs[chunk * (D + 1) + d], own_hi = offs[chunk * (D + 1) + d + 1];
-                own_at = ((i64)p * pb.n_cta + c_own / chunks_per_region) * pb.cap + (i64)(c_own % chunks_per_region) * STBPE_SUB_CHUNK;
+                own_at = ((i64)p * pb.n_cta + c_own / chunks_per_region) * pb.cap + (i64)(c_own % chunks_per_region) * chunk_words;
             }
             unsigned int next_lo = __shfl_sync(0xFFFFFFFFu, own_lo, 0), next_hi = __shfl_sync(0xFFFFFFFFu, own_hi, 0);
             const uint32_t *next_w = pb.words + __shfl_sync(0xFFFFFFFFu, own_at, 0);
