@@ -90,44 +90,66 @@ def _flatten_batch(batch) -> Tuple[torch.Tensor, np.ndarray]:
     return ids, off
 
 
+class _HostRows:
+    """Rows of padded host batches one behind the other, as bytes while every id is below 256 and as int32 from the
+    first larger one on.  A batch is copied when it is added: loaders yield views of buffers that they refill
+    (``gpu_tokenizer/datasets.py:58-92``), so none of a batch is looked at again once the next one is asked for."""
+
+    def __init__(self, cells: int):
+        # room for some more batches like the first: pages that nothing has been written to take no memory
+        self.ids = torch.empty(max(cells, min(8 * cells, 1 << 26)), dtype=torch.uint8)
+        self.n = 0
+        self.lengths: List[np.ndarray] = [np.zeros(1, dtype=np.int64)]
+
+    def add(self, tokens: torch.Tensor, valid: torch.Tensor) -> None:
+        if self.n + tokens.numel() > self.ids.numel():
+            self._move(2 * self.ids.numel() + tokens.numel(), self.ids.dtype)
+        tokens, valid = tokens.contiguous(), valid.contiguous()
+        lens = np.empty(tokens.shape[0], dtype=np.int64)
+        rc = self._flatten(tokens, valid, lens)
+        if rc == L.E_ID_OVERFLOW and self.ids.dtype == torch.uint8:
+            self._move(self.ids.numel(), torch.int32)
+            rc = self._flatten(tokens, valid, lens)
+        if rc == L.E_STATE:
+            raise ValueError("valid must mark a prefix of every row")
+        if rc != L.OK:
+            raise RuntimeError(f"stbpe_flatten_rows returned {rc}")
+        self.n += int(lens.sum())
+        self.lengths.append(lens)
+
+    def _flatten(self, tokens, valid, lens) -> int:
+        return L.load().stbpe_flatten_rows(tokens.data_ptr(), valid.data_ptr(), tokens.shape[0], tokens.shape[1],
+                                           self.ids.element_size(), self.ids.data_ptr() + self.n * self.ids.element_size(),
+                                           lens.ctypes.data)
+
+    def _move(self, cells: int, dtype: torch.dtype) -> None:
+        ids = torch.empty(cells, dtype=dtype)
+        ids[:self.n] = self.ids[:self.n]
+        self.ids = ids
+
+    def rows(self) -> Tuple[torch.Tensor, np.ndarray]:
+        return self.ids[:self.n], np.cumsum(np.concatenate(self.lengths))
+
+
 def _flatten_batches(batches) -> List[Tuple[torch.Tensor, np.ndarray]]:
-    """Flat ids (uint8 while every id is below 256, else int32) and row offsets: host batches of the usual types
-    through the native pass into one piece, any other batch by ``_flatten_batch`` into a piece of its own."""
+    """Flat ids (uint8 while every id is below 256, else int32) and row offsets: consecutive host batches of the usual
+    types through the native pass into one piece, any other batch by ``_flatten_batch`` into a piece of its own."""
     out: List[Tuple[torch.Tensor, np.ndarray]] = []
-    host: list = []
-
-    def flush():
-        if not host:
-            return
-        room = sum(t.numel() for t, _ in host)
-        lens = np.empty(sum(t.shape[0] for t, _ in host) + 1, dtype=np.int64)
-        lens[0] = 0
-        for dtype in (torch.uint8, torch.int32):
-            ids = torch.empty(room, dtype=dtype)
-            rows = n = 0
-            for t, v in host:
-                part = lens[1 + rows:1 + rows + t.shape[0]]
-                rc = L.load().stbpe_flatten_rows(t.data_ptr(), v.data_ptr(), t.shape[0], t.shape[1], ids.element_size(),
-                                                 ids.data_ptr() + n * ids.element_size(), part.ctypes.data)
-                if rc != 0:
-                    break
-                rows, n = rows + t.shape[0], n + int(part.sum())
-            if rc == 0:
-                break
-            if rc == L.E_STATE:
-                raise ValueError("valid must mark a prefix of every row")
-        host.clear()
-        out.append((ids[:n], np.cumsum(lens)))
-
+    host: Optional[_HostRows] = None
     for b in batches:
         t, v = b[0], b[1]
         if t.dim() == 2 and v.shape == t.shape and not t.is_cuda and not v.is_cuda and t.dtype == torch.int32 and \
                 v.dtype in (torch.uint8, torch.bool):
-            host.append((t.contiguous(), v.contiguous()))
+            if host is None:
+                host = _HostRows(t.numel())
+            host.add(t, v)
         else:
-            flush()
+            if host is not None:
+                out.append(host.rows())
+                host = None
             out.append(_flatten_batch(b))
-    flush()
+    if host is not None:
+        out.append(host.rows())
     return out
 
 
@@ -237,14 +259,19 @@ class GPUBPETrainer(BaseTrainer):
                  "histogram_size": 0, "source": "ngram"}
         if top_k is None or top_k <= 0:
             return empty
-        flat = [_flatten_batch(b) for b in batches]
+        return cls._plan_from_rows([_flatten_batch(b) for b in batches], top_k, device)
+
+    @staticmethod
+    def _plan_from_rows(flat, top_k: int, device) -> dict:
+        empty = {"merges": [], "counts": [], "top_k": 0, "requested_top_k": int(top_k or 0), "order": 2,
+                 "histogram_size": 0, "source": "ngram"}
         total = sum(int(ids.numel()) for ids, _ in flat)
         eng = Engine(max(total, 1), base_vocab=0, max_merges=1,
                      device=torch.device(device) if device is not None else None)
         try:
             for ids, off in flat:
                 if ids.numel():
-                    eng.append_ids(ids, off)
+                    (eng.append_bytes if ids.dtype == torch.uint8 else eng.append_ids)(ids, off)
             eng.count_initial()
             keys, counts = eng.export_histogram()
         finally:
@@ -293,11 +320,15 @@ class GPUBPETrainer(BaseTrainer):
             warm_start_merges = list(self.merges)
         elif warm_start_merges is None and warm_start_plan is not None:
             warm_start_merges = [tuple(p) for p in warm_start_plan.get("merges", [])]
-        elif warm_start_merges is None and warm_start_ngrams:
-            batches = list(batches)
-            plan = self.precompute_warm_start_plan(batches, int(warm_start_ngrams), device=warm_start_device or self.device)
-            warm_start_merges = plan["merges"]
         t0 = time.perf_counter()
+        flat = None
+        if resume_state is None and warm_start_merges is None and warm_start_plan is None and warm_start_ngrams:
+            # the batches are needed twice but may be looked at only as they come
+            flat = _flatten_batches(batches)
+            if int(warm_start_ngrams) > 0:
+                warm_start_merges = self._plan_from_rows(flat, int(warm_start_ngrams), warm_start_device or self.device)["merges"]
+            else:
+                warm_start_merges = []
         if restored_rows is not None:
             if self._sharded_mode() is not None:
                 self._reject_in_sharded_mode(warm_start_merges, checkpoint_interval)
@@ -313,10 +344,11 @@ class GPUBPETrainer(BaseTrainer):
                                   already=list(self.merges), dataset_state=dataset_state)
         mode = self._sharded_mode()
         if mode is not None:
-            flat = [_flatten_batch(b) for b in batches]
+            flat = [_flatten_batch(b) for b in batches] if flat is None else [(ids.to(torch.int32), off) for ids, off in flat]
             self._reject_in_sharded_mode(warm_start_merges, checkpoint_interval)
             return self._fit_sharded(mode, flat, False, log_every, t0)
-        flat = _flatten_batches(batches)
+        if flat is None:
+            flat = _flatten_batches(batches)
         total = sum(int(ids.numel()) for ids, _ in flat)
         eng = self._make_engine(total)
         for ids, off in flat:

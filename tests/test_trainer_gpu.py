@@ -162,6 +162,28 @@ def test_resume_equals_uninterrupted_run_and_warm_start_plan(tmp_path):
     assert plan["merges"][0] == full.merges[0]
 
 
+@pytest.mark.parametrize("ngrams", [None, 5])
+def test_loader_that_refills_its_buffers(ngrams):
+    # the batches are views of one buffer: what a run learns is what it learns from independent batches
+    c = synth.config2_mixed(1 << 17, seed=6, lexicon=900, mean_doc_bytes=300)
+    rows = [r.tolist() for r in corpus_rows(c)]
+    batches = [make_batch(rows[i:i + 40]) for i in range(0, len(rows), 40)]
+    room = [torch.empty(max(b[k].numel() for b in batches), dtype=batches[0][k].dtype) for k in range(3)]
+
+    def loader():
+        for b in batches:
+            for buf, x in zip(room, b):
+                buf[:x.numel()] = x.reshape(-1)
+            yield tuple(buf[:x.numel()].reshape(x.shape) for buf, x in zip(room, b))
+
+    runs = []
+    for data in (loader(), batches):
+        t = GPUBPETrainer(merges=40, device="cuda")
+        t.fit(data, log_every=0, warm_start_ngrams=ngrams)
+        runs.append((t.merges, t.merge_counts))
+    assert len(batches) > 2 and runs[0] == runs[1]
+
+
 def test_cli_train_bpe(tmp_path):
     from supertoken_b200 import cli
     c = synth.config1_text(1 << 16, seed=2, file_bytes=1 << 13)
