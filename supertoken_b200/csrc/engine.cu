@@ -86,6 +86,7 @@ struct stbpe_engine {
     bool cand_stale;      // the candidate list is used up: collect one before the next choice
     bool foreign_ids;     // a merge of the caller's may have brought an id of 65 536 or more
     unsigned int max_id;  // largest id appended through stbpe_append_ids
+    i64 bytes_below, made_below;  // the stream's bytes, and the ids that merges have brought, lie below these
     unsigned int load_err;  // error bits of the rows appended so far
     bool merges_known;    // merges_done mirrors the device (several host-driven merges in a row)
     int merges_done;
@@ -207,6 +208,11 @@ static bool starts_wide(const stbpe_config &c) {
     return last >= (i64)Tok<uint16_t>::IDMASK;
 }
 static size_t tok_bytes(const stbpe_engine *e) { return e->wide ? 4 : 2; }
+
+// Every id of the stream lies below this.
+static i64 ids_below(const stbpe_engine *e) {
+    return std::max({e->bytes_below, e->made_below, e->only_bytes ? (i64)0 : (i64)e->max_id + 1});
+}
 
 // log2 of the tiles a CTA takes together from the pair filter: eight once every CTA gets several units, fewer on
 // smaller streams, so that the visited tiles spread over all CTAs.  (Whole words of the filter, 32 tiles, are fewer
@@ -333,6 +339,7 @@ static void drop_stream(stbpe_engine *e) {
     e->filter_valid = false;
     e->wide_counted = e->full_refresh_pending = false;
     e->load_err = e->max_id = 0;
+    e->bytes_below = e->made_below = 0;
     e->merges_known = e->foreign_ids = false;
     e->state_stale = true;
 }
@@ -584,7 +591,10 @@ static int append_common(stbpe_engine *e, const void *data, i64 n, size_t elem, 
     e->n_tokens += n;
     e->recs_stale = true;
     e->counted = false;
-    if (elem != 1) e->only_bytes = false;
+    if (elem == 1)
+        e->bytes_below = 256;
+    else
+        e->only_bytes = false;
     return STBPE_OK;
 }
 
@@ -895,10 +905,11 @@ static int launch_count(stbpe_engine *e, bool mg, cudaStream_t s) {
         CK(cudaGetLastError());
         CK(cudaEventRecord(e->ev1, s));
         e->count_timed = true;
-        unsigned int *derr = (unsigned int *)e->pinned.p;
-        CK(cudaMemcpyAsync(derr, &e->d.st->error, sizeof(*derr), cudaMemcpyDeviceToHost, s));
+        unsigned int *derr = (unsigned int *)e->pinned.p;  // error bits and the largest id behind them
+        CK(cudaMemcpyAsync(derr, &e->d.st->error, 2 * sizeof(*derr), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         if (!(*derr & STBPE_DERR_DENSE_OVERFLOW)) {
+            if (!mg) e->bytes_below = (i64)derr[1] + 1;
             if (mg) dense_to_table_kernel<true><<<256, 256, 0, s>>>(e->d, e->dense);
             CK(cudaGetLastError());
             return STBPE_OK;
@@ -1302,7 +1313,7 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
         la.filter_count = fc >= 9e18 ? (i64)9000000000000000000ll : (i64)fc;
         la.repack_tiles = 64;
         la.grow_keys = e->table_auto ? (i64)(e->slots / 4) : (i64)0x7FFFFFFFFFFFFFFFll;
-        la.ids_below = e->only_bytes ? 256 : (int)e->max_id + 1;
+        la.ids_below = (int)std::min(ids_below(e), (i64)0x7FFFFFFF);
         la.unit_shift = unit_shift(e, grid);
         EngineDev d = e->d;
         // Candidates that have run out are collected in front of the launch without waiting for the result: one pass
@@ -1328,6 +1339,7 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
         }
         if (int rc_ = read_state(e, out, s)) return rc_;
         at += out->forced_done;
+        e->made_below = std::max(e->made_below, mode == LOOP_BEST ? (i64)e->cfg.base_vocab + out->merges_done : (i64)forced_new + at);
         if (n_done) *n_done = at;
         int rc = check_error_bits(e, out->error);
         if (rc != STBPE_OK) {
@@ -1411,6 +1423,7 @@ STBPE_VISIBLE int stbpe_train_timed(stbpe_engine *e, int32_t n_merges, float *ke
     if (int rc_ = read_state(e, &h, s)) return rc_;
     i64 target = (i64)h.merges_done + n_merges;
     if (target > e->cfg.max_merges) target = e->cfg.max_merges;
+    e->made_below = std::max(e->made_below, (i64)e->cfg.base_vocab + target);
     set_target_kernel<<<1, 1, 0, s>>>(e->d, (int)target);
     CK(cudaGetLastError());
     const int todo = (int)(target - h.merges_done);

@@ -246,13 +246,14 @@ __global__ void rehash_kernel(EngineDev e, const Slot *__restrict__ old, u64 n) 
 
 #include "wide_count.cuh"
 
-// dense 16-bit keys -> entries of the pair table (or of the rank-local delta table)
+// dense 16-bit keys -> entries of the pair table (or of the rank-local delta table), and the largest id of a pair
 template <bool MG>
-__global__ void dense_to_table_kernel(EngineDev e, const u64 *g_dense) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= 65536) return;
+__global__ void __launch_bounds__(256) dense_to_table_kernel(EngineDev e, const u64 *g_dense) {
+    const int k = blockIdx.x * 256 + threadIdx.x;  // 256 CTAs: every counter has its thread
     const u64 c = g_dense[k];
     if (c) sink_add<MG>(e, ((u64)(k >> 8) << 32) | (u64)(k & 0xFF), (i64)c);
+    const unsigned int largest = __reduce_max_sync(0xFFFFFFFFu, c ? (unsigned int)max(k >> 8, k & 0xFF) : 0u);
+    if ((threadIdx.x & 31) == 0 && largest) atomicMax(&e.st->max_id, largest);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -15,12 +15,17 @@
 // read the counts that chose merge m; that wait runs under the rewriting of the tiles.
 //
 // A step takes several merges.  Let p1, p2, ... = (a1, b1), (a2, b2), ... be the pairs in selection order (larger count,
-// then smaller key), and let no ai be a bj with i != j (of a pair of equal tokens no token may occur elsewhere).  Then
-// an occurrence of pj overlaps no match of the others, so merging them leaves its count as it is.  They make or raise
+// then smaller key), let no ai be a bj with i != j (of a pair of equal tokens no token may occur elsewhere), and let every
+// id of the stream be smaller than the new ones.  Then an occurrence of pj overlaps no match of the others, so merging
+// them leaves its count as it is.  They make
 // only pairs with one of their new tokens; such a pair (x, new i) occurs at most as often as (x, ai) did, and (x, ai),
 // which is none of p1 .. pj, came after pj; where the counts are equal the larger key, new > every token of pj,
 // loses (and the same for (new i, y) and (bi, y)).  So pj is the best pair after p1 .. pj-1, exactly as if the
 // counts had been taken after each merge, and p1 .. pj are applied at once.
+// (A new id that the stream holds already may lift a pair that was there: with base_vocab 5 and rows 50 x 012, 50 x 01,
+// 60 x 34, 40 x 52 the merge (0,1) -> 5 takes (5,2) from 40 to 90, past (3,4).  Ids at or above base_vocab come from the
+// caller: streams with marker ids, merges with ids of their own.  Such merges go one by one until the new ids
+// have passed them; the host keeps the bound, LoopArgs::ids_below.)
 // The batch ends at the first pair that breaks the rule, at Batch<T>::MAX, and wherever a stop rule or
 // maintenance has to be decided first.  On text a batch is 4.7 merges on average (3.9 while no token was to be
 // shared at all): the grid barrier, the choice and the flush of the deltas, some 9 of the 12 us of a sparse merge,
@@ -47,7 +52,7 @@ struct LoopArgs {
     int repack_tiles;       // leave for a re-pack at three quarters live from this many tiles on
     int unit_shift;         // tiles per filter unit, log2 (cta_merge)
     i64 grow_keys;          // leave for a larger pair table when a merge could take the number of keys beyond this ...
-    int ids_below;          // ... given that the stream's own ids lie below this
+    int ids_below;          // every id of the stream lies below this (those of the launch's own merges apart)
 };
 
 enum { LOOP_BEST, LOOP_NONE, LOOP_UNTIED };
@@ -287,12 +292,13 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             const i64 live = s_live - before;
             // every merge makes at most two pairs per match and two per id
             const i64 ids = max((int)nw, la.ids_below), made = min(before + count, ids * (j + 1));
-            // a later member: the order is exact so far, no token is second in one pair and first in another, none is one of
-            // the members' new ones (a pair that the host gives may name one, or be given twice)
+            // a later member: the order is exact so far (which takes new ids above all of the stream), no token is second in
+            // one pair and first in another, none is one of the members' new ones (a pair that the host gives, in whatever
+            // order, may name one, or be given twice)
             bool out = false;
             if constexpr (KB > 1) {
                 const uint32_t same = __match_any_sync(0xFFFFFFFFu, lane >= 2 * KB ? 0x80000000u | lane : lane & 1 ? b : a);
-                out = out || (!host && !(mine > bound)) || max(a, b) >= nw0 || (same & ((1u << (lane & ~1)) - 1u) & (lane & 1 ? 0x5555u : 0xAAAAu));
+                out = out || (!host && (!(mine > bound) || nw0 < (uint32_t)la.ids_below)) || max(a, b) >= nw0 || (same & ((1u << (lane & ~1)) - 1u) & (lane & 1 ? 0x5555u : 0xAAAAu));
                 if (host) {
                     const uint32_t twice = __match_any_sync(0xFFFFFFFFu, lane >= 2 * KB ? 0x80000000u | lane : (a << 15) | b);
                     out = out || (twice & ((1u << (lane & ~1)) - 1u));

@@ -102,6 +102,102 @@ def test_merges_given_by_the_host(n):
     e.close()
 
 
+def _apply_checked(e, ids, off, merges, first):
+    for i, (a, b) in enumerate(merges):
+        O.apply_merge_flat(ids, off, a, b, first + i)
+    gi, _ = e.export_stream()
+    assert np.array_equal(gi, ids[:off[-1]])
+    _check_histogram(e, ids[:off[-1]].copy(), off)
+
+
+OVERTAKEN = [[0, 1, 2]] * 50 + [[0, 1]] * 50 + [[3, 4]] * 60 + [[5, 2]] * 40  # (0,1) -> 5 takes (5,2) past (3,4)
+
+
+@pytest.mark.parametrize("as_bytes", [False, True])
+@pytest.mark.parametrize("base_vocab", [5, 6])
+def test_merge_that_lifts_a_pair_with_an_id_of_the_stream(as_bytes, base_vocab):
+    ids, off = O.flatten_rows(OVERTAKEN)
+    e = Engine(len(ids), base_vocab=base_vocab, max_merges=3)
+    e.append_bytes(ids.astype(np.uint8), off) if as_bytes else e.append_ids(ids, off)
+    e.count_initial()
+    e.train(3)
+    assert (e.merges()[0][1] == (5, 2)) == (base_vocab == 5)
+    _check(e, ids, off, base_vocab, 3)
+    e.close()
+
+
+@pytest.mark.parametrize("seed", range(8))
+def test_new_ids_that_occur_in_the_stream(seed):
+    # bytes and ids at and above base_vocab: the first new ids are among them, the later ones are not
+    rng = np.random.RandomState(seed)
+    top = (14, 40, 200, 256, 300)[seed % 5]
+    ids = rng.choice(top, 12000, p=rng.dirichlet(np.full(top, 0.3))).astype(np.int32)
+    off = _rows(ids, rng, 60)
+    base = int(rng.randint(3, top))
+    e = Engine(len(ids), base_vocab=base, max_merges=60, table_slots=1 << 18)
+    half = int(off[len(off) // 2])
+    if top <= 256 and seed % 2:
+        e.append_bytes(ids.astype(np.uint8), off)
+    elif top <= 256 and seed % 4 == 0:  # bytes, counted, then ids
+        e.append_bytes(ids[:half].astype(np.uint8), off[:len(off) // 2 + 1])
+        e.count_initial()
+        e.append_ids(ids[half:].copy(), off[len(off) // 2:] - half)
+    else:
+        e.append_ids(ids, off)
+    e.count_initial()
+    for n in (7, 53):
+        e.train(n)
+    _check(e, ids, off, base, 60)
+    e.close()
+
+
+def test_best_pairs_after_merges_that_the_host_numbers():
+    # the host's new ids lie above, among and below those of the loop, which must not take them for unused
+    ids, off = O.flatten_rows([[0, 1, 2]] * 50 + [[0, 1]] * 50 + [[3, 4]] * 60 + [[7, 8, 2]] * 40)
+    e = _engine(ids, off, 4, 8)
+    e.apply_merge(7, 8, 5)  # the stream's (5,2) has 40, as in OVERTAKEN
+    ids2, off2 = ids.copy(), off.copy()
+    O.apply_merge_flat(ids2, off2, 7, 8, 5)
+    om, oc, _ = O.train_flat(ids2[:off2[-1]].copy(), off2, 5, 7, 1)  # merge 1 of the log gets id 5
+    e.train(7)
+    got, counts, _ = e.merges()
+    assert got[1:] == om and counts.tolist()[1:] == oc and (5, 2) in om[:2]
+    _apply_checked(e, ids2, off2, om, 5)
+    e.close()
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_untied_runs_with_ids_of_the_stream(seed):
+    # pairs that are lifted again and again by merges into ids that were there before, then runs with unused ids
+    rng = np.random.RandomState(seed)
+    ids = rng.choice(10, 6000, p=rng.dirichlet(np.ones(10))).astype(np.int32)
+    off = _rows(ids, rng, 50)
+    e = _engine(ids, off, 6, 60)
+    ids2, off2 = ids.copy(), off.copy()
+    made, drawn, new = [], None, 6
+    for _ in range(6):
+        a, b = (int(x) for x in rng.randint(0, 10, 2))
+        e.apply_merge(a, b, 3)
+        O.apply_merge_flat(ids2, off2, a, b, 3)
+        made.append((a, b))
+    for most in (0, 2, 9, 9, 9):
+        done, count, tied = e.next_tied(drawn, new, most)
+        for j in range(done):
+            k, c = O.count_pairs_flat(ids2[:off2[-1]].copy(), off2, 1)
+            best = np.sort(k[c == c.max()])
+            pair = drawn if drawn is not None and j == 0 else (int(best[0]) >> 32, int(best[0]) & 0xFFFFFFFF)
+            assert (drawn is not None and j == 0) or len(best) == 1
+            O.apply_merge_flat(ids2, off2, *pair, new + j)
+            made.append(pair)
+        k, c = O.count_pairs_flat(ids2[:off2[-1]].copy(), off2, 1)
+        assert count == c.max() and tied == np.sort(k[c == c.max()]).tolist()
+        drawn = (tied[-1] >> 32, tied[-1] & 0xFFFFFFFF)
+        new = new + done if most < 9 else 20 + len(made)
+    assert e.merges()[0] == made
+    _apply_checked(e, ids2, off2, [], 0)
+    e.close()
+
+
 @pytest.mark.parametrize("most", [0, 3, 50])
 def test_ties_are_left_to_the_host(most):
     rng = np.random.RandomState(5)
