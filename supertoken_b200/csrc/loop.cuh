@@ -308,12 +308,14 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             int stop = 0, why = STBPE_EXIT_STOP;
             bool go = false;
             // LOOP_UNTIED: alone with its count, among the candidates and among the pairs that are not listed.  (The pairs
-            // that the merges before it make are rarer than some pair after it, hence rarer than it.)
+            // that the merges before it make are rarer than some pair after it, hence rarer than it.)  A slot that is listed
+            // twice, as one can be whose pair a merge has lifted again with an id that was there before, takes one place and
+            // leaves a gap behind it: then, too, the host looks.
             bool tied = true;
             if constexpr (KB > 1) {
                 if (la.mode == LOOP_UNTIED) {
                     const Slot after = Bs::slot(max(s_sorted[j + 1], bound));
-                    tied = count <= after.count || count <= mc.theta.count || count < 2 || merges_done + j >= la.target;
+                    tied = !s_sorted[j + 1] || count <= after.count || count <= mc.theta.count || count < 2 || merges_done + j >= la.target;
                 }
             }
             if (err & 0x7FFFFFFFu) stop = 4;

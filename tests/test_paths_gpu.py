@@ -166,6 +166,19 @@ def test_best_pairs_after_merges_that_the_host_numbers():
     e.close()
 
 
+@pytest.mark.parametrize("new_id", [8, 20])
+def test_tie_with_a_pair_that_was_lifted_again(new_id):
+    # (5,2) falls to nothing and comes back, so the candidate list, which holds every pair here, names it twice and far
+    # apart; (10,11) has as many
+    ids, off = O.flatten_rows([[5, 2]] * 10 + [[7, 8, 2]] * 60 + [[10, 11]] * 60 + [[12, 13]] * 90 +
+                              [[i, i + 1] for i in range(100, 1300, 2)] * 2)
+    e = _engine(ids, off, 16, 8)
+    e.apply_merge(5, 2, 9)
+    e.apply_merge(7, 8, 5)
+    assert e.next_tied(None, new_id, 5) == (1, 60, [5 << 32 | 2, 10 << 32 | 11])  # (12,13) is alone with its count
+    e.close()
+
+
 @pytest.mark.parametrize("seed", range(6))
 def test_untied_runs_with_ids_of_the_stream(seed):
     # pairs that are lifted again and again by merges into ids that were there before, then runs with unused ids
