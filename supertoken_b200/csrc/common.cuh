@@ -78,7 +78,7 @@ struct DevState {
     int pad0;
     u64 n_keys;
     i64 n_live;
-    i64 n_matches;
+    i64 n_matches;             // of the last host-given merges (a launch that takes any starts at zero)
     u64 peek_key;
     i64 peek_count;
     i64 peek_ties;

@@ -211,6 +211,24 @@ def test_untied_runs_with_ids_of_the_stream(seed):
     e.close()
 
 
+def test_matches_reported_for_each_host_given_merge():
+    # whatever ran before: the matches of this merge alone
+    rng = np.random.RandomState(2)
+    ids = rng.randint(0, 9, 30000).astype(np.int32)
+    off = _rows(ids, rng, 400)
+    e = _engine(ids, off, 16, 30)
+    ids2, off2 = ids.copy(), off.copy()
+    for n in (0, 3, 1, 0, 6):
+        e.train(n)
+        for i, (a, b) in enumerate(e.merges()[0][len(e.merges()[0]) - n:] if n else []):
+            O.apply_merge_flat(ids2, off2, a, b, e.state().merges_done + 16 - n + i)
+        a, b = (int(x) for x in rng.randint(0, 9, 2))
+        live = int(off2[-1])
+        O.apply_merge_flat(ids2, off2, a, b, 16 + e.state().merges_done)
+        assert e.apply_merge(a, b, 16 + e.state().merges_done) == live - int(off2[-1])
+    e.close()
+
+
 @pytest.mark.parametrize("most", [0, 3, 50])
 def test_ties_are_left_to_the_host(most):
     rng = np.random.RandomState(5)
