@@ -217,9 +217,11 @@ __global__ void __launch_bounds__(STBPE_SUB_THREADS, CHUNK > 8192 ? 2 : 3) sub_p
     __shared__ unsigned int s_cnt[1 << STBPE_SUB_MAX_BITS], s_base[(1 << STBPE_SUB_MAX_BITS) + 1];
     constexpr int PER = CHUNK / STBPE_SUB_THREADS;
     const int D = 1 << sub_bits, lane = threadIdx.x & 31;
-    const i64 n_chunks = (i64)STBPE_PARTS * pb.n_cta * chunks_per_region;
-    for (i64 chunk = blockIdx.x; chunk < n_chunks; chunk += gridDim.x) {
-        const i64 region = chunk / chunks_per_region, first = (chunk - region * chunks_per_region) * CHUNK;
+    // All regions' first pieces, then all second ones: the later pieces of a region, which has room for every token of its
+    // share, are mostly empty, and would otherwise fall to the same CTAs (1.7 x 10^9 ids, four pieces: 23.5 ms, now 21.3).
+    const i64 n_regions = (i64)STBPE_PARTS * pb.n_cta;
+    for (i64 j = blockIdx.x; j < n_regions * chunks_per_region; j += gridDim.x) {
+        const i64 piece = j / n_regions, region = j - piece * n_regions, chunk = region * chunks_per_region + piece, first = piece * CHUNK;
         const i64 left = (i64)pb.fill[region] - first;
         const int n = left <= 0 ? 0 : (left < CHUNK ? (int)left : CHUNK);
         uint32_t *w = pb.words + region * pb.cap + first;
@@ -287,7 +289,7 @@ __global__ void __launch_bounds__(STBPE_BUILD_THREADS, 3) build_table_kernel(Eng
         __syncthreads();
         const int p = task >> sub_bits, d = task & (D - 1);
         const int chunks = pb.n_cta * chunks_per_region;
-        // A warp takes every sixteenth chunk.  Where a chunk's words are, each lane reads for another chunk, and the
+        // A warp takes every sixteenth chunk, again first pieces before second ones (29.9 -> 23.5 ms on 1.7 x 10^9 ids).  Where a chunk's words are, each lane reads for another chunk, and the
         // next chunk's first words are on their way while one is counted: on 2^31 ids a chunk holds 32 words of
         // a range, and one dependent load after the other took 30 ms.
         constexpr int WARPS = STBPE_BUILD_THREADS / 32;
@@ -296,9 +298,9 @@ __global__ void __launch_bounds__(STBPE_BUILD_THREADS, 3) build_table_kernel(Eng
             unsigned int own_lo = 0, own_hi = 0;
             i64 own_at = 0;
             if (c_own < chunks) {
-                const i64 chunk = (i64)p * chunks + c_own;
+                const i64 piece = c_own / pb.n_cta, region = (i64)p * pb.n_cta + c_own - piece * pb.n_cta, chunk = region * chunks_per_region + piece;
                 own_lo = offs[chunk * (D + 1) + d], own_hi = offs[chunk * (D + 1) + d + 1];
-                own_at = ((i64)p * pb.n_cta + c_own / chunks_per_region) * pb.cap + (i64)(c_own % chunks_per_region) * chunk_words;
+                own_at = region * pb.cap + piece * chunk_words;
             }
             unsigned int next_lo = __shfl_sync(0xFFFFFFFFu, own_lo, 0), next_hi = __shfl_sync(0xFFFFFFFFu, own_hi, 0);
             const uint32_t *next_w = pb.words + __shfl_sync(0xFFFFFFFFu, own_at, 0);

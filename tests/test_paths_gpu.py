@@ -279,6 +279,21 @@ def test_partitioned_count_builds_tables_of_any_size(slots, n, monkeypatch):
     e.close()
 
 
+@pytest.mark.parametrize("slots,max_tokens,batches", [(1 << 18, 3 * 10**8, 2), (1 << 28, 10**9, 4)])
+def test_partitioned_count_with_several_pieces_per_region(slots, max_tokens, batches, monkeypatch):
+    # four pairs only, so that regions fill beyond a piece (8 192 or 16 384 words; about 0.3 of a CTA's 16 384 tokens a batch)
+    monkeypatch.setenv("STBPE_DENSE32_MIN_TOKENS", "1")
+    n = torch.cuda.get_device_properties(0).multi_processor_count * 16384 * batches
+    ids = np.random.RandomState(batches).choice([300, 301], n, p=[0.55, 0.45]).astype(np.int32)
+    off = np.arange(0, n + 1, n // 8, dtype=np.int64)
+    e = Engine(max_tokens, base_vocab=512, max_merges=1, table_slots=slots)
+    e.append_ids(ids, off)
+    e.count_initial()
+    assert e.state().count_convert_ms > 0
+    _check_histogram(e, ids, off)
+    e.close()
+
+
 def test_pair_table_grows_in_mid_run():
     # random bytes: every merge makes some hundred pairs that were not there before
     n = 16 << 20
