@@ -290,7 +290,7 @@ static const DeviceInfo &device_info(int dev) {
     SMEM(partition_pairs_kernel<uint16_t>, STBPE_PART_SMEM_BYTES);
     SMEM(partition_pairs_kernel<uint32_t>, STBPE_PART_SMEM_BYTES);
     SMEM(sub_partition_kernel<16384>, 16384 * sizeof(uint32_t));
-    SMEM(build_table_kernel, 8 << 14);
+    SMEM(build_table_kernel, 8 << 13);
     SMEM(presence_rebuild_kernel<uint16_t>, STBPE_PROWS * sizeof(unsigned int));
     SMEM(presence_rebuild_kernel<uint32_t>, STBPE_PROWS * sizeof(unsigned int));
 #undef SMEM
@@ -835,15 +835,41 @@ static int wide_pass1(stbpe_engine *e, int *ok, cudaStream_t s) {
     return STBPE_OK;
 }
 
+// From here on the partitions' words are added to a cleared table one by one, as several ranks do it, instead of
+// being ordered and built range by range.  2^30 slots: the ranges outgrow the 64 KB of shared memory that let three
+// CTAs share an SM (2.5e8 ids 7.3 instead of 8.8 ms, 2^30 ids 16.7 instead of 25.9).  2^29 slots: 256 ranges per
+// partition leave a piece few words of each, while the adds of a partition stay inside 32 MB of L2 and the longer
+// a region, the more of them the word caches take.  Ordered / one by one, whole count in ms: 2^30 ids 14.8 / 15.4, 1.4e9
+// 17.7 / 17.7, 1.7e9 21.3 / 20.0, 2^31 25.6 / 24.1, 2.8e9 31.7 / 30.4 (ids below 4 096: 1.4e9 12.3 / 13.1, 1.7e9 15.6 / 14.7).
+// Smaller tables: 2^28 slots and 1.7e9 ids 19.2 / 21.4.
+static bool wide_one_by_one(const stbpe_engine *e) {
+    return e->slots > (1ull << 29) || (e->slots == (1ull << 29) && e->n_tokens >= 3ll << 29);
+}
+
 // second and third pass of the partitioned count; *ok = 0 when the spill list ran over
 static int wide_build(stbpe_engine *e, int *ok, cudaStream_t s) {
     const PartBuffers &pb = e->parts;
+    if (wide_one_by_one(e)) {
+        WidePeers own = {};
+        own.block[0] = e->wide_block;
+        own.world = 1;
+        CK(cudaEventRecord(e->ev0, s));
+        clear_table_kernel<<<e->sm_count * 8, 256, 0, s>>>(e->d);
+        dense_to_table_kernel<false><<<256, 256, 0, s>>>(e->d, e->wide_dense);
+        partition_table_peers_kernel<<<pb.n_cta * 2 * STBPE_PARTS, 1024, 0, s>>>(e->d, own, 0, 1, pb.n_cta);
+        CK(cudaGetLastError());
+        CK(cudaEventRecord(e->ev1, s));
+        CK(cudaEventSynchronize(e->ev1));
+        CK(cudaEventElapsedTime(&e->convert_ms, e->ev0, e->ev1));
+        e->count_ms += e->convert_ms;
+        *ok = 1;
+        return STBPE_OK;
+    }
     int lg = 0;
     while ((1ull << lg) < e->slots) ++lg;
     // ranges of 2^13 slots: 64 KB of shared memory, three CTAs per SM; at least one bit and at most eight bits of
-    // ordering, so small tables get smaller ranges and the largest (2^30 slots) larger ones
-    int task_bits = lg - STBPE_PART_BITS - 1 < 13 ? lg - STBPE_PART_BITS - 1 : 13;
-    if (lg - STBPE_PART_BITS - task_bits > STBPE_SUB_MAX_BITS) task_bits = lg - STBPE_PART_BITS - STBPE_SUB_MAX_BITS;
+    // ordering, so small tables get smaller ranges
+    const int task_bits = lg - STBPE_PART_BITS - 1 < 13 ? lg - STBPE_PART_BITS - 1 : 13;
     const int sub_bits = lg - STBPE_PART_BITS - task_bits;
     const int chunk = sub_bits > 6 ? 16384 : 8192;
     const int cpr = (int)((pb.cap + chunk - 1) / chunk);
@@ -862,8 +888,7 @@ static int wide_build(stbpe_engine *e, int *ok, cudaStream_t s) {
         sub_partition_kernel<8192><<<e->sm_count * 3, STBPE_SUB_THREADS, 8192 * sizeof(uint32_t), s>>>(pb, cpr, sub_bits, offs);
     else
         sub_partition_kernel<16384><<<e->sm_count * 2, STBPE_SUB_THREADS, 16384 * sizeof(uint32_t), s>>>(pb, cpr, sub_bits, offs);
-    build_table_kernel<<<e->sm_count * (build_smem > 65536 ? 1 : 3), STBPE_BUILD_THREADS, build_smem, s>>>(e->d, pb, chunk, cpr, sub_bits, task_bits, offs, spill,
-                                                                                                   n_spill, spill_cap);
+    build_table_kernel<<<e->sm_count * 3, STBPE_BUILD_THREADS, build_smem, s>>>(e->d, pb, chunk, cpr, sub_bits, task_bits, offs, spill, n_spill, spill_cap);
     spill_to_table_kernel<<<e->sm_count, 256, 0, s>>>(e->d, spill, n_spill, spill_cap);
     dense_to_table_kernel<false><<<256, 256, 0, s>>>(e->d, e->wide_dense);
     CK(cudaGetLastError());
@@ -889,7 +914,7 @@ static int launch_count(stbpe_engine *e, bool mg, cudaStream_t s) {
         return STBPE_OK;
     }
     const bool fresh = e->recs_stale, wide = !mg && wide_eligible(e, fresh);
-    int rc = count_prologue(e, !wide, s);  // the partitioned count writes every slot of the table itself
+    int rc = count_prologue(e, !wide, s);  // the partitioned count writes or clears every slot of the table itself
     if (rc != STBPE_OK) return rc;
     if (e->d.n_tiles > 0 && fresh && e->only_bytes && !getenv("STBPE_NO_DENSE_COUNT")) {
         // byte-level fast path: dense stream, ids < 256

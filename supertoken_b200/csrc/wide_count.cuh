@@ -24,7 +24,8 @@
 //           200 M ids, 31 M pairs: 1.6 ms for both passes (6.2 ms when every word was added to the table with
 //           one or two atomics in L2, a partition at a time).
 // Several ranks: the owner of a partition adds its words out of every rank's regions
-// (partition_table_peers_kernel); the table slice that a launch touches stays in L2.
+// (partition_table_peers_kernel); the table slice that a launch touches stays in L2.  One rank does the same with a long
+// stream into a table of 2^29 slots or more (wide_one_by_one in engine.cu has the measurements).
 //
 // An id of 65 536 or more, or a partition region that outgrows its buffer, raises
 // STBPE_DERR_DENSE_OVERFLOW and the host recounts with the general kernel.
@@ -365,8 +366,8 @@ __global__ void spill_to_table_kernel(EngineDev e, const uint32_t *__restrict__ 
     if (fresh) atomicAdd(&e.st->n_keys, (u64)fresh);
 }
 
-// pass 2, several ranks: partition p, owned by this rank, out of the regions of every rank.  The grid
-// is one wave of blocks whatever the number of ranks; a block walks over its share of the
+// pass 2, several ranks, or one with a large table: partition p, owned by this rank, out of the regions of every rank.
+// The grid of a partition is one wave of blocks whatever the number of ranks; a block walks over its share of the
 // (source rank, region, half) units with one cache, which it adds to the table at the end.
 __global__ void __launch_bounds__(1024)
     partition_table_peers_kernel(EngineDev e, WidePeers wp, int p_first, int p_step, int n_cta) {

@@ -268,7 +268,7 @@ def test_more_equal_counts_than_candidates(n):
 
 
 @pytest.mark.parametrize("slots,n", [(1 << 10, 3), (1 << 13, 1025), (1 << 18, 8193), (1 << 21, 400001),
-                                     (1 << 28, 90001)])
+                                     (1 << 28, 90001), (1 << 30, 150001)])
 def test_partitioned_count_builds_tables_of_any_size(slots, n, monkeypatch):
     monkeypatch.setenv("STBPE_DENSE32_MIN_TOKENS", "1")
     rng = np.random.RandomState(n)
