@@ -287,6 +287,12 @@ struct Theta {
     __device__ __forceinline__ bool admits(i64 c, u64 k) const { return c > count || (c == count && k < key); }
 };
 
+// Whether a probe of the pair table goes on: a long one stops when another has found the table full.  (Otherwise every
+// add to a full table walks STBPE_MAX_PROBE slots: 2.5e8 ids into 2^25 slots took 2.5 minutes to report it.)
+__device__ __forceinline__ bool probe_on(const EngineDev &e, unsigned int probe) {
+    return probe < STBPE_MAX_PROBE && ((probe & 255u) != 255u || !(*(volatile unsigned int *)&e.st->error & STBPE_DERR_TABLE_FULL));
+}
+
 // Add delta to key in the pair table, inserting the key when absent.  `fresh` counts inserted keys
 // (the caller adds them to DevState::n_keys).  `made`: the key probably does not exist yet, so the first
 // access is the compare-and-swap that claims a slot instead of a load that would find it empty.
@@ -307,7 +313,7 @@ __device__ __forceinline__ void table_add(const EngineDev &e, u64 key, i64 delta
     Slot mx;
     if (NOTE == NOTE_DIRTY) mx = ldcg_slot(e.blockmax + blk);  // fetched together with the first probe
 #pragma unroll 1
-    for (unsigned int probe = 0; probe < STBPE_MAX_PROBE; ++probe) {
+    for (unsigned int probe = 0; probe_on(e, probe); ++probe) {
         Slot *s = &e.table[h];
         u64 k = made ? STBPE_EMPTY : __ldcg(&s->key);
         if (k == STBPE_EMPTY) {

@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(STBPE_DENSE_THREADS, 1)
 // store, and nothing is marked dirty because a full refresh follows the initial count.
 __device__ __forceinline__ bool table_insert_unique(const EngineDev &e, u64 key, i64 count) {
     u64 h = slot_of(e, key);
-    for (unsigned int probe = 0; probe < STBPE_MAX_PROBE; ++probe) {
+    for (unsigned int probe = 0; probe_on(e, probe); ++probe) {
         Slot *s = &e.table[h];
         if (atomicCAS(&s->key, STBPE_EMPTY, key) == STBPE_EMPTY) {
             s->count = count;

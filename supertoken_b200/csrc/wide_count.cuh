@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(STBPE_PART_THREADS, 1)
 // Add n occurrences of a key to the pair table during the first count: no maxima to keep (a full
 // refresh follows), and a key that is already there costs one load and one reduction without result.
 __device__ __forceinline__ bool table_count_n(const EngineDev &e, u64 key, u64 h, u64 n, unsigned int &fresh) {
-    for (unsigned int probe = 0; probe < STBPE_MAX_PROBE; ++probe) {
+    for (unsigned int probe = 0; probe_on(e, probe); ++probe) {
         Slot *s = &e.table[h];
         u64 k = __ldcg(&s->key);
         if (k == STBPE_EMPTY) {

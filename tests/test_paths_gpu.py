@@ -1,12 +1,14 @@
 """Dispatch edges of the CUDA engine against the CPU oracle: merges taken together, streams that widen, merges the
 host gives, many equal counts, tables that are rebuilt, the row seam's table sizes.  Every comparison is exact."""
+import time
+
 import numpy as np
 import pytest
 import torch
 
 from oracle import oracle as O
 from supertoken_b200 import ops
-from supertoken_b200.engine import Engine
+from supertoken_b200.engine import CapacityError, Engine
 
 pytestmark = pytest.mark.gpu
 
@@ -291,6 +293,20 @@ def test_partitioned_count_with_several_pieces_per_region(slots, max_tokens, bat
     e.count_initial()
     assert e.state().count_convert_ms > 0
     _check_histogram(e, ids, off)
+    e.close()
+
+
+@pytest.mark.parametrize("partitioned", [False, True])
+def test_full_pair_table_is_reported_at_once(partitioned, monkeypatch):
+    # some 4 million distinct pairs, 65 536 slots: an add that walked the whole table each time would take half a minute
+    monkeypatch.setenv("STBPE_DENSE32_MIN_TOKENS", "1" if partitioned else str(1 << 40))
+    ids = np.random.RandomState(1).randint(0, 65536, 1 << 22).astype(np.int32)
+    e = Engine(len(ids), base_vocab=65536, max_merges=1, table_slots=1 << 16)
+    e.append_ids(ids)
+    t = time.perf_counter()
+    with pytest.raises(CapacityError):
+        e.count_initial()
+    assert time.perf_counter() - t < 10
     e.close()
 
 
