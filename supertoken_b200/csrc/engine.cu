@@ -298,10 +298,10 @@ static const DeviceInfo &device_info(int dev) {
 }
 
 // Slots of a table that is sized by the caller's stream of ids: keys are never removed, so it must hold every
-// pair a run ever creates; 2^27 slots carried 32 000 merges on 2^30 tokens, streams of 2^32 tokens and more get
-// 2^29 (8 GiB).
-static u64 auto_slots(i64 max_tokens) {
-    const u64 cap = max_tokens >= (1ll << 32) ? (1ull << 29) : (1ull << 27);
+// pair a run ever creates.  One rank: up to 2^29 (8 GiB; 2^31 Zipf ids over 65 536 hold 1.7e8 pairs, more than 2^27 slots).
+// Several ranks: 2^27 slots carried 32 000 merges on 2^30 tokens, streams of 2^32 tokens and more get 2^29.
+static u64 auto_slots(i64 max_tokens, int world) {
+    const u64 cap = world == 1 || max_tokens >= (1ll << 32) ? (1ull << 29) : (1ull << 27);
     u64 slots = (u64)max_tokens / 4;
     if (slots < (1ull << 20)) slots = 1ull << 20;
     return slots < cap ? slots : cap;
@@ -387,7 +387,7 @@ STBPE_VISIBLE int stbpe_create(stbpe_engine **out, const stbpe_config *cfg) {
     e->d.rank = cfg->rank;
     e->wide = starts_wide(*cfg);
     e->table_auto = cfg->table_slots <= 0 && cfg->world_size == 1;
-    set_slots(e, cfg->table_slots > 0 ? (u64)cfg->table_slots : auto_slots(cfg->max_tokens));
+    set_slots(e, cfg->table_slots > 0 ? (u64)cfg->table_slots : auto_slots(cfg->max_tokens, cfg->world_size));
 
 #define ALLOC(ptr, n)                                                  \
     if ((c = dev_alloc(e, &(ptr), (size_t)(n))) != cudaSuccess) return bail(cuda_fail(e, c, "cudaMalloc " #ptr))
@@ -782,7 +782,7 @@ static int count_prologue(stbpe_engine *e, bool clear, cudaStream_t s) {
         // A stream of bytes starts with at most 65 536 pairs and its table grows with the keys (grow_table): a table
         // of 16 MB stays in L2 and costs nothing to clear or scan, one for every pair a run might create is
         // half a gigabyte on 128 MB of text.  Other streams may hold any number of pairs from the start.
-        u64 want = e->only_bytes ? (u64)1 << 20 : auto_slots(e->max_tokens);
+        u64 want = e->only_bytes ? (u64)1 << 20 : auto_slots(e->max_tokens, 1);
         if (!fresh && e->slots > want) want = e->slots;  // a recount of the rewritten stream
         rc = set_table(e, want);
         if (rc != STBPE_OK) return rc;

@@ -310,6 +310,16 @@ def test_full_pair_table_is_reported_at_once(partitioned, monkeypatch):
     e.close()
 
 
+@pytest.mark.parametrize("lg,slots", [(21, 1 << 20), (31, 1 << 29)])
+def test_automatic_table_of_a_stream_of_ids(lg, slots):
+    # 2^31 ids over 65 536 hold 1.7e8 pairs
+    e = Engine(1 << lg, base_vocab=65536, max_merges=1)
+    e.append_ids(np.array([7, 40000, 7, 40000, 9], dtype=np.int32))
+    e.count_initial()
+    assert e.state().table_slots == slots and e.select_best() == (7 << 32 | 40000, 2, 0)
+    e.close()
+
+
 def test_pair_table_grows_in_mid_run():
     # random bytes: every merge makes some hundred pairs that were not there before
     n = 16 << 20
