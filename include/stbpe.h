@@ -75,6 +75,10 @@ int stbpe_destroy(stbpe_engine *e);
 const char *stbpe_last_error(const stbpe_engine *e);
 const char *stbpe_version(void);
 
+/* Memory of destroyed engines stays cached for the next one, at most 4 GiB per device and 64 MiB of pinned host memory.
+ * This gives it back, oldest blocks first, until at most keep_bytes stay; device -1 = the pinned host memory. */
+int stbpe_trim(int32_t device, int64_t keep_bytes);
+
 /* Host only: the valid prefixes of a padded batch (tokens and valid: rows x width, valid != 0 marks a token) one behind
  * the other into out, as bytes (elem 1) or int32 ids (elem 4), and their lengths.  STBPE_E_STATE: a row's valid
  * marks are no prefix; STBPE_E_ID_OVERFLOW: elem 1 and an id outside 0 .. 255. */

@@ -3,5 +3,6 @@
 The CUDA library (``libstbpe.so``, sm_100a) is required; nothing here falls back to a CPU
 implementation."""
 from .bpe_trainer import GPUBPETrainer  # noqa: F401
+from .engine import trim_cache  # noqa: F401
 
-__all__ = ["GPUBPETrainer"]
+__all__ = ["GPUBPETrainer", "trim_cache"]

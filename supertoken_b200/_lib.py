@@ -39,6 +39,7 @@ SIGNATURES = {
     "stbpe_destroy": (_int, [_vp]),
     "stbpe_last_error": (ctypes.c_char_p, [_vp]),
     "stbpe_version": (ctypes.c_char_p, []),
+    "stbpe_trim": (_int, [_i32, _i64]),
     "stbpe_reset": (_int, [_vp]),
     "stbpe_append_bytes": (_int, [_vp, _vp, _i64, _vp, _i64, _vp]),
     "stbpe_flatten_rows": (_int, [_vp, _vp, _i64, _i64, _i32, _vp, _vp]),

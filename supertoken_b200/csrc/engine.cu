@@ -257,6 +257,15 @@ STBPE_VISIBLE int stbpe_destroy(stbpe_engine *e) {
     return STBPE_OK;
 }
 
+STBPE_VISIBLE int stbpe_trim(int32_t device, int64_t keep_bytes) {
+    if (device < -1 || device >= 64 || keep_bytes < 0) return STBPE_E_BADARG;
+    if (device < 0)
+        stbpe::pinned_blocks().trim(0, (size_t)keep_bytes);
+    else
+        stbpe::device_blocks().trim(device, (size_t)keep_bytes);
+    return STBPE_OK;
+}
+
 static const DeviceInfo &device_info(int dev) {
     static std::mutex mu;
     static DeviceInfo infos[64];

@@ -28,6 +28,21 @@ def _stream_ptr(device: torch.device) -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
 
 
+def trim_cache(device: Optional[torch.device | str | int] = None, keep_bytes: int = 0) -> None:
+    """Give back the memory that destroyed engines left for the next one (at most 4 GiB per device, 64 MiB pinned), until
+    at most ``keep_bytes`` of each stay; ``device`` None: of every device.  What ``torch.cuda.empty_cache`` is to torch's
+    own cache, which cannot reach this one."""
+    if device is None:
+        indices = range(torch.cuda.device_count())
+    else:
+        index = torch.device("cuda", device).index if isinstance(device, int) else torch.device(device).index
+        indices = [torch.cuda.current_device() if index is None else index]
+    for i in (*indices, -1):
+        st = L.load().stbpe_trim(i, int(keep_bytes))
+        if st != L.OK:
+            _raise(st, "bad device or size")
+
+
 class Engine:
     """Token stream + pair table of one GPU.  Thin wrapper: every method is one C-ABI call."""
 

@@ -30,6 +30,13 @@ def test_library_exports_every_declared_symbol():
     assert lib.stbpe_version().startswith(b"stbpe")
 
 
+def test_trim_checks_its_arguments():
+    from supertoken_b200 import _lib
+    lib = _lib.load()
+    assert lib.stbpe_trim(-1, 0) == lib.stbpe_trim(0, 1 << 30) == _lib.OK  # nothing is cached here
+    assert lib.stbpe_trim(-2, 0) == lib.stbpe_trim(64, 0) == lib.stbpe_trim(0, -1) == _lib.E_BADARG
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     from supertoken_b200 import _lib
     monkeypatch.setattr(_lib, "_lib", None)

@@ -472,3 +472,23 @@ def test_full_size_properties_on_a_256_mib_corpus():
     e.train(600)
     assert e.merges()[0] == m
     e.close()
+
+
+def test_cached_memory_is_given_back():
+    import supertoken_b200
+
+    def used():
+        torch.cuda.synchronize()
+        free, total = torch.cuda.mem_get_info()
+        return total - free
+
+    supertoken_b200.trim_cache("cuda")
+    base = used()
+    Engine(1 << 28, base_vocab=256, max_merges=1).close()
+    assert used() - base >= 1 << 29      # 16-bit tokens, kept for the next engine
+    supertoken_b200.trim_cache(keep_bytes=1 << 40)
+    assert used() - base >= 1 << 29
+    supertoken_b200.trim_cache()
+    assert used() - base < 1 << 26
+    with pytest.raises(ValueError):
+        supertoken_b200.trim_cache(0, keep_bytes=-1)
