@@ -1231,6 +1231,9 @@ static int repack_stream(stbpe_engine *e, bool to_wide, i64 *total, cudaStream_t
     CK(cudaStreamSynchronize(s));
     const size_t want = (size_t)((*total + STBPE_TILE - 1) / STBPE_TILE) * STBPE_TILE * (to_wide ? 4 : 2);
     if (want > e->alt_bytes || !e->tiles_alt) {
+        dev_free(e, e->tiles_alt);  // (the stream is idle: it has just been waited for)
+        e->tiles_alt = nullptr;
+        e->alt_bytes = 0;
         unsigned char *t = nullptr;
         cudaError_t c = dev_alloc(e, &t, want);
         if (c != cudaSuccess) return cuda_fail(e, c, "cudaMalloc second stream buffer");

@@ -492,3 +492,35 @@ def test_cached_memory_is_given_back():
     assert used() - base < 1 << 26
     with pytest.raises(ValueError):
         supertoken_b200.trim_cache(0, keep_bytes=-1)
+
+
+def test_repack_keeps_two_stream_buffers_at_most(monkeypatch):
+    # a re-pack leaves a 16-bit buffer behind; the 32-bit stream that follows does not fit it and takes its place
+    import supertoken_b200
+
+    def used():
+        supertoken_b200.trim_cache("cuda")
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free, total = torch.cuda.mem_get_info()
+        return (total - free) / (1 << 20)
+
+    monkeypatch.setenv("STBPE_DENSE32_MIN_TOKENS", str(1 << 40))
+    n = 1 << 25
+    e = Engine(n, base_vocab=32760, max_merges=12, table_slots=1 << 20)
+    e.append_ids(torch.randint(0, 200, (n,), device="cuda", dtype=torch.int32, generator=torch.Generator("cuda").manual_seed(1)))
+    e.count_initial()
+    e.train(2)
+    e.repack(force=True)
+    e.train(10)
+    assert e.state().merges_done == 12 and e.state().repacks >= 1  # ids 32760 .. 32771: wide from 32767 on
+    k, c = e.export_histogram()
+    e.count_initial()
+    k2, c2 = e.export_histogram()
+    assert torch.equal(k, k2) and torch.equal(c, c2)
+    del k, c, k2, c2
+    held = used()
+    e.close()
+    held -= used()
+    # 4 and 2 bytes per token of stream, 65 KB of filter per 32 tiles, 16 MiB of table, records: 128 + 64 + 64 + 16 + 4
+    assert 256 < held < 320
