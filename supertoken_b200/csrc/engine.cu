@@ -23,6 +23,7 @@
 #define STBPE_PINNED_BYTES ((size_t)4 << 20)
 #define STBPE_PINNED_STATE 16384  // bytes in front that the device state travels through
 #define STBPE_COUNT_SMEM (STBPE_COUNT_SLOTS * 12)
+#define STBPE_MAX_SLOTS (1ll << 32)  // of one rank's pair table
 
 #define STBPE_VISIBLE __attribute__((visibility("default")))
 
@@ -54,6 +55,7 @@ struct stbpe_engine {
     bool wide_open, wide_counted;          // peers mapped / the table holds a count made by stbpe_mg_wide_pass2
     bool full_refresh_pending;             // that count marked no block dirty: the next refresh recomputes all maxima
     i64 dense32_min;      // streams shorter than this use the general kernel
+    i64 narrow_counts;    // the merge loop on 16-bit tokens compares counts below this
     bool only_bytes;      // every token so far came from stbpe_append_bytes (ids < 256)
     ncclComm_t comm;      // own NCCL communicator for the native multi-GPU round loop
     i64 *all_cands;       // world x 4 gathered candidates (native loop)
@@ -367,12 +369,17 @@ STBPE_VISIBLE int stbpe_create(stbpe_engine **out, const stbpe_config *cfg) {
     if (cfg->max_tokens < 0 || cfg->max_merges < 0 || cfg->base_vocab < 0 || cfg->world_size < 1 ||
         cfg->rank < 0 || cfg->rank >= cfg->world_size)
         return fail(nullptr, STBPE_E_BADARG, "invalid configuration");
+    if (cfg->max_tokens > 0x7FFFFFFFll * STBPE_TILE) return fail(nullptr, STBPE_E_BADARG, "max_tokens: tiles are numbered with 31 bits");
+    if (cfg->world_size == 1 && cfg->table_slots > STBPE_MAX_SLOTS)
+        return fail(nullptr, STBPE_E_BADARG, "table_slots: the candidate list holds 32-bit slot numbers");
     if ((i64)cfg->base_vocab + (i64)cfg->max_merges >= 0x7FFFFFFFll)
         return fail(nullptr, STBPE_E_ID_OVERFLOW, "Token id overflow: ids must stay below 2^31-1");
     stbpe_engine *e = new stbpe_engine();  // all members zero
     e->cfg = *cfg;
     e->dense32_min = 1ll << 24;
     if (const char *v = getenv("STBPE_DENSE32_MIN_TOKENS")) e->dense32_min = atoll(v);
+    e->narrow_counts = Best<uint16_t>::COUNTS;
+    if (const char *v = getenv("STBPE_NARROW_COUNTS")) e->narrow_counts = atoll(v);
     e->use_graph = getenv("STBPE_NO_GRAPH") == nullptr;
     e->part_group = STBPE_PARTS;
     if (const char *v = getenv("STBPE_PART_GROUP")) e->part_group = atoi(v) > 0 ? atoi(v) : STBPE_PARTS;
@@ -760,7 +767,7 @@ static int grow_table(stbpe_engine *e, cudaStream_t s) {
     Slot *old = e->d.table;
     const u64 old_slots = e->slots;
     Slot *fresh = nullptr;
-    cudaError_t c = dev_alloc(e, &fresh, old_slots * 4);
+    cudaError_t c = old_slots * 4 > (u64)STBPE_MAX_SLOTS ? cudaErrorMemoryAllocation : dev_alloc(e, &fresh, old_slots * 4);
     if (c != cudaSuccess) {
         cudaGetLastError();
         e->table_auto = false;  // no room: go on in the table there is, a full one is an error status
@@ -1338,6 +1345,14 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
     if (!e->sync_zeroed) {
         CK(cudaMemsetAsync(e->d.sync, 0, 2 * sizeof(LoopSync), s));
         e->sync_zeroed = true;
+    }
+    if (!e->wide && e->n_tokens >= e->narrow_counts) {  // no count is larger than the stream is long; the largest only falls
+        if (int rc_ = choose(e, false, out, s)) return rc_;
+        if (out->peek_count >= e->narrow_counts) {
+            int rc = widen_stream(e, s);
+            if (rc == STBPE_OK) rc = filter_policy(e, *out, true, s);
+            if (rc != STBPE_OK) return rc;
+        }
     }
     for (;;) {
         const int grid = e->sm_count;  // one CTA per SM; the barrier is no faster with fewer

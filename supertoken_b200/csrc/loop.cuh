@@ -89,12 +89,14 @@ struct BoundedWait {
 };
 
 // The arg-max in registers.  With 15-bit ids a pair and its count fit 64 bits whose order is the
-// order of the selection (larger count, then smaller key), and a warp's maximum is two redux steps.
+// order of the selection (larger count, then smaller key), and a warp's maximum is two redux steps.  That leaves 34
+// bits for the count; a stream with more equal pairs is widened before the loop starts.
 template <typename T>
 struct Best;
 template <>
 struct Best<uint16_t> {
     typedef u64 type;
+    static constexpr i64 COUNTS = 1ll << 34;
     static __device__ __forceinline__ u64 none() { return 0ull; }
     static __device__ __forceinline__ u64 make(u64 key, i64 count) {
         const u64 k30 = ((key >> 32) << 15) | (key & 0x7FFFull);

@@ -57,6 +57,9 @@ def test_create_rejects_bad_config_without_gpu_work():
     h = ctypes.c_void_p()
     cfg = _lib.Config(0, 256, -5, 0, 10, 1, 0, 0)
     assert lib.stbpe_create(ctypes.byref(h), ctypes.byref(cfg)) == _lib.E_BADARG
+    for tokens, slots in ((1 << 41, 0), (10, (1 << 32) + 1)):  # tile and slot numbers would wrap
+        cfg = _lib.Config(0, 256, tokens, slots, 10, 1, 0, 0)
+        assert lib.stbpe_create(ctypes.byref(h), ctypes.byref(cfg)) == _lib.E_BADARG
     cfg = _lib.Config(0, 0x7FFFFFF0, 10, 0, 100, 1, 0, 0)
     assert lib.stbpe_create(ctypes.byref(h), ctypes.byref(cfg)) == _lib.E_ID_OVERFLOW
     assert b"overflow" in lib.stbpe_last_error(None)

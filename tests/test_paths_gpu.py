@@ -85,6 +85,23 @@ def test_stream_widens_while_training_and_while_appending(top):
     e.close()
 
 
+@pytest.mark.parametrize("above,wide", [(1, False), (0, True), (-1000, True)])
+def test_counts_that_16_bit_tokens_leave_no_room_for(above, wide, monkeypatch):
+    # the limit, 2^34 in earnest, one above the largest count, at it and below it
+    rng = np.random.RandomState(4)
+    ids = rng.choice([1, 2, 3], 20000, p=[0.5, 0.3, 0.2]).astype(np.int32)
+    off = _rows(ids, rng, 300)
+    top = int(O.count_pairs_flat(ids, off, 1)[1].max())
+    monkeypatch.setenv("STBPE_NARROW_COUNTS", str(top + above))
+    e = _engine(ids, off, 16, 30)
+    e.train(1)
+    st = e.state()
+    assert (st.tile_bytes_in > st.n_tiles * 1024 * 4) == wide
+    e.train(29)
+    _check(e, ids, off, 16, 30)
+    e.close()
+
+
 @pytest.mark.parametrize("n", [1, 2, 9, 40])
 def test_merges_given_by_the_host(n):
     # absent pairs, a pair twice in a row, pairs of the new ids, pairs that share tokens
