@@ -615,13 +615,11 @@ __device__ __forceinline__ void block_best(u64 &bk, i64 &bc, u64 *s_k, i64 *s_c)
 #include "peer_kernels.cuh"
 
 // Best pair over all block maxima: every CTA reduces its share, the last one to finish reduces theirs.
-// mode 0: peek (result into the state); 1: single rank, advance or stop; 2: candidate of this rank
-// into cand; 3: candidate of this rank into every peer mailbox, then wait for the peers' candidates
-// and commit (target = the merge target of the engine)
+// mode 0: peek (result into the state); 2: candidate of this rank into cand; 3: candidate of this rank into every
+// peer mailbox, then wait for the peers' candidates and commit (target = the merge target of the engine)
 __global__ void __launch_bounds__(STBPE_SELECT_THREADS)
     select_kernel(EngineDev e, int mode, Slot *partial, i64 *cand, int target = 0) {
     DevState *st = e.st;
-    if (mode == 1 && st->stopped) return;
     __shared__ u64 s_k[STBPE_SELECT_THREADS / 32];
     __shared__ i64 s_c[STBPE_SELECT_THREADS / 32];
     __shared__ int s_last;
@@ -656,8 +654,6 @@ __global__ void __launch_bounds__(STBPE_SELECT_THREADS)
     if (mode == 0) {
         st->peek_key = bk;
         st->peek_count = bc;
-    } else if (mode == 1) {
-        advance_or_stop(e, bk, bc);
     } else if (mode == 2) {
         cand[0] = (i64)bk;
         cand[1] = bc;
