@@ -35,6 +35,7 @@
 #define STBPE_PROWS 16384  // rows of the pair filter: pair keys are hashed onto them (three hashes)
 #define STBPE_PPITCH (STBPE_PROWS + 32)  // words per group of 32 tiles: the rows and the wildcard word (row STBPE_PROWS)
 #define STBPE_MAX_PROBE (1u << 20)
+#define STBPE_AUTO_PROBE (1u << 12)  // where the table grows instead: the longest probe to be expected at 90 % load is 3 000 slots
 
 // device error bits
 #define STBPE_DERR_TABLE_FULL 1u
@@ -149,6 +150,7 @@ struct EngineDev {
     int n_tiles;
     Slot *table;
     u64 mask;
+    unsigned int max_probe;  // slots an add looks at before it calls the table full
     int slot_bits;  // slot index bits below the table slice of a partition (slots = slices << slot_bits)
     unsigned int *cand;        // slots of the candidates
     unsigned int *cand_hist;   // STBPE_CAND_BUCKETS counters of the threshold search
@@ -288,9 +290,9 @@ struct Theta {
 };
 
 // Whether a probe of the pair table goes on: a long one stops when another has found the table full.  (Otherwise every
-// add to a full table walks STBPE_MAX_PROBE slots: 2.5e8 ids into 2^25 slots took 2.5 minutes to report it.)
+// add to a full table walks `max_probe` slots: 2.5e8 ids into 2^25 slots took 2.5 minutes to report it.)
 __device__ __forceinline__ bool probe_on(const EngineDev &e, unsigned int probe) {
-    return probe < STBPE_MAX_PROBE && ((probe & 255u) != 255u || !(*(volatile unsigned int *)&e.st->error & STBPE_DERR_TABLE_FULL));
+    return probe < e.max_probe && ((probe & 255u) != 255u || !(*(volatile unsigned int *)&e.st->error & STBPE_DERR_TABLE_FULL));
 }
 
 // Add delta to key in the pair table, inserting the key when absent.  `fresh` counts inserted keys

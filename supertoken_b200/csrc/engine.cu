@@ -95,6 +95,7 @@ struct stbpe_engine {
     bool state_stale;     // the device state is that of a stream that has been dropped
     bool table_auto;      // the table is sized by the stream and grows with the keys
     u64 table_cap;        // slots the allocated table has room for
+    u64 slots_needed;     // a count of this stream has overflowed a quarter of these
     size_t presence_cap;  // groups of 32 tiles the pair filter has room for
     void *off_dev;        // row offsets of an append
     size_t off_cap;
@@ -308,14 +309,20 @@ static const DeviceInfo &device_info(int dev) {
     return i;
 }
 
-// Slots of a table that is sized by the caller's stream of ids: keys are never removed, so it must hold every
-// pair a run ever creates.  One rank: up to 2^29 (8 GiB; 2^31 Zipf ids over 65 536 hold 1.7e8 pairs, more than 2^27 slots).
-// Several ranks: 2^27 slots carried 32 000 merges on 2^30 tokens, streams of 2^32 tokens and more get 2^29.
-static u64 auto_slots(i64 max_tokens, int world) {
-    const u64 cap = world == 1 || max_tokens >= (1ll << 32) ? (1ull << 29) : (1ull << 27);
-    u64 slots = (u64)max_tokens / 4;
-    if (slots < (1ull << 20)) slots = 1ull << 20;
-    return slots < cap ? slots : cap;
+// Slots of a table that is sized by the stream.
+// One rank: for the first count of n ids below `ids`; a count that does not fit takes four times as many (stbpe_count_initial), merges
+// grow the table (grow_table).  Of Zipf ids over 65 536, 42 % of 2^20 pairs are distinct, 17 % of 2^27, 8 % of 2^31: a slot
+// per token up to 2^25 of them, one for four tokens of long streams, up to 2^29 (8 GiB); no more than pairs can differ.
+static u64 auto_slots(i64 n, i64 ids) {
+    u64 slots = std::max((u64)std::min(n, (i64)1 << 25), (u64)n / 4);
+    if (ids < 65536) slots = std::min(slots, 2 * (u64)ids * (u64)ids);
+    return std::min(std::max(slots, (u64)1 << 20), (u64)1 << 29);
+}
+// Several ranks: keys are never removed and nothing grows, so it must hold every pair a run ever creates; 2^27 slots
+// carried 32 000 merges on 2^30 tokens, streams of 2^32 tokens and more get 2^29 (8 GiB).
+static u64 auto_slots_mg(i64 max_tokens) {
+    const u64 cap = max_tokens >= (1ll << 32) ? (1ull << 29) : (1ull << 27);
+    return std::min(std::max((u64)max_tokens / 4, (u64)1 << 20), cap);
 }
 
 static void set_slots(stbpe_engine *e, u64 want) {
@@ -351,6 +358,7 @@ static void drop_stream(stbpe_engine *e) {
     e->wide_counted = e->full_refresh_pending = false;
     e->load_err = e->max_id = 0;
     e->bytes_below = e->made_below = 0;
+    e->slots_needed = 0;
     e->merges_known = e->foreign_ids = false;
     e->state_stale = true;
 }
@@ -403,7 +411,8 @@ STBPE_VISIBLE int stbpe_create(stbpe_engine **out, const stbpe_config *cfg) {
     e->d.rank = cfg->rank;
     e->wide = starts_wide(*cfg);
     e->table_auto = cfg->table_slots <= 0 && cfg->world_size == 1;
-    set_slots(e, cfg->table_slots > 0 ? (u64)cfg->table_slots : auto_slots(cfg->max_tokens, cfg->world_size));
+    e->d.max_probe = e->table_auto ? STBPE_AUTO_PROBE : STBPE_MAX_PROBE;
+    set_slots(e, cfg->table_slots > 0 ? (u64)cfg->table_slots : e->table_auto ? (u64)1 << 20 : auto_slots_mg(cfg->max_tokens));
 
 #define ALLOC(ptr, n)                                                  \
     if ((c = dev_alloc(e, &(ptr), (size_t)(n))) != cudaSuccess) return bail(cuda_fail(e, c, "cudaMalloc " #ptr))
@@ -666,10 +675,11 @@ static int check_error_bits(stbpe_engine *e, unsigned int err) {
     return STBPE_OK;
 }
 
-static int check_device_error(stbpe_engine *e, cudaStream_t s) {
+static int check_device_error(stbpe_engine *e, cudaStream_t s, unsigned int *bits = nullptr) {
     unsigned int err = 0;
     CK(cudaMemcpyAsync(&err, &e->d.st->error, sizeof(err), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    if (bits) *bits = err;
     return check_error_bits(e, err);
 }
 
@@ -771,6 +781,7 @@ static int grow_table(stbpe_engine *e, cudaStream_t s) {
     if (c != cudaSuccess) {
         cudaGetLastError();
         e->table_auto = false;  // no room: go on in the table there is, a full one is an error status
+        e->d.max_probe = STBPE_MAX_PROBE;
         return STBPE_OK;
     }
     set_slots(e, old_slots * 4);
@@ -798,7 +809,7 @@ static int count_prologue(stbpe_engine *e, bool clear, cudaStream_t s) {
         // A stream of bytes starts with at most 65 536 pairs and its table grows with the keys (grow_table): a table
         // of 16 MB stays in L2 and costs nothing to clear or scan, one for every pair a run might create is
         // half a gigabyte on 128 MB of text.  Other streams may hold any number of pairs from the start.
-        u64 want = e->only_bytes ? (u64)1 << 20 : auto_slots(e->max_tokens, 1);
+        u64 want = std::max(e->only_bytes ? (u64)1 << 20 : auto_slots(e->n_tokens, ids_below(e)), e->slots_needed);
         if (!fresh && e->slots > want) want = e->slots;  // a recount of the rewritten stream
         rc = set_table(e, want);
         if (rc != STBPE_OK) return rc;
@@ -1009,10 +1020,22 @@ STBPE_VISIBLE int stbpe_count_initial(stbpe_engine *e, void *stream) {
     cudaStream_t s = (cudaStream_t)stream;
     CK(cudaSetDevice(e->cfg.device));
     if (e->cfg.world_size > 1) return fail(e, STBPE_E_STATE, "use stbpe_mg_count_local on a multi-rank engine");
-    int rc = launch_count(e, false, s);
-    if (rc != STBPE_OK) return rc;
-    e->counted = true;
-    return check_device_error(e, s);
+    for (;;) {
+        const bool fresh = e->recs_stale;
+        int rc = launch_count(e, false, s);
+        if (rc != STBPE_OK) return rc;
+        unsigned int err = 0;
+        rc = check_device_error(e, s, &err);
+        if ((err & STBPE_DERR_TABLE_FULL) && e->table_auto && e->slots * 4 <= (u64)STBPE_MAX_SLOTS) {
+            // more distinct pairs than the table was sized for: the same count once more, with four times the slots
+            e->slots_needed = e->slots * 4;
+            e->recs_stale = fresh;
+            CK(cudaMemsetAsync(&e->d.st->error, 0, sizeof(err), s));
+            continue;
+        }
+        e->counted = true;
+        return rc;
+    }
 }
 
 // Candidate list of the pair table as it stands: threshold search (one pass over the table in the usual case,

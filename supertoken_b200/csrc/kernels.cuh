@@ -308,7 +308,7 @@ __global__ void refresh_kernel(EngineDev e, int all) {
 
 static __device__ __noinline__ i64 find_slot(const EngineDev &e, u64 key) {
     u64 h = slot_of(e, key);
-    for (unsigned int probe = 0; probe < STBPE_MAX_PROBE; ++probe) {
+    for (unsigned int probe = 0; probe < e.max_probe; ++probe) {
         const u64 k = *(volatile u64 *)&e.table[h].key;
         if (k == key) return (i64)h;
         if (k == STBPE_EMPTY) return -1;

@@ -327,13 +327,26 @@ def test_full_pair_table_is_reported_at_once(partitioned, monkeypatch):
     e.close()
 
 
-@pytest.mark.parametrize("lg,slots", [(21, 1 << 20), (31, 1 << 29)])
-def test_automatic_table_of_a_stream_of_ids(lg, slots):
-    # 2^31 ids over 65 536 hold 1.7e8 pairs
-    e = Engine(1 << lg, base_vocab=65536, max_merges=1)
-    e.append_ids(np.array([7, 40000, 7, 40000, 9], dtype=np.int32))
+@pytest.mark.parametrize("lg,vocab,slots", [(15, 65536, 1 << 20), (22, 65536, 1 << 24), (22, 256, 1 << 20), (22, 1500, 1 << 22),
+                                            (26, 65536, 1 << 27)])
+def test_automatic_table_of_a_stream_of_ids(lg, vocab, slots):
+    # uniform ids: nearly every pair is another one, so 2^22 of them do not fit 2^22 slots, 2^26 not the 2^25 they get first
+    n = 1 << lg
+    ids = torch.randint(0, vocab, (n,), dtype=torch.int32, device="cuda", generator=torch.Generator("cuda").manual_seed(lg))
+    e = Engine(2 * n, base_vocab=65536, max_merges=4)
+    for _ in range(2):
+        e.reset()
+        e.append_ids(ids)
+        e.count_initial()
+        assert e.state().table_slots == slots
+        k, c = e.export_histogram()
+        ref, rc = torch.unique((ids[:-1].to(torch.int64) << 32) | ids[1:], return_counts=True)
+        assert torch.equal(k, ref) and torch.equal(c, rc)
+    e.train(4)  # (of the shortest stream every pair is alone: nothing to merge)
+    k, c = e.export_histogram()
     e.count_initial()
-    assert e.state().table_slots == slots and e.select_best() == (7 << 32 | 40000, 2, 0)
+    k2, c2 = e.export_histogram()
+    assert torch.equal(k, k2) and torch.equal(c, c2)
     e.close()
 
 
