@@ -54,7 +54,7 @@ struct stbpe_engine {
     WidePeers wide_peers;
     bool wide_open, wide_counted;          // peers mapped / the table holds a count made by stbpe_mg_wide_pass2
     bool full_refresh_pending;             // that count marked no block dirty: the next refresh recomputes all maxima
-    i64 dense32_min;      // streams shorter than this use the general kernel
+    i64 dense32_min;      // streams shorter than this use the general kernel; < 0: by the rule of wide_eligible
     i64 narrow_counts;    // the merge loop on 16-bit tokens compares counts below this
     bool only_bytes;      // every token so far came from stbpe_append_bytes (ids < 256)
     ncclComm_t comm;      // own NCCL communicator for the native multi-GPU round loop
@@ -384,7 +384,7 @@ STBPE_VISIBLE int stbpe_create(stbpe_engine **out, const stbpe_config *cfg) {
         return fail(nullptr, STBPE_E_ID_OVERFLOW, "Token id overflow: ids must stay below 2^31-1");
     stbpe_engine *e = new stbpe_engine();  // all members zero
     e->cfg = *cfg;
-    e->dense32_min = 1ll << 24;
+    e->dense32_min = -1;
     if (const char *v = getenv("STBPE_DENSE32_MIN_TOKENS")) e->dense32_min = atoll(v);
     e->narrow_counts = Best<uint16_t>::COUNTS;
     if (const char *v = getenv("STBPE_NARROW_COUNTS")) e->narrow_counts = atoll(v);
@@ -832,9 +832,16 @@ static int count_prologue(stbpe_engine *e, bool clear, cudaStream_t s) {
     return STBPE_OK;
 }
 
+// Whether the partitioned count takes a stream: fresh, ids below 65 536, and long enough for its fixed 0.4 ms (six launches, two
+// reads of the error bits).  What the general kernel takes depends on how many pairs are distinct, that is on the ids: over
+// 65 536 ids, general / partitioned on an engine that has counted before, 2^19 0.44 / 0.45 ms, 2^20 0.57 / 0.48, 2^21 0.84 /
+// 0.50, 2^22 1.45 / 0.54, 2^24 4.3 / 0.68; over 4 096, 2^20 0.38 / 0.47, 2^21 0.52 / 0.49, 2^22 1.01 / 0.56; over 512, 2^22
+// 0.37 / 0.48, 2^23 0.61 / 0.51, 2^24 1.15 / 0.55.  A new engine pays 0.1 ms more for the partition buffers: 2^21 0.85 / 0.64,
+// 0.52 / 0.61 and 0.28 / 0.61, 2^23 over 512 ids 0.63 / 0.63.
 static bool wide_eligible(const stbpe_engine *e, bool fresh) {
+    const i64 ids = ids_below(e), least = e->dense32_min >= 0 ? e->dense32_min : ids >= 4096 ? 1ll << 21 : 1ll << 23;
     return e->n_tokens > 0 && e->n_tokens < (1ll << 32) && e->slots <= (1ull << 30) && fresh && !e->only_bytes && e->cfg.base_vocab <= 65536 &&
-           e->n_tokens >= e->dense32_min && !getenv("STBPE_NO_DENSE_COUNT");
+           ids <= 65536 && e->n_tokens >= least && !getenv("STBPE_NO_DENSE_COUNT");
 }
 
 // first pass of the partitioned count; *ok = 0 when an id of 65 536 or more or a full region made it give up

@@ -350,6 +350,28 @@ def test_automatic_table_of_a_stream_of_ids(lg, vocab, slots):
     e.close()
 
 
+@pytest.mark.parametrize("n,top,partitioned", [((1 << 21) - 1, 65535, False), (1 << 21, 65535, True), ((1 << 21) + 1025, 30000, True),
+                                               (1 << 21, 65536, False), (1 << 21, 4094, False), (1 << 21, 4095, True),
+                                               ((1 << 23) - 1, 511, False), ((1 << 23) + 3, 511, True)])
+def test_streams_on_both_sides_of_the_partitioned_count(n, top, partitioned):
+    # rows of one token among long ones, ids up to `top`, most of them small
+    g = torch.Generator("cuda").manual_seed(n + top)
+    ids = (torch.rand(n, device="cuda", generator=g) ** 4 * (top + 1)).to(torch.int32).clamp_(max=top)
+    ids[n // 2] = top
+    starts = torch.unique(torch.cat([torch.randint(1, n, (n // 900,), device="cuda", generator=g), torch.arange(1, 40, device="cuda")]))
+    off = np.concatenate([[0], starts.cpu().numpy(), [n]]).astype(np.int64)
+    e = Engine(n + 77, base_vocab=65536, max_merges=1)
+    e.append_ids(ids, off)
+    e.count_initial()
+    assert (e.state().count_convert_ms > 0) == partitioned
+    keep = torch.ones(n - 1, dtype=torch.bool, device="cuda")
+    keep[starts - 1] = False  # a pair does not reach into the next row
+    ref, rc = torch.unique(((ids[:-1].to(torch.int64) << 32) | ids[1:])[keep], return_counts=True)
+    k, c = e.export_histogram()
+    assert torch.equal(k, ref) and torch.equal(c, rc)
+    e.close()
+
+
 def test_pair_table_grows_in_mid_run():
     # random bytes: every merge makes some hundred pairs that were not there before
     n = 16 << 20
