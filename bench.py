@@ -14,8 +14,9 @@ Printed JSON (one line, rank 0):
   value      merges/s with the corpus already packed in HBM (device time, CUDA events)
   e2e        merges/s through ``GPUBPETrainer.fit_bytes`` from pinned host bytes: H2D copy, pack,
              initial histogram, K merges, merge list back to the host
-  pair_count GB/s of the initial histogram pass at 4 bytes per token
-  roofline   merge kernel: 4 bytes x live tokens per launch / its average device time
+  pair_count GB/s of the initial histogram pass at 4 bytes per token (the metric's definition; the fraction of the
+             HBM rate counts the 2 bytes per token that the stream holds)
+  roofline   merge loop: bytes that its kernel loaded and stored, counted by the kernel, / device time of the loop
   cpu_baseline  the CPU oracle (C restatement of the reference's recount loop) on a bounded sample
 
 ``--impl reference`` times that CPU restatement on the host cores instead (the reference is a
@@ -116,6 +117,27 @@ class ClockSampler:
         except Exception:
             pass
         return out
+
+
+def count_launches(work):
+    """Launches of this repository's kernels by name while `work` runs (untimed: under the profiler), or None when the
+    profiler sees none.  Library kernels (radix sort and scan, torch's own) are left out."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    ran, names = False, {}
+    try:
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            ran = True
+            work()
+            torch.cuda.synchronize()
+        for e in p.events():
+            name = e.name.split("(")[0].split("<")[0].removeprefix("void ").strip()
+            if e.device_type == torch.autograd.DeviceType.CUDA and name.endswith("_kernel") and "::" not in name:
+                names[name] = names.get(name, 0) + 1
+    except RuntimeError:  # no profiler on this machine
+        if not ran:
+            work()
+    return names or None
 
 
 def merges_sha256(merges, counts) -> str:
@@ -295,6 +317,9 @@ def count_bench(wl, dev, K, W, with_e2e=True):
             conv.append(float(st.count_convert_ms))
     clocks = sampler.stop()
     st = eng.state()
+    eng.reset()
+    eng.append_ids(ids, off_np)
+    launches = count_launches(eng.count_initial)
     key, count, ties = eng.select_best(True)
     # size-independent check of the whole histogram: every pair position is counted exactly once
     # (tokens minus non-empty rows), and the exported keys are strictly ascending (no key twice)
@@ -334,15 +359,16 @@ def count_bench(wl, dev, K, W, with_e2e=True):
                    "sum_of_counts_equals_pair_positions": sum_ok,
                    "l2": "inputs larger than L2", "bytes_per_token": 4},
         "roofline": {"bound": "hbm",
-                     "kernel": ("partition_pairs_kernel, sub_partition_kernel, build_table_kernel: all passes, until the pair table is "
-                                "complete") if conv and conv[0] > 0 else "count_kernel",
+                     "kernel": "all passes, until the pair table is complete: " + ", ".join(launches or ["(not profiled)"]),
                      "achieved": gbs, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": gbs / peak,
                      "frac_of_8tbs": gbs / 8000.0, "kernel_ms": med, "second_pass_ms": float(np.median(conv)),
                      "call_ms": float(np.median(call)), "traffic": None},
         "e2e": None if e2e_s is None else {"value": 4.0 * n_tokens / e2e_s / 1e9, "unit": "GB/s", "seconds": e2e_s,
                                            "h2d_bytes_per_step": 4.0 * n_tokens + off_np.nbytes,
                                            "d2h_bytes_per_step": 24.0},
-        "gpu_launches": 3 * K, "clocks": clocks, "cpu_baseline": None,   # first pass, hot pairs, second pass
+        # passes of the partitioned count and the table's set-up, in every step
+        "gpu_launches": K * (sum(launches.values()) if launches else 3), "launches_per_step": launches,
+        "clocks": clocks, "cpu_baseline": None,
     }
     return line
 
@@ -436,6 +462,7 @@ def main():
     tc = ev()
     if M:
         eng.train(M)
+    st_b = eng.state()
     t1 = ev()
     eng.train(K)
     t2 = ev()
@@ -444,30 +471,26 @@ def main():
     count_call_ms = t0.elapsed_time(tc)
     loop_ms = t1.elapsed_time(t2)
     st = eng.state()
-    count_ms = float(st.count_kernel_ms)   # histogram kernel(s) only; the call also clears the table,
-    # builds the tile records, the pair filter and the block maxima
+    count_ms = float(st.count_kernel_ms)   # histogram kernels only; the call also clears the table and builds the tile records
+    # what the loop's kernel loaded and stored during the timed merges
+    tile_bytes = float(st.tile_bytes_in + st.tile_bytes_out) - float(st_b.tile_bytes_in + st_b.tile_bytes_out)
     done = st.merges_done - M
     merges_gpu, counts_gpu, live_before = eng.merges(M, done)
     if done < 1:
         raise SystemExit("no merge was learned")
     value = done / (loop_ms / 1000.0)
 
-    # per-kernel device time of the same K merges (events around every launch)
+    # the kernels of the same region, counted in an untimed repetition
     load()
     eng.count_initial()
     if M:
         eng.train(M)
-    st_b = eng.state()
-    sel_ms, mrg_ms, ref_ms, repack_ms = eng.train_timed(K)
-    torch.cuda.synchronize()
-    st_t = eng.state()
-    # what the merge kernel loaded and stored during the timed merges
-    tile_bytes = float(st_t.tile_bytes_in + st_t.tile_bytes_out) - float(st_b.tile_bytes_in + st_b.tile_bytes_out)
+    launches = count_launches(lambda: eng.train(K))
     merges_again, _, _ = eng.merges(M, eng.state().merges_done - M)
     assert merges_again == merges_gpu, "merge list changed between two runs on the same input"
     algo_bytes = 4.0 * float(live_before.sum())
     peak, peak_kind = peaks()
-    achieved = algo_bytes / (mrg_ms / 1000.0) / 1e9
+    achieved = tile_bytes / (loop_ms / 1000.0) / 1e9
     eng.close()
     del eng
 
@@ -535,24 +558,27 @@ def main():
                    "merges_timed": done, "first_merge": M, "stop_reason": int(st.stop_reason),
                    "merges_sha256": merges_sha256(merges_gpu, counts_gpu),
                    "oracle_prefix_ok": oracle_ok, "oracle_prefix_merges": oracle_n,
-                   "l2": "inputs larger than L2 (4 bytes x tokens per merge)", "tile_tokens": 1024},
+                   "l2": "inputs larger than L2 (2 bytes x tokens per pass over the stream)", "tile_tokens": 1024},
         "pair_count": {"kernel": "count_dense_kernel (byte-level path)", "call_ms": count_call_ms, "ms": count_ms, "gbs": 4.0 * n_tokens / (count_ms / 1e3) / 1e9,
-                       "frac_of_measured_peak": 4.0 * n_tokens / (count_ms / 1e3) / 1e9 / peak,
-                       "frac_of_8tbs": 4.0 * n_tokens / (count_ms / 1e3) / 1e9 / 8000.0,
-                       "bytes_per_token": 4, "distinct_pairs": None},
+                       "bytes_per_token": 4, "stream_gbs": 2.0 * n_tokens / (count_ms / 1e3) / 1e9, "stream_bytes_per_token": 2,
+                       "frac_of_measured_peak": 2.0 * n_tokens / (count_ms / 1e3) / 1e9 / peak,
+                       "frac_of_8tbs": 2.0 * n_tokens / (count_ms / 1e3) / 1e9 / 8000.0, "distinct_pairs": None},
         "pair_count_c3": pair_count_c3,
-        "roofline": {"bound": "hbm", "kernel": "merge_kernel", "achieved": achieved, "peak": peak,
+        "roofline": {"bound": "hbm", "kernel": "loop_kernel", "achieved": achieved, "peak": peak,
                      "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
-                     "algorithmic_bytes": algo_bytes, "kernel_ms": mrg_ms, "launches": done,
-                     "other_kernels_ms": {"select_kernel": sel_ms, "refresh_kernel": ref_ms, "repack": repack_ms},
+                     "kernel_ms": loop_ms, "kernel_ms_note": "the whole timed region: loop_kernel, the candidate kernels in front "
+                                                             "of its launches, maintenance between them",
                      "traffic": tile_bytes / done,
-                     "traffic_note": "bytes per launch that the kernel loaded and stored in this run (tiles of 16-bit tokens and tile "
-                                     "records read + rewritten units and records stored, counted by the kernel); "
-                                     "the ncu summaries under profiles/ give dram__bytes for the same kernel"},
+                     "traffic_note": "bytes per merge that loop_kernel loaded and stored in the timed run (tiles of 16-bit tokens and "
+                                     "tile records read + rewritten units and records stored, counted by the kernel); "
+                                     "one pass over the stream takes several merges",
+                     "algorithmic_bytes": algo_bytes, "algorithmic_note": "4 bytes x live tokens before every merge",
+                     "algorithmic_gbs": algo_bytes / (loop_ms / 1000.0) / 1e9},
         "e2e": {"value": e2e, "unit": "merges/s", "seconds": e2e_s,
                 "h2d_bytes_per_step": (n_tokens + off_np.nbytes) / max(len(learned), 1),
                 "d2h_bytes_per_step": 24.0},
-        "gpu_launches": 7,   # at least: table clear, count, its transfer to the table, three for the candidates, the loop
+        "gpu_launches": sum(launches.values()) if launches else 4,   # (three for the candidates and the loop, at least)
+        "launches": launches,
         "clocks": clocks,
         "cpu_baseline": cpu,
     }

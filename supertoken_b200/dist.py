@@ -587,7 +587,9 @@ def run_bench_multi(args, wl, rank: int, local_rank: int, world: int) -> None:
     if rank == 0:
         from bench import merges_sha256, peaks  # type: ignore
         peak, peak_kind = peaks()
-        algo = 4.0 * float(live_all.item())
+        # bytes of live tokens before every merge, in the width that the stream has (16 bits while all ids of the job fit 15)
+        width = 2 if 256 + K < 32767 else 4
+        algo = width * float(live_all.item())
         line = {
             "metric": "bpe_merges_per_sec", "value": done / (loop_ms / 1e3), "unit": "merges/s",
             "n_gpus": world, "steps": done, "warmup": W, "ms_per_step": loop_ms / max(done, 1),
@@ -601,13 +603,13 @@ def run_bench_multi(args, wl, rank: int, local_rank: int, world: int) -> None:
                        "round_driver": {"peer": "kernels over NVLink peer memory, CUDA graph of 16 rounds (stbpe_mg_peer_run)",
                                         "nccl": "native NCCL loop (stbpe_mg_run)",
                                         "python": "python rounds over torch.distributed"}[driver],
-                       "l2": "inputs larger than L2 (4 bytes x tokens per merge)", "tile_tokens": 1024},
+                       "l2": "inputs larger than L2 (2 or 4 bytes x tokens per merge)", "tile_tokens": 1024},
             "pair_count": {"ms": count_ms, "gbs": 4.0 * float(tokens_all.item()) / (count_ms / 1e3) / 1e9,
                            "note": "local histogram + all-to-all + owner insert + first decision"},
             "roofline": {"bound": "hbm", "kernel": "merge round (all kernels and the exchange)",
                          "achieved": algo / (loop_ms / 1e3) / 1e9, "peak": peak * world, "peak_kind": peak_kind,
                          "unit": "GB/s", "frac": algo / (loop_ms / 1e3) / 1e9 / (peak * world),
-                         "algorithmic_bytes": algo, "traffic": None},
+                         "algorithmic_bytes": algo, "bytes_per_token": width, "traffic": None},
             "e2e": {"value": done2 / e2e_s, "unit": "merges/s", "seconds": e2e_s,
                     "h2d_bytes_per_step": float(tokens_all.item()) / max(done2, 1), "d2h_bytes_per_step": 24.0},
             "gpu_launches": rounds * launches_per_round,
