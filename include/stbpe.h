@@ -59,12 +59,12 @@ typedef struct stbpe_state {
     int32_t n_tiles;
     int64_t fixups;           /* matches whose dropped token sits in another tile than their head (statistics) */
     int64_t repacks;          /* dense re-packs of the stream so far */
-    int64_t work_tiles;       /* tiles visited by the last merge (after the pair filter) */
+    int64_t work_tiles;       /* tiles visited by the last step, of up to eight merges (after the pair filter; < 0 = all) */
     double count_kernel_ms;   /* device time of the histogram kernel(s) of the last count; on the
-                                 16-bit-vocabulary path both passes, i.e. until the pair table is complete */
-    double count_convert_ms;  /* 16-bit-vocabulary path only: the part of count_kernel_ms spent in the
-                                 second pass (per-partition counting and table inserts; 0 otherwise) */
-    int64_t tile_bytes_in;    /* merge kernel, since the last load: bytes of tiles and tile records read ... */
+                                 16-bit-vocabulary path all passes, i.e. until the pair table is complete */
+    double count_convert_ms;  /* 16-bit-vocabulary path only: the part of count_kernel_ms behind the
+                                 first pass (ordering the words and building the table; 0 otherwise) */
+    int64_t tile_bytes_in;    /* merges, since the last load: bytes of tiles and tile records read ... */
     int64_t tile_bytes_out;   /* ... and bytes of rewritten tile parts and records stored (statistics) */
 } stbpe_state;
 
@@ -85,7 +85,8 @@ int stbpe_trim(int32_t device, int64_t keep_bytes);
 int stbpe_flatten_rows(const int32_t *tokens, const uint8_t *valid, int64_t rows, int64_t width, int32_t elem,
                        void *out, int64_t *lengths);
 
-/* Ingest: pack rows into the flat int32 token stream (bit 31 = first token of a row).
+/* Ingest: pack rows into the token stream (16 bits per token while every id is below 32 767, else 32; the top bit
+ * marks the first token of a row).
  * Replaces BytePacker.encode_view + the batcher fill + GPUBatchRecord.from_cpu
  * (gpu_tokenizer/cpu_packer.py:17-61, datasets.py:75-84, bpe_trainer.py:137-222).
  * Rows are appended after the rows of earlier calls; empty rows own no pair and
@@ -135,14 +136,15 @@ int stbpe_next_tied(stbpe_engine *e, int32_t a, int32_t b, int32_t new_id, int32
  * stop rule fires.  Synchronises the stream before returning. */
 int stbpe_train(stbpe_engine *e, int32_t n_merges, void *stream);
 
-/* stbpe_train with one launch per choice and merge and CUDA events around each: kernel_ms[0..3]
- * receive the summed device time of the select, merge and refresh kernels and of the re-packs.  Measurement aid
+/* The merges of stbpe_train one at a time, with CUDA events around each choice and each merge_kernel launch: kernel_ms[0],
+ * [1] and [3] receive the summed device time of the choices (with the host's look at each), the merges and the re-packs,
+ * kernel_ms[2] zero.  Its times are not those of stbpe_train, which takes several merges per step in one launch.  Measurement aid
  * for the per-stage timings the reference records (gpu_tokenizer/bpe_trainer.py:4249-4260,
  * :4385-4396). */
 int stbpe_train_timed(stbpe_engine *e, int32_t n_merges, float *kernel_ms, void *stream);
 
 /* Dense re-pack of the token stream (tiles only shrink; stbpe_train does this by itself whenever
- * at most half of the tile capacity in use is live).  force != 0 re-packs regardless.  *did (may
+ * at most three quarters of the tile capacity in use are live).  force != 0 re-packs regardless.  *did (may
  * be NULL) reports whether it happened.  Replaces nothing in the reference, whose rows are
  * re-compacted by every merge (gpu_tokenizer/utils.py:347-410). */
 int stbpe_repack(stbpe_engine *e, int force, int *did, void *stream);

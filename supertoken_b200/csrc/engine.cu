@@ -706,7 +706,7 @@ static int prepare_stream_state(stbpe_engine *e, cudaStream_t s) {
 }
 
 __global__ void clear_skip_state_kernel(EngineDev e, int valid) {
-    e.st->n_work = 0;  // a merge that is committed but not yet applied builds its worklist from here
+    e.st->n_work = 0;  // a merge that is committed but not yet applied counts its tiles from here
     e.st->filter_valid = valid;
 }
 
@@ -1493,8 +1493,8 @@ STBPE_VISIBLE int stbpe_train(stbpe_engine *e, int32_t n_merges, void *stream) {
     return run_loop(e, (int)target, LOOP_BEST, nullptr, make_int2(0, 0), 0, 0, &h, s);
 }
 
-// Same loop as stbpe_train, launched kernel by kernel with CUDA events around every launch so
-// that a caller can attribute device time to the three kernels (select / merge / refresh).
+// The merges of stbpe_train one at a time: choose_kernel with the host's look at its result, then merge_kernel, with CUDA
+// events around both.
 STBPE_VISIBLE int stbpe_train_timed(stbpe_engine *e, int32_t n_merges, float *kernel_ms, void *stream) {
     if (!e || n_merges < 0 || !kernel_ms) return STBPE_E_BADARG;
     cudaStream_t s = (cudaStream_t)stream;
@@ -1512,7 +1512,7 @@ STBPE_VISIBLE int stbpe_train_timed(stbpe_engine *e, int32_t n_merges, float *ke
     e->merges_known = false;
     const int P = 128;
     DevState h2;
-    std::vector<cudaEvent_t> ev(4 * P);
+    std::vector<cudaEvent_t> ev(3 * P);
     for (auto &x : ev) CK(cudaEventCreate(&x));
     kernel_ms[0] = kernel_ms[1] = kernel_ms[2] = kernel_ms[3] = 0.f;
     int rc = STBPE_OK;
@@ -1547,23 +1547,22 @@ STBPE_VISIBLE int stbpe_train_timed(stbpe_engine *e, int32_t n_merges, float *ke
             if (rc != STBPE_OK) break;
         }
         for (int i = 0; i < n && rc == STBPE_OK; ++i) {
-            cudaEventRecord(ev[4 * i], s);
+            cudaEventRecord(ev[3 * i], s);
             rc = choose(e, true, &h2, s);
-            cudaEventRecord(ev[4 * i + 1], s);
+            cudaEventRecord(ev[3 * i + 1], s);
             if (rc == STBPE_OK && e->table_auto && (i64)h2.n_keys + 131072 > (i64)(e->slots / 4)) {
                 rc = grow_table(e, s);  // every merge adds at most two pairs per id of the vocabulary
                 if (rc == STBPE_OK) rc = refill_candidates(e, s);
             }
             if (rc != STBPE_OK) break;
             rc = launch_merge(e, false, s);
-            cudaEventRecord(ev[4 * i + 2], s);
-            cudaEventRecord(ev[4 * i + 3], s);
+            cudaEventRecord(ev[3 * i + 2], s);
         }
         cudaStreamSynchronize(s);
         for (int i = 0; i < n && rc == STBPE_OK; ++i)
-            for (int k = 0; k < 3; ++k) {
+            for (int k = 0; k < 2; ++k) {
                 float ms = 0.f;
-                cudaEventElapsedTime(&ms, ev[4 * i + k], ev[4 * i + k + 1]);
+                cudaEventElapsedTime(&ms, ev[3 * i + k], ev[3 * i + k + 1]);
                 kernel_ms[k] += ms;
             }
     }

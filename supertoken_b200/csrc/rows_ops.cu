@@ -524,8 +524,8 @@ STBPE_VISIBLE int stbpe_rows_apply_merge(int32_t *tokens, uint8_t *valid, int32_
 // ---------------------------------------------------------------------------------------
 // Pair counting for callers that must not allocate.
 //
-// stbpe_rows_count_pairs above takes its hash table, staging arrays and sort workspace from
-// the stream-ordered allocator on every call.  Two kinds of caller of this library cannot
+// stbpe_rows_count_pairs above takes its hash table, staging arrays and sort workspace from the
+// process-wide block cache, which allocates when it holds nothing that fits.  Two kinds of caller of this library cannot
 // afford that.  The reference's trainer sizes its batches to fill device memory (its
 // --target-util flag) and hands every byte to preallocated workspaces before the merge loop
 // starts, so an allocation made in the middle of the loop is the one that fails; and it

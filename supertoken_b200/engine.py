@@ -168,13 +168,14 @@ class Engine:
         self._check(self._lib.stbpe_train(self._h, int(n_merges), self._s))
 
     def train_timed(self, n_merges: int):
-        """Like ``train`` but returns device milliseconds spent in (select, merge, refresh)."""
+        """The merges of ``train`` one at a time; returns device milliseconds spent in (choices with the host's look at
+        each, merges, 0, re-packs)."""
         ms = (ctypes.c_float * 4)()
         self._check(self._lib.stbpe_train_timed(self._h, int(n_merges), ms, self._s))
         return float(ms[0]), float(ms[1]), float(ms[2]), float(ms[3])
 
     def repack(self, force: bool = False) -> bool:
-        """Dense re-pack of the stream if at most half of the tile capacity is live (or forced)."""
+        """Dense re-pack of the stream if at most three quarters of the tile capacity are live (or forced)."""
         did = ctypes.c_int(0)
         self._check(self._lib.stbpe_repack(self._h, int(force), ctypes.byref(did), self._s))
         return bool(did.value)

@@ -127,7 +127,7 @@ def select_best_pair(histogram: PairHistogramResult, *,
                      ) -> Tuple[Optional[int], int, Optional[int]]:
     """Best ``(key, count, index)`` of an exported histogram: highest count, ties to the smallest
     key or to ``tie_breaker(candidate_indices, keys)`` (``trainers/bpe_gpu.py:96-130``).  Works on
-    the small exported tensors; inside the engine the same rule runs in ``select_kernel``."""
+    the small exported tensors; inside the engine the same rule runs in ``loop_kernel``."""
     if histogram.is_empty():
         return None, 0, None
     counts, keys = histogram.counts, histogram.keys

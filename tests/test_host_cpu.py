@@ -155,7 +155,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 REFERENCE = os.environ.get("STBPE_REFERENCE_DIR") or os.path.join(os.path.dirname(os.path.dirname(_HERE)), "reference")
 
 
-@pytest.mark.skipif(not os.path.isdir(REFERENCE), reason="needs the reference checkout")
+@pytest.mark.skipif(not os.path.isdir(os.path.join(REFERENCE, "gpu_tokenizer")), reason="needs the reference checkout")
 def test_drop_in_seam_of_the_reference_command_line(tmp_path, monkeypatch):
     """The swap a maintainer makes: rebind ``GPUBPETrainer`` in the reference's modules, then use the
     reference's own ``train-bpe`` parser and trainer factory (``main.py:21-30``, ``:661-689``, ``:2180-2363``).

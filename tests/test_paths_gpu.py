@@ -230,6 +230,18 @@ def test_untied_runs_with_ids_of_the_stream(seed):
     e.close()
 
 
+def test_timed_merges_are_the_merges_of_train():
+    rng = np.random.RandomState(7)
+    ids = rng.choice(12, 150000, p=rng.dirichlet(np.ones(12))).astype(np.int32)
+    off = _rows(ids, rng, 500)
+    e = _engine(ids, off, 12, 40)
+    choose, merge, none, repack = e.train_timed(25)
+    assert choose > 0 and merge > 0 and none == 0 and repack >= 0
+    e.train(15)
+    _check(e, ids, off, 12, 40)
+    e.close()
+
+
 def test_matches_reported_for_each_host_given_merge():
     # whatever ran before: the matches of this merge alone
     rng = np.random.RandomState(2)
