@@ -14,9 +14,9 @@
 // A second counter keeps the CTAs apart the other way round: a CTA adds its deltas of merge m only when all have
 // read the counts that chose merge m (and CTA 0 has reset the step's counters); that wait runs under the rewriting of
 // the tiles.  Both counters are raised with release and polled with acquire.  (Raised without, `chosen` would rest on
-// loads whose values have been used; the release, by a thread that decides nothing, costs 0 to 0.6 %: 1 MiB of text
-// 2.961 ms instead of 2.947, 256 MiB of mixed text 141.0 instead of 140.7, the first 20 merges of 1 GiB 23.9 either way.
-// By the same thread after the decision: 3.01 instead of 2.96 ms on 1 MiB.)
+// loads whose values have been used.  The release holds up its warp, so it is done while warp 0 decides: 10 MB of
+// mixed text, 3 000 merges, 15.11 ms against 15.08 without any ordering; in front of the ranking, where a CTA barrier waits
+// for that warp, 15.30, and with relaxed polls and a fence behind them 16.5.)
 //
 // A step takes several merges.  Let p1, p2, ... = (a1, b1), (a2, b2), ... be the pairs in selection order (larger count,
 // then smaller key), let no ai be a bj with i != j (of a pair of equal tokens no token may occur elsewhere), and let every
@@ -237,7 +237,6 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             }
         }
         __syncthreads();
-        if (tid == THREADS - 1) red_release_u32(&sync->chosen, 1u);  // this CTA has read all that it decides by
         if constexpr (KB > 1) {
             // place of this warp's candidates among those of all warps
             constexpr int PER = (WARPS * TOP + 31) / 32;
@@ -255,6 +254,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             }
             __syncthreads();
         }
+        if (tid == THREADS - 1) red_release_u32(&sync->chosen, 1u);  // this CTA has read all that it decides by
         // warp 0 decides; the lanes of pair j take the j-th best pair (or the j-th one the host gives) and test whether it
         // can be merge j of the batch, given that all before it are
         if (warp == 0) {
