@@ -1027,6 +1027,7 @@ STBPE_VISIBLE int stbpe_count_initial(stbpe_engine *e, void *stream) {
     cudaStream_t s = (cudaStream_t)stream;
     CK(cudaSetDevice(e->cfg.device));
     if (e->cfg.world_size > 1) return fail(e, STBPE_E_STATE, "use stbpe_mg_count_local on a multi-rank engine");
+    e->counted = false;  // (a recount that finds no memory for a larger table leaves none)
     for (;;) {
         const bool fresh = e->recs_stale;
         int rc = launch_count(e, false, s);
