@@ -141,7 +141,11 @@ struct Best<uint32_t> {
 };
 
 
-template <typename T>
+// FV: FILTER_ON or FILTER_OFF.  PLANES: 15, or 9 on 16-bit tokens for a launch whose ids, old and new, stay below 511 (early
+// merges, the ones that visit every tile): the kernel leaves when the next id would not.  Every tile's 32 x 16 bits per lane
+// are transposed, a quarter of the instructions of the arithmetic pipe that bounds a dense step; nine planes and code
+// without the filter took the first 20 merges of 1 GiB from 20.3 to 16.3 ms (24 warps per SM instead of 20: no faster).
+template <typename T, int FV, int PLANES>
 __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __grid_constant__ EngineDev e, const __grid_constant__ LoopArgs la) {
     typedef Best<T> Bs;
     typedef typename Bs::type Bt;
@@ -166,7 +170,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
     const unsigned int G = gridDim.x, cta = blockIdx.x;
     int merges_done = st->merges_done, forced_i = 0;
     const int base_vocab = st->base_vocab;
-    const bool fv = st->filter_valid != 0;
+    constexpr bool fv = FV == FILTER_ON;  // (the host launches by DevState::filter_valid)
     MergeCtx mc;
     mc.fv = fv;
     mc.theta.count = st->theta_count, mc.theta.key = st->theta_key;
@@ -325,7 +329,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             else if (e.n_tiles >= la.repack_tiles && s_live * 4 <= (i64)e.n_tiles * STBPE_TILE * 3) why = STBPE_EXIT_REPACK;
             else if (!fv && e.n_tiles > 0 && count <= la.filter_count) why = STBPE_EXIT_FILTER;
             else if (s_keys + 2 * made + 2 * (j + 1) > la.grow_keys) why = STBPE_EXIT_GROW;
-            else if (sizeof(T) == 2 && max(nw, max(a, b)) >= Tok<uint16_t>::IDMASK) why = STBPE_EXIT_WIDEN;
+            else if (sizeof(T) == 2 && max(nw, max(a, b)) >= (1u << PLANES) - 1u) why = STBPE_EXIT_WIDEN;
             else go = true;
             const uint32_t bad = __ballot_sync(0xFFFFFFFFu, j >= KB || !go || (j > 0 && out)) | (KB > 1 ? 1u << (2 * KB) : 2u);
             const int nb = lsb(bad) >> (KB > 1 ? 1 : 0);
@@ -368,7 +372,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
         forced_i += nb;
         mc.m = merges_done;
         mc.zero = cta == G - 1;
-        cta_merge<T, false>(e, s, mc, la.unit_shift, [&] {
+        cta_merge<T, false, FV, PLANES>(e, s, mc, la.unit_shift, [&] {
             if (tid == THREADS - 1) {
                 BoundedWait wait;
                 while (ld_acquire_u32(&sync->chosen) < G * (step + 1))

@@ -127,6 +127,9 @@ struct CtaMerge {
     }
 };
 
+// How a kernel knows whether the pair filter is being maintained: compiled for streams without it, with it, or for both.
+enum { FILTER_OFF, FILTER_ON, FILTER_ASK };
+
 struct MergeCtx {
     int m;         // number of the batch's last merge (>= 1)
     bool fv;       // the pair filter is being maintained
@@ -272,17 +275,18 @@ __device__ __forceinline__ int lsb(uint32_t x) { return 31 - __clz(x & (0u - x))
 
 // One warp, one tile (already in the warp's shared-memory slot; every lane reads and writes its own group of
 // 32 tokens only).  `rv`: load_recs3 of the tile; `pm`: the pairs that may occur in it (bit k = pair k).
-template <typename T, bool MG>
+template <typename T, bool MG, int FV, int PLANES>
 __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s, const MergeCtx &c, uint32_t *wm, int lane,
                                            int tile, uint32_t pm, const uint4 &rv, WarpStats &ws) {
     typedef Tok<T> K;
     constexpr bool MANY = Batch<T>::MAX > 1;
+    const bool fv = FV == FILTER_ASK ? c.fv : FV == FILTER_ON;
     T *tok = reinterpret_cast<T *>(wm + lane * K::PITCH);
     const BatchPairs *const P = s.p;
 
     uint32_t L, F;
     Group<T> grp;
-    grp.load(wm + lane * K::PITCH, L, F);
+    grp.template load<PLANES>(wm + lane * K::PITCH, L, F);
     const uint32_t ne = __ballot_sync(0xFFFFFFFFu, L != 0u);
     if (ne == 0u) return;  // every token of the tile is gone
     // the live tokens right before and right behind the tile: from the neighbours' records, or by walking
@@ -313,7 +317,7 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
 #pragma unroll 1
     for (uint32_t left = pm; left; left &= left - 1u) {
         const int k = MANY ? lsb(left) : 0;
-        const uint32_t A = grp.eq(P->pa[k]), B = grp.eq(P->pb[k]) & ~F;  // a partner does not start a row
+        const uint32_t A = grp.template eq<PLANES>(P->pa[k]), B = grp.template eq<PLANES>(P->pb[k]) & ~F;  // a partner does not start a row
         const uint32_t d = next_live_bits(A, H) & B;
         D |= d;
         if (A & top) firsts |= 1u << k;
@@ -450,7 +454,7 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
                     reds_add_s32(&s.p->touch[i * 8 + k], 1);
                 else
                     key_h = Batch<T>::key(id, 0u, (uint32_t)k);
-                if (c.fv) filter_set(e, tile, tile2, ((u64)(i >= 0 ? P->nw[i] : id) << 32) | nw);
+                if (fv) filter_set(e, tile, tile2, ((u64)(i >= 0 ? P->nw[i] : id) << 32) | nw);
             }
         }
         if (at_e >= 0) {
@@ -480,7 +484,7 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
             }
             if (!skip) {
                 key_e = Batch<T>::key(id, 1u, (uint32_t)k);
-                if (c.fv) filter_set(e, tile, tile2, made_key(P, (uint32_t)k, id, 1u));
+                if (fv) filter_set(e, tile, tile2, made_key(P, (uint32_t)k, id, 1u));
             }
         }
         agg_add2<T, MG>(s, e, c, key_h, key_e);
@@ -503,12 +507,12 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
             const int i = find_pair(P, y, h.nxt[2]);
             if (i < P->n) {
                 // y's tile counts the two touching matches, but sees the dropped token only, not the new one here
-                if (c.fv) filter_set(e, tile, -1, ((u64)P->nw[kt] << 32) | P->nw[i]);
+                if (fv) filter_set(e, tile, -1, ((u64)P->nw[kt] << 32) | P->nw[i]);
             } else if (!(y & STBPE_FLAG)) {
                 agg_add<T, MG>(s, e, c, Batch<T>::key(y, 1u, (uint32_t)kt));
-                if (c.fv) filter_set(e, tile, h.next2_tile, made_key(P, kt, y, 1u));
+                if (fv) filter_set(e, tile, h.next2_tile, made_key(P, kt, y, 1u));
             }
-        } else if (c.fv) {
+        } else if (fv) {
             // a run of a's that goes on in the next tile: the pair that will start at the collapsed token is
             // decided by whoever finds the run's tail, so visit this tile from now on
             atomicOr(e.presence + (size_t)((unsigned int)tile >> 5) * STBPE_PPITCH + STBPE_PROWS, 1u << (tile & 31));
@@ -584,22 +588,23 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
 // c + gridDim.x, ... (words of the filter when there are enough of them, single tiles on a small stream).
 // Ends with all of the CTA's adds issued; the caller synchronises.
 // `before_adds`: called by every thread between the tiles and the CTA-wide barrier in front of the table adds.
-template <typename T, bool MG, typename F>
+template <typename T, bool MG, int FV, int PLANES, typename F>
 __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s, const MergeCtx &c, int unit_shift, F &&before_adds) {
     constexpr int WARPS = MergeGeom<T>::WARPS;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t *wm = s.warp_mem + (size_t)warp * MergeGeom<T>::WARP_WORDS;
     WarpStats ws = {0, 0, 0, 0, 0};
+    const bool fv = FV == FILTER_ASK ? c.fv : FV == FILTER_ON;
     const int nb = Batch<T>::MAX > 1 ? s.p->n : 1;
-    if (!c.fv) __syncthreads();  // the pairs are in place (with the filter, the barriers of the list come first)
+    if (!fv) __syncthreads();  // the pairs are in place (with the filter, the barriers of the list come first)
     // Without the filter: every tile, consecutive tiles on different CTAs so that a small stream uses all of
     // them.  With it: batches of filter units, each turned into a list of tiles that the warps share.
-    const i64 n_units = c.fv ? ((i64)e.n_tiles + (1 << unit_shift) - 1) >> unit_shift : blockIdx.x + 1;
+    const i64 n_units = fv ? ((i64)e.n_tiles + (1 << unit_shift) - 1) >> unit_shift : blockIdx.x + 1;
     const uint32_t unit_bits = (1u << (1 << unit_shift)) - 1u;
 #pragma unroll 1
     for (i64 u0 = blockIdx.x; u0 < n_units; u0 += (i64)STBPE_LIST_UNITS * gridDim.x) {
         int n = (e.n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;  // tiles blockIdx.x, + gridDim.x, ...
-        if (c.fv) {
+        if (fv) {
             // one thread per pair and unit asks the filter ...
             int lg = 2;
             while (lg < 8 && u0 + ((i64)gridDim.x << lg) < n_units) ++lg;
@@ -645,19 +650,19 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
         int cur = -1;
         uint32_t pairs = (1u << nb) - 1u, next_pairs = pairs;
 #pragma unroll 1
-        for (int j = warp, taken = 0;; j = c.fv ? __shfl_sync(0xFFFFFFFFu, taken, 0) + WARPS : j + WARPS) {
+        for (int j = warp, taken = 0;; j = fv ? __shfl_sync(0xFFFFFFFFu, taken, 0) + WARPS : j + WARPS) {
             if (cur >= 0) store_units<T>(wm, lane, v);
             const uint4 rc = rv;
-            const int next = j < n ? (c.fv ? (int)s.list[j] : (int)blockIdx.x + j * (int)gridDim.x) : -1;
+            const int next = j < n ? (fv ? (int)s.list[j] : (int)blockIdx.x + j * (int)gridDim.x) : -1;
             if (next >= 0) {
-                if (c.fv) next_pairs = s.list_pairs[j];
+                if (fv) next_pairs = s.list_pairs[j];
                 load_units<T>(e, next, lane, v);
                 rv = load_recs3(e, next, lane);
-                if (c.fv && lane == 0) taken = atoms_add_s32(&s.ctr[CTR_NEXT], 1);
+                if (fv && lane == 0) taken = atoms_add_s32(&s.ctr[CTR_NEXT], 1);
             }
             __syncwarp();
             if (cur >= 0) {
-                merge_tile<T, MG>(e, s, c, wm, lane, cur, pairs, rc, ws);
+                merge_tile<T, MG, FV, PLANES>(e, s, c, wm, lane, cur, pairs, rc, ws);
                 ws.tiles += 1;
                 __syncwarp();
             }
@@ -665,7 +670,7 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
             pairs = next_pairs;
             if (cur < 0) break;
         }
-        if (c.fv) {
+        if (fv) {
             __syncthreads();
             if (threadIdx.x == 0) s.ctr[CTR_LIST] = s.ctr[CTR_NEXT] = 0;
             if (u0 + (i64)STBPE_LIST_UNITS * gridDim.x < n_units) __syncthreads();
@@ -734,7 +739,7 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
             if (k == CTR_SEAM) atomicAdd(&st->n_fixups, (unsigned int)x);
             if (k == CTR_FRESH && !MG) atomicAdd(&st->n_keys, (u64)x);
             if (k == CTR_TILES) {
-                if (c.fv) atomicAdd(&st->n_work, x);
+                if (fv) atomicAdd(&st->n_work, x);
                 atomicAdd(&st->tile_bytes_in, (u64)x * (STBPE_TILE * sizeof(T) + 2 * sizeof(TileRec)));
             }
             if (k == CTR_UNITS) atomicAdd(&st->tile_bytes_out, (u64)x * 16);
@@ -762,5 +767,5 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) merge_kernel(const _
     if (!c.fv && blockIdx.x == 0 && threadIdx.x == 0) st->n_work = -1;
     __syncthreads();
     if (threadIdx.x < 32) s.p->set_plane<T>(0, (int)threadIdx.x);
-    cta_merge<T, MG>(e, s, c, unit_shift, [] {});
+    cta_merge<T, MG, FILTER_ASK, 15>(e, s, c, unit_shift, [] {});
 }

@@ -110,6 +110,9 @@ struct Group<uint16_t> {
             }
         }
     }
+    // PLANES: bits of an id that are looked at; 15, or fewer where every id lies below 2^PLANES - 1 (the planes between
+    // them and the last one are then equal to the holes and need not be worked out)
+    template <int PLANES>
     __device__ __forceinline__ void load(const uint32_t *group, uint32_t &L, uint32_t &F) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -120,23 +123,27 @@ struct Group<uint16_t> {
         exchange<4>(0x0F0F0F0Fu);
         exchange<2>(0x33333333u);
         exchange<1>(0x55555555u);
-        uint32_t hole = w[0] & w[1] & w[2];
+        uint32_t hole = w[14];
+        if (PLANES == 15) {
 #pragma unroll
-        for (int i = 3; i < 15; i += 2) hole &= w[i] & w[i + 1];  // only a hole has all 15 low bits set
+            for (int i = 0; i < 14; i += 2) hole &= w[i] & w[i + 1];  // only a hole has all 15 low bits set
+        }
         L = ~hole, F = w[15];
     }
+    template <int PLANES>
     __device__ __forceinline__ uint32_t eq(const PlaneId &id) const {
         const uint4 m0 = id.m[0], m1 = id.m[1], m2 = id.m[2], m3 = id.m[3];
         const uint32_t m[15] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w, m2.x, m2.y, m2.z, m2.w, m3.x, m3.y, m3.z};
         uint32_t r = ~(w[0] ^ m[0]);
 #pragma unroll
-        for (int i = 1; i < 15; ++i) r &= ~(w[i] ^ m[i]);
+        for (int i = 1; i < PLANES; ++i) r &= ~(w[i] ^ m[i]);
         return r;
     }
 };
 template <>
 struct Group<uint32_t> {
     uint32_t w[32];
+    template <int>
     __device__ __forceinline__ void load(const uint32_t *group, uint32_t &L, uint32_t &F) {
         L = F = 0;
 #pragma unroll
@@ -151,6 +158,7 @@ struct Group<uint32_t> {
             w[i] &= STBPE_IDMASK;
         }
     }
+    template <int>
     __device__ __forceinline__ uint32_t eq(const PlaneId &p) const {
         const uint32_t id = p.m[0].x;
         uint32_t m = 0;

@@ -85,6 +85,22 @@ def test_stream_widens_while_training_and_while_appending(top):
     e.close()
 
 
+@pytest.mark.parametrize("base_vocab,largest,tiles", [(505, 504, 8193), (511, 510, 8192), (509, 510, 8192), (505, 511, 8192), (505, 504, 8191)])
+def test_new_ids_pass_nine_bits(base_vocab, largest, tiles, filter_mode):
+    # long streams without the pair filter look at nine bits of an id while all lie below 511: the new ids reach that in
+    # mid-run, at once, or an id of the stream is there already
+    if filter_mode == "filter_always":
+        pytest.skip("streams without the filter")
+    rng = np.random.RandomState(base_vocab + largest + tiles)
+    n = tiles * 1024 - 100
+    ids = rng.choice(np.array([1, 2, 3, 255, 256, largest], dtype=np.int32), n, p=[0.3, 0.25, 0.2, 0.15, 0.06, 0.04])
+    off = _rows(ids, rng, 4000)
+    e = _engine(ids, off, base_vocab, 12)
+    e.train(12)
+    _check(e, ids, off, base_vocab, 12)
+    e.close()
+
+
 @pytest.mark.parametrize("above,wide", [(1, False), (0, True), (-1000, True)])
 def test_counts_that_16_bit_tokens_leave_no_room_for(above, wide, monkeypatch):
     # the limit, 2^34 in earnest, one above the largest count, at it and below it
