@@ -219,6 +219,7 @@ __device__ __forceinline__ void agg_add(const CtaMerge &s, const EngineDev &e, c
     else
         agg_probe<T, MG>(s.agg_key, s.ctr, e, s.p, c.theta.count, c.theta.key, key);
 }
+
 // two at once (STBPE_NONE: no neighbour): the look-ups overlap, and the lanes that have to probe for either do it together
 template <typename T, bool MG>
 __device__ __forceinline__ void agg_add2(const CtaMerge &s, const EngineDev &e, const MergeCtx &c, uint32_t key0, uint32_t key1) {
@@ -273,6 +274,11 @@ __device__ __forceinline__ uint32_t pick_recs(const uint4 &rv, int m) {
 // the rate of ordinary instructions.)
 __device__ __forceinline__ int lsb(uint32_t x) { return 31 - __clz(x & (0u - x)); }
 
+template <int S>
+struct SideTag {
+    static constexpr int value = S;
+};
+
 // One warp, one tile (already in the warp's shared-memory slot; every lane reads and writes its own group of
 // 32 tokens only).  `rv`: load_recs3 of the tile; `pm`: the pairs that may occur in it (bit k = pair k).
 template <typename T, bool MG, int FV, int PLANES>
@@ -289,28 +295,35 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
     grp.template load<PLANES>(wm + lane * K::PITCH, L, F);
     const uint32_t ne = __ballot_sync(0xFFFFFFFFu, L != 0u);
     if (ne == 0u) return;  // every token of the tile is gone
-    // the live tokens right before and right behind the tile: from the neighbours' records, or by walking
-    // when they hold too few tokens
-    Halo h;
-    const uint32_t second = pick_recs(rv, c.m);
-    const int lp = second & 4u ? 2 : 0, ln = second & 0x400u ? 10 : 8;
-    const uint32_t enough = __ballot_sync(0xFFFFFFFFu, (int)rv.y >= (lane < 4 ? 2 : 3));
-    const bool near = (enough >> lp) & (enough >> ln) & 1u;
-    if (near) {
-        h.prev = __shfl_sync(0xFFFFFFFFu, rv.y, lp + 1);
-        h.nxt[0] = __shfl_sync(0xFFFFFFFFu, rv.z, ln);
-        h.prev_tile = tile - 1;
-        h.next_tile = h.next2_tile = tile + 1;
-    } else {
-        Halo walked;
-        gather_halo(e, tile, c.m, walked);
-        h = walked;
-    }
     const uint32_t H = ~L;
     const uint32_t low = L & (0u - L);                       // this lane's first live token ...
     const uint32_t top = L ? 0x80000000u >> __clz(L) : 0u;   // ... and its last
     const uint32_t above = ne & ~((2u << lane) - 1u), below = ne & ((1u << lane) - 1u);
     const int up = lsb(above), down = 31 - __clz(below);  // the next lanes that hold live tokens, if any
+    // The live tokens right before and right behind the tile: from the neighbours' records, or by walking when they hold
+    // too few tokens.  A sparse visit reads them when it turns out to need them; in a dense one most tiles do, and the
+    // shuffles run beside the comparisons (first 20 merges of 1 GiB 16.5 ms, 17.4 where they are read late).
+    Halo h;
+    uint32_t second = 0;  // pick_recs of the tile
+    auto read_halo = [&] {
+        second = pick_recs(rv, c.m);
+        const int lp = second & 4u ? 2 : 0, ln = second & 0x400u ? 10 : 8;
+        const uint32_t enough = __ballot_sync(0xFFFFFFFFu, (int)rv.y >= (lane < 4 ? 2 : 3));
+        if ((enough >> lp) & (enough >> ln) & 1u) {
+            h.prev = __shfl_sync(0xFFFFFFFFu, rv.y, lp + 1);
+            h.prev2 = __shfl_sync(0xFFFFFFFFu, rv.z, lp + 1);
+            h.nxt[0] = __shfl_sync(0xFFFFFFFFu, rv.z, ln);
+            h.nxt[1] = __shfl_sync(0xFFFFFFFFu, rv.w, ln);
+            h.nxt[2] = __shfl_sync(0xFFFFFFFFu, rv.x, ln + 1);
+            h.prev_tile = tile - 1;
+            h.next_tile = h.next2_tile = tile + 1;
+        } else {
+            Halo walked;
+            gather_halo(e, tile, c.m, walked);
+            h = walked;
+        }
+    };
+    if (FV != FILTER_ON) read_halo();
     // Dropped tokens: positions of some b_k whose previous live position holds a_k.  k0, k1, k2: bits of k there.
     uint32_t D = 0, k0 = 0, k1 = 0, k2 = 0;
     uint32_t firsts = 0, seconds = 0;  // pairs whose a is this lane's last token, whose b is its first
@@ -330,72 +343,85 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
     }
     // heads: the previous live position of every dropped one
     uint32_t M = prev_live_bits(D, H);
-    // matches across lanes and tiles: kt = pair of the one that this lane's last token heads, kl = of the one whose
-    // partner is its first, -1 for none
+    // matches across lanes: kt = pair of the one that this lane's last token heads, kl = of the one whose partner is its
+    // first, -1 for none
+    auto drop_first = [&](int k) {
+        D |= low;
+        if (MANY) {
+            if (k & 1) k0 |= low;
+            if (k & 2) k1 |= low;
+            if (k & 4) k2 |= low;
+        }
+    };
     int kt = -1, kl = -1;
     {
-        uint32_t both = firsts & __shfl_sync(0xFFFFFFFFu, seconds, above ? up : lane);
-        if (!above) {
-            both = 0;
+        const uint32_t both = firsts & __shfl_sync(0xFFFFFFFFu, seconds, above ? up : lane);
+        if (above && both) kt = lsb(both), M |= top;
+        kl = __shfl_sync(0xFFFFFFFFu, kt, below ? down : lane);
+        if (!below) kl = -1;
+        if (L != 0u && kl >= 0) drop_first(kl);
+    }
+    // ---- the tile's edges: what stands beyond them matters, and the tile's record changes, only when one of the first
+    // three or last two live tokens is touched or could belong to a match with the tile next to it
+    const int first_lane = lsb(ne), last_lane = 31 - __clz(ne);
+    const uint32_t l2 = L & ~low, l3 = l2 & (l2 - 1u), low3 = L & ~(l3 & (l3 - 1u));
+    const uint32_t t2 = L & ~top, top2 = top | (t2 ? 0x80000000u >> __clz(t2) : 0u);
+    const bool edge = (lane == first_lane && (!l3 || ((M | D) & low3) || seconds)) || (lane == last_lane && (!t2 || ((M | D) & top2) || firsts));
+    const bool edges = __any_sync(0xFFFFFFFFu, edge);
+    bool last_head = false;  // the last token's partner sits in another tile
+    bool carry_in = false;   // this lane's first token is the partner of a token in another tile
+    if (edges) {
+        if (FV == FILTER_ON) read_halo();
+        if (lane == last_lane) {
+            uint32_t both = 0;
             for (uint32_t o = firsts; o; o &= o - 1u)
                 if (h.nxt[0] == P->b[lsb(o)]) both = o & (0u - o);
+            if (both) kt = lsb(both), M |= top;
         }
-        if (both) kt = lsb(both), M |= top;
-        kl = __shfl_sync(0xFFFFFFFFu, kt, below ? down : lane);
-        if (!below) {
-            kl = -1;
+        if (lane == first_lane) {
             for (uint32_t o = seconds; o; o &= o - 1u)
                 if ((h.prev & STBPE_IDMASK) == P->a[lsb(o)]) kl = lsb(o);
+            if (kl >= 0) carry_in = true, drop_first(kl);
         }
-        if (L != 0u && kl >= 0) {
-            D |= low;
-            if (MANY) {
-                if (kl & 1) k0 |= low;
-                if (kl & 2) k1 |= low;
-                if (kl & 4) k2 |= low;
-            }
-        }
+        last_head = (__ballot_sync(0xFFFFFFFFu, kt >= 0) >> last_lane) & 1u;
     }
-    const bool carry_in = below == 0u && kl >= 0;
-    const uint32_t hb = __ballot_sync(0xFFFFFFFFu, kt >= 0);
     const uint32_t touched = M | D;
     if (__ballot_sync(0xFFFFFFFFu, touched != 0u) == 0u) return;  // nothing to merge here
     ws.removed += __popc(D);
-    const int first_lane = lsb(ne), last_lane = 31 - __clz(ne);
-    const bool last_head = ((hb >> last_lane) & 1u) != 0u;  // its partner sits in another tile
-    if (near) {
-        h.prev2 = __shfl_sync(0xFFFFFFFFu, rv.z, lp + 1);
-        h.nxt[1] = __shfl_sync(0xFFFFFFFFu, rv.w, ln);
-        h.nxt[2] = __shfl_sync(0xFFFFFFFFu, rv.x, ln + 1);
-    }
     const uint32_t heads = M & ~D;  // (a position in both is inside a run of equal tokens)
     const uint32_t ends = D & ~M;   // last tokens of matches and runs
     // of a match whose head sits in the tile before, the head's tile takes care (of a run, the last token's tile)
     const uint32_t own = ends & ~(carry_in && P->a[kl] != P->b[kl] ? low : 0u);
-    // ---- the neighbours whose pairs change.  Heads (left neighbours) and own ends (right neighbours) are shared out over
-    // the lanes, one of each per lane and round, whatever group they sit in.  What a lane has to know of another's group
-    // it reads from shared memory.  Tokens that are read as neighbours are never rewritten: in front of a head stands
-    // no head, a dropped token counts by its pair, and a head behind an end is skipped.
-    // (Every lane walking over its own matches, first the heads, then the ends, waited for the fullest lane: an early batch
-    // has 1 to 2.5 matches per lane, the fullest lane four to eight.  First 20 merges of 1 GiB 23.9 ms, now 20.3; 8 000
-    // merges of 256 MiB 134 ms, now 125.)
+    // ---- the neighbours whose pairs change.  Heads (left neighbours) and own ends (right neighbours) go through a list
+    // and are taken 32 at a time, one per lane, whatever group they sit in and whichever of the two they are.  What a
+    // lane has to know of another's group it reads from shared memory.  Tokens that are read as neighbours are never
+    // rewritten: in front of a head stands no head, a dropped token counts by its pair, and a head behind an end is skipped.
+    // (A visit has 2.4 matches on average over the 8 000 merges of a 256 MiB corpus, mostly in lanes of their own: a lane that
+    // takes its head and then its end holds up the warp for both.  Every lane walking
+    // over its own matches waited for the fullest lane: first 20 merges of 1 GiB 23.9 ms instead of 20.3.)
     uint4 *const sa = reinterpret_cast<uint4 *>(wm + MergeGeom<T>::RAW_WORDS), *const sb = sa + 32;
     T *const all = reinterpret_cast<T *>(wm);
     sa[lane] = make_uint4(L, D, k0, k1);
     sb[lane] = make_uint4(k2, F, heads, (uint32_t)kt);
-    uint16_t *const list_h = reinterpret_cast<uint16_t *>(sb + 32), *const list_e = list_h + STBPE_TILE / 2;
-    int at_h = heads ? lane * 32 + 31 - __clz(heads) : -1, at_e = own ? lane * 32 + 31 - __clz(own) : -1;
-    int total = 0;
-    if (__any_sync(0xFFFFFFFFu, ((heads & (heads - 1u)) | (own & (own - 1u))) != 0u)) {  // some lane has several
-        const uint32_t n = (uint32_t)__popc(heads) | ((uint32_t)__popc(own) << 16);
-        uint32_t incl = n;
+    uint16_t *const list = reinterpret_cast<uint16_t *>(sb + 32);
+    uint32_t at, sum;  // places in front of this lane's, places in all: heads, and ends in the upper half
+    {
+        if (__any_sync(0xFFFFFFFFu, ((heads & (heads - 1u)) | (own & (own - 1u))) != 0u)) {  // some lane has several
+            const uint32_t n = (uint32_t)__popc(heads) | ((uint32_t)__popc(own) << 16);
+            at = n;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-            if (lane >= d) incl += o;
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, at, d);
+                if (lane >= d) at += o;
+            }
+            sum = __shfl_sync(0xFFFFFFFFu, at, 31);
+            at -= n;
+        } else {
+            const uint32_t hb = __ballot_sync(0xFFFFFFFFu, heads != 0u), eb = __ballot_sync(0xFFFFFFFFu, own != 0u), lt = (1u << lane) - 1u;
+            at = (uint32_t)__popc(hb & lt) | ((uint32_t)__popc(eb & lt) << 16);
+            sum = (uint32_t)__popc(hb) | ((uint32_t)__popc(eb) << 16);
         }
-        const uint32_t sum = __shfl_sync(0xFFFFFFFFu, incl, 31), at = incl - n;
-        uint16_t *lh = list_h + (at & 0xFFFFu), *le = list_e + (at >> 16);
+        uint16_t *lh = list + (at & 0xFFFFu), *le = list + (sum & 0xFFFFu) + (at >> 16);
         uint32_t oh = heads, oe = own;
 #pragma unroll 1
         while (oh | oe) {
@@ -407,91 +433,78 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
             if (oe) {
                 const int r = 31 - __clz(oe);
                 oe ^= 1u << r;
-                *le++ = (uint16_t)(lane * 32 + r);
+                *le++ = (uint16_t)(STBPE_TILE + lane * 32 + r);
             }
         }
-        __syncwarp();
-        at_h = lane < (int)(sum & 0xFFFFu) ? (int)list_h[lane] : -1;
-        at_e = lane < (int)(sum >> 16) ? (int)list_e[lane] : -1;
-        total = (int)sum;
     }
     __syncwarp();
     auto pair_at = [&](const uint4 &x, uint32_t x2, int r) {
         return MANY ? (int)(((x.z >> r) & 1u) | (((x.w >> r) & 1u) << 1) | (((x2 >> r) & 1u) << 2)) : 0;
     };
+    // One entry of the list: rewrites the token and returns its neighbour's key.  SIDE: 0 a head, 1 an end, 2 either.
+    auto visit = [&](int item, auto side) -> uint32_t {
+        constexpr int SIDE = decltype(side)::value;
+        const int at = item & (STBPE_TILE - 1), l = at >> 5, q = at & 31;
+        const bool end = SIDE == 2 ? item >= STBPE_TILE : SIDE == 1;
+        uint4 x = sa[l], y = sb[l];
+        const uint32_t over = x.x & ~((2u << q) - 1u), under = x.x & ((1u << q) - 1u);
+        const int k = !MANY ? 0 : end || over ? pair_at(x, y.x, end ? q : lsb(over)) : (int)y.w;
+        const uint32_t nw = P->nw[k];
+        const bool starts = !end && ((y.y >> q) & 1u);  // first of its row: no left neighbour
+        all[K::sindex(at)] = (T)(end ? K::HOLE : nw | (starts ? K::FLAG : 0u));
+        if (starts) return STBPE_NONE;
+        uint32_t n = end ? over : under;
+        int ln = l;
+        if (!n) {
+            const uint32_t lanes = end ? ne & ~((2u << l) - 1u) : ne & ((1u << l) - 1u);
+            if (lanes) {
+                ln = end ? lsb(lanes) : 31 - __clz(lanes);
+                x = sa[ln], y = sb[ln];
+                n = x.x;
+            }
+        }
+        uint32_t id;
+        int i = -1, tile2 = -1;  // pair of the match that ends in front of this one; tile of the neighbour, if another
+        if (n) {
+            const int p = end ? lsb(n) : 31 - __clz(n);
+            id = (uint32_t)all[K::sindex(ln * 32 + p)] & K::IDMASK;
+            if (((end ? y.y | y.z : x.y) >> p) & 1u) {
+                if (end) return STBPE_NONE;  // another row, or the head of a match, which counts the pair
+                i = pair_at(x, y.x, p);
+            }
+        } else if (end) {
+            id = h.nxt[0];
+            if ((id & STBPE_FLAG) || find_pair(P, id, h.nxt[1]) < P->n) return STBPE_NONE;
+            tile2 = h.next_tile;
+        } else {
+            id = h.prev & STBPE_IDMASK;
+            const int j = find_pair(P, h.prev2 & STBPE_IDMASK, h.prev);
+            if (j < P->n) i = j;
+            tile2 = h.prev_tile;
+        }
+        if (fv) filter_set(e, tile, tile2, made_key(P, (uint32_t)k, i >= 0 ? P->nw[i] : id, end));
+        if (i < 0) return Batch<T>::key(id, end, (uint32_t)k);
+        reds_add_s32(&s.p->touch[i * 8 + k], 1);
+        return STBPE_NONE;
+    };
+    // Many matches in the tile: a head and an end per lane and round, each by code of its own, which is less of it (first 20
+    // merges of 1 GiB 16.65 ms, 17.6 with either); with the filter, hardly any tile has as many.
+    const int n_heads = (int)(sum & 0xFFFFu), n_ends = (int)(sum >> 16);
+    if (FV != FILTER_ON && n_heads + n_ends > 32) {
 #pragma unroll 1
-    for (int base = 0;;) {
-        uint32_t key_h = STBPE_NONE, key_e = STBPE_NONE;
-        if (at_h >= 0) {
-            const int l = at_h >> 5, q = at_h & 31;
-            uint4 x = sa[l], y = sb[l];
-            const uint32_t next = x.x & ~((2u << q) - 1u);
-            uint32_t prev = x.x & ((1u << q) - 1u);
-            const int k = !MANY ? 0 : next ? pair_at(x, y.x, lsb(next)) : (int)y.w;
-            const uint32_t nw = P->nw[k];
-            const bool starts = (y.y >> q) & 1u;
-            all[K::sindex(at_h)] = (T)(nw | (starts ? K::FLAG : 0u));
-            if (!starts) {
-                int lp = l, i = -1, tile2 = -1;
-                const uint32_t down_lanes = ne & ((1u << l) - 1u);
-                if (!prev && down_lanes) {
-                    lp = 31 - __clz(down_lanes);
-                    x = sa[lp], y.x = sb[lp].x;
-                    prev = x.x;
-                }
-                uint32_t id;
-                if (prev) {
-                    const int p = 31 - __clz(prev);
-                    id = (uint32_t)all[K::sindex(lp * 32 + p)] & K::IDMASK;
-                    if ((x.y >> p) & 1u) i = pair_at(x, y.x, p);
-                } else {
-                    id = h.prev & STBPE_IDMASK;
-                    const int j = find_pair(P, h.prev2 & STBPE_IDMASK, h.prev);
-                    if (j < P->n) i = j;
-                    tile2 = h.prev_tile;
-                }
-                if (i >= 0)
-                    reds_add_s32(&s.p->touch[i * 8 + k], 1);
-                else
-                    key_h = Batch<T>::key(id, 0u, (uint32_t)k);
-                if (fv) filter_set(e, tile, tile2, ((u64)(i >= 0 ? P->nw[i] : id) << 32) | nw);
-            }
+        for (int base = lane; base - lane < max(n_heads, n_ends); base += 32) {
+            uint32_t head = STBPE_NONE, end = STBPE_NONE;
+            if (base < n_heads) head = visit((int)list[base], SideTag<0>());
+            if (base < n_ends) end = visit((int)list[n_heads + base], SideTag<1>());
+            agg_add2<T, MG>(s, e, c, head, end);
         }
-        if (at_e >= 0) {
-            const int l = at_e >> 5, r = at_e & 31;
-            const uint4 x = sa[l];
-            uint4 y = sb[l];
-            const int k = pair_at(x, y.x, r);
-            all[K::sindex(at_e)] = (T)K::HOLE;
-            int lu = l, tile2 = -1;
-            uint32_t u = x.x & ~((2u << r) - 1u);
-            const uint32_t up_lanes = ne & ~((2u << l) - 1u);
-            if (!u && up_lanes) {
-                lu = lsb(up_lanes);
-                u = sa[lu].x;
-                y = sb[lu];
+    } else {
+#pragma unroll 1
+        for (int base = lane; base - lane < n_heads + n_ends; base += 32)
+            if (base < n_heads + n_ends) {
+                const uint32_t key = visit((int)list[base], SideTag<2>());
+                if (key != STBPE_NONE) agg_add<T, MG>(s, e, c, key);
             }
-            uint32_t id;
-            bool skip;
-            if (u) {
-                const int p = lsb(u);
-                id = (uint32_t)all[K::sindex(lu * 32 + p)] & K::IDMASK;
-                skip = ((y.y | y.z) >> p) & 1u;
-            } else {
-                id = h.nxt[0];
-                skip = (id & STBPE_FLAG) || find_pair(P, id, h.nxt[1]) < P->n;
-                tile2 = h.next_tile;
-            }
-            if (!skip) {
-                key_e = Batch<T>::key(id, 1u, (uint32_t)k);
-                if (fv) filter_set(e, tile, tile2, made_key(P, (uint32_t)k, id, 1u));
-            }
-        }
-        agg_add2<T, MG>(s, e, c, key_h, key_e);
-        base += 32;
-        if (base >= max(total & 0xFFFF, total >> 16)) break;
-        at_h = base + lane < (total & 0xFFFF) ? (int)list_h[base + lane] : -1;
-        at_e = base + lane < (total >> 16) ? (int)list_e[base + lane] : -1;
     }
     // dropped tokens that are no end of this tile's: inside a run, or of a match that starts in the tile before
 #pragma unroll 1
@@ -535,10 +548,7 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
         if (last_head) ws.seam += 1;
     }
     // ---- the record, unless the tile's first three and last two live tokens are as they were
-    const uint32_t l2 = L & ~low, l3 = l2 & (l2 - 1u), low3 = L & ~(l3 & (l3 - 1u));
-    const uint32_t t2 = L & ~top, top2 = top | (t2 ? 0x80000000u >> __clz(t2) : 0u);
-    const bool edge_ok = (lane != first_lane || (l3 && !(touched & low3))) && (lane != last_lane || (t2 && !(touched & top2)));
-    if (!__all_sync(0xFFFFFFFFu, edge_ok)) {
+    if (edges) {
         // readers of this merge never pick a record stamped m, so payload and stamp need no ordering
         uint32_t *r = reinterpret_cast<uint32_t *>(e.recs + 2 * (i64)tile + ((second & 0x40u) ? 0 : 1));
         const uint32_t ne2 = __ballot_sync(0xFFFFFFFFu, NL != 0u), n2 = NL & (NL - 1u), n3 = n2 & (n2 - 1u);

@@ -435,3 +435,25 @@ def test_seam_count_at_its_table_and_rank_limits(rows, width, alphabet):
     assert np.array_equal(got.cpu().numpy().astype(np.uint64), ok) and np.array_equal(counts[:n].cpu().numpy(), oc)
     best = ops.select_best_pair(ops.PairHistogramResult(got.contiguous(), counts[:n]))
     assert tuple(best[:2]) == O.select_best(ok, oc)
+
+
+@pytest.mark.parametrize("per", [1, 2, 16, 17, 32, 33, 340])
+def test_tiles_by_their_number_of_matches(per):
+    # few matches per tile go through the lanes one side at a time, more than sixteen with both sides; at a tile's ends the
+    # neighbours come out of the next tile's record
+    rng = np.random.RandomState(per)
+    tiles = 70
+    ids = rng.randint(10, 200, tiles * 1024).astype(np.int32)
+    for t in range(tiles):
+        at = rng.choice(341, per, replace=False) * 3
+        if t % 3 == 0:
+            at[0] = 1022  # ends with the tile ...
+        if t % 3 == 1:
+            at[0] = 1023  # ... or goes over its end
+        for p in t * 1024 + at:
+            ids[p:p + 2] = (1, 2)[:len(ids) - p]
+    off = _rows(ids, rng, 3000)
+    e = _engine(ids, off, 256, 40)
+    e.train(40)
+    _check(e, ids, off, 256, 40)
+    e.close()
