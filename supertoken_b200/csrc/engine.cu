@@ -292,7 +292,10 @@ static const DeviceInfo &device_info(int dev) {
     SMEM((merge_kernel<uint32_t, false>), MergeGeom<uint32_t>::BYTES);
     SMEM((merge_kernel<uint32_t, true>), MergeGeom<uint32_t>::BYTES);
     SMEM((loop_kernel<uint16_t, FILTER_OFF, 9>), optin - 4096);
+    SMEM((loop_kernel<uint16_t, FILTER_OFF, 11>), optin - 4096);
     SMEM((loop_kernel<uint16_t, FILTER_OFF, 15>), optin - 4096);
+    SMEM((loop_kernel<uint16_t, FILTER_ON, 11>), optin - 4096);
+    SMEM((loop_kernel<uint16_t, FILTER_ON, 13>), optin - 4096);
     SMEM((loop_kernel<uint16_t, FILTER_ON, 15>), optin - 4096);
     SMEM((loop_kernel<uint32_t, FILTER_OFF, 15>), optin - 4096);
     SMEM((loop_kernel<uint32_t, FILTER_ON, 15>), optin - 4096);
@@ -1388,7 +1391,7 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
             if (rc != STBPE_OK) return rc;
         }
     }
-    bool ids_grown = false;  // an id of nine bits or more is due
+    int planes_due = 0;  // the next id needs more planes than this
     for (;;) {
         const int grid = e->sm_count;  // one CTA per SM; the barrier is no faster with fewer
         la.target = target;
@@ -1403,9 +1406,16 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
         la.ids_below = (int)std::min(ids_below(e), (i64)0x7FFFFFFF);
         la.unit_shift = unit_shift(e, grid);
         EngineDev d = e->d;
-        // nine planes of every group are enough while all ids are below 511.  The kernel leaves for the next id, which costs a
-        // launch (some 40 us); a step over 8192 tiles takes 25 us and a tenth of it is saved.
-        const bool few_planes = !e->wide && !e->filter_valid && !ids_grown && la.ids_below < 511 && e->d.n_tiles >= 8192;
+        // Bits of an id that the loop looks at: as few as all ids, old and new, allow.  It returns for the id that needs more,
+        // which costs a launch (some 40 us): nine bits only where steps are long (over 8192 tiles one takes 25 us and a tenth
+        // of it is saved), thirteen where the filter is in use (8 000 merges of 256 MiB: 68 million visits, 2 % off each).
+        int planes = 15;
+        if (!e->wide) {
+            auto enough = [&](int p) { return p > planes_due && la.ids_below < (1 << p) - 1; };
+            if (!e->filter_valid && e->d.n_tiles >= 8192 && enough(9)) planes = 9;
+            else if (enough(11)) planes = 11;
+            else if (e->filter_valid && enough(13)) planes = 13;
+        }
         // Candidates that have run out are collected in front of the launch without waiting for the result: one pass
         // settles the threshold but for tables with very many equal counts, and then the launch comes back at once.
         const bool queued = e->cand_stale;
@@ -1419,9 +1429,10 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
         void *args[2] = {&d, &la};
         const cudaError_t c = with_tok(e, [&](auto t) {
             typedef decltype(t) T;
-            const void *kernel = e->filter_valid ? (const void *)loop_kernel<T, FILTER_ON, 15>
-                                 : few_planes    ? (const void *)loop_kernel<uint16_t, FILTER_OFF, 9>
-                                                 : (const void *)loop_kernel<T, FILTER_OFF, 15>;
+            const void *kernel = e->filter_valid ? (const void *)loop_kernel<T, FILTER_ON, 15> : (const void *)loop_kernel<T, FILTER_OFF, 15>;
+            if (planes == 9) kernel = (const void *)loop_kernel<uint16_t, FILTER_OFF, 9>;
+            if (planes == 11) kernel = e->filter_valid ? (const void *)loop_kernel<uint16_t, FILTER_ON, 11> : (const void *)loop_kernel<uint16_t, FILTER_OFF, 11>;
+            if (planes == 13) kernel = (const void *)loop_kernel<uint16_t, FILTER_ON, 13>;
             return cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(MergeGeom<T>::THREADS), args,
                                                MergeGeom<T>::BYTES + STBPE_CAND_CAP * sizeof(unsigned int), s);
         });
@@ -1451,8 +1462,8 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
             rc = maybe_repack(e, false, nullptr, s);
         } else if (out->run_exit == STBPE_EXIT_FILTER) {
             rc = rebuild_presence(e, s);
-        } else if (few_planes) {
-            ids_grown = true;
+        } else if (planes < 15) {
+            planes_due = planes;
         } else {
             rc = widen_stream(e, s);
             if (rc == STBPE_OK) rc = filter_policy(e, *out, true, s);

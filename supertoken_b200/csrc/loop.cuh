@@ -141,10 +141,11 @@ struct Best<uint32_t> {
 };
 
 
-// FV: FILTER_ON or FILTER_OFF.  PLANES: 15, or 9 on 16-bit tokens for a launch whose ids, old and new, stay below 511 (early
-// merges, the ones that visit every tile): the kernel leaves when the next id would not.  Every tile's 32 x 16 bits per lane
-// are transposed, a quarter of the instructions of the arithmetic pipe that bounds a dense step; nine planes and code
-// without the filter took the first 20 merges of 1 GiB from 20.3 to 16.3 ms (24 warps per SM instead of 20: no faster).
+// FV: FILTER_ON or FILTER_OFF.  PLANES: 15, or fewer on 16-bit tokens for a launch whose ids, old and new, all stay below
+// 2^PLANES - 1; the kernel leaves when the next id would not.  Every tile's 32 x 16 bits per lane are transposed, a quarter of
+// the instructions of a dense step and an eighth of a sparse one, and every pair is compared plane by plane.  Nine planes
+// and code without the filter took the first 20 merges of 1 GiB from 20.3 to 16.3 ms (24 warps per SM instead of 20: no
+// faster); eleven, then thirteen, 8 000 merges of 256 MiB from 121.6 to 118.3 ms.
 template <typename T, int FV, int PLANES>
 __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __grid_constant__ EngineDev e, const __grid_constant__ LoopArgs la) {
     typedef Best<T> Bs;

@@ -101,6 +101,19 @@ def test_new_ids_pass_nine_bits(base_vocab, largest, tiles, filter_mode):
     e.close()
 
 
+@pytest.mark.parametrize("base_vocab,largest", [(2041, 2040), (2047, 2046), (2045, 2046), (2041, 2047), (8185, 8184), (8191, 8190), (8185, 8191),
+                                                (2041, 8190)])
+def test_new_ids_pass_eleven_and_thirteen_bits(base_vocab, largest):
+    # with and without the filter: the new ids need another bit in mid-run or at once, or an id of the stream is above them
+    rng = np.random.RandomState(base_vocab + largest)
+    ids = rng.choice(np.array([1, 2, 3, 1023, 1024, largest], dtype=np.int32), 70000, p=[0.3, 0.25, 0.2, 0.15, 0.06, 0.04])
+    off = _rows(ids, rng, 700)
+    e = _engine(ids, off, base_vocab, 24)
+    e.train(24)
+    _check(e, ids, off, base_vocab, 24)
+    e.close()
+
+
 @pytest.mark.parametrize("above,wide", [(1, False), (0, True), (-1000, True)])
 def test_counts_that_16_bit_tokens_leave_no_room_for(above, wide, monkeypatch):
     # the limit, 2^34 in earnest, one above the largest count, at it and below it
