@@ -161,7 +161,6 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
     __shared__ int s_go;                  // merges in this step's batch
     __shared__ unsigned int s_err;        // device error bits
     __shared__ int s_ok;                  // every wait so far succeeded
-    __shared__ int s_work;                // CTA 0: tiles the last merge visited
     CtaMerge s;
     unsigned int *s_cand = reinterpret_cast<unsigned int *>(s.carve<T>(smem_raw, s_ctr));  // slots of the candidates
     s.clear();
@@ -177,9 +176,9 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
     mc.theta.count = st->theta_count, mc.theta.key = st->theta_key;
     unsigned int n_cand = 0;  // candidates this CTA knows
     if (tid == 0) s_ok = 1;
+    WarpStats ws = {0, 0, 0, 0, 0};
+    int visited = 0;  // tiles of this CTA in the last step
     if (cta == 0 && tid == 32) {
-        s_work = st->n_work;
-        st->n_work = 0;
         if (la.mode != LOOP_BEST) st->n_matches = 0;
         la.other_sync->arrived = la.other_sync->chosen = 0;
     }
@@ -235,10 +234,6 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
                 s_live = (i64)__ldcg((const u64 *)&st->n_live);
                 s_keys = (i64)__ldcg(&st->n_keys);
                 s_err = __ldcg(&st->error) | (n > STBPE_CAND_CAP || __ldcg(&st->cand_state) != STBPE_CAND_READY ? 0x80000000u : 0u);
-                if (cta == 0 && step > 0) {
-                    s_work = fv ? __ldcg(&st->n_work) : -1;
-                    st->n_work = 0;
-                }
             }
         }
         __syncthreads();
@@ -360,20 +355,25 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
                     st->peek_count = best.count;
                     st->peek_valid = !dry;
                     st->forced_done = forced_i;
-                    st->n_work = s_work;
+                    if (!fv && step > 0) st->n_work = -1;
                 }
             }
         }
         __syncthreads();
         const int nb = s_go;
         if (tid < 32 * nb) s.p->set_plane<T>(tid >> 5, lane);  // (barriers of cta_merge come before they are read)
-        if (nb == 0 || !s_ok) return;
+        if (nb == 0 || !s_ok) {
+            if (fv && tid == 0 && visited) atomicAdd(&st->n_work, visited);
+            add_stats<T>(e, ws);
+            return;
+        }
+        if (cta == 0 && tid == 0 && step == 0) st->n_work = 0;
         // ---- the merges
         merges_done += nb;
         forced_i += nb;
         mc.m = merges_done;
         mc.zero = cta == G - 1;
-        cta_merge<T, false, FV, PLANES>(e, s, mc, la.unit_shift, [&] {
+        visited = cta_merge<T, false, FV, PLANES>(e, s, mc, la.unit_shift, ws, [&] {
             if (tid == THREADS - 1) {
                 BoundedWait wait;
                 while (ld_acquire_u32(&sync->chosen) < G * (step + 1))
@@ -384,7 +384,6 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             }
         });
         // ---- grid barrier: every delta is in the table
-        __syncthreads();
         if (tid == 0) {
             red_release_u32(&sync->arrived, 1u);
             BoundedWait wait;

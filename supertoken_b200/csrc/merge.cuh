@@ -83,7 +83,7 @@ struct MergeGeom {
     static constexpr size_t BYTES = (size_t)WARPS * WARP_WORDS * 4 + (size_t)STBPE_AGG * 10 + STBPE_LIST * 5 + STBPE_LIST_UNITS * Batch<T>::MAX + sizeof(BatchPairs);
 };
 
-enum { CTR_LIST, CTR_NEXT, CTR_AGG, CTR_REMOVED, CTR_SEAM, CTR_FRESH, CTR_TILES, CTR_UNITS, CTR_RECS, CTR_N };
+enum { CTR_LIST, CTR_NEXT, CTR_AGG, CTR_REMOVED, CTR_FRESH, CTR_N };
 
 struct CtaMerge {
     uint32_t *warp_mem;    // WARPS x WARP_WORDS
@@ -251,10 +251,30 @@ __device__ __forceinline__ int find_pair(const BatchPairs *p, uint32_t x, uint32
     return k;
 }
 
-struct WarpStats {  // per lane
+struct WarpStats {  // per lane, over all steps of a launch but for `removed`
     int removed, seam, units, recs;
-    int tiles;  // per warp
+    i64 tiles;  // of the CTA
 };
+// Statistics of a launch into the device state.  Called by the whole CTA at its end.
+template <typename T>
+__device__ __forceinline__ void add_stats(const EngineDev &e, const WarpStats &ws) {
+    __shared__ u64 sums[3];
+    if (threadIdx.x < 3) sums[threadIdx.x] = 0;
+    __syncthreads();
+    const unsigned int part[3] = {(unsigned int)ws.seam, (unsigned int)ws.units, (unsigned int)ws.recs};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const u64 lo = __reduce_add_sync(0xFFFFFFFFu, part[k] & 0xFFFFu), hi = __reduce_add_sync(0xFFFFFFFFu, part[k] >> 16);
+        if ((threadIdx.x & 31) == 0 && (lo | hi)) atomicAdd(&sums[k], lo + (hi << 16));
+    }
+    __syncthreads();
+    DevState *st = e.st;
+    if (threadIdx.x == 0) {
+        if (sums[0]) atomicAdd(&st->n_fixups, (unsigned int)sums[0]);
+        if (ws.tiles) atomicAdd(&st->tile_bytes_in, (u64)ws.tiles * (STBPE_TILE * sizeof(T) + 2 * sizeof(TileRec)));
+        if (sums[1] | sums[2]) atomicAdd(&st->tile_bytes_out, sums[1] * 16 + sums[2] * sizeof(TileRec));
+    }
+}
 
 // the records of tiles tile - 1, tile, tile + 1 (two versions each, 192 consecutive bytes), 16 bytes per lane
 __device__ __forceinline__ uint4 load_recs3(const EngineDev &e, int tile, int lane) {
@@ -596,14 +616,15 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
 // Applies the batch of merges to this CTA's tiles and adds its delta terms to the pair table (or, several ranks, to
 // the rank-local delta table).  `unit_shift`: log2 of the tiles per filter unit; CTA c takes the units c,
 // c + gridDim.x, ... (words of the filter when there are enough of them, single tiles on a small stream).
-// Ends with all of the CTA's adds issued; the caller synchronises.
+// Returns the tiles it visited.  Ends behind a CTA-wide barrier with all of the CTA's adds issued, the last ones by thread 0.
 // `before_adds`: called by every thread between the tiles and the CTA-wide barrier in front of the table adds.
 template <typename T, bool MG, int FV, int PLANES, typename F>
-__device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s, const MergeCtx &c, int unit_shift, F &&before_adds) {
+__device__ __forceinline__ int cta_merge(const EngineDev &e, const CtaMerge &s, const MergeCtx &c, int unit_shift, WarpStats &ws, F &&before_adds) {
     constexpr int WARPS = MergeGeom<T>::WARPS;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t *wm = s.warp_mem + (size_t)warp * MergeGeom<T>::WARP_WORDS;
-    WarpStats ws = {0, 0, 0, 0, 0};
+    ws.removed = 0;
+    int visited = 0;
     const bool fv = FV == FILTER_ASK ? c.fv : FV == FILTER_ON;
     const int nb = Batch<T>::MAX > 1 ? s.p->n : 1;
     if (!fv) __syncthreads();  // the pairs are in place (with the filter, the barriers of the list come first)
@@ -615,6 +636,11 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
     for (i64 u0 = blockIdx.x; u0 < n_units; u0 += (i64)STBPE_LIST_UNITS * gridDim.x) {
         int n = (e.n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;  // tiles blockIdx.x, + gridDim.x, ...
         if (fv) {
+            if (u0 != blockIdx.x) {  // the list before this one has been worked off
+                __syncthreads();
+                if (threadIdx.x == 0) s.ctr[CTR_LIST] = s.ctr[CTR_NEXT] = 0;
+                __syncthreads();
+            }
             // one thread per pair and unit asks the filter ...
             int lg = 2;
             while (lg < 8 && u0 + ((i64)gridDim.x << lg) < n_units) ++lg;
@@ -654,49 +680,51 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
             __syncthreads();
             n = s.ctr[CTR_LIST];
         }
+        visited += n;
         // the loads of a tile are issued before the one before it is worked on; of a list, a warp takes the
         // next tile that is left (visiting every tile, the warps stay together: fixed shares save an atomic per tile)
+        // (Loading the first tile of a step under the table adds of the one before, where every tile is visited: no faster on a
+        // small stream, and 8 % slower on 1 GiB, for the registers.)
         uint4 v[Tok<T>::VEC], rv;
-        int cur = -1;
-        uint32_t pairs = (1u << nb) - 1u, next_pairs = pairs;
+        int next = -1, taken = 0;
+        uint32_t next_pairs = (1u << nb) - 1u;
+        auto fetch = [&](int j) {
+            next = j < n ? (fv ? (int)s.list[j] : (int)blockIdx.x + j * (int)gridDim.x) : -1;
+            if (next < 0) return;
+            if (fv) next_pairs = s.list_pairs[j];
+            load_units<T>(e, next, lane, v);
+            rv = load_recs3(e, next, lane);
+            if (fv && lane == 0) taken = atoms_add_s32(&s.ctr[CTR_NEXT], 1);
+        };
+        fetch(warp);
 #pragma unroll 1
-        for (int j = warp, taken = 0;; j = fv ? __shfl_sync(0xFFFFFFFFu, taken, 0) + WARPS : j + WARPS) {
-            if (cur >= 0) store_units<T>(wm, lane, v);
+        for (int j = warp; next >= 0;) {
+            const int tile = next;
+            const uint32_t pairs = next_pairs;
             const uint4 rc = rv;
-            const int next = j < n ? (fv ? (int)s.list[j] : (int)blockIdx.x + j * (int)gridDim.x) : -1;
-            if (next >= 0) {
-                if (fv) next_pairs = s.list_pairs[j];
-                load_units<T>(e, next, lane, v);
-                rv = load_recs3(e, next, lane);
-                if (fv && lane == 0) taken = atoms_add_s32(&s.ctr[CTR_NEXT], 1);
-            }
+            store_units<T>(wm, lane, v);
+            j = fv ? __shfl_sync(0xFFFFFFFFu, taken, 0) + WARPS : j + WARPS;
+            fetch(j);
             __syncwarp();
-            if (cur >= 0) {
-                merge_tile<T, MG, FV, PLANES>(e, s, c, wm, lane, cur, pairs, rc, ws);
-                ws.tiles += 1;
-                __syncwarp();
-            }
-            cur = next;
-            pairs = next_pairs;
-            if (cur < 0) break;
-        }
-        if (fv) {
-            __syncthreads();
-            if (threadIdx.x == 0) s.ctr[CTR_LIST] = s.ctr[CTR_NEXT] = 0;
-            if (u0 + (i64)STBPE_LIST_UNITS * gridDim.x < n_units) __syncthreads();
+            merge_tile<T, MG, FV, PLANES>(e, s, c, wm, lane, tile, pairs, rc, ws);
+            __syncwarp();
         }
     }
-    {
-        const int part[5] = {ws.removed, ws.seam, lane == 0 ? ws.tiles : 0, ws.units, ws.recs};
-        constexpr int slot[5] = {CTR_REMOVED, CTR_SEAM, CTR_TILES, CTR_UNITS, CTR_RECS};
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            const int x = __reduce_add_sync(0xFFFFFFFFu, part[k]);
-            if (lane == 0 && x) reds_add_s32(&s.ctr[slot[k]], x);
-        }
-    }
+    ws.tiles += visited;
+    const int removed = __reduce_add_sync(0xFFFFFFFFu, ws.removed);
+    if (lane == 0 && removed) reds_add_s32(&s.ctr[CTR_REMOVED], removed);
     before_adds();
     __syncthreads();
+    DevState *st = e.st;
+    if (threadIdx.x == MergeGeom<T>::THREADS - 1) {
+        s.ctr[CTR_LIST] = s.ctr[CTR_NEXT] = 0;
+        const int x = s.ctr[CTR_REMOVED];
+        s.ctr[CTR_REMOVED] = 0;
+        if (x) {  // one dropped token per match; results unused: reductions
+            atomicAdd((u64 *)&st->n_live, (u64)(-(i64)x));
+            atomicAdd((u64 *)&st->n_matches, (u64)x);
+        }
+    }
     // ---- neighbour histogram -> pair table: two lanes per neighbour, one for the pair that is gone and one for
     // the pair that came into being; behind them, likewise, the matches that touch, and the merged pairs themselves
     constexpr int KB = Batch<T>::MAX, TOUCH = 2 * KB * 8;
@@ -737,25 +765,12 @@ __device__ __forceinline__ void cta_merge(const EngineDev &e, const CtaMerge &s,
     fresh = __reduce_add_sync(0xFFFFFFFFu, fresh);
     if (lane == 0 && fresh) reds_add_s32(&s.ctr[CTR_FRESH], (int)fresh);
     __syncthreads();
-    DevState *st = e.st;
-    if (threadIdx.x < CTR_N) {
-        const int k = threadIdx.x, x = s.ctr[k];
-        s.ctr[k] = 0;
-        if (x) {  // results unused: reductions
-            if (k == CTR_REMOVED) {  // one dropped token per match
-                atomicAdd((u64 *)&st->n_live, (u64)(-(i64)x));
-                atomicAdd((u64 *)&st->n_matches, (u64)x);
-            }
-            if (k == CTR_SEAM) atomicAdd(&st->n_fixups, (unsigned int)x);
-            if (k == CTR_FRESH && !MG) atomicAdd(&st->n_keys, (u64)x);
-            if (k == CTR_TILES) {
-                if (fv) atomicAdd(&st->n_work, x);
-                atomicAdd(&st->tile_bytes_in, (u64)x * (STBPE_TILE * sizeof(T) + 2 * sizeof(TileRec)));
-            }
-            if (k == CTR_UNITS) atomicAdd(&st->tile_bytes_out, (u64)x * 16);
-            if (k == CTR_RECS) atomicAdd(&st->tile_bytes_out, (u64)x * sizeof(TileRec));
-        }
+    if (threadIdx.x == 0) {
+        const int x = s.ctr[CTR_FRESH];
+        s.ctr[CTR_FRESH] = s.ctr[CTR_AGG] = 0;
+        if (x && !MG) atomicAdd(&st->n_keys, (u64)x);
     }
+    return visited;
 }
 
 // One merge as a launch of its own (several ranks, timed runs): the merge that DevState names.
@@ -777,5 +792,8 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) merge_kernel(const _
     if (!c.fv && blockIdx.x == 0 && threadIdx.x == 0) st->n_work = -1;
     __syncthreads();
     if (threadIdx.x < 32) s.p->set_plane<T>(0, (int)threadIdx.x);
-    cta_merge<T, MG, FILTER_ASK, 15>(e, s, c, unit_shift, [] {});
+    WarpStats ws = {0, 0, 0, 0, 0};
+    const int visited = cta_merge<T, MG, FILTER_ASK, 15>(e, s, c, unit_shift, ws, [] {});
+    if (c.fv && threadIdx.x == 0 && visited) atomicAdd(&st->n_work, visited);
+    add_stats<T>(e, ws);
 }
