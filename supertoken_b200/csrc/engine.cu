@@ -546,8 +546,8 @@ static int append_common(stbpe_engine *e, const void *data, i64 n, size_t elem, 
                 if (blocks > (i64)e->sm_count * 32) blocks = (i64)e->sm_count * 32;
                 pack_bytes_kernel<T><<<(unsigned int)blocks, 256, 0, s>>>((const uint8_t *)src, cnt, e->d.tiles, at);
             } else {
-                i64 blocks = (cnt + 255) / 256;
-                if (blocks > (i64)e->sm_count * 32) blocks = (i64)e->sm_count * 32;
+                i64 blocks = (cnt / 16 + 255) / 256 + 1;
+                if (blocks > (i64)e->sm_count * 8) blocks = (i64)e->sm_count * 8;
                 pack_ids_kernel<T><<<(unsigned int)blocks, 256, 0, s>>>((const int32_t *)src, cnt, e->d.tiles, at, bad);
             }
         });

@@ -49,20 +49,71 @@ __global__ void pack_bytes_kernel(const uint8_t *__restrict__ src, i64 n, void *
 // ids must leave the top bit and the hole value free: out-of-range ids raise BAD_ID, ids that only a wider
 // stream can hold NARROW (the host then widens the stream and packs again)
 template <typename T>
-__global__ void pack_ids_kernel(const int32_t *__restrict__ src, i64 n, void *tiles, i64 at, unsigned int *bad) {
+struct PackedIds {
     unsigned int err = 0, largest = 0;
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-        const int32_t v = __ldcs(src + i);
+    __device__ __forceinline__ uint32_t operator()(int32_t v) {
         largest = max(largest, (unsigned int)v & STBPE_IDMASK);
         if (v < 0 || v == 0x7FFFFFFF)
             err |= STBPE_DERR_BAD_ID;
         else if ((uint32_t)v >= Tok<T>::IDMASK)
             err |= STBPE_DERR_NARROW;
-        put_token<T>(tiles, at + i, (uint32_t)v & Tok<T>::IDMASK);
+        return (uint32_t)v & Tok<T>::IDMASK;
     }
-    if (err) atomicOr(bad, err);
-    largest = __reduce_max_sync(0xFFFFFFFFu, largest);
-    if ((threadIdx.x & 31) == 0) atomicMax(bad + 1, largest);  // DevState::max_id
+};
+// Bound by HBM (4 bytes read, 2 or 4 written per id).  Whole groups of the stream are written as 16-byte units, four per thread
+// and turn with all loads in front; what lies before and behind them, and a source that is not 16-byte aligned there, goes
+// token by token.  (All token by token, one load in flight per thread: 200 M ids into 32-bit tokens 0.63 ms, now 0.26.)
+template <typename T>
+__global__ void __launch_bounds__(256) pack_ids_kernel(const int32_t *__restrict__ src, i64 n, void *tiles, i64 at, unsigned int *bad) {
+    PackedIds<T> pack;
+    i64 head = min(n, (32 - (at & 31)) & 31), body = (n - head) & ~(i64)31;
+    if (((uintptr_t)(src + head) & 15) != 0) head = n, body = 0;
+    const i64 tid = (i64)blockIdx.x * blockDim.x + threadIdx.x, stride = (i64)gridDim.x * blockDim.x;
+    {
+        constexpr int PER = 4, LOADS = sizeof(T) == 2 ? 2 : 1;  // units per turn; 16-byte loads per unit
+        const int4 *q = reinterpret_cast<const int4 *>(src + head);
+        uint4 *d = reinterpret_cast<uint4 *>(reinterpret_cast<T *>(tiles) + at + head);
+        const i64 units = body / (4 * LOADS);
+        for (i64 u0 = tid; u0 < units; u0 += PER * stride) {
+            int4 x[PER][LOADS];
+#pragma unroll
+            for (int k = 0; k < PER; ++k) {
+                const i64 u = u0 + k * stride;
+                if (u >= units) break;
+                if (LOADS == 2) {  // unit j of a group: tokens 4j .. 4j + 3 and 16 + 4j .. 16 + 4j + 3
+                    const i64 g = (u >> 2) * 8 + (u & 3);
+                    x[k][0] = __ldcs(q + g), x[k][LOADS - 1] = __ldcs(q + g + 4);
+                } else {
+                    x[k][0] = __ldcs(q + u);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < PER; ++k) {
+                const i64 u = u0 + k * stride;
+                if (u >= units) break;
+                const int4 lo = x[k][0];
+                uint4 w = make_uint4(pack(lo.x), pack(lo.y), pack(lo.z), pack(lo.w));
+                if (LOADS == 2) {
+                    const int4 hi = x[k][LOADS - 1];
+                    w.x |= pack(hi.x) << 16, w.y |= pack(hi.y) << 16, w.z |= pack(hi.z) << 16, w.w |= pack(hi.w) << 16;
+                }
+                d[u] = w;
+            }
+        }
+    }
+    for (i64 k = tid; k < n - body; k += stride) {
+        const i64 i = k < head ? k : k + body;
+        put_token<T>(tiles, at + i, pack(__ldcs(src + i)));
+    }
+    if (pack.err) atomicOr(bad, pack.err);
+    __shared__ unsigned int s_largest[8];
+    const unsigned int largest = __reduce_max_sync(0xFFFFFFFFu, pack.largest);
+    if ((threadIdx.x & 31) == 0) s_largest[threadIdx.x >> 5] = largest;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const unsigned int all = __reduce_max_sync(0xFFFFFFFFu, threadIdx.x < 8 ? s_largest[threadIdx.x] : 0u);
+        if (threadIdx.x == 0) atomicMax(bad + 1, all);  // DevState::max_id
+    }
 }
 
 template <typename T>

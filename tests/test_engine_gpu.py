@@ -524,3 +524,23 @@ def test_repack_keeps_two_stream_buffers_at_most(monkeypatch):
     held -= used()
     # 4 and 2 bytes per token of stream, 65 KB of filter per 32 tiles, 16 MiB of table, records: 128 + 64 + 64 + 16 + 4
     assert 256 < held < 320
+
+
+@pytest.mark.parametrize("base_vocab", [300, 40000])
+@pytest.mark.parametrize("shift", [0, 1, 4])
+@pytest.mark.parametrize("pieces", [(1,), (31, 33), (32, 4097), (5, 70000, 1), (64, 64, 100001)])
+def test_ids_packed_at_any_offset_and_alignment(base_vocab, shift, pieces):
+    # whole groups go as 16-byte units, what lies before and behind them, and a source that is not aligned there, token by token
+    rng = np.random.RandomState(sum(pieces) + shift)
+    n = sum(pieces)
+    ids = rng.randint(0, base_vocab, n).astype(np.int32)
+    dev = torch.zeros(n + 8, dtype=torch.int32, device="cuda")
+    dev[shift:shift + n] = torch.from_numpy(ids)
+    eng = Engine(n, base_vocab=base_vocab, max_merges=1)
+    at = 0
+    for p in pieces:
+        eng.append_ids(dev[shift + at:shift + at + p], np.array([0, p], dtype=np.int64))
+        at += p
+    got, off = eng.export_stream()
+    assert np.array_equal(got, ids) and off.tolist() == [0] + np.cumsum(pieces).tolist()
+    eng.close()
