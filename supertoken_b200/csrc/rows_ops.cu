@@ -15,6 +15,7 @@
 #define ROWS_NT 256
 #define ROWS_IPT 8
 #define ROWS_CHUNK (ROWS_NT * ROWS_IPT)
+#define ROWS_BYTE_PAIRS 65536
 
 namespace {
 
@@ -23,6 +24,7 @@ struct RowsTable {
     u64 mask;
     unsigned int *error;
     u64 *n_keys;
+    u64 *bytes;  // large batches: counters of the pairs of two ids below 256, which are not in the table; else null
 };
 
 __device__ __forceinline__ void rows_table_add(const RowsTable &t, u64 key) {
@@ -69,15 +71,32 @@ __global__ void rows_count_kernel(const int32_t *__restrict__ tokens, const uint
     }
 }
 
+// (also the byte pairs, which then count among the keys)
 __global__ void rows_export_kernel(RowsTable t, u64 *keys, i64 *counts, u64 *n_out, i64 cap) {
-    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i <= t.mask; i += (u64)gridDim.x * blockDim.x) {
-        const Slot s = t.table[i];
-        if (s.key != STBPE_EMPTY) {
-            const u64 j = atomicAdd(n_out, 1ull);
-            if ((i64)j < cap) {
-                keys[j] = s.key;
-                counts[j] = s.count;
-            }
+    const u64 slots = (t.mask | 31u) + 1, all = slots + (t.bytes ? ROWS_BYTE_PAIRS : 0);  // whole warps
+    const int lane = threadIdx.x & 31;
+    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < all; i += (u64)gridDim.x * blockDim.x) {
+        Slot s;
+        s.key = STBPE_EMPTY, s.count = 0;
+        if (i <= t.mask) {
+            s = t.table[i];
+        } else if (i >= slots) {
+            const u64 k = i - slots;
+            s.count = (i64)t.bytes[k];
+            if (s.count) s.key = ((k >> 8) << 32) | (k & 0xFFull);
+        }
+        const bool have = s.key != STBPE_EMPTY;
+        const unsigned int who = __ballot_sync(0xFFFFFFFFu, have);
+        if (!who) continue;
+        u64 at = 0;
+        if (lane == 0) {
+            at = atomicAdd(n_out, (u64)__popc(who));
+            if (i >= slots) atomicAdd(t.n_keys, (u64)__popc(who));
+        }
+        at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(who & ((1u << lane) - 1u));
+        if (have && (i64)at < cap) {
+            keys[at] = s.key;
+            counts[at] = s.count;
         }
     }
 }
@@ -101,12 +120,15 @@ __global__ void rows_write_kernel(const u64 *__restrict__ keys, const i64 *__res
 
 // ---- stbpe_rows_count_pairs
 // Threads and shared-memory slots of a counting CTA.  Small batches: short to clear, and several CTAs per SM.  From 2^18
-// cells on: a table for the some 10^4 pairs that byte-level text holds (a pair that finds no slot is added in L2 by
+// cells on a kernel with one CTA per SM (a pair that finds no slot is added in L2 by
 // itself: with 2048 slots 2048 x 4096 cells of mixed text, 6 900 pairs, took 181 us).
 #define ROWS_SMALL_NT 256
 #define ROWS_SMALL_SLOTS 2048
 #define ROWS_LARGE_NT 1024
-#define ROWS_LARGE_SLOTS 16384
+#define ROWS_LARGE_SLOTS 16384  // of a CTA whose pairs are mostly not of bytes ...
+#define ROWS_MIXED_SLOTS 8192   // ... and beside the byte pairs' counters
+#define ROWS_LARGE_SMEM (ROWS_BYTE_PAIRS * 2 + ROWS_MIXED_SLOTS * 12)
+static_assert(ROWS_LARGE_SLOTS * 12 <= ROWS_LARGE_SMEM, "either layout fits");
 #define ROWS_LARGE_CELLS (1 << 18)
 #define ROWS_RANK_MAX 16384   // up to this many pairs are sorted by counting smaller keys, two launches instead of a radix sort's nine
 #define ROWS_RANK_TILE 512
@@ -118,6 +140,8 @@ __global__ void rows_init_kernel(RowsTable t, unsigned int *rank, unsigned int n
     s.count = 0;
     for (u64 i = first; i <= t.mask; i += step) t.table[i] = s;
     for (u64 i = first; i < n_rank; i += step) rank[i] = 0u;
+    if (t.bytes)
+        for (u64 i = first; i < ROWS_BYTE_PAIRS; i += step) t.bytes[i] = 0;
     if (first < 3) t.n_keys[first] = 0;  // number of keys, error, export cursor
 }
 
@@ -144,25 +168,36 @@ __device__ __forceinline__ void rows_add(const RowsTable &t, u64 key, u64 n) {
     atomicOr(t.error, 1u);
 }
 
-// A pair (i, i+1) of a row counts when both positions are valid (gpu_tokenizer/utils.py:586).  Four cells per thread
-// and step as one 16-byte and one 4-byte load over the flat batch; a CTA collects its pairs in shared memory
-// and adds each distinct one once.
-template <int ROWS_COUNT_NT, int ROWS_SMEM_SLOTS>
-__global__ void __launch_bounds__(ROWS_COUNT_NT) rows_pairs_kernel(const int32_t *__restrict__ tokens, const uint8_t *__restrict__ valid,
-                                                                   i64 B, i64 L, RowsTable t) {
-    extern __shared__ __align__(16) unsigned char s_rows[];
-    u64 *s_key = reinterpret_cast<u64 *>(s_rows);
-    int *s_val = reinterpret_cast<int *>(s_key + ROWS_SMEM_SLOTS);
-    for (int i = threadIdx.x; i < ROWS_SMEM_SLOTS; i += ROWS_COUNT_NT) s_key[i] = STBPE_EMPTY, s_val[i] = 0;
-    __syncthreads();
-    const i64 cells = B * L;
-    const int lane = threadIdx.x & 31;
-    const bool aligned = (((uintptr_t)tokens & 15) | ((uintptr_t)valid & 3)) == 0;
-    const i64 step = (i64)gridDim.x * ROWS_COUNT_NT * 4;
-    i64 q = ((i64)blockIdx.x * ROWS_COUNT_NT + threadIdx.x) * 4;
-    for (i64 q0 = (i64)blockIdx.x * ROWS_COUNT_NT * 4; q0 < cells; q0 += step, q += step) {  // uniform per CTA
-        int32_t w[5] = {0, 0, 0, 0, 0};
-        unsigned int v[5] = {0, 0, 0, 0, 0};
+// key + 1 into a CTA's table, or false where no place is near
+template <unsigned int SLOTS>
+__device__ __forceinline__ bool rows_smem_add(u64 *s_key, int *s_val, u64 key) {
+    unsigned int h = hash32(key) & (SLOTS - 1);
+    bool done = false;
+#pragma unroll 1
+    for (int probe = 0; probe < 4 && !done; ++probe) {
+        u64 x = lds_u64_volatile(&s_key[h]);
+        if (x == STBPE_EMPTY) {
+            x = atoms_cas_u64(&s_key[h], STBPE_EMPTY, key);
+            if (x == STBPE_EMPTY) x = key;
+        }
+        if (x == key) {
+            reds_add_s32(&s_val[h], 1);
+            done = true;
+        }
+        h = (h + 1) & (SLOTS - 1);
+    }
+    return done;
+}
+__device__ __forceinline__ bool rows_byte_pair(u64 key) { return ((uint32_t)(key >> 32) | (uint32_t)key) < 256u; }
+__device__ __forceinline__ unsigned int rows_byte_index(u64 key) { return ((uint32_t)(key >> 32) << 8) | (uint32_t)key; }
+
+// Four cells (and the one behind them) of a flat batch, as one 16-byte and one 4-byte load
+struct RowsQuad {
+    int32_t w[5];
+    unsigned int v[5];
+    __device__ __forceinline__ void load(const int32_t *__restrict__ tokens, const uint8_t *__restrict__ valid, i64 q, i64 cells, bool aligned) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) w[k] = 0, v[k] = 0;
         if (aligned && q + 4 <= cells) {
             const int4 x = __ldg(reinterpret_cast<const int4 *>(tokens + q));
             const uchar4 y = __ldg(reinterpret_cast<const uchar4 *>(valid + q));
@@ -172,39 +207,142 @@ __global__ void __launch_bounds__(ROWS_COUNT_NT) rows_pairs_kernel(const int32_t
             for (int k = 0; k < 4; ++k)
                 if (q + k < cells) w[k] = tokens[q + k], v[k] = valid[q + k];
         }
-        w[4] = __shfl_down_sync(0xFFFFFFFFu, w[0], 1);
-        v[4] = __shfl_down_sync(0xFFFFFFFFu, v[0], 1);
-        if (lane == 31 && q + 4 < cells) w[4] = tokens[q + 4], v[4] = valid[q + 4];
-        i64 col = q < cells ? q - q / L * L : 0;  // column of the first cell
+        if ((threadIdx.x & 31) == 31 && q + 4 < cells) w[4] = tokens[q + 4], v[4] = valid[q + 4];
+    }
+    __device__ __forceinline__ void neighbour() {  // all lanes: the cell behind comes from the next lane
+        const int32_t nw = __shfl_down_sync(0xFFFFFFFFu, w[0], 1);
+        const unsigned int nv = __shfl_down_sync(0xFFFFFFFFu, v[0], 1);
+        if ((threadIdx.x & 31) != 31) w[4] = nw, v[4] = nv;
+    }
+    // f(key) for every pair; `col` = column of the first cell.  A pair (i, i+1) of a row counts when both positions are valid
+    // (gpu_tokenizer/utils.py:586).
+    template <typename F>
+    __device__ __forceinline__ void pairs(i64 col, i64 L, F &&f) const {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const bool last = ++col == L;  // the row ends here
             if (last) col = 0;
-            if (last || !v[k] || !v[k + 1]) continue;
-            const u64 key = ((u64)(uint32_t)w[k] << 32) | (u64)(uint32_t)w[k + 1];
-            unsigned int h = hash32(key) & (ROWS_SMEM_SLOTS - 1);
-            bool done = false;
-#pragma unroll 1
-            for (int probe = 0; probe < 4 && !done; ++probe) {
-                u64 x = lds_u64_volatile(&s_key[h]);
-                if (x == STBPE_EMPTY) {
-                    x = atoms_cas_u64(&s_key[h], STBPE_EMPTY, key);
-                    if (x == STBPE_EMPTY) x = key;
-                }
-                if (x == key) {
-                    reds_add_s32(&s_val[h], 1);
-                    done = true;
-                }
-                h = (h + 1) & (ROWS_SMEM_SLOTS - 1);
-            }
-            if (!done && !(*(volatile unsigned int *)t.error)) rows_add(t, key, 1ull);
+            if (!last && v[k] && v[k + 1]) f(((u64)(uint32_t)w[k] << 32) | (u64)(uint32_t)w[k + 1]);
+            __syncwarp();
         }
     }
+};
+
+// Small batches: a CTA collects its pairs in shared memory and adds each distinct one once.
+__global__ void __launch_bounds__(ROWS_SMALL_NT) rows_pairs_kernel(const int32_t *__restrict__ tokens, const uint8_t *__restrict__ valid, i64 B, i64 L,
+                                                                   RowsTable t) {
+    __shared__ u64 s_key[ROWS_SMALL_SLOTS];
+    __shared__ int s_val[ROWS_SMALL_SLOTS];
+    for (int i = threadIdx.x; i < ROWS_SMALL_SLOTS; i += ROWS_SMALL_NT) s_key[i] = STBPE_EMPTY, s_val[i] = 0;
     __syncthreads();
-    for (int k = threadIdx.x; k < ROWS_SMEM_SLOTS; k += ROWS_COUNT_NT) {  // each CTA from another place on
-        const int i = (k + (int)blockIdx.x * (ROWS_SMEM_SLOTS / 128)) & (ROWS_SMEM_SLOTS - 1);
+    const i64 cells = B * L;
+    const bool aligned = (((uintptr_t)tokens & 15) | ((uintptr_t)valid & 3)) == 0;
+    const i64 step = (i64)gridDim.x * ROWS_SMALL_NT * 4;
+    i64 q = ((i64)blockIdx.x * ROWS_SMALL_NT + threadIdx.x) * 4;
+    for (i64 q0 = (i64)blockIdx.x * ROWS_SMALL_NT * 4; q0 < cells; q0 += step, q += step) {  // uniform per CTA
+        RowsQuad x;
+        x.load(tokens, valid, q, cells, aligned);
+        x.neighbour();
+        x.pairs(q < cells ? q % L : 0, L, [&](u64 key) {
+            if (!rows_smem_add<ROWS_SMALL_SLOTS>(s_key, s_val, key) && !(*(volatile unsigned int *)t.error)) rows_add(t, key, 1ull);
+        });
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < ROWS_SMALL_SLOTS; k += ROWS_SMALL_NT) {  // each CTA from another place on
+        const int i = (k + (int)blockIdx.x * (ROWS_SMALL_SLOTS / 128)) & (ROWS_SMALL_SLOTS - 1);
         if (s_val[i] && !(*(volatile unsigned int *)t.error)) rows_add(t, s_key[i], (u64)s_val[i]);
     }
+}
+
+// Large batches.  Bound by shared memory: a probe of the table costs two or three accesses that collide, an add to a directly
+// indexed counter one, and early in a training nearly all pairs are of two bytes.  So a CTA whose first cells hold mostly
+// such pairs (BYTES) counts them in 65 536 16-bit counters and the others in a smaller table beside them; else all go to one
+// table of the whole room.  Every 15 turns of 4096 cells the counters are added to the batch's, so none overflows.
+// (2048 x 4096 cells of mixed text: a count of 115 us with one table for all, now 60; 65 536 pairs of bytes 840 us for the call, now 230.)
+struct RowsCells {
+    const int32_t *__restrict__ tokens;
+    const uint8_t *__restrict__ valid;
+    i64 cells, L;
+    bool aligned;
+};
+template <bool BYTES>
+__device__ __forceinline__ void rows_count_large(const RowsCells &c, const RowsTable &t, unsigned char *smem) {
+    constexpr unsigned int SLOTS = BYTES ? ROWS_MIXED_SLOTS : ROWS_LARGE_SLOTS;
+    constexpr int TURNS = 65535 / (ROWS_LARGE_NT * 4);
+    unsigned int *const s_count = reinterpret_cast<unsigned int *>(smem);  // two counters per word
+    u64 *const s_key = reinterpret_cast<u64 *>(smem + (BYTES ? ROWS_BYTE_PAIRS * 2 : 0));
+    int *const s_val = reinterpret_cast<int *>(s_key + SLOTS);
+    if (BYTES)
+        for (int i = threadIdx.x; i < ROWS_BYTE_PAIRS / 2; i += ROWS_LARGE_NT) s_count[i] = 0u;
+    for (unsigned int i = threadIdx.x; i < SLOTS; i += ROWS_LARGE_NT) s_key[i] = STBPE_EMPTY, s_val[i] = 0;
+    __syncthreads();
+    // what a CTA has not collected itself
+    auto add = [&](u64 key, u64 n) {
+        if (*(volatile unsigned int *)t.error) return;
+        if (!BYTES && rows_byte_pair(key))
+            atomicAdd(t.bytes + rows_byte_index(key), n);
+        else
+            rows_add(t, key, n);
+    };
+    // (the counters of one first id are spread over the banks, those of neighbouring first ids shifted)
+    auto flush_bytes = [&] {
+        __syncthreads();
+        for (unsigned int k = threadIdx.x; k < ROWS_BYTE_PAIRS / 2; k += ROWS_LARGE_NT) {
+            const unsigned int i = (k + blockIdx.x * (ROWS_BYTE_PAIRS / 256)) & (ROWS_BYTE_PAIRS / 2 - 1);  // each CTA from another place on
+            const unsigned int p = i ^ ((i >> 7) & 31u), x = s_count[p];
+            if (!x) continue;
+            s_count[p] = 0u;
+            if (x & 0xFFFFu) atomicAdd(t.bytes + 2 * i, (u64)(x & 0xFFFFu));
+            if (x >> 16) atomicAdd(t.bytes + 2 * i + 1, (u64)(x >> 16));
+        }
+        __syncthreads();
+    };
+    const i64 step = (i64)gridDim.x * ROWS_LARGE_NT * 4, col_step = step % c.L;
+    i64 q = ((i64)blockIdx.x * ROWS_LARGE_NT + threadIdx.x) * 4, col = q % c.L;
+    int turn = 0;
+    for (i64 q0 = (i64)blockIdx.x * ROWS_LARGE_NT * 4; q0 < c.cells; q0 += step, q += step) {  // uniform per CTA
+        RowsQuad x;
+        x.load(c.tokens, c.valid, q, c.cells, c.aligned);
+        if (BYTES && turn++ == TURNS) {
+            flush_bytes();
+            turn = 1;
+        }
+        x.neighbour();
+        x.pairs(col, c.L, [&](u64 key) {
+            if (BYTES && rows_byte_pair(key)) {
+                const unsigned int i = rows_byte_index(key);
+                reds_add_s32(reinterpret_cast<int *>(s_count + ((i >> 1) ^ ((i >> 8) & 31u))), (int)(1u << (16 * (i & 1u))));
+            } else if (!rows_smem_add<SLOTS>(s_key, s_val, key)) {
+                add(key, 1ull);
+            }
+        });
+        col += col_step;
+        if (col >= c.L) col -= c.L;
+    }
+    if (BYTES)
+        flush_bytes();
+    else
+        __syncthreads();
+    for (unsigned int k = threadIdx.x; k < SLOTS; k += ROWS_LARGE_NT) {
+        const unsigned int i = (k + blockIdx.x * (SLOTS / 128)) & (SLOTS - 1);
+        if (s_val[i]) add(s_key[i], (u64)s_val[i]);
+    }
+}
+__global__ void __launch_bounds__(ROWS_LARGE_NT) rows_pairs_large_kernel(const int32_t *__restrict__ tokens, const uint8_t *__restrict__ valid, i64 B,
+                                                                         i64 L, RowsTable t) {
+    extern __shared__ __align__(16) unsigned char s_rows[];
+    const RowsCells c = {tokens, valid, B * L, L, (((uintptr_t)tokens & 15) | ((uintptr_t)valid & 3)) == 0};
+    const i64 q = ((i64)blockIdx.x * ROWS_LARGE_NT + threadIdx.x) * 4;
+    RowsQuad x;
+    x.load(tokens, valid, q, c.cells, c.aligned);
+    x.neighbour();
+    int balance = 0;
+    x.pairs(q % L, L, [&](u64 key) { balance += rows_byte_pair(key) ? 1 : -1; });
+    const int most = __syncthreads_count(balance > 0);
+    if (2 * most > __syncthreads_count(balance != 0))
+        rows_count_large<true>(c, t, s_rows);
+    else
+        rows_count_large<false>(c, t, s_rows);
 }
 
 // rank[i] += keys of the tile blockIdx.y that are smaller than key i
@@ -402,12 +540,13 @@ STBPE_VISIBLE int stbpe_rows_count_pairs(const int32_t *tokens, const uint8_t *v
     RCK(stbpe::pinned_blocks().get(0, 4096, &pin));
     volatile u64 *got = (volatile u64 *)pin.p;
     int rc = STBPE_OK;
+    const bool large = B * L >= ROWS_LARGE_CELLS;
     for (;;) {
-        const u64 most = slots < (u64)(total > 0 ? total : 1) ? slots : (u64)(total > 0 ? total : 1);
+        const u64 room = slots + (large ? ROWS_BYTE_PAIRS : 0), most = room < (u64)(total > 0 ? total : 1) ? room : (u64)(total > 0 ? total : 1);
         const size_t keys_at = slots * sizeof(Slot), counts_at = keys_at + most * 8, rank_at = counts_at + most * 8,
-                     meta_at = (rank_at + most * 4 + 255) & ~(size_t)255;
+                     meta_at = (rank_at + most * 4 + 255) & ~(size_t)255, bytes_at = meta_at + 256;
         stbpe::Block b;
-        cudaError_t c = stbpe::device_blocks().get(dev, meta_at + 256, &b);
+        cudaError_t c = stbpe::device_blocks().get(dev, bytes_at + (large ? ROWS_BYTE_PAIRS * sizeof(u64) : 0), &b);
         if (c == cudaSuccess) {
             unsigned char *base = (unsigned char *)b.p;
             RowsTable t;
@@ -415,22 +554,22 @@ STBPE_VISIBLE int stbpe_rows_count_pairs(const int32_t *tokens, const uint8_t *v
             t.mask = slots - 1;
             t.n_keys = (u64 *)(base + meta_at);
             t.error = (unsigned int *)(t.n_keys + 1);
+            t.bytes = large ? (u64 *)(base + bytes_at) : nullptr;
             u64 *n_out = t.n_keys + 2;
             u64 *keys = (u64 *)(base + keys_at);
             i64 *counts = (i64 *)(base + counts_at);
             unsigned int *rank = (unsigned int *)(base + rank_at);
             const i64 quads = (B * L + 3) / 4;
             const i64 ranked = (i64)most < ROWS_RANK_MAX ? (i64)most : ROWS_RANK_MAX;  // more pairs than these take the radix sort
-            const bool large = B * L >= ROWS_LARGE_CELLS;
             const int nt = large ? ROWS_LARGE_NT : ROWS_SMALL_NT;
             const i64 want = (quads + nt - 1) / nt, most_ctas = large ? 148 : 148 * 4;
             const unsigned int grid = (unsigned int)(want < most_ctas ? want : most_ctas);
             rows_init_kernel<<<slots < (1u << 18) ? 64 : 592, 256, 0, s>>>(t, rank, (unsigned int)(most < ROWS_RANK_MAX ? most : ROWS_RANK_MAX));
             if (total > 0 && large) {
-                cudaFuncSetAttribute(rows_pairs_kernel<ROWS_LARGE_NT, ROWS_LARGE_SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_LARGE_SLOTS * 12);
-                rows_pairs_kernel<ROWS_LARGE_NT, ROWS_LARGE_SLOTS><<<grid, ROWS_LARGE_NT, ROWS_LARGE_SLOTS * 12, s>>>(tokens, valid, B, L, t);
+                cudaFuncSetAttribute(rows_pairs_large_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_LARGE_SMEM);
+                rows_pairs_large_kernel<<<grid, ROWS_LARGE_NT, ROWS_LARGE_SMEM, s>>>(tokens, valid, B, L, t);
             } else if (total > 0) {
-                rows_pairs_kernel<ROWS_SMALL_NT, ROWS_SMALL_SLOTS><<<grid, ROWS_SMALL_NT, ROWS_SMALL_SLOTS * 12, s>>>(tokens, valid, B, L, t);
+                rows_pairs_kernel<<<grid, ROWS_SMALL_NT, 0, s>>>(tokens, valid, B, L, t);
             }
             if (total > 0) rows_export_kernel<<<slots < (1u << 18) ? 64 : 592, 256, 0, s>>>(t, keys, counts, n_out, (i64)most);
             if (total > 0) rows_rank_kernel<<<dim3((unsigned int)((ranked + 255) / 256), (unsigned int)((ranked + ROWS_RANK_TILE - 1) / ROWS_RANK_TILE)), 256, 0, s>>>(keys, t.n_keys, t.error, rank);
@@ -641,6 +780,7 @@ extern "C" STBPE_VISIBLE int stbpe_rows_count_pairs_noalloc(const int32_t *token
         t.mask = STBPE_STATIC_TABLE_SLOTS - 1;
         t.n_keys = meta;
         t.error = reinterpret_cast<unsigned int *>(meta + 1);
+        t.bytes = nullptr;
         // the block still holds the previous call's table and counters: start from zero
         SCK(cudaMemsetAsync(meta, 0, 256, s));
         rows_clear_kernel<<<256, 256, 0, s>>>(t);

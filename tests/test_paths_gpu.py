@@ -470,3 +470,40 @@ def test_tiles_by_their_number_of_matches(per):
     e.train(40)
     _check(e, ids, off, 256, 40)
     e.close()
+
+
+@pytest.mark.parametrize("kind", ["bytes", "constant", "byte_rows_then_ids", "ids_then_byte_rows", "mixed_ids", "negative_and_large"])
+@pytest.mark.parametrize("rows,width,shift", [(512, 513, 0), (300, 1777, 1), (148 * 17, 4099, 0)])
+def test_seam_count_of_byte_pairs_and_others(kind, rows, width, shift, filter_mode):
+    # every CTA decides by its first cells how it counts; a pair counted both ways is one entry; the 16-bit counters are
+    # emptied in time (a constant batch of more than 15 turns)
+    if filter_mode == "filter_always":
+        pytest.skip("no stream")
+    g = np.random.RandomState(rows + width)
+    t = g.randint(0, 256, (rows, width)).astype(np.int32)
+    if kind == "constant":
+        t[:] = 255
+    elif kind == "byte_rows_then_ids":
+        t[rows // 2:] += g.randint(0, 300, (rows - rows // 2, width)).astype(np.int32)
+    elif kind == "ids_then_byte_rows":
+        t[:rows // 2] = t[:rows // 2] % 40 + 240
+    elif kind == "mixed_ids":
+        t = g.randint(200, 312, (rows, width)).astype(np.int32)
+    elif kind == "negative_and_large":
+        t = np.where(g.rand(rows, width) < 0.1, g.choice([-2, -2**31, 2**31 - 1, 65536], (rows, width)), t % 8).astype(np.int32)
+    v = (g.rand(rows, width) < 0.97).astype(np.uint8)
+    flat_t, flat_v = torch.zeros(rows * width + 4, dtype=torch.int32, device="cuda"), torch.zeros(rows * width + 4, dtype=torch.uint8, device="cuda")
+    flat_t[shift:shift + rows * width] = torch.from_numpy(t.ravel()).cuda()
+    flat_v[shift:shift + rows * width] = torch.from_numpy(v.ravel()).cuda()
+    dt, dv = flat_t[shift:shift + rows * width].view(rows, width), flat_v[shift:shift + rows * width].view(rows, width)
+    cap = 1 << 20
+    keys, counts = torch.empty((cap, 2), dtype=torch.int32, device="cuda"), torch.empty(cap, dtype=torch.int64, device="cuda")
+    length = torch.empty(1, dtype=torch.int64, device="cuda")
+    ops.count_pairs(dt, dv, keys, counts, length)
+    a, b = t[:, :-1].astype(np.int64) & 0xFFFFFFFF, t[:, 1:].astype(np.int64) & 0xFFFFFFFF
+    both = (v[:, :-1] & v[:, 1:]).astype(bool)
+    ok, oc = np.unique((a.astype(np.uint64)[both] << np.uint64(32)) | b.astype(np.uint64)[both], return_counts=True)
+    n = int(length.item())
+    got = (keys[:n, 0].to(torch.int64) << 32) | (keys[:n, 1].to(torch.int64) & 0xFFFFFFFF)
+    assert np.array_equal(got.cpu().numpy().view(np.uint64), ok) and np.array_equal(counts[:n].cpu().numpy(), oc)
+    assert bool((keys[n:] == -1).all()) and not bool(counts[n:].any())
