@@ -386,14 +386,15 @@ __global__ void rows_place_kernel(const u64 *__restrict__ keys, const i64 *__res
     if (first == 0 && length) *length = n;
 }
 
-// best of n entries (per CTA): key, count, index into out[blockIdx.x], out[256 + ...], out[512 + ...]
-__global__ void __launch_bounds__(256) rows_best_kernel(const i64 *keys, const i64 *counts, const i64 *index, i64 n, i64 *out) {
+// best of n entries (per CTA): key, count, index into out[3 * blockIdx.x ...].  Entry i is keys[i * stride] and so on.  (One
+// read-back of three words instead of three: four rounds of the seam on 16 x 512 cells 0.82 -> 0.79 ms.)
+__global__ void __launch_bounds__(256) rows_best_kernel(const i64 *keys, const i64 *counts, const i64 *index, i64 stride, i64 n, i64 *out) {
     __shared__ i64 s_k[8], s_c[8], s_i[8];
     i64 bk = 0x7FFFFFFFFFFFFFFFll, bc = 0, bi = 0x7FFFFFFFFFFFFFFFll;
     auto take = [&](i64 k, i64 c, i64 i) {
         if (c > bc || (c == bc && (k < bk || (k == bk && i < bi)))) bk = k, bc = c, bi = i;
     };
-    for (i64 i = (i64)blockIdx.x * 256 + threadIdx.x; i < n; i += (i64)gridDim.x * 256) take(keys[i], counts[i], index ? index[i] : i);
+    for (i64 i = (i64)blockIdx.x * 256 + threadIdx.x; i < n; i += (i64)gridDim.x * 256) take(keys[i * stride], counts[i * stride], index ? index[i * stride] : i);
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
         const i64 k = __shfl_down_sync(0xFFFFFFFFu, bk, d), c = __shfl_down_sync(0xFFFFFFFFu, bc, d), i = __shfl_down_sync(0xFFFFFFFFu, bi, d);
@@ -403,9 +404,9 @@ __global__ void __launch_bounds__(256) rows_best_kernel(const i64 *keys, const i
     __syncthreads();
     if (threadIdx.x != 0) return;
     for (int w = 1; w < 8; ++w) take(s_k[w], s_c[w], s_i[w]);
-    out[blockIdx.x] = bk;
-    out[256 + blockIdx.x] = bc;
-    out[512 + blockIdx.x] = bi;
+    out[3 * blockIdx.x] = bk;
+    out[3 * blockIdx.x + 1] = bc;
+    out[3 * blockIdx.x + 2] = bi;
 }
 
 // One CTA per row, walking the row in chunks with a running output offset.  Writes never
@@ -634,11 +635,11 @@ STBPE_VISIBLE int stbpe_select_pair(const int64_t *keys, const int64_t *counts, 
     RCK(stbpe::pinned_blocks().get(0, 4096, &pin));
     const i64 want = (n + 1023) / 1024;
     const int grid = (int)(want < 148 ? want : 148);
-    rows_best_kernel<<<grid, 256, 0, s>>>((const i64 *)keys, (const i64 *)counts, nullptr, n, (i64 *)b.p);
-    if (grid > 1) rows_best_kernel<<<1, 256, 0, s>>>((const i64 *)b.p, (const i64 *)b.p + 256, (const i64 *)b.p + 512, grid, (i64 *)b.p);
+    rows_best_kernel<<<grid, 256, 0, s>>>((const i64 *)keys, (const i64 *)counts, nullptr, 1, n, (i64 *)b.p);
+    if (grid > 1) rows_best_kernel<<<1, 256, 0, s>>>((const i64 *)b.p, (const i64 *)b.p + 1, (const i64 *)b.p + 2, 3, grid, (i64 *)b.p + 3 * 256);
     RCK(cudaGetLastError());
     i64 *h = (i64 *)pin.p;
-    for (int k = 0; k < 3; ++k) RCK(cudaMemcpyAsync(h + k, (i64 *)b.p + 256 * k, sizeof(i64), cudaMemcpyDeviceToHost, s));
+    RCK(cudaMemcpyAsync(h, (i64 *)b.p + (grid > 1 ? 3 * 256 : 0), 3 * sizeof(i64), cudaMemcpyDeviceToHost, s));
     RCK(cudaStreamSynchronize(s));
     if (h[1] > 0) *key = h[0], *count = h[1], *index = h[2];
     stbpe::device_blocks().put(dev, b);
