@@ -613,11 +613,11 @@ class GPUBPETrainer(BaseTrainer):
 
 
     def _loop_random_ties(self, eng: Engine, remaining: int, checkpoint_interval=None, checkpoint=None) -> int:
-        """Host-driven loop for ``randomize_ties``: the seeded ``random.Random`` picks an index
+        """Loop for ``randomize_ties``: the seeded ``random.Random`` picks an index
         into the tied candidates in ascending key order (``bpe_trainer.py:915-923``,
-        ``trainers/bpe_gpu.py:112-123``).  ``checkpoint`` is called every ``checkpoint_interval``
+        ``trainers/bpe_gpu.py:112-123``), on the device out of the generator's next outputs where it can.  ``checkpoint`` is called every ``checkpoint_interval``
         merges (the checkpoint carries the generator's state, so a resumed run draws on)."""
-        # Merges without a tie need no draw, so the engine runs through them; the log brings them back.
+        # The engine runs through merges without a tie and breaks most ties itself; the log brings them back.
         first, base = eng.state().merges_done, len(self.merges)
 
         def collect():
@@ -635,7 +635,7 @@ class GPUBPETrainer(BaseTrainer):
                 eng.apply_merge(*merge, self.vocab_size)
                 done, count, cands = 1, 0, []
             else:
-                done, count, cands = eng.next_tied(merge, self.vocab_size, most)
+                done, count, cands = eng.next_tied(merge, self.vocab_size, most, self._tie_rng)
             remaining -= done
             since += done
             self.vocab_size += done

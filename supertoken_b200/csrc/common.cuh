@@ -91,6 +91,7 @@ struct DevState {
     int exchange_only;         // multi-GPU: deltas still in flight, the next round only exchanges
     int round_incomplete;      // multi-GPU: this rank saw a full chunk or kept entries this round
     int forced_done;           // host-given merges the last loop_kernel launch applied
+    int draws_used;            // outputs of the tie-breaking generator it used
     unsigned int n_cand;       // entries of the candidate list (may exceed its capacity: then it is incomplete)
     i64 theta_count;           // the list holds every pair with a larger count, or with this count and
     u64 theta_key;             // a key below this one

@@ -42,6 +42,7 @@ struct stbpe_engine {
     int select_grid, refresh_grid;
     size_t count_smem;
     int2 *forced;         // device copy of host-given merges
+    uint32_t *draws;      // STBPE_DRAWS outputs of a tie-breaking generator, from the first call that brings any
     int forced_cap;
     bool recs_stale, counted;
     bool filter_valid;    // host mirror of DevState::filter_valid
@@ -297,6 +298,8 @@ static const DeviceInfo &device_info(int dev) {
     SMEM((loop_kernel<uint16_t, FILTER_ON, 11>), optin - 4096);
     SMEM((loop_kernel<uint16_t, FILTER_ON, 13>), optin - 4096);
     SMEM((loop_kernel<uint16_t, FILTER_ON, 15>), optin - 4096);
+    SMEM((loop_kernel<uint16_t, FILTER_OFF, 15, true>), optin - 4096);
+    SMEM((loop_kernel<uint16_t, FILTER_ON, 15, true>), optin - 4096);
     SMEM((loop_kernel<uint32_t, FILTER_OFF, 15>), optin - 4096);
     SMEM((loop_kernel<uint32_t, FILTER_ON, 15>), optin - 4096);
     SMEM((count_kernel<uint16_t, false>), STBPE_COUNT_SMEM);
@@ -1165,8 +1168,12 @@ STBPE_VISIBLE int stbpe_select_best(stbpe_engine *e, uint64_t *key, int64_t *cou
 }
 
 static int filter_policy(stbpe_engine *e, const DevState &h, bool layout_changed, cudaStream_t s);
+struct Draws {  // outputs of a tie-breaking generator on the device
+    const uint32_t *dev;
+    int n, used;
+};
 static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t first_new, int64_t *n_matches, cudaStream_t s, bool then_ties = false,
-                      int most = 0, int *n_done = nullptr);
+                      int most = 0, int *n_done = nullptr, Draws *draws = nullptr);
 
 static int launch_merge(stbpe_engine *e, bool mg, cudaStream_t s) {
     if (e->d.n_tiles < 1) return STBPE_OK;
@@ -1207,9 +1214,9 @@ STBPE_VISIBLE int stbpe_apply_merges(stbpe_engine *e, const int32_t *pairs, int3
     return run_forced(e, pairs, n, first_new_id, nullptr, (cudaStream_t)stream);
 }
 
-STBPE_VISIBLE int stbpe_next_tied(stbpe_engine *e, int32_t a, int32_t b, int32_t new_id, int32_t most, int32_t *n_done, int64_t *count,
-                                  uint64_t *keys, int64_t cap, int64_t *n_ties, void *stream) {
-    if (!e || !count || !n_ties || !n_done || most < 0 || cap < 0 || (cap > 0 && !keys)) return STBPE_E_BADARG;
+STBPE_VISIBLE int stbpe_next_drawn(stbpe_engine *e, int32_t a, int32_t b, int32_t new_id, int32_t most, const uint32_t *draws, int32_t n_draws,
+                                   int32_t *n_used, int32_t *n_done, int64_t *count, uint64_t *keys, int64_t cap, int64_t *n_ties, void *stream) {
+    if (!e || n_draws < 0 || (n_draws > 0 && (!draws || !n_used)) || !count || !n_ties || !n_done || most < 0 || cap < 0 || (cap > 0 && !keys)) return STBPE_E_BADARG;
     cudaStream_t s = (cudaStream_t)stream;
     CK(cudaSetDevice(e->cfg.device));
     if (!e->counted) return fail(e, STBPE_E_STATE, "count the pairs before selecting");
@@ -1217,11 +1224,21 @@ STBPE_VISIBLE int stbpe_next_tied(stbpe_engine *e, int32_t a, int32_t b, int32_t
     const int given = a >= 0 ? 1 : 0;
     const bool run = given || most > 0;
     *n_done = 0;
+    if (n_used) *n_used = 0;
     if (run) {
         if (new_id < 0 || (i64)new_id + most >= 0x7FFFFFFFll || (given && (b < 0 || a == 0x7FFFFFFF || b == 0x7FFFFFFF)))
             return fail(e, STBPE_E_ID_OVERFLOW, "Token id overflow: ids must be in [0, 2^31-2]");
         const int32_t pair[2] = {a, b};
-        int rc = run_forced(e, pair, given, new_id, nullptr, s, true, most, n_done);
+        Draws d = {nullptr, n_draws < STBPE_DRAWS ? n_draws : STBPE_DRAWS, 0};
+        if (d.n > 0) {
+            if (!e->draws) CK(dev_alloc(e, &e->draws, (size_t)STBPE_DRAWS));
+            static_assert(STBPE_DRAWS * sizeof(uint32_t) <= STBPE_PINNED_BYTES - STBPE_PINNED_STATE, "the draws travel through the pinned block");
+            void *pin = memcpy((char *)e->pinned.p + STBPE_PINNED_STATE, draws, (size_t)d.n * sizeof(uint32_t));
+            CK(cudaMemcpyAsync(e->draws, pin, (size_t)d.n * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+            d.dev = e->draws;
+        }
+        int rc = run_forced(e, pair, given, new_id, nullptr, s, true, most, n_done, d.n > 0 ? &d : nullptr);
+        if (n_used) *n_used = d.used;
         if (rc != STBPE_OK) return rc;
     }
     std::vector<u64> tied;
@@ -1233,6 +1250,11 @@ STBPE_VISIBLE int stbpe_next_tied(stbpe_engine *e, int32_t a, int32_t b, int32_t
     if ((i64)tied.size() <= cap)
         for (size_t i = 0; i < tied.size(); ++i) keys[i] = tied[i];
     return STBPE_OK;
+}
+
+STBPE_VISIBLE int stbpe_next_tied(stbpe_engine *e, int32_t a, int32_t b, int32_t new_id, int32_t most, int32_t *n_done, int64_t *count,
+                                  uint64_t *keys, int64_t cap, int64_t *n_ties, void *stream) {
+    return stbpe_next_drawn(e, a, b, new_id, most, nullptr, 0, nullptr, n_done, count, keys, cap, n_ties, stream);
 }
 
 static int maybe_repack(stbpe_engine *e, bool force, int *did, cudaStream_t s);
@@ -1374,7 +1396,7 @@ __global__ void set_target_kernel(EngineDev e, int target) {
 // Runs loop_kernel until a stop rule fires, doing the maintenance it asks for between launches.  `forced`
 // (device, n_forced pairs): these merges instead of the best pairs.  *out = the device state at the end.
 static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, int2 one, int n_forced, int forced_new, DevState *out,
-                    cudaStream_t s, bool then_ties = false, int *n_done = nullptr) {
+                    cudaStream_t s, bool then_ties = false, int *n_done = nullptr, Draws *draws = nullptr) {
     LoopArgs la;
     int at = 0;
     la.mode = mode;
@@ -1405,12 +1427,15 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
         la.grow_keys = e->table_auto ? (i64)(e->slots / 4) : (i64)0x7FFFFFFFFFFFFFFFll;
         la.ids_below = (int)std::min(ids_below(e), (i64)0x7FFFFFFF);
         la.unit_shift = unit_shift(e, grid);
+        la.draws = draws ? draws->dev + draws->used : nullptr;
+        la.n_draws = draws ? draws->n - draws->used : 0;
         EngineDev d = e->d;
         // Bits of an id that the loop looks at: as few as all ids, old and new, allow.  It returns for the id that needs more,
         // which costs a launch (some 40 us): nine bits only where steps are long (over 8192 tiles one takes 25 us and a tenth
         // of it is saved), thirteen where the filter is in use (8 000 merges of 256 MiB: 68 million visits, 2 % off each).
         int planes = 15;
-        if (!e->wide) {
+        const bool drawing = la.n_draws > 0 && !e->wide;
+        if (!e->wide && !drawing) {
             auto enough = [&](int p) { return p > planes_due && la.ids_below < (1 << p) - 1; };
             if (!e->filter_valid && e->d.n_tiles >= 8192 && enough(9)) planes = 9;
             else if (enough(11)) planes = 11;
@@ -1430,11 +1455,12 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
         const cudaError_t c = with_tok(e, [&](auto t) {
             typedef decltype(t) T;
             const void *kernel = e->filter_valid ? (const void *)loop_kernel<T, FILTER_ON, 15> : (const void *)loop_kernel<T, FILTER_OFF, 15>;
+            if (drawing) kernel = e->filter_valid ? (const void *)loop_kernel<uint16_t, FILTER_ON, 15, true> : (const void *)loop_kernel<uint16_t, FILTER_OFF, 15, true>;
             if (planes == 9) kernel = (const void *)loop_kernel<uint16_t, FILTER_OFF, 9>;
             if (planes == 11) kernel = e->filter_valid ? (const void *)loop_kernel<uint16_t, FILTER_ON, 11> : (const void *)loop_kernel<uint16_t, FILTER_OFF, 11>;
             if (planes == 13) kernel = (const void *)loop_kernel<uint16_t, FILTER_ON, 13>;
             return cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(MergeGeom<T>::THREADS), args,
-                                               MergeGeom<T>::BYTES + STBPE_CAND_CAP * sizeof(unsigned int), s);
+                                               MergeGeom<T>::BYTES + (STBPE_CAND_CAP + (drawing ? STBPE_DRAWS : 0)) * sizeof(unsigned int), s);
         });
         if (c != cudaSuccess) return cuda_fail(e, c, "cudaLaunchCooperativeKernel");
         if (then_ties) {  // enqueued behind the merge: one round trip for both
@@ -1443,6 +1469,7 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
         }
         if (int rc_ = read_state(e, out, s)) return rc_;
         at += out->forced_done;
+        if (draws) draws->used += out->draws_used;
         e->made_below = std::max(e->made_below, mode == LOOP_BEST ? (i64)e->cfg.base_vocab + out->merges_done : (i64)forced_new + at);
         if (n_done) *n_done = at;
         int rc = check_error_bits(e, out->error);
@@ -1474,7 +1501,7 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
 
 // host-given merges, applied in order as merges of the log
 static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t first_new, int64_t *n_matches, cudaStream_t s,
-                      bool then_ties, int most, int *n_done) {
+                      bool then_ties, int most, int *n_done, Draws *draws) {
     DevState h;
     if (!then_ties || !e->merges_known) {
         if (int rc_ = read_state(e, &h, s)) return rc_;
@@ -1496,7 +1523,7 @@ static int run_forced(stbpe_engine *e, const int32_t *pairs, int n, int32_t firs
     if (n > 1) CK(cudaMemcpyAsync(e->forced, src, (size_t)n * sizeof(int2), cudaMemcpyHostToDevice, s));
     if ((i64)first_new + n + most > 65536) e->foreign_ids = true;
     int rc = run_loop(e, e->merges_done + n + most, most > 0 ? LOOP_UNTIED : LOOP_NONE, n > 1 ? e->forced : nullptr,
-                      n == 1 ? make_int2(pairs[0], pairs[1]) : make_int2(0, 0), n, first_new, &h, s, then_ties, n_done);
+                      n == 1 ? make_int2(pairs[0], pairs[1]) : make_int2(0, 0), n, first_new, &h, s, then_ties, n_done, draws);
     e->merges_known = rc == STBPE_OK;
     e->merges_done = h.merges_done;
     if (rc == STBPE_OK && n_matches) *n_matches = h.n_matches;

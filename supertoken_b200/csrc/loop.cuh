@@ -57,7 +57,10 @@ struct LoopArgs {
     int unit_shift;         // tiles per filter unit, log2 (cta_merge)
     i64 grow_keys;          // leave for a larger pair table when a merge could take the number of keys beyond this ...
     int ids_below;          // every id of the stream lies below this (those of the launch's own merges apart)
+    const uint32_t *draws;  // LOOP_UNTIED, 16-bit tokens: outputs of the generator that breaks ties; without any, a tie ends the launch
+    int n_draws;
 };
+#define STBPE_DRAWS 1024  // at most
 
 enum { LOOP_BEST, LOOP_NONE, LOOP_UNTIED };
 
@@ -146,7 +149,8 @@ struct Best<uint32_t> {
 // the instructions of a dense step and an eighth of a sparse one, and every pair is compared plane by plane.  Nine planes
 // and code without the filter took the first 20 merges of 1 GiB from 20.3 to 16.3 ms (24 warps per SM instead of 20: no
 // faster); eleven, then thirteen, 8 000 merges of 256 MiB from 121.6 to 118.3 ms.
-template <typename T, int FV, int PLANES>
+// DRAW: with the code that breaks ties (16-bit tokens, 15 planes; inside the other kernels it cost 1 % of them, for registers).
+template <typename T, int FV, int PLANES, bool DRAW = false>
 __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __grid_constant__ EngineDev e, const __grid_constant__ LoopArgs la) {
     typedef Best<T> Bs;
     typedef typename Bs::type Bt;
@@ -159,6 +163,8 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
     __shared__ i64 s_live, s_keys;        // live tokens, keys in the table
     __shared__ i64 s_forced[KB];          // counts of the next host-given pairs
     __shared__ int s_go;                  // merges in this step's batch
+    __shared__ int s_tie;                 // this step's merge is drawn among the best pairs
+    __shared__ int s_ties, s_drawn, s_used;  // how many they are; which one it is, in ascending order; outputs of the generator used
     __shared__ unsigned int s_err;        // device error bits
     __shared__ int s_ok;                  // every wait so far succeeded
     CtaMerge s;
@@ -175,7 +181,22 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
     mc.fv = fv;
     mc.theta.count = st->theta_count, mc.theta.key = st->theta_key;
     unsigned int n_cand = 0;  // candidates this CTA knows
-    if (tid == 0) s_ok = 1;
+    uint32_t *const s_draws = s_cand + STBPE_CAND_CAP;
+    const bool draws = DRAW && la.n_draws > 0;
+    if (draws)
+        for (int i = tid; i < la.n_draws; i += THREADS) s_draws[i] = la.draws[i];  // (a barrier comes before they are read)
+    if (tid == 0) s_ok = 1, s_used = 0;
+    auto leave = [&](int why, int stop, const Slot &best, bool valid) {  // one thread of CTA 0
+        st->merges_done = merges_done;
+        st->run_exit = why;
+        st->stopped = stop > 0;
+        st->stop_reason = stop;
+        st->peek_key = best.key;
+        st->peek_count = best.count;
+        st->peek_valid = valid;
+        st->forced_done = forced_i;
+        st->draws_used = DRAW ? s_used : 0;
+    };
     WarpStats ws = {0, 0, 0, 0, 0};
     int visited = 0;  // tiles of this CTA in the last step
     if (cta == 0 && tid == 32) {
@@ -254,7 +275,8 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             }
             __syncthreads();
         }
-        if (tid == THREADS - 1) red_release_u32(&sync->chosen, 1u);  // this CTA has read all that it decides by
+        // this CTA has read all that it decides by (if no tie is to be broken, which takes another look)
+        if (!draws && tid == THREADS - 1) red_release_u32(&sync->chosen, 1u);
         // warp 0 decides; the lanes of pair j take the j-th best pair (or the j-th one the host gives) and test whether it
         // can be merge j of the batch, given that all before it are
         if (warp == 0) {
@@ -306,17 +328,19 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             // that the merges before it make are rarer than some pair after it, hence rarer than it.)  A slot that is listed
             // twice, as one can be whose pair a merge has lifted again with an id that was there before, takes one place and
             // leaves a gap behind it: then, too, the host looks.
-            bool tied = true;
+            bool tied = true, draw = false;
             if constexpr (KB > 1) {
                 if (la.mode == LOOP_UNTIED) {
                     const Slot after = Bs::slot(max(s_sorted[j + 1], bound));
+                    draw = draws && j == 0 && !host && !dry && s_sorted[1] && count == after.count && count > mc.theta.count && count >= 2 &&
+                           merges_done < la.target;
                     tied = !s_sorted[j + 1] || count <= after.count || count <= mc.theta.count || count < 2 || merges_done + j >= la.target;
                 }
             }
             if (err & 0x7FFFFFFFu) stop = 4;
             else if (la.mode != LOOP_BEST && host && !forced) stop = 0;
             else if (la.mode == LOOP_NONE && !host) stop = 0;
-            else if (la.mode == LOOP_UNTIED && !host && !dry && tied) stop = 0;  // the host looks at what there is
+            else if (la.mode == LOOP_UNTIED && !host && !dry && tied && !draw) stop = 0;  // the host looks at what there is
             else if (!host && merges_done + j >= la.target) stop = la.mode == LOOP_BEST ? 1 : 0;
             // maintenance the host does between launches
             else if (!host && dry) why = STBPE_EXIT_REFILL;
@@ -327,9 +351,10 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             else if (s_keys + 2 * made + 2 * (j + 1) > la.grow_keys) why = STBPE_EXIT_GROW;
             else if (sizeof(T) == 2 && max(nw, max(a, b)) >= (1u << PLANES) - 1u) why = STBPE_EXIT_WIDEN;
             else go = true;
-            const uint32_t bad = __ballot_sync(0xFFFFFFFFu, j >= KB || !go || (j > 0 && out)) | (KB > 1 ? 1u << (2 * KB) : 2u);
+            draw = __any_sync(0xFFFFFFFFu, draw);
+            const uint32_t bad = __ballot_sync(0xFFFFFFFFu, j >= KB || !go || (j > 0 && (out || draw))) | (KB > 1 ? 1u << (2 * KB) : 2u);
             const int nb = lsb(bad) >> (KB > 1 ? 1 : 0);
-            if (KB > 1 ? j < nb && !(lane & 1) : lane < nb) {
+            if ((KB > 1 ? j < nb && !(lane & 1) : lane < nb) && !draw) {
                 s.p->a[j] = a, s.p->b[j] = b, s.p->nw[j] = nw;
                 s.p->count[j] = count;
                 if (cta == 0) {
@@ -346,20 +371,80 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             if (lane == 0) {
                 s.p->n = nb;
                 s_go = nb;
-                if (cta == 0 && nb == 0) {
-                    st->merges_done = merges_done;
-                    st->run_exit = why;
-                    st->stopped = stop > 0;
-                    st->stop_reason = stop;
-                    st->peek_key = best.key;
-                    st->peek_count = best.count;
-                    st->peek_valid = !dry;
-                    st->forced_done = forced_i;
-                    if (!fv && step > 0) st->n_work = -1;
-                }
+                s_tie = nb > 0 && draw;
+                s_ties = 0;
+                if (s_tie) s.p->count[0] = count;
+                if (cta == 0 && nb == 0) leave(why, stop, best, !dry);
             }
         }
         __syncthreads();
+        if constexpr (DRAW) {
+            if (s_tie) {
+                // The generator picks one of the best pairs in ascending order of their keys (random.Random.randrange: the top
+                // bits of an output, again while they are not below the number of pairs).  All CTAs draw the same.
+                const i64 c = s.p->count[0];
+                u64 *const keys = reinterpret_cast<u64 *>(smem_raw);  // the tiles' slots are free
+                for (unsigned int i = tid; i < n_cand; i += THREADS) {
+                    const Slot y = ldcg_slot(e.table + s_cand[i]);
+                    if (y.count != c) continue;
+                    const int at = atoms_add_s32(&s_ties, 1);
+                    if (at < STBPE_TIES_CAP) keys[at] = y.key;
+                }
+                __syncthreads();
+                const int n = s_ties;
+                constexpr int PER = (STBPE_TIES_CAP + THREADS - 1) / THREADS;
+                int place[PER];
+                bool odd = n < 2 || n > STBPE_TIES_CAP;  // a pair that is listed twice, or more of them than fit: the host looks
+#pragma unroll
+                for (int r = 0; r < PER; ++r) {
+                    const int i = tid + r * THREADS;
+                    place[r] = -1;
+                    if (n > STBPE_TIES_CAP || i >= n) continue;
+                    const u64 mine = keys[i];
+                    int below = 0;
+                    for (int q = 0; q < n; ++q) {
+                        const u64 other = keys[q];
+                        below += other < mine;
+                        odd = odd || (other == mine && q != i);
+                    }
+                    place[r] = below;
+                }
+                odd = __syncthreads_or(odd);
+                if (tid == 0) {
+                    int used = s_used, x = -1;
+                    if (!odd) {
+                        do {
+                            x = used < la.n_draws ? (int)(s_draws[used++] >> __clz(n)) : -1;
+                        } while (x >= n);
+                        if (x >= 0) s_used = used;
+                    }
+                    s_drawn = x;
+                    if (x < 0) {
+                        s_go = 0;
+                        Slot none;
+                        none.key = STBPE_EMPTY, none.count = 0;
+                        if (cta == 0) leave(STBPE_EXIT_STOP, 0, none, false);
+                    }
+                }
+                __syncthreads();
+#pragma unroll
+                for (int r = 0; r < PER; ++r) {
+                    if (place[r] < 0 || place[r] != s_drawn) continue;
+                    const u64 key = keys[tid + r * THREADS];
+                    const int nw = la.forced_new + forced_i;
+                    s.p->a[0] = (uint32_t)(key >> 32), s.p->b[0] = (uint32_t)key, s.p->nw[0] = (uint32_t)nw;
+                    if (cta == 0) {
+                        *reinterpret_cast<int2 *>(e.merges + 2 * merges_done) = make_int2((int)(key >> 32), (int)(uint32_t)key);
+                        e.merge_counts[merges_done] = c;
+                        e.live_before[merges_done] = s_live;
+                        st->cur_a = (int)(key >> 32), st->cur_b = (int)(uint32_t)key, st->cur_new = nw;
+                        st->cur_count = c;
+                    }
+                }
+                __syncthreads();
+            }
+        }
+        if (draws && tid == THREADS - 1) red_release_u32(&sync->chosen, 1u);
         const int nb = s_go;
         if (tid < 32 * nb) s.p->set_plane<T>(tid >> 5, lane);  // (barriers of cta_merge come before they are read)
         if (nb == 0 || !s_ok) {

@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import ctypes
+import random
 from typing import List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -146,18 +147,31 @@ class Engine:
         p = np.asarray(pairs, dtype=np.int32)
         self._check(self._lib.stbpe_apply_merges(self._h, p.ctypes.data, len(p), int(first_new_id), self._s))
 
-    def next_tied(self, merge: Optional[Tuple[int, int]] = None, new_id: int = 0, most: int = 0) -> Tuple[int, int, List[int]]:
-        """One step of a loop that breaks ties on the host: apply ``merge`` = (a, b) as ``new_id``, if given, go on
+    def next_tied(self, merge: Optional[Tuple[int, int]] = None, new_id: int = 0, most: int = 0,
+                  rng: Optional[random.Random] = None) -> Tuple[int, int, List[int]]:
+        """One step of a loop that breaks ties: apply ``merge`` = (a, b) as ``new_id``, if given, go on
         with up to ``most`` best pairs while each is the only one with its count, and return the number of merges
-        applied, the best count and the keys that hold it, ascending."""
+        applied, the best count and the keys that hold it, ascending.  With ``rng`` ties are broken on the device too, as
+        ``keys[rng.randrange(len(keys))]`` would, and ``rng`` is moved on by what that took; it may still return with a tie."""
         a, b = merge if merge is not None else (-1, -1)
         if max(a, b) > 0x7FFFFFFE or new_id + most > 0x7FFFFFFE or (merge is not None and min(a, b) < 0):
             raise OverflowError("Token id overflow: ids must be in [0, 2^31-2]")
         if getattr(self, "_tied", None) is None:
             self._tied = np.empty(1024, dtype=np.uint64)
+        words, n_draws = None, 0
+        if rng is not None and most > 0:
+            # the generator's next outputs (the first one in the lowest bits), without moving it
+            n_draws = min(2 * most + 16, 1024)
+            before = rng.getstate()
+            words = rng.getrandbits(32 * n_draws).to_bytes(4 * n_draws, "little")
+            rng.setstate(before)
+        used = ctypes.c_int32(0)
         done, count, n = ctypes.c_int32(0), ctypes.c_int64(0), ctypes.c_int64(0)
-        self._check(self._lib.stbpe_next_tied(self._h, a, b, new_id, most, ctypes.byref(done), ctypes.byref(count),
-                                              self._tied.ctypes.data, len(self._tied), ctypes.byref(n), self._s))
+        self._check(self._lib.stbpe_next_drawn(self._h, a, b, new_id, most, words, n_draws, ctypes.byref(used), ctypes.byref(done),
+                                               ctypes.byref(count), self._tied.ctypes.data, len(self._tied), ctypes.byref(n),
+                                               self._s))
+        if used.value:
+            rng.getrandbits(32 * used.value)
         if count.value <= 0:
             return done.value, 0, []
         if n.value > len(self._tied):

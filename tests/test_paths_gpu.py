@@ -507,3 +507,46 @@ def test_seam_count_of_byte_pairs_and_others(kind, rows, width, shift, filter_mo
     got = (keys[:n, 0].to(torch.int64) << 32) | (keys[:n, 1].to(torch.int64) & 0xFFFFFFFF)
     assert np.array_equal(got.cpu().numpy().view(np.uint64), ok) and np.array_equal(counts[:n].cpu().numpy(), oc)
     assert bool((keys[n:] == -1).all()) and not bool(counts[n:].any())
+
+
+def _drawn_run(ids, off, base_vocab, target, seed, device, start=None):
+    """Merges of a loop that breaks ties by random.Random(seed), drawn on the host or on the device, and the generator's state."""
+    import random
+    rng, merge, done = random.Random(seed), start, 0
+    e = _engine(ids, off, base_vocab, target)
+    trips = 0
+    while done < target:
+        n, count, cands = e.next_tied(merge, base_vocab + done, target - done - (merge is not None), rng if device else None)
+        done, merge, trips = done + n, None, trips + 1
+        if done >= target or not cands or count < 2:
+            break
+        key = cands[rng.randrange(len(cands))] if len(cands) > 1 else cands[0]
+        merge = (key >> 32, key & 0xFFFFFFFF)
+        if done == target - 1:
+            e.apply_merge(*merge, base_vocab + done)
+            done += 1
+    m, c, live = e.merges()
+    stream = e.export_stream()[0]
+    e.close()
+    return m, c.tolist(), live.tolist(), stream.tolist(), rng.getstate(), trips
+
+
+@pytest.mark.parametrize("seed,n,alphabet,target", [(0, 3000, 6, 90), (1, 3000, 40, 150), (2, 40000, 300, 120), (3, 200, 200, 30), (4, 9000, 1000, 60),
+                                                    (5, 70000, 12, 200), (6, 2500, 3, 400)])
+def test_ties_drawn_on_the_device_as_on_the_host(seed, n, alphabet, target):
+    # few and many tied pairs (more than the device keeps, too), counts that fall to the threshold and below 2, draws that run out
+    rng = np.random.RandomState(seed)
+    ids = rng.randint(0, alphabet, n).astype(np.int32)
+    off = _rows(ids, rng, 90)
+    host, dev = (_drawn_run(ids, off, 1000, target, seed, d) for d in (False, True))
+    assert host[:5] == dev[:5]
+    assert dev[5] <= host[5]
+
+
+@pytest.mark.parametrize("base_vocab", [508, 2040, 32760])
+def test_ties_drawn_where_the_loop_leaves_for_more_bits(base_vocab):
+    rng = np.random.RandomState(base_vocab)
+    ids = rng.choice([1, 2, 3, 4, 5], 30000).astype(np.int32)
+    off = _rows(ids, rng, 60)
+    host, dev = (_drawn_run(ids, off, base_vocab, 40, 7, d, start=(1, 2)) for d in (False, True))
+    assert host[:5] == dev[:5]
