@@ -436,6 +436,7 @@ class GPUBPETrainer(BaseTrainer):
         t = time.perf_counter()
         remaining = self.target_merges - len(self.merges)
         reason = L.RUNNING
+        st = None  # the engine's state, while nothing has run behind it
         if remaining > 0:
             if self.randomize_ties:
                 reason = self._loop_random_ties(eng, remaining, checkpoint_interval,
@@ -462,10 +463,11 @@ class GPUBPETrainer(BaseTrainer):
                     reason = st.stop_reason
                     if checkpoint_interval and checkpoint_dir and remaining > 0:
                         checkpoint()
+                        st = None
                     if len(got) < n:
                         break
         loop_s = time.perf_counter() - t
-        return self._finalize(eng.state(), reason, timings, events, warm_applied + skip, loop_s, t0, log_every)
+        return self._finalize(st if st is not None else eng.state(), reason, timings, events, warm_applied + skip, loop_s, t0, log_every)
 
     def _finalize(self, st, reason, timings, events, warm_applied, loop_s, t0, log_every) -> dict:
         timings["apply_merge"].record(loop_s)

@@ -706,7 +706,8 @@ static int prepare_stream_state(stbpe_engine *e, cudaStream_t s) {
         init_state_kernel<<<1, 1, 0, s>>>(e->d, e->cfg.base_vocab, e->n_tokens);
         CK(cudaGetLastError());
         e->state_stale = false;
-        e->merges_known = false;
+        e->merges_done = 0;
+        e->merges_known = true;
         e->recs_stale = false;
         e->repacks_since_load = 0;
         e->filter_valid = false;  // a fresh stream starts without a pair filter (see filter_policy)
@@ -951,7 +952,8 @@ static int wide_build(stbpe_engine *e, int *ok, cudaStream_t s) {
     return STBPE_OK;
 }
 
-static int launch_count(stbpe_engine *e, bool mg, cudaStream_t s) {
+// *err: the device error bits, where they have been read behind the last kernel (*err_known).
+static int launch_count(stbpe_engine *e, bool mg, cudaStream_t s, unsigned int *err = nullptr, bool *err_known = nullptr) {
     if (mg && e->wide_counted) {  // stbpe_mg_wide_pass2 has filled the table already
         e->wide_counted = false;
         return STBPE_OK;
@@ -978,6 +980,7 @@ static int launch_count(stbpe_engine *e, bool mg, cudaStream_t s) {
         CK(cudaStreamSynchronize(s));
         if (!(*derr & STBPE_DERR_DENSE_OVERFLOW)) {
             if (!mg) e->bytes_below = (i64)derr[1] + 1;
+            if (!mg && err) *err = *derr, *err_known = true;
             if (mg) dense_to_table_kernel<true><<<256, 256, 0, s>>>(e->d, e->dense);
             CK(cudaGetLastError());
             return STBPE_OK;
@@ -1039,10 +1042,11 @@ STBPE_VISIBLE int stbpe_count_initial(stbpe_engine *e, void *stream) {
     e->counted = false;  // (a recount that finds no memory for a larger table leaves none)
     for (;;) {
         const bool fresh = e->recs_stale;
-        int rc = launch_count(e, false, s);
-        if (rc != STBPE_OK) return rc;
         unsigned int err = 0;
-        rc = check_device_error(e, s, &err);
+        bool err_known = false;
+        int rc = launch_count(e, false, s, &err, &err_known);
+        if (rc != STBPE_OK) return rc;
+        rc = err_known ? check_error_bits(e, err) : check_device_error(e, s, &err);
         if ((err & STBPE_DERR_TABLE_FULL) && e->table_auto && e->slots * 4 <= (u64)STBPE_MAX_SLOTS) {
             // more distinct pairs than the table was sized for: the same count once more, with four times the slots
             e->slots_needed = e->slots * 4;
@@ -1537,11 +1541,16 @@ STBPE_VISIBLE int stbpe_train(stbpe_engine *e, int32_t n_merges, void *stream) {
     if (!e->counted) return fail(e, STBPE_E_STATE, "count the pairs before training");
     if (e->cfg.world_size > 1) return fail(e, STBPE_E_STATE, "single-rank entry point");
     DevState h;
-    if (int rc_ = read_state(e, &h, s)) return rc_;
-    e->merges_known = false;
-    i64 target = (i64)h.merges_done + n_merges;
+    if (!e->merges_known) {
+        if (int rc_ = read_state(e, &h, s)) return rc_;
+        e->merges_done = h.merges_done;
+    }
+    i64 target = (i64)e->merges_done + n_merges;
     if (target > e->cfg.max_merges) target = e->cfg.max_merges;
-    return run_loop(e, (int)target, LOOP_BEST, nullptr, make_int2(0, 0), 0, 0, &h, s);
+    e->merges_known = false;
+    const int rc = run_loop(e, (int)target, LOOP_BEST, nullptr, make_int2(0, 0), 0, 0, &h, s);
+    if (rc == STBPE_OK) e->merges_done = h.merges_done, e->merges_known = true;
+    return rc;
 }
 
 // The merges of stbpe_train one at a time: choose_kernel with the host's look at its result, then merge_kernel, with CUDA
@@ -1656,7 +1665,20 @@ STBPE_VISIBLE int stbpe_get_merges(stbpe_engine *e, int32_t first, int32_t n, in
         return fail(e, STBPE_E_BADARG, "bad merge range");
     CK(cudaSetDevice(e->cfg.device));
     if (n == 0) return STBPE_OK;
-    CK(cudaMemcpy(merges, e->d.merges + 2 * first, (size_t)n * 2 * sizeof(int32_t), cudaMemcpyDeviceToHost));
+    const size_t third = (size_t)n * 8;  // a pair, a count and a number of tokens are eight bytes each
+    static_assert(2 * sizeof(int32_t) == 8 && sizeof(i64) == 8, "three columns of eight bytes");
+    if (3 * third <= STBPE_PINNED_BYTES - STBPE_PINNED_STATE) {  // one wait for all of them
+        char *pin = (char *)e->pinned.p + STBPE_PINNED_STATE;
+        CK(cudaMemcpyAsync(pin, e->d.merges + 2 * first, third, cudaMemcpyDeviceToHost, 0));
+        if (counts) CK(cudaMemcpyAsync(pin + third, e->d.merge_counts + first, third, cudaMemcpyDeviceToHost, 0));
+        if (live_before) CK(cudaMemcpyAsync(pin + 2 * third, e->d.live_before + first, third, cudaMemcpyDeviceToHost, 0));
+        CK(cudaStreamSynchronize(0));
+        memcpy(merges, pin, third);
+        if (counts) memcpy(counts, pin + third, third);
+        if (live_before) memcpy(live_before, pin + 2 * third, third);
+        return STBPE_OK;
+    }
+    CK(cudaMemcpy(merges, e->d.merges + 2 * first, third, cudaMemcpyDeviceToHost));
     if (counts) CK(cudaMemcpy(counts, e->d.merge_counts + first, (size_t)n * sizeof(i64), cudaMemcpyDeviceToHost));
     if (live_before) CK(cudaMemcpy(live_before, e->d.live_before + first, (size_t)n * sizeof(i64), cudaMemcpyDeviceToHost));
     return STBPE_OK;
