@@ -508,7 +508,7 @@ __device__ __forceinline__ void merge_tile(const EngineDev &e, const CtaMerge &s
         return STBPE_NONE;
     };
     // Many matches in the tile: a head and an end per lane and round, each by code of its own, which is less of it (first 20
-    // merges of 1 GiB 16.65 ms, 17.6 with either); with the filter, hardly any tile has as many.
+    // merges of 1 GiB 16.42 ms, 16.7 if each takes one side of either kind); with the filter, hardly any tile has as many.
     const int n_heads = (int)(sum & 0xFFFFu), n_ends = (int)(sum >> 16);
     if (FV != FILTER_ON && n_heads + n_ends > 32) {
 #pragma unroll 1
