@@ -21,7 +21,7 @@
 //   pass 3  build_table_kernel: the slot index of a key starts with the same bits as its word, so a CTA that
 //           takes a range of words owns a range of slots.  It counts the words in shared memory and
 //           writes the slots out, occupied or not: the table is not cleared before and no atomic reaches L2.
-//           200 M ids, 31 M pairs: 1.6 ms for both passes (6.2 ms when every word was added to the table with
+//           200 M ids, 31 M pairs: 1.2 ms for both passes (6.2 ms when every word was added to the table with
 //           one or two atomics in L2, a partition at a time).
 // Several ranks: the owner of a partition adds its words out of every rank's regions
 // (partition_table_peers_kernel); the table slice that a launch touches stays in L2.  One rank does the same with a long
