@@ -130,7 +130,7 @@ __global__ void rows_write_kernel(const u64 *__restrict__ keys, const i64 *__res
 #define ROWS_LARGE_SMEM (ROWS_BYTE_PAIRS * 2 + ROWS_MIXED_SLOTS * 12)
 static_assert(ROWS_LARGE_SLOTS * 12 <= ROWS_LARGE_SMEM, "either layout fits");
 #define ROWS_LARGE_CELLS (1 << 18)
-#define ROWS_DIRECT_CELLS (1 << 15)
+#define ROWS_DIRECT_CELLS (1 << 16)
 #define ROWS_RANK_MAX 16384   // up to this many pairs are sorted by counting smaller keys, two launches instead of a radix sort's nine
 #define ROWS_RANK_TILE 512
 
@@ -255,10 +255,10 @@ __global__ void __launch_bounds__(ROWS_SMALL_NT) rows_pairs_kernel(const int32_t
     }
 }
 
-// Up to 2^15 cells, a pair per thread straight into the table, equal pairs of a warp together: collecting them first costs a
+// Up to 2^16 cells, a pair per thread straight into the table, equal pairs of a warp together: collecting them first costs a
 // chain of trips to L2 for every entry that a thread adds afterwards (count of 16 x 512 cells of text 75 us, now 63, of 32 x 1024 cells
-// with 32 736 pairs 212 and 174).  Beyond, and without the look at the warp, equal pairs queue up at their slot: 32 x 1024 equal cells
-// took 91 us instead of 50.
+// with 32 736 pairs 212 and 174; 64 x 1024 cells of text 74 and 58).  Equal pairs queue up at their slot: 32 x 1024 equal cells took
+// 91 us without the look at the warp, 50 with it as with tables; beyond 2^17 cells they are slower (255 x 1024: 64 and 50).
 __global__ void __launch_bounds__(ROWS_SMALL_NT) rows_pairs_direct_kernel(const int32_t *__restrict__ tokens, const uint8_t *__restrict__ valid, i64 cells,
                                                                           i64 L, RowsTable t) {
     const i64 i = (i64)blockIdx.x * ROWS_SMALL_NT + threadIdx.x;

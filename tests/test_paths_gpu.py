@@ -430,7 +430,7 @@ def test_pair_table_grows_in_mid_run():
     e.close()
 
 
-@pytest.mark.parametrize("rows,width,alphabet", [(1, 2, 4), (32, 1024, 1), (32, 1024, 300), (33, 993, 2), (33, 992, 70000), (64, 4095, 128), (64, 4096, 128), (64, 4096, 129), (16, 16385, 70000),
+@pytest.mark.parametrize("rows,width,alphabet", [(1, 2, 4), (64, 1024, 1), (64, 1024, 300), (65, 1009, 2), (65, 1008, 70000), (64, 4095, 128), (64, 4096, 128), (64, 4096, 129), (16, 16385, 70000),
                                                  (40, 4000, 70000)])
 def test_seam_count_at_its_table_and_rank_limits(rows, width, alphabet):
     # both shared-memory tables (from 2^18 cells on the large one), up to and beyond 16 384 pairs, and a repeated count
