@@ -13,7 +13,7 @@
 // vote of the CTAs on the best of them, the same step took 4.3 us instead of 1.5.)
 // A second counter keeps the CTAs apart the other way round: a CTA adds its deltas of merge m only when all have
 // read the counts that chose merge m (and CTA 0 has reset the step's counters); that wait runs under the rewriting of
-// the tiles.  Both counters are raised with release and polled with acquire.  (Raised without, `chosen` would rest on
+// the tiles, but for a delta that finds no place in the CTA's histogram, which waits at once (agg_probe).  Both counters are raised with release and polled with acquire.  (Raised without, `chosen` would rest on
 // loads whose values have been used.  The release holds up its warp, so it is done while warp 0 decides: 10 MB of
 // mixed text, 3 000 merges, 15.11 ms against 15.08 without any ordering; in front of the ranking, where a CTA barrier waits
 // for that warp, 15.30, and with relaxed polls and a fence behind them 16.5.)
@@ -42,8 +42,6 @@
 #pragma once
 #include "kernels.cuh"
 
-#define STBPE_LOOP_WAIT_NS 4000000000ull
-
 struct LoopArgs {
     int target;             // merge count to stop at
     const int2 *forced;     // host-given merges (a, b), applied in order before any choice ...
@@ -63,33 +61,6 @@ struct LoopArgs {
 #define STBPE_DRAWS 1024  // at most
 
 enum { LOOP_BEST, LOOP_NONE, LOOP_UNTIED };
-
-__device__ __forceinline__ u64 loop_timer_ns() {
-    u64 t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ void red_release_u32(unsigned int *p, unsigned int v) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int *p) {
-    unsigned int v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-// retries of a bounded wait; false when the time is up or another wait has given up
-struct BoundedWait {
-    u64 t0;
-    unsigned int n;
-    __device__ __forceinline__ BoundedWait() : t0(0), n(0) {}
-    __device__ __forceinline__ bool again(DevState *st) {
-        if ((++n & 1023u) != 0u) return true;
-        const u64 t = loop_timer_ns();
-        if (t0 == 0) t0 = t;
-        if (t - t0 > STBPE_LOOP_WAIT_NS) atomicOr(&st->error, STBPE_DERR_TIMEOUT);
-        return (*(volatile unsigned int *)&st->error & STBPE_DERR_TIMEOUT) == 0u;
-    }
-};
 
 // The arg-max in registers.  With 15-bit ids a pair and its count fit 64 bits whose order is the
 // order of the selection (larger count, then smaller key), and a warp's maximum is two redux steps.  That leaves 34
@@ -370,6 +341,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             }
             if (lane == 0) {
                 s.p->n = nb;
+                s.p->chosen = &sync->chosen, s.p->all_chosen = G * (step + 1);
                 s_go = nb;
                 s_tie = nb > 0 && draw;
                 s_ties = 0;

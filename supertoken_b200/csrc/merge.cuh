@@ -59,12 +59,44 @@ struct Batch<uint32_t> {
     static __device__ __forceinline__ uint32_t pair(uint32_t) { return 0u; }
     static __device__ __forceinline__ uint32_t home(uint32_t key) { return key; }
 };
+#define STBPE_LOOP_WAIT_NS 4000000000ull
+__device__ __forceinline__ u64 loop_timer_ns() {
+    u64 t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ void red_release_u32(unsigned int *p, unsigned int v) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int *p) {
+    unsigned int v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+// retries of a bounded wait; false when the time is up or another wait has given up
+struct BoundedWait {
+    u64 t0;
+    unsigned int n;
+    __device__ __forceinline__ BoundedWait() : t0(0), n(0) {}
+    __device__ __forceinline__ bool again(DevState *st) {
+        if ((++n & 1023u) != 0u) return true;
+        const u64 t = loop_timer_ns();
+        if (t0 == 0) t0 = t;
+        if (t - t0 > STBPE_LOOP_WAIT_NS) atomicOr(&st->error, STBPE_DERR_TIMEOUT);
+        return (*(volatile unsigned int *)&st->error & STBPE_DERR_TIMEOUT) == 0u;
+    }
+};
+
 struct BatchPairs {  // in shared memory
     PlaneId pa[8], pb[8];  // a and b once more, as Group::eq takes them
     uint32_t a[8], b[8], nw[8];
     i64 count[8];
     int touch[64];  // matches of pair i (row) followed at once by one of pair k (column)
     int n;
+    // the pair table stays as it is until this counter has reached this value: all CTAs have then read what they choose the
+    // batch by (null: they read nothing while the batch is applied)
+    const unsigned int *chosen;
+    unsigned int all_chosen;
     // called by the 32 lanes of a warp: word i of the masks is all ones where bit i of the id is set
     template <typename T>
     __device__ __forceinline__ void set_plane(int k, int lane) {
@@ -173,7 +205,8 @@ __device__ __forceinline__ u64 made_key(const BatchPairs *p, uint32_t k, uint32_
     return side ? (((u64)p->nw[k] << 32) | id) : (((u64)id << 32) | p->nw[k]);
 }
 
-// Slow path: probe for the entry, claim a free one, or give up.
+// Slow path: probe for the entry, claim a free one, or give up and add to the pair table, in the middle of the tiles: other
+// CTAs may still be choosing the batch by its counts.
 template <typename T, bool MG>
 static __device__ __noinline__ void agg_probe(uint32_t *agg_key, int *ctr, const EngineDev &e, const BatchPairs *p, i64 theta_count, u64 theta_key,
                                               uint32_t key) {
@@ -197,6 +230,11 @@ static __device__ __noinline__ void agg_probe(uint32_t *agg_key, int *ctr, const
             return;
         }
         h = (h + 1) & (STBPE_AGG - 1);
+    }
+    if (!MG && p->chosen) {
+        BoundedWait wait;
+        while (ld_acquire_u32(p->chosen) < p->all_chosen)
+            if (!wait.again(e.st)) return;  // the launch ends with STBPE_DERR_TIMEOUT
     }
     Theta theta;
     theta.count = theta_count, theta.key = theta_key;
@@ -784,7 +822,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) merge_kernel(const _
     s.carve<T>(smem_raw, s_ctr);
     s.clear();
     MergeCtx c;
-    if (threadIdx.x == 0) s.p->n = 1, s.p->a[0] = (uint32_t)st->cur_a, s.p->b[0] = (uint32_t)st->cur_b, s.p->nw[0] = (uint32_t)st->cur_new;
+    if (threadIdx.x == 0) s.p->n = 1, s.p->a[0] = (uint32_t)st->cur_a, s.p->b[0] = (uint32_t)st->cur_b, s.p->nw[0] = (uint32_t)st->cur_new, s.p->chosen = nullptr;
     c.m = st->merges_done;
     c.fv = st->filter_valid != 0;
     c.zero = false;  // done when the merge was selected

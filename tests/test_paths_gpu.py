@@ -509,11 +509,11 @@ def test_seam_count_of_byte_pairs_and_others(kind, rows, width, shift, filter_mo
     assert bool((keys[n:] == -1).all()) and not bool(counts[n:].any())
 
 
-def _drawn_run(ids, off, base_vocab, target, seed, device, start=None):
+def _drawn_run(ids, off, base_vocab, target, seed, device, start=None, slots=1 << 18):
     """Merges of a loop that breaks ties by random.Random(seed), drawn on the host or on the device, and the generator's state."""
     import random
     rng, merge, done = random.Random(seed), start, 0
-    e = _engine(ids, off, base_vocab, target)
+    e = _engine(ids, off, base_vocab, target, slots)
     trips = 0
     while done < target:
         n, count, cands = e.next_tied(merge, base_vocab + done, target - done - (merge is not None), rng if device else None)
@@ -550,3 +550,39 @@ def test_ties_drawn_where_the_loop_leaves_for_more_bits(base_vocab):
     off = _rows(ids, rng, 60)
     host, dev = (_drawn_run(ids, off, base_vocab, 40, 7, d, start=(1, 2)) for d in (False, True))
     assert host[:5] == dev[:5]
+
+
+def _crowded(pairs, tiles_per_cta, seed):
+    """Matches of the pairs (0, 1), (2, 3), ... in turn, each behind a token out of 30 000: every CTA meets more distinct
+    neighbours than its histogram has entries, so some go to the pair table while tiles are still being worked on."""
+    rng = np.random.RandomState(seed)
+    ctas = torch.cuda.get_device_properties(0).multi_processor_count
+    ids = rng.randint(16, 30000, tiles_per_cta * ctas * 1024).astype(np.int32)
+    n = len(ids) // 3 // pairs * pairs
+    k = rng.permutation(np.arange(n) % pairs)
+    ids[1:3 * n:3], ids[2:3 * n:3] = 2 * k, 2 * k + 1
+    keys = set()
+    for t in ids.reshape(-1, 1024)[::ctas]:  # the tiles of CTA 0
+        at = np.flatnonzero((t[:-1] < 16) & (t[:-1] % 2 == 0) & (t[1:] == t[:-1] + 1))
+        at = at[(at > 0) & (at < 1022)]
+        keys |= {(x, k, 0) for x, k in zip(t[at - 1].tolist(), t[at].tolist())} | {(y, k, 1) for y, k in zip(t[at + 2].tolist(), t[at].tolist())}
+    return ids, keys
+
+
+def test_more_neighbours_than_the_histogram_of_a_cta_has_entries():
+    ids, keys = _crowded(8, 9, 1)
+    assert len(keys) > 4096  # in one step, as all eight pairs go together
+    off = np.array([0, len(ids)], dtype=np.int64)
+    e = _engine(ids, off, 30000, 24, 1 << 23)
+    e.train(24)
+    _check(e, ids, off, 30000, 24)
+    e.close()
+
+
+def test_more_neighbours_than_entries_while_ties_are_drawn():
+    ids, keys = _crowded(2, 14, 2)
+    assert min(sum(k == p for _, k, _ in keys) for p in (0, 2)) > 4096  # for the one pair that is drawn
+    off = np.array([0, len(ids)], dtype=np.int64)
+    host, dev = (_drawn_run(ids, off, 30000, 6, 3, d, slots=1 << 23) for d in (False, True))
+    assert host[:5] == dev[:5]
+    assert dev[5] < host[5]  # the tie was broken on the device
