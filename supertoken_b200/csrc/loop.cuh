@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(MergeGeom<T>::THREADS, 1) loop_kernel(const __
             add_stats<T>(e, ws);
             return;
         }
-        if (cta == 0 && tid == 0 && step == 0) st->n_work = 0;
+        if (cta == 0 && tid == 0 && step == 0) st->n_work = fv ? 0 : -1;  // (what the last step visits is added when the CTAs leave)
         // ---- the merges
         merges_done += nb;
         forced_i += nb;

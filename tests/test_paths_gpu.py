@@ -586,3 +586,17 @@ def test_more_neighbours_than_entries_while_ties_are_drawn():
     host, dev = (_drawn_run(ids, off, 30000, 6, 3, d, slots=1 << 23) for d in (False, True))
     assert host[:5] == dev[:5]
     assert dev[5] < host[5]  # the tie was broken on the device
+
+
+@pytest.mark.parametrize("density,timed", [("0", False), ("0", True), ("1e30", False)])
+def test_tiles_that_the_last_step_visited(density, timed, monkeypatch):
+    # below zero: every tile; with the pair filter their number, here those of one pair in one tile
+    monkeypatch.setenv("STBPE_FILTER_DENSITY", density)
+    ids = np.random.RandomState(0).randint(10, 10000, 64 * 1024).astype(np.int32)
+    ids[5 * 1024 + 100:5 * 1024 + 300] = np.tile([1, 2], 100)
+    e = _engine(ids, np.array([0, len(ids)], dtype=np.int64), 10000, 1)
+    (e.train_timed if timed else e.train)(1)
+    assert e.merges()[0] == [(1, 2)]
+    visited = e.state().work_tiles
+    assert visited < 0 if density == "0" else 1 <= visited < 64
+    e.close()
