@@ -146,11 +146,12 @@ __global__ void rows_init_kernel(RowsTable t, unsigned int *rank, unsigned int n
     if (first < 3) t.n_keys[first] = 0;  // number of keys, error, export cursor
 }
 
-// key + n into the table; a table that fills up ends the count (the host repeats it with a larger one)
+// key + n into the table; a table that fills up ends the count (the host repeats it with a larger one).  Only the number of
+// keys says that it is full: a table of twice as many slots as the batch has pairs may well hold 64 keys side by side.
 __device__ __forceinline__ void rows_add(const RowsTable &t, u64 key, u64 n) {
     u64 h = mix64(key) & t.mask;
 #pragma unroll 1
-    for (int probe = 0; probe < 64; ++probe) {
+    for (u64 probe = 0; probe <= t.mask; ++probe) {
         Slot *s = &t.table[h];
         u64 k = __ldcg(&s->key);
         if (k == STBPE_EMPTY) {
@@ -165,6 +166,7 @@ __device__ __forceinline__ void rows_add(const RowsTable &t, u64 key, u64 n) {
             return;
         }
         h = (h + 1) & t.mask;
+        if ((probe & 63) == 63 && *(volatile unsigned int *)t.error) return;
     }
     atomicOr(t.error, 1u);
 }

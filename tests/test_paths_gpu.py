@@ -600,3 +600,19 @@ def test_tiles_that_the_last_step_visited(density, timed, monkeypatch):
     visited = e.state().work_tiles
     assert visited < 0 if density == "0" else 1 <= visited < 64
     e.close()
+
+
+@pytest.mark.parametrize("n", [60, 130, 256])
+def test_seam_count_of_pairs_that_start_at_one_slot(n):
+    # rows of one pair each, whose keys all begin their search at the same slot of the table (1024 slots for up to 512 pairs)
+    g = np.random.RandomState(n)
+    ab = g.randint(0, 1 << 30, (600000, 2)).astype(np.int32)
+    h = (ab[:, 0].astype(np.uint64) << np.uint64(32)) | ab[:, 1].astype(np.uint64)
+    for mul in (0xff51afd7ed558ccd, 0xc4ceb9fe1a85ec53, 1):
+        h = (h ^ (h >> np.uint64(33))) * np.uint64(mul)
+    t = torch.from_numpy(np.ascontiguousarray(ab[(h & np.uint64(1023)) == 1000][:n])).cuda()
+    assert t.shape[0] == n
+    keys, counts = torch.empty((n, 2), dtype=torch.int32, device="cuda"), torch.empty(n, dtype=torch.int64, device="cuda")
+    length = torch.empty(1, dtype=torch.int64, device="cuda")
+    ops.count_pairs(t, torch.ones_like(t, dtype=torch.uint8), keys, counts, length)
+    assert int(length) == n and sorted(map(tuple, keys.tolist())) == sorted(map(tuple, t.tolist())) and bool((counts == 1).all())
