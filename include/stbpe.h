@@ -134,10 +134,14 @@ int stbpe_next_tied(stbpe_engine *e, int32_t a, int32_t b, int32_t new_id, int32
 /* stbpe_next_tied that breaks ties itself while it can: draws = the next n_draws 32-bit outputs of the generator (at most
  * 1024 are looked at), out of which a tie of n pairs takes the top bits of one, as many as n has, again while they
  * are not below n, and with them a pair in ascending order (random.Random.randrange).  *n_used = the outputs taken.  It returns
- * before `most` when the draws run out, when more pairs are tied than it keeps (1024), and on a stream of 32-bit tokens. */
+ * before `most` when the draws run out, when more pairs are tied than it keeps (1024), and on a stream of 32-bit tokens
+ * (stbpe_token_bytes). */
 int stbpe_next_drawn(stbpe_engine *e, int32_t a, int32_t b, int32_t new_id, int32_t most, const uint32_t *draws,
                      int32_t n_draws, int32_t *n_used, int32_t *n_done, int64_t *count, uint64_t *keys, int64_t cap,
                      int64_t *n_ties, void *stream);
+
+/* Bytes per token of the stream as it is now: 2, or 4 from the first id on that takes more than 15 bits. */
+int stbpe_token_bytes(const stbpe_engine *e);
 
 /* The merge loop (gpu_tokenizer/bpe_trainer.py:4193-4517) run on the device without
  * a host round trip per merge: select -> stop rules -> apply, n_merges times or until a

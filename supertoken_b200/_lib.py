@@ -50,6 +50,7 @@ SIGNATURES = {
     "stbpe_apply_merges": (_int, [_vp, _vp, _i32, _i32, _vp]),
     "stbpe_next_drawn": (_int, [_vp, _i32, _i32, _i32, _i32, _vp, _i32, _P(_i32), _P(_i32), _P(_i64), _vp, _i64, _P(_i64), _vp]),
     "stbpe_next_tied": (_int, [_vp, _i32, _i32, _i32, _i32, _P(_i32), _P(_i64), _vp, _i64, _P(_i64), _vp]),
+    "stbpe_token_bytes": (_int, [_vp]),
     "stbpe_train": (_int, [_vp, _i32, _vp]),
     "stbpe_train_timed": (_int, [_vp, _i32, _P(ctypes.c_float), _vp]),
     "stbpe_repack": (_int, [_vp, _int, _P(_int), _vp]),

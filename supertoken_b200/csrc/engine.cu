@@ -1261,6 +1261,8 @@ STBPE_VISIBLE int stbpe_next_tied(stbpe_engine *e, int32_t a, int32_t b, int32_t
     return stbpe_next_drawn(e, a, b, new_id, most, nullptr, 0, nullptr, n_done, count, keys, cap, n_ties, stream);
 }
 
+STBPE_VISIBLE int stbpe_token_bytes(const stbpe_engine *e) { return e && e->wide ? 4 : 2; }
+
 static int maybe_repack(stbpe_engine *e, bool force, int *did, cudaStream_t s);
 
 // Keep or drop the pair filter.  A merge whose matches outnumber the tiles visits nearly every tile

@@ -616,3 +616,30 @@ def test_seam_count_of_pairs_that_start_at_one_slot(n):
     length = torch.empty(1, dtype=torch.int64, device="cuda")
     ops.count_pairs(t, torch.ones_like(t, dtype=torch.uint8), keys, counts, length)
     assert int(length) == n and sorted(map(tuple, keys.tolist())) == sorted(map(tuple, t.tolist())) and bool((counts == 1).all())
+
+
+@pytest.mark.parametrize("base_vocab,tied,calls", [(40000, 50, 0), (10000, 1100, 1)])
+def test_outputs_are_taken_ahead_only_where_the_device_may_draw(base_vocab, tied, calls):
+    # 32-bit tokens, and more tied pairs than the device keeps: rows of one pair each, all pairs twice
+    import random
+
+    class Counted(random.Random):
+        ahead = 0
+
+        def getrandbits(self, k):
+            self.ahead += k > 32
+            return super().getrandbits(k)
+
+    pairs = np.stack([np.arange(tied), np.arange(tied) + tied], 1).astype(np.int32)
+    ids = np.concatenate([pairs, pairs]).ravel()
+    e = _engine(ids, np.arange(0, len(ids) + 1, 2).astype(np.int64), base_vocab, 20)
+    rng, merge, left, want, plain = Counted(3), None, list(map(tuple, pairs.tolist())), [], random.Random(3)
+    for done in range(20):
+        want.append(left.pop(plain.randrange(len(left))))
+        _, count, cands = e.next_tied(merge, base_vocab + max(done - 1, 0), 20 - done, rng)
+        assert count == 2 and len(cands) == len(left) + 1
+        key = cands[rng.randrange(len(cands))]
+        merge = (key >> 32, key & 0xFFFFFFFF)
+        assert merge == want[-1]
+    assert rng.ahead == calls
+    e.close()
