@@ -534,22 +534,45 @@ def _drawn_run(ids, off, base_vocab, target, seed, device, start=None, slots=1 <
 @pytest.mark.parametrize("seed,n,alphabet,target", [(0, 3000, 6, 90), (1, 3000, 40, 150), (2, 40000, 300, 120), (3, 200, 200, 30), (4, 9000, 1000, 60),
                                                     (5, 70000, 12, 200), (6, 2500, 3, 400)])
 def test_ties_drawn_on_the_device_as_on_the_host(seed, n, alphabet, target):
-    # few and many tied pairs (more than the device keeps, too), counts that fall to the threshold and below 2, draws that run out
+    # few and many tied pairs, counts that fall to the threshold and below 2; the device breaks every tie, in one call
     rng = np.random.RandomState(seed)
     ids = rng.randint(0, alphabet, n).astype(np.int32)
     off = _rows(ids, rng, 90)
     host, dev = (_drawn_run(ids, off, 1000, target, seed, d) for d in (False, True))
     assert host[:5] == dev[:5]
-    assert dev[5] <= host[5]
+    assert dev[5] == 1 < host[5]
 
 
+@pytest.mark.parametrize("few", [None, 1, 3])
 @pytest.mark.parametrize("base_vocab", [508, 2040, 32760])
-def test_ties_drawn_where_the_loop_leaves_for_more_bits(base_vocab):
+def test_ties_drawn_while_the_ids_pass_a_number_of_bits(base_vocab, few, monkeypatch):
+    # The device looks at all bits of an id while it holds outputs of the generator, and may look at fewer once they have run
+    # out (few: as many per call).  From 32 767 on the tokens are 32 bits wide and the host breaks the ties.
     rng = np.random.RandomState(base_vocab)
     ids = rng.choice([1, 2, 3, 4, 5], 30000).astype(np.int32)
     off = _rows(ids, rng, 60)
+    if few is not None:
+        init = Engine.__init__
+
+        class Few:
+            def __init__(self, lib):
+                self.lib = lib
+
+            def __getattr__(self, name):
+                return getattr(self.lib, name)
+
+            def stbpe_next_drawn(self, h, a, b, new_id, most, words, n, *rest):
+                return self.lib.stbpe_next_drawn(h, a, b, new_id, most, words, min(n, few), *rest)
+
+        def with_few(self, *args, **kwargs):
+            init(self, *args, **kwargs)
+            self._lib = Few(self._lib)
+
+        monkeypatch.setattr(Engine, "__init__", with_few)
     host, dev = (_drawn_run(ids, off, base_vocab, 40, 7, d, start=(1, 2)) for d in (False, True))
     assert host[:5] == dev[:5]
+    if few is None and base_vocab < 32760:
+        assert dev[5] == 1 < host[5]
 
 
 def _crowded(pairs, tiles_per_cta, seed):
