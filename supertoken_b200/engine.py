@@ -157,12 +157,13 @@ class Engine:
         if max(a, b) > 0x7FFFFFFE or new_id + most > 0x7FFFFFFE or (merge is not None and min(a, b) < 0):
             raise OverflowError("Token id overflow: ids must be in [0, 2^31-2]")
         if getattr(self, "_tied", None) is None:
-            self._tied, self._n_tied = np.empty(1024, dtype=np.uint64), 0
+            self._tied, self._not_ahead, self._pause = np.empty(1024, dtype=np.uint64), 0, 0
         words, n_draws = None, 0
         # The generator's next outputs (the first one in the lowest bits), without moving it.  That costs some 15 us, so not
-        # where the device breaks no tie: on 32-bit tokens (300 ties 26.3 ms, 23.3 without) and while more pairs are tied than
-        # it keeps, as they were a call ago (300 merges among 3 000 pairs 249 ms, 241 without).
-        if rng is not None and most > 0 and self._n_tied <= len(self._tied) and self._lib.stbpe_token_bytes(self._h) == 2:
+        # where the device breaks no tie: on 32-bit tokens (300 ties 26.3 ms, 22.2 without), and not for the next 1, 3, 7, 15,
+        # 15, ... calls when it has left one to the host, as it does while more pairs are tied than it keeps or its list of
+        # candidates is sure of (300 merges among 1 200 pairs: 2.2 of 83.8 ms).
+        if rng is not None and most > 0 and self._not_ahead == 0 and self._lib.stbpe_token_bytes(self._h) == 2:
             n_draws = min(2 * most + 16, 1024)
             before = rng.getstate()
             words = rng.getrandbits(32 * n_draws).to_bytes(4 * n_draws, "little")
@@ -174,7 +175,11 @@ class Engine:
                                                self._s))
         if used.value:
             rng.getrandbits(32 * used.value)
-        self._n_tied = n.value
+        if n_draws:
+            self._pause = min(2 * self._pause + 1, 15) if not used.value and n.value > 1 else 0
+            self._not_ahead = self._pause
+        elif self._not_ahead:
+            self._not_ahead -= 1
         if count.value <= 0:
             return done.value, 0, []
         if n.value > len(self._tied):
