@@ -1419,7 +1419,8 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
             if (rc != STBPE_OK) return rc;
         }
     }
-    int planes_due = 0;  // the next id needs more planes than this
+    int planes_due = 0;  // a merge that is due needs more planes than this
+    int merges = e->merges_done;
     for (;;) {
         const int grid = e->sm_count;  // one CTA per SM; the barrier is no faster with fewer
         la.target = target;
@@ -1436,16 +1437,23 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
         la.draws = draws ? draws->dev + draws->used : nullptr;
         la.n_draws = draws ? draws->n - draws->used : 0;
         EngineDev d = e->d;
-        // Bits of an id that the loop looks at: as few as all ids, old and new, allow.  It returns for the id that needs more,
-        // which costs a launch (some 40 us): nine bits only where steps are long (over 8192 tiles one takes 25 us and a tenth
-        // of it is saved), thirteen where the filter is in use (8 000 merges of 256 MiB: 68 million visits, 2 % off each).
+        // Bits of an id that the loop looks at: as few as all ids allow, old ones and the new ones of the next merges.  For the
+        // id that needs more it returns, which costs a launch of 25 to 35 us.  That is earned back where steps are long: over
+        // 8192 tiles nine bits lose 22 us against eleven when they serve for 32 merges and gain 14 at 64 (over 2^17 tiles 50 and
+        // 123); eleven against fifteen over 16384 tiles -6 at 32 and 29 at 128; thirteen over 65536 tiles -2 at 128 and 38 at
+        // 512.  Over 1024 tiles nothing does (eleven for 512 merges: -25), so there they have to serve for all that are left.
         int planes = 15;
         const bool drawing = la.n_draws > 0 && !e->wide;
         if (!e->wide && !drawing) {
-            auto enough = [&](int p) { return p > planes_due && la.ids_below < (1 << p) - 1; };
-            if (!e->filter_valid && e->d.n_tiles >= 8192 && enough(9)) planes = 9;
-            else if (enough(11)) planes = 11;
-            else if (e->filter_valid && enough(13)) planes = 13;
+            const bool long_steps = e->d.n_tiles >= 8192;
+            const i64 next = mode == LOOP_BEST ? (i64)e->cfg.base_vocab + merges : (i64)la.forced_new, left = (i64)target - merges;
+            auto enough = [&](int p, i64 worth) {
+                const i64 ids = (1 << p) - 1;
+                return p > planes_due && la.ids_below < ids && next + (long_steps ? std::min(left, worth) : left) <= ids;
+            };
+            if (!e->filter_valid && long_steps && enough(9, 64)) planes = 9;
+            else if (enough(11, 128)) planes = 11;
+            else if (e->filter_valid && enough(13, 512)) planes = 13;
         }
         // Candidates that have run out are collected in front of the launch without waiting for the result: one pass
         // settles the threshold but for tables with very many equal counts, and then the launch comes back at once.
@@ -1475,6 +1483,7 @@ static int run_loop(stbpe_engine *e, int target, int mode, const int2 *forced, i
         }
         if (int rc_ = read_state(e, out, s)) return rc_;
         at += out->forced_done;
+        merges = out->merges_done;
         if (draws) draws->used += out->draws_used;
         e->made_below = std::max(e->made_below, mode == LOOP_BEST ? (i64)e->cfg.base_vocab + out->merges_done : (i64)forced_new + at);
         if (n_done) *n_done = at;

@@ -670,3 +670,42 @@ def test_outputs_are_taken_ahead_only_where_the_device_may_draw(base_vocab, tied
         assert merge == want[-1]
     assert rng.ahead == calls
     e.close()
+
+
+def _loop_launches(run):
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        run()
+        torch.cuda.synchronize()
+    return sum("loop_kernel" in ev.name for ev in prof.events())
+
+
+@pytest.mark.parametrize("base_vocab,tiles", [(2047, 40), (2040, 40), (8191, 40), (505, 8192), (2047, 8192)])
+def test_no_launch_that_leaves_for_the_bits_of_its_first_ids(base_vocab, tiles, filter_mode, monkeypatch):
+    if filter_mode == "policy":
+        monkeypatch.setenv("STBPE_FILTER_DENSITY", "0")
+    rng = np.random.RandomState(base_vocab)
+    data = rng.randint(0, 200, tiles * 1024, dtype=np.uint8)
+    e = Engine(len(data), base_vocab=base_vocab, max_merges=20)
+    e.append_bytes(data, np.array([0, len(data)], dtype=np.int64))
+    e.count_initial()
+    # (with the filter, the first launch returns for the host to build it)
+    assert _loop_launches(lambda: e.train(20)) == (1 if filter_mode == "policy" else 2)
+    assert len(e.merges()[0]) == 20
+    e.close()
+
+
+@pytest.mark.parametrize("base_vocab,target", [(441, 90), (1917, 150), (7676, 530)])
+def test_long_streams_pass_nine_eleven_and_thirteen_bits_in_mid_run(base_vocab, target, filter_mode, monkeypatch):
+    # enough merges before the bound to look at fewer bits up to it: 64 below 511, 128 below 2 047, 512 below 8 191
+    if filter_mode == "policy":
+        if target == 530:
+            pytest.skip("thirteen bits only with the filter")
+        monkeypatch.setenv("STBPE_FILTER_DENSITY", "0")
+    rng = np.random.RandomState(target)
+    ids = rng.randint(0, 200, 8192 * 1024 - 100).astype(np.int32)
+    off = _rows(ids, rng, 4000)
+    e = _engine(ids, off, base_vocab, target, 1 << 20)
+    e.train(target)
+    _check(e, ids, off, base_vocab, target)
+    e.close()
