@@ -138,9 +138,9 @@ __global__ void __launch_bounds__(STBPE_PART_THREADS, 1)
             });
         if (base + step < n_units) load_unit_batch<T, UNROLL, STBPE_PART_THREADS>(units, base + step, n_units, v, nx);
         __syncthreads();
-        // flush into this CTA's regions: a warp serves its eight rings four at a time, eight lanes per ring, so that a turn stores
-        // whole sectors (eight rings at once, four lanes each, took as many turns of half sectors: the pass over 200 M ids
-        // 0.75 ms, now 0.68; one ring at a time cost eight times the bookkeeping)
+        // flush into this CTA's regions: a warp serves its eight rings four at a time, eight lanes per ring, 32
+        // consecutive bytes a turn, which start where the region has got to (eight rings at once, four lanes each, took as many
+        // turns of 16 bytes: the pass over 200 M ids 0.75 ms, now 0.68; one ring at a time cost eight times the bookkeeping)
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const int p = warp * (STBPE_PARTS / (STBPE_PART_THREADS / 32)) + half * 4 + (lane >> 3);
